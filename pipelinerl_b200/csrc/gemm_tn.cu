@@ -30,7 +30,14 @@ constexpr int kBK = 64;         // bf16 per k-block row = one 128-B swizzle atom
 constexpr int kStages = 6;
 constexpr int kStageBytes = 2 * kHalf * kBK * 2;  // 32 KB
 constexpr int kMnChunkBytes = 64 * kBK * 2;        // one 64(MN) x 64(k) box of an MN-major operand: 8 KB
-constexpr int kThreadsTN = 192;
+constexpr int kEpiBytes = 4096;  // staging of one epilogue warp: 32 rows x 128 B (fp32 chunk), or twice 32 rows x 64 B (bf16)
+// Epilogue warps: two per TMEM lane quarter, each with every other 64-column group.  One per quarter leaves one warp per
+// scheduler, and the SiLU epilogue (exponential, division, three stores) was then longer than a K = 3584 main loop.  The head's
+// statistics stay with one thread per row.
+template <bool kHead> constexpr int kEpiWarps = kHead ? 4 : 8;
+template <bool kHead> constexpr int kThreadsTN = 64 + 32 * kEpiWarps<kHead>;
+constexpr int kSmemTN = kStages * kStageBytes + 8 * kEpiBytes + 1024 + 8 * (2 * kStages + 4) + 16;
+static_assert(kSmemTN <= 232448, "the ring and the epilogue staging exceed the 227 KB shared-memory limit");
 constexpr int kGroupM = 8;      // row tiles per raster super-group
 
 struct TnParams {
@@ -42,6 +49,7 @@ struct TnParams {
   int split;         // > 1 (fp32 output, plain epilogue): the k-blocks of a tile are shared by `split` clusters' worth of work, slice s of
                      // C = rows s * M .. of an output [split][M][ldc] that the consumer sums
   int m_tiles, n_tiles;
+  int tile_n;        // output columns per tile (multiple of 16, at most 256): pick_tile_n
   int a_mn, b_mn;    // operand stored MN-major: A as [K, M] / B as [K, N] row-major (no transposed copy needed)
   void* C;
   int64_t ldc;
@@ -90,7 +98,7 @@ struct TnParams {
 
 // 0.5 z (1 + tanh(u)) = z sigmoid(2 u), u = sqrt(2 / pi) (z + 0.044715 z^3)
 __device__ __forceinline__ float gelu_tanh(float z) {
-  return z / (1.f + __expf(-1.5957691216057308f * (z + 0.044715f * z * z * z)));
+  return div_ge1(z, 1.f + __expf(-1.5957691216057308f * (z + 0.044715f * z * z * z)));
 }
 
 // k-blocks of work item t: all of them, or the item's share of a split tile (items of a tile are neighbours)
@@ -116,13 +124,68 @@ __device__ __forceinline__ void tile_coords(int t, const TnParams& p, int& tm, i
   tn = r / rows;
 }
 
+// ---- epilogue staging -------------------------------------------------------------------------------------------------------
+// tcgen05.ld hands a thread one output ROW, so stores straight from the registers touch 32 rows per instruction and every
+// access is a sector of its own: the fp32 accumulate epilogue (152064 x 3584, K = 2048) took 3.02 ms against 1.4 ms of
+// products, 1.69 ms now.  A warp therefore turns each 32-column chunk through its own shared memory (no barrier across warps):
+// rows go in as 16-byte pieces under an XOR swizzle (conflict-free both ways) and come out with 8 lanes on one row's 128
+// bytes, so residual, accumulated and stored values move in whole lines.
+__device__ __forceinline__ void sts16(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ uint4 lds16(uint32_t a) {
+  uint4 u;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "r"(a) : "memory");
+  return u;
+}
+// 128-byte rows (32 fp32): piece `c` (16 bytes) of row `r`
+__device__ __forceinline__ uint32_t at128(uint32_t st, int r, int c) { return st + (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
+// 64-byte rows (32 bf16): two rows share a 128-byte line
+__device__ __forceinline__ uint32_t at64(uint32_t st, int r, int c) {
+  return st + (uint32_t)(r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
+}
+__device__ __forceinline__ void stage_bf16_row(uint32_t st, int lane, const uint32_t (&h)[16]) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c) sts16(at64(st, lane, c), h[4 * c], h[4 * c + 1], h[4 * c + 2], h[4 * c + 3]);
+}
+// the warp's staged 32 x 32 bf16 chunk to `dst` (the chunk's first column in row 0 of the tensor): 4 lanes per row, 16 bytes each.
+// my_row: this lane's destination row or -1
+__device__ __forceinline__ void store_bf16_chunk(uint32_t st, int lane, int my_row, __nv_bfloat16* dst, int64_t ld, int n_ok, bool vec) {
+  const int c = lane & 3;
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int r = it * 8 + (lane >> 2);
+    const int row = __shfl_sync(0xffffffffu, my_row, r);
+    const uint4 u = lds16(at64(st, r, c));
+    if (row >= 0) {
+      __nv_bfloat16* d = dst + (int64_t)row * ld + c * 8;
+      if (vec && c * 8 + 8 <= n_ok) {
+        *reinterpret_cast<uint4*>(d) = u;
+      } else {
+        const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&u);
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (c * 8 + e < n_ok) d[e] = h[e];
+      }
+    }
+  }
+}
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ bool aligned16(const void* p, int64_t ld_bytes) {
+  return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)ld_bytes) & 15) == 0;
+}
+
 template <bool kHead>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsTN, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsTN<kHead>, 1)
 gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                const __grid_constant__ CUtensorMap tm_a2, const __grid_constant__ CUtensorMap tm_b2, TnParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t bar_base = smem_base + (uint32_t)(kStages * kStageBytes);
+  const uint32_t epi_base = smem_base + (uint32_t)(kStages * kStageBytes);
+  const uint32_t bar_base = epi_base + 8u * (uint32_t)kEpiBytes;
   auto full_bar = [&](int s) { return bar_base + 8u * (uint32_t)s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (uint32_t)(kStages + s); };
   auto acc_full_bar = [&](int a) { return bar_base + 8u * (uint32_t)(2 * kStages + a); };       // MMA -> epilogue
@@ -162,20 +225,28 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
 
   if (warp == 0) {
     // ===== TMA producer (both CTAs) =====
-    if (lane == 0) {
-      int it = 0;
-      for (int t = cluster; t < total_tiles; t += n_clusters) {
-        int tm, tn;
-        tile_coords(t, p, tm, tn);
-        int kb0, kb1;
-        k_range(t, p, kb0, kb1);
-        const int a_row = (p.g_tiles ? p.g_tiles[3 * tm + 1] : tm * kTile) + (int)rank * kHalf;
-        const int b_row = p.g_tiles ? p.g_tiles[3 * tm] * (int)p.N + tn * kTile + (int)rank * kHalf : p.swiglu_I ? tn * kHalf + (int)rank * (int)p.swiglu_I : tn * kTile + (int)rank * kHalf;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % kStages;
-          const uint32_t ph = (uint32_t)((it / kStages) & 1);
-          ptx::mbar_wait(empty_bar(s), ph ^ 1u);
-          if (rank == 0) ptx::mbar_arrive_expect_tx(full_bar(s), 2u * (uint32_t)kStageBytes);
+    // Both issuing warps run CONVERGED and elect one lane around each batch of instructions: from inside `if (lane == 0)`
+    // every UMMA / TMA pays an operand waterfall of ~180 cycles (tc_ptx.cuh, elect_one), more than the 128 cycles of a
+    // 256 x 256 x 16 UMMA -- the main loop then took ~700 cycles per k-block whatever the tile's width.
+    int it = 0;
+    for (int t = cluster; t < total_tiles; t += n_clusters) {
+      int tm, tn;
+      tile_coords(t, p, tm, tn);
+      int kb0, kb1;
+      k_range(t, p, kb0, kb1);
+      const int half_n = p.tile_n >> 1;
+      const int a_row = ptx::warp_uniform((p.g_tiles ? p.g_tiles[3 * tm + 1] : tm * kTile) + (int)rank * kHalf);
+      const int b_row = ptx::warp_uniform(p.g_tiles ? p.g_tiles[3 * tm] * (int)p.N + tn * kTile + (int)rank * kHalf
+                                          : p.swiglu_I ? tn * kHalf + (int)rank * (int)p.swiglu_I
+                                                       : tn * p.tile_n + (int)rank * half_n);
+      // an MN-major B arrives in 64-column boxes, whole ones also where the tile ends inside one
+      const uint32_t stage_tx = (uint32_t)(kHalf * kBK * 2 + (p.b_mn ? (half_n > 64 ? 2 : 1) * kMnChunkBytes : half_n * kBK * 2));
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        const int s = it % kStages;
+        const uint32_t ph = (uint32_t)((it / kStages) & 1);
+        ptx::mbar_wait(empty_bar(s), ph ^ 1u);
+        if (ptx::elect_one()) {
+          if (rank == 0) ptx::mbar_arrive_expect_tx(full_bar(s), 2u * stage_tx);
           else ptx::mbar_arrive_remote(full_bar(s), 0);
           const uint32_t a_dst = smem_base + (uint32_t)(s * kStageBytes);
           const uint32_t b_dst = a_dst + kHalf * kBK * 2;
@@ -192,23 +263,25 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             ptx::tma_load_2d_2sm(b_dst, tb, kk, b_row, full_bar(s), ptx::kEvictNormal);
           } else {
             ptx::tma_load_2d_2sm(b_dst, tb, b_row, kk, full_bar(s), ptx::kEvictNormal);
-            ptx::tma_load_2d_2sm(b_dst + kMnChunkBytes, tb, b_row + 64, kk, full_bar(s), ptx::kEvictNormal);
+            if (half_n > 64) ptx::tma_load_2d_2sm(b_dst + kMnChunkBytes, tb, b_row + 64, kk, full_bar(s), ptx::kEvictNormal);
           }
         }
+        __syncwarp();
       }
     }
   } else if (warp == 1) {
     // ===== MMA issuer (leader CTA only) =====
-    if (lane == 0 && rank == 0) {
-      const uint32_t idesc = ptx::make_idesc_bf16_f32(kTile, kTile) | ((uint32_t)p.a_mn << 15) | ((uint32_t)p.b_mn << 16);
+    if (rank == 0) {
+      const uint32_t idesc = ptx::make_idesc_bf16_f32(kTile, p.tile_n) | ((uint32_t)p.a_mn << 15) | ((uint32_t)p.b_mn << 16);
       const uint64_t a_step = p.a_mn ? 128u : 2u, b_step = p.b_mn ? 128u : 2u;  // K += 16 in (addr >> 4) units
+      const uint32_t tm0 = ptx::warp_uniform(tmem_base), sm0 = ptx::warp_uniform(smem_base);
       int it = 0, local = 0;
       for (int t = cluster; t < total_tiles; t += n_clusters, ++local) {
         const int acc = local & 1;
         const uint32_t acc_ph = (uint32_t)((local >> 1) & 1);
         ptx::mbar_wait(acc_empty_bar(acc), acc_ph ^ 1u);  // both CTAs' epilogues have drained this accumulator
         ptx::tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + (uint32_t)(acc * kTile);
+        const uint32_t d_tmem = tm0 + (uint32_t)(acc * kTile);
         int kb0, kb1;
         k_range(t, p, kb0, kb1);
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
@@ -216,33 +289,38 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
           const uint32_t ph = (uint32_t)((it / kStages) & 1);
           ptx::mbar_wait(full_bar(s), ph);
           ptx::tc_fence_after_sync();
-          const uint32_t a_addr = smem_base + (uint32_t)(s * kStageBytes);
+          const uint32_t a_addr = sm0 + (uint32_t)(s * kStageBytes);
           const uint32_t b_addr = a_addr + kHalf * kBK * 2;
           const uint64_t a_desc = p.a_mn ? ptx::make_mnmajor_sw128_desc(a_addr, kMnChunkBytes) : ptx::make_kmajor_sw128_desc(a_addr);
           const uint64_t b_desc = p.b_mn ? ptx::make_mnmajor_sw128_desc(b_addr, kMnChunkBytes) : ptx::make_kmajor_sw128_desc(b_addr);
+          if (ptx::elect_one()) {
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k)
-            ptx::mma_bf16_ss_2sm(d_tmem, a_desc + a_step * (uint64_t)k, b_desc + b_step * (uint64_t)k, idesc,
-                                 (kb > kb0 || k > 0) ? 1u : 0u);
-          ptx::tc_commit_2sm(empty_bar(s), 3);
+            for (int k = 0; k < kBK / 16; ++k)
+              ptx::mma_bf16_ss_2sm(d_tmem, a_desc + a_step * (uint64_t)k, b_desc + b_step * (uint64_t)k, idesc,
+                                   (kb > kb0 || k > 0) ? 1u : 0u);
+            ptx::tc_commit_2sm(empty_bar(s), 3);
+          }
+          __syncwarp();
         }
-        ptx::tc_commit_2sm(acc_full_bar(acc), 3);
+        if (ptx::elect_one()) ptx::tc_commit_2sm(acc_full_bar(acc), 3);
+        __syncwarp();
       }
     }
     __syncwarp();
   } else {
-    // ===== epilogue (both CTAs): thread = one output row, 256 columns in 32-column chunks =====
+    // ===== epilogue (both CTAs): a thread reads one accumulator row from TMEM, 32 columns at a time =====
     const int q = warp & 3;
+    const int half = kHead ? 0 : (warp - 2) >> 2;                // which of the quarter's two warps
+    const uint32_t st = epi_base + (uint32_t)(warp - 2) * (uint32_t)kEpiBytes;
     int local = 0;
     for (int t = cluster; t < total_tiles; t += n_clusters, ++local) {
       int tm, tn;
       tile_coords(t, p, tm, tn);
       const int acc = local & 1;
       const uint32_t acc_ph = (uint32_t)((local >> 1) & 1);
-      ptx::mbar_wait(acc_full_bar(acc), acc_ph);
-      ptx::tc_fence_after_sync();
+      const uint32_t acc_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kTile);
       int64_t row = (int64_t)tm * kTile + (int64_t)rank * kHalf + q * 32 + lane;
-      const int64_t col0 = (int64_t)tn * kTile;
+      const int64_t col0 = (int64_t)tn * p.tile_n;
       bool row_ok = row < p.M;
       float row_w = 0.f;
       if (!kHead && p.g_tiles) {
@@ -255,6 +333,9 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
           else row = pair;
         }
       }
+      const int my_row = row_ok ? (int)row : -1;
+      ptx::mbar_wait(acc_full_bar(acc), acc_ph);
+      ptx::tc_fence_after_sync();
       if constexpr (kHead) {
         // thread = one token; online softmax statistics over this tile's 256 vocabulary columns, all thread-local
         constexpr float kLog2e = 1.4426950408889634f;
@@ -269,36 +350,29 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
           for (int c0 = 0; c0 < kTile; c0 += 32) {
             if (col0 + c0 >= p.N) break;
             uint32_t r[32];
-            ptx::tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kTile + c0), r);
+            ptx::tmem_ld_32x32b_x32(acc_addr + (uint32_t)c0, r);
             ptx::tmem_ld_wait();
-            if (!row_ok) continue;
             const int64_t col = col0 + c0;
             const int n_ok = (int)((p.N - col) < 32 ? (p.N - col) : 32);
-            __nv_bfloat16* dst = p.dz + row * p.ld_dz + col;
             const uint64_t rel = (uint64_t)(tgt - col);
-            float g[32];
+            uint32_t h[16];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float lp = __uint_as_float(r[j]) * p.alpha - lse;
-              const float pr = __expf(lp);
-              float v = -gl * pr - ge * pr * (lp + H);
-              if (rel == (uint64_t)j) v += gl;
-              g[j] = v * p.alpha;
-            }
-            if (n_ok == 32) {
+            for (int j = 0; j < 32; j += 2) {
+              float g[2];
 #pragma unroll
-              for (int j = 0; j < 32; j += 8) {
-                uint4 u;
-                __nv_bfloat162* hb = reinterpret_cast<__nv_bfloat162*>(&u);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) hb[e] = __floats2bfloat162_rn(g[j + 2 * e], g[j + 2 * e + 1]);
-                *reinterpret_cast<uint4*>(dst + j) = u;
+              for (int e = 0; e < 2; ++e) {
+                const float lp = __uint_as_float(r[j + e]) * p.alpha - lse;
+                const float pr = __expf(lp);
+                float v = -gl * pr - ge * pr * (lp + H);
+                if (rel == (uint64_t)(j + e)) v += gl;
+                g[e] = v * p.alpha;
               }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (j < n_ok) dst[j] = __float2bfloat16_rn(g[j]);
+              h[j >> 1] = pack2(g[0], g[1]);
             }
+            stage_bf16_row(st, lane, h);
+            __syncwarp();
+            store_bf16_chunk(st, lane, my_row, p.dz + col, p.ld_dz, n_ok, aligned16(p.dz, p.ld_dz * 2));
+            __syncwarp();
           }
         } else {
         float m = -INFINITY, ssum = 0.f, usum = 0.f, zt = -INFINITY;
@@ -306,7 +380,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
         for (int c0 = 0; c0 < kTile; c0 += 32) {
           if (col0 + c0 >= p.N) break;
           uint32_t r[32];
-          ptx::tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kTile + c0), r);
+          ptx::tmem_ld_32x32b_x32(acc_addr + (uint32_t)c0, r);
           ptx::tmem_ld_wait();
           const int64_t col = col0 + c0;
           const int n_ok = (int)((p.N - col) < 32 ? (p.N - col) : 32);
@@ -342,116 +416,98 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
         // columns 0..127 of the accumulator = gate, 128..255 = up of features [tn * 128, tn * 128 + 128)
         const int64_t f0 = (int64_t)tn * kHalf;
 #pragma unroll 1
-        for (int c0 = 0; c0 < kHalf; c0 += 32) {
+        for (int c0 = half * 64; c0 < half * 64 + 64; c0 += 32) {
           uint32_t rg[32], ru[32];
-          ptx::tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kTile + c0), rg);
-          ptx::tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kTile + kHalf + c0), ru);
+          ptx::tmem_ld_32x32b_x32(acc_addr + (uint32_t)c0, rg);
+          ptx::tmem_ld_32x32b_x32(acc_addr + (uint32_t)(kHalf + c0), ru);
           ptx::tmem_ld_wait();
-          if (!row_ok) continue;
-          __nv_bfloat16* ap = p.act + row * p.ld_act + f0 + c0;
-          __nv_bfloat16* gp = p.C ? reinterpret_cast<__nv_bfloat16*>(p.C) + row * p.ldc + f0 + c0 : nullptr;
+          uint32_t ha[16], hg[16], hu[16];
 #pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            uint4 ua, ug, uu;
-            __nv_bfloat162* ha = reinterpret_cast<__nv_bfloat162*>(&ua);
-            __nv_bfloat162* hg = reinterpret_cast<__nv_bfloat162*>(&ug);
-            __nv_bfloat162* hu = reinterpret_cast<__nv_bfloat162*>(&uu);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              // same rounding points as the two-kernel path: gate_up is rounded to bf16 first, SiLU * up is taken of the
-              // ROUNDED values (prl_silu_mul_fwd reads the bf16 tensor), so fused and unfused results are bit-identical
-              if (p.swiglu_fp32) {   // sampler prefill: identical bits to the fp32 GEMM output + silu_mul_kernel pair
-                const float g0 = __uint_as_float(rg[j + 2 * e]), g1 = __uint_as_float(rg[j + 2 * e + 1]);
-                const float u0 = __uint_as_float(ru[j + 2 * e]), u1 = __uint_as_float(ru[j + 2 * e + 1]);
-                if (p.glu_gelu) {
-                  ha[e] = __floats2bfloat162_rn(gelu_tanh(g0) * u0, gelu_tanh(g1) * u1);
-                  continue;
-                }
-                if (p.glu_limit > 0.f) {
-                  const float l = p.glu_limit, b = p.glu_beta;
-                  const float c0g = fminf(g0, l), c1g = fminf(g1, l);
-                  const float c0u = fminf(fmaxf(u0, -l), l), c1u = fminf(fmaxf(u1, -l), l);
-                  ha[e] = __floats2bfloat162_rn(c0g / (1.f + __expf(-b * c0g)) * (c0u + 1.f),
-                                                c1g / (1.f + __expf(-b * c1g)) * (c1u + 1.f));
-                  continue;
-                }
-                ha[e] = __floats2bfloat162_rn((g0 / (1.f + __expf(-g0))) * u0, (g1 / (1.f + __expf(-g1))) * u1);
-                continue;
+          for (int j = 0; j < 16; ++j) {
+            // same rounding points as the two-kernel path: gate_up is rounded to bf16 first, SiLU * up is taken of the
+            // ROUNDED values (prl_silu_mul_fwd reads the bf16 tensor), so fused and unfused results are bit-identical
+            const float g0 = __uint_as_float(rg[2 * j]), g1 = __uint_as_float(rg[2 * j + 1]);
+            const float u0 = __uint_as_float(ru[2 * j]), u1 = __uint_as_float(ru[2 * j + 1]);
+            if (p.swiglu_fp32) {   // sampler prefill: identical bits to the fp32 GEMM output + silu_mul_kernel pair
+              if (p.glu_gelu) {
+                ha[j] = pack2(gelu_tanh(g0) * u0, gelu_tanh(g1) * u1);
+              } else if (p.glu_limit > 0.f) {
+                const float l = p.glu_limit, b = p.glu_beta;
+                const float c0g = fminf(g0, l), c1g = fminf(g1, l);
+                const float c0u = fminf(fmaxf(u0, -l), l), c1u = fminf(fmaxf(u1, -l), l);
+                ha[j] = pack2(div_ge1(c0g, 1.f + __expf(-b * c0g)) * (c0u + 1.f), div_ge1(c1g, 1.f + __expf(-b * c1g)) * (c1u + 1.f));
+              } else {
+                ha[j] = pack2(div_ge1(g0, 1.f + __expf(-g0)) * u0, div_ge1(g1, 1.f + __expf(-g1)) * u1);
               }
-              hg[e] = __floats2bfloat162_rn(__uint_as_float(rg[j + 2 * e]), __uint_as_float(rg[j + 2 * e + 1]));
-              hu[e] = __floats2bfloat162_rn(__uint_as_float(ru[j + 2 * e]), __uint_as_float(ru[j + 2 * e + 1]));
-              const float2 g = __bfloat1622float2(hg[e]), u = __bfloat1622float2(hu[e]);
-              ha[e] = __floats2bfloat162_rn(g.x / (1.f + __expf(-g.x)) * u.x, g.y / (1.f + __expf(-g.y)) * u.y);
-            }
-            *reinterpret_cast<uint4*>(ap + j) = ua;
-            if (gp) {
-              *reinterpret_cast<uint4*>(gp + j) = ug;
-              *reinterpret_cast<uint4*>(gp + p.swiglu_I + j) = uu;
+            } else {
+              hg[j] = pack2(g0, g1);
+              hu[j] = pack2(u0, u1);
+              const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hg[j]));
+              const float2 u = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hu[j]));
+              ha[j] = pack2(div_ge1(g.x, 1.f + __expf(-g.x)) * u.x, div_ge1(g.y, 1.f + __expf(-g.y)) * u.y);
             }
           }
+          stage_bf16_row(st, lane, ha);
+          const bool keep = p.C != nullptr;
+          if (keep) stage_bf16_row(st + 2048, lane, hg);
+          __syncwarp();
+          store_bf16_chunk(st, lane, my_row, p.act + f0 + c0, p.ld_act, 32, aligned16(p.act, p.ld_act * 2));
+          if (keep) {
+            __nv_bfloat16* gp = reinterpret_cast<__nv_bfloat16*>(p.C) + f0 + c0;
+            const bool vec = aligned16(p.C, p.ldc * 2);
+            store_bf16_chunk(st + 2048, lane, my_row, gp, p.ldc, 32, vec);
+            __syncwarp();
+            stage_bf16_row(st, lane, hu);
+            __syncwarp();
+            store_bf16_chunk(st, lane, my_row, gp + p.swiglu_I, p.ldc, 32, vec);   // swiglu_I is a multiple of 128
+          }
+          __syncwarp();
         }
       } else {
+      const int n_tile = (int)((p.N - col0) < p.tile_n ? (p.N - col0) : p.tile_n);   // columns of this tile
+      // lanes of the store phase: 8 lanes on a row, 4 columns each; rows it * 4 + lane / 8
+      const int c4 = (lane & 7) * 4, sub = lane >> 3;
+      const int64_t slice = p.split > 1 ? (int64_t)(t % p.split) * p.M : 0;
+      const bool vec_c = aligned16(p.C, p.ldc * (p.c_f32 ? 4 : 2)), vec_r = aligned16(p.residual, p.ldr * 2);
+      int rows[8];
+#pragma unroll
+      for (int it = 0; it < 8; ++it) rows[it] = __shfl_sync(0xffffffffu, my_row, it * 4 + sub);
 #pragma unroll 1
-      for (int c0 = 0; c0 < kTile; c0 += 32) {
-        if (col0 + c0 >= p.N) break;  // uniform across the CTA
-        uint32_t r[32];
-        ptx::tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kTile + c0), r);
-        ptx::tmem_ld_wait();
-        if (!row_ok) continue;
+      for (int cc = 0; cc < 4; ++cc) {   // a warp's chunks come in pairs: 64 neighbouring columns are whole lines of a bf16 row too
+        const int c0 = half * 64 + (cc >> 1) * 128 + (cc & 1) * 32;
+        if (c0 >= n_tile) break;
         const int64_t col = col0 + c0;
-        const bool full = (col + 32 <= p.N);
-        float v[32];
+        const int n_ok = n_tile - c0 < 32 ? n_tile - c0 : 32;
+        const bool in4 = c4 + 4 <= n_ok;
+        uint2 res[8];    // asked for before the accumulator is read
+        if (p.residual && vec_r && in4) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
-        if (p.bias) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (full || col + j < p.N) v[j] += __bfloat162float(p.bias[col + j]);
+          for (int it = 0; it < 8; ++it)
+            if (rows[it] >= 0) res[it] = *reinterpret_cast<const uint2*>(p.residual + rows[it] * p.ldr + col + c4);
         }
-        if (p.residual) {
-          const __nv_bfloat16* rp = p.residual + row * p.ldr + col;
-          if (full && ((p.ldr & 7) == 0)) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              const uint4 u = *reinterpret_cast<const uint4*>(rp + j);
-              const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float2 f = __bfloat1622float2(h[e]);
-                v[j + 2 * e] += f.x;
-                v[j + 2 * e + 1] += f.y;
-              }
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (col + j < p.N) v[j] += __bfloat162float(rp[j]);
-          }
-        }
+        uint32_t r[32];
+        ptx::tmem_ld_32x32b_x32(acc_addr + (uint32_t)c0, r);
+        ptx::tmem_ld_wait();
         if (p.g_w) {
-          __nv_bfloat16* ap = p.act + row * p.ld_act + col;
+          uint32_t h[16];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float z = fmaxf(v[j], 0.f);
-            v[j] = (p.g_act == 2 ? 0.5f * v[j] * (1.f + erff(v[j] * 0.70710678118654752f)) : z * z) * row_w;
-          }
-          if (full && ((p.ld_act & 7) == 0)) {
+          for (int j = 0; j < 16; ++j) {
+            float v[2];
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              uint4 u;
-              __nv_bfloat162* hb = reinterpret_cast<__nv_bfloat162*>(&u);
-#pragma unroll
-              for (int e = 0; e < 4; ++e) hb[e] = __floats2bfloat162_rn(v[j + 2 * e], v[j + 2 * e + 1]);
-              *reinterpret_cast<uint4*>(ap + j) = u;
+            for (int e = 0; e < 2; ++e) {
+              const float a = __uint_as_float(r[2 * j + e]) * p.alpha, z = fmaxf(a, 0.f);
+              v[e] = (p.g_act == 2 ? 0.5f * a * (1.f + erff(a * 0.70710678118654752f)) : z * z) * row_w;
             }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (col + j < p.N) ap[j] = __float2bfloat16_rn(v[j]);
+            h[j] = pack2(v[0], v[1]);
           }
+          stage_bf16_row(st, lane, h);
+          __syncwarp();
+          store_bf16_chunk(st, lane, my_row, p.act + col, p.ld_act, n_ok, aligned16(p.act, p.ld_act * 2));
+          __syncwarp();
           continue;
         }
         if (p.dgu != nullptr) {
+          if (!row_ok) continue;
           // d act tile -> (d gate, d up): same rounding points as the two-kernel path (d act rounded to bf16, then
           // silu_mul_bwd_kernel's arithmetic, learner_ops.cu), so fused and unfused results are bit-identical
           const __nv_bfloat16* gp = p.bwd_gu + row * p.ld_gu + col;
@@ -468,8 +524,9 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const float2 g = __bfloat1622float2(hg[e]), u = __bfloat1622float2(hu[e]);
-              const float2 d = __bfloat1622float2(__floats2bfloat162_rn(v[j + 2 * e], v[j + 2 * e + 1]));
-              const float s0 = 1.f / (1.f + __expf(-g.x)), s1 = 1.f / (1.f + __expf(-g.y));
+              const float2 d = __bfloat1622float2(__floats2bfloat162_rn(__uint_as_float(r[j + 2 * e]) * p.alpha,
+                                                                       __uint_as_float(r[j + 2 * e + 1]) * p.alpha));
+              const float s0 = div_ge1(1.f, 1.f + __expf(-g.x)), s1 = div_ge1(1.f, 1.f + __expf(-g.y));
               const float l0 = g.x * s0, l1 = g.y * s1;
               du[e] = __floats2bfloat162_rn(d.x * l0, d.y * l1);
               dg[e] = __floats2bfloat162_rn(d.x * u.x * (s0 + l0 * (1.f - s0)), d.y * u.y * (s1 + l1 * (1.f - s1)));
@@ -479,45 +536,67 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
           }
           continue;
         }
-        if (p.c_f32) {
-          float* cp = reinterpret_cast<float*>(p.C) + (row + (p.split > 1 ? (int64_t)(t % p.split) * p.M : 0)) * p.ldc + col;
-          if (full && ((p.ldc & 3) == 0)) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              float4 o = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-              if (p.accumulate) {
-                const float4 old = *reinterpret_cast<const float4*>(cp + j);
-                o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-              }
-              *reinterpret_cast<float4*>(cp + j) = o;
-            }
-          } else {
+        for (int c = 0; c < 8; ++c) sts16(at128(st, lane, c), r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
+        __syncwarp();
+        float b4[4] = {0.f, 0.f, 0.f, 0.f};
+        if (p.bias) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (col + j < p.N) cp[j] = p.accumulate ? cp[j] + v[j] : v[j];
+          for (int e = 0; e < 4; ++e)
+            if (c4 + e < n_ok) b4[e] = __bfloat162float(p.bias[col + c4 + e]);
+        }
+#pragma unroll
+        for (int it = 0; it < 8; ++it) {
+          const uint4 u = lds16(at128(st, it * 4 + sub, lane & 7));
+          if (rows[it] < 0) continue;
+          float v[4] = {__uint_as_float(u.x) * p.alpha, __uint_as_float(u.y) * p.alpha, __uint_as_float(u.z) * p.alpha,
+                        __uint_as_float(u.w) * p.alpha};
+          if (p.bias) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] += b4[e];
           }
-        } else {
-          __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(p.C) + row * p.ldc + col;
-          if (full && ((p.ldc & 7) == 0)) {
+          if (p.residual) {
+            if (vec_r && in4) {
+              const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&res[it].x));
+              const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&res[it].y));
+              v[0] += f0.x; v[1] += f0.y; v[2] += f1.x; v[3] += f1.y;
+            } else {
+              const __nv_bfloat16* rp = p.residual + rows[it] * p.ldr + col + c4;
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              uint4 u;
-              __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
+              for (int e = 0; e < 4; ++e)
+                if (c4 + e < n_ok) v[e] += __bfloat162float(rp[e]);
+            }
+          }
+          if (p.c_f32) {
+            float* cp = reinterpret_cast<float*>(p.C) + (rows[it] + slice) * p.ldc + col + c4;
+            if (vec_c && in4) {
+              const float4 o = make_float4(v[0], v[1], v[2], v[3]);
+              // every element is added to exactly once per launch, so the sum has one order; adding in L2 spares the read's
+              // latency, which 32 KB of loads in flight per SM do not cover (3584 x 18944, K = 1000: loads 224 us, this 156)
+              if (p.accumulate) atomicAdd(reinterpret_cast<float4*>(cp), o);
+              else *reinterpret_cast<float4*>(cp) = o;
+            } else {
 #pragma unroll
-              for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(v[j + 2 * e], v[j + 2 * e + 1]);
-              *reinterpret_cast<uint4*>(cp + j) = u;
+              for (int e = 0; e < 4; ++e)
+                if (c4 + e < n_ok) cp[e] = p.accumulate ? cp[e] + v[e] : v[e];
             }
           } else {
+            __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(p.C) + rows[it] * p.ldc + col + c4;
+            if (vec_c && in4) {
+              *reinterpret_cast<uint2*>(cp) = make_uint2(pack2(v[0], v[1]), pack2(v[2], v[3]));
+            } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (col + j < p.N) cp[j] = __float2bfloat16(v[j]);
+              for (int e = 0; e < 4; ++e)
+                if (c4 + e < n_ok) cp[e] = __float2bfloat16(v[e]);
+            }
           }
         }
+        __syncwarp();
       }
       }  // !kHead
       // this CTA's four epilogue warps are done with the accumulator -> tell the leader's MMA warp
       ptx::tc_fence_before_sync();
-      asm volatile("bar.sync 1, 128;" ::: "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps<kHead>) : "memory");
       if (threadIdx.x == 64) {
         if (rank == 0) ptx::mbar_arrive(acc_empty_bar(acc));
         else ptx::mbar_arrive_remote(acc_empty_bar(acc), 0);
@@ -615,6 +694,24 @@ __global__ void __launch_bounds__(256) transpose_bf16_kernel(const __nv_bfloat16
 
 using namespace prl;
 
+// Width of the output tiles.  74 CTA pairs walk the tiles in waves, so 256 columns leave most of a wave idle where the tiles just
+// miss a multiple of 74 (4096 x 3584: 224 tiles, 3.03 waves), and all but a few pairs idle where there are few.  A k-block costs
+// about as much as 520 + n columns, whatever bounds it (the products alone would be 2 n: the operands' way through L2 has the
+// larger part), fitted to 4096 / 1024 / 452 x 3584, K = 18944: 256 columns 438 / 115 / 107 us, 224 399 / 106 / 98, 208 387 / 104 /
+// 96, 128 642 / 164 / 90.  An MN-major B arrives in 64-column boxes and its column steps keep to whole 32-byte sectors (n a
+// multiple of 32: 4096 x 3584, K = 37888, took 1105 us with 208 columns, whose second half starts at byte 208, 820 with 224).
+static int pick_tile_n(int64_t M, int64_t N, int b_mn) {
+  const int64_t clusters = num_sms() / 2, m_tiles = (M + kTile - 1) / kTile;
+  int best = kTile;
+  int64_t best_cost = 0;
+  for (int n = kTile; n >= 64; n -= b_mn ? 32 : 16) {
+    const int64_t tiles = m_tiles * ((N + n - 1) / n), waves = (tiles + clusters - 1) / clusters;
+    const int64_t cost = waves * (520 + n);
+    if (n == kTile || cost < best_cost) { best = n; best_cost = cost; }
+  }
+  return best;
+}
+
 extern "C" int prl_gemm_tn(const void* A, int64_t lda, const void* B, int64_t ldb, int64_t M, int64_t N, int64_t K,
                            void* C, int64_t ldc, int32_t c_is_f32, int32_t accumulate, const void* bias,
                            const void* residual, int64_t ldr, float alpha, prl_stream_t stream_) {
@@ -635,11 +732,13 @@ extern "C" int prl_gemm_ex(const void* A, int64_t lda, int32_t a_mn_major, const
   PRL_CHECK_ARG(!accumulate || c_is_f32, "prl_gemm_tn: accumulate needs an fp32 output");
   PRL_CHECK_ARG(!residual || ldr >= N, "prl_gemm_tn: ldr %lld < N %lld", (long long)ldr, (long long)N);
   TnParams p = {};
+  p.tile_n = kTile;
   p.M = M; p.N = N; p.K = K;
   p.kblocks = (int)((K + kBK - 1) / kBK);
   p.k_wrap = p.kblocks;
+  p.tile_n = pick_tile_n(M, N, b_mn_major);
   p.m_tiles = (int)((M + kTile - 1) / kTile);
-  p.n_tiles = (int)((N + kTile - 1) / kTile);
+  p.n_tiles = (int)((N + p.tile_n - 1) / p.tile_n);
   p.C = C; p.ldc = ldc; p.c_f32 = c_is_f32; p.accumulate = accumulate;
   p.bias = (const __nv_bfloat16*)bias;
   p.residual = (const __nv_bfloat16*)residual;
@@ -652,15 +751,15 @@ extern "C" int prl_gemm_ex(const void* A, int64_t lda, int32_t a_mn_major, const
                       : make_tmap_2d_bf16(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2, kBK, kHalf);
   if (rc) return rc;
   rc = b_mn_major ? make_tmap_2d_bf16(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb * 2, 64, kBK)
-                  : make_tmap_2d_bf16(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb * 2, kBK, kHalf);
+                  : make_tmap_2d_bf16(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb * 2, kBK, (uint32_t)(p.tile_n / 2));
   if (rc) return rc;
-  const int smem = kStages * kStageBytes + 1024 + 8 * (2 * kStages + 4) + 16;
+  const int smem = kSmemTN;
   static SmemAttr smem_attr = {};
   PRL_CUDA(ensure_smem(gemm_tn_kernel<false>, smem, smem_attr));
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   int clusters = num_sms() / 2;
   if (tiles < clusters) clusters = (int)tiles;
-  gemm_tn_kernel<false><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta, tb, p);
+  gemm_tn_kernel<false><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta, tb, p);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -685,6 +784,7 @@ extern "C" int prl_gemm_tn_dual(const void* A1, const void* B1, int64_t K1, cons
                 "prl_gemm_tn_dual: need M, N >= 1 and K1, K2 multiples of 8 (M=%lld N=%lld K1=%lld K2=%lld)", (long long)M, (long long)N,
                 (long long)K1, (long long)K2);
   TnParams p = {};
+  p.tile_n = kTile;
   p.M = M; p.N = N; p.K = K1 + K2;
   p.k_wrap = (int)((K1 + kBK - 1) / kBK);
   p.kblocks = p.k_wrap + (int)((K2 + kBK - 1) / kBK);
@@ -700,13 +800,13 @@ extern "C" int prl_gemm_tn_dual(const void* A1, const void* B1, int64_t K1, cons
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tb2, B2, (uint64_t)K2, (uint64_t)N, (uint64_t)K2 * 2, kBK, kHalf);
   if (rc) return rc;
-  const int smem = kStages * kStageBytes + 1024 + 8 * (2 * kStages + 4) + 16;
+  const int smem = kSmemTN;
   static SmemAttr smem_attr = {};
   PRL_CUDA(ensure_smem(gemm_tn_kernel<false>, smem, smem_attr));
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles * split_k;
   int clusters = num_sms() / 2;
   if (tiles < clusters) clusters = (int)tiles;
-  gemm_tn_kernel<false><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta2, tb2, p);
+  gemm_tn_kernel<false><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta2, tb2, p);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -723,6 +823,7 @@ extern "C" int prl_moe_gemm_tc(const void* A, int64_t rows_cap, const void* W, i
   PRL_CHECK_ARG(rows_cap >= 1 && experts >= 1 && N >= 1 && K >= 8 && K % 8 == 0 && ldc >= N && experts * N < (1ll << 31),
                 "prl_moe_gemm_tc: bad shape (rows=%lld experts=%d N=%lld K=%lld)", (long long)rows_cap, experts, (long long)N, (long long)K);
   TnParams p = {};
+  p.tile_n = kTile;
   p.M = rows_cap; p.N = N; p.K = K;
   p.kblocks = p.k_wrap = (int)((K + kBK - 1) / kBK);
   p.m_tiles = 1;
@@ -736,13 +837,13 @@ extern "C" int prl_moe_gemm_tc(const void* A, int64_t rows_cap, const void* W, i
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tb, W, (uint64_t)K, (uint64_t)(experts * N), (uint64_t)K * 2, kBK, kHalf);
   if (rc) return rc;
-  const int smem = kStages * kStageBytes + 1024 + 8 * (2 * kStages + 4) + 16;
+  const int smem = kSmemTN;
   static SmemAttr smem_attr = {};
   PRL_CUDA(ensure_smem(gemm_tn_kernel<false>, smem, smem_attr));
   const int64_t items = ((rows_cap + kTile - 1) / kTile + experts) * p.n_tiles;
   int clusters = num_sms() / 2;
   if (items < clusters) clusters = (int)items;
-  gemm_tn_kernel<false><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta, tb, p);
+  gemm_tn_kernel<false><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta, tb, p);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -757,6 +858,7 @@ extern "C" int prl_gemm_dgrad_swiglu(const void* dY, int64_t ldy, const void* W_
                 ld_gu >= 2 * I && ld_gu % 8 == 0, "prl_gemm_dgrad_swiglu: bad shape (M=%lld I=%lld H=%lld)", (long long)M,
                 (long long)I, (long long)H);
   TnParams p = {};
+  p.tile_n = kTile;
   p.M = M; p.N = I; p.K = H;
   p.kblocks = (int)((H + kBK - 1) / kBK);
   p.k_wrap = p.kblocks;
@@ -770,13 +872,13 @@ extern "C" int prl_gemm_dgrad_swiglu(const void* dY, int64_t ldy, const void* W_
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tb, W_down, (uint64_t)I, (uint64_t)H, (uint64_t)ldw * 2, 64, kBK);
   if (rc) return rc;
-  const int smem = kStages * kStageBytes + 1024 + 8 * (2 * kStages + 4) + 16;
+  const int smem = kSmemTN;
   static SmemAttr smem_attr = {};
   PRL_CUDA(ensure_smem(gemm_tn_kernel<false>, smem, smem_attr));
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   int clusters = num_sms() / 2;
   if (tiles < clusters) clusters = (int)tiles;
-  gemm_tn_kernel<false><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta, tb, p);
+  gemm_tn_kernel<false><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta, tb, p);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -824,6 +926,7 @@ static int gemm_swiglu_impl(const void* X, int64_t ldx, const void* W, int64_t l
                     (!gate_up || (ld_gu >= 2 * I && ld_gu % 8 == 0)),
                 "prl_gemm_swiglu: row strides must cover a row and be multiples of 8 elements");
   TnParams p = {};
+  p.tile_n = kTile;
   p.M = M; p.N = 2 * I; p.K = K;
   p.kblocks = (int)((K + kBK - 1) / kBK);
   p.k_wrap = p.kblocks;
@@ -837,13 +940,13 @@ static int gemm_swiglu_impl(const void* X, int64_t ldx, const void* W, int64_t l
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tb, W, (uint64_t)K, (uint64_t)(2 * I), (uint64_t)ldw * 2, kBK, kHalf);
   if (rc) return rc;
-  const int smem = kStages * kStageBytes + 1024 + 8 * (2 * kStages + 4) + 16;
+  const int smem = kSmemTN;
   static SmemAttr smem_attr = {};
   PRL_CUDA(ensure_smem(gemm_tn_kernel<false>, smem, smem_attr));
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   int clusters = num_sms() / 2;
   if (tiles < clusters) clusters = (int)tiles;
-  gemm_tn_kernel<false><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta, tb, p);
+  gemm_tn_kernel<false><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta, tb, p);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -855,6 +958,7 @@ int head_logprob_tn(const void* W, const void* W_lo, const void* X, int64_t M, i
                     const int64_t* targets, float* logprob_target, float* entropy, float* lse, void* workspace,
                     cudaStream_t stream) {
   TnParams p = {};
+  p.tile_n = kTile;
   p.M = M; p.N = V; p.K = K;
   p.kblocks = (int)((K + kBK - 1) / kBK);
   p.k_wrap = p.kblocks;
@@ -871,13 +975,13 @@ int head_logprob_tn(const void* W, const void* W_lo, const void* X, int64_t M, i
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tb2, W_lo ? W_lo : W, (uint64_t)K, (uint64_t)V, (uint64_t)K * 2, kBK, kHalf);
   if (rc) return rc;
-  const int smem = kStages * kStageBytes + 1024 + 8 * (2 * kStages + 4) + 16;
+  const int smem = kSmemTN;
   static SmemAttr smem_attr = {};
   PRL_CUDA(ensure_smem(gemm_tn_kernel<true>, smem, smem_attr));
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   int clusters = num_sms() / 2;
   if (tiles < clusters) clusters = (int)tiles;
-  gemm_tn_kernel<true><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN), (size_t)smem, stream>>>(ta, tb, ta, tb2, p);
+  gemm_tn_kernel<true><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<true>), (size_t)smem, stream>>>(ta, tb, ta, tb2, p);
   PRL_LAUNCH_CHECK();
   head_tn_combine_kernel<<<(unsigned)((M + 3) / 4), 128, 0, stream>>>((const float4*)workspace, p.n_tiles, M,
                                                                       targets ? 1 : 0, logprob_target, entropy, lse);
@@ -902,6 +1006,7 @@ extern "C" int prl_head_dlogits(const void* W, const void* W_lo, const void* X, 
                 (long long)ld_dz);
   PRL_CHECK_ARG(!g_entropy || entropy, "prl_head_dlogits: g_entropy needs the forward entropy");
   TnParams p = {};
+  p.tile_n = kTile;
   p.M = M; p.N = V; p.K = K;
   p.kblocks = (int)((K + kBK - 1) / kBK);
   p.k_wrap = p.kblocks;
@@ -919,13 +1024,13 @@ extern "C" int prl_head_dlogits(const void* W, const void* W_lo, const void* X, 
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tb2, W_lo ? W_lo : W, (uint64_t)K, (uint64_t)V, (uint64_t)K * 2, kBK, kHalf);
   if (rc) return rc;
-  const int smem = kStages * kStageBytes + 1024 + 8 * (2 * kStages + 4) + 16;
+  const int smem = kSmemTN;
   static SmemAttr smem_attr = {};
   PRL_CUDA(ensure_smem(gemm_tn_kernel<true>, smem, smem_attr));
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   int clusters = num_sms() / 2;
   if (tiles < clusters) clusters = (int)tiles;
-  gemm_tn_kernel<true><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta, tb2, p);
+  gemm_tn_kernel<true><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<true>), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta, tb2, p);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }

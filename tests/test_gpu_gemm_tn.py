@@ -232,3 +232,74 @@ def test_dgrad_with_silu_backward_epilogue_is_bit_identical(cuda_device, T, H, I
     got = o.dgrad_swiglu(dY, W, gu)
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+# one shape per tile width that the width rule takes on 148 SMs (noted), columns that end inside a 32-column chunk and a 4-column
+# piece, rows that end inside a tile; the strides of C make its rows 16-byte aligned or not
+@pytest.mark.parametrize("M,N,K,b_mn,pad", [
+    (4096, 3581, 192, False, 3),    # 208
+    (1000, 3578, 72, False, 2),     # 208
+    (3070, 2045, 136, False, 0),    # 176, rows of C not 16-byte aligned
+    (4000, 2048, 64, False, 8),     # 240
+    (1024, 8226, 64, False, 6),     # 224
+    (452, 3584, 128, False, 0),     # 112
+    (200, 2041, 72, False, 7),      # 64
+    (1, 24, 8, False, 0),           # 64
+    (2048, 3576, 136, True, 0),     # 224, MN-major B
+    (1000, 2040, 64, True, 4),      # 128
+    (130, 1016, 72, True, 1),       # 64
+    (3072, 2048, 64, True, 0),      # 192
+])
+def test_gemm_output_widths_and_epilogues(cuda_device, M, N, K, b_mn, pad):
+    """plain fp32, fp32 accumulate, bf16 + bias + residual over the widths of the output tiles.  fp32: products of bf16 sum to
+    within K * 2^-24 of the sum of their magnitudes; bf16: one more rounding of the result."""
+    from pipelinerl_b200 import _lib
+    lib = _lib.load()
+    g = torch.Generator().manual_seed(M + N + K)
+    A = torch.randn(M, K, generator=g).to(torch.bfloat16).to(cuda_device)
+    B = torch.randn(N, K, generator=g).to(torch.bfloat16).to(cuda_device)
+    Bs = B.T.contiguous() if b_mn else B
+    want = A.double() @ B.double().T
+    slack = K * 2.0 ** -24 * (A.double().abs() @ B.double().abs().T) + 1e-12
+    old = torch.randn(M, N, generator=g).to(cuda_device)
+    bias = torch.randn(N, generator=g).to(torch.bfloat16).to(cuda_device)
+    res = torch.randn(M, N + pad, generator=g).to(torch.bfloat16).to(cuda_device)[:, :N]
+
+    def run(C, acc=0, bias=None, res=None, alpha=1.0):
+        _lib.check(lib.prl_gemm_ex(A.data_ptr(), K, 0, Bs.data_ptr(), Bs.stride(0), int(b_mn), M, N, K, C.data_ptr(), C.stride(0),
+                                   int(C.dtype == torch.float32), acc, bias.data_ptr() if bias is not None else None,
+                                   res.data_ptr() if res is not None else None, res.stride(0) if res is not None else 0, alpha,
+                                   _lib.stream_ptr()))
+        return C
+    wide = torch.full((M, N + pad), 7.0, device=cuda_device)
+    got = run(wide[:, :N])
+    assert ((got.double() - want).abs() <= slack).all()
+    assert (wide[:, N:] == 7.0).all(), "columns beyond the output were written"
+    wide[:, :N] = old
+    got = run(wide[:, :N], acc=1, alpha=0.5)
+    total = old.double() + 0.5 * want
+    assert ((got.double() - total).abs() <= slack + 2.0 ** -23 * (old.abs().double() + total.abs())).all()
+    assert (wide[:, N:] == 7.0).all()
+    half = torch.full((M, N + pad), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    got = run(half[:, :N], bias=bias, res=res)
+    total = want + bias.double() + res.double()
+    assert ((got.double() - total).abs() <= 2 * slack + 2.0 ** -8 * total.abs() + 1e-6).all()
+    assert (half[:, N:] == 7.0).all()
+
+
+def test_gate_quotient_over_its_range(cuda_device):
+    """SiLU in the GEMM's epilogue against the device's own division: gates from far below to far above zero, the overflow of
+    exp among them.  One feature per gate value, up = 1; both sides round to bf16, a tie may fall either way (one bf16 ulp)."""
+    from pipelinerl_b200.learner_body import Ops
+    n, K = 512, 512
+    gate = torch.cat([torch.linspace(-130, 130, n - 8), torch.tensor([-1e30, -88.7, -87.4, -1e-30, 0.0, 1e-30, 88.7, 1e30])])
+    gate = gate.to(torch.bfloat16).to(cuda_device)
+    W = torch.zeros(2 * n, K, dtype=torch.bfloat16, device=cuda_device)
+    W[torch.arange(n), torch.arange(n)] = gate
+    W[n:, :] = torch.eye(n, dtype=torch.bfloat16, device=cuda_device)
+    X = torch.eye(K, dtype=torch.bfloat16, device=cuda_device)       # row i: gate i and up = 1 at feature i
+    _, act = Ops().gemm_swiglu(X, W, need_gate_up=False)
+    got, g = act.diagonal().float(), gate.float()
+    want = (g / (1 + torch.exp(-g))).to(torch.bfloat16).float()
+    assert torch.isfinite(got).all()
+    assert ((got - want).abs() <= 2.0 ** -7 * want.abs() + 1e-36).all(), (got - want).abs().max()
