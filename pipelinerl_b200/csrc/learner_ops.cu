@@ -11,7 +11,7 @@ namespace {
 
 constexpr int kRowThreads = 256;
 constexpr int kMaxVec = 4;          // 8-element vectors per thread -> rows of up to 8192 elements
-constexpr int kPartialBlocks = 592; // 4 per SM: grid of the persistent row kernels = rows of the partial workspace
+constexpr int kPartialBlocks = 148 * 8; // most blocks of a persistent row kernel = rows of the partial workspace
 
 struct Vec8 { float v[8]; };
 
@@ -35,16 +35,39 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const Vec8& r) {
   *reinterpret_cast<uint4*>(p) = u;
 }
 
+__device__ __forceinline__ Vec8 unpack8(const uint4& u) {
+  Vec8 r;
+  const uint32_t h[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    r.v[2 * e] = __uint_as_float(h[e] << 16);
+    r.v[2 * e + 1] = __uint_as_float(h[e] & 0xFFFF0000u);
+  }
+  return r;
+}
+// sum over the block; the caller alternates between two s_red buffers, so one barrier serves
 __device__ __forceinline__ float block_sum(float v, float* s_red) {
   v = warp_sum(v);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();  // s_red may still be read from the previous call
-  if (lane == 0) s_red[warp] = v;
+  if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
   __syncthreads();
   float t = 0.f;
 #pragma unroll
-  for (int w = 0; w < kRowThreads / 32; ++w) t += s_red[w];
+  for (int w = 0; w < kRowThreads / 32; ++w) t += w < (int)(blockDim.x >> 5) ? s_red[w] : 0.f;
   return t;
+}
+
+// The row kernels are bound by HBM.  A block walks its rows with the next row already asked for (registers, raw bf16) while the
+// current one goes through its block sum: without that the reads stop at every row's barrier (16384 x 3584: backward 170 us,
+// 0.42 of the copy rate).  The block has just the threads that a row fills (448 pieces of 16 bytes: 224 threads, two each), and
+// the grid just the blocks that are resident at once.  With the faster column sums below: 16384 x 3584 forward 49 -> 47 us, backward
+// 214 -> 87 us (5.4 TB/s, cold L2); 4096 x 5120 27 -> 21, 150 -> 44; 16384 x 1024 25 -> 21, 79 -> 38.
+template <int kVec>
+__device__ __forceinline__ void load_row(const __nv_bfloat16* __restrict__ p, int64_t row, int H, uint4 (&r)[kVec]) {
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) {
+    const int v = threadIdx.x + i * blockDim.x;
+    if (v < (H >> 3)) r[i] = ld_stream_u4(reinterpret_cast<const uint4*>(p + row * H) + v);
+  }
 }
 
 // y = bf16(x * rstd) * gamma  (the rounding order of HF's Qwen2RMSNorm); rstd kept for the backward
@@ -53,30 +76,36 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_fwd_kernel(const __nv_bfl
                                                                   const __nv_bfloat16* __restrict__ gamma, int64_t T,
                                                                   int H, float eps, __nv_bfloat16* __restrict__ y,
                                                                   float* __restrict__ rstd) {
-  __shared__ float s_red[kRowThreads / 32];
+  __shared__ float s_red[2][kRowThreads / 32];
   const int nvec = H >> 3;
-  for (int64_t row = blockIdx.x; row < T; row += gridDim.x) {
-    Vec8 xv[kVec];
+  uint4 g[kVec], next[kVec];
+  load_row<kVec>(gamma, 0, H, g);
+  load_row<kVec>(x, blockIdx.x, H, next);
+  int buf = 0;
+  for (int64_t row = blockIdx.x; row < T; row += gridDim.x, buf ^= 1) {
+    uint4 xr[kVec];
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) xr[i] = next[i];
+    if (row + gridDim.x < T) load_row<kVec>(x, row + gridDim.x, H, next);
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < kVec; ++i) {
-      const int v = threadIdx.x + i * kRowThreads;
-      if (v < nvec) {
-        xv[i] = load8(x + row * H + v * 8);
+      if (threadIdx.x + i * blockDim.x < nvec) {
+        const Vec8 xv = unpack8(xr[i]);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) ss += xv[i].v[e] * xv[i].v[e];
+        for (int e = 0; e < 8; ++e) ss += xv.v[e] * xv.v[e];
       }
     }
-    const float r = rsqrtf(block_sum(ss, s_red) / (float)H + eps);
+    const float r = rsqrtf(block_sum(ss, s_red[buf]) / (float)H + eps);
     if (threadIdx.x == 0) rstd[row] = r;
 #pragma unroll
     for (int i = 0; i < kVec; ++i) {
-      const int v = threadIdx.x + i * kRowThreads;
+      const int v = threadIdx.x + i * blockDim.x;
       if (v < nvec) {
-        const Vec8 g = load8(gamma + v * 8);
+        const Vec8 xv = unpack8(xr[i]), gv = unpack8(g[i]);
         Vec8 o;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o.v[e] = __bfloat162float(__float2bfloat16(xv[i].v[e] * r)) * g.v[e];
+        for (int e = 0; e < 8; ++e) o.v[e] = __bfloat162float(__float2bfloat16(xv.v[e] * r)) * gv.v[e];
         store8(y + row * H + v * 8, o);
       }
     }
@@ -85,54 +114,63 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_fwd_kernel(const __nv_bfl
 
 // dx = dres + rstd * (dy*gamma - xhat * mean(dy*gamma*xhat));  partial[block][c] = sum over this block's rows of dy*xhat
 template <int kVec>
-__global__ void __launch_bounds__(kRowThreads, kVec <= 2 ? 3 : 1) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x,
-                                                                  const __nv_bfloat16* __restrict__ gamma,
-                                                                  const float* __restrict__ rstd,
-                                                                  const __nv_bfloat16* __restrict__ dy,
-                                                                  const __nv_bfloat16* __restrict__ dres, int64_t T, int H,
-                                                                  __nv_bfloat16* __restrict__ dx,
-                                                                  float* __restrict__ partial) {
-  __shared__ float s_red[kRowThreads / 32];
+__global__ void __launch_bounds__(kRowThreads, kVec == 1 ? 4 : (kVec == 2 ? 2 : 1))
+rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ rstd,
+                   const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ dres, int64_t T, int H,
+                   __nv_bfloat16* __restrict__ dx, float* __restrict__ partial) {
+  __shared__ float s_red[2][kRowThreads / 32];
   const int nvec = H >> 3;
-  Vec8 gv[kVec], acc[kVec];
+  uint4 g[kVec], xn[kVec], dn[kVec], sn[kVec];
+  Vec8 acc[kVec];
 #pragma unroll
   for (int i = 0; i < kVec; ++i) {
-    const int v = threadIdx.x + i * kRowThreads;
+    sn[i] = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[i].v[e] = 0.f;
-    if (v < nvec) gv[i] = load8(gamma + v * 8);
   }
-  for (int64_t row = blockIdx.x; row < T; row += gridDim.x) {
-    const float r = rstd[row];
-    Vec8 xh[kVec], dxh[kVec];
+  load_row<kVec>(gamma, 0, H, g);
+  load_row<kVec>(x, blockIdx.x, H, xn);
+  load_row<kVec>(dy, blockIdx.x, H, dn);
+  if (dres) load_row<kVec>(dres, blockIdx.x, H, sn);
+  float rn = rstd[blockIdx.x];
+  int buf = 0;
+  for (int64_t row = blockIdx.x; row < T; row += gridDim.x, buf ^= 1) {
+    uint4 xr[kVec], dr[kVec], sr[kVec];
+    const float r = rn;
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) { xr[i] = xn[i]; dr[i] = dn[i]; sr[i] = sn[i]; }
+    const int64_t nx = row + gridDim.x;
+    if (nx < T) {
+      load_row<kVec>(x, nx, H, xn);
+      load_row<kVec>(dy, nx, H, dn);
+      if (dres) load_row<kVec>(dres, nx, H, sn);
+      rn = rstd[nx];
+    }
     float dot = 0.f;
 #pragma unroll
     for (int i = 0; i < kVec; ++i) {
-      const int v = threadIdx.x + i * kRowThreads;
-      if (v < nvec) {
-        xh[i] = load8(x + row * H + v * 8);
-        const Vec8 d = load8(dy + row * H + v * 8);
+      if (threadIdx.x + i * blockDim.x < nvec) {
+        const Vec8 xv = unpack8(xr[i]), dv = unpack8(dr[i]), gv = unpack8(g[i]);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          xh[i].v[e] *= r;
-          acc[i].v[e] += d.v[e] * xh[i].v[e];
-          dxh[i].v[e] = d.v[e] * gv[i].v[e];
-          dot += dxh[i].v[e] * xh[i].v[e];
+          const float xh = xv.v[e] * r;
+          acc[i].v[e] += dv.v[e] * xh;
+          dot += dv.v[e] * gv.v[e] * xh;
         }
       }
     }
-    const float m = block_sum(dot, s_red) / (float)H;
+    const float m = block_sum(dot, s_red[buf]) / (float)H;
 #pragma unroll
     for (int i = 0; i < kVec; ++i) {
-      const int v = threadIdx.x + i * kRowThreads;
+      const int v = threadIdx.x + i * blockDim.x;
       if (v < nvec) {
+        const Vec8 xv = unpack8(xr[i]), dv = unpack8(dr[i]), gv = unpack8(g[i]), sv = unpack8(sr[i]);
         Vec8 o;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o.v[e] = r * (dxh[i].v[e] - xh[i].v[e] * m);
+        for (int e = 0; e < 8; ++e) o.v[e] = r * (dv.v[e] * gv.v[e] - xv.v[e] * r * m);
         if (dres) {
-          const Vec8 dr = load8(dres + row * H + v * 8);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) o.v[e] += dr.v[e];
+          for (int e = 0; e < 8; ++e) o.v[e] += sv.v[e];
         }
         store8(dx + row * H + v * 8, o);
       }
@@ -140,7 +178,7 @@ __global__ void __launch_bounds__(kRowThreads, kVec <= 2 ? 3 : 1) rmsnorm_bwd_ke
   }
 #pragma unroll
   for (int i = 0; i < kVec; ++i) {
-    const int v = threadIdx.x + i * kRowThreads;
+    const int v = threadIdx.x + i * blockDim.x;
     if (v < nvec) {
       float* pp = partial + (int64_t)blockIdx.x * H + v * 8;
       *reinterpret_cast<float4*>(pp) = make_float4(acc[i].v[0], acc[i].v[1], acc[i].v[2], acc[i].v[3]);
@@ -180,14 +218,31 @@ __global__ void __launch_bounds__(kRowThreads) colsum_kernel(const __nv_bfloat16
   }
 }
 
-// out[c] += sum_b partial[b][c], b ascending
-__global__ void __launch_bounds__(256) partial_reduce_kernel(const float* __restrict__ partial, int n_blocks, int Cc,
-                                                             float* __restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= Cc) return;
-  float s = 0.f;
-  for (int b = 0; b < n_blocks; ++b) s += partial[(int64_t)b * Cc + c];
-  out[c] += s;
+// out[c] += sum_b partial[b][c]: warp w of a block adds rows w, w + 16, ... of the block's 32 columns, then the warps' sums are
+// added in order (one fixed order).  One thread per column walking all the rows took 36 us for 592 x 3584.
+constexpr int kReduceWarps = 16;
+__global__ void __launch_bounds__(32 * kReduceWarps) partial_reduce_kernel(const float* __restrict__ partial, int n_blocks, int Cc,
+                                                                          float* __restrict__ out) {
+  __shared__ float s_sum[kReduceWarps][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane;
+  pdl_wait();
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+  if (c < Cc) {
+    int b = warp;
+    for (; b + 3 * kReduceWarps < n_blocks; b += 4 * kReduceWarps) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) s[k] += partial[(int64_t)(b + k * kReduceWarps) * Cc + c];
+    }
+    for (; b < n_blocks; b += kReduceWarps) s[0] += partial[(int64_t)b * Cc + c];
+  }
+  s_sum[warp][lane] = (s[0] + s[1]) + (s[2] + s[3]);
+  __syncthreads();
+  if (warp == 0 && c < Cc) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < kReduceWarps; ++w) t += s_sum[w][lane];
+    out[c] += t;
+  }
 }
 
 // in-place rotation of the first n_heads heads of each row: (x1, x2) -> (x1 cos - s x2 sin, x2 cos + s x1 sin)
@@ -222,34 +277,33 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, int64_t ld, int64_t T
   }
 }
 
-__global__ void __launch_bounds__(256) silu_mul_fwd_kernel(const __nv_bfloat16* __restrict__ gu, int64_t T, int I,
+__global__ void __launch_bounds__(256) silu_mul_fwd_kernel(const __nv_bfloat16* __restrict__ gu, int I,
                                                            __nv_bfloat16* __restrict__ act) {
-  const int64_t nvec = T * (I >> 3);
-  const int per_row = I >> 3;
-  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < nvec; v += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = v / per_row;
-    const int c = (int)(v % per_row) * 8;
-    const Vec8 g = load8(gu + row * 2 * I + c), u = load8(gu + row * 2 * I + I + c);
+  const int64_t row = blockIdx.x;                // blocks of one row: no division per element
+  const __nv_bfloat16* gp = gu + row * 2 * I;
+  for (int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8; c < I; c += gridDim.y * blockDim.x * 8) {
+    const Vec8 g = unpack8(ld_stream_u4(reinterpret_cast<const uint4*>(gp + c)));
+    const Vec8 u = unpack8(ld_stream_u4(reinterpret_cast<const uint4*>(gp + I + c)));
     Vec8 o;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) o.v[e] = g.v[e] / (1.f + __expf(-g.v[e])) * u.v[e];
+    for (int e = 0; e < 8; ++e) o.v[e] = div_ge1(g.v[e], 1.f + __expf(-g.v[e])) * u.v[e];
     store8(act + row * I + c, o);
   }
 }
 
 __global__ void __launch_bounds__(256) silu_mul_bwd_kernel(const __nv_bfloat16* __restrict__ gu,
-                                                           const __nv_bfloat16* __restrict__ dact, int64_t T, int I,
+                                                           const __nv_bfloat16* __restrict__ dact, int I,
                                                            __nv_bfloat16* __restrict__ dgu) {
-  const int64_t nvec = T * (I >> 3);
-  const int per_row = I >> 3;
-  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < nvec; v += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = v / per_row;
-    const int c = (int)(v % per_row) * 8;
-    const Vec8 g = load8(gu + row * 2 * I + c), u = load8(gu + row * 2 * I + I + c), d = load8(dact + row * I + c);
+  const int64_t row = blockIdx.x;
+  const __nv_bfloat16* gp = gu + row * 2 * I;
+  for (int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8; c < I; c += gridDim.y * blockDim.x * 8) {
+    const Vec8 g = unpack8(ld_stream_u4(reinterpret_cast<const uint4*>(gp + c)));
+    const Vec8 u = unpack8(ld_stream_u4(reinterpret_cast<const uint4*>(gp + I + c)));
+    const Vec8 d = unpack8(ld_stream_u4(reinterpret_cast<const uint4*>(dact + row * I + c)));
     Vec8 dg, du;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const float s = 1.f / (1.f + __expf(-g.v[e]));
+      const float s = div_ge1(1.f, 1.f + __expf(-g.v[e]));
       const float silu = g.v[e] * s;
       du.v[e] = d.v[e] * silu;
       dg.v[e] = d.v[e] * u.v[e] * (s + silu * (1.f - s));
@@ -277,13 +331,33 @@ __global__ void __launch_bounds__(256) embed_scatter_kernel(float* __restrict__ 
     const int64_t id = ids[row];
     for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
       const Vec8 d = load8(dh + row * H + v * 8);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) atomicAdd(dtable + id * H + v * 8 + e, d.v[e]);
+      atomicAdd(reinterpret_cast<float4*>(dtable + id * H + v * 8), make_float4(d.v[0], d.v[1], d.v[2], d.v[3]));
+      atomicAdd(reinterpret_cast<float4*>(dtable + id * H + v * 8 + 4), make_float4(d.v[4], d.v[5], d.v[6], d.v[7]));
     }
   }
 }
 
-int row_grid(int64_t T) { return (int)(T < kPartialBlocks ? T : kPartialBlocks); }
+int silu_threads(int64_t I) {
+  const int64_t n = (I + 7) / 8;
+  return n >= 256 ? 256 : (int)((n + 31) / 32 * 32);
+}
+dim3 silu_grid(int64_t T, int64_t I) {   // a block per row; few rows are cut, so that eight blocks per SM are there
+  const int64_t pieces = (I / 8 + silu_threads(I) - 1) / silu_threads(I), want = ((int64_t)num_sms() * 8 + T - 1) / T;
+  return dim3((unsigned)T, (unsigned)(want < pieces ? want : pieces));
+}
+int row_grid(int64_t T) { return (int)(T < kPartialBlocks / 2 ? T : kPartialBlocks / 2); }
+int row_vecs(int64_t H) { return (int)((H / 8 + kRowThreads - 1) / kRowThreads); }                       // 16-byte pieces per thread
+int row_threads(int64_t H) { return (int)(((H / 8 + row_vecs(H) - 1) / row_vecs(H) + 31) / 32 * 32); }   // as many as the pieces need
+// resident blocks of the backward: two of 256 threads with 128 registers each per SM, or the threads' worth of narrow rows
+int row_bwd_grid(int64_t T, int64_t H) {
+  const int per_sm = row_vecs(H) == 1 ? 1024 / row_threads(H) : (row_vecs(H) == 2 ? 2 : 1);
+  const int64_t n = (int64_t)num_sms() * (per_sm < 8 ? per_sm : 8);
+  const int64_t most = n < kPartialBlocks ? n : kPartialBlocks;
+  return (int)(T < most ? T : most);
+}
+cudaError_t launch_partial_reduce(const float* ws, int blocks, int64_t cols, float* out, cudaStream_t stream) {
+  return launch_pdl(partial_reduce_kernel, dim3((unsigned)((cols + 31) / 32)), dim3(32 * kReduceWarps), 0, stream, ws, blocks, (int)cols, out);
+}
 
 }  // namespace
 }  // namespace prl
@@ -300,10 +374,12 @@ extern "C" int prl_rmsnorm_fwd(const void* x, const void* gamma, int64_t T, int6
                                prl_stream_t stream) {
   PRL_CHECK_ARG(x && gamma && y && rstd && T >= 1, "prl_rmsnorm_fwd: bad argument");
   PRL_ROW_ARGS("prl_rmsnorm_fwd", H);
-  const unsigned grid = (unsigned)(T < 4 * kPartialBlocks ? T : 4 * kPartialBlocks);
-#define PRL_FWD(V) rmsnorm_fwd_kernel<V><<<grid, kRowThreads, 0, (cudaStream_t)stream>>>( \
+  const int threads = row_threads(H);
+  const int64_t most = (int64_t)num_sms() * (row_vecs(H) == 4 ? 3 : 1024 / threads);   // resident at once: 80 registers a thread for four pieces
+  const unsigned grid = (unsigned)(T < most ? T : most);
+#define PRL_FWD(V) rmsnorm_fwd_kernel<V><<<grid, threads, 0, (cudaStream_t)stream>>>( \
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)gamma, T, (int)H, eps, (__nv_bfloat16*)y, rstd)
-  if (H <= 2048) PRL_FWD(1); else if (H <= 4096) PRL_FWD(2); else PRL_FWD(4);
+  switch (row_vecs(H)) { case 1: PRL_FWD(1); break; case 2: PRL_FWD(2); break; case 3: PRL_FWD(3); break; default: PRL_FWD(4); }
 #undef PRL_FWD
   PRL_LAUNCH_CHECK();
   return PRL_OK;
@@ -315,15 +391,14 @@ extern "C" int prl_rmsnorm_bwd(const void* x, const void* gamma, const float* rs
   PRL_CHECK_ARG(x && gamma && rstd && dy && dx && dgamma && workspace && T >= 1, "prl_rmsnorm_bwd: bad argument");
   PRL_ROW_ARGS("prl_rmsnorm_bwd", H);
   PRL_CHECK_ARG(workspace_bytes >= prl_rowops_workspace_bytes(H), "prl_rmsnorm_bwd: workspace too small");
-  const int g = row_grid(T);
-#define PRL_BWD(V) rmsnorm_bwd_kernel<V><<<g, kRowThreads, 0, (cudaStream_t)stream>>>( \
+  const int g = row_bwd_grid(T, H), threads = row_threads(H);
+#define PRL_BWD(V) rmsnorm_bwd_kernel<V><<<g, threads, 0, (cudaStream_t)stream>>>( \
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)gamma, rstd, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)dres, T, \
       (int)H, (__nv_bfloat16*)dx, (float*)workspace)
-  if (H <= 2048) PRL_BWD(1); else if (H <= 4096) PRL_BWD(2); else PRL_BWD(4);
+  switch (row_vecs(H)) { case 1: PRL_BWD(1); break; case 2: PRL_BWD(2); break; case 3: PRL_BWD(3); break; default: PRL_BWD(4); }
 #undef PRL_BWD
   PRL_LAUNCH_CHECK();
-  partial_reduce_kernel<<<(unsigned)((H + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const float*)workspace, g, (int)H,
-                                                                                       dgamma);
+  PRL_CUDA(launch_partial_reduce((const float*)workspace, g, H, dgamma, (cudaStream_t)stream));
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -339,8 +414,7 @@ extern "C" int prl_colsum_bf16(const void* x, int64_t ld, int64_t T, int64_t col
   if (cols <= 2048) PRL_CS(1); else if (cols <= 4096) PRL_CS(2); else PRL_CS(4);
 #undef PRL_CS
   PRL_LAUNCH_CHECK();
-  partial_reduce_kernel<<<(unsigned)((cols + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const float*)workspace, g,
-                                                                                          (int)cols, out);
+  PRL_CUDA(launch_partial_reduce((const float*)workspace, g, cols, out, (cudaStream_t)stream));
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -352,7 +426,7 @@ extern "C" int prl_rope_inplace(void* x, int64_t ld, int64_t T, int32_t n_heads,
                 "prl_rope_inplace: head_dim must be a multiple of 16 and ld a multiple of 8 covering the rotated heads");
   int threads = n_heads * (head_dim / 16);
   threads = threads > 256 ? 256 : ((threads + 31) / 32 * 32);
-  rope_kernel<<<(unsigned)(T < 8 * kPartialBlocks ? T : 8 * kPartialBlocks), threads, (size_t)head_dim * sizeof(float),
+  rope_kernel<<<(unsigned)(T < 4 * kPartialBlocks ? T : 4 * kPartialBlocks), threads, (size_t)head_dim * sizeof(float),
                 (cudaStream_t)stream>>>((__nv_bfloat16*)x, ld, T, n_heads, head_dim, pos, inv_freq, sign);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
@@ -360,9 +434,8 @@ extern "C" int prl_rope_inplace(void* x, int64_t ld, int64_t T, int32_t n_heads,
 
 extern "C" int prl_silu_mul_fwd(const void* gate_up, int64_t T, int64_t I, void* act, prl_stream_t stream) {
   PRL_CHECK_ARG(gate_up && act && T >= 1 && I >= 8 && I % 8 == 0, "prl_silu_mul_fwd: bad argument (I %% 8 == 0)");
-  const int64_t blocks = (T * (I / 8) + 255) / 256;
-  silu_mul_fwd_kernel<<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)gate_up, T, (int)I, (__nv_bfloat16*)act);
+  silu_mul_fwd_kernel<<<silu_grid(T, I), silu_threads(I), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gate_up, (int)I,
+                                                                                (__nv_bfloat16*)act);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -370,9 +443,9 @@ extern "C" int prl_silu_mul_fwd(const void* gate_up, int64_t T, int64_t I, void*
 extern "C" int prl_silu_mul_bwd(const void* gate_up, const void* dact, int64_t T, int64_t I, void* dgate_up,
                                 prl_stream_t stream) {
   PRL_CHECK_ARG(gate_up && dact && dgate_up && T >= 1 && I >= 8 && I % 8 == 0, "prl_silu_mul_bwd: bad argument");
-  const int64_t blocks = (T * (I / 8) + 255) / 256;
-  silu_mul_bwd_kernel<<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)gate_up, (const __nv_bfloat16*)dact, T, (int)I, (__nv_bfloat16*)dgate_up);
+  silu_mul_bwd_kernel<<<silu_grid(T, I), silu_threads(I), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gate_up,
+                                                                                (const __nv_bfloat16*)dact, (int)I,
+                                                                                (__nv_bfloat16*)dgate_up);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }

@@ -347,3 +347,42 @@ def test_native_learner_fp32_equivalent_head(cuda_device):
     err_bf16 = (head(None) - want).abs().max().item()
     print(f"[fp32-equivalent head] max |dlogprob| hi+lo {err_lo:.2e}   bf16 head {err_bf16:.2e}")
     assert err_lo <= 2e-4 and err_lo < 0.2 * err_bf16
+
+
+@pytest.mark.parametrize("T,H", [(1, 8), (3, 264), (149, 2048), (297, 2056), (600, 4096), (310, 4104), (299, 6144), (150, 6152),
+                                 (445, 8192), (1300, 896)])
+def test_norm_rows_at_the_edges_of_their_blocks(cuda_device, T, H):
+    """Widths around the pieces a thread holds, row counts around the resident blocks, with and without the residual gradient.
+    bf16 outputs: one rounding of the fp32 result, whose sums over H terms are within H * 2^-24 of their magnitudes."""
+    from pipelinerl_b200.learner_body import Ops
+    o, g = Ops(), torch.Generator().manual_seed(T + H)
+    x, dy, dres = (torch.randn(T, H, generator=g).to(torch.bfloat16).to(cuda_device) for _ in range(3))
+    gamma = (1 + 0.1 * torch.randn(H, generator=g)).to(torch.bfloat16).to(cuda_device)
+    y, rstd = o.rmsnorm(x, gamma, 1e-6)
+    xd, gd, dd = x.double(), gamma.double(), dy.double()
+    r = torch.rsqrt((xd * xd).mean(-1, keepdim=True) + 1e-6)
+    xh = xd * r
+    assert ((rstd.double() - r[:, 0]).abs() <= (H * 2.0 ** -24 + 2.0 ** -21) * r[:, 0]).all()
+    assert ((y.double() - xh * gd).abs() <= 2.0 ** -7 * (xh * gd).abs() + 1e-30).all()
+    for res in (dres, None):
+        dgamma = torch.ones(H, device=cuda_device)
+        dx = o.rmsnorm_bwd(x, gamma, rstd, dy, res, dgamma)
+        want = r * (dd * gd - xh * (dd * gd * xh).mean(-1, keepdim=True)) + (0 if res is None else res.double())
+        slack = 2.0 ** -8 * want.abs() + 1e-5 * (r * (dd * gd).abs() + r * xh.abs()) + 1e-6
+        assert ((dx.double() - want).abs() <= slack).all()
+        total = 1 + (dd * xh).sum(0)
+        assert ((dgamma.double() - total).abs() <= (T + 64) * 2.0 ** -23 * (1 + (dd * xh).abs().sum(0))).all()
+
+
+@pytest.mark.parametrize("T,I", [(1, 8), (2, 18944), (37, 2056), (700, 24), (1500, 4096)])
+def test_silu_rows_cut_over_blocks(cuda_device, T, I):
+    from pipelinerl_b200.learner_body import Ops
+    o, g = Ops(), torch.Generator().manual_seed(T + I)
+    gu = (3 * torch.randn(T, 2 * I, generator=g)).to(torch.bfloat16).to(cuda_device)
+    da = torch.randn(T, I, generator=g).to(torch.bfloat16).to(cuda_device)
+    a, u, d = gu[:, :I].double(), gu[:, I:].double(), da.double()
+    s = torch.sigmoid(a)
+    assert ((o.silu_mul(gu).double() - a * s * u).abs() <= 2.0 ** -8 * (a * s * u).abs() + 1e-6).all()
+    dgu = o.silu_mul_bwd(gu, da).double()
+    want = torch.cat([d * u * (s + a * s * (1 - s)), d * a * s], 1)
+    assert ((dgu - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
