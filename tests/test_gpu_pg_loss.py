@@ -290,3 +290,44 @@ def test_gspo_under_sequence_parallelism_matches_the_whole_row(cuda_device, sp):
             assert dlp_f[a + Tl - 1].item() == 0.0        # the position that would score the next slice's first token
     assert abs(loss_sum - loss_f.item()) <= 1e-5 * max(1.0, abs(loss_f.item())), (loss_sum, loss_f.item())
     assert abs(loss_f.item()) > 1e-3                      # the case is not degenerate
+
+
+@pytest.mark.parametrize("T,V,pad", [(2, 1, 0), (3, 7, 1), (5, 2048, 0), (4, 8191, 0), (3, 8192, 4), (3, 8197, 3), (2, 151936, 0)])
+def test_logprob_tail_at_the_edges_of_its_groups(cuda_device, T, V, pad):
+    """Log-probs and entropies of rows around the groups of 16 values a thread adds at once, rows that start off 16 bytes, values
+    that rise along the row (a new maximum in every group).  Sums of V terms in fp32: V * 2^-24 of the sum, and the exponentials'
+    own error of 2^-21."""
+    from pipelinerl_b200 import _lib
+    lib, g = _lib.load(), torch.Generator().manual_seed(T + V)
+    z = 3 * torch.randn(T, V + pad, generator=g)
+    z[0] += torch.linspace(-20, 20, V + pad)
+    z = z.to(cuda_device)[:, :V]
+    ids = torch.randint(0, V, (T,), generator=g).to(cuda_device)
+    lp, ent, lse = (torch.empty(T - 1, device=cuda_device) for _ in range(3))
+    _lib.check(lib.prl_logprob_tail_fwd(z.data_ptr(), T, V, z.stride(0), ids.data_ptr(), 0.7, lp.data_ptr(), ent.data_ptr(),
+                                        lse.data_ptr(), _lib.stream_ptr()))
+    ref = torch.log_softmax(z[:-1].double() / 0.7, -1)
+    want = ref.gather(1, ids[1:, None])[:, 0]
+    entropy = -(ref.exp() * ref).sum(-1)
+    top = (z[:-1].double().abs().amax() / 0.7 + 20).item()
+    slack = top * (2.0 ** -20 + min(V, 4096) * 2.0 ** -24)
+    assert (lp.double() - want).abs().max().item() <= slack
+    assert (ent.double() - entropy).abs().max().item() <= 2 * slack
+
+
+def test_rl_step_over_several_rows_of_logits(cuda_device):
+    """Two unpacked rows: every row's gradient arrives in its own place of the [B, L, V] logits."""
+    from pipelinerl_b200.finetune.rl import RLConfig, rl_step
+    arrs, meta = load_rl_case("unpacked")
+    batch = batch_from_arrays(arrs, cuda_device)
+    both = LogitsModel(torch.from_numpy(arrs["logits"]).to(cuda_device))
+    loss, _ = rl_step(both, batch, 0, 10, RLConfig(**meta["config"]))
+    loss.backward()
+    half = torch.from_numpy(arrs["logits"]).to(cuda_device).to(torch.bfloat16).requires_grad_()
+    model = LogitsModel(half.detach())
+    loss16, _ = rl_step(model, batch, 0, 10, RLConfig(**meta["config"]))
+    loss16.backward()
+    assert model.logits.grad.dtype == torch.bfloat16 and model.logits.grad.shape == both.logits.grad.shape
+    scale = both.logits.grad.abs().max()
+    assert (model.logits.grad.float() - both.logits.grad).abs().max() <= 0.05 * scale   # 2^-8 logits: their log-probs are ~1e-2 off
+    assert both.logits.grad.shape[0] > 1 and all(g.abs().max() > 0 for g in both.logits.grad)
