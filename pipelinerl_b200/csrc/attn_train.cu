@@ -23,7 +23,7 @@
 // Both: warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner (the WHOLE warp runs converged and elects one lane per batch of
 // UMMAs: issued from `if (lane == 0)` every UMMA costs ~180 cycles of R2UR + ELECT waterfall, tc_ptx.cuh: elect_one), the other
 // warps = softmax: 8 in lock-step in generations 1-3, 16 that never meet in generation 4 (the default; further down).
-// All four generations produce the same bits.
+// All four generations produce the same bits (generation 4 where its dK / dV kernel takes one CTA per key tile, see dkdv_split).
 //
 // Tensor-bound (profiles/r2_attention.md: the MMA warps sit in UMMA issue back-pressure).  Per (128 query rows x 128 keys)
 // pair: 4 + 3 UMMA products of 4.2 MFLOP against 5 for the atomics-based single-kernel formulation; 2 x 16 K exp2.
@@ -60,6 +60,8 @@ struct BwdParams {
   __nv_bfloat16* dkv;            // where dK / dV rows go: [kv rows, dkv_stride], columns dkv_col_k / dkv_col_v (+ head * 128)
   int64_t dkv_stride;
   int dkv_col_k, dkv_col_v;
+  int n_lin;                     // generation-4 dK / dV kernel: kv heads x sequences, the fast index of its one-dimensional grid
+  int split;                     // CTAs (one cluster) that share the queries of a key tile in the generation-4 dK / dV kernel
 };
 
 __device__ __forceinline__ float ex2f(float x) {
@@ -722,6 +724,28 @@ __device__ __forceinline__ void group_bar256(int g) {
   else asm volatile("bar.sync 2, 256;" ::: "memory");
 }
 
+// A key tile at the start of a long sequence sees all its queries, one at the end few: with a tile per CTA the first tile's walk is
+// the kernel's time wherever the tiles do not fill the chip several times (14 / 2 heads, longest of six samples 2300: 256 steps in
+// the longest CTA, 235 us, where the work of all CTAs is 54 steps per SM).  `split` CTAs of one cluster therefore share a tile's
+// queries and add their dV / dK in the end through each other's shared memory (the drained Q / dO ring), in the order of the
+// cluster's ranks: still no atomics, one order, every run the same bits.
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t cta) {
+  float4 v;
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\t"
+      "mapa.shared::cluster.u32 ra, %4, %5;\n\t"
+      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n\t}"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "r"(addr), "r"(cta)
+      : "memory");
+  return v;
+}
+// 16-byte piece c4 of row `row` of dV (which = 0) or dK (1), [128 keys x 128] fp32 each, pieces of a row swizzled
+__device__ __forceinline__ uint32_t acc_piece(uint32_t ring, int which, int row, int c4) {
+  return ring + (uint32_t)(which * 65536 + row * 512 + ((c4 ^ (row & 31)) << 4));
+}
+static_assert(kQStages4 * kQSlot >= 2 * 128 * 128 * 4, "the ring holds a tile's dV and dK");
+
 template <bool kTimed>
 __global__ void __launch_bounds__(kThreadsB4, 1)
 attn_bwd_dkdv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
@@ -737,17 +761,21 @@ attn_bwd_dkdv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const uint32_t tmem_slot = bar(14);
   float* meta = reinterpret_cast<float*>(smem_raw + (meta_smem - ptx::smem_u32(smem_raw)));
 
-  const int jt = blockIdx.x, kvh = blockIdx.y, z = blockIdx.z;
+  // the first, longest tiles of all heads and sequences come first (eight samples of 2048: 1034 -> 915 us with the dQ kernel, which
+  // like the forward got slower in this order: 8 x 2048 forward 397 -> 427)
+  const int item = (int)blockIdx.x / p.split, part = (int)blockIdx.x - item * p.split;
+  const int jt = item / p.n_lin, lin = item - jt * p.n_lin, kvh = lin % p.n_kv, z = lin / p.n_kv;
   const int q_len = ptx::warp_uniform(p.seg_len[z]);
   const int key0 = jt * 128;
   const int pos0 = p.seg_pos0 ? ptx::warp_uniform(p.seg_pos0[z]) : 0;   // position of local query 0 (sequence-parallel slice)
-  if (key0 >= pos0 + q_len) return;                // before any barrier / TMEM use
+  if (key0 >= pos0 + q_len) return;                // the whole cluster, before any barrier / TMEM use
   const int seg0 = ptx::warp_uniform(p.seg_start[z]);
   const int kv0 = p.seg_kv_start ? ptx::warp_uniform(p.seg_kv_start[z]) : seg0;
   const int nqa = p.nq;
-  const int u_first = (key0 > pos0 ? key0 - pos0 : 0) / nqa;   // first 64-row query sub-tile holding a position >= key0
-  const int u_end = (q_len + nqa - 1) / nqa;
-  const int n_it = u_end - u_first;
+  const int u_tile = (key0 > pos0 ? key0 - pos0 : 0) / nqa;   // first 64-row query sub-tile holding a position >= key0
+  const int u_count = (q_len + nqa - 1) / nqa - u_tile;
+  const int u_first = u_tile + u_count * part / p.split;      // this CTA's share of them
+  const int n_it = u_tile + u_count * (part + 1) / p.split - u_first;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   {
@@ -834,11 +862,11 @@ attn_bwd_dkdv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           ptx::tc_commit(bar(9 + s));
         }
       };
-      const bool timed = kTimed && p.timing != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
+      const bool timed = kTimed && p.timing != nullptr && blockIdx.x == 0;
       long long w_pds = 0;
       const long long w0 = clock64();
       ptx::mbar_wait(bar(0), 0);
-      issue_sdp(0);
+      if (n_it > 0) issue_sdp(0);
       for (int it = 0; it < n_it; ++it) {
         if (it + 1 < n_it) issue_sdp(it + 1);
         const int st = it % kQStages4, s = it & 1;
@@ -897,7 +925,7 @@ attn_bwd_dkdv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     float nxt = (g + 2 < n_it) ? fetch(u_first + g + 2) : 0.f;
     group_bar256(g);                             // metadata of own step 0 is visible to the whole group
 
-    const bool timed = kTimed && p.timing != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && warp == 2 && lane == 0;
+    const bool timed = kTimed && p.timing != nullptr && blockIdx.x == 0 && warp == 2 && lane == 0;
     long long tph[5] = {0, 0, 0, 0, 0};
     for (int j = 0; j < n_own; ++j) {
       const int it = 2 * j + g;
@@ -971,6 +999,20 @@ attn_bwd_dkdv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     // ---- epilogue: 32 head-dim columns of this key's dV and dK rows ----
     ptx::mbar_wait(bar(13), 0);
     ptx::tc_fence_after_sync();
+    if (p.split > 1) {                            // fp32, to this CTA's ring: its loads and products are all done
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        uint32_t v0[32];
+        ptx::tmem_ld_32x32b_x32(lane_addr + (uint32_t)(256 + which * 128 + idx * 32), v0);
+        ptx::tmem_ld_wait();
+#pragma unroll
+        for (int d = 0; d < 32; d += 4) {
+          const uint32_t a = acc_piece(q_ring, which, m, (idx * 32 + d) >> 2);
+          if (n_it > 0) sts_v4(a, v0[d], v0[d + 1], v0[d + 2], v0[d + 3]);
+          else sts_v4(a, 0u, 0u, 0u, 0u);         // no share of the queries: the accumulators were never written
+        }
+      }
+    } else {
     const bool valid = kpos < pos0 + q_len;
     __nv_bfloat16* drow = p.dkv + (int64_t)(kv0 + kpos) * p.dkv_stride + kvh * kD + idx * 32;
 #pragma unroll
@@ -992,10 +1034,38 @@ attn_bwd_dkdv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         }
       }
     }
+    }
   }
 
   ptx::tc_fence_before_sync();
-  __syncthreads();
+  if (p.split > 1) {
+    __syncwarp();
+    ptx::cluster_sync();                          // every CTA's dV and dK are in its ring
+    const int rows = 128 / p.split;               // keys that this CTA adds up and writes
+    for (int i = threadIdx.x; i < 2 * rows * 16; i += kThreadsB4) {   // [dV | dK][key][8 columns]
+      const int which = i / (rows * 16), r = part * rows + (i >> 4) % rows, c8 = i & 15;
+      float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+      for (int c = 0; c < p.split; ++c) {
+        const float4 a = ld_cluster_f4(acc_piece(q_ring, which, r, 2 * c8), (uint32_t)c);
+        const float4 b = ld_cluster_f4(acc_piece(q_ring, which, r, 2 * c8 + 1), (uint32_t)c);
+        lo.x += a.x; lo.y += a.y; lo.z += a.z; lo.w += a.w;
+        hi.x += b.x; hi.y += b.y; hi.z += b.z; hi.w += b.w;
+      }
+      if (key0 + r < pos0 + q_len) {
+        const float sc = which ? p.sm_scale : 1.f;
+        uint4 o;
+        o.x = pk2(lo.x * sc, lo.y * sc);
+        o.y = pk2(lo.z * sc, lo.w * sc);
+        o.z = pk2(hi.x * sc, hi.y * sc);
+        o.w = pk2(hi.z * sc, hi.w * sc);
+        *reinterpret_cast<uint4*>(p.dkv + (int64_t)(kv0 + key0 + r) * p.dkv_stride + kvh * kD + c8 * 8 +
+                                  (which ? p.dkv_col_k : p.dkv_col_v)) = o;
+      }
+    }
+    ptx::cluster_sync();                          // nobody leaves while its ring is read
+  } else {
+    __syncthreads();
+  }
   if (warp == 1) {
     ptx::tc_fence_after_sync();
     ptx::tmem_dealloc(tmem_base, 512);
@@ -1288,6 +1358,41 @@ extern "C" int prl_attn_debug_bwd_timing_dkdv(int64_t* out16_device) {
   return PRL_OK;
 }
 
+// CTAs per key tile of the generation-4 dK / dV kernel: the fewest microseconds of a model with 0.92 us per step (128 keys x 64
+// query rows) and 8 us around a CTA's steps, over the longest CTA and over the work of all of them spread on the SMs.  The tokens'
+// split into sequences is known on the device only: T tokens in sequences of at most `longest` are taken as the bound that they
+// are.  Whole backward, one CTA per tile -> the rule's choice: 28 / 4 heads, samples of 2049, 1500 and 547: 334 -> 246 us (2);
+// 14 / 2 heads, longest of six samples 2300: 323 -> 208 (4); 16 / 1 heads, 5000 and 300: 1219 -> 442 (4); 28 / 4, 8192: 1405 ->
+// 1370 (1); 16384: one CTA, whose tiles fill the chip three times (2: +2 %, 4: +11 %).
+static int dkdv_split(int64_t T, int64_t longest, int n_seg, int n_kv, int nq) {
+  const double steps = (double)n_kv * (double)T * (double)longest / (256.0 * nq), tiles = (double)n_kv * ((double)T / 128 + n_seg);
+  int best = 1;
+  double best_us = 0;
+  for (int s = 1; s <= 8; s *= 2) {
+    const double path = (double)longest / nq / s * 0.92 + 8.0;
+    const double all = (steps * 0.92 + tiles * s * 8.0) / num_sms();
+    const double us = path > all ? path : all;
+    if (s == 1 || us < 0.9 * best_us) { best = s; best_us = us; }
+  }
+  return best;
+}
+template <bool kTimed>
+static cudaError_t launch_dkdv4(dim3 grid, cudaStream_t stream, const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap& tkv,
+                                const BwdParams& p) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid.x * grid.y * grid.z * (unsigned)p.split);
+  cfg.blockDim = dim3(kThreadsB4);
+  cfg.dynamicSmemBytes = kSmemDkdv4;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)p.split;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, attn_bwd_dkdv4_kernel<kTimed>, tq, tdo, tkv, p);
+}
+
 extern "C" int prl_attn_set_bwd_generation(int32_t gen) {
   PRL_CHECK_ARG(gen >= 1 && gen <= 4, "prl_attn_set_bwd_generation: 1 (P / dS operands through shared memory), 2 (through TMEM), "
                 "3 (2 + the dQ kernel keeps Q and dO in TMEM) or 4 (16 decoupled softmax warps)");
@@ -1330,6 +1435,8 @@ extern "C" int prl_attn_varlen_bwd(const void* qkv, int64_t qkv_stride, int32_t 
   p.timing = g_bwd_timing;
   p.seg_pos0 = nullptr; p.seg_kv_start = nullptr; p.dkv = (__nv_bfloat16*)dqkv; p.dkv_stride = dqkv_stride;
   p.dkv_col_k = p.col_k; p.dkv_col_v = p.col_v;
+  p.n_lin = n_kv * n_seg;
+  p.split = dkdv_split(T, max_seg_len, n_seg, n_kv, 64 / p.R);
   CUtensorMap tkv, tq, tdo;
   int rc = make_tmap_2d_bf16(&tkv, qkv, (uint64_t)width, (uint64_t)T, (uint64_t)qkv_stride * 2, 64, 64);
   if (rc) return rc;
@@ -1347,10 +1454,10 @@ extern "C" int prl_attn_varlen_bwd(const void* qkv, int64_t qkv_stride, int32_t 
       if (g_bwd_timing != nullptr && g_bwd_timing_kernel == 0) {
         static SmemAttr attr4t = {};
         PRL_CUDA(ensure_smem(attn_bwd_dkdv4_kernel<true>, kSmemDkdv4, attr4t));
-        attn_bwd_dkdv4_kernel<true><<<grid, kThreadsB4, (size_t)kSmemDkdv4, stream>>>(tq, tdo, tkv, p);
+        PRL_CUDA(launch_dkdv4<true>(grid, stream, tq, tdo, tkv, p));
       } else {
         PRL_CUDA(ensure_smem(attn_bwd_dkdv4_kernel<false>, kSmemDkdv4, attr4));
-        attn_bwd_dkdv4_kernel<false><<<grid, kThreadsB4, (size_t)kSmemDkdv4, stream>>>(tq, tdo, tkv, p);
+        PRL_CUDA(launch_dkdv4<false>(grid, stream, tq, tdo, tkv, p));
       }
     } else if (g_bwd_generation == 1) {   // generations 2 and 3 share the dK / dV kernel
       PRL_CUDA(ensure_smem(attn_bwd_dkdv_kernel<false>, kSmemDkdv, attr));
@@ -1436,6 +1543,8 @@ extern "C" int prl_attn_varlen_bwd_kv(const void* q, int64_t q_stride, int32_t T
   p.timing = nullptr;
   p.seg_pos0 = seg_pos0; p.seg_kv_start = seg_kv_start; p.dkv = (__nv_bfloat16*)dkv; p.dkv_stride = dkv_stride;
   p.dkv_col_k = 0; p.dkv_col_v = n_kv * kD;
+  p.n_lin = n_kv * n_seg;
+  p.split = 1;                   // one CTA per key tile: the split's rule is about whole sequences
   CUtensorMap tkv, tq, tdo;
   int rc = make_tmap_2d_bf16(&tkv, kv, (uint64_t)kvw, (uint64_t)Tkv, (uint64_t)kv_stride * 2, 64, 64);
   if (rc) return rc;
@@ -1448,7 +1557,7 @@ extern "C" int prl_attn_varlen_bwd_kv(const void* q, int64_t q_stride, int32_t T
     dim3 grid((unsigned)((max_kv_len + 127) / 128), (unsigned)n_kv, (unsigned)n_seg);
     static SmemAttr attr = {};
     PRL_CUDA(ensure_smem(attn_bwd_dkdv4_kernel<false>, kSmemDkdv4, attr));
-    attn_bwd_dkdv4_kernel<false><<<grid, kThreadsB4, (size_t)kSmemDkdv4, stream>>>(tq, tdo, tkv, p);
+    PRL_CUDA(launch_dkdv4<false>(grid, stream, tq, tdo, tkv, p));
     PRL_LAUNCH_CHECK();
   }
   {

@@ -197,3 +197,25 @@ def test_sequence_parallel_slices_match_full_attention(cuda_device, n_q, n_kv, l
     err = (dkv_sum - want).abs().max().item() / scale
     print(f"[attn sp={sp}] n_q={n_q} n_kv={n_kv} lens={lens}: sum of rank dK/dV vs single rank rel {err:.2e}")
     assert err <= 2 ** -7, err
+
+
+@pytest.mark.parametrize("n_q,n_kv,lens", [
+    (16, 1, [1500, 3]),        # eight CTAs per key tile
+    (5, 1, [700, 20]),         # four; shares of one or two steps in the short sample, empty ones at the end of the long one
+    (14, 2, [900, 130, 129]),  # two to four
+    (28, 4, [300]),
+    (64, 1, [70, 1]),          # one query token per step
+])
+def test_varlen_backward_with_shared_key_tiles(cuda_device, n_q, n_kv, lens):
+    """Several CTAs share a key tile's queries: gradients against the oracle, and the same bits in every run."""
+    _run(cuda_device, n_q, n_kv, lens, seed=17, fwd_gen=2, bwd_gen=4)
+    o, T = _ops(), sum(lens)
+    g = torch.Generator().manual_seed(1)
+    qkv = torch.randn(T, (n_q + 2 * n_kv) * 128, generator=g).to(torch.bfloat16).to(cuda_device)
+    d = torch.randn(T, n_q * 128, generator=g).to(torch.bfloat16).to(cuda_device)
+    st = torch.tensor([sum(lens[:i]) for i in range(len(lens))], dtype=torch.int32, device=cuda_device)
+    ln = torch.tensor(lens, dtype=torch.int32, device=cuda_device)
+    shape = (st, ln, max(lens), n_q, n_kv, 128)
+    out, lse = o.attn_fwd(qkv, *shape)
+    first = o.attn_bwd(qkv, out, d, lse, *shape)
+    assert all(torch.equal(first, o.attn_bwd(qkv, out, d, lse, *shape)) for _ in range(3))
