@@ -373,6 +373,8 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   auto bar = [&](int i) { return bar_base + 8u * (uint32_t)i; };
   // 0 q_full | 1..3 k_full | 4..6 k_empty | 7,8 s_full | 9,10 p_full | 11,12 o_full | 13..15 v_full | 16..18 v_empty
   const uint32_t tmem_slot = bar(19);
+  pdl_launch_dependents();
+  pdl_wait();                                            // the sequence tables below may be fresh
 
   const int qtile = kContig ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
   const int kvh = blockIdx.y, z = blockIdx.z;
@@ -725,7 +727,7 @@ static int prefill_tc_impl(const void* q, int32_t q_rows, const void* kv_cache, 
   if (g_prefill_generation == 2 || window || sink || gate) {      // ping-pong softmax groups, P and O in TMEM (see attn_fwd_v2_kernel)
     static SmemAttr smem_attr2 = {};
     PRL_CUDA(ensure_smem(attn_fwd_v2_kernel<false>, smem, smem_attr2));
-    attn_fwd_v2_kernel<false><<<grid, kThreadsT, (size_t)smem, (cudaStream_t)stream_>>>(tq, tkv, p);
+    PRL_CUDA(launch_pdl(attn_fwd_v2_kernel<false>, grid, dim3(kThreadsT), (size_t)smem, (cudaStream_t)stream_, tq, tkv, p));
   } else {
     PRL_CUDA(ensure_smem(attn_prefill_tc_kernel<false>, smem, smem_attr));
     attn_prefill_tc_kernel<false><<<grid, kThreadsT, (size_t)smem, (cudaStream_t)stream_>>>(tq, tkv, p);
@@ -811,11 +813,11 @@ extern "C" int prl_attn_varlen_fwd(const void* qkv, int64_t qkv_stride, int32_t 
   } else if (g_fwd_timing != nullptr) {
     static SmemAttr smem_attr_t = {};
     PRL_CUDA(ensure_smem(attn_fwd_v2_kernel<true, true>, smem, smem_attr_t));
-    attn_fwd_v2_kernel<true, true><<<grid, kThreadsT, (size_t)smem, (cudaStream_t)stream_>>>(tq, tkv, p);
+    PRL_CUDA(launch_pdl(attn_fwd_v2_kernel<true, true>, grid, dim3(kThreadsT), (size_t)smem, (cudaStream_t)stream_, tq, tkv, p));
   } else {
     static SmemAttr smem_attr2 = {};
     PRL_CUDA(ensure_smem(attn_fwd_v2_kernel<true>, smem, smem_attr2));
-    attn_fwd_v2_kernel<true><<<grid, kThreadsT, (size_t)smem, (cudaStream_t)stream_>>>(tq, tkv, p);
+    PRL_CUDA(launch_pdl(attn_fwd_v2_kernel<true>, grid, dim3(kThreadsT), (size_t)smem, (cudaStream_t)stream_, tq, tkv, p));
   }
   PRL_LAUNCH_CHECK();
   return PRL_OK;
@@ -854,7 +856,7 @@ extern "C" int prl_attn_varlen_fwd_kv(const void* q, int64_t q_stride, int32_t T
   dim3 grid((unsigned)(((max_q_len + p.nq - 1) / p.nq + 1) & ~1), (unsigned)n_kv, (unsigned)n_seg);
   static SmemAttr smem_attr = {};
   PRL_CUDA(ensure_smem(attn_fwd_v2_kernel<true>, smem, smem_attr));
-  attn_fwd_v2_kernel<true><<<grid, kThreadsT, (size_t)smem, (cudaStream_t)stream_>>>(tq, tkv, p);
+  PRL_CUDA(launch_pdl(attn_fwd_v2_kernel<true>, grid, dim3(kThreadsT), (size_t)smem, (cudaStream_t)stream_, tq, tkv, p));
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }

@@ -196,7 +196,9 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
   const uint32_t rank = ptx::cluster_ctarank();
   const int n_clusters = (int)gridDim.x >> 1;
   const int cluster = (int)blockIdx.x >> 1;
-  const int total_tiles = p.g_tiles ? p.g_meta[0] * p.n_tiles : p.m_tiles * p.n_tiles * (p.split > 1 ? p.split : 1);
+  // Programmatic launch: barriers, tensor memory and tensor maps are set up under the tail of the kernel before (about 4 of the
+  // 10 us that a launch takes beside its main loop); nothing it wrote, and nothing it still reads, is touched before pdl_wait
+  pdl_launch_dependents();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -222,6 +224,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
   ptx::tc_fence_after_sync();
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+  pdl_wait();
+  const int total_tiles = p.g_tiles ? p.g_meta[0] * p.n_tiles : p.m_tiles * p.n_tiles * (p.split > 1 ? p.split : 1);
 
   if (warp == 0) {
     // ===== TMA producer (both CTAs) =====
@@ -759,7 +763,7 @@ extern "C" int prl_gemm_ex(const void* A, int64_t lda, int32_t a_mn_major, const
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   int clusters = num_sms() / 2;
   if (tiles < clusters) clusters = (int)tiles;
-  gemm_tn_kernel<false><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta, tb, p);
+  PRL_CUDA(launch_pdl(gemm_tn_kernel<false>, dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_, ta, tb, ta, tb, p));
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -806,7 +810,7 @@ extern "C" int prl_gemm_tn_dual(const void* A1, const void* B1, int64_t K1, cons
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles * split_k;
   int clusters = num_sms() / 2;
   if (tiles < clusters) clusters = (int)tiles;
-  gemm_tn_kernel<false><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta2, tb2, p);
+  PRL_CUDA(launch_pdl(gemm_tn_kernel<false>, dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_, ta, tb, ta2, tb2, p));
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -843,7 +847,7 @@ extern "C" int prl_moe_gemm_tc(const void* A, int64_t rows_cap, const void* W, i
   const int64_t items = ((rows_cap + kTile - 1) / kTile + experts) * p.n_tiles;
   int clusters = num_sms() / 2;
   if (items < clusters) clusters = (int)items;
-  gemm_tn_kernel<false><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta, tb, p);
+  PRL_CUDA(launch_pdl(gemm_tn_kernel<false>, dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_, ta, tb, ta, tb, p));
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -878,7 +882,7 @@ extern "C" int prl_gemm_dgrad_swiglu(const void* dY, int64_t ldy, const void* W_
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   int clusters = num_sms() / 2;
   if (tiles < clusters) clusters = (int)tiles;
-  gemm_tn_kernel<false><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta, tb, p);
+  PRL_CUDA(launch_pdl(gemm_tn_kernel<false>, dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_, ta, tb, ta, tb, p));
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -946,7 +950,7 @@ static int gemm_swiglu_impl(const void* X, int64_t ldx, const void* W, int64_t l
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   int clusters = num_sms() / 2;
   if (tiles < clusters) clusters = (int)tiles;
-  gemm_tn_kernel<false><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta, tb, p);
+  PRL_CUDA(launch_pdl(gemm_tn_kernel<false>, dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_, ta, tb, ta, tb, p));
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -981,7 +985,7 @@ int head_logprob_tn(const void* W, const void* W_lo, const void* X, int64_t M, i
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   int clusters = num_sms() / 2;
   if (tiles < clusters) clusters = (int)tiles;
-  gemm_tn_kernel<true><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<true>), (size_t)smem, stream>>>(ta, tb, ta, tb2, p);
+  PRL_CUDA(launch_pdl(gemm_tn_kernel<true>, dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<true>), (size_t)smem, stream, ta, tb, ta, tb2, p));
   PRL_LAUNCH_CHECK();
   head_tn_combine_kernel<<<(unsigned)((M + 3) / 4), 128, 0, stream>>>((const float4*)workspace, p.n_tiles, M,
                                                                       targets ? 1 : 0, logprob_target, entropy, lse);
@@ -1030,7 +1034,7 @@ extern "C" int prl_head_dlogits(const void* W, const void* W_lo, const void* X, 
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   int clusters = num_sms() / 2;
   if (tiles < clusters) clusters = (int)tiles;
-  gemm_tn_kernel<true><<<dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<true>), (size_t)smem, (cudaStream_t)stream_>>>(ta, tb, ta, tb2, p);
+  PRL_CUDA(launch_pdl(gemm_tn_kernel<true>, dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<true>), (size_t)smem, (cudaStream_t)stream_, ta, tb, ta, tb2, p));
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
