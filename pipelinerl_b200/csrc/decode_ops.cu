@@ -40,8 +40,29 @@ __device__ __forceinline__ float block_sum(float v, float* s_red) {
   return t;
 }
 
+// W neighbouring bf16 as floats / floats to W neighbouring bf16: one 8-byte access for W = 4
+template <int W>
+__device__ __forceinline__ void load_bf16(const __nv_bfloat16* p, float (&v)[W]) {
+  if constexpr (W == 4) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    v[0] = bf16_bits_to_float(u.x & 0xffffu); v[1] = bf16_bits_to_float(u.x >> 16);
+    v[2] = bf16_bits_to_float(u.y & 0xffffu); v[3] = bf16_bits_to_float(u.y >> 16);
+  } else {
+    v[0] = __bfloat162float(p[0]);
+  }
+}
+template <int W>
+__device__ __forceinline__ void store_bf16(__nv_bfloat16* p, const float (&v)[W]) {
+  if constexpr (W == 4)
+    *reinterpret_cast<uint2*>(p) = make_uint2(float_to_bf16_bits(v[0]) | (float_to_bf16_bits(v[1]) << 16),
+                                              float_to_bf16_bits(v[2]) | (float_to_bf16_bits(v[3]) << 16));
+  else p[0] = __float2bfloat16_rn(v[0]);
+}
+
 // ---- embedding gather + RMSNorm ------------------------------------------------------
-// h[b,:] = embed[token[b],:] ; x[b,:] = bf16(h * rsqrt(mean(h^2) + eps) * g)
+// h[b,:] = embed[token[b],:] ; x[b,:] = bf16(h * rsqrt(mean(h^2) + eps) * g).  W = 4: rows of whole 8-byte pieces
+// (1024 x 3584: 13.2 us with one channel per access).
+template <int W>
 __global__ void __launch_bounds__(256) embed_rmsnorm_kernel(const int32_t* __restrict__ tokens,
                                                            const __nv_bfloat16* __restrict__ embed,
                                                            const __nv_bfloat16* __restrict__ gamma, float eps, int H,
@@ -55,16 +76,23 @@ __global__ void __launch_bounds__(256) embed_rmsnorm_kernel(const int32_t* __res
   if (tok < 0 || tok >= vocab) tok = 0;
   const __nv_bfloat16* row = embed + (int64_t)tok * H;
   float ss = 0.f;
-  for (int i = threadIdx.x; i < H; i += blockDim.x) {
-    const float v = __bfloat162float(row[i]);
-    h[(int64_t)b * H + i] = v;
-    ss += v * v;
+  for (int i = threadIdx.x * W; i < H; i += blockDim.x * W) {
+    float v[W];
+    load_bf16<W>(row + i, v);
+    if constexpr (W == 4) *reinterpret_cast<float4*>(h + (int64_t)b * H + i) = make_float4(v[0], v[1], v[2], v[3]);
+    else h[(int64_t)b * H + i] = v[0];
+#pragma unroll
+    for (int e = 0; e < W; ++e) ss += v[e] * v[e];
   }
   const float tot = block_sum(ss, s_red);
   const float r = rsqrtf(tot / (float)H + eps);
-  for (int i = threadIdx.x; i < H; i += blockDim.x) {
-    const float v = __bfloat162float(row[i]);
-    x[(int64_t)b * H + i] = __float2bfloat16_rn(v * r * __bfloat162float(gamma[i]));
+  for (int i = threadIdx.x * W; i < H; i += blockDim.x * W) {
+    float v[W], g[W];
+    load_bf16<W>(row + i, v);
+    load_bf16<W>(gamma + i, g);
+#pragma unroll
+    for (int e = 0; e < W; ++e) v[e] = v[e] * r * g[e];
+    store_bf16<W>(x + (int64_t)b * H + i, v);
   }
 }
 
@@ -118,6 +146,63 @@ __global__ void __launch_bounds__(1024) residual_rmsnorm_kernel(const float* __r
   }
 }
 
+// The same for MANY rows (prompt chunks), whose time is the rows' way through the SMs and not one row's latency: four pieces per
+// thread in flight, so that a 3584-channel row takes 224 threads and eight rows share an SM, and h is written back only where
+// something was added to it (the wide GEMM of a prompt has added its tile itself: n_split = 0).  1024 x 3584: 17.6 us with a
+// thread per piece and two rows on an SM.
+template <int kPer>
+__global__ void __launch_bounds__(1024) residual_rmsnorm_rows_kernel(const float* __restrict__ part, int n_split, int B, int H,
+                                                                     const __nv_bfloat16* __restrict__ gamma, float eps,
+                                                                     float* __restrict__ h, __nv_bfloat16* __restrict__ x) {
+  pdl_launch_dependents();
+  const int H4 = H >> 2, b = blockIdx.x;
+  float g[kPer][4];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int i = threadIdx.x + k * blockDim.x;
+    if (i < H4) load_bf16<4>(gamma + 4 * i, g[k]);
+  }
+  pdl_wait();
+  __shared__ float s_red[32];
+  float4* hrow = reinterpret_cast<float4*>(h + (int64_t)b * H);
+  float4 v[kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int i = threadIdx.x + k * blockDim.x;
+    v[k] = i < H4 ? hrow[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (n_split > 0) {
+    for (int s = 0; s < n_split; ++s) {
+      const float4* p = reinterpret_cast<const float4*>(part + ((int64_t)s * B + b) * H);
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i < H4) { const float4 a = p[i]; v[k].x += a.x; v[k].y += a.y; v[k].z += a.z; v[k].w += a.w; }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const int i = threadIdx.x + k * blockDim.x;
+      if (i < H4) hrow[i] = v[k];
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
+  const float r = rsqrtf(block_sum(ss, s_red) / (float)H + eps);
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int i = threadIdx.x + k * blockDim.x;
+    if (i >= H4) continue;
+    const float o[4] = {v[k].x * r * g[k][0], v[k].y * r * g[k][1], v[k].z * r * g[k][2], v[k].w * r * g[k][3]};
+    store_bf16<4>(x + (int64_t)b * H + 4 * i, o);
+  }
+}
+
+// the rotated pair, contracted one way in every kernel
+__device__ __forceinline__ float rot_first(float a, float c, float cs, float sn) { return fmaf(a, cs, -__fmul_rn(c, sn)); }
+__device__ __forceinline__ float rot_second(float a, float c, float cs, float sn) { return fmaf(c, cs, __fmul_rn(a, sn)); }
+
 // ---- split-K reduce + bias + RoPE + KV-page write ---------------------------------------
 // part [n_split, B, (n_q + 2 n_kv) * 128]; one block per (token, head), 64 threads = 64 rotation pairs.
 // q -> q_out [B, n_q, 128] bf16 ; k, v -> cache rows ((layer*2 + kv) * n_pages + page) * n_kv * PAGE + kvh*PAGE + slot
@@ -159,8 +244,8 @@ __global__ void __launch_bounds__(64) qkv_rope_cache_kernel(const float* __restr
     const float inv_freq = inv_freq_tab[i];
     float sn, cs;
     sincosf((float)pos * inv_freq, &sn, &cs);
-    o1 = x1 * cs - x2 * sn;
-    o2 = x2 * cs + x1 * sn;
+    o1 = rot_first(x1, x2, cs, sn);
+    o2 = rot_second(x1, x2, cs, sn);
   }
   if (head < n_q) {
     __nv_bfloat16* q = q_out + ((int64_t)b * n_q + head) * D;
@@ -181,7 +266,9 @@ __global__ void __launch_bounds__(64) qkv_rope_cache_kernel(const float* __restr
 
 // Same arithmetic, laid out for MANY rows (prefill chunks): one block walks whole token rows, the row's 64
 // (cos, sin) pairs are computed once (the per-head kernel above recomputes them for each of the n_q + 2 n_kv heads)
-// and every thread handles (head, pair) items with coalesced 4-byte loads.  Bitwise identical results.
+// and every thread handles (head, W neighbouring pairs) items: W = 4 on 16-byte aligned buffers (1024 rows of 36 heads: 12.1 us
+// with a pair per item).  Bitwise identical results.
+template <int W>
 __global__ void __launch_bounds__(256) qkv_rope_cache_rows_kernel(const float* __restrict__ part, int n_split, int B,
                                                                 const __nv_bfloat16* __restrict__ bias, int n_q, int n_kv,
                                                                 const int32_t* __restrict__ positions,
@@ -210,38 +297,49 @@ __global__ void __launch_bounds__(256) qkv_rope_cache_rows_kernel(const float* _
     const int slot_row = row_slot ? row_slot[b] : b;
     const int page = block_table[(int64_t)slot_row * max_blocks + pos / page_size];
     const int slot = pos % page_size;
-    for (int w = threadIdx.x; w < n_heads * 64; w += blockDim.x) {
-      const int head = w >> 6, i = w & 63;
+    for (int w = threadIdx.x; w < n_heads * (64 / W); w += blockDim.x) {
+      const int head = w / (64 / W), i = (w % (64 / W)) * W;
       const int col = head * D + i;
-      float x1 = 0.f, x2 = 0.f;
+      float x1[W], x2[W];
+#pragma unroll
+      for (int e = 0; e < W; ++e) x1[e] = x2[e] = 0.f;
       for (int s = 0; s < n_split; ++s) {
-        const float* p = part + ((int64_t)s * B + b) * ncol;
-        x1 += p[col];
-        x2 += p[col + 64];
+        const float* p = part + ((int64_t)s * B + b) * ncol + col;
+        if constexpr (W == 4) {
+          const float4 a = *reinterpret_cast<const float4*>(p), c = *reinterpret_cast<const float4*>(p + 64);
+          x1[0] += a.x; x1[1] += a.y; x1[2] += a.z; x1[3] += a.w;
+          x2[0] += c.x; x2[1] += c.y; x2[2] += c.z; x2[3] += c.w;
+        } else {
+          x1[0] += p[0];
+          x2[0] += p[64];
+        }
       }
       if (bias) {
-        x1 += __bfloat162float(bias[col]);
-        x2 += __bfloat162float(bias[col + 64]);
+        float b1[W], b2[W];
+        load_bf16<W>(bias + col, b1);
+        load_bf16<W>(bias + col + 64, b2);
+#pragma unroll
+        for (int e = 0; e < W; ++e) { x1[e] += b1[e]; x2[e] += b2[e]; }
       }
       const bool is_v = head >= n_q + n_kv;
-      float o1 = x1, o2 = x2;
       if (!is_v) {
-        const float cs = s_cs[i], sn = s_sn[i];
-        o1 = x1 * cs - x2 * sn;
-        o2 = x2 * cs + x1 * sn;
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+          const float cs = s_cs[i + e], sn = s_sn[i + e], a = x1[e], c = x2[e];
+          x1[e] = rot_first(a, c, cs, sn);
+          x2[e] = rot_second(a, c, cs, sn);
+        }
       }
+      __nv_bfloat16* dst;
       if (head < n_q) {
-        __nv_bfloat16* q = q_out + ((int64_t)b * n_q + head) * D;
-        q[i] = __float2bfloat16_rn(o1);
-        q[i + 64] = __float2bfloat16_rn(o2);
+        dst = q_out + ((int64_t)b * n_q + head) * D;
       } else {
         const int kv = is_v ? 1 : 0;
         const int kvh = is_v ? head - n_q - n_kv : head - n_q;
-        const int64_t row = (((int64_t)(layer * 2 + kv) * n_pages + page) * n_kv + kvh) * page_size + slot;
-        __nv_bfloat16* dst = kv_cache + row * D;
-        dst[i] = __float2bfloat16_rn(o1);
-        dst[i + 64] = __float2bfloat16_rn(o2);
+        dst = kv_cache + ((((int64_t)(layer * 2 + kv) * n_pages + page) * n_kv + kvh) * page_size + slot) * D;
       }
+      store_bf16<W>(dst + i, x1);
+      store_bf16<W>(dst + i + 64, x2);
     }
   }
 }
@@ -449,8 +547,9 @@ using namespace prl;
 extern "C" int prl_embed_rmsnorm(const int32_t* tokens, const void* embed, const void* gamma, float eps, int32_t B,
                                  int32_t H, int32_t vocab, float* h, void* x_bf16, prl_stream_t st) {
   PRL_CHECK_ARG(tokens && embed && gamma && h && x_bf16 && B >= 1 && H >= 1, "prl_embed_rmsnorm: bad argument");
-  PRL_CUDA(launch_pdl(embed_rmsnorm_kernel, dim3(B), dim3(256), 0, (cudaStream_t)st, tokens, (const __nv_bfloat16*)embed,
-                      (const __nv_bfloat16*)gamma, eps, (int)H, (int)vocab, h, (__nv_bfloat16*)x_bf16));
+  const bool vec = H % 4 == 0 && (((uintptr_t)embed | (uintptr_t)gamma | (uintptr_t)x_bf16) & 7) == 0 && ((uintptr_t)h & 15) == 0;
+  PRL_CUDA(launch_pdl(vec ? embed_rmsnorm_kernel<4> : embed_rmsnorm_kernel<1>, dim3(B), dim3(256), 0, (cudaStream_t)st, tokens,
+                      (const __nv_bfloat16*)embed, (const __nv_bfloat16*)gamma, eps, (int)H, (int)vocab, h, (__nv_bfloat16*)x_bf16));
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -461,6 +560,13 @@ extern "C" int prl_residual_rmsnorm(const float* partials, int32_t n_split, int3
   PRL_CHECK_ARG(partials && gamma && h && x_bf16 && B >= 1 && H >= 4 && n_split >= 0, "prl_residual_rmsnorm: bad argument");
   PRL_CHECK_ARG(H % 4 == 0, "prl_residual_rmsnorm: hidden size must be a multiple of 4 (got %d)", H);
   PRL_CHECK_ARG(H * 4 <= 96 * 1024, "prl_residual_rmsnorm: hidden size too large for the row buffer");
+  if (B > 128 && H <= 4 * 4 * 1024 && !l2_prefetch) {   // a prompt chunk; a token step's rows (up to 128) want one row's latency short
+    const int per_row = ((H / 4 + 3) / 4 + 31) / 32 * 32;
+    PRL_CUDA(launch_pdl(residual_rmsnorm_rows_kernel<4>, dim3(B), dim3(per_row), 0, (cudaStream_t)st, partials, (int)n_split, (int)B,
+                        (int)H, (const __nv_bfloat16*)gamma, eps, h, (__nv_bfloat16*)x_bf16));
+    PRL_LAUNCH_CHECK();
+    return PRL_OK;
+  }
   static SmemAttr smem_attr = {};
   PRL_CUDA(ensure_smem(residual_rmsnorm_kernel, 96 * 1024, smem_attr));
   int threads = ((H / 4 + 31) / 32) * 32;
@@ -484,7 +590,9 @@ extern "C" int prl_qkv_rope_cache(const float* partials, int32_t n_split, int32_
   PRL_CHECK_ARG(B >= 1 && n_q >= 1 && n_kv >= 1 && page_size >= 1 && max_blocks >= 1, "prl_qkv_rope_cache: bad shape");
   if (B > 128) {  // prefill chunk: row-walking variant (same results, ~4x less time at 1024 rows)
     const unsigned blocks = (unsigned)(B < 148 * 8 ? B : 148 * 8);
-    PRL_CUDA(launch_pdl(qkv_rope_cache_rows_kernel, dim3(blocks), dim3(256), 0, (cudaStream_t)st, partials, (int)n_split,
+    const bool vec = ((uintptr_t)partials & 15) == 0 && (((uintptr_t)bias | (uintptr_t)q_out | (uintptr_t)kv_cache) & 7) == 0;
+    PRL_CUDA(launch_pdl(vec ? qkv_rope_cache_rows_kernel<4> : qkv_rope_cache_rows_kernel<1>, dim3(blocks), dim3(vec ? 192 : 256), 0,
+                        (cudaStream_t)st, partials, (int)n_split,
                         (int)B, (const __nv_bfloat16*)bias, (int)n_q, (int)n_kv, positions, block_table, (int)max_blocks,
                         row_slot, inv_freq, (__nv_bfloat16*)q_out, (__nv_bfloat16*)kv_cache, n_pages, (int)layer,
                         (int)page_size));

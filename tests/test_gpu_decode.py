@@ -421,3 +421,54 @@ def test_token_step_with_and_without_the_swiglu_epilogue_is_bit_identical(cuda_d
         logits[fuse] = torch.stack(rows)
         del eng
     assert torch.equal(logits[True], logits[False])
+
+
+@pytest.mark.parametrize("B,H,n_split", [(129, 4, 1), (130, 1036, 2), (300, 3584, 0), (200, 4100, 1), (129, 16384, 1), (140, 16388, 1)])
+def test_residual_norm_of_many_rows(cuda_device, B, H, n_split):
+    """Prompt chunks (more than 128 rows): widths around a thread's four pieces and the widest block.  One bf16 rounding, and an
+    fp32 sum of H squares within H * 2^-24."""
+    from pipelinerl_b200 import _lib
+    lib, g = _lib.load(), torch.Generator().manual_seed(B + H)
+    h = torch.randn(B, H, generator=g).to(cuda_device)
+    part = torch.randn(max(n_split, 1), B, H, generator=g).to(cuda_device)
+    gamma = (1 + 0.1 * torch.randn(H, generator=g)).to(torch.bfloat16).to(cuda_device)
+    x = torch.empty(B, H, dtype=torch.bfloat16, device=cuda_device)
+    want_h = h.clone()
+    for s in range(n_split):
+        want_h += part[s]
+    _lib.check(lib.prl_residual_rmsnorm(part.data_ptr(), n_split, B, H, gamma.data_ptr(), 1e-6, h.data_ptr(), x.data_ptr(), None, 0,
+                                        _lib.stream_ptr()))
+    assert torch.equal(h, want_h)
+    d = want_h.double()
+    want = d * torch.rsqrt((d * d).mean(-1, keepdim=True) + 1e-6) * gamma.double()
+    assert ((x.double() - want).abs() <= (2.0 ** -8 + H * 2.0 ** -24) * want.abs() + 1e-30).all()
+
+
+@pytest.mark.parametrize("B,n_q,n_kv,n_split", [(129, 1, 1, 1), (257, 7, 1, 1), (1300, 28, 4, 1), (140, 5, 5, 3)])
+def test_rope_rows_on_aligned_and_unaligned_buffers(cuda_device, B, n_q, n_kv, n_split):
+    """The four-pair form and the pair-by-pair form (queries and cache two bytes off) write the same bits."""
+    from pipelinerl_b200 import _lib
+    lib, g = _lib.load(), torch.Generator().manual_seed(B)
+    heads, pages = n_q + 2 * n_kv, (B + 63) // 64 + 1
+    part = torch.randn(n_split, B, heads * 128, generator=g).to(cuda_device)
+    bias = torch.randn(heads * 128, generator=g).to(torch.bfloat16).to(cuda_device)
+    pos = torch.arange(B, dtype=torch.int32, device=cuda_device)
+    slot = torch.zeros(B, dtype=torch.int32, device=cuda_device)
+    table = torch.arange(1, pages, dtype=torch.int32, device=cuda_device)[None].contiguous()
+    inv = (1.0 / (1e6 ** (torch.arange(0, 128, 2).float() / 128))).to(cuda_device)
+    got = []
+    for off in (0, 1):
+        q = torch.zeros(B * n_q * 128 + 1, dtype=torch.bfloat16, device=cuda_device)[off:]
+        kv = torch.zeros(2 * pages * n_kv * 64 * 128 + 1, dtype=torch.bfloat16, device=cuda_device)[off:]
+        _lib.check(lib.prl_qkv_rope_cache(part.data_ptr(), n_split, B, bias.data_ptr(), n_q, n_kv, 128, pos.data_ptr(), table.data_ptr(),
+                                          pages - 1, slot.data_ptr(), inv.data_ptr(), q.data_ptr(), kv.data_ptr(), pages, 0, 64, None, 0,
+                                          _lib.stream_ptr()))
+        got.append((q[:B * n_q * 128].clone(), kv[:2 * pages * n_kv * 64 * 128].clone()))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    x = (part.sum(0) + bias.float()).view(B, heads, 128).double()
+    a = pos.double()[:, None] * inv.double()
+    c, s = torch.cos(a)[:, None], torch.sin(a)[:, None]
+    want = torch.cat([x[..., :64] * c - x[..., 64:] * s, x[..., 64:] * c + x[..., :64] * s], -1)[:, :n_q]
+    # the angle is an fp32 product: position * 2^-24 off at most
+    assert (got[0][0].view(B, n_q, 128).double() - want).abs().max().item() <= (2.0 ** -8 + B * 2.0 ** -23) * x.abs().max().item()
+    assert got[0][1].abs().sum() > 0
