@@ -13,9 +13,10 @@
 //     mma.sync m16n8k16 (the work is ~7 FLOP per KV byte, far below any tensor roof:
 //     tensor cores are used for issue efficiency, not throughput), online softmax in
 //     fp32 (exp2 domain), ldmatrix with the matching XOR swizzle (conflict-free);
-//   * per-split (m, l, O) partials are merged either by a small combine kernel (default) or by whichever split
-//     CTA of the (sequence, kv head) finishes last (arrival ticket; prl_attn_set_fused_combine) — A/B measured in
-//     profiles/r1_ablation*.jsonl.
+//   * a single split (short contexts) writes the output itself; the (m, l, O) partials of several are merged either by a small
+//     combine kernel (default) or by whichever split CTA of the (sequence, kv head) finishes last (arrival ticket;
+//     prl_attn_set_fused_combine), A/B measured in profiles/r1_ablation*.jsonl.  Splits as one cluster that merges through its
+//     shared memory were slower where it counts (64 x 8192: 1498 -> 1515 us a step of four layers).
 // KV cache layout (bf16): row = (((layer*2 + kv) * n_pages + page) * n_kv + kvh) * 64 + slot,
 // 128 contiguous d per row — written by qkv_rope_cache_kernel (decode_ops.cu).
 #include "prl_common.cuh"
@@ -45,6 +46,7 @@ struct AttnParams {
   float* ml_part;              // [B, n_q, n_splits, 2]
   unsigned int* tickets;       // [B, n_kv] arrival counters (zero on entry, self-resetting); NULL = separate combine kernel
   __nv_bfloat16* out;          // [B, n_q*128]
+  int direct;                  // one split: the output is written here, no partials
 };
 
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
@@ -93,6 +95,19 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p
   const int n_it = p_end > p_begin ? p_end - p_begin : 0;
   const int R = p.R;
 
+  auto store = [&](int r, int d, float O, float M, float L) {
+    const int64_t head = (int64_t)b * p.n_q + kvh * R + r;
+    if (p.direct) {
+      p.out[head * kD + d] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
+    } else {
+      p.o_part[(head * p.n_splits + split) * kD + d] = O;
+      if (d == 0) {
+        p.ml_part[(head * p.n_splits + split) * 2 + 0] = M;
+        p.ml_part[(head * p.n_splits + split) * 2 + 1] = L;
+      }
+    }
+  };
+
   // last-arriving split of a (sequence, kv head) merges all splits and writes the bf16 output: no combine launch
   auto finish = [&]() {
     if (p.tickets == nullptr) return;   // the stand-alone combine kernel merges the splits
@@ -121,15 +136,7 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p
   };
 
   if (n_it == 0) {  // empty split (short sequence): neutral partial
-    for (int i = threadIdx.x; i < R * kD; i += kThreads) {
-      const int r = i / kD, d = i % kD;
-      const int64_t head = (int64_t)b * p.n_q + kvh * R + r;
-      p.o_part[(head * p.n_splits + split) * kD + d] = 0.f;
-      if (d == 0) {
-        p.ml_part[(head * p.n_splits + split) * 2 + 0] = -INFINITY;
-        p.ml_part[(head * p.n_splits + split) * 2 + 1] = 0.f;
-      }
-    }
+    for (int i = threadIdx.x; i < R * kD; i += kThreads) store(i / kD, i % kD, 0.f, -INFINITY, 0.f);
     finish();
     return;
   }
@@ -293,12 +300,7 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p
       L += s_ml[(w * 16 + r) * 2 + 1] * f;
       O += s_o[(w * 16 + r) * kD + d] * f;
     }
-    const int64_t head = (int64_t)b * p.n_q + kvh * R + r;
-    p.o_part[(head * p.n_splits + split) * kD + d] = O;
-    if (d == 0) {
-      p.ml_part[(head * p.n_splits + split) * 2 + 0] = M;
-      p.ml_part[(head * p.n_splits + split) * 2 + 1] = L;
-    }
+    store(r, d, O, M, L);
   }
   finish();
 }
@@ -575,6 +577,8 @@ extern "C" int prl_paged_attn_decode(const void* q, const void* kv_cache, int64_
   p.ml_part = p.o_part + (size_t)B * n_q * n_splits * kD;
   p.tickets = g_fused_combine ? reinterpret_cast<unsigned int*>(p.ml_part + (size_t)B * n_q * n_splits * 2) : nullptr;
   p.out = (__nv_bfloat16*)out_bf16;
+  p.direct = n_splits == 1;    // 4 x 333 keys, eight layers: one launch of nine a layer less, 285 -> 274 us a step
+  if (p.direct) p.tickets = nullptr;
   const int smem = kStages * kStageBytes + 1024 + 8 * 2 * kStages + 4 * kMaxPagesPerSplit + 16;
   static SmemAttr smem_attr = {};
   PRL_CUDA(ensure_smem(paged_attn_decode_kernel, smem, smem_attr));
@@ -582,7 +586,7 @@ extern "C" int prl_paged_attn_decode(const void* q, const void* kv_cache, int64_
   dim3 grid((unsigned)n_splits, (unsigned)n_kv, (unsigned)B);
   PRL_CUDA(launch_pdl(paged_attn_decode_kernel, grid, dim3(kThreads), (size_t)smem, stream, tm, p));
   PRL_LAUNCH_CHECK();
-  if (!g_fused_combine) {
+  if (!g_fused_combine && !p.direct) {
     PRL_CUDA(launch_pdl(attn_combine_kernel, dim3((unsigned)(B * n_q)), dim3(kD), 0, stream, (const float*)p.o_part,
                         (const float*)p.ml_part, (int)n_splits, (__nv_bfloat16*)out_bf16));
     PRL_LAUNCH_CHECK();

@@ -472,3 +472,27 @@ def test_rope_rows_on_aligned_and_unaligned_buffers(cuda_device, B, n_q, n_kv, n
     # the angle is an fp32 product: position * 2^-24 off at most
     assert (got[0][0].view(B, n_q, 128).double() - want).abs().max().item() <= (2.0 ** -8 + B * 2.0 ** -23) * x.abs().max().item()
     assert got[0][1].abs().sum() > 0
+
+
+@pytest.mark.parametrize("R,n_kv", [(1, 3), (7, 4), (16, 1)])
+def test_attention_of_one_split_writes_the_output(cuda_device, R, n_kv):
+    """One split, no merge launch: empty sequences (zeros), page edges, stale contents of the output and the workspace.  Probabilities
+    are rounded to bf16 for the product with V and the output once more (2^-9 each), and fp32 sums take the rest of 2^-7."""
+    from pipelinerl_b200 import _lib
+    lib, g = _lib.load(), torch.Generator().manual_seed(R)
+    lens, P, D = [0, 1, 63, 64, 65, 200, 0], 64, 128
+    B, mb = len(lens), 4
+    kv = torch.randn(1, 2, B * mb + 1, n_kv, P, D, generator=g).to(torch.bfloat16).to(cuda_device)
+    bt = (torch.randperm(B * mb, generator=g).int() + 1).view(B, mb).to(cuda_device)
+    q = torch.randn(B, n_kv * R, D, generator=g).to(torch.bfloat16).to(cuda_device)
+    sl = torch.tensor(lens, dtype=torch.int32, device=cuda_device)
+    out = torch.full((B, n_kv, R, D), float("nan"), dtype=torch.bfloat16, device=cuda_device)
+    n = int(lib.prl_paged_attn_workspace_bytes(B, n_kv * R, 1))
+    ws = torch.full((n,), 255, dtype=torch.uint8, device=cuda_device)
+    _lib.check(lib.prl_paged_attn_decode(q.data_ptr(), kv.data_ptr(), B * mb + 1, 1, 0, bt.data_ptr(), mb, sl.data_ptr(), B, n_kv * R,
+                                         n_kv, D, P, 1, D ** -0.5, out.data_ptr(), ws.data_ptr(), n, _lib.stream_ptr()))
+    for b, l in enumerate(lens):
+        K, V = (kv[0, i, bt[b].long()].transpose(0, 1).reshape(n_kv, mb * P, D)[:, :l].double() for i in (0, 1))
+        w = torch.softmax(torch.einsum("grd,gsd->grs", q[b].view(n_kv, R, D).double(), K) * D ** -0.5, -1)
+        want, bound = torch.einsum("grs,gsd->grd", w, V), torch.einsum("grs,gsd->grd", w, V.abs())
+        assert ((out[b].double() - want).abs() <= 2.0 ** -7 * bound + 1e-30).all(), l
