@@ -526,6 +526,14 @@ class EngineCore:
         self.free_slots.append(req.slot)
 
 
+def swiglu_epilogue_pays(I: int, H: int, split_k: int, sms: int) -> bool:
+    """Whether a token step's gate_up takes the gated epilogue, which cannot split K, over the split pair: where there is no
+    split anyway, or where the SMs that its I / 64 tiles leave idle cost less than 5 k-blocks of a full wave (0.37 us each), which
+    is about what the second launch and the fp32 partials cost.  2048 wide, I 8192 (128 tiles of 148): a step of four layers
+    251 -> 234 us at 4 sequences, 649 -> 613 at 64; 1024 wide, I 4096 (64 tiles, 9 k-blocks): 273 -> 290 with the epilogue."""
+    return split_k == 1 or (I // 64 < sms and -(-H // 64) * (sms - I // 64) <= 5 * sms)
+
+
 class DecodeEngine(EngineCore):
     """The Qwen2-family program on the engine core: GQA attention with head size 128 over one bf16 KV pool, pre-norm
     blocks, SwiGLU; tcgen05 GEMMs with split-K partials consumed by fused epilogue kernels, the paged-attention decode
@@ -612,6 +620,9 @@ class DecodeEngine(EngineCore):
                   "down": (cfg.hidden_size, cfg.intermediate_size), "head": (cfg.head_rows, cfg.hidden_size)}
         self.split_k = {k: int(self.lib.prl_gemm_auto_split_k(B, n, kk)) for k, (n, kk) in shapes.items()}
         self.split_k["head"] = 1  # the sampler reads plain logits
+        self.swiglu_epilogue = (cfg.intermediate_size % 64 == 0 and B <= 128 and swiglu_epilogue_pays(
+            cfg.intermediate_size, cfg.hidden_size, self.split_k["gate_up"],
+            torch.cuda.get_device_properties(self.dev).multi_processor_count))
         need = max(self.split_k[k] * B * shapes[k][0] for k in ("qkv", "o", "gate_up", "down"))
         self.partials = torch.zeros(need, dtype=torch.float32, device=self.dev)
 
@@ -631,7 +642,7 @@ class DecodeEngine(EngineCore):
         part = self.partials
         skip = self._skip
         pf = self.l2_prefetch_bytes  # cross-kernel L2 prefetch budget per site (0 disables)
-        fuse_swiglu = (self.fuse_swiglu and not skip and not pf and self.split_k["gate_up"] == 1 and I % 64 == 0 and B <= 128)
+        fuse_swiglu = self.fuse_swiglu and not skip and not pf and self.swiglu_epilogue
 
         def wbytes(name):  # whole weight tensor, capped by the budget
             shape = a.layout.shapes[name]
@@ -671,8 +682,8 @@ class DecodeEngine(EngineCore):
                                                     wbytes(p + "down_proj.weight"), st))
             nxt_qkv = f"layers.{l + 1}.qkv_proj.weight" if l + 1 < cfg.num_layers else None
             if fuse_swiglu:
-                # SiLU(gate) * up in the gate_up GEMM's epilogue (no split-K here: 2 I / 128 tiles fill the SMs): one launch
-                # less per layer and no [B, 2 I] fp32 tile between the two; same bits as the pair below
+                # SiLU(gate) * up in the gate_up GEMM's epilogue: one launch less per layer and no [B, 2 I] fp32 tiles between
+                # the two; same bits as the pair below without a split
                 _lib.check(lib.prl_gemm_swiglu_decode(a.ptr(p + "gate_up_proj.weight"), self.x.data_ptr(), B, I, H,
                                                       self.act.data_ptr(), st))
             else:
