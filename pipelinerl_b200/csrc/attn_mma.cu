@@ -244,12 +244,10 @@ int launch_mma(const void* q, const void* kp, const void* vp, const int32_t* bt,
 
 // ---- single-token segments (a decode step) ------------------------------------------------------------------------------
 // The query heads that share a key / value head are the rows of one 16-row product (up to 16 per CTA), so a key is read once
-// for all of them.  CTA = 8 warps of one (segment, key / value head, group of 16 heads); the warps take the visible key tiles
-// (16 keys at absolute multiples of 16: the kept first tokens, then the window) in turn, each through a pipeline of its own
-// (two buffers filled by cp.async, no barrier between the warps), and their partial softmaxes are merged in warp order.  A warp's
-// tile is a serial chain (copy, scores, softmax, output), so twice the warps on half the keys each hide more of it in the same
-// shared memory: 4 warps x 32 keys 24.3 us, 8 x 16 20.5 (32 sequences x 1024 keys, 4 heads); 3 x 300: 11.4 and 9.4.
-constexpr int kDecWarps = 8, kDecKeys = 16, kDecHeads = 16;
+// for all of them.  CTA = 4 warps of one (segment, key / value head, group of 16 heads); the warps take the visible key tiles
+// (32 keys at absolute multiples of 32: the kept first tokens, then the window) in turn, each through a pipeline of its own
+// (two buffers filled by cp.async, no barrier between the warps), and their partial softmaxes are merged in warp order.
+constexpr int kDecWarps = 4, kDecKeys = 32, kDecHeads = 16;
 
 template <int DV, bool OUT_BF16>
 __global__ void __launch_bounds__(kDecWarps * 32) attn_mma_decode_kernel(
