@@ -491,18 +491,19 @@ __global__ void __launch_bounds__(256) moe_gemm_kernel(const TA* __restrict__ A,
 }
 
 // ---- bf16 tensor-core variant ------------------------------------------------------------------------------------------
-// A token step's experts are a weight stream (16 experts x 2048 x 2048: 134 MB of weights for 128 token rows).  A warp owns 16
-// weight rows and reads them straight into the A fragments of m16n8k16, 16 bytes a lane: the k order inside a block of 32 is the
-// lanes' (lane t of four holds k = 8 t .. 8 t + 7), and the token rows, staged in shared memory in chunks of K, are read in the
-// same order.  Two batches of blocks are on their way per warp; shared memory stays at 40 KB because loads in flight need the
-// rest of it as L1 (the same loop beside 110 KB took 52 us).  Weights staged through cp.async with a barrier every 64 of K took
-// 29 us at 8 rows an expert, 41.4 at 64; this takes 22.2 and 40.5; the weights alone at the rate of a copy 20.5.
-constexpr int kBN = 128;                          // weight rows of a CTA: 16 a warp
-constexpr int kRowsSmem = 2 * 64 * (2 * 128 + 64);   // two chunks of 64 rows x 128, of 32 x 256, 16 x 512 or 8 x 1024 (each smaller)
+constexpr int kBN = 128, kBK = 64, kPad = 8;      // tile N, K step, padding (halves) that keeps ldmatrix conflict-free
+constexpr int kLds = kBK + kPad;                  // 72 halves = 144 bytes per staged row
+constexpr int kStages = 4;                        // cp.async stages in flight: a few-row tile is a pure weight stream
+constexpr size_t kMmaSmem = (size_t)kStages * (kTile + kBN) * kLds * sizeof(__nv_bfloat16);
 
 __device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, int bytes) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void* p) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
 }
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -511,126 +512,113 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
 }
 
 template <int ACT>
-__device__ __forceinline__ void expert_store(void* C_v, int64_t at, float z, float w) {
-  if constexpr (ACT != kActNone) reinterpret_cast<__nv_bfloat16*>(C_v)[at] = __float2bfloat16_rn(expert_act<ACT>(z) * w);
-  else reinterpret_cast<float*>(C_v)[at] = z;
-}
-
-__device__ __forceinline__ uint4 ld_stream(const __nv_bfloat16* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  return v;
-}
-
-// Up to 8 * NG token rows against the CTA's 128 weight rows; s0: the tile's first sorted place.
-template <int ACT, int NG>
-__device__ __forceinline__ void moe_rows(const __nv_bfloat16* __restrict__ A, int64_t lda, int a_mod,
-                                         const __nv_bfloat16* __restrict__ We, int64_t ldw, const int32_t* __restrict__ perm, int s0,
-                                         int n0, int N, int K, int M, void* __restrict__ C_v, int64_t ldc, int c_perm,
-                                         const float* __restrict__ wsel, unsigned char* smem, int32_t* a_row) {
-  constexpr int kBatch = NG == 8 ? 2 : 4, kChunk = 1024 / NG, kRow = kChunk * 2 + 64;   // + 64: two rows fill the 32 banks
-  constexpr int kBuf = 8 * NG * kRow;
-  static_assert(2 * kBuf <= kRowsSmem && kChunk % (64 * kBatch) == 0, "two chunks of token rows, pairs of batches");
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int n1 = n0 + warp * 16 + g, n2 = n1 + 8;
-  const __nv_bfloat16* w1 = We + (int64_t)(n1 < N ? n1 : 0) * ldw + 8 * t;
-  const __nv_bfloat16* w2 = We + (int64_t)(n2 < N ? n2 : 0) * ldw + 8 * t;
-  float acc[NG][4];
-#pragma unroll
-  for (int j = 0; j < NG; ++j)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) acc[j][q] = 0.f;
-  uint4 f1[2][kBatch], f2[2][kBatch];
-  auto load = [&](int b, int k0) {
-    if (k0 + 32 * kBatch <= K) {                 // uniform
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u) { f1[b][u] = ld_stream(w1 + k0 + 32 * u); f2[b][u] = ld_stream(w2 + k0 + 32 * u); }
-    } else {
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u) {
-        const bool ok = k0 + 32 * u + 8 * t < K; // K % 8 == 0
-        f1[b][u] = ok ? ld_stream(w1 + k0 + 32 * u) : make_uint4(0, 0, 0, 0);
-        f2[b][u] = ok ? ld_stream(w2 + k0 + 32 * u) : make_uint4(0, 0, 0, 0);
-      }
-    }
-  };
-  auto multiply = [&](int b, const unsigned char* x) {
-#pragma unroll
-    for (int u = 0; u < kBatch; ++u) {
-      const uint32_t lo[4] = {f1[b][u].x, f2[b][u].x, f1[b][u].y, f2[b][u].y};
-      const uint32_t hi[4] = {f1[b][u].z, f2[b][u].z, f1[b][u].w, f2[b][u].w};
-#pragma unroll
-      for (int j = 0; j < NG; ++j) {
-        const uint4 v = *reinterpret_cast<const uint4*>(x + j * 8 * kRow + 64 * u);
-        mma_bf16(acc[j], lo, v.x, v.y);
-        mma_bf16(acc[j], hi, v.z, v.w);
-      }
-    }
-  };
-  load(0, 0);
-  load(1, 32 * kBatch);
-  if (tid < M) a_row[tid] = a_mod > 0 ? perm[s0 + tid] % a_mod : s0 + tid;
-  __syncthreads();
-  auto stage = [&](int c0) {                     // token rows c0 .. c0 + kChunk, zeros past K and M
-    unsigned char* dst = smem + ((c0 / kChunk) & 1) * kBuf;
-    for (int i = tid; i < 8 * NG * (kChunk / 8); i += 256) {
-      const int r = i / (kChunk / 8), k = (i % (kChunk / 8)) * 8;
-      const bool ok = c0 + k < K && r < M;
-      cp_async16_zfill(dst + r * kRow + k * 2, A + (ok ? (int64_t)a_row[r] * lda + c0 + k : 0), ok ? 16 : 0);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  stage(0);
-  for (int c0 = 0; c0 < K; c0 += kChunk) {
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();                             // chunk c0 has landed for every thread, and every warp is done with the other one
-    if (c0 + kChunk < K) stage(c0 + kChunk);
-    const unsigned char* x = smem + ((c0 / kChunk) & 1) * kBuf + g * kRow + 16 * t;
-    const int len = min(kChunk, K - c0);
-    for (int k = 0; k < len; k += 64 * kBatch) {   // past K: zeros on both sides
-      multiply(0, x + 2 * k);
-      load(0, c0 + k + 64 * kBatch);
-      multiply(1, x + 2 * (k + 32 * kBatch));
-      load(1, c0 + k + 96 * kBatch);
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < NG; ++j)
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int m = 8 * j + 2 * t + half;
-      if (m >= M) continue;
-      const int p = (c_perm || ACT != kActNone) ? perm[s0 + m] : 0;
-      const int64_t at = (int64_t)(c_perm ? p : s0 + m) * ldc;
-      const float w = ACT != kActNone ? wsel[p] : 1.f;
-      if (n1 < N) expert_store<ACT>(C_v, at + n1, acc[j][half], w);
-      if (n2 < N) expert_store<ACT>(C_v, at + n2, acc[j][2 + half], w);
-    }
-}
-
-template <int ACT>
-__global__ void __launch_bounds__(256, 2) moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, int a_mod,
-                                                              const __nv_bfloat16* __restrict__ W, int64_t expert_stride,
-                                                              int64_t ldw, const int32_t* __restrict__ perm,
-                                                              const int32_t* __restrict__ meta, const int32_t* __restrict__ tiles,
-                                                              int N, int K, void* __restrict__ C_v, int64_t ldc, int c_perm,
-                                                              const float* __restrict__ wsel) {
+__global__ void __launch_bounds__(256) moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, int a_mod,
+                                                           const __nv_bfloat16* __restrict__ W, int64_t expert_stride,
+                                                           int64_t ldw, const int32_t* __restrict__ perm,
+                                                           const int32_t* __restrict__ meta, const int32_t* __restrict__ tiles,
+                                                           int N, int K, void* __restrict__ C_v, int64_t ldc, int c_perm,
+                                                           const float* __restrict__ wsel) {
   pdl_wait();
   const int tile = blockIdx.y;
   if (tile >= meta[0]) return;
+  extern __shared__ __align__(16) unsigned char mma_smem[];
+  typedef __nv_bfloat16 (*ATile)[kTile][kLds];
+  typedef __nv_bfloat16 (*BTile)[kBN][kLds];
+  ATile As = reinterpret_cast<ATile>(mma_smem);                                           // [kStages][64][72]
+  BTile Bs = reinterpret_cast<BTile>(mma_smem + (size_t)kStages * kTile * kLds * sizeof(__nv_bfloat16));   // [kStages][128][72]
+  __shared__ int32_t a_row[kTile], c_row[kTile];
+  __shared__ float c_w[kTile];
   const int e = tiles[3 * tile], s0 = tiles[3 * tile + 1], M = tiles[3 * tile + 2];
-  extern __shared__ __align__(16) unsigned char rows_smem[];
-  __shared__ int32_t a_row[kTile];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid < kTile) {
+    const int s = s0 + min(tid, M - 1);
+    const int p = perm[s];
+    if constexpr (ACT != kActNone) c_w[tid] = wsel[p];
+    a_row[tid] = a_mod > 0 ? p % a_mod : s;
+    c_row[tid] = c_perm ? p : s;
+  }
+  __syncthreads();
   const __nv_bfloat16* We = W + (int64_t)e * expert_stride;
   const int n0 = blockIdx.x * kBN;
-#define PRL_ROWS(NG) moe_rows<ACT, NG>(A, lda, a_mod, We, ldw, perm, s0, n0, N, K, M, C_v, ldc, c_perm, wsel, rows_smem, a_row)
-  if (M <= 8) PRL_ROWS(1);
-  else if (M <= 16) PRL_ROWS(2);
-  else if (M <= 32) PRL_ROWS(4);
-  else PRL_ROWS(8);
-#undef PRL_ROWS
+  const int wm = (warp >> 2) * 32, wn = (warp & 3) * 32;       // warp tile 32 x 32
+  float acc[2][4][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.f;
+  // loaders: A 64 rows x 8 chunks of 8 halves (two per thread), B 128 rows x 8 chunks (four per thread)
+  const int lr = tid >> 3, lc = (tid & 7) * 8;
+  const int64_t a_off[2] = {(int64_t)a_row[lr] * lda, (int64_t)a_row[lr + 32] * lda};
+  auto stage = [&](int k0, int buf) {
+    const int k = k0 + lc;
+    const bool kin = k < K;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (32 * h < M)         // uniform: the upper half of a short tile is not staged, and the warps that own it do nothing
+        cp_async16_zfill(&As[buf][lr + 32 * h][lc], A + a_off[h] + (kin ? k : 0), (kin && lr + 32 * h < M) ? 16 : 0);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const int r = lr + 32 * h, nn = n0 + r;
+      const bool ok = kin && nn < N;
+      cp_async16_zfill(&Bs[buf][r][lc], We + (int64_t)(ok ? nn : 0) * ldw + (kin ? k : 0), ok ? 16 : 0);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // kStages - 1 steps in flight; a commit per step keeps the group count regular (empty past the end, where `stage`
+  // copies nothing but zero fill into a buffer nobody reads)
+#pragma unroll
+  for (int st = 0; st < kStages - 1; ++st) stage(st * kBK, st);
+  int buf = 0;
+  for (int k0 = 0; k0 < K; k0 += kBK, buf = (buf + 1) % kStages) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+    __syncthreads();            // step k0 has landed for every thread, and every warp is done with the buffer refilled next
+    stage(k0 + (kStages - 1) * kBK, (buf + kStages - 1) % kStages);
+    if (wm < M)                 // warp-uniform
+#pragma unroll
+    for (int kk = 0; kk < kBK; kk += 16) {
+      uint32_t af[2][4], bf[2][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) ldsm_x4(af[i], &As[buf][wm + 16 * i + (lane & 15)][kk + (lane >> 4) * 8]);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) ldsm_x4(bf[j], &Bs[buf][wn + 16 * j + (lane & 7) + ((lane >> 4) << 3)][kk + ((lane >> 3) & 1) * 8]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma_bf16(acc[i][j], af[i], bf[j >> 1][(j & 1) * 2], bf[j >> 1][(j & 1) * 2 + 1]);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int m = wm + 16 * i + (lane >> 2) + 8 * half;
+      if (m >= M) continue;
+      const int64_t at = (int64_t)c_row[m] * ldc;
+      if constexpr (ACT != kActNone) {
+        __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(C_v) + at;
+        const float w = c_w[m];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int nn = n0 + wn + 8 * j + (lane & 3) * 2;
+          if (nn < N) crow[nn] = __float2bfloat16_rn(expert_act<ACT>(acc[i][j][2 * half]) * w);
+          if (nn + 1 < N) crow[nn + 1] = __float2bfloat16_rn(expert_act<ACT>(acc[i][j][2 * half + 1]) * w);
+        }
+        continue;
+      }
+      float* crow = reinterpret_cast<float*>(C_v) + at;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int nn = n0 + wn + 8 * j + (lane & 3) * 2;
+        if (nn < N) crow[nn] = acc[i][j][2 * half];
+        if (nn + 1 < N) crow[nn + 1] = acc[i][j][2 * half + 1];
+      }
+    }
 }
 
+// act[s] = g * sigmoid(beta g) * (u + 1),  g = min(w * gate, lim), u = clamp(w * up, -lim, lim),  w = wsel[perm[s]]
 template <typename T>
 __global__ void moe_glu_kernel(const float* __restrict__ gu, int64_t ld, int F, const int32_t* __restrict__ perm,
                                const float* __restrict__ wsel, float lim, float beta, T* __restrict__ out) {
@@ -790,8 +778,8 @@ static int moe_gemm_impl(const void* A, int32_t a_is_f32, int64_t lda, int32_t a
       ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0) {
     dim3 grid_tc((unsigned)((N + kBN - 1) / kBN), (unsigned)max_tiles);
     static SmemAttr attr = {};
-    PRL_CUDA(ensure_smem(moe_gemm_mma_kernel<ACT>, kRowsSmem, attr));
-    PRL_CUDA(launch_pdl(moe_gemm_mma_kernel<ACT>, grid_tc, dim3(256), (size_t)kRowsSmem, s, (const bf16*)A, lda, a_mod, (const bf16*)W,
+    PRL_CUDA(ensure_smem(moe_gemm_mma_kernel<ACT>, (int)kMmaSmem, attr));
+    PRL_CUDA(launch_pdl(moe_gemm_mma_kernel<ACT>, grid_tc, dim3(256), kMmaSmem, s, (const bf16*)A, lda, a_mod, (const bf16*)W,
                         expert_stride, ldw, perm, meta, tiles, (int)N, (int)K, C, ldc, c_perm, wsel));
     PRL_LAUNCH_CHECK();
     return PRL_OK;

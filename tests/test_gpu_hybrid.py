@@ -387,39 +387,3 @@ def test_rollouts_through_the_plugin_interface(cuda_device):
                 assert abs(lp - ref[n_prompt - 1 + k, ids[n_prompt + k]].item()) < 2e-3
                 checked += 1
     assert checked >= 9
-
-
-@pytest.mark.parametrize("N,K,act", [(130, 8, 0), (256, 72, 1), (100, 1032, 0), (129, 2056, 1), (128, 4104, 0), (40, 8200, 0)])
-def test_grouped_products_of_few_rows(cuda_device, N, K, act):
-    """One tile per number of rows around the 8 / 16 / 32 row forms and the full tile, K around a batch, a chunk and its end, N off
-    the tile: fp32 sums of K exact products, within K * 2^-24 of the sum of their sizes; bf16 outputs round once more."""
-    from pipelinerl_b200 import _lib
-    lib, g, st = _lib.load(), torch.Generator().manual_seed(N + K), _lib.stream_ptr()
-    rows = [1, 8, 9, 16, 17, 32, 33, 64]
-    pairs, E = sum(rows), len(rows)
-    i32 = dict(dtype=torch.int32, device=cuda_device)
-    A = torch.randn(pairs, K, generator=g).to(torch.bfloat16).to(cuda_device)
-    W = torch.randn(E, N, K, generator=g).to(torch.bfloat16).to(cuda_device)
-    perm = torch.randperm(pairs, generator=g).int()
-    wsel = torch.rand(pairs, generator=g).to(cuda_device)
-    starts = [sum(rows[:e]) for e in range(E)]
-    tiles = torch.tensor([(e, starts[e], rows[e]) for e in range(E)], **i32)
-    meta, perm_d = torch.tensor([E, pairs, 0, 0], **i32), perm.to(cuda_device)
-    out = torch.full((pairs, N), float("nan"), device=cuda_device, dtype=torch.bfloat16 if act else torch.float32)
-    table = (perm_d.data_ptr(), meta.data_ptr(), tiles.data_ptr(), E + 2)
-    a = (A.data_ptr(), 0, K, 0 if not act else pairs, W.data_ptr(), 0, N * K, K, *table, N, K)
-    if act:
-        _lib.check(lib.prl_moe_gemm_act(*a, act, wsel.data_ptr(), out.data_ptr(), N, st))
-    else:
-        _lib.check(lib.prl_moe_gemm(*a, out.data_ptr(), N, 1, st))
-    for e, (s0, m) in enumerate(zip(starts, rows)):
-        p = perm_d[s0:s0 + m].long()
-        x, w = (A[p] if act else A[s0:s0 + m]).double(), W[e].double()
-        z, bound = x @ w.t(), (x.abs() @ w.abs().t()) * K * 2.0 ** -24
-        if act:
-            c = wsel[p].double()[:, None]
-            want, tol = z.clamp(min=0) ** 2 * c, (2 * z.abs() + bound) * bound * c
-            got, tol = out[s0:s0 + m].double(), tol + 2.0 ** -8 * want + 1e-30
-        else:
-            want, got, tol = z, out[p].double(), bound
-        assert ((got - want).abs() <= tol).all(), (m, (got - want).abs().max())
