@@ -39,7 +39,7 @@ int prl_version(void);
 /* Number of kernel launches issued by this library since load (bench.py's gpu_launches). */
 uint64_t prl_launch_count(void);
 /* Tuning switches (A/B measurements): programmatic dependent launch on the token-step kernels (default on,
- * env PRL_PDL=0 disables) and in-kernel merge of the attention context splits (default off). */
+ * env PRL_PDL=0 disables) and in-kernel merge of the attention context splits (default off; a single split is written without a merge). */
 int prl_set_pdl(int32_t on);
 int prl_attn_set_fused_combine(int32_t on);
 
@@ -298,7 +298,7 @@ int prl_gemm_set_cta_pair(int32_t on);
  *     C[M,N] (=|+=) alpha * A[M,K] * B[N,K]^T (+ bias[N]) (+ residual[M,N])
  * A, B bf16 row-major with row strides lda / ldb (elements, multiples of 8, base 16-byte aligned); C bf16 or fp32
  * (c_is_f32), `accumulate` (fp32 only) adds into C; bias / residual bf16 or NULL.  Persistent CTA-pair kernel
- * (tcgen05.mma.cta_group::2, 256x256 tiles, double-buffered TMEM accumulators). */
+ * (tcgen05.mma.cta_group::2, tiles of 256 rows and 64 to 256 columns, double-buffered TMEM accumulators). */
 int prl_gemm_tn(const void* A, int64_t lda, const void* B, int64_t ldb, int64_t M, int64_t N, int64_t K,
                 void* C, int64_t ldc, int32_t c_is_f32, int32_t accumulate, const void* bias,
                 const void* residual, int64_t ldr, float alpha, prl_stream_t stream);
