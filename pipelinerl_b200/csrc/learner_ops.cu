@@ -58,8 +58,8 @@ __device__ __forceinline__ float block_sum(float v, float* s_red) {
 
 // The row kernels are bound by HBM.  A block walks its rows with the next row already asked for (registers, raw bf16) while the
 // current one goes through its block sum: without that the reads stop at every row's barrier (16384 x 3584: backward 170 us,
-// 0.42 of the copy rate).  The block has just the threads that a row fills (448 pieces of 16 bytes: 224 threads, two each), and
-// the grid just the blocks that are resident at once.  With the faster column sums below: 16384 x 3584 forward 49 -> 47 us, backward
+// 0.42 of the copy rate).  A narrow row's block has just the threads that it fills (row_threads), and the grid
+// just the blocks that are resident at once.  With the faster column sums below: 16384 x 3584 forward 49 -> 47 us, backward
 // 214 -> 87 us (5.4 TB/s, cold L2); 4096 x 5120 27 -> 21, 150 -> 44; 16384 x 1024 25 -> 21, 79 -> 38.
 template <int kVec>
 __device__ __forceinline__ void load_row(const __nv_bfloat16* __restrict__ p, int64_t row, int H, uint4 (&r)[kVec]) {
@@ -167,10 +167,11 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
         const Vec8 xv = unpack8(xr[i]), dv = unpack8(dr[i]), gv = unpack8(g[i]), sv = unpack8(sr[i]);
         Vec8 o;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o.v[e] = r * (dv.v[e] * gv.v[e] - xv.v[e] * r * m);
+        for (int e = 0; e < 8; ++e)    // contracted by hand, so that the bits don't hang on how the loop is compiled
+          o.v[e] = __fmul_rn(r, fmaf(-(xv.v[e] * r), m, dv.v[e] * gv.v[e]));
         if (dres) {
 #pragma unroll
-          for (int e = 0; e < 8; ++e) o.v[e] += sv.v[e];
+          for (int e = 0; e < 8; ++e) o.v[e] = __fadd_rn(o.v[e], sv.v[e]);
         }
         store8(dx + row * H + v * 8, o);
       }
@@ -347,7 +348,10 @@ dim3 silu_grid(int64_t T, int64_t I) {   // a block per row; few rows are cut, s
 }
 int row_grid(int64_t T) { return (int)(T < kPartialBlocks / 2 ? T : kPartialBlocks / 2); }
 int row_vecs(int64_t H) { return (int)((H / 8 + kRowThreads - 1) / kRowThreads); }                       // 16-byte pieces per thread
-int row_threads(int64_t H) { return (int)(((H / 8 + row_vecs(H) - 1) / row_vecs(H) + 31) / 32 * 32); }   // as many as the pieces need
+// Threads of a row's block: as many as one piece each needs, all of them where a thread holds several.  Thread t then adds pieces
+// t, t + 256, ... whatever the width, so a row's sum has one order.  With 224 threads for 3584 (two pieces each, none idle) the
+// last bit of some rstd moved, and with it single bf16 values of everything behind the norm.
+int row_threads(int64_t H) { return row_vecs(H) > 1 ? kRowThreads : (int)((H / 8 + 31) / 32 * 32); }
 // resident blocks of the backward: two of 256 threads with 128 registers each per SM, or the threads' worth of narrow rows
 int row_bwd_grid(int64_t T, int64_t H) {
   const int per_sm = row_vecs(H) == 1 ? 1024 / row_threads(H) : (row_vecs(H) == 2 ? 2 : 1);

@@ -374,6 +374,30 @@ def test_norm_rows_at_the_edges_of_their_blocks(cuda_device, T, H):
         assert ((dgamma.double() - total).abs() <= (T + 64) * 2.0 ** -23 * (1 + (dd * xh).abs().sum(0))).all()
 
 
+@pytest.mark.parametrize("T,H", [(5, 896), (200, 2048), (333, 2056), (999, 3584), (120, 4104), (64, 8192)])
+def test_norm_rows_add_their_squares_in_one_order(cuda_device, T, H):
+    """Thread t of 256 adds the squares of pieces t, t + 256, ... of 8 channels (exact products of bf16), a warp its lanes by
+    halves, the block its warps in turn: the same bits at every width, so a log-prob behind the norm moves only with its inputs."""
+    from pipelinerl_b200.learner_body import Ops
+    x = torch.randn(T, H, generator=torch.Generator().manual_seed(H)).to(torch.bfloat16).to(cuda_device)
+    pieces = -(-H // 2048)
+    v = torch.zeros(T, pieces * 2048, device=cuda_device)
+    v[:, :H] = x.float() ** 2
+    v = v.view(T, pieces, 256, 8)
+    s = torch.zeros(T, 256, device=cuda_device)
+    for i in range(pieces):
+        for e in range(8):
+            s = s + v[:, i, :, e]
+    s = s.view(T, 8, 32)
+    for o in (16, 8, 4, 2, 1):
+        s = s + s[..., torch.arange(32, device=cuda_device) ^ o]
+    total = torch.zeros(T, device=cuda_device)
+    for w in range(8):
+        total = total + s[:, w, 0]
+    _, rstd = Ops().rmsnorm(x, torch.ones(H, dtype=torch.bfloat16, device=cuda_device), 1e-6)
+    assert torch.equal(rstd, torch.rsqrt(total / torch.full_like(total, H) + 1e-6))    # a number as divisor: torch multiplies by 1 / H
+
+
 @pytest.mark.parametrize("T,I", [(1, 8), (2, 18944), (37, 2056), (700, 24), (1500, 4096)])
 def test_silu_rows_cut_over_blocks(cuda_device, T, I):
     from pipelinerl_b200.learner_body import Ops
