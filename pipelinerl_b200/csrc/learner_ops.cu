@@ -325,6 +325,8 @@ __global__ void __launch_bounds__(256) embed_gather_kernel(const __nv_bfloat16* 
   }
 }
 
+// kVec: four sums per access, on tables that start on 16 bytes (rows of a multiple of 8 numbers keep that); else one by one
+template <bool kVec>
 __global__ void __launch_bounds__(256) embed_scatter_kernel(float* __restrict__ dtable, const int64_t* __restrict__ ids,
                                                             const __nv_bfloat16* __restrict__ dh, int64_t T, int H) {
   const int nvec = H >> 3;
@@ -332,8 +334,14 @@ __global__ void __launch_bounds__(256) embed_scatter_kernel(float* __restrict__ 
     const int64_t id = ids[row];
     for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
       const Vec8 d = load8(dh + row * H + v * 8);
-      atomicAdd(reinterpret_cast<float4*>(dtable + id * H + v * 8), make_float4(d.v[0], d.v[1], d.v[2], d.v[3]));
-      atomicAdd(reinterpret_cast<float4*>(dtable + id * H + v * 8 + 4), make_float4(d.v[4], d.v[5], d.v[6], d.v[7]));
+      float* to = dtable + id * H + v * 8;
+      if constexpr (kVec) {
+        atomicAdd(reinterpret_cast<float4*>(to), make_float4(d.v[0], d.v[1], d.v[2], d.v[3]));
+        atomicAdd(reinterpret_cast<float4*>(to + 4), make_float4(d.v[4], d.v[5], d.v[6], d.v[7]));
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) atomicAdd(to + e, d.v[e]);
+      }
     }
   }
 }
@@ -466,8 +474,9 @@ extern "C" int prl_embed_gather(const void* table, const int64_t* ids, int64_t T
 extern "C" int prl_embed_scatter_add(float* dtable, const int64_t* ids, const void* dh, int64_t T, int64_t H,
                                      prl_stream_t stream) {
   PRL_CHECK_ARG(dtable && ids && dh && T >= 1 && H >= 8 && H % 8 == 0, "prl_embed_scatter_add: bad argument");
-  embed_scatter_kernel<<<(unsigned)(T < 4096 ? T : 4096), 256, 0, (cudaStream_t)stream>>>(dtable, ids,
-                                                                                          (const __nv_bfloat16*)dh, T, (int)H);
+  PRL_CHECK_ARG(((uintptr_t)dtable & 3) == 0 && ((uintptr_t)dh & 15) == 0, "prl_embed_scatter_add: dh must start on 16 bytes, dtable on 4");
+  const auto kernel = ((uintptr_t)dtable & 15) == 0 ? embed_scatter_kernel<true> : embed_scatter_kernel<false>;
+  kernel<<<(unsigned)(T < 4096 ? T : 4096), 256, 0, (cudaStream_t)stream>>>(dtable, ids, (const __nv_bfloat16*)dh, T, (int)H);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }

@@ -398,6 +398,24 @@ def test_norm_rows_add_their_squares_in_one_order(cuda_device, T, H):
     assert torch.equal(rstd, torch.rsqrt(total / torch.full_like(total, H) + 1e-6))    # a number as divisor: torch multiplies by 1 / H
 
 
+@pytest.mark.parametrize("offset", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("T,H", [(1, 8), (300, 904), (5000, 256)])
+def test_embedding_gradient_into_a_view_at_any_offset(cuda_device, T, H, offset):
+    """The table may start at any number of a flat gradient buffer.  Sums of the same fp32 terms in any order: (terms) * 2^-24."""
+    from pipelinerl_b200.learner_body import Ops
+    g, V = torch.Generator().manual_seed(T + offset), 37
+    flat = torch.randn(V * H + 8, generator=g).to(cuda_device)
+    want = flat.double()
+    ids = torch.randint(0, V, (T,), generator=g).to(cuda_device)
+    dh = torch.randn(T, H, generator=g).to(torch.bfloat16).to(cuda_device)
+    want[offset:offset + V * H].view(V, H).index_add_(0, ids, dh.double())
+    size = flat.double().abs()
+    size[offset:offset + V * H].view(V, H).index_add_(0, ids, dh.double().abs())
+    Ops().embed_bwd(flat[offset:offset + V * H].view(V, H), ids, dh)
+    assert ((flat.double() - want).abs() <= (T + 1) * 2.0 ** -24 * size).all()
+    assert torch.equal(flat[:offset].double(), want[:offset]) and torch.equal(flat[offset + V * H:].double(), want[offset + V * H:])
+
+
 @pytest.mark.parametrize("T,I", [(1, 8), (2, 18944), (37, 2056), (700, 24), (1500, 4096)])
 def test_silu_rows_cut_over_blocks(cuda_device, T, I):
     from pipelinerl_b200.learner_body import Ops
