@@ -272,6 +272,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       return __ldg(src + (int64_t)(seg0 + tok) * p.n_q + (kvh * p.R + mr));
     };
     if (mwhich < 3) meta[mwhich * 64 + mc] = fetch(u_first);
+    softmax_bar();                               // the first sub-tile's metadata, written by all, is read by all
 
     for (int it = 0; it < n_it; ++it) {
       const int s = it & 1;

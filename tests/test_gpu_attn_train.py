@@ -219,3 +219,29 @@ def test_varlen_backward_with_shared_key_tiles(cuda_device, n_q, n_kv, lens):
     out, lse = o.attn_fwd(qkv, *shape)
     first = o.attn_bwd(qkv, out, d, lse, *shape)
     assert all(torch.equal(first, o.attn_bwd(qkv, out, d, lse, *shape)) for _ in range(3))
+
+
+@pytest.mark.parametrize("gen", [1, 2, 3, 4])
+def test_varlen_backward_keeps_its_bits_with_cold_row_statistics(cuda_device, gen):
+    """The first sub-tile's log-sum-exp and delta come from far memory in one run and from L2 in the next: the softmax threads meet
+    after they are stored, so none reads an entry before it is there."""
+    from pipelinerl_b200 import _lib
+    o, lens, n_q, n_kv = _ops(), [700, 129, 64, 1, 300], 14, 2
+    T, g = sum(lens), torch.Generator().manual_seed(gen)
+    qkv = torch.randn(T, (n_q + 2 * n_kv) * 128, generator=g).to(torch.bfloat16).to(cuda_device)
+    d = torch.randn(T, n_q * 128, generator=g).to(torch.bfloat16).to(cuda_device)
+    st = torch.tensor([sum(lens[:i]) for i in range(len(lens))], dtype=torch.int32, device=cuda_device)
+    shape = (st, torch.tensor(lens, dtype=torch.int32, device=cuda_device), max(lens), n_q, n_kv, 128)
+    out, lse = o.attn_fwd(qkv, *shape)
+    flush = torch.empty(1 << 28, dtype=torch.uint8, device=cuda_device)
+    _lib.check(o.lib.prl_attn_set_bwd_generation(gen))
+    try:
+        runs = []
+        for i in range(8):
+            if i % 2:
+                flush.zero_()
+            runs.append(o.attn_bwd(qkv, out, d, lse, *shape))
+        torch.cuda.synchronize()
+    finally:
+        _lib.check(o.lib.prl_attn_set_bwd_generation(4))
+    assert all(torch.equal(runs[0], r) for r in runs[1:])
