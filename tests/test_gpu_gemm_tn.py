@@ -303,3 +303,37 @@ def test_gate_quotient_over_its_range(cuda_device):
     want = (g / (1 + torch.exp(-g))).to(torch.bfloat16).float()
     assert torch.isfinite(got).all()
     assert ((got - want).abs() <= 2.0 ** -7 * want.abs() + 1e-36).all(), (got - want).abs().max()
+
+
+@pytest.mark.parametrize("M,N,pad", [(256, 256, 0), (300, 516, 0), (129, 66, 1)])
+def test_fp32_accumulation_keeps_subnormal_numbers(cuda_device, M, N, pad):
+    """A sum below 2^-126, a product below it and an old value below it: all exact in fp32, none is a zero."""
+    from pipelinerl_b200 import _lib
+    lib, K = _lib.load(), 64
+    A = torch.full((M, K), 2.0 ** -70, dtype=torch.bfloat16, device=cuda_device)
+    for b, old in ((2.0 ** -70, 2.0 ** -133), (2.0 ** -63, -2.0 ** -126), (2.0 ** -70, -2.0 ** -134), (2.0 ** -62, 2.0 ** -140)):
+        B = torch.full((N, K), b, dtype=torch.bfloat16, device=cuda_device)
+        wide = torch.full((M, N + pad), old, device=cuda_device)
+        _lib.check(lib.prl_gemm_ex(A.data_ptr(), K, 0, B.data_ptr(), K, 0, M, N, K, wide.data_ptr(), N + pad, 1, 1, None, None, 0, 1.0,
+                                   _lib.stream_ptr()))
+        want = torch.tensor(K * 2.0 ** -70 * b + old, dtype=torch.float64).float().item()
+        assert want != 0.0 or old == -2.0 ** -134
+        assert (wide[:, :N] == want).all() and (wide[:, N:] == old).all(), (b, old)
+
+
+def test_fp32_accumulation_over_many_tiles_of_a_pair(cuda_device):
+    """More tiles than CTA pairs, ragged on both sides: what a tile adds to is read under the tile before it."""
+    from pipelinerl_b200 import _lib
+    lib, g = _lib.load(), torch.Generator().manual_seed(3)
+    M, N, K = 4000, 9220, 72
+    At = torch.randn(K, M, generator=g).to(torch.bfloat16).to(cuda_device)
+    Bt = torch.randn(K, 9224, generator=g).to(torch.bfloat16).to(cuda_device)
+    old = torch.randn(M, N, generator=g).to(cuda_device)
+    C = old.clone()
+    for _ in range(2):
+        _lib.check(lib.prl_gemm_ex(At.data_ptr(), M, 1, Bt.data_ptr(), 9224, 1, M, N, K, C.data_ptr(), N, 1, 1, None, None, 0, 1.0,
+                                   _lib.stream_ptr()))
+    plain = torch.empty(M, N, device=cuda_device)
+    _lib.check(lib.prl_gemm_ex(At.data_ptr(), M, 1, Bt.data_ptr(), 9224, 1, M, N, K, plain.data_ptr(), N, 1, 0, None, None, 0, 1.0,
+                               _lib.stream_ptr()))
+    assert torch.equal(C, old + plain + plain)
