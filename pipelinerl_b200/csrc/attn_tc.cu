@@ -77,7 +77,7 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
 }
 
 template <bool kContig>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsT, 1)
+__global__ void __launch_bounds__(kThreadsT, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
                        TcPrefillParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -92,29 +92,27 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   // so K of step i+2 streams in during the softmax of step i and S is always ready when the softmax warps want it.
   const uint32_t tmem_slot = bar(19);
 
-  // The two CTAs of a cluster own ADJACENT query tiles of the same (sequence, kv head): they walk the same K/V pages,
-  // so each CTA fetches one of the two pages of a step and TMA-multicasts it into both CTAs' shared memory -- the
-  // kernel is bound by L2 -> SM bandwidth (64 KB of K/V per 8.4 MFLOP step and CTA), and this halves it.
-  // packed training rows are long and causal: walk the query tiles heaviest-first (adjacent tiles stay a cluster pair)
+  // Every CTA loads its own K/V pages by plain TMA: no load of these kernels, which ranks on several GPUs run too, is a cluster
+  // multicast.  Neighbouring query tiles walk the same pages at about the same time, so the second read is an L2 hit; a pair of
+  // CTAs that shared its loads, and its slots, was not faster (forward 16384 x 28 / 4 heads 1650 -> 1646 us, 8 x 2048 446 -> 408,
+  // six samples of 14 / 2 heads 84 -> 79; backward 16384 5830 -> 5810).
+  // packed training rows are long and causal: walk the query tiles heaviest-first
   const int qtile = kContig ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
   const int kvh = blockIdx.y, z = blockIdx.z;
-  const uint32_t rank = ptx::cluster_ctarank();
   const int q_len = ptx::warp_uniform(p.seq_q_len[z]);
   const int pos0 = kContig ? 0 : ptx::warp_uniform(p.seq_pos0[z]);
-  if ((qtile & ~1) * p.nq >= q_len) return;              // uniform across the CLUSTER, before any barrier / TMEM use
   const int t0 = qtile * p.nq;
+  if (t0 >= q_len) return;                               // before any barrier / TMEM use
   const int row0 = ptx::warp_uniform(p.seq_q_start[z]) + t0;
   const int pos_first = pos0 + t0;
-  const int n_valid = t0 >= q_len ? 0 : ((q_len - t0) < p.nq ? (q_len - t0) : p.nq);  // 0: partner-only CTA
-  // both CTAs run the step count of the LATER tile (the earlier tile's extra step is fully masked)
-  const int pair_rows = ((qtile | 1) + 1) * p.nq;
-  const int kv_end = pos0 + (pair_rows < q_len ? pair_rows : q_len);
+  const int n_valid = (q_len - t0) < p.nq ? (q_len - t0) : p.nq;
+  const int kv_end = pos_first + n_valid;
   const int n_it = (kv_end + kKeys - 1) / kKeys;
   const int last_page = (kv_end - 1) / kPageT;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 19; ++i) ptx::mbar_init(bar(i), (i == 3 || i == 4 || i == 17 || i == 18) ? 2 : 1);  // *_empty: both CTAs' MMA warps
+    for (int i = 0; i < 19; ++i) ptx::mbar_init(bar(i), 1);
     ptx::fence_barrier_init();
     ptx::fence_proxy_async();
     ptx::prefetch_tensormap(&tm_q);
@@ -125,7 +123,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     ptx::tmem_relinquish();
   }
   ptx::tc_fence_before_sync();
-  ptx::cluster_sync();                                   // the partner's barriers exist before anything targets them
+  __syncthreads();
   ptx::tc_fence_after_sync();
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
@@ -139,26 +137,31 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       ptx::tma_load_3d(q_smem + kTile16K, &tm_q, 64, kvh * p.R, row0, bar(0), ptx::kEvictFirst);
       const int32_t* bt = kContig ? nullptr : p.block_table + (int64_t)p.seq_slot[z] * p.max_blocks;
       const int seq_row0 = p.seq_q_start[z];
-      // this CTA fetches ONE of the two pages of a step (rank 0: keys 0..63, rank 1: keys 64..127) and multicasts it
       auto load_page = [&](int it, int kv, uint32_t full_bar, uint32_t empty_bar) {
         const int s = it & 1;
         const uint32_t ph = (uint32_t)((it >> 1) & 1);
-        ptx::mbar_wait(empty_bar + 8u * (uint32_t)s, ph ^ 1u);
-        ptx::mbar_arrive_expect_tx(full_bar + 8u * (uint32_t)s, (uint32_t)(2 * kTile16K));
-        int pg = 2 * it + (int)rank;
-        if (pg > last_page) pg = last_page;              // the tail step re-reads the last page; its keys are masked
-        int row, c0;
-        if (kContig) {                                   // rows past the sequence / past T: masked keys (TMA zero-fills OOB)
-          row = seq_row0 + pg * kPageT;
+        int row[2], c0 = 0;                              // keys 0..63 and 64..127 of the step; page numbers before the wait
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          int pg = 2 * it + half;
+          if (pg > last_page) pg = last_page;              // the tail step re-reads the last page; its keys are masked
+          row[half] = kContig ? seq_row0 + pg * kPageT : bt[pg];   // contiguous rows past the sequence / past T: masked keys (TMA zero-fills OOB)
+        }
+        if (kContig) {
           c0 = (kv ? p.col_v : p.col_k) + kvh * kDT;
         } else {
-          const int page = bt[pg];
-          row = (int)(((((int64_t)p.layer * 2 + kv) * p.n_pages + page) * p.n_kv + kvh) * kPageT);
-          c0 = 0;
+#pragma unroll
+          for (int half = 0; half < 2; ++half)
+            row[half] = (int)(((((int64_t)p.layer * 2 + kv) * p.n_pages + row[half]) * p.n_kv + kvh) * kPageT);
         }
-        const uint32_t dst = kv_smem + (uint32_t)(s * kStageBytesT + kv * 2 * kTile16K) + (uint32_t)(rank * 8192);
-        ptx::tma_load_2d_multicast(dst, &tm_kv, c0, row, full_bar + 8u * (uint32_t)s, 3, ptx::kEvictLast);
-        ptx::tma_load_2d_multicast(dst + kTile16K, &tm_kv, c0 + 64, row, full_bar + 8u * (uint32_t)s, 3, ptx::kEvictLast);
+        ptx::mbar_wait(empty_bar + 8u * (uint32_t)s, ph ^ 1u);
+        ptx::mbar_arrive_expect_tx(full_bar + 8u * (uint32_t)s, (uint32_t)(2 * kTile16K));
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const uint32_t dst = kv_smem + (uint32_t)(s * kStageBytesT + kv * 2 * kTile16K + half * 8192);
+          ptx::tma_load_2d(dst, &tm_kv, c0, row[half], full_bar + 8u * (uint32_t)s, ptx::kEvictLast);
+          ptx::tma_load_2d(dst + kTile16K, &tm_kv, c0 + 64, row[half], full_bar + 8u * (uint32_t)s, ptx::kEvictLast);
+        }
       };
       load_page(0, 0, bar(1), bar(3));
       for (int it = 0; it < n_it; ++it) {                // same order as the MMA warp consumes: K(it+1), then V(it)
@@ -186,7 +189,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             ptx::mma_bf16_ss(tmem_base + (uint32_t)(s * 128), a, b, idesc_qk, ks > 0 ? 1u : 0u);
           }
           ptx::tc_commit(bar(5 + s));
-          ptx::tc_commit_multicast(bar(3 + s), 3);  // K slot consumed here: tell BOTH producers
+          ptx::tc_commit(bar(3 + s));  // K slot consumed
         }
       };
       ptx::mbar_wait(bar(0), 0);
@@ -208,8 +211,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             const uint64_t b = ptx::make_mnmajor_sw128_desc(v_addr, kTile16K) + (uint64_t)(128 * ks);
             ptx::mma_bf16_ss(tmem_base + (uint32_t)(256 + s * 128), a, b, idesc_pv, ks > 0 ? 1u : 0u);
           }
-          ptx::tc_commit(bar(10 + s));   // Ot[s] complete (and P[s] free again)
-          ptx::tc_commit_multicast(bar(17 + s), 3);  // V slot consumed here: tell BOTH producers
+          ptx::tc_commit(bar(17 + s));   // V slot consumed
+          ptx::tc_commit(bar(10 + s));   // Ot[s] complete (and P[s] free again): the last arrival of the walk, waited for
         }
       }
     }
@@ -326,7 +329,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   }
 
   ptx::tc_fence_before_sync();
-  ptx::cluster_sync();   // the partner may still multicast into this CTA's shared memory / arrive on its barriers
+  __syncthreads();
   if (warp == 1) {
     ptx::tc_fence_after_sync();
     ptx::tmem_dealloc(tmem_base, 512);
@@ -352,7 +355,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 //     (tcgen05.ld / scale / tcgen05.st) only when its running maximum grew by more than 2^8 since the reference was
 //     set -- P stays below 256, exact in bf16's range, and for trained or random scores the rescale branch is taken in
 //     the first steps of a row only.
-// TMEM: S_0 | S_1 | O_0 | O_1 (4 x 128 columns).  Shared memory and the K/V cluster multicast are those of generation 1.
+// TMEM: S_0 | S_1 | O_0 | O_1 (4 x 128 columns).  Shared memory and the K/V loads are those of generation 1.
 // =====================================================================================================
 __device__ __forceinline__ void group_bar(int g) {
   if (g == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -360,7 +363,7 @@ __device__ __forceinline__ void group_bar(int g) {
 }
 
 template <bool kContig, bool kTimed = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsT, 1)   // 10 warps: 3 share one SMSP -> 168 registers
+__global__ void __launch_bounds__(kThreadsT, 1)   // 10 warps: 3 share one SMSP -> 168 registers
 attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv, TcPrefillParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -378,24 +381,23 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 
   const int qtile = kContig ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
   const int kvh = blockIdx.y, z = blockIdx.z;
-  const uint32_t rank = ptx::cluster_ctarank();
   const int q_len = ptx::warp_uniform(p.seq_q_len[z]);
   const int pos0 = (kContig && p.seq_pos0 == nullptr) ? 0 : ptx::warp_uniform(p.seq_pos0[z]);
-  if ((qtile & ~1) * p.nq >= q_len) return;              // uniform across the CLUSTER, before any barrier / TMEM use
   const int t0 = qtile * p.nq;
+  if (t0 >= q_len) return;                               // before any barrier / TMEM use
   const int row0 = ptx::warp_uniform(p.seq_q_start[z]) + t0;
   const int pos_first = pos0 + t0;
-  const int n_valid = t0 >= q_len ? 0 : ((q_len - t0) < p.nq ? (q_len - t0) : p.nq);
-  const int pair_rows = ((qtile | 1) + 1) * p.nq;
-  const int kv_end = pos0 + (pair_rows < q_len ? pair_rows : q_len);
-  // with a window the walk starts at the first step the pair's first row still sees
+  const int n_valid = (q_len - t0) < p.nq ? (q_len - t0) : p.nq;
+  const int kv_end = pos_first + n_valid;
+  // with a window the walk starts at the first step that some row of this tile and its even neighbour still sees: a step's place
+  // in the walk decides the softmax group it belongs to, and with it the order of the sums
   const int it0 = (!kContig && p.window > 0) ? max(0, pos0 + (qtile & ~1) * p.nq - p.window + 1) / kKeys : 0;
   const int n_it = (kv_end + kKeys - 1) / kKeys - it0;
   const int last_page = (kv_end - 1) / kPageT;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 19; ++i) ptx::mbar_init(bar(i), ((i >= 4 && i <= 6) || (i >= 16 && i <= 18)) ? 2 : 1);   // *_empty: both CTAs
+    for (int i = 0; i < 19; ++i) ptx::mbar_init(bar(i), 1);
     ptx::fence_barrier_init();
     ptx::fence_proxy_async();
     ptx::prefetch_tensormap(&tm_q);
@@ -406,7 +408,7 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     ptx::tmem_relinquish();
   }
   ptx::tc_fence_before_sync();
-  ptx::cluster_sync();
+  __syncthreads();
   ptx::tc_fence_after_sync();
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
@@ -423,22 +425,28 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       auto load_page = [&](int it, int kv, uint32_t full_bar, uint32_t empty_bar) {
         const int s = it % kSt;
         const uint32_t ph = (uint32_t)((it / kSt) & 1);
-        ptx::mbar_wait(empty_bar + 8u * (uint32_t)s, ph ^ 1u);
-        ptx::mbar_arrive_expect_tx(full_bar + 8u * (uint32_t)s, (uint32_t)(2 * kTile16K));
-        int pg = 2 * (it + it0) + (int)rank;
-        if (pg > last_page) pg = last_page;
-        int row, c0;
+        int row[2], c0 = 0;                              // keys 0..63 and 64..127 of the step; page numbers before the wait
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          int pg = 2 * (it + it0) + half;
+          if (pg > last_page) pg = last_page;
+          row[half] = kContig ? seq_row0 + pg * kPageT : bt[pg];
+        }
         if (kContig) {
-          row = seq_row0 + pg * kPageT;
           c0 = (kv ? p.col_v : p.col_k) + kvh * kDT;
         } else {
-          const int page = bt[pg];
-          row = (int)(((((int64_t)p.layer * 2 + kv) * p.n_pages + page) * p.n_kv + kvh) * kPageT);
-          c0 = 0;
+#pragma unroll
+          for (int half = 0; half < 2; ++half)
+            row[half] = (int)(((((int64_t)p.layer * 2 + kv) * p.n_pages + row[half]) * p.n_kv + kvh) * kPageT);
         }
-        const uint32_t dst = kv_smem + (uint32_t)(s * kStageBytesT + kv * 2 * kTile16K) + (uint32_t)(rank * 8192);
-        ptx::tma_load_2d_multicast(dst, &tm_kv, c0, row, full_bar + 8u * (uint32_t)s, 3, ptx::kEvictLast);
-        ptx::tma_load_2d_multicast(dst + kTile16K, &tm_kv, c0 + 64, row, full_bar + 8u * (uint32_t)s, 3, ptx::kEvictLast);
+        ptx::mbar_wait(empty_bar + 8u * (uint32_t)s, ph ^ 1u);
+        ptx::mbar_arrive_expect_tx(full_bar + 8u * (uint32_t)s, (uint32_t)(2 * kTile16K));
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const uint32_t dst = kv_smem + (uint32_t)(s * kStageBytesT + kv * 2 * kTile16K + half * 8192);
+          ptx::tma_load_2d(dst, &tm_kv, c0, row[half], full_bar + 8u * (uint32_t)s, ptx::kEvictLast);
+          ptx::tma_load_2d(dst + kTile16K, &tm_kv, c0 + 64, row[half], full_bar + 8u * (uint32_t)s, ptx::kEvictLast);
+        }
       };
       load_page(0, 0, bar(1), bar(4));
       for (int it = 0; it < n_it; ++it) {
@@ -467,7 +475,7 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             ptx::mma_bf16_ss(tmem_base + (uint32_t)(s * 128), a, b, idesc_qk, ks > 0 ? 1u : 0u);
           }
           ptx::tc_commit(bar(7 + s));
-          ptx::tc_commit_multicast(bar(4 + ks_), 3);
+          ptx::tc_commit(bar(4 + ks_));
         }
       };
       const bool timed = kTimed && p.timing != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
@@ -493,8 +501,8 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             ptx::mma_bf16_ts(tmem_base + (uint32_t)(256 + s * 128), tmem_base + (uint32_t)(s * 128 + ks * 8), b, idesc_pv,
                              (i >= 2 || ks > 0) ? 1u : 0u);
           }
-          ptx::tc_commit(bar(11 + s));                 // O_s updated
-          ptx::tc_commit_multicast(bar(16 + vs_), 3);  // V slot consumed: tell BOTH producers
+          ptx::tc_commit(bar(16 + vs_));               // V slot consumed
+          ptx::tc_commit(bar(11 + s));                 // O_s updated: the last arrival of the walk, waited for
         }
       }
       if (timed && lane == 0) { p.timing[16] = w_p; p.timing[17] = w_v; p.timing[18] = clock64() - w_tot0; p.timing[19] = n_it; }
@@ -665,7 +673,7 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   }
 
   ptx::tc_fence_before_sync();
-  ptx::cluster_sync();
+  __syncthreads();
   if (warp == 1) {
     ptx::tc_fence_after_sync();
     ptx::tmem_dealloc(tmem_base, 512);
@@ -723,7 +731,7 @@ static int prefill_tc_impl(const void* q, int32_t q_rows, const void* kv_cache, 
   if (rc) return rc;
   const int smem = 2 * kTile16K + 2 * kStageBytesT + 4 * kTile16K + 1024 + 8 * 20 + 2 * 128 * 4 + 16;
   static SmemAttr smem_attr = {};
-  dim3 grid((unsigned)(((max_q_len + p.nq - 1) / p.nq + 1) & ~1), (unsigned)n_kv, (unsigned)n_seqs);  // pairs of q tiles
+  dim3 grid((unsigned)((max_q_len + p.nq - 1) / p.nq), (unsigned)n_kv, (unsigned)n_seqs);
   if (g_prefill_generation == 2 || window || sink || gate) {      // ping-pong softmax groups, P and O in TMEM (see attn_fwd_v2_kernel)
     static SmemAttr smem_attr2 = {};
     PRL_CUDA(ensure_smem(attn_fwd_v2_kernel<false>, smem, smem_attr2));
@@ -805,7 +813,7 @@ extern "C" int prl_attn_varlen_fwd(const void* qkv, int64_t qkv_stride, int32_t 
                          (uint32_t)p.nq);
   if (rc) return rc;
   const int smem = 2 * kTile16K + 2 * kStageBytesT + 4 * kTile16K + 1024 + 8 * 20 + 2 * 128 * 4 + 16;
-  dim3 grid((unsigned)(((max_seg_len + p.nq - 1) / p.nq + 1) & ~1), (unsigned)n_kv, (unsigned)n_seg);
+  dim3 grid((unsigned)((max_seg_len + p.nq - 1) / p.nq), (unsigned)n_kv, (unsigned)n_seg);
   if (g_fwd_generation == 1) {      // A/B and tests only (prl_attn_set_fwd_generation)
     static SmemAttr smem_attr = {};
     PRL_CUDA(ensure_smem(attn_prefill_tc_kernel<true>, smem, smem_attr));
@@ -853,7 +861,7 @@ extern "C" int prl_attn_varlen_fwd_kv(const void* q, int64_t q_stride, int32_t T
   rc = make_tmap_3d_bf16(&tq, q, kDT, (uint64_t)n_q, (uint64_t)Tq, kDT * 2, (uint64_t)q_stride * 2, 64, (uint32_t)p.R, (uint32_t)p.nq);
   if (rc) return rc;
   const int smem = 2 * kTile16K + 2 * kStageBytesT + 4 * kTile16K + 1024 + 8 * 20 + 2 * 128 * 4 + 16;
-  dim3 grid((unsigned)(((max_q_len + p.nq - 1) / p.nq + 1) & ~1), (unsigned)n_kv, (unsigned)n_seg);
+  dim3 grid((unsigned)((max_q_len + p.nq - 1) / p.nq), (unsigned)n_kv, (unsigned)n_seg);
   static SmemAttr smem_attr = {};
   PRL_CUDA(ensure_smem(attn_fwd_v2_kernel<true>, smem, smem_attr));
   PRL_CUDA(launch_pdl(attn_fwd_v2_kernel<true>, grid, dim3(kThreadsT), (size_t)smem, (cudaStream_t)stream_, tq, tkv, p));

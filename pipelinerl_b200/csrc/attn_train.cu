@@ -17,9 +17,8 @@
 //     (UMMA 128 x 64, all operands K-major), so a softmax thread owns a KEY and writes P^T / dS^T rows straight into
 //     the K-major shared-memory layout that  dV += P^T dO  and  dK += dS^T Q  consume as operand A, while dO / Q are
 //     read AS STORED as MN-major operand B.  TMEM: S^T, dP^T double-buffered (4 x 64 columns) + dV + dK (2 x 128).
-//   * attn_bwd_dq_kernel    (Q stationary): the forward's structure (cluster pair of adjacent query tiles, K/V pages
-//     TMA-multicast to both CTAs, 128 keys per step) with  dP = dO V^T  as a third MMA and  dQ += dS K  in place of
-//     P V (K read as stored, MN-major).  TMEM: S double-buffered + dP + dQ.
+//   * attn_bwd_dq_kernel    (Q stationary): the forward's structure (a query tile per CTA, 128 keys per step) with
+//     dP = dO V^T  as a third MMA and  dQ += dS K  in place of P V (K read as stored, MN-major).  TMEM: S double-buffered + dP + dQ.
 // Both: warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner (the WHOLE warp runs converged and elects one lane per batch of
 // UMMAs: issued from `if (lane == 0)` every UMMA costs ~180 cycles of R2UR + ELECT waterfall, tc_ptx.cuh: elect_one), the other
 // warps = softmax: 8 in lock-step in generations 1-3, 16 that never meet in generation 4 (the default; further down).
@@ -391,7 +390,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 }
 
 // =====================================================================================================
-// dQ: Q-stationary (cluster pair of adjacent query tiles, K/V pages multicast)
+// dQ: Q-stationary
 // =====================================================================================================
 constexpr int kStageKV = 4 * kT16;   // K lo | K hi | V lo | V hi   (128 keys)
 constexpr int kSmemDq = 1024 + 4 * kT16 + 2 * kStageKV + 2 * kT16 + 8 * 20 + 16;
@@ -402,7 +401,7 @@ static_assert(kSmemDq <= 232448, "dq kernel exceeds the 227 KB shared-memory lim
 //    by the softmax threads straight from global memory; S single-buffered to make room): the A operands of all three
 //    UMMAs of a step then cost no shared-memory bandwidth -- 288 -> 160 KB of shared-memory traffic per step.
 template <int kGen>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsB, 1)
+__global__ void __launch_bounds__(kThreadsB, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                    const __grid_constant__ CUtensorMap tm_kv, BwdParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -421,23 +420,21 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   // TMEM columns: gen 1/2: S[2] 0,128 | dP 256 | dQ 384.   gen 3: S 0 | dP 128 | dQ 256 | Q 384 | dO 448
   constexpr uint32_t cDP = kQT ? 128u : 256u, cDQ = kQT ? 256u : 384u, cQ = 384u, cDO = 448u;
 
-  const int qtile = (int)(gridDim.x - 1 - blockIdx.x);  // heaviest (latest) query tiles first; pairs stay adjacent
+  const int qtile = (int)(gridDim.x - 1 - blockIdx.x);  // heaviest (latest) query tiles first
   const int kvh = blockIdx.y, z = blockIdx.z;
-  const uint32_t rank = ptx::cluster_ctarank();
   const int q_len = ptx::warp_uniform(p.seg_len[z]);
-  if ((qtile & ~1) * p.nq >= q_len) return;             // uniform across the cluster
-  const int seg0 = ptx::warp_uniform(p.seg_start[z]);
   const int t0 = qtile * p.nq;
+  if (t0 >= q_len) return;
+  const int seg0 = ptx::warp_uniform(p.seg_start[z]);
   const int row0 = seg0 + t0;
-  const int n_valid = t0 >= q_len ? 0 : ((q_len - t0) < p.nq ? (q_len - t0) : p.nq);
-  const int pair_rows = ((qtile | 1) + 1) * p.nq;
-  const int kv_end = pair_rows < q_len ? pair_rows : q_len;
+  const int n_valid = (q_len - t0) < p.nq ? (q_len - t0) : p.nq;
+  const int kv_end = t0 + n_valid;
   const int n_it = (kv_end + 127) / 128;
   const int last_page = (kv_end - 1) / 64;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 18; ++i) ptx::mbar_init(bar(i), (i == 3 || i == 4 || i == 15 || i == 16) ? 2 : 1);
+    for (int i = 0; i < 18; ++i) ptx::mbar_init(bar(i), 1);
     ptx::fence_barrier_init();
     ptx::fence_proxy_async();
     ptx::prefetch_tensormap(&tm_q);
@@ -449,7 +446,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     ptx::tmem_relinquish();
   }
   ptx::tc_fence_before_sync();
-  ptx::cluster_sync();
+  __syncthreads();
   ptx::tc_fence_after_sync();
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
@@ -465,20 +462,22 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         ptx::tma_load_3d(do_smem, &tm_do, 0, kvh * p.R, row0, bar(0), ptx::kEvictFirst);
         ptx::tma_load_3d(do_smem + kT16, &tm_do, 64, kvh * p.R, row0, bar(0), ptx::kEvictFirst);
       }
-      // this CTA fetches ONE of the two 64-key pages of a step and multicasts it to both CTAs of the pair
       auto load_page = [&](int it, int kv) {
         const int s = it & 1;
         const uint32_t ph = (uint32_t)((it >> 1) & 1);
         const uint32_t full = bar((kv ? 13 : 1) + s), empty = bar((kv ? 15 : 3) + s);
         ptx::mbar_wait(empty, ph ^ 1u);
         ptx::mbar_arrive_expect_tx(full, (uint32_t)(2 * kT16));
-        int pg = 2 * it + (int)rank;
-        if (pg > last_page) pg = last_page;            // tail: re-read the last page, its keys are causally masked
-        const int row = seg0 + pg * 64;
         const int c0 = (kv ? p.col_v : p.col_k) + kvh * kD;
-        const uint32_t dst = kv_smem + (uint32_t)(s * kStageKV + kv * 2 * kT16) + (uint32_t)(rank * kT8);
-        ptx::tma_load_2d_multicast(dst, &tm_kv, c0, row, full, 3, ptx::kEvictLast);
-        ptx::tma_load_2d_multicast(dst + kT16, &tm_kv, c0 + 64, row, full, 3, ptx::kEvictLast);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {          // the two 64-key pages of a step
+          int pg = 2 * it + half;
+          if (pg > last_page) pg = last_page;          // tail: re-read the last page, its keys are causally masked
+          const int row = seg0 + pg * 64;
+          const uint32_t dst = kv_smem + (uint32_t)(s * kStageKV + kv * 2 * kT16) + (uint32_t)(half * kT8);
+          ptx::tma_load_2d(dst, &tm_kv, c0, row, full, ptx::kEvictLast);
+          ptx::tma_load_2d(dst + kT16, &tm_kv, c0 + 64, row, full, ptx::kEvictLast);
+        }
       };
       for (int it = 0; it < n_it; ++it) {
         load_page(it, 0);
@@ -527,7 +526,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                                   idesc_kk, ks > 0 ? 1u : 0u);
           }
           ptx::tc_commit(bar(9));
-          ptx::tc_commit_multicast(bar(15 + s), 3);  // V slot consumed: tell BOTH producers
+          ptx::tc_commit(bar(15 + s));  // V slot consumed
         }
       };
       ptx::mbar_wait(bar(0), 0);
@@ -551,7 +550,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                                   b, idesc_dq, (i > 0 || ks > 0) ? 1u : 0u);
           }
           ptx::tc_commit(bar(12));                   // dS may be rewritten
-          ptx::tc_commit_multicast(bar(3 + s), 3);   // K slot consumed: tell BOTH producers
+          ptx::tc_commit(bar(3 + s));   // K slot consumed
         }
         if (kTS && i + 1 < n_it) issue_dp(i + 1);  // dP of the next step goes where dS of this one was: after its dQ UMMAs
       }
@@ -691,7 +690,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   }
 
   ptx::tc_fence_before_sync();
-  ptx::cluster_sync();   // the partner may still multicast into this CTA's shared memory / arrive on its barriers
+  __syncthreads();
   if (warp == 1) {
     ptx::tc_fence_after_sync();
     ptx::tmem_dealloc(tmem_base, 512);
@@ -1078,7 +1077,7 @@ constexpr int kSmemDq4 = 1024 + 4 * kT16 + kKSlots4 * 2 * kT16 + 2 * 2 * kT16 + 
 static_assert(kSmemDq4 <= 232448, "dq4 kernel exceeds the 227 KB shared-memory limit");
 
 template <bool kTimed>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsB4, 1)
+__global__ void __launch_bounds__(kThreadsB4, 1)
 attn_bwd_dq4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                     const __grid_constant__ CUtensorMap tm_kv, BwdParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -1096,28 +1095,21 @@ attn_bwd_dq4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 
   const int qtile = (int)(gridDim.x - 1 - blockIdx.x);
   const int kvh = blockIdx.y, z = blockIdx.z;
-  const uint32_t rank = ptx::cluster_ctarank();
   const int q_len = ptx::warp_uniform(p.seg_len[z]);
-  if ((qtile & ~1) * p.nq >= q_len) return;             // uniform across the cluster
+  const int t0 = qtile * p.nq;
+  if (t0 >= q_len) return;
   const int seg0 = ptx::warp_uniform(p.seg_start[z]);
   const int pos0 = p.seg_pos0 ? ptx::warp_uniform(p.seg_pos0[z]) : 0;
   const int kv0 = p.seg_kv_start ? ptx::warp_uniform(p.seg_kv_start[z]) : seg0;
-  const int t0 = qtile * p.nq;
   const int row0 = seg0 + t0;
-  const int n_valid = t0 >= q_len ? 0 : ((q_len - t0) < p.nq ? (q_len - t0) : p.nq);
-  const int pair_rows = ((qtile | 1) + 1) * p.nq;
-  const int kv_end = pos0 + (pair_rows < q_len ? pair_rows : q_len);
+  const int n_valid = (q_len - t0) < p.nq ? (q_len - t0) : p.nq;
+  const int kv_end = pos0 + t0 + n_valid;
   const int n_it = (kv_end + 127) / 128;
   const int last_page = (kv_end - 1) / 64;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 18; ++i) {
-      int cnt = 1;
-      if ((i >= 4 && i <= 6) || i == 15 || i == 16) cnt = 2;
-      if (i == 9 || i == 10 || i == 12) cnt = 16;
-      ptx::mbar_init(bar(i), cnt);
-    }
+    for (int i = 0; i < 18; ++i) ptx::mbar_init(bar(i), (i == 9 || i == 10 || i == 12) ? 16 : 1);
     ptx::fence_barrier_init();
     ptx::fence_proxy_async();
     ptx::prefetch_tensormap(&tm_q);
@@ -1129,7 +1121,7 @@ attn_bwd_dq4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     ptx::tmem_relinquish();
   }
   ptx::tc_fence_before_sync();
-  ptx::cluster_sync();
+  __syncthreads();
   ptx::tc_fence_after_sync();
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
@@ -1149,13 +1141,16 @@ attn_bwd_dq4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const uint32_t full = bar((kv ? 13 : 1) + s), empty = bar((kv ? 15 : 4) + s);
         ptx::mbar_wait(empty, ph ^ 1u);
         ptx::mbar_arrive_expect_tx(full, (uint32_t)(2 * kT16));
-        int pg = 2 * it + (int)rank;
-        if (pg > last_page) pg = last_page;            // tail: re-read the last page, its keys are causally masked
-        const int row = kv0 + pg * 64;
         const int c0 = (kv ? p.col_v : p.col_k) + kvh * kD;
-        const uint32_t dst = (kv ? v_smem : k_smem) + (uint32_t)(s * 2 * kT16) + (uint32_t)(rank * kT8);
-        ptx::tma_load_2d_multicast(dst, &tm_kv, c0, row, full, 3, ptx::kEvictLast);
-        ptx::tma_load_2d_multicast(dst + kT16, &tm_kv, c0 + 64, row, full, 3, ptx::kEvictLast);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {          // the two 64-key pages of a step
+          int pg = 2 * it + half;
+          if (pg > last_page) pg = last_page;          // tail: re-read the last page, its keys are causally masked
+          const int row = kv0 + pg * 64;
+          const uint32_t dst = (kv ? v_smem : k_smem) + (uint32_t)(s * 2 * kT16) + (uint32_t)(half * kT8);
+          ptx::tma_load_2d(dst, &tm_kv, c0, row, full, ptx::kEvictLast);
+          ptx::tma_load_2d(dst + kT16, &tm_kv, c0 + 64, row, full, ptx::kEvictLast);
+        }
       };
       load_page(0, 0);
       for (int it = 0; it < n_it; ++it) {
@@ -1209,7 +1204,7 @@ attn_bwd_dq4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                              idesc_kk, ks > 0 ? 1u : 0u);
           }
           ptx::tc_commit(bar(11));
-          ptx::tc_commit_multicast(bar(15 + s), 3);  // V slot consumed: tell BOTH producers
+          ptx::tc_commit(bar(15 + s));  // V slot consumed
         }
       };
       ptx::mbar_wait(bar(0), 0);
@@ -1230,7 +1225,7 @@ attn_bwd_dq4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             ptx::mma_bf16_ts(tmem_base + cDQ, tmem_base + cDP + (uint32_t)((ks >> 1) * 32 + (ks & 1) * 8), b, idesc_dq,
                              (i > 0 || ks > 0) ? 1u : 0u);
           }
-          ptx::tc_commit_multicast(bar(4 + ks_), 3);   // K slot consumed: tell BOTH producers
+          ptx::tc_commit(bar(4 + ks_));   // K slot consumed
         }
         if (i + 1 < n_it) issue_dp(i + 1);
       }
@@ -1328,7 +1323,7 @@ attn_bwd_dq4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   }
 
   ptx::tc_fence_before_sync();
-  ptx::cluster_sync();   // the partner may still multicast into this CTA's shared memory / arrive on its barriers
+  __syncthreads();
   if (warp == 1) {
     ptx::tc_fence_after_sync();
     ptx::tmem_dealloc(tmem_base, 512);
@@ -1478,7 +1473,7 @@ extern "C" int prl_attn_varlen_bwd(const void* qkv, int64_t qkv_stride, int32_t 
     rc = make_tmap_3d_bf16(&tdo, d_out_bf16, kD, (uint64_t)n_q, (uint64_t)T, kD * 2, (uint64_t)n_q * kD * 2, 64, (uint32_t)p.R, (uint32_t)p.nq);
     if (rc) return rc;
     static SmemAttr attr = {};
-    dim3 grid((unsigned)(((max_seg_len + p.nq - 1) / p.nq + 1) & ~1), (unsigned)n_kv, (unsigned)n_seg);
+    dim3 grid((unsigned)((max_seg_len + p.nq - 1) / p.nq), (unsigned)n_kv, (unsigned)n_seg);
     if (g_bwd_generation == 4) {
       static SmemAttr attr4 = {};
       if (g_bwd_timing != nullptr && g_bwd_timing_kernel == 1) {
@@ -1567,7 +1562,7 @@ extern "C" int prl_attn_varlen_bwd_kv(const void* q, int64_t q_stride, int32_t T
     if (rc) return rc;
     rc = make_tmap_3d_bf16(&tdo, d_out_bf16, kD, (uint64_t)n_q, (uint64_t)Tq, kD * 2, (uint64_t)n_q * kD * 2, 64, (uint32_t)p.R, (uint32_t)p.nq);
     if (rc) return rc;
-    dim3 grid((unsigned)(((max_q_len + p.nq - 1) / p.nq + 1) & ~1), (unsigned)n_kv, (unsigned)n_seg);
+    dim3 grid((unsigned)((max_q_len + p.nq - 1) / p.nq), (unsigned)n_kv, (unsigned)n_seg);
     static SmemAttr attr = {};
     PRL_CUDA(ensure_smem(attn_bwd_dq4_kernel<false>, kSmemDq4, attr));
     attn_bwd_dq4_kernel<false><<<grid, kThreadsB4, (size_t)kSmemDq4, stream>>>(tq, tdo, tkv, p);

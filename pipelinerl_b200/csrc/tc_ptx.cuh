@@ -79,16 +79,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t smem_dst, const CUtensorMap
       : "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "l"(hint)
       : "memory");
 }
-// 2-D tile load delivered to the same shared-memory offset (and mbarrier offset) of every CTA in `cta_mask`
-__device__ __forceinline__ void tma_load_2d_multicast(uint32_t smem_dst, const CUtensorMap* map, int c0, int c1,
-                                                      uint32_t bar, uint16_t cta_mask, uint64_t hint) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster.L2::cache_hint"
-      " [%0], [%1, {%4, %5}], [%2], %3, %6;"
-      :
-      : "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "h"(cta_mask), "r"(c0), "r"(c1), "l"(hint)
-      : "memory");
-}
 // 1-D bulk copy global -> shared (no tensor map), completes on an mbarrier
 __device__ __forceinline__ void bulk_load_1d(uint32_t smem_dst, const void* gsrc, uint32_t bytes, uint32_t bar,
                                              uint64_t hint) {
@@ -119,11 +109,6 @@ __device__ __forceinline__ void tc_fence_after_sync() {
 // arrive on an mbarrier when all tcgen05 ops previously issued by this thread have completed
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-// same, arriving on the same-offset mbarrier of every CTA in `cta_mask` (single-CTA MMAs, cluster-shared operands)
-__device__ __forceinline__ void tc_commit_multicast(uint32_t bar, uint16_t cta_mask) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(bar), "h"(cta_mask) : "memory");
 }
 // One lane of a CONVERGED warp.  tcgen05.mma / commit take their operands from uniform registers: issued from inside an
 // `if (lane == 0)` region the compiler cannot prove the operands warp-uniform and wraps every UMMA in a
@@ -317,9 +302,6 @@ __device__ __forceinline__ void mma_bf16_ts_w(uint32_t d_tmem, uint32_t a_tmem, 
 }
 __device__ __forceinline__ void tc_commit_w(uint32_t bar) {
   if (elect_one()) tc_commit(bar);
-}
-__device__ __forceinline__ void tc_commit_multicast_w(uint32_t bar, uint16_t cta_mask) {
-  if (elect_one()) tc_commit_multicast(bar, cta_mask);
 }
 
 }  // namespace ptx

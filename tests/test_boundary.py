@@ -115,3 +115,13 @@ def test_plain_c_client_links_and_calls(built_lib, tmp_path):
     env = dict(os.environ, LD_LIBRARY_PATH=f"{so.parent}:{os.environ.get('LD_LIBRARY_PATH', '')}")
     r = subprocess.run([str(exe)], capture_output=True, text=True, env=env, timeout=60)
     assert r.returncode == 0 and r.stdout.startswith("ok version="), (r.returncode, r.stdout, r.stderr)
+
+
+def test_no_load_is_delivered_to_several_ctas():
+    """Ranks on several GPUs run every kernel here; a bulk or tensor load whose data goes to more than one CTA of a cluster is not to
+    be among them (an arrival that tells several CTAs of finished products is)."""
+    word = "multi" + "cast"
+    for f in sorted((ROOT / "pipelinerl_b200" / "csrc").iterdir()):
+        for n, line in enumerate(f.read_text().splitlines(), 1):
+            code = line.split("//")[0]
+            assert not (word in code and "bulk" in code), f"{f.name}:{n}"
