@@ -344,8 +344,9 @@ int prl_gemm_ex(const void* A, int64_t lda, int32_t a_mn_major, const void* B, i
  * Bit-identical to prl_gemm_ex + prl_silu_mul_fwd.  I must be a multiple of 128. */
 int prl_gemm_swiglu(const void* X, int64_t ldx, const void* W, int64_t ldw, int64_t M, int64_t I, int64_t K, void* act,
                     int64_t ld_act, void* gate_up /*or NULL*/, int64_t ld_gate_up, prl_stream_t stream);
-/* sampler form (chunked prefill): act = bf16(SiLU(gate) * up) of the fp32 accumulators, i.e. the bits of
- * prl_gemm_tn(fp32 out) + prl_silu_mul without the [M, 2I] fp32 round trip through HBM */
+/* sampler form (chunked prefill): act = bf16(SiLU(gate) * up) of the fp32 accumulators: the rounding points of
+ * prl_gemm_tn(fp32 out) + prl_silu_mul without the [M, 2I] fp32 round trip through HBM (the quotient of the sigmoid may differ in its
+ * last fp32 bit, which less than one quotient in 10^6 does) */
 int prl_gemm_swiglu_f32(const void* X_bf16, int64_t ldx, const void* W_gate_up_bf16, int64_t ldw, int64_t M, int64_t I,
                         int64_t K, void* act_bf16, int64_t ld_act, prl_stream_t stream);
 /* down_proj dgrad with the backward of SiLU(gate) * up in its epilogue: d_gate_up[M, 2 I] (= d gate | d up) from dY[M, H],
@@ -499,6 +500,8 @@ int prl_attn_debug_timing(int64_t* out20_device);
 int prl_attn_debug_bwd_timing(int64_t* out16_device);
 int prl_attn_debug_bwd_timing_dkdv(int64_t* out16_device);
 int prl_debug_mma_bench(int32_t mode, int32_t iters, int64_t* out2_device, prl_stream_t stream);
+/* test helper: q[i] = a[i] / b[i], b[i] >= 1, as the gated activations of the CTA-pair GEMM and of the learner's row kernels divide */
+int prl_debug_quotient(const float* a, const float* b, int64_t n, float* q, prl_stream_t stream);
 /* Sampling with in-kernel logprob capture: id ~ softmax(logits/T) (Gumbel-max, counter-based RNG on
  * (seed, step, row, vocab id)) or argmax when greedy; logprob = log_softmax(logits/T)[id]. */
 size_t prl_sample_workspace_bytes(int32_t B);

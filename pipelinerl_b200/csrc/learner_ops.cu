@@ -346,6 +346,11 @@ __global__ void __launch_bounds__(256) embed_scatter_kernel(float* __restrict__ 
   }
 }
 
+__global__ void __launch_bounds__(256) quotient_kernel(const float* __restrict__ a, const float* __restrict__ b, int64_t n,
+                                                       float* __restrict__ q) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) q[i] = div_ge1(a[i], b[i]);
+}
+
 int silu_threads(int64_t I) {
   const int64_t n = (I + 7) / 8;
   return n >= 256 ? 256 : (int)((n + 31) / 32 * 32);
@@ -477,6 +482,13 @@ extern "C" int prl_embed_scatter_add(float* dtable, const int64_t* ids, const vo
   PRL_CHECK_ARG(((uintptr_t)dtable & 3) == 0 && ((uintptr_t)dh & 15) == 0, "prl_embed_scatter_add: dh must start on 16 bytes, dtable on 4");
   const auto kernel = ((uintptr_t)dtable & 15) == 0 ? embed_scatter_kernel<true> : embed_scatter_kernel<false>;
   kernel<<<(unsigned)(T < 4096 ? T : 4096), 256, 0, (cudaStream_t)stream>>>(dtable, ids, (const __nv_bfloat16*)dh, T, (int)H);
+  PRL_LAUNCH_CHECK();
+  return PRL_OK;
+}
+
+extern "C" int prl_debug_quotient(const float* a, const float* b, int64_t n, float* q, prl_stream_t stream) {
+  PRL_CHECK_ARG(a && b && q && n >= 1, "prl_debug_quotient: bad argument");
+  quotient_kernel<<<(unsigned)(n < 256 * 4096 ? (n + 255) / 256 : 4096), 256, 0, (cudaStream_t)stream>>>(a, b, n, q);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }

@@ -305,6 +305,66 @@ def test_gate_quotient_over_its_range(cuda_device):
     assert ((got - want).abs() <= 2.0 ** -7 * want.abs() + 1e-36).all(), (got - want).abs().max()
 
 
+def _quotient(a, b):
+    from pipelinerl_b200 import _lib
+    lib, q = _lib.load(), torch.empty_like(a)
+    _lib.check(lib.prl_debug_quotient(a.data_ptr(), b.data_ptr(), a.numel(), q.data_ptr(), _lib.stream_ptr()))
+    return q
+
+
+@pytest.mark.parametrize("name", ["plain", "scaled", "silu", "sigmoid", "small", "subnormal", "midpoints"])
+def test_quotient_of_the_gates_in_fp32(cuda_device, name):
+    """a / b, b >= 1, against the device's own division.  From 2^-100 on: another value than the rounded one only within 2^-21 ulp of
+    a midpoint, which one quotient in 2^20 is, and then its neighbour.  Below: one unit in the last place.  "midpoints" are the
+    quotients nearest to one: mantissas A, B (B odd) with A 2^24 or A 2^25 = M B + 1, M a 25-bit midpoint, found by inverting B."""
+    n, g = 1 << 22, torch.Generator(device=cuda_device).manual_seed(len(name))
+
+    def draw(lo, hi):
+        return (1 + torch.rand(n, generator=g, device=cuda_device)) * torch.exp2(torch.randint(lo, hi + 1, (n,), generator=g, device=cuda_device).float())
+    gate = torch.linspace(-75, 100, n, device=cuda_device)
+    if name == "plain":
+        a, b = draw(-30, 100) * torch.where(torch.rand(n, generator=g, device=cuda_device) < 0.5, -1.0, 1.0), draw(0, 60)
+    elif name == "scaled":
+        a, b = draw(30, 100), draw(60, 126)
+    elif name == "silu":
+        a, b = gate, 1 + torch.exp(-gate)
+    elif name == "sigmoid":
+        a, b = torch.ones_like(gate), 1 + torch.exp(-gate.clamp(min=-69))
+    elif name == "small":
+        a, b = draw(-126, -100), draw(0, 30)
+    elif name == "subnormal":
+        a, b = draw(-149, -126), draw(0, 20)
+    else:
+        B = torch.arange((1 << 23) + 1, 1 << 24, 2, device=cuda_device)
+        parts = []
+        for bits in (24, 25):
+            m, inv = (1 << bits) - 1, B.clone()
+            for _ in range(5):
+                inv = (inv * ((2 - (B * inv & m)) & m)) & m
+            M = (-inv & m) + ((1 << 24) if bits == 24 else 0)
+            A = (M * B + 1) >> bits
+            ok = (M >= 1 << 24) & (M < 1 << 25) & (A >= 1 << 23) & (A < 1 << 24)
+            assert ((M * B + 1)[ok] & m == 0).all() and ok.sum() > 1000000
+            parts.append((A[ok].float() * 2.0 ** -23, B[ok].float() * 2.0 ** -23))
+        a, b = torch.cat([x[0] for x in parts]), torch.cat([x[1] for x in parts])
+    got, want = _quotient(a, b), a / b
+    off = (got.view(torch.int32).long() - want.view(torch.int32).long()).abs()
+    assert off.max().item() <= 1
+    if name in ("plain", "scaled", "silu", "sigmoid"):
+        assert (want.abs() >= 2.0 ** -100).sum() >= 0.99 * n and (off != 0).sum().item() <= 8 + n / 2 ** 20
+
+
+def test_quotient_of_the_gates_at_zero_and_infinity(cuda_device):
+    inf, nan = float("inf"), float("nan")
+    a = torch.tensor([0.0, -0.0, 1.0, -1.0, inf, -inf, nan, 3.4e38, -3.4e38, 88.0, -104.0], device=cuda_device)
+    b = torch.tensor([1.0, 2.0, 3.0, inf, 3.4e38, 1.8446744e19, 2.0e19, nan, 1.0000001], device=cuda_device)
+    a, b = (t.contiguous() for t in torch.cartesian_prod(a, b).T)
+    got, want = _quotient(a, b), a / b
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    ok = ~torch.isnan(want)
+    assert torch.equal(got[ok], want[ok]) and torch.equal(torch.signbit(got[ok]), torch.signbit(want[ok]))
+
+
 @pytest.mark.parametrize("M,N,pad", [(256, 256, 0), (300, 516, 0), (129, 66, 1)])
 def test_fp32_accumulation_keeps_subnormal_numbers(cuda_device, M, N, pad):
     """A sum below 2^-126, a product below it and an old value below it: all exact in fp32, none is a zero."""
