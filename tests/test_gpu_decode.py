@@ -423,6 +423,34 @@ def test_token_step_with_and_without_the_swiglu_epilogue_is_bit_identical(cuda_d
     assert torch.equal(logits[True], logits[False])
 
 
+def test_token_step_takes_the_swiglu_epilogue_where_gate_up_could_split_k(cuda_device):
+    """2048 wide, I 8192: 128 tiles, which the planner would cut in K.  The engine takes the gated epilogue all the same; its
+    log-probs and those of the split pair meet the oracle within the bar that the 7B width has (bf16 activations, one layer), and
+    differ from one another by less: both sums are fp32, an activation may fall to the other side of a bf16 rounding."""
+    from pipelinerl_b200.engine import SamplingParams
+    from pipelinerl_b200.model import ModelConfig
+    cfg = ModelConfig(vocab_size=4096, hidden_size=2048, intermediate_size=8192, num_layers=1, num_q_heads=16, num_kv_heads=4)
+    w = tiny_weights(cfg, std=0.02, bias_std=0.1)
+    tokens = torch.randint(0, cfg.vocab_size, (40,), generator=torch.Generator().manual_seed(7)).tolist()
+    want = OracleQwen2(cfg, w).score(tokens, 1.0).numpy()
+    got = {}
+    for fuse in (True, False):
+        eng = make_engine(cfg, w, cuda_device, max_batch=4, max_seq_len=128, max_new_tokens=4, use_cuda_graph=False,
+                          prefill_chunk=0, fused_head=False)
+        assert eng.split_k["gate_up"] > 1 and eng.swiglu_epilogue     # otherwise neither side is what its name says
+        eng.fuse_swiglu = fuse
+        eng.add_request(tokens, SamplingParams(max_tokens=2, temperature=1.0, greedy=True))
+        lp = []
+        for t in range(len(tokens) - 1):
+            eng.step()
+            lp.append(torch.log_softmax(eng.logits[0], -1)[tokens[t + 1]].item())
+        got[fuse] = np.array(lp)
+        rel = np.abs(got[fuse] - want) / np.abs(want)
+        assert rel.mean() <= 1e-3 and rel.max() <= 2.1e-3, (fuse, rel.max(), rel.mean())
+        del eng
+    assert np.abs(got[True] - got[False]).max() <= 1e-3 * np.abs(want).max()
+
+
 @pytest.mark.parametrize("B,H,n_split", [(129, 4, 1), (130, 1036, 2), (300, 3584, 0), (200, 4100, 1), (129, 16384, 1), (140, 16388, 1)])
 def test_residual_norm_of_many_rows(cuda_device, B, H, n_split):
     """Prompt chunks (more than 128 rows): widths around a thread's four pieces and the widest block.  One bf16 rounding, and an

@@ -397,3 +397,93 @@ def test_fp32_accumulation_over_many_tiles_of_a_pair(cuda_device):
     _lib.check(lib.prl_gemm_ex(At.data_ptr(), M, 1, Bt.data_ptr(), 9224, 1, M, N, K, plain.data_ptr(), N, 1, 0, None, None, 0, 1.0,
                                _lib.stream_ptr()))
     assert torch.equal(C, old + plain + plain)
+
+
+def _at(t, offset):
+    """A copy of `t` whose storage starts `offset` elements into a buffer (for bf16 one element is two bytes off 16)."""
+    buf = torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)
+    out = buf[offset:offset + t.numel()].view(t.shape)
+    out.copy_(t)
+    return out
+
+
+@pytest.mark.parametrize("M,K,I,offset", [(130, 72, 128, 1), (300, 264, 384, 4)])
+def test_silu_epilogue_into_unaligned_rows(cuda_device, M, K, I, offset):
+    """act and gate_up that start off 16 bytes leave the staged chunk element by element: the same bits, nothing beside them."""
+    from pipelinerl_b200 import _lib
+    from pipelinerl_b200.learner_body import Ops
+    lib, g = _lib.load(), torch.Generator().manual_seed(M)
+    X = torch.randn(M, K, generator=g).to(torch.bfloat16).to(cuda_device)
+    W = (0.2 * torch.randn(2 * I, K, generator=g)).to(torch.bfloat16).to(cuda_device)
+    want_gu, want = Ops().gemm_swiglu(X, W)
+    act = torch.full((M * I + 8,), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    gu = torch.full((M * 2 * I + 8,), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    _lib.check(lib.prl_gemm_swiglu(X.data_ptr(), K, W.data_ptr(), K, M, I, K, act[offset:].data_ptr(), I, gu[offset:].data_ptr(), 2 * I,
+                                   _lib.stream_ptr()))
+    assert torch.equal(act[offset:offset + M * I].view(M, I), want) and torch.equal(gu[offset:offset + 2 * M * I].view(M, 2 * I), want_gu)
+    for t, n in ((act, M * I), (gu, 2 * M * I)):
+        assert (t[:offset] == 7.0).all() and (t[offset + n:] == 7.0).all()
+
+
+@pytest.mark.parametrize("M,N,K,ldc,offset", [(300, 200, 72, 200, 0), (257, 1000, 136, 1000, 1), (130, 66, 64, 67, 0), (2049, 3584, 64, 3584, 4)])
+def test_residual_in_the_output_buffer(cuda_device, M, N, K, ldc, offset):
+    """C = A B^T + C in bf16, aligned and not: every element is read before it is written, by the thread that writes it."""
+    from pipelinerl_b200 import _lib
+    lib, g = _lib.load(), torch.Generator().manual_seed(M + N)
+    A = torch.randn(M, K, generator=g).to(torch.bfloat16).to(cuda_device)
+    B = torch.randn(N, K, generator=g).to(torch.bfloat16).to(cuda_device)
+    C = _at(torch.randn(M, ldc, generator=g).to(torch.bfloat16).to(cuda_device), offset)
+    res, want = C.clone(), torch.empty(M, ldc, dtype=torch.bfloat16, device=cuda_device)
+    for out, r in ((want, res), (C, C)):
+        _lib.check(lib.prl_gemm_ex(A.data_ptr(), K, 0, B.data_ptr(), K, 0, M, N, K, out.data_ptr(), ldc, 0, 0, None, r.data_ptr(), ldc, 1.0,
+                                   _lib.stream_ptr()))
+    assert torch.equal(C[:, :N], want[:, :N]) and torch.equal(C[:, N:], res[:, N:])
+    exact = A.double() @ B.double().T + res[:, :N].double()
+    slack = K * 2.0 ** -24 * (A.double().abs() @ B.double().abs().T)
+    assert ((C[:, :N].double() - exact).abs() <= 2 * slack + 2.0 ** -8 * exact.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("K1,K2,N", [(72, 64, 1002), (128, 1000, 301)])
+def test_dual_product_into_unaligned_rows(cuda_device, K1, K2, N):
+    """Slices of a split whose rows are not a multiple of 16 bytes."""
+    from pipelinerl_b200 import _lib
+    lib, g, M = _lib.load(), torch.Generator().manual_seed(N), 300
+    A1, B1, A2, B2 = ((torch.randn(r, k, generator=g) / k ** 0.5).to(torch.bfloat16).to(cuda_device) for r, k in ((M, K1), (N, K1), (M, K2), (N, K2)))
+    want = A1.double() @ B1.double().T + A2.double() @ B2.double().T
+    size = A1.double().abs() @ B1.double().abs().T + A2.double().abs() @ B2.double().abs().T
+    for k in (1, 2):
+        flat = torch.full((k * M * N + 8,), 7.0, device=cuda_device)
+        out = flat[1:1 + k * M * N].view(k, M, N)
+        _lib.check(lib.prl_gemm_tn_dual(A1.data_ptr(), B1.data_ptr(), K1, A2.data_ptr(), B2.data_ptr(), K2, M, N, k, out.data_ptr(),
+                                        _lib.stream_ptr()))
+        assert ((out.double().sum(0) - want).abs() <= (K1 + K2 + k) * 2.0 ** -24 * size + 1e-12).all()
+        assert flat[0] == 7.0 and (flat[1 + k * M * N:] == 7.0).all()
+
+
+@pytest.mark.parametrize("N,ldc", [(72, 75), (136, 136), (300, 303)])
+def test_grouped_products_into_unaligned_rows(cuda_device, N, ldc):
+    """The gated (bf16, weighted) and the plain (fp32) output of the grouped GEMM with rows off 16 bytes: the bits of aligned rows."""
+    from pipelinerl_b200 import _lib
+    lib, g = _lib.load(), torch.Generator().manual_seed(N)
+    n, W, experts, top = 300, 64, 3, 2
+    x = torch.randn(n, W, generator=g).to(torch.bfloat16).to(cuda_device)
+    w = (torch.randn(experts * N, W, generator=g) / 8).to(torch.bfloat16).to(cuda_device)
+    z = torch.randn(n, experts, generator=g).to(cuda_device)
+    i32 = dict(dtype=torch.int32, device=cuda_device)
+    sel, perm, meta = torch.zeros(top, n, **i32), torch.zeros(top * n, **i32), torch.zeros(4, **i32)
+    wsel, tiles = torch.zeros(top, n, device=cuda_device), torch.zeros(3 * int(lib.prl_moe_max_tiles(top * n, experts)), **i32)
+    st, table = _lib.stream_ptr(), (perm.data_ptr(), meta.data_ptr(), tiles.data_ptr())
+    _lib.check(lib.prl_moe_choose(z.data_ptr(), experts, None, n, experts, experts, top, 1, 1, 1, 0, 0, 1.0, 256, sel.data_ptr(), wsel.data_ptr(),
+                                  *table, st))
+    xs = torch.zeros(top * n, W, dtype=torch.bfloat16, device=cuda_device)
+    _lib.check(lib.prl_moe_gather(x.data_ptr(), *table[:2], n, top * n, W, xs.data_ptr(), st))
+    for dtype, weights in ((torch.bfloat16, wsel.data_ptr()), (torch.float32, None)):
+        got = []
+        for ld, off in ((N + -N % 8, 0), (ldc, 1)):
+            flat = torch.full((top * n * ld + 8,), 7.0, dtype=dtype, device=cuda_device)
+            out = flat[off:off + top * n * ld].view(top * n, ld)
+            _lib.check(lib.prl_moe_gemm_tc(xs.data_ptr(), top * n, w.data_ptr(), experts, N, W, *table, weights, 1 if weights else 0,
+                                           out.data_ptr(), ld, st))
+            assert (out[:, N:] == 7.0).all() and (flat[:off] == 7.0).all() and (flat[off + top * n * ld:] == 7.0).all()
+            got.append(out[:, :N].clone())
+        assert torch.equal(got[0], got[1]) and got[0].float().abs().max() < 100 and (got[0] != 7.0).any()

@@ -315,6 +315,27 @@ def test_logprob_tail_at_the_edges_of_its_groups(cuda_device, T, V, pad):
     assert (ent.double() - entropy).abs().max().item() <= 2 * slack
 
 
+def test_logprob_tail_of_masked_and_infinite_logits(cuda_device):
+    """-inf logits (masked vocabulary), a thread's first values and whole 16-value groups among them, leave the log-probs of the
+    others alone; a +inf or NaN logit makes the row's log-prob NaN, as in torch, which rl_step reports as not finite."""
+    from pipelinerl_b200 import _lib
+    lib, g, T, V = _lib.load(), torch.Generator().manual_seed(2), 6, 20000
+    z = torch.randn(T, V, generator=g)
+    z[0, :9000] = -torch.inf
+    z[1, ::2] = -torch.inf
+    z[2, 17:] = -torch.inf
+    z[3, 5] = torch.inf
+    z[4, 12345] = torch.nan
+    z = z.to(cuda_device)
+    ids = torch.tensor([0, 9001, 1, 3, 7, 7], device=cuda_device)
+    lp, ent, lse = (torch.empty(T - 1, device=cuda_device) for _ in range(3))
+    _lib.check(lib.prl_logprob_tail_fwd(z.data_ptr(), T, V, V, ids.data_ptr(), 1.0, lp.data_ptr(), ent.data_ptr(), lse.data_ptr(),
+                                        _lib.stream_ptr()))
+    want = torch.log_softmax(z[:-1].double(), -1).gather(1, ids[1:, None])[:, 0]
+    assert (lp[:3].double() - want[:3]).abs().max().item() <= 20 * (2.0 ** -20 + 4096 * 2.0 ** -24)
+    assert torch.isnan(lp[3:]).all() and torch.isnan(want[3:]).all()
+
+
 def test_rl_step_over_several_rows_of_logits(cuda_device):
     """Two unpacked rows: every row's gradient arrives in its own place of the [B, L, V] logits."""
     from pipelinerl_b200.finetune.rl import RLConfig, rl_step
@@ -323,6 +344,8 @@ def test_rl_step_over_several_rows_of_logits(cuda_device):
     both = LogitsModel(torch.from_numpy(arrs["logits"]).to(cuda_device))
     loss, _ = rl_step(both, batch, 0, 10, RLConfig(**meta["config"]))
     loss.backward()
+    np.testing.assert_allclose(both.logits.grad.cpu().numpy(), arrs["grad_logits"], rtol=1e-4, atol=2e-7)   # torch autograd's, row by row
+    assert not np.allclose(arrs["grad_logits"][0], arrs["grad_logits"][1], rtol=1e-2, atol=1e-6)               # rows told apart
     half = torch.from_numpy(arrs["logits"]).to(cuda_device).to(torch.bfloat16).requires_grad_()
     model = LogitsModel(half.detach())
     loss16, _ = rl_step(model, batch, 0, 10, RLConfig(**meta["config"]))
