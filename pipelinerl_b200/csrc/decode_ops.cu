@@ -61,7 +61,8 @@ __device__ __forceinline__ void store_bf16(__nv_bfloat16* p, const float (&v)[W]
 
 // ---- embedding gather + RMSNorm ------------------------------------------------------
 // h[b,:] = embed[token[b],:] ; x[b,:] = bf16(h * rsqrt(mean(h^2) + eps) * g).  W = 4: rows of whole 8-byte pieces
-// (1024 x 3584: 13.2 us with one channel per access).
+// (1024 x 3584: 13.2 us with one channel per access).  The squares are added channel t, t + 256, ... by thread t in both forms (out of
+// L1 the second time), so that the norm's bits do not hang on the form.
 template <int W>
 __global__ void __launch_bounds__(256) embed_rmsnorm_kernel(const int32_t* __restrict__ tokens,
                                                            const __nv_bfloat16* __restrict__ embed,
@@ -81,8 +82,14 @@ __global__ void __launch_bounds__(256) embed_rmsnorm_kernel(const int32_t* __res
     load_bf16<W>(row + i, v);
     if constexpr (W == 4) *reinterpret_cast<float4*>(h + (int64_t)b * H + i) = make_float4(v[0], v[1], v[2], v[3]);
     else h[(int64_t)b * H + i] = v[0];
-#pragma unroll
-    for (int e = 0; e < W; ++e) ss += v[e] * v[e];
+    if (W == 1) ss += v[0] * v[0];
+  }
+  if (W > 1) {
+#pragma unroll 8
+    for (int i = threadIdx.x; i < H; i += blockDim.x) {
+      const float v = __bfloat162float(row[i]);
+      ss += v * v;
+    }
   }
   const float tot = block_sum(ss, s_red);
   const float r = rsqrtf(tot / (float)H + eps);
@@ -102,6 +109,10 @@ __global__ void __launch_bounds__(256) embed_rmsnorm_kernel(const int32_t* __res
 // n_split partial loads back to back (independent, L2-resident), so the kernel costs about one
 // L2 round trip + one block reduction instead of a serial chain per element.
 constexpr int kMaxSplitUnroll = 8;
+// one contraction for every kernel that norms a residual row
+__device__ __forceinline__ float add_squares(const float4& v, float ss) {
+  return __fadd_rn(ss, fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, __fmul_rn(v.x, v.x)))));
+}
 __global__ void __launch_bounds__(1024) residual_rmsnorm_kernel(const float* __restrict__ part, int n_split, int B,
                                                                int H, const __nv_bfloat16* __restrict__ gamma,
                                                                float eps, float* __restrict__ h,
@@ -131,7 +142,7 @@ __global__ void __launch_bounds__(1024) residual_rmsnorm_kernel(const float* __r
     }
     hrow[i] = v;
     if (single) keep = v; else reinterpret_cast<float4*>(s_row)[i] = v;
-    ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+    ss = add_squares(v, ss);
   }
   const float tot = block_sum(ss, s_red);
   const float r = rsqrtf(tot / (float)H + eps);
@@ -149,18 +160,19 @@ __global__ void __launch_bounds__(1024) residual_rmsnorm_kernel(const float* __r
 // The same for MANY rows (prompt chunks), whose time is the rows' way through the SMs and not one row's latency: four pieces per
 // thread in flight, so that a 3584-channel row takes 224 threads and eight rows share an SM, and h is written back only where
 // something was added to it (the wide GEMM of a prompt has added its tile itself: n_split = 0).  1024 x 3584: 17.6 us with a
-// thread per piece and two rows on an SM.
-template <int kPer>
-__global__ void __launch_bounds__(1024) residual_rmsnorm_rows_kernel(const float* __restrict__ part, int n_split, int B, int H,
+// thread per piece and two rows on an SM.  The squares are added in that form's order: it has a thread for each piece, at most 1024,
+// which then add their pieces one after the other.  Here a thread does the sums of kSub of its threads (pieces k, k + kSub, ...).
+template <int kPer, int kSub>
+__global__ void __launch_bounds__(256) residual_rmsnorm_rows_kernel(const float* __restrict__ part, int n_split, int B, int H,
                                                                      const __nv_bfloat16* __restrict__ gamma, float eps,
                                                                      float* __restrict__ h, __nv_bfloat16* __restrict__ x) {
   pdl_launch_dependents();
   const int H4 = H >> 2, b = blockIdx.x;
-  float g[kPer][4];
+  uint2 g[kPer];
 #pragma unroll
   for (int k = 0; k < kPer; ++k) {
     const int i = threadIdx.x + k * blockDim.x;
-    if (i < H4) load_bf16<4>(gamma + 4 * i, g[k]);
+    if (i < H4) g[k] = reinterpret_cast<const uint2*>(gamma)[i];
   }
   pdl_wait();
   __shared__ float s_red[32];
@@ -186,15 +198,26 @@ __global__ void __launch_bounds__(1024) residual_rmsnorm_rows_kernel(const float
       if (i < H4) hrow[i] = v[k];
     }
   }
-  float ss = 0.f;
+  float ss[kSub], tot = 0.f;
 #pragma unroll
-  for (int k = 0; k < kPer; ++k) ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
-  const float r = rsqrtf(block_sum(ss, s_red) / (float)H + eps);
+  for (int j = 0; j < kSub; ++j) ss[j] = 0.f;
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) ss[k % kSub] = add_squares(v[k], ss[k % kSub]);
+  const int nw = blockDim.x >> 5;
+#pragma unroll
+  for (int j = 0; j < kSub; ++j) {
+    const float w = warp_sum(ss[j]);
+    if ((threadIdx.x & 31) == 0) s_red[j * nw + (threadIdx.x >> 5)] = w;
+  }
+  __syncthreads();
+  for (int i = 0; i < kSub * nw; ++i) tot += s_red[i];
+  const float r = rsqrtf(tot / (float)H + eps);
 #pragma unroll
   for (int k = 0; k < kPer; ++k) {
     const int i = threadIdx.x + k * blockDim.x;
     if (i >= H4) continue;
-    const float o[4] = {v[k].x * r * g[k][0], v[k].y * r * g[k][1], v[k].z * r * g[k][2], v[k].w * r * g[k][3]};
+    const float o[4] = {v[k].x * r * bf16_bits_to_float(g[k].x & 0xffffu), v[k].y * r * bf16_bits_to_float(g[k].x >> 16),
+                        v[k].z * r * bf16_bits_to_float(g[k].y & 0xffffu), v[k].w * r * bf16_bits_to_float(g[k].y >> 16)};
     store_bf16<4>(x + (int64_t)b * H + 4 * i, o);
   }
 }
@@ -561,8 +584,9 @@ extern "C" int prl_residual_rmsnorm(const float* partials, int32_t n_split, int3
   PRL_CHECK_ARG(H % 4 == 0, "prl_residual_rmsnorm: hidden size must be a multiple of 4 (got %d)", H);
   PRL_CHECK_ARG(H * 4 <= 96 * 1024, "prl_residual_rmsnorm: hidden size too large for the row buffer");
   if (B > 128 && H <= 4 * 4 * 1024 && !l2_prefetch) {   // a prompt chunk; a token step's rows (up to 128) want one row's latency short
-    const int per_row = ((H / 4 + 3) / 4 + 31) / 32 * 32;
-    PRL_CUDA(launch_pdl(residual_rmsnorm_rows_kernel<4>, dim3(B), dim3(per_row), 0, (cudaStream_t)st, partials, (int)n_split, (int)B,
+    const int H4 = H / 4, per_row = H4 > 1024 ? 256 : ((H4 + 3) / 4 + 31) / 32 * 32;
+    const auto kernel = H4 > 2048 ? residual_rmsnorm_rows_kernel<16, 4> : H4 > 1024 ? residual_rmsnorm_rows_kernel<8, 4> : residual_rmsnorm_rows_kernel<4, 4>;
+    PRL_CUDA(launch_pdl(kernel, dim3(B), dim3(per_row), 0, (cudaStream_t)st, partials, (int)n_split, (int)B,
                         (int)H, (const __nv_bfloat16*)gamma, eps, h, (__nv_bfloat16*)x_bf16));
     PRL_LAUNCH_CHECK();
     return PRL_OK;

@@ -472,6 +472,45 @@ def test_residual_norm_of_many_rows(cuda_device, B, H, n_split):
     assert ((x.double() - want).abs() <= (2.0 ** -8 + H * 2.0 ** -24) * want.abs() + 1e-30).all()
 
 
+@pytest.mark.parametrize("B,H,n_split", [(129, 4, 1), (130, 1036, 2), (200, 2048, 1), (300, 3584, 0), (150, 4096, 3), (200, 4100, 1), (140, 8192, 2),
+                                         (129, 16384, 1)])
+def test_norm_of_many_rows_has_the_bits_of_few(cuda_device, B, H, n_split):
+    """A prompt chunk's norm (more than 128 rows) and the token step's add a row's squares in one order: chunking changes no bit."""
+    from pipelinerl_b200 import _lib
+    lib, g = _lib.load(), torch.Generator().manual_seed(H)
+    h = torch.randn(B, H, generator=g).to(cuda_device)
+    part = torch.randn(max(n_split, 1), B, H, generator=g).to(cuda_device)
+    gamma = (1 + 0.1 * torch.randn(H, generator=g)).to(torch.bfloat16).to(cuda_device)
+    x, x1, h1 = torch.empty(B, H, dtype=torch.bfloat16, device=cuda_device), torch.empty(B, H, dtype=torch.bfloat16, device=cuda_device), h.clone()
+    for r0 in range(0, B, 64):
+        m = min(64, B - r0)
+        few = part[:, r0:r0 + m].contiguous()
+        _lib.check(lib.prl_residual_rmsnorm(few.data_ptr(), n_split, m, H, gamma.data_ptr(), 1e-6, h1[r0:].data_ptr(), x1[r0:].data_ptr(), None, 0,
+                                            _lib.stream_ptr()))
+    _lib.check(lib.prl_residual_rmsnorm(part.data_ptr(), n_split, B, H, gamma.data_ptr(), 1e-6, h.data_ptr(), x.data_ptr(), None, 0,
+                                        _lib.stream_ptr()))
+    assert torch.equal(h, h1) and torch.equal(x, x1)
+
+
+@pytest.mark.parametrize("B,H", [(1, 4), (64, 1024), (300, 3584), (33, 5124)])
+def test_embedding_norm_has_one_order_of_sums(cuda_device, B, H):
+    """Eight-byte pieces and single channels (a table two bytes off): the same bits."""
+    from pipelinerl_b200 import _lib
+    lib, g, V = _lib.load(), torch.Generator().manual_seed(B), 50
+    emb = torch.randn(V, H, generator=g).to(torch.bfloat16).to(cuda_device)
+    off = torch.empty(V * H + 1, dtype=torch.bfloat16, device=cuda_device)[1:].view(V, H)
+    off.copy_(emb)
+    gamma = (1 + 0.1 * torch.randn(H, generator=g)).to(torch.bfloat16).to(cuda_device)
+    tok = torch.randint(0, V, (B,), generator=g).int().to(cuda_device)
+    got = []
+    for e in (emb, off):
+        h, x = torch.empty(B, H, device=cuda_device), torch.empty(B, H, dtype=torch.bfloat16, device=cuda_device)
+        _lib.check(lib.prl_embed_rmsnorm(tok.data_ptr(), e.data_ptr(), gamma.data_ptr(), 1e-6, B, H, V, h.data_ptr(), x.data_ptr(),
+                                         _lib.stream_ptr()))
+        got.append((h, x))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 @pytest.mark.parametrize("B,n_q,n_kv,n_split", [(129, 1, 1, 1), (257, 7, 1, 1), (1300, 28, 4, 1), (140, 5, 5, 3)])
 def test_rope_rows_on_aligned_and_unaligned_buffers(cuda_device, B, n_q, n_kv, n_split):
     """The four-pair form and the pair-by-pair form (queries and cache two bytes off) write the same bits."""
