@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""bench.py — headline measurement of the hot path (contract in the task statement / DESIGN.md §Measurement).
+"""bench.py — headline measurement of the hot path.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
@@ -7,9 +7,9 @@ Metric: rollout tokens/s (the reference's actor/output_tokens_per_second, pipeli
 sampler's token step on random-init Qwen2.5-7B: 64 running sequences per GPU (actor.llm_max_rollouts,
 conf/base.yaml:17,63), synthetic 8192-token prompts already in the paged KV cache, temperature 1.
 A "step" = one token for each of the 64 sequences (one pass of hot path 1).  N > 1: one engine replica per
-GPU (SURVEY §8e: the token step shards as replicas only, no data-path collective) -> weak scaling.
+GPU (the token step shards as replicas only, no data-path collective) -> weak scaling.
 
-Under torchrun (N >= 2) the same run then re-partitions the N GPUs into the actor-learner split of the north star
+Under torchrun (N >= 2) the same run then re-partitions the N GPUs into an actor-learner split
 (`components.pipeline`, tools/split_bench.py): 1+1 at N=2, 3+1 at N=4, 6+2 and 4+4 at N=8 -- samplers keep
 generating while data-parallel learners train and push weights after every optimizer step; rollout tokens/s while
 training, trainer tokens/s and steps/s, DP exchange ms, push ms, STALL ms, `bytes_identical`, `dp_equals_single`.
@@ -35,7 +35,7 @@ from pathlib import Path
 ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
-CONTEXT = 8192          # synthetic prompt tokens per sequence (BASELINE.json configs[1])
+CONTEXT = 8192          # synthetic prompt tokens per sequence
 BATCH = 64              # running sequences per engine (conf/base.yaml:63 max-num-seqs)
 METRIC = "rollout_tokens_per_s"
 UNIT = "tokens/s"
@@ -75,7 +75,7 @@ def parse():
 
 def workload_config(args, n_gpus):
     return {"workload": f"Qwen2.5-7B random-init token step, {args.batch} seqs/GPU x {args.context}-token synthetic "
-                        f"prompts in paged KV, temperature 1.0 (BASELINE.json configs[1], sampler side)",
+                        f"prompts in paged KV, temperature 1.0 (sampler side)",
             "batch_per_gpu": args.batch, "context": args.context, "parallelism": f"replicas x{n_gpus}",
             "lm_head": "fp32-equivalent (bf16 hi + bf16 lo operand streams, vllm_quantization.py:266-278)",
             "l2": "inputs_exceed_l2 (weights 16.3 GB + KV 30 GB read per step)", "cuda_graph": True}
@@ -315,7 +315,7 @@ def run_ours(args):
     if rank == 0 and world == 1 and not args.no_components and not args.no_vllm:
         out.setdefault("components", {})["vllm_baseline"] = vllm_baseline(args)
     if world > 1 and not args.no_components and not args.no_pipeline:
-        # ---- the actor-learner split on the same N GPUs (north star: N inference + (8 - N) learner GPUs) ----
+        # ---- the actor-learner split on the same N GPUs (N inference + (8 - N) learner GPUs) ----
         import gc
         try:
             del eng, attn_all_layers
@@ -337,7 +337,7 @@ def run_ours(args):
 
 
 def default_splits(world: int) -> list[int]:
-    """learner counts per world size: 1+1 (N=2), 3+1 (N=4), 6+2 and 4+4 (N=8: BASELINE.json configs[1] and [2])"""
+    """learner counts per world size: 1+1 (N=2), 3+1 (N=4), 6+2 and 4+4 (N=8)"""
     if world >= 8:
         return [2, 4]
     return [1]

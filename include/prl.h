@@ -2,7 +2,7 @@
  * prl.h — C ABI of libprl.so, the B200 (sm_100a) hot-path library behind the
  * PipelineRL plugin / stream API.
  *
- * Conventions (SURVEY.md §8b):
+ * Conventions:
  *   - plain pointers and sizes only; no torch / C++ types cross this boundary;
  *   - every device buffer is owned by the caller; the library owns only opaque
  *     handles it hands out from *_create and frees in *_destroy;
@@ -237,7 +237,7 @@ int prl_adamw_sharded_reduce(const prl_adamw_shard_args* args, void* workspace, 
 int prl_adamw_sharded_update(const prl_adamw_shard_args* args, float* grad_norm_out, prl_stream_t stream);
 
 /* ======================================================================= *
- * Feeder of hot path (2), GPU-resident (SURVEY §8 f1): one packed micro-batch row built on the learner's GPU from a
+ * Feeder of hot path (2), GPU-resident: one packed micro-batch row built on the learner's GPU from a
  * compact binary record (pipelinerl_b200/records.py) -- replaces populate_rl_data's pandas pipeline
  * (pipelinerl/finetune/rl/__init__.py:453-570), collate_packed's list -> tensor building (finetune/data.py:215-283)
  * and the JSONL round trip of the twelve [1, T] columns (streams.py:269-277, finetune_loop.py:109).
@@ -542,7 +542,7 @@ typedef struct {
 } prl_engine_state;
 int prl_advance_state(const prl_engine_state* state, prl_stream_t stream);
 
-/* ---- tensor parallelism inside one engine (BASELINE config 4: Qwen2.5-32B, TP=2; the reference passes
+/* ---- tensor parallelism inside one engine (Qwen2.5-32B, TP=2; the reference passes
  * tensor-parallel-size to vLLM, world.py:56-59, which all-reduces twice per layer with NCCL/custom all-reduce).
  * Here the row-parallel GEMMs (o_proj, down_proj) store their fp32 partial tiles into the local AND the peer GPU's
  * reduction buffer in their epilogue (prl_gemm_bf16_splitk_peer: the all-reduce is fused into the GEMM over NVLink

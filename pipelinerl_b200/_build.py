@@ -1,8 +1,8 @@
 """In-tree build of libprl.so (hand-written sm_100a CUDA behind the C ABI in include/prl.h).
 
 nvcc cross-compiles for sm_100a without a GPU.  The .so is written next to the
-package (pipelinerl_b200/_lib/libprl.so) so that it travels to the GPU box with
-the repository snapshot; it is git-ignored, never pip-installed.
+package (pipelinerl_b200/_lib/libprl.so) so that it travels with
+a copy of the repository; it is git-ignored, never pip-installed.
 """
 from __future__ import annotations
 

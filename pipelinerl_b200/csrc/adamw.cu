@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kThreads) adamw_kernel(prl_adamw_args a, Updat
 
 
 // =====================================================================================================
-// Learner data parallelism as ONE fused exchange step over NVLink peer memory (SURVEY §8e, row a7):
+// Learner data parallelism as ONE fused exchange step over NVLink peer memory:
 //   reduce-scatter(grad) -> clip -> AdamW on this rank's 1/Ng shard -> all-gather(bf16 params)
 // Every rank maps every other rank's full gradient arena and bf16 parameter arena (CUDA IPC).  Kernel A
 // (shard_reduce) sums the Ng gradients of this rank's shard straight out of peer memory (P2P loads) into an

@@ -1540,7 +1540,8 @@ extern "C" int prl_attn_varlen_bwd_kv(const void* q, int64_t q_stride, int32_t T
   p.seg_pos0 = seg_pos0; p.seg_kv_start = seg_kv_start; p.dkv = (__nv_bfloat16*)dkv; p.dkv_stride = dkv_stride;
   p.dkv_col_k = 0; p.dkv_col_v = n_kv * kD;
   p.n_lin = n_kv * n_seg;
-  p.split = 1;                   // one CTA per key tile: the split's rule is about whole sequences
+  p.split = 1;                   // one CTA per key tile: the split's cost counts a causal triangle, but a slice's queries all see every
+                                 // key of the ranks before it; no rule has been measured for that
   CUtensorMap tkv, tq, tdo;
   int rc = make_tmap_2d_bf16(&tkv, kv, (uint64_t)kvw, (uint64_t)Tkv, (uint64_t)kv_stride * 2, 64, 64);
   if (rc) return rc;

@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(64) qkv_rope_cache_kernel(const float* __restr
 
 // Same arithmetic, laid out for MANY rows (prefill chunks): one block walks whole token rows, the row's 64
 // (cos, sin) pairs are computed once (the per-head kernel above recomputes them for each of the n_q + 2 n_kv heads)
-// and every thread handles (head, W neighbouring pairs) items: W = 4 on 16-byte aligned buffers (1024 rows of 36 heads: 12.1 us
+// and every thread handles (head, W neighbouring pairs) items: W = 4 on fp32 aligned to 16 and bf16 to 8 bytes (1024 rows of 36 heads: 12.1 us
 // with a pair per item).  Bitwise identical results.
 template <int W>
 __global__ void __launch_bounds__(256) qkv_rope_cache_rows_kernel(const float* __restrict__ part, int n_split, int B,

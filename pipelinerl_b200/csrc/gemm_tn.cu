@@ -208,8 +208,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
   const uint32_t rank = ptx::cluster_ctarank();
   const int n_clusters = (int)gridDim.x >> 1;
   const int cluster = (int)blockIdx.x >> 1;
-  // Programmatic launch: barriers, tensor memory and tensor maps are set up under the tail of the kernel before (about 4 of the
-  // 10 us that a launch takes beside its main loop); nothing it wrote, and nothing it still reads, is touched before pdl_wait
+  // Programmatic launch: barriers, tensor memory and tensor maps are set up under the tail of the kernel before (1.1 of the 17.7 us
+  // of a 1024 x 2048 launch, K = 2048); nothing it wrote, and nothing it still reads, is touched before pdl_wait
   pdl_launch_dependents();
 
   if (threadIdx.x == 0) {
@@ -644,7 +644,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
       }
       }
       }  // !kHead
-      // this CTA's four epilogue warps are done with the accumulator -> tell the leader's MMA warp
+      // this CTA's epilogue warps are done with the accumulator -> tell the leader's MMA warp
       ptx::tc_fence_before_sync();
       asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps<kHead>) : "memory");
       if (threadIdx.x == 64) {

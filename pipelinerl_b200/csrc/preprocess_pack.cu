@@ -1,4 +1,4 @@
-// GPU-resident preprocess (SURVEY §8 f1): rollout samples -> RL columns -> ONE packed micro-batch row, on the learner's
+// GPU-resident preprocess: rollout samples -> RL columns -> ONE packed micro-batch row, on the learner's
 // GPU, from a compact binary record (pipelinerl_b200/records.py) -- replaces the pandas pipeline of
 // populate_rl_data (pipelinerl/finetune/rl/__init__.py:453-570), the Python-list collate_packed
 // (finetune/data.py:215-283) and the JSONL round trip of twelve [1, T] tensors (streams.py:269-277,

@@ -1,7 +1,7 @@
-"""Synthetic single-turn domain for the BASELINE configs 2-4 (random-init model, synthetic prompts).
+"""Synthetic single-turn domain for the 7B and 32B workloads (random-init model, synthetic prompts).
 
 Same plugin surface as a real domain (cf. pipelinerl/domains/math/rollouts.py:58-149): one LLM call per
-rollout on a fixed token-id prompt, reward ~ Bernoulli(0.5) seeded per (problem, attempt) as SURVEY §8d
+rollout on a fixed token-id prompt, reward ~ Bernoulli(0.5) seeded per (problem, attempt)
 prescribes (random-init weights never solve anything, so the reward must be synthetic).
 """
 from __future__ import annotations

@@ -1,4 +1,4 @@
-"""Checkpoint / resume of the learner in safetensors (SURVEY §8 f4; reference: pipelinerl/finetune/checkpoints.py).
+"""Checkpoint / resume of the learner in safetensors (reference: pipelinerl/finetune/checkpoints.py).
 
 Same entry points and on-disk discipline as the reference:
   save_model_only(output_dir, ...)            :388-445   HF-named weights a sampler / HF / vLLM can load

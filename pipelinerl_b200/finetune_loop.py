@@ -43,7 +43,7 @@ class TrainerConfig:
 
 def allreduce_gradients(flat_grad: torch.Tensor, group=None) -> None:
     """Learner data parallelism: ONE sum all-reduce of the flat gradient arena per optimizer step — the only
-    collective on the hot path (SURVEY §2c C4; the reference's DDP/ZeRO traffic at finetune_loop.py:716-755).
+    collective on the hot path (the reference's DDP/ZeRO traffic at finetune_loop.py:716-755).
     A plain SUM is exact because every rank's loss is already normalised by the GLOBAL samples-per-step
     (rl/__init__.py:250, finetune_loop.py:644-646).  NCCL over NVLink on GPUs, gloo in the CPU tests."""
     import torch.distributed as dist

@@ -3,7 +3,7 @@
 The reference's actor reaches its sampler over HTTP (vLLM's OpenAI-compatible server started by
 pipelinerl/launch.py:191-247 / vllm1.py:189-273).  On one box this package talks to the engine in process
 (serving.py), but REMOTE reference actors — or an unmodified `pipelinerl.async_llm.llm_async_generate` — can be pointed
-at this shim instead of a vLLM server (SURVEY §8b "wire format"):
+at this shim instead of a vLLM server:
 
   POST /v1/chat/completions   request fields the reference sends (async_llm.py:96-131): model, messages, logprobs,
                               include_stop_str_in_output, skip_special_tokens, tools?, max_tokens?, chat_template_kwargs?

@@ -71,7 +71,7 @@ class ModelConfig:
 
     @staticmethod
     def tiny(**kw) -> "ModelConfig":
-        """Plumbing / parity-test model (config 1 of BASELINE.json is not defined by the reference)."""
+        """Plumbing / parity-test model (the reference defines none of this size)."""
         base = dict(vocab_size=512, hidden_size=256, intermediate_size=640, num_layers=2, num_q_heads=4,
                     num_kv_heads=2)
         base.update(kw)

@@ -1,4 +1,4 @@
-"""Binary micro-batch records and the GPU-resident preprocess (SURVEY §8 f1).
+"""Binary micro-batch records and the GPU-resident preprocess.
 
 The reference moves training data as JSON: the preprocessor serialises twelve `[1, T]` tensors per micro-batch to a JSONL
 line (pipelinerl/streams.py:269-277, ~170 bytes per token) and the trainer parses and validates it back

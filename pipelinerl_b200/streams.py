@@ -7,7 +7,7 @@ Public API of the reference kept as is (pipelinerl/streams.py:33-69, 390-423):
     with read_stream(spec) as r: for x in r.read(): ...      (blocking tail from the beginning)
 File layout <exp>/streams/<topic>/<instance>/<partition>/0.jsonl (:238-243), one JSON object per
 line, flushed per write; pydantic models, tensors and numpy arrays are serialised as plain lists.
-Redis is a deployment option of the reference, outside the hot path (SURVEY §2a #10).
+Redis is a deployment option of the reference, outside the hot path.
 """
 from __future__ import annotations
 

@@ -1,4 +1,4 @@
-"""Tensor-parallel sampler engine (BASELINE config 4: Qwen2.5-32B, TP=2 inference).
+"""Tensor-parallel sampler engine (Qwen2.5-32B, TP=2 inference).
 
 One process per GPU, SPMD: every rank of a TP group runs the same admission / step sequence (a serving
 deployment would broadcast the leader's scheduling decisions; tests and the bench drive the ranks in lockstep).
@@ -59,7 +59,7 @@ class TPDecodeEngine(DecodeEngine):
             self._peer_bufs += [bp, bs, bf]
             self._peer_part[r], self._peer_samp[r], self._peer_flag[r] = bp.ptr, bs.ptr, bf.ptr
         if self.tp != 2:
-            raise NotImplementedError("peer-store epilogue currently targets one peer (tp=2, BASELINE config 4)")
+            raise NotImplementedError("peer-store epilogue currently targets one peer (tp=2)")
         self.peer = 1 - tp_rank
         self._eager_done: set[int] = set()
         self.signals_per_step = 2 * cfg.num_layers + 1

@@ -1,11 +1,10 @@
 """Generate golden fixtures by EXECUTING the reference (ServiceNow/PipelineRL) on fixed seeds.
 
-Run in the authoring container only (needs /root/reference, which does not exist
-on the GPU box):
+Needs the reference's sources in /root/reference:
 
     python tests/golden/make_golden.py
 
-The reference has no tests / golden vectors of its own (SURVEY.md §4, §8c), so
+The reference has no tests / golden vectors of its own, so
 these fixtures are what pins oracle/ (and through it the CUDA kernels) to the
 reference's behaviour.  Outputs: tests/golden/*.npz + *.json (small, committed).
 
@@ -240,7 +239,7 @@ def gen_preprocess_cases(ref_rl, ref_data, ref_utils):
 
 
 def gen_preprocess_large_cases(ref_rl, ref_data, ref_utils):
-    """Big groups (64 attempts, BASELINE config 5), real-valued rewards, two steps per rollout (multi-turn: several
+    """Big groups (64 attempts), real-valued rewards, two steps per rollout (multi-turn: several
     samples share a rollout_index) and unfinished samples without finish_reason: exercises pandas' Kahan sum / Welford std
     beyond what 4-member groups can, and the "eos in input_ids" overflow rule."""
     out = {}

@@ -7,7 +7,7 @@ statement is cut out of the reference file with ast and exec'd in a namespace ho
 reference sets up at :463-483, the reference's own `collate_packed`, `create_sentinel_batch` and
 `write_micro_batch_slices`, and a recording `data_writer`.  The statements that run are the reference's.
 
-    python tests/golden/make_golden_dealer.py      (authoring container only)
+    python tests/golden/make_golden_dealer.py
 
 Recorded (tests/golden/dealer_cases.json): per scenario the entries fed (in arrival chunks) and every write in order:
 target rank, sentinel flag, and the full micro-batch columns."""

@@ -1,7 +1,7 @@
 """Golden fixtures for the token step: HF transformers' Qwen2ForCausalLM (what the reference's trainer
 runs, finetune/checkpoints.py:151-222) in fp32 on bf16-valued weights.
 
-    python tests/golden/make_golden_decode.py      (authoring container; needs transformers only)
+    python tests/golden/make_golden_decode.py      (needs transformers only)
 
 Weights are NOT stored: tests regenerate them with tests.helpers.tiny_weights (CPU torch RNG, seed 42).
 Stored: teacher-forced logprobs of a fixed 150-token sequence and the full logits of its last 4 positions.

@@ -2,7 +2,7 @@
 (its source is cut out of the reference file with ast and exec'd, because importing pipelinerl.preprocess pulls in
 packages that are not installed here) on synthetic grouped entries.
 
-    python tests/golden/make_golden_filter.py      (authoring container only)
+    python tests/golden/make_golden_filter.py
 """
 import ast
 import json

@@ -1,7 +1,7 @@
 """Interop recording for the HTTP shim: the REFERENCE's client (pipelinerl/async_llm.py:86-212, executed from
 /root/reference) talks to pipelinerl_b200.http_shim.HttpShim (fake engine of tests/test_http_shim.py) over loopback.
 
-    python tests/golden/make_golden_http_shim.py      (authoring container only)
+    python tests/golden/make_golden_http_shim.py
 
 Stored in tests/golden/http_shim_interop.json: the payload the reference sent, the shim's response, and the LLMCall
 fields the reference parsed from it.  litellm / jsonref / accelerate / omegaconf are stubbed as in

@@ -10,7 +10,7 @@ out of the reference file with ast and exec'd / eval'd in a namespace holding a 
 One tick of the script = one iteration of the reference's outer loop: the version block once, then submit attempts until
 blocked (the reference's inner `while True`).  The statements that run are the reference's.
 
-    python tests/golden/make_golden_lag_budget.py      (authoring container only)
+    python tests/golden/make_golden_lag_budget.py
 
 Recorded (tests/golden/lag_budget_cases.json): per case the configuration, the ticks, and after every tick the number of
 groups submitted in it, the running total and `can_submit_before_update`."""

@@ -3,7 +3,7 @@ driving HF transformers' `Qwen2ForCausalLM` (the model class the reference train
 fp32 on CPU, on one packed micro-batch; loss, the 32 statistics, the per-token new logprobs and the gradient of
 EVERY parameter.
 
-    python tests/golden/make_golden_learner.py      (authoring container: needs /root/reference + transformers)
+    python tests/golden/make_golden_learner.py      (needs /root/reference and transformers)
 
 Packed rows: on GPUs the reference reaches block-diagonal causal attention through flash-attn's varlen path, which HF
 selects from `position_ids` that restart per sample (conf/finetune/base.yaml attn_implementation=flash_attention_2).

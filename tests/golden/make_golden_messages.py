@@ -3,7 +3,7 @@ reference's pydantic classes and its `TrainerMessage` union (cut out of the refe
 dumps of this package's message classes (pipelinerl_b200/weights.py), as `TrainerState.start_listening` does
 (pipelinerl/state.py:35-47).  Recorded: each dump, and the reference class + fields it was parsed into.
 
-    python tests/golden/make_golden_messages.py      (authoring container only)
+    python tests/golden/make_golden_messages.py
 """
 import ast
 import json

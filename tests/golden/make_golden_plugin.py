@@ -4,7 +4,7 @@ llm_async_generate, make_training_text`, `from pipelinerl.llm import Prompt, Tra
 import BaseMetrics, RolloutResult` are resolved to pipelinerl_b200's modules (what "switching the package" means for a
 plugin author).  The sampler behind it is a scripted fake registered under an inproc:// address.
 
-    python tests/golden/make_golden_plugin.py      (authoring container only)
+    python tests/golden/make_golden_plugin.py
 
 Stored in tests/golden/plugin_guessing.json: per scenario the messages of every LLM call the reference plugin made and
 the RolloutResult it returned; tests/test_host_logic.py::test_guessing_plugin_matches_reference_plugin replays the same

@@ -1,7 +1,7 @@
 """Golden for the rollout record types (pipelinerl/rollouts.py:6-110): the reference classes and helpers are imported
 (pydantic only) and their dumps / derived values recorded; tests build the same objects with pipelinerl_b200.rollouts.
 
-    python tests/golden/make_golden_rollouts.py      (authoring container only)
+    python tests/golden/make_golden_rollouts.py
 """
 import json
 import sys

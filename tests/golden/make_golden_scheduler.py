@@ -3,7 +3,7 @@ rollout policy, scripted queues and a scripted trainer state.  The function's so
 with ast and exec'd in a namespace that provides the names it uses (importing pipelinerl.actor pulls in wandb, hydra,
 uvloop ... which are not installed here); the body that runs is the reference's.
 
-    python tests/golden/make_golden_scheduler.py      (authoring container only)
+    python tests/golden/make_golden_scheduler.py
 
 Recorded (tests/golden/scheduler_case.json): the launch order with the LLM each rollout was routed to (least-busy
 routing, :268-273), and for every finished group the stamping the downstream stages rely on (:207-219): group id

@@ -2,7 +2,7 @@
 `set_streams_backend("files")`, `write_to_streams(SingleStreamSpec | StreamRangeSpec)`, round-robin and explicit
 partition writes, BaseModel / tensor payloads.
 
-    python tests/golden/make_golden_streams.py      (authoring container only)
+    python tests/golden/make_golden_streams.py
 
 orjson and redis are not installed here.  redis is never touched by the file backend; orjson is replaced by a stand-in
 built on `json` (compact separators, numpy arrays as lists), so what this fixture pins is the PROTOCOL — directory layout

@@ -4,7 +4,7 @@ message classes, in the order `run_training` / `WeightUpdateManager` emit them),
 `TrainerMessage` union (finetune_loop.py:138-171) and this package's stream reader standing in for `pipelinerl.streams`
 (whose file format is pinned separately by make_golden_streams.py).
 
-    python tests/golden/make_golden_trainer_state.py      (authoring container only)
+    python tests/golden/make_golden_trainer_state.py
 
 Recorded: the topic file and the state the reference listener ended up in; tests replay the same file through
 pipelinerl_b200.state.TrainerState.

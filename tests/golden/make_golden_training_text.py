@@ -1,7 +1,7 @@
 """Golden fixture for row a2: the reference's `make_training_text` (pipelinerl/async_llm.py:215-346) executed on a
 locally built chat tokenizer (tests.helpers.tiny_chat_tokenizer: no files, no network).
 
-    python tests/golden/make_golden_training_text.py      (authoring container: needs /root/reference)
+    python tests/golden/make_golden_training_text.py      (needs /root/reference)
 
 litellm and jsonref (third-party, not installed here) are only used by the reference for type aliases / schema
 helpers on this path and are stubbed; the function body that runs is the reference's.

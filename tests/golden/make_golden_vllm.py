@@ -2,7 +2,7 @@
 pyproject.toml:22; the image ships 0.22.0 with FlashInfer sm_100) loaded with the SAME tiny bf16 weights the parity
 tests use (tests.helpers.tiny_weights), on a GPU:
 
-    gpurun -- python tests/golden/make_golden_vllm.py gpurun_out/vllm_golden       (GPU box only: vLLM needs libcuda)
+    python tests/golden/make_golden_vllm.py vllm_golden       (on a GPU: vLLM needs libcuda)
 
 Recorded per model kind (gqa2: 4q/2kv heads, gqa7: Qwen2.5-7B's 7:1 grouping) into vllm_tiny_<kind>.json:
   * greedy continuations (temperature 0) of fixed prompts with the logprob vLLM reports for every sampled token
@@ -49,7 +49,7 @@ def write_checkpoint(kind: str, d: str):
 
 
 def main():
-    out_dir = Path(sys.argv[1] if len(sys.argv) > 1 else "gpurun_out/vllm_golden")
+    out_dir = Path(sys.argv[1] if len(sys.argv) > 1 else "vllm_golden")
     out_dir.mkdir(parents=True, exist_ok=True)
     import vllm
     from vllm import LLM, SamplingParams

@@ -3,7 +3,7 @@
 The op: block-diagonal causal attention over one packed row -- what the reference gets from flash-attn varlen
 through HF when `position_ids` restart per packed sample (pipelinerl/finetune/rl/__init__.py:204,
 conf/finetune/base.yaml:12-13,64).  Reference here: plain fp32 softmax(Q K^T / sqrt(d) + causal mask) V per segment and
-head with torch autograd, on the same bf16-representable inputs.  Bar (VERDICT r1 item 1): every output / gradient
+head with torch autograd, on the same bf16-representable inputs.  Bar: every output / gradient
 element within 2^-7 of the tensor's scale (bf16 P / dS operands + bf16 result rounding); the measured maxima are printed.
 The backward must also be bitwise reproducible (fixed-order GQA reduction, no atomics)."""
 import math

@@ -119,7 +119,7 @@ def test_sampling_distribution_and_logprob_capture(cuda_device):
 
 
 def test_paged_attention_long_context_vs_fp32(cuda_device):
-    """Decode attention alone at BASELINE-like context (8192+ tokens, 7:1 GQA, ragged lengths, scattered pages)."""
+    """Decode attention alone at long context (8192+ tokens, 7:1 GQA, ragged lengths, scattered pages)."""
     from pipelinerl_b200 import _lib
     lib = _lib.load()
     dev = cuda_device
@@ -259,7 +259,7 @@ def test_prefill_attention_long_context_vs_fp32(cuda_device, kernel, n_q, n_kv, 
 
 
 def test_kv_reuse_across_turns(cuda_device):
-    """Multi-turn rollouts (BASELINE config 5): turn 2's prompt = turn 1's prompt + answer + new message; every
+    """Multi-turn rollouts: turn 2's prompt = turn 1's prompt + answer + new message; every
     full page of the common prefix is reused from the cache even after turn 1 finished."""
     from pipelinerl_b200.engine import SamplingParams
     cfg = tiny_cfg("gqa2")
@@ -300,7 +300,7 @@ def test_score_reference_logprobs(cuda_device, kind):
 
 def test_per_request_sampling_parameters_share_one_batch(cuda_device):
     """Requests admitted with different temperature / greedy settings decode in the same batch and each one's sampled
-    logprob is log_softmax(logits / ITS temperature) at ITS sampled id (sampling params were engine-global)."""
+    logprob is log_softmax(logits / ITS temperature) at ITS sampled id (sampling parameters belong to a request, not to the engine)."""
     from pipelinerl_b200.engine import SamplingParams
     cfg = tiny_cfg("gqa2")
     w = tiny_weights(cfg)
@@ -343,7 +343,7 @@ def test_engine_matches_vllm_golden(cuda_device, kind):
     import json
     f = GOLDEN / f"vllm_tiny_{kind}.json"
     if not f.exists():
-        pytest.skip("vLLM golden not recorded yet (needs a GPU box: tests/golden/make_golden_vllm.py)")
+        pytest.skip("vLLM golden not recorded yet (tests/golden/make_golden_vllm.py, on a GPU)")
     gold = json.loads(f.read_text())
     cfg = tiny_cfg(kind)
     w = tiny_weights(cfg)
@@ -374,7 +374,7 @@ def test_one_layer_qwen7b_width_decode_step_vs_oracle(cuda_device):
     decode step (tcgen05 split-K GEMMs, RoPE + KV write, paged attention, residual RMSNorm, SiLU, fp32-equivalent head)
     against the oracle on identical bf16-valued weights and the same rounding points: with a single layer there is no
     chain of bf16 re-roundings to amplify summation-order noise.  Measured on a B200: mean relative |dlogprob| 4.7e-4, max
-    1.39e-3 (one position of 47) -- the mean meets the north star's 1e-3, the max is bounded at 1.5 x measured."""
+    1.39e-3 (one position of 47) -- the mean meets 1e-3, the max is bounded at 1.5 x measured."""
     from dataclasses import replace
     from pipelinerl_b200.engine import SamplingParams
     from pipelinerl_b200.model import ModelConfig

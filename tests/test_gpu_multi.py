@@ -1,5 +1,5 @@
-"""Cross-process, cross-GPU weight update (CUDA IPC + NVLink P2P).  Needs >= 2 GPUs: skipped on the
-single-GPU test box, run with `gpurun --gpus 2`."""
+"""Cross-process, cross-GPU weight update (CUDA IPC + NVLink P2P).  Needs >= 2 GPUs: skipped
+where there is one."""
 import json
 import os
 import subprocess

@@ -1,6 +1,6 @@
 """Parity of the CUDA PG-loss path (through the C ABI / rl_step facade) with the oracle and with the
-reference's own outputs (golden fixtures).  Tolerances: loss / logprobs / stats 1e-4 relative
-(north star asks for 1e-3); gradients 1e-4 relative + 1e-7 absolute."""
+reference's own outputs (golden fixtures).  Tolerances: loss / logprobs / stats 1e-4 relative;
+gradients 1e-4 relative + 1e-7 absolute."""
 import numpy as np
 import pytest
 import torch
@@ -126,7 +126,7 @@ def test_nonfinite_is_reported(cuda_device):
 
 
 def test_large_row_properties(cuda_device):
-    """Size-independent properties at a BASELINE-scale packed row (T = 16384 tokens x vocab 152064 would be
+    """Size-independent properties at a full-size packed row (T = 16384 tokens x vocab 152064 would be
     10 GB of logits; the loss tail itself is tested at T = 2^20 through the C ABI directly)."""
     import ctypes as C
     from pipelinerl_b200 import _lib

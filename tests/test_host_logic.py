@@ -416,7 +416,7 @@ def test_model_checkpoint_roundtrip_hf_names(tmp_path):
 
 
 def test_tokenizer_is_never_silently_substituted():
-    """a missing / misspelt tokenizer must raise; the synthetic tokenizer is used only when asked for by name or
+    """A missing / misspelt tokenizer must raise; the synthetic tokenizer is used only when asked for by name or
     injected (the reference resolves `tokenizer_name` through AutoTokenizer, llm.py:366-374)."""
     from pipelinerl_b200.llm import SyntheticTokenizer, TrainableLLM
     assert isinstance(TrainableLLM("inproc://x", "m", tokenizer_name="synthetic").load_tokenizer(), SyntheticTokenizer)

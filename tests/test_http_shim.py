@@ -1,6 +1,6 @@
 """HTTP shim (pipelinerl_b200/http_shim.py) over a FAKE engine: wire format of the reference's vLLM server.
 
-tests/golden/http_shim_interop.json was recorded in the authoring container by pointing the REFERENCE's own client
+tests/golden/http_shim_interop.json was recorded by pointing the REFERENCE's own client
 (`pipelinerl.async_llm.llm_async_generate`, async_llm.py:86-212) at this shim (make_golden_http_shim.py): it holds the
 request payload the reference sent, the response the shim gave and the LLMCall fields the reference parsed out of it.
 Here the same payload is replayed: the response must be the recorded one (so what the reference accepted stays what the

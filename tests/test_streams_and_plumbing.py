@@ -337,7 +337,7 @@ def test_trainer_messages_are_what_the_reference_parses():
 
 
 def test_config1_plumbing_end_to_end_on_cpu(tmp_path):
-    """BASELINE configs[0]-style plumbing run without a GPU: the guessing plugin on a scripted sampler -> scheduler with
+    """Plumbing run without a GPU: the guessing plugin on a scripted sampler -> scheduler with
     groups of 4 -> `actor` topic on the file stream backend -> preprocess (RL columns, leave-one-out advantages) ->
     packed micro-batches -> the ORACLE learner (oracle/learner_oracle + pg_oracle: the CPU stand-in for the CUDA hot
     path) -> AdamW oracle.  Everything between the sampler and the loss is this package's host code."""

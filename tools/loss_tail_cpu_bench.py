@@ -1,11 +1,11 @@
 #!/usr/bin/env python
-"""CPU timing of the finetune loss tail (SURVEY §8d "Reference CPU path timing", item 2): `rl_step` on a stub model
+"""CPU timing of the finetune loss tail: `rl_step` on a stub model
 that returns fixed random fp32 logits [1, T, 152064] (T = 2048 to fit RAM; the tail is linear in T).
 
     python tools/loss_tail_cpu_bench.py [--tokens 2048] [--reference /root/reference]
 
 Times (a) the REFERENCE's own rl_step (pipelinerl/finetune/rl/__init__.py:136-450) when the reference tree is
-importable (authoring container), (b) the oracle port (oracle/pg_oracle.py) — forward+backward, all host threads.
+importable, (b) the oracle port (oracle/pg_oracle.py) — forward+backward, all host threads.
 One JSON line: microseconds per token for each, next to the GPU kernels' numbers quoted from bench.py components.
 """
 import argparse

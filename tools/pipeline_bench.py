@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""All three hot paths at once on Qwen2.5-7B (BASELINE.json configs[1] shape, reduced to the GPUs at hand):
+"""All three hot paths at once on Qwen2.5-7B (reduced to the GPUs at hand):
 
     python -m torch.distributed.run --nnodes=1 --nproc-per-node N --master-addr 127.0.0.1 --master-port P \
         tools/pipeline_bench.py [--updates 3] [--context 8192] [--batch 64]

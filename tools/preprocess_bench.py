@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """CPU feeder of hot path 2 (rows a4/a5): reference pandas/python-list pipeline vs this repo's host code on
-identical inputs (groups of 8 samples x 16384 tokens).  Run in the authoring container (needs
-/root/reference for the reference arm; elsewhere only ours + the oracle port are timed).
+identical inputs (groups of 8 samples x 16384 tokens).  Needs
+/root/reference for the reference arm; elsewhere only ours + the oracle port are timed.
 
     python tools/preprocess_bench.py [--groups 4]
 """

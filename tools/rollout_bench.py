@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Full rollouts through the plugin API on one B200 (sampler side, NOT a static-state microbench):
+"""Full rollouts through the plugin API on one B200 (64 sequences of Qwen2.5-7B, sampler side, NOT a static-state microbench):
 
     generate_synthetic_rollout -> llm_async_generate -> EngineServer thread -> chunked prefill (1024-token chunks, the
     prompt shared by the 8 attempts of a GRPO group prefilled ONCE: page-hash prefix cache) -> decode with the context

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""The actor-learner split of BASELINE.json configs[1]/[2] on one box: `--learners M` learner GPUs (data-parallel
+"""The actor-learner split of Qwen2.5-7B on one box: `--learners M` learner GPUs (data-parallel
 NativeQwen2, gradients exchanged by ShardedFusedAdamW over NVLink peer memory) + the remaining ranks as samplers
 (DecodeEngine token steps that never pause), one in-flight weight update after EVERY optimizer step with the arena's byte
 range split across the learner ranks (every learner pushes its slice to every sampler).
@@ -7,8 +7,8 @@ range split across the learner ranks (every learner pushes its slice to every sa
     python -m torch.distributed.run --nnodes=1 --nproc-per-node N --master-addr 127.0.0.1 --master-port P \
         tools/split_bench.py --learners M [--updates 2] [--context 8192] [--batch 64]
 
-`run_split()` is also what bench.py calls under torchrun (components.pipeline), so the numbers land in the driver's
-BENCH / SCALE records.  Reported by rank 0:
+`run_split()` is also what bench.py calls under torchrun (components.pipeline), so the numbers land in its
+JSON line.  Reported by rank 0:
   rollout tokens/s summed over the samplers WHILE the learners train and push, trainer tokens/s and optimizer steps/s
   (batch stated), DP exchange ms (reduce-scatter / update+all-gather phases), push ms (max over learners), stall ms per
   update (slowest token step around a flip minus the median step, max over samplers), `bytes_identical` (every sampler's

@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Tensor-parallel sampler engine (TP=2) on a 2-GPU box: parity check on a tiny model, or the token-step bench for
-random-init Qwen2.5-32B (BASELINE config 4) with 64 sequences x 8192-token synthetic context.
+random-init Qwen2.5-32B with 64 sequences x 8192-token synthetic context.
 
     torchrun --nproc-per-node 2 tools/tp_bench.py --check
     torchrun --nproc-per-node 2 tools/tp_bench.py [--model 32b] [--steps 20]

@@ -3,7 +3,7 @@
 the image ships 0.22, the reference pins 0.18.1) on random-init Qwen2.5-7B, 64 sequences x 8192-token synthetic
 prompts, temperature 1, logprobs on, prefix caching off, 1024-token chunked prefill (conf/base.yaml:59-73).
 Decode tokens/s = 64 * (N2 - N1) / (T(N2 new tokens) - T(N1 new tokens)), which cancels prefill.
-NOT part of the product path: a library baseline for SURVEY §8d / BASELINE.md B4.  One JSON line."""
+NOT part of the product path: a library baseline.  One JSON line."""
 import json
 import os
 import sys
