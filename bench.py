@@ -119,7 +119,7 @@ class ClockSampler:
 
 def ncu_traffic_bytes(algorithmic_bytes: int):
     """DRAM bytes per launch of the dominant kernel from the committed `ncu --set full` capture
-    (profiles/r1_attn_full_raw.csv: dram__bytes_read.sum 1.08266 GB + dram__bytes_write.sum 0.9 MB at B=64, S=8240 -> ratio
+    (profiles/r1_summary.md: dram__bytes_read.sum 1.08266 GB + dram__bytes_write.sum 0.9 MB at B=64, S=8240 -> ratio
     to the algorithmic bytes 1.0004), scaled to the bytes of the launch timed here."""
     f = ROOT / "profiles" / "ncu_traffic.json"
     try:
@@ -281,7 +281,7 @@ def run_ours(args):
     roofline = {"kernel": "paged_attn_decode_kernel(+combine)", "bound": "hbm", "achieved": round(achieved, 1),
                 "peak": peak, "peak_source": peak_src, "unit": "GB/s", "frac": round(achieved / peak, 4),
                 "traffic": ncu_traffic_bytes(kv_bytes), "traffic_source": "ncu --set full dram__bytes_read.sum + "
-                "dram__bytes_write.sum of this kernel (profiles/r1_attn_full_raw.csv: read 1.0004 x, read+write 1.0046 x algorithmic), scaled to this launch",
+                "dram__bytes_write.sum of this kernel (profiles/r1_summary.md: read 1.0004 x, read+write 1.0046 x algorithmic), scaled to this launch",
                 "launch_ms": round(attn_ms, 4), "algorithmic_bytes_per_launch": kv_bytes,
                 "share_of_step": round(attn_ms * cfg.num_layers / (ms / args.steps), 4),
                 "whole_step": {"algorithmic_bytes": step_bytes,
