@@ -465,6 +465,8 @@ int prl_attn_set_prefill_generation(int32_t generation);
 /* backward kernels: 2 (default) = P^T / dS^T / dS reach the tensor core through TMEM (A operand in tensor memory);
  * 1 = through shared memory.  For A/B runs and tests. */
 int prl_attn_set_bwd_generation(int32_t generation);
+/* CTAs (1, 2, 4 or 8) that prl_attn_varlen_bwd lets share the queries of a key tile, from what the host knows of the row */
+int prl_attn_bwd_split(int32_t T, int32_t max_seg_len, int32_t n_seg, int32_t n_q, int32_t n_kv);
 size_t prl_attn_varlen_bwd_workspace_bytes(int32_t T, int32_t n_q);
 int prl_attn_varlen_bwd(const void* qkv_bf16, int64_t qkv_stride, int32_t T, const int32_t* seg_start,
                         const int32_t* seg_len, int32_t n_seg, int32_t max_seg_len, int32_t n_q, int32_t n_kv,

@@ -1355,11 +1355,13 @@ extern "C" int prl_attn_debug_bwd_timing_dkdv(int64_t* out16_device) {
 }
 
 // CTAs per key tile of the generation-4 dK / dV kernel: the fewest microseconds of a model with 0.92 us per step (128 keys x 64
-// query rows) and 8 us around a CTA's steps, over the longest CTA and over the work of all of them spread on the SMs.  The tokens'
-// split into sequences is known on the device only: T tokens in sequences of at most `longest` are taken as the bound that they
-// are.  Whole backward, one CTA per tile -> the rule's choice: 28 / 4 heads, samples of 2049, 1500 and 547: 334 -> 246 us (2);
-// 14 / 2 heads, longest of six samples 2300: 323 -> 208 (4); 16 / 1 heads, 5000 and 300: 1219 -> 442 (4); 28 / 4, 8192: 1405 ->
-// 1370 (1); 16384: one CTA, whose tiles fill the chip three times (2: +2 %, 4: +11 %).
+// query rows) and 8 us around a CTA's steps, over the longest CTA and over the work of all of them spread on the SMs, and 2.5 + s us
+// for the start and the sums of a cluster of s: samples of 20 to 80 tokens took 3 to 10 us more without that term (28 / 4 heads, 40
+// tokens: 19.5 us with one CTA, 23.3 with four; 4 / 4, 80: 17.3, 27.2 with eight).  The tokens' split into sequences is known on the
+// device only: T tokens in sequences of at most `longest` are taken as the bound that they are.  Whole backward, one CTA per tile ->
+// the rule's choice: 28 / 4 heads, samples of 2049, 1500 and 547: 334 -> 246 us (2); 14 / 2 heads, longest of six samples 2300:
+// 323 -> 208 (4); 16 / 1 heads, 5000 and 300: 1219 -> 442 (8); 28 / 4, 8192: 1405 -> 1370 (2); 16384: one CTA, whose tiles fill the
+// chip three times (2: +2 %, 4: +11 %).
 static int dkdv_split(int64_t T, int64_t longest, int n_seg, int n_kv, int nq) {
   const double steps = (double)n_kv * (double)T * (double)longest / (256.0 * nq), tiles = (double)n_kv * ((double)T / 128 + n_seg);
   int best = 1;
@@ -1367,10 +1369,15 @@ static int dkdv_split(int64_t T, int64_t longest, int n_seg, int n_kv, int nq) {
   for (int s = 1; s <= 8; s *= 2) {
     const double path = (double)longest / nq / s * 0.92 + 8.0;
     const double all = (steps * 0.92 + tiles * s * 8.0) / num_sms();
-    const double us = path > all ? path : all;
+    const double us = (path > all ? path : all) + (s > 1 ? 2.5 + s : 0.0);
     if (s == 1 || us < 0.9 * best_us) { best = s; best_us = us; }
   }
   return best;
+}
+extern "C" int prl_attn_bwd_split(int32_t T, int32_t max_seg_len, int32_t n_seg, int32_t n_q, int32_t n_kv) {
+  PRL_CHECK_ARG(T >= 1 && n_seg >= 1 && max_seg_len >= 1 && n_kv >= 1 && n_q % n_kv == 0 && n_q / n_kv >= 1 && n_q / n_kv <= 64,
+                "prl_attn_bwd_split: bad shape");
+  return dkdv_split(T, max_seg_len, n_seg, n_kv, 64 / (n_q / n_kv));
 }
 template <bool kTimed>
 static cudaError_t launch_dkdv4(dim3 grid, cudaStream_t stream, const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap& tkv,
