@@ -127,7 +127,7 @@ __device__ __forceinline__ void tile_coords(int t, const TnParams& p, int& tm, i
 // ---- epilogue staging -------------------------------------------------------------------------------------------------------
 // tcgen05.ld hands a thread one output ROW, so stores straight from the registers touch 32 rows per instruction and every
 // access is a sector of its own: the fp32 accumulate epilogue (152064 x 3584, K = 2048) took 3.02 ms against 1.4 ms of
-// products, 1.76 ms now.  A warp therefore turns each 32-column chunk through its own shared memory (no barrier across warps):
+// products, 1.69 ms now.  A warp therefore turns each 32-column chunk through its own shared memory (no barrier across warps):
 // rows go in as 16-byte pieces under an XOR swizzle (conflict-free both ways) and come out with 8 lanes on one row's 128
 // bytes, so residual, accumulated and stored values move in whole lines.
 __device__ __forceinline__ void sts16(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
@@ -170,16 +170,22 @@ __device__ __forceinline__ void store_bf16_chunk(uint32_t st, int lane, int my_r
     }
   }
 }
-// 16 bytes into registers that are left alone where `on` is false: as a C++ branch the loaded values are merged, and waited for, at
-// the branch's end instead of at their use (3584 x 18944, K = 1000, accumulating: 213 us)
-__device__ __forceinline__ void ld_if(float4& v, const float* p, bool on) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\t"
-      "setp.ne.s32 q, %5, 0;\n\t"
-      "@q ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
-      : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)
-      : "l"(p), "r"((int)on)
-      : "memory");
+// *cp += v, rounded once, by the only thread of the launch that adds to this element.  A reduction in L2 spares the read's latency,
+// but takes subnormal numbers for zeros.  From |v| = 2^-100 on that is never seen: a subnormal old value is less than a quarter ulp
+// of v, and a sum that is not zero is at least 2^-124.  What is smaller reads and writes.  3584 x 18944, K = 1000: 154 us, 181 with
+// reads throughout, two chunks ahead.
+constexpr float kRedMin = 7.8886090522101181e-31f;   // 2^-100
+__device__ __forceinline__ void add_one(float* cp, float v) {
+  if (fabsf(v) >= kRedMin) atomicAdd(cp, v);
+  else *cp = __fadd_rn(__ldcg(cp), v);
+}
+__device__ __forceinline__ void add_four(float* cp, const float (&v)[4]) {
+  if (fminf(fminf(fabsf(v[0]), fabsf(v[1])), fminf(fabsf(v[2]), fabsf(v[3]))) >= kRedMin) {
+    atomicAdd(reinterpret_cast<float4*>(cp), make_float4(v[0], v[1], v[2], v[3]));
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) add_one(cp + e, v[e]);
+  }
 }
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
@@ -189,7 +195,8 @@ __device__ __forceinline__ bool aligned16(const void* p, int64_t ld_bytes) {
   return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)ld_bytes) & 15) == 0;
 }
 
-// kAcc: the launch adds into an fp32 C (plain epilogue only); its lookahead takes 64 registers that the other epilogues need
+// kAcc: the launch adds into an fp32 C (plain epilogue only).  An instance of its own, since the other epilogues feel every register:
+// 3584 x 18944, K = 1000, without accumulation 142 us beside this branch, 114 without it
 template <bool kHead, bool kAcc = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsTN<kHead>, 1)
 gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
@@ -328,28 +335,6 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     const int q = warp & 3;
     const int half = kHead ? 0 : (warp - 2) >> 2;                // which of the quarter's two warps
     const uint32_t st = epi_base + (uint32_t)(warp - 2) * (uint32_t)kEpiBytes;
-    // fp32 accumulation: what is added to is asked for two chunks ahead, the first two of a tile under the tile before
-    constexpr int kBufs = kAcc ? 2 : 1;
-    float4 old[2][8];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) old[i >> 3][i & 7] = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto ask = [&](int t2, int cc, float4 (&o)[8]) {
-      const bool any = aligned16(p.C, p.ldc * 4) && t2 < total_tiles;
-      const int c4 = (lane & 7) * 4, sub = lane >> 3;
-      int tm, tn;
-      tile_coords(t2, p, tm, tn);
-      const int64_t col = (int64_t)tn * p.tile_n + half * 64 + (cc >> 1) * 128 + (cc & 1) * 32 + c4;
-      const bool on = any && col + 4 <= p.N && col + 4 <= (int64_t)(tn + 1) * p.tile_n;
-      const int64_t row = (int64_t)tm * kTile + (int64_t)rank * kHalf + q * 32 + sub;
-      const float* cp = reinterpret_cast<const float*>(p.C) + row * p.ldc + col;
-#pragma unroll
-      for (int it = 0; it < 8; ++it)
-        ld_if(o[it], cp + it * 4 * p.ldc, on && row + it * 4 < p.M);
-    };
-    if (kAcc) {
-      ask(cluster, 0, old[0]);
-      ask(cluster, 1, old[1]);
-    }
     int local = 0;
     for (int t = cluster; t < total_tiles; t += n_clusters, ++local) {
       int tm, tn;
@@ -514,16 +499,14 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
 #pragma unroll
       for (int it = 0; it < 8; ++it) rows[it] = __shfl_sync(0xffffffffu, my_row, it * 4 + sub);
 #pragma unroll 1
-      for (int c2 = 0; c2 < 4; c2 += kBufs) {
-#pragma unroll
-      for (int j2 = 0; j2 < kBufs; ++j2) {   // a warp's chunks come in pairs: 64 neighbouring columns are whole lines of a bf16 row too
-        const int cc = c2 + j2, c0 = half * 64 + (cc >> 1) * 128 + (cc & 1) * 32;
+      for (int cc = 0; cc < 4; ++cc) {   // a warp's chunks come in pairs: 64 neighbouring columns are whole lines of a bf16 row too
+        const int c0 = half * 64 + (cc >> 1) * 128 + (cc & 1) * 32;
         if (c0 < n_tile) {
         const int64_t col = col0 + c0;
         const int n_ok = n_tile - c0 < 32 ? n_tile - c0 : 32;
         const bool in4 = c4 + 4 <= n_ok;
         uint2 res[8];    // asked for before the accumulator is read
-        if (!kAcc && p.residual && vec_r && in4) {
+        if (p.residual && vec_r && in4) {
 #pragma unroll
           for (int it = 0; it < 8; ++it)
             if (rows[it] >= 0) res[it] = *reinterpret_cast<const uint2*>(p.residual + rows[it] * p.ldr + col + c4);
@@ -599,7 +582,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             for (int e = 0; e < 4; ++e) v[e] += b4[e];
           }
           if (p.residual) {
-            if (!kAcc && vec_r && in4) {
+            if (vec_r && in4) {
               const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&res[it].x));
               const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&res[it].y));
               v[0] += f0.x; v[1] += f0.y; v[2] += f1.x; v[3] += f1.y;
@@ -613,13 +596,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
           if (p.c_f32) {
             float* cp = reinterpret_cast<float*>(p.C) + (rows[it] + slice) * p.ldc + col + c4;
             if (vec_c && in4) {
-              // A reduction in L2 would spare the read (3584 x 18944, K = 1000: 154 us, so 181; K = 3072: 273, 279), but it takes
-              // subnormal numbers for zeros.
-              if (kAcc) {
-                const float4 a = old[j2][it];
-                v[0] = __fadd_rn(v[0], a.x); v[1] = __fadd_rn(v[1], a.y); v[2] = __fadd_rn(v[2], a.z); v[3] = __fadd_rn(v[3], a.w);
-              }
-              *reinterpret_cast<float4*>(cp) = make_float4(v[0], v[1], v[2], v[3]);
+              if (kAcc) add_four(cp, v);
+              else *reinterpret_cast<float4*>(cp) = make_float4(v[0], v[1], v[2], v[3]);
             } else {
 #pragma unroll
               for (int e = 0; e < 4; ++e)
@@ -638,10 +616,6 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
         }
         __syncwarp();
         }
-        if (kAcc) {
-          ask(cc < 2 ? t : t + n_clusters, cc ^ 2, old[j2]);
-        }
-      }
       }
       }  // !kHead
       // this CTA's epilogue warps are done with the accumulator -> tell the leader's MMA warp

@@ -381,8 +381,47 @@ def test_fp32_accumulation_keeps_subnormal_numbers(cuda_device, M, N, pad):
         assert (wide[:, :N] == want).all() and (wide[:, N:] == old).all(), (b, old)
 
 
+@pytest.mark.parametrize("pad", [0, 1])
+def test_fp32_accumulation_rounds_as_the_cpu_does(cuda_device, pad):
+    """Products around 2^-100, where adding in L2 begins, and at zero, infinity and NaN; old values from zero to far above them, their
+    negatives and neighbours (cancellation) among them.  One term per sum, so the product is exact and the sum has one rounding."""
+    from pipelinerl_b200 import _lib
+    lib, g, N, K = _lib.load(), torch.Generator().manual_seed(pad), 320, 64
+    e = torch.tensor([0, -60, -99, -100, -101, -102, -110, -125, -126, -130, -140, -149, 3, 40])
+    M = 2 * len(e)
+    A, B = torch.zeros(M, K), torch.zeros(N, K)
+    A[:, 0] = torch.cat([torch.exp2((e // 2).float()), -torch.exp2((e // 2).float())])
+    A[-1, 0] = 0.0
+    scale = torch.exp2((e - e // 2).float()).repeat(2)                    # the rest of the exponent, row by row, in a second operand
+    B[:, 0] = 1 + torch.randint(0, 128, (N,), generator=g).float() / 128
+    B[0, 0], B[1, 0], B[2, 0] = 0.0, torch.inf, torch.nan
+    prod = A[:, :1] * B[:, 0]
+    olds = []
+    for row in range(M):
+        m = prod[row] * scale[row]
+        old = torch.randn(N, generator=g) * torch.exp2(torch.randint(-149, 20, (N,), generator=g).float())
+        old[64:128] = -m[64:128]
+        old[128:192] = torch.nextafter(-m[128:192], torch.tensor(0.0))
+        old[192:256] = torch.exp2(torch.randint(-149, -120, (64,), generator=g).float())
+        old[256:264] = 0.0
+        olds.append(old)
+    old = torch.stack(olds)
+    for row in range(0, M):                                               # a launch per row: its own scale in alpha
+        wide = torch.full((M, N + pad), 7.0)
+        wide[:, :N] = old
+        wide = wide.to(cuda_device)
+        a, b = A.to(torch.bfloat16).to(cuda_device), B.to(torch.bfloat16).to(cuda_device)
+        _lib.check(lib.prl_gemm_ex(a.data_ptr(), K, 0, b.data_ptr(), K, 0, M, N, K, wide.data_ptr(), N + pad, 1, 1, None, None, 0,
+                                   float(scale[row]), _lib.stream_ptr()))
+        want = prod[row].double().float() * scale[row] + old[row]         # exact product and scale (a power of two), one rounded sum
+        got = wide[row, :N].cpu()
+        nan = torch.isnan(want)
+        assert torch.equal(torch.isnan(got), nan) and torch.equal(got[~nan], want[~nan]), row
+        assert (wide[:, N:] == 7.0).all()
+
+
 def test_fp32_accumulation_over_many_tiles_of_a_pair(cuda_device):
-    """More tiles than CTA pairs, ragged on both sides: what a tile adds to is read under the tile before it."""
+    """More tiles than CTA pairs, ragged on both sides."""
     from pipelinerl_b200 import _lib
     lib, g = _lib.load(), torch.Generator().manual_seed(3)
     M, N, K = 4000, 9220, 72
