@@ -278,9 +278,12 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, int64_t ld, int64_t T
   }
 }
 
-__global__ void __launch_bounds__(256) silu_mul_fwd_kernel(const __nv_bfloat16* __restrict__ gu, int I,
+// kLines: eight rows of at most 256 features per block, a warp each; else a row per block or blocks
+template <bool kLines>
+__global__ void __launch_bounds__(256) silu_mul_fwd_kernel(const __nv_bfloat16* __restrict__ gu, int64_t T, int I,
                                                            __nv_bfloat16* __restrict__ act) {
-  const int64_t row = blockIdx.x;                // blocks of one row: no division per element
+  const int64_t row = kLines ? (int64_t)blockIdx.x * 8 + threadIdx.y : blockIdx.x;   // no division per element
+  if (kLines && row >= T) return;
   const __nv_bfloat16* gp = gu + row * 2 * I;
   for (int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8; c < I; c += gridDim.y * blockDim.x * 8) {
     const Vec8 g = unpack8(ld_stream_u4(reinterpret_cast<const uint4*>(gp + c)));
@@ -292,10 +295,12 @@ __global__ void __launch_bounds__(256) silu_mul_fwd_kernel(const __nv_bfloat16* 
   }
 }
 
+template <bool kLines>
 __global__ void __launch_bounds__(256) silu_mul_bwd_kernel(const __nv_bfloat16* __restrict__ gu,
-                                                           const __nv_bfloat16* __restrict__ dact, int I,
+                                                           const __nv_bfloat16* __restrict__ dact, int64_t T, int I,
                                                            __nv_bfloat16* __restrict__ dgu) {
-  const int64_t row = blockIdx.x;
+  const int64_t row = kLines ? (int64_t)blockIdx.x * 8 + threadIdx.y : blockIdx.x;
+  if (kLines && row >= T) return;
   const __nv_bfloat16* gp = gu + row * 2 * I;
   for (int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8; c < I; c += gridDim.y * blockDim.x * 8) {
     const Vec8 g = unpack8(ld_stream_u4(reinterpret_cast<const uint4*>(gp + c)));
@@ -351,6 +356,8 @@ __global__ void __launch_bounds__(256) quotient_kernel(const float* __restrict__
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) q[i] = div_ge1(a[i], b[i]);
 }
 
+// rows of up to a warp's 32 pieces share a block: with a block each, 16384 rows of 128 features took 9.7 us forward, so 4.8
+bool silu_lines(int64_t I) { return I <= 256; }
 int silu_threads(int64_t I) {
   const int64_t n = (I + 7) / 8;
   return n >= 256 ? 256 : (int)((n + 31) / 32 * 32);
@@ -451,8 +458,12 @@ extern "C" int prl_rope_inplace(void* x, int64_t ld, int64_t T, int32_t n_heads,
 
 extern "C" int prl_silu_mul_fwd(const void* gate_up, int64_t T, int64_t I, void* act, prl_stream_t stream) {
   PRL_CHECK_ARG(gate_up && act && T >= 1 && I >= 8 && I % 8 == 0, "prl_silu_mul_fwd: bad argument (I %% 8 == 0)");
-  silu_mul_fwd_kernel<<<silu_grid(T, I), silu_threads(I), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gate_up, (int)I,
-                                                                                (__nv_bfloat16*)act);
+  if (silu_lines(I))
+    silu_mul_fwd_kernel<true><<<(unsigned)((T + 7) / 8), dim3(32, 8), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gate_up, T, (int)I,
+                                                                                                 (__nv_bfloat16*)act);
+  else
+    silu_mul_fwd_kernel<false><<<silu_grid(T, I), silu_threads(I), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gate_up, T, (int)I,
+                                                                                              (__nv_bfloat16*)act);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -460,9 +471,12 @@ extern "C" int prl_silu_mul_fwd(const void* gate_up, int64_t T, int64_t I, void*
 extern "C" int prl_silu_mul_bwd(const void* gate_up, const void* dact, int64_t T, int64_t I, void* dgate_up,
                                 prl_stream_t stream) {
   PRL_CHECK_ARG(gate_up && dact && dgate_up && T >= 1 && I >= 8 && I % 8 == 0, "prl_silu_mul_bwd: bad argument");
-  silu_mul_bwd_kernel<<<silu_grid(T, I), silu_threads(I), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gate_up,
-                                                                                (const __nv_bfloat16*)dact, (int)I,
-                                                                                (__nv_bfloat16*)dgate_up);
+  if (silu_lines(I))
+    silu_mul_bwd_kernel<true><<<(unsigned)((T + 7) / 8), dim3(32, 8), 0, (cudaStream_t)stream>>>(
+        (const __nv_bfloat16*)gate_up, (const __nv_bfloat16*)dact, T, (int)I, (__nv_bfloat16*)dgate_up);
+  else
+    silu_mul_bwd_kernel<false><<<silu_grid(T, I), silu_threads(I), 0, (cudaStream_t)stream>>>(
+        (const __nv_bfloat16*)gate_up, (const __nv_bfloat16*)dact, T, (int)I, (__nv_bfloat16*)dgate_up);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }

@@ -416,7 +416,7 @@ def test_embedding_gradient_into_a_view_at_any_offset(cuda_device, T, H, offset)
     assert torch.equal(flat[:offset].double(), want[:offset]) and torch.equal(flat[offset + V * H:].double(), want[offset + V * H:])
 
 
-@pytest.mark.parametrize("T,I", [(1, 8), (2, 18944), (37, 2056), (700, 24), (1500, 4096)])
+@pytest.mark.parametrize("T,I", [(1, 8), (2, 18944), (37, 2056), (700, 24), (1500, 4096), (1003, 256), (9, 264)])
 def test_silu_rows_cut_over_blocks(cuda_device, T, I):
     from pipelinerl_b200.learner_body import Ops
     o, g = Ops(), torch.Generator().manual_seed(T + I)
