@@ -95,10 +95,67 @@ struct ChoiceRule {
   float scale;                // constant factor on the weights
 };
 
+// Index of the largest of the lanes' values (one per lane), the lowest lane on a tie; 0x7fffffff where no lane holds more than minus
+// infinity (NaN counts as less).  A float's bits in an order that integers share, and one reduction instead of five pairs of shuffles.
+__device__ __forceinline__ int warp_best(float v) {
+  const uint32_t u = __float_as_uint(v + 0.f);             // -0 and +0 tie
+  const uint32_t key = v > -INFINITY ? (u >> 31 ? ~u : u | 0x80000000u) : 0u;
+  const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+  const uint32_t at = __ballot_sync(0xffffffffu, key == top);
+  return top ? __ffs(at) - 1 : 0x7fffffff;
+}
+
+// choose_row for at most 32 outputs: a lane holds one, so that a round of the ranking is three instructions instead of a walk through
+// shared memory and a shuffle tree (16 outputs, 8 groups, 6 + 4 rounds: with the walk the choice was half of the router kernel's 13 us
+// on 32 rows).  The same values, sums and ties.
+__device__ __forceinline__ void choose_row_lanes(const float* z, int E, const ChoiceRule& r, int n, int t, int32_t* __restrict__ sel,
+                                                 float* __restrict__ wsel) {
+  const int lane = threadIdx.x & 31;
+  const bool have = lane < E;
+  const float ze = have ? z[lane] : -INFINITY;
+  float score;
+  if (r.sigmoid) score = sigmoid_f(ze);
+  else {
+    const float zmax = warp_max(ze);
+    const float ex = have ? expf(ze - zmax) : 0.f;
+    const float inv = 1.f / warp_sum(ex);
+    score = ex * inv;
+  }
+  float c = have ? score + (r.correction ? r.correction[lane] : 0.f) : -INFINITY;
+  if (r.keep < r.groups) {
+    const int size = E / r.groups;
+    float m = -INFINITY, m2 = -INFINITY;                   // lane g < groups: the two largest of group g
+    for (int e = 0; e < size; ++e) {
+      const float v = __shfl_sync(0xffffffffu, c, (lane * size + e) & 31);
+      m2 = fmaxf(m2, fminf(m, v));
+      m = fmaxf(m, v);
+    }
+    float gs = lane < r.groups ? ((r.group_top > 1 && size > 1) ? m + m2 : m) : -INFINITY;
+    for (int k = 0; k < r.keep; ++k)
+      if (warp_best(gs) == lane) gs = -INFINITY;           // an open group is marked by taking it out of the ranking
+    if (__shfl_sync(0xffffffffu, gs, have ? lane / size : 0) != -INFINITY) c = -INFINITY;     // still ranked: a closed group
+  }
+  float total = 0.f, mine = 0.f;
+  for (int k = 0; k < r.top; ++k) {
+    const int e = warp_best(c);
+    const bool ok = e < E;                                 // always, for finite logits
+    const float w = ok ? __shfl_sync(0xffffffffu, score, e & 31) : 0.f;
+    total += w;
+    if (lane == k) {
+      mine = w * r.scale;
+      sel[(int64_t)k * n + t] = ok ? e : 0;
+    }
+    if (lane == e) c = -INFINITY;
+  }
+  const float div = r.renorm ? total + 1e-20f : 1.f;
+  if (lane < r.top) wsel[(int64_t)lane * n + t] = mine / div;
+}
+
 // The choice for one row by one warp: c [E] and gs [groups] are the warp's scratch in shared memory, z [E] the logits.
 // Outputs are ranked by score + correction, closed groups count as minus infinity; ties go to the lower index.
 __device__ __forceinline__ void choose_row(const float* z, int E, const ChoiceRule& r, float* c, float* gs, int n, int t,
                                            int32_t* __restrict__ sel, float* __restrict__ wsel) {
+  if (E <= 32) return choose_row_lanes(z, E, r, n, t, sel, wsel);
   const int lane = threadIdx.x & 31;
   float zmax = 0.f, inv = 1.f;
   if (!r.sigmoid) {
@@ -182,66 +239,10 @@ __global__ void __launch_bounds__(kChooseWarps * 32) moe_choose_kernel(const flo
   choose_row(logits + (int64_t)t * ld, E, rule, c, c + E, n, t, sel, wsel);
 }
 
-// Router and choice in one kernel: logits[e] = x . Wr[e] in fp32 (block per row, warps
-// take experts in turn, a lane sums every 32nd group of channels, then the warp's shuffle tree: a fixed order), then the top-k
-// pass of moe_route_kernel over the logits in shared memory (RULED: choose_row instead, with scratch behind the logits).
-template <typename TX, typename TW, bool RULED>
-__global__ void __launch_bounds__(256) moe_router_kernel(const TX* __restrict__ x, const TW* __restrict__ Wr,
-                                                         const float* __restrict__ bias, int n, int W, int E, int top,
-                                                         int softmax_weights, ChoiceRule rule, int32_t* __restrict__ sel,
-                                                         float* __restrict__ wsel) {
-  pdl_wait();
-  extern __shared__ __align__(16) float rsm[];       // [W] the row | [E] logits | RULED: [E] choice scores | [groups] group scores
-  float* xs = rsm;
-  float* z = rsm + W;
-  const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  constexpr int V = 16 / sizeof(TW);              // router weights per 16-byte load
-  const bool vec = W % V == 0 && ((uintptr_t)Wr & 15) == 0;
-  // one element type and aligned rows: the row is read beside the weights (from L1 for all warps but the first), not staged
-  const bool direct = sizeof(TX) == sizeof(TW) && vec && ((uintptr_t)x & 15) == 0;
-  if (!direct) {
-    for (int c = threadIdx.x; c < W; c += blockDim.x) xs[c] = to_f32(x[(int64_t)t * W + c]);
-    __syncthreads();
-  }
-  for (int e = warp; e < E; e += nw) {
-    const TW* w = Wr + (int64_t)e * W;
-    float a = 0.f;
-    if (direct) {                                 // a lane sums its channels in ascending order
-      const TX* xr = x + (int64_t)t * W;
-#pragma unroll 4
-      for (int c = V * lane; c < W; c += 32 * V) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(w + c), xraw = *reinterpret_cast<const uint4*>(xr + c);
-        const TW* wv = reinterpret_cast<const TW*>(&raw);
-        const TX* xv = reinterpret_cast<const TX*>(&xraw);
-#pragma unroll
-        for (int j = 0; j < V; ++j) a = fmaf(to_f32(xv[j]), to_f32(wv[j]), a);
-      }
-    } else if (vec) {
-#pragma unroll 4
-      for (int c = V * lane; c < W; c += 32 * V) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(w + c);
-        const TW* wv = reinterpret_cast<const TW*>(&raw);
-#pragma unroll
-        for (int j = 0; j < V; j += 4) {
-          const float4 xv = *reinterpret_cast<const float4*>(xs + c + j);
-          a = fmaf(xv.x, to_f32(wv[j]), a); a = fmaf(xv.y, to_f32(wv[j + 1]), a);
-          a = fmaf(xv.z, to_f32(wv[j + 2]), a); a = fmaf(xv.w, to_f32(wv[j + 3]), a);
-        }
-      }
-    } else {
-#pragma unroll 8
-      for (int c = lane; c < W; c += 32) a = fmaf(xs[c], to_f32(w[c]), a);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if (lane == 0) z[e] = a + (bias ? bias[e] : 0.f);
-  }
-  __syncthreads();
-  if (warp != 0) return;
-  if constexpr (RULED) {
-    choose_row(z, E, rule, z + E, z + 2 * E, n, t, sel, wsel);
-    return;
-  }
+// The `top` largest of a row's logits z [E] in shared memory and their weights, by one warp (the ranking of moe_route_kernel).
+__device__ __forceinline__ void top_of_row(const float* z, int E, int top, int softmax_weights, int n, int t, int32_t* __restrict__ sel,
+                                           float* __restrict__ wsel) {
+  const int lane = threadIdx.x & 31;
   uint32_t taken = 0;
   float zsel_max = 0.f, denom = 0.f;
   for (int c = 0; c < top; ++c) {
@@ -279,6 +280,117 @@ __global__ void __launch_bounds__(256) moe_router_kernel(const TX* __restrict__ 
   }
   if (softmax_weights && lane == 0)
     for (int c = 0; c < top; ++c) wsel[(int64_t)c * n + t] /= denom;
+}
+
+// Router and choice in one kernel: logits[e] = x . Wr[e] in fp32 (block per row, warps
+// take experts in turn, a lane sums every 32nd group of channels, then the warp's shuffle tree: a fixed order), then the top-k
+// pass of moe_route_kernel over the logits in shared memory (RULED: choose_row instead, with scratch behind the logits).
+template <typename TX, typename TW, bool RULED>
+__global__ void __launch_bounds__(256) moe_router_kernel(const TX* __restrict__ x, const TW* __restrict__ Wr,
+                                                         const float* __restrict__ bias, int n, int W, int E, int top,
+                                                         int softmax_weights, ChoiceRule rule, int32_t* __restrict__ sel,
+                                                         float* __restrict__ wsel) {
+  pdl_wait();
+  extern __shared__ __align__(16) float rsm[];       // [W] the row | [E] logits | RULED: [E] choice scores | [groups] group scores
+  float* xs = rsm;
+  float* z = rsm + W;
+  const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  constexpr int V = 16 / sizeof(TW);              // router weights per 16-byte load
+  const bool vec = W % V == 0 && ((uintptr_t)Wr & 15) == 0;
+  for (int c = threadIdx.x; c < W; c += blockDim.x) xs[c] = to_f32(x[(int64_t)t * W + c]);
+  __syncthreads();
+  for (int e = warp; e < E; e += nw) {
+    const TW* w = Wr + (int64_t)e * W;
+    float a = 0.f;
+    if (vec) {
+#pragma unroll 4
+      for (int c = V * lane; c < W; c += 32 * V) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(w + c);
+        const TW* wv = reinterpret_cast<const TW*>(&raw);
+#pragma unroll
+        for (int j = 0; j < V; j += 4) {
+          const float4 xv = *reinterpret_cast<const float4*>(xs + c + j);
+          a = fmaf(xv.x, to_f32(wv[j]), a); a = fmaf(xv.y, to_f32(wv[j + 1]), a);
+          a = fmaf(xv.z, to_f32(wv[j + 2]), a); a = fmaf(xv.w, to_f32(wv[j + 3]), a);
+        }
+      }
+    } else {
+#pragma unroll 8
+      for (int c = lane; c < W; c += 32) a = fmaf(xs[c], to_f32(w[c]), a);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane == 0) z[e] = a + (bias ? bias[e] : 0.f);
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  if constexpr (RULED) {
+    choose_row(z, E, rule, z + E, z + 2 * E, n, t, sel, wsel);
+    return;
+  }
+  top_of_row(z, E, top, softmax_weights, n, t, sel, wsel);
+}
+
+// moe_router_kernel for rows and router weights of one element type, both on 16-byte boundaries: ROWS rows per block of 16 warps, which
+// take experts in turn.  A weight chunk is read once for the block's rows and the rows beside it, all chunks of a batch in flight
+// together; the first expert's weights, which no earlier kernel writes, are on their way before the wait for the row.  A lane sums its
+// channels in ascending order, then the shuffle tree: per (row, expert) the sums of moe_router_kernel.
+// Bound by the latency of its loads and of the choice.  2048 channels, 16 experts, with the grouping behind it: 1024 rows 24.8 -> 15.3 us,
+// 32 rows of a token step 17 -> 11 us (its weights come from HBM there), 128 experts on 32 rows 33.5 -> 20.0.
+constexpr int kRouterWarps = 16;
+template <typename T, bool RULED, int ROWS>
+__global__ void __launch_bounds__(32 * kRouterWarps) moe_router_rows_kernel(const T* __restrict__ x, const T* __restrict__ Wr,
+                                                                            const float* __restrict__ bias, int n, int W, int E, int top,
+                                                                            int softmax_weights, ChoiceRule rule,
+                                                                            int32_t* __restrict__ sel, float* __restrict__ wsel) {
+  extern __shared__ __align__(16) float rsm[];       // [ROWS][E] logits | RULED: per row [E] choice scores | [groups] group scores
+  const int t0 = blockIdx.x * ROWS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int V = 16 / sizeof(T), U = 8;           // elements per 16-byte load, loads of a batch
+  uint4 wq[U];
+  auto load = [&](uint4 (&q)[U], const T* row, int c0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int c = c0 + V * (lane + 32 * u);
+      if (c < W) q[u] = *reinterpret_cast<const uint4*>(row + c);
+    }
+  };
+  if (warp < E) load(wq, Wr + (int64_t)warp * W, 0);
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int e = warp; e < E; e += kRouterWarps) {
+    float a[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) a[r] = 0.f;
+    for (int c0 = 0; c0 < W; c0 += 32 * V * U) {
+      if (e != warp || c0 > 0) load(wq, Wr + (int64_t)e * W, c0);
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        if (t0 + r >= n) break;
+        uint4 xq[U];
+        load(xq, x + (int64_t)(t0 + r) * W, c0);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (c0 + V * (lane + 32 * u) >= W) break;
+          const T* wv = reinterpret_cast<const T*>(&wq[u]);
+          const T* xv = reinterpret_cast<const T*>(&xq[u]);
+#pragma unroll
+          for (int j = 0; j < V; ++j) a[r] = fmaf(to_f32(xv[j]), to_f32(wv[j]), a[r]);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      a[r] = warp_sum(a[r]);
+      if (lane == 0) rsm[r * E + e] = a[r] + (bias ? bias[e] : 0.f);
+    }
+  }
+  __syncthreads();
+  const int t = t0 + warp;
+  if (warp >= ROWS || t >= n) return;
+  float* z = rsm + warp * E;
+  float* c = rsm + ROWS * E + warp * (E + rule.groups);
+  if constexpr (RULED) choose_row(z, E, rule, c, c + E, n, t, sel, wsel);
+  else top_of_row(z, E, top, softmax_weights, n, t, sel, wsel);
 }
 
 // meta[0] = number of tiles, meta[1] = sorted pairs; tiles[3 * i + {0, 1, 2}] = expert, first sorted place, rows (<= tile_rows)
@@ -688,6 +800,30 @@ static int moe_router_impl(const void* x, int32_t x_is_f32, const void* Wr, int3
   const size_t smem = ((size_t)W + outputs + (rule ? outputs + rule->groups : 0)) * sizeof(float);
   PRL_CHECK_ARG(smem <= 160 * 1024, "prl_moe_router: a row of %d channels does not fit in shared memory", W);
   cudaStream_t s = (cudaStream_t)st;
+  const int per = x_is_f32 ? 4 : 8;
+  if (!x_is_f32 == !w_is_f32 && W % per == 0 && (((uintptr_t)x | (uintptr_t)Wr) & 15) == 0) {
+    // one block of 16 warps fits an SM: as many rows share a block as keep the blocks in one wave (with the grouping behind it, 2048
+    // channels, 16 experts: 452 rows 18.3 us by one, 10.9 by four; 1024 rows 17.9 by four, 15.3 by eight)
+    const size_t per_row = (outputs + (rule ? outputs + rule->groups : 0)) * sizeof(float);      // at most 12 KB
+    const int rows = n > 4 * 148 && 8 * per_row <= 48 * 1024 ? 8 : n > 148 ? 4 : 1;
+    const size_t sm = rows * per_row;
+#define PRL_RR(T, RULED, ROWS)                                                                                                    \
+  PRL_CUDA(launch_pdl((moe_router_rows_kernel<T, RULED, ROWS>), dim3((n + ROWS - 1) / ROWS), dim3(32 * kRouterWarps), sm, s, (const T*)x, \
+                      (const T*)Wr, bias, n, W, outputs, top, softmax_weights, rule ? *rule : ChoiceRule{}, sel, wsel))
+#define PRL_RR2(T, ROWS)                  \
+  do {                                    \
+    if (rule) PRL_RR(T, true, ROWS);      \
+    else PRL_RR(T, false, ROWS);          \
+  } while (0)
+    if (x_is_f32) { if (rows == 8) PRL_RR2(float, 8); else if (rows == 4) PRL_RR2(float, 4); else PRL_RR2(float, 1); }
+    else { if (rows == 8) PRL_RR2(bf16, 8); else if (rows == 4) PRL_RR2(bf16, 4); else PRL_RR2(bf16, 1); }
+#undef PRL_RR2
+#undef PRL_RR
+    PRL_LAUNCH_CHECK();
+    PRL_CUDA(launch_group(sel, n * top, experts, tile_rows, perm, meta, tiles, s));
+    PRL_LAUNCH_CHECK();
+    return PRL_OK;
+  }
   static SmemAttr attr[8] = {};
 #define PRL_RT(TX, TW, RULED, I)                                                                                       \
   do {                                                                                                                 \

@@ -309,6 +309,40 @@ BIG = mc.model([P(heads=8, kv_heads=2, dim=32, vdim=32, rot_dims=16, window=100,
                   mlp=M(experts=8, top=2, ff=96, groups=(4, 2)))], vocab=200, width=128)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,W,experts,groups,keep,top", [(1, 8, 4, 1, 1, 4), (33, 2048, 16, 8, 6, 4), (592, 264, 32, 4, 2, 16), (593, 1032, 33, 3, 1, 5),
+                                                         (1023, 2056, 16, 8, 8, 1)])
+def test_router_rows_equal_the_staged_router(cuda_device, dtype, n, W, experts, groups, keep, top):
+    """Rows and weights on 16-byte boundaries take a kernel of their own; rows one element further on, the one that stages them.
+    Sums, ranking and weights are the same in both, also for rows with infinities and NaN."""
+    from pipelinerl_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(n + W)
+    x = torch.randn(n, W, generator=g, device="cuda").to(dtype)
+    w = (torch.randn(experts, W, generator=g, device="cuda") * W ** -0.5).to(dtype)
+    shifted = torch.empty(n * W + 1, dtype=dtype, device="cuda")[1:]
+    shifted.copy_(x.view(-1))
+    corr = torch.randn(experts, generator=g, device="cuda")
+    lib, st = _lib.load(), _lib.stream_ptr()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    for sigmoid in (2, 0, 1):                       # 2: prl_moe_router (softmax over the chosen), for finite logits
+        if sigmoid == 0 and n > 8:
+            x[3, 1], x[5, W // 2], x[7, 0] = float("inf"), float("nan"), -float("inf")
+            shifted.copy_(x.view(-1))
+        got = []
+        for rows in (x, shifted):
+            sel, wsel, perm = torch.full((top, n), -7, **i32), torch.full((top, n), -7.0, device="cuda"), torch.zeros(top * n, **i32)
+            meta, tiles = torch.zeros(4, **i32), torch.zeros(3 * int(lib.prl_moe_max_tiles(top * n, experts)), **i32)
+            f32 = int(dtype == torch.float32)
+            tail = (sel.data_ptr(), wsel.data_ptr(), perm.data_ptr(), meta.data_ptr(), tiles.data_ptr(), st)
+            if sigmoid == 2:
+                _lib.check(lib.prl_moe_router(rows.data_ptr(), f32, w.data_ptr(), f32, corr.data_ptr(), n, W, experts, top, 1, *tail))
+            else:
+                _lib.check(lib.prl_moe_router_choose(rows.data_ptr(), f32, w.data_ptr(), f32, corr.data_ptr(), n, W, experts, experts, top,
+                                                     groups, keep, 2, sigmoid, 1, 1.25, 64, *tail))
+            got.append((sel, wsel.view(torch.int32)))
+        assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 @pytest.mark.parametrize("plain_gemm", [False, True])
 def test_bf16_serving_mode(cuda_device, plain_gemm):
     """bf16 operands and cache with the tensor-core GEMMs (and with the CUDA-core GEMM) against the float64 oracle.  Only the
