@@ -506,84 +506,110 @@ __global__ void joint_close_kernel(const float* __restrict__ y0, int ns0, int64_
   }
 }
 
+// block_sum of two values at once: the same sums, one pair of barriers
+__device__ __forceinline__ float2 block_sum2(float u, float v, float2* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  u = warp_sum(u);
+  v = warp_sum(v);
+  __syncthreads();
+  if (lane == 0) red[warp] = make_float2(u, v);
+  __syncthreads();
+  float2 t = make_float2(0.f, 0.f);
+  for (int w = 0; w < nw; ++w) { t.x += red[w].x; t.y += red[w].y; }
+  return t;
+}
+
 // sublayer_close_kernel for rows of a multiple of four channels: a thread keeps NC groups of four channels of the row (and of
 // the second branch) in registers from the sums to the normed store.
-template <typename T, int NC>
-__global__ void sublayer_close_vec_kernel(const float* __restrict__ y0, int64_t ld0, int ns0, int64_t stride0,
-                                          const float* __restrict__ gain0, float s0, const float* __restrict__ y1, int64_t ld1,
-                                          int ns1, int64_t stride1, const float* __restrict__ gain1, float s1,
-                                          const float* __restrict__ post_gain, const float* __restrict__ bias, int add,
-                                          const float* __restrict__ next_gain, float eps, int W, float* __restrict__ x,
-                                          T* __restrict__ xa) {
+// Bound by latency: a row is read once by one block, and a token step has fewer rows than SMs.  So all slices of both branches, the
+// residual and the branch gains are asked for before the first sum waits for any of them, the gains (which no kernel of a step writes)
+// come to L2 before the wait for the predecessor (asked for by the first block: all share them), and both branches' sums share their barriers: in L2 5.8 -> 5.5 us for 32 rows x 2048
+// of eight slices each (a token step of four such layers, with attn_front_lanes_kernel: 728 -> 704), 12.8 -> 11.7 for 1024 rows of one.
+// FEW: a token step's rows.  Many narrow rows (one group a thread, 256 threads) do better with one branch after the other and more blocks
+// on an SM: 1024 x 1024, one slice each 7.6 us, 8.6 with FEW's loads; 1024 threads of four groups have no registers for two branches.
+template <typename T, int NC, bool FEW>
+__global__ void __launch_bounds__(NC == 2 ? 512 : NC == 1 && !FEW ? 256 : 1024, NC == 2 ? 2 : NC == 1 && !FEW ? 8 : 1) sublayer_close_vec_kernel(
+    const float* __restrict__ y0, int64_t ld0, int ns0, int64_t stride0, const float* __restrict__ gain0, float s0,
+    const float* __restrict__ y1, int64_t ld1, int ns1, int64_t stride1, const float* __restrict__ gain1, float s1,
+    const float* __restrict__ post_gain, const float* __restrict__ bias, int add, const float* __restrict__ next_gain, float eps, int W,
+    float* __restrict__ x, T* __restrict__ xa) {
+  if (blockIdx.x == 0 && (int)threadIdx.x * 32 < W) {
+    const int c = threadIdx.x * 32;
+    for (const float* g : {gain0, gain1, post_gain, bias, next_gain})
+      if (g) asm volatile("prefetch.global.L2 [%0];" ::"l"(g + c));
+  }
   pdl_wait();
+  pdl_launch_dependents();          // the next kernel's weights
+  __shared__ float2 red2[32];
   __shared__ float red[32];
+  constexpr bool kAhead = NC == 2 || (NC == 1 && FEW);   // else one branch after the other, the gains where they are used
   const int64_t r = blockIdx.x, at = r * W;
   const int n4 = W / 4;
   auto sumsq = [](const float4& a) { return a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w; };
-  auto scaled = [](const float4& a, float f, const float* g) {       // a * f * g (g NULL: a * f)
-    if (!g) return make_float4(a.x * f, a.y * f, a.z * f, a.w * f);
-    const float4 w = ld4(g);
-    return make_float4(a.x * f * w.x, a.y * f * w.y, a.z * f * w.z, a.w * f * w.w);
-  };
-  float4 v[NC], xr[NC];
+  auto scaled = [](const float4& a, float f) { return make_float4(a.x * f, a.y * f, a.z * f, a.w * f); };
+  auto gained = [](const float4& a, float f, const float4& w) { return make_float4(a.x * f * w.x, a.y * f * w.y, a.z * f * w.z, a.w * f * w.w); };
+  float4 v[NC], b[NC], xr[NC], g0[NC], g1[NC];
 #pragma unroll
   for (int u = 0; u < NC; ++u) {
-    v[u] = xr[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    v[u] = b[u] = xr[u] = g0[u] = g1[u] = make_float4(0.f, 0.f, 0.f, 0.f);
     const int c = threadIdx.x + u * blockDim.x;
-    if (c < n4 && add) xr[u] = ld4(x + at + 4 * c);
+    if (c >= n4) continue;
+    if (add) xr[u] = ld4(x + at + 4 * c);
+    if (kAhead && gain0) g0[u] = ld4(gain0 + 4 * c);
+    if (kAhead && gain1) g1[u] = ld4(gain1 + 4 * c);
   }
-#pragma unroll 4
-  for (int k = 0; k < ns0; ++k)
-#pragma unroll
-    for (int u = 0; u < NC; ++u) {
-      const int c = threadIdx.x + u * blockDim.x;
-      if (c < n4) add4(v[u], ld4(y0 + k * stride0 + r * ld0 + 4 * c));
-    }
-  float f0 = s0;
-  if (gain0) {
-    float ss = 0.f;
-#pragma unroll
-    for (int u = 0; u < NC; ++u) ss += sumsq(v[u]);
-    f0 = s0 / sqrtf(block_sum(ss, red) / (float)W + eps);
-  }
-#pragma unroll
-  for (int u = 0; u < NC; ++u) {
-    const int c = threadIdx.x + u * blockDim.x;
-    if (c < n4) v[u] = scaled(v[u], f0, gain0 ? gain0 + 4 * c : nullptr);
-  }
-  if (y1) {
-    float4 b[NC];
-#pragma unroll
-    for (int u = 0; u < NC; ++u) b[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-    for (int k = 0; k < ns1; ++k)
+  auto slices = [&](float4 (&a)[NC], const float* y, int64_t ld, int ns, int64_t stride) {
+#pragma unroll (NC == 1 && FEW ? 8 : 4)
+    for (int k = 0; k < ns; ++k)
 #pragma unroll
       for (int u = 0; u < NC; ++u) {
         const int c = threadIdx.x + u * blockDim.x;
-        if (c < n4) add4(b[u], ld4(y1 + k * stride1 + r * ld1 + 4 * c));
+        if (c < n4) add4(a[u], ld4(y + k * stride + r * ld + 4 * c));
       }
-    float f1 = s1;
-    if (gain1) {
-      float ss = 0.f;
+  };
+  auto squares = [&](const float4 (&a)[NC]) {
+    float ss = 0.f;
 #pragma unroll
-      for (int u = 0; u < NC; ++u) ss += sumsq(b[u]);
-      f1 = s1 / sqrtf(block_sum(ss, red) / (float)W + eps);
+    for (int u = 0; u < NC; ++u) ss += sumsq(a[u]);
+    return ss;
+  };
+  auto branch = [&](const float4& a, float f, const float* gain, const float4& ahead, int c) {
+    return gain ? gained(a, f, kAhead ? ahead : ld4(gain + 4 * c)) : scaled(a, f);
+  };
+  slices(v, y0, ld0, ns0, stride0);
+  float f0 = s0, f1 = s1;
+  if (kAhead) {
+    if (y1) slices(b, y1, ld1, ns1, stride1);
+    if (gain0 || (y1 && gain1)) {
+      const float2 t = block_sum2(squares(v), squares(b), red2);
+      if (gain0) f0 = s0 / sqrtf(t.x / (float)W + eps);
+      if (gain1) f1 = s1 / sqrtf(t.y / (float)W + eps);
+    }
+  } else if (gain0) {
+    f0 = s0 / sqrtf(block_sum(squares(v), red) / (float)W + eps);
+  }
+#pragma unroll
+  for (int u = 0; u < NC; ++u) {
+    const int c = threadIdx.x + u * blockDim.x;
+    if (c < n4) v[u] = branch(v[u], f0, gain0, g0[u], c);
+  }
+  if (y1) {
+    if (!kAhead) {
+      slices(b, y1, ld1, ns1, stride1);
+      if (gain1) f1 = s1 / sqrtf(block_sum(squares(b), red) / (float)W + eps);
     }
 #pragma unroll
     for (int u = 0; u < NC; ++u) {
       const int c = threadIdx.x + u * blockDim.x;
-      if (c < n4) add4(v[u], scaled(b[u], f1, gain1 ? gain1 + 4 * c : nullptr));
+      if (c < n4) add4(v[u], branch(b[u], f1, gain1, g1[u], c));
     }
   }
   if (post_gain) {
-    float ss = 0.f;
-#pragma unroll
-    for (int u = 0; u < NC; ++u) ss += sumsq(v[u]);
-    const float fp = 1.f / sqrtf(block_sum(ss, red) / (float)W + eps);
+    const float fp = 1.f / sqrtf(block_sum(squares(v), red) / (float)W + eps);
 #pragma unroll
     for (int u = 0; u < NC; ++u) {
       const int c = threadIdx.x + u * blockDim.x;
-      if (c < n4) v[u] = scaled(v[u], fp, post_gain + 4 * c);
+      if (c < n4) v[u] = gained(v[u], fp, ld4(post_gain + 4 * c));
     }
   }
   float sx = 0.f;
@@ -595,6 +621,7 @@ __global__ void sublayer_close_vec_kernel(const float* __restrict__ y0, int64_t 
       add4(v[u], xr[u]);
       st4(x + at + 4 * c, v[u]);
       sx += sumsq(v[u]);
+      if (kAhead && next_gain) g0[u] = ld4(next_gain + 4 * c);
     }
   }
   float fn = 1.f;
@@ -602,7 +629,7 @@ __global__ void sublayer_close_vec_kernel(const float* __restrict__ y0, int64_t 
 #pragma unroll
   for (int u = 0; u < NC; ++u) {
     const int c = threadIdx.x + u * blockDim.x;
-    if (c < n4) st4(xa + at + 4 * c, next_gain ? scaled(v[u], fn, next_gain + 4 * c) : v[u]);
+    if (c < n4) st4(xa + at + 4 * c, next_gain ? gained(v[u], fn, kAhead ? g0[u] : ld4(next_gain + 4 * c)) : v[u]);
   }
 }
 
@@ -1014,6 +1041,103 @@ __global__ void attn_front_kernel(const float* __restrict__ P, int64_t ldp, int 
   }
 }
 
+// attn_front_kernel for heads of whole warps' widths (dim and vdim multiples of 32 up to 128, rot a multiple of 64): a lane holds channels
+// lane + 32 k of its head, so both channels of a turned pair are its own, and a head is read once.
+// Bound by the chain of its loads on a token step (row -> page -> store): the head's channels, the row's position and slot are asked for
+// together, the page while the angles are computed, and a warp has one head.  The values of attn_front_kernel, bit for bit.
+// 16 + 2 x 4 heads of 128, 64 turned channels: 32 rows 3.9 -> 3.4 us, 1024 rows 25.0 -> 12.4.
+template <typename T>
+__global__ void __launch_bounds__(1024) attn_front_lanes_kernel(
+    const float* __restrict__ P, int64_t ldp, int off_q, int off_k, int off_v, int H, int G, int dim, int vdim,
+    const float* __restrict__ q_bias, const float* __restrict__ k_bias, const float* __restrict__ v_bias, int qk_norm,
+    const float* __restrict__ q_gain, const float* __restrict__ k_gain, int gain_period, float eps, int rot,
+    const double* __restrict__ freq, float mag, int v_norm, int v_blend, const float* __restrict__ v_lambda, float* __restrict__ v_first,
+    const int32_t* __restrict__ row_pos, const int32_t* __restrict__ row_slot, const int32_t* __restrict__ block_table, int max_blocks,
+    int page_size, T* __restrict__ q_out, T* __restrict__ k_pool, T* __restrict__ v_pool) {
+  __shared__ float trig[128];        // [rot / 2] cos | [rot / 2] sin of the row's angles, times mag
+  const int half = rot / 2, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+  const double fr = tid < half ? freq[tid] : 0.0;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int r = blockIdx.x;
+  float raw[4];
+  auto fetch = [&](int hh) {         // past the head's width: not read
+    const bool is_v = hh >= H + G;
+    const int head = hh < H ? hh : is_v ? hh - H - G : hh - H, width = is_v ? vdim : dim;
+    const float* src = P + (int64_t)r * ldp + (hh < H ? off_q : is_v ? off_v : off_k) + head * width;
+    const float* bias = hh < H ? q_bias : is_v ? v_bias : k_bias;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      raw[k] = 32 * k < width ? src[lane + 32 * k] + (bias ? bias[head * width + lane + 32 * k] : 0.f) : 0.f;
+  };
+  if (warp < H + 2 * G) fetch(warp);
+  const int slot = row_slot[r], pos = row_pos[r];
+  if (slot < 0) return;
+  const int page = block_table[(int64_t)slot * max_blocks + pos / page_size], within = pos % page_size;
+  if (tid < half) {
+    // angle and its reduction to [-pi, pi] in double, then the fp32 sincos of a small argument (see qk_norm_rope_cache_kernel)
+    const double ang = (double)pos * fr;
+    const double turns = rint(ang * 0.15915494309189535);
+    float sn, cs;
+    sincosf((float)fma(-turns, 6.283185307179586, ang), &sn, &cs);
+    trig[tid] = cs * mag;
+    trig[half + tid] = sn * mag;
+  }
+  __syncthreads();
+  for (int hh = warp; hh < H + 2 * G; hh += nw) {
+    if (hh != warp) fetch(hh);
+    const bool is_v = hh >= H + G;
+    const int width = is_v ? vdim : dim;
+    float inv = 1.f;
+    if (is_v ? v_norm : qk_norm) {
+      float ss = 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (32 * k < width) ss += raw[k] * raw[k];
+      inv = 1.f / sqrtf(warp_sum(ss) / (float)width + eps);
+    }
+    if (!is_v) {
+      const bool is_q = hh < H;
+      const int head = is_q ? hh : hh - H;
+      const float* gain = is_q ? q_gain : k_gain;
+      T* dst = is_q ? q_out + ((int64_t)r * H + head) * dim : k_pool + (((int64_t)page * G + head) * page_size + within) * dim;
+      float val[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        val[k] = 32 * k < width ? raw[k] * inv * (gain ? gain[(head * dim + lane + 32 * k) % gain_period] : 1.f) : 0.f;
+      if (half == 32) {
+        const float u = val[0], v = val[1], cs = trig[lane], sn = trig[32 + lane];
+        val[0] = u * cs - v * sn;
+        val[1] = v * cs + u * sn;
+      } else if (half == 64) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const float u = val[k], v = val[k + 2], cs = trig[lane + 32 * k], sn = trig[64 + lane + 32 * k];
+          val[k] = u * cs - v * sn;
+          val[k + 2] = v * cs + u * sn;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (32 * k < width) stf(dst, lane + 32 * k, val[k]);
+    } else {
+      const int head = hh - H - G;
+      const float lam = v_blend == 2 ? *v_lambda : 0.f;
+      float* vf = v_first ? v_first + ((int64_t)r * G + head) * vdim : nullptr;
+      T* dst = v_pool + (((int64_t)page * G + head) * page_size + within) * vdim;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int j = lane + 32 * k;
+        if (32 * k >= width) continue;
+        float v = raw[k] * inv;
+        if (v_blend == 1) vf[j] = v;
+        else if (v_blend == 2) v = (1.f - lam) * v + lam * vf[j];
+        stf(dst, j, v);
+      }
+    }
+  }
+}
+
 // z <- cap * tanh(z / cap): the model's capped logits, in place
 __global__ void soft_cap_kernel(float* __restrict__ z, int64_t count, float cap) {
   pdl_wait();
@@ -1213,10 +1337,18 @@ extern "C" int prl_sublayer_close(const float* y0, int64_t ld0, int32_t n_split0
     const int n4 = W / 4, nc = n > 256 ? (n4 <= 256 ? 1 : n4 <= 1024 ? 2 : 4) : (n4 <= 1024 ? 1 : 4);
     const int th = ((n4 + nc - 1) / nc + 31) / 32 * 32;
     const int64_t st0 = (int64_t)n * ld0, st1 = (int64_t)n * ld1;
-#define PRL_SC(T, NC) PRL_CUDA(launch_pdl((sublayer_close_vec_kernel<T, NC>), dim3(n), dim3(th), (size_t)0, (cudaStream_t)st, y0, ld0, n_split0, st0, gain0, s0, \
+#define PRL_SC(T, NC, FEW) PRL_CUDA(launch_pdl((sublayer_close_vec_kernel<T, NC, FEW>), dim3(n), dim3(th), (size_t)0, (cudaStream_t)st, y0, ld0, n_split0, st0, gain0, s0, \
                                           y1, ld1, n_split1, st1, gain1, s1, post_gain, bias, add, next_gain, eps, W, x, (T*)xa))
-    if (f32) { if (nc == 1) PRL_SC(float, 1); else if (nc == 2) PRL_SC(float, 2); else PRL_SC(float, 4); }
-    else { if (nc == 1) PRL_SC(bf16, 1); else if (nc == 2) PRL_SC(bf16, 2); else PRL_SC(bf16, 4); }
+#define PRL_SCT(T)                                 \
+  do {                                             \
+    if (nc == 1 && n > 256) PRL_SC(T, 1, false);   \
+    else if (nc == 1) PRL_SC(T, 1, true);          \
+    else if (nc == 2) PRL_SC(T, 2, false);         \
+    else PRL_SC(T, 4, false);                      \
+  } while (0)
+    if (f32) PRL_SCT(float);
+    else PRL_SCT(bf16);
+#undef PRL_SCT
 #undef PRL_SC
     PRL_LAUNCH_CHECK();
     return PRL_OK;
@@ -1383,6 +1515,19 @@ extern "C" int prl_attn_front(const float* P, int64_t ldp, int32_t off_q, int32_
                 "prl_attn_front: bad shape (H=%d G=%d dim=%d vdim=%d rot=%d)", H, G, dim, vdim, rot);
   PRL_CHECK_ARG(v_blend >= 0 && v_blend <= 2 && (v_blend == 0 || v_first) && (v_blend != 2 || v_lambda),
                 "prl_attn_front: blending the values needs the first layer's values and the weight");
+  if (dim % 32 == 0 && dim <= 128 && vdim % 32 == 0 && vdim <= 128 && rot % 64 == 0) {
+    // few rows: a warp per head, the shortest chain; rows that fill the SMs: eight warps, so that several blocks share one
+    const int heads = H + 2 * G, most = n > 2 * 148 ? 8 : 32, w = heads < most ? heads : most, th = 32 * (w < 2 ? 2 : w);   // rot / 2 <= th
+#define PRL_AF(T)                                                                                                                      \
+  PRL_CUDA(launch_pdl(attn_front_lanes_kernel<T>, dim3(n), dim3(th), (size_t)0, (cudaStream_t)st, P, ldp, off_q, off_k, off_v, H, G, dim, \
+                      vdim, q_bias, k_bias, v_bias, qk_norm, q_gain, k_gain, gain_period, eps, rot, freq, mag, v_norm, v_blend, v_lambda, \
+                      v_first, row_pos, row_slot, block_table, max_blocks, page_size, (T*)q_out, (T*)k_pool, (T*)v_pool))
+    if (f32) PRL_AF(float);
+    else PRL_AF(bf16);
+#undef PRL_AF
+    PRL_LAUNCH_CHECK();
+    return PRL_OK;
+  }
   int warps = H + 2 * G;
   warps = warps > 16 ? 16 : warps;
   const size_t smem = (size_t)(rot > 0 ? rot : 1) * sizeof(float);

@@ -387,3 +387,70 @@ def test_rollouts_through_the_plugin_interface(cuda_device):
                 assert abs(lp - ref[n_prompt - 1 + k, ids[n_prompt + k]].item()) < 2e-3
                 checked += 1
     assert checked >= 9
+
+
+# ---- row kernels alone ---------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("n,W,k0,k1", [(1, 4, 1, 0), (33, 2048, 8, 8), (300, 1028, 1, 4), (7, 16384, 16, 3), (260, 4096, 2, 1), (5, 4100, 1, 9)])
+def test_sublayer_close_rows(cuda_device, n, W, k0, k1):
+    """prl_sublayer_close with every norm, against 64 bits: rows of one, two and four groups of channels per thread."""
+    from pipelinerl_b200 import _lib
+    lib, g = _lib.load(), torch.Generator(device="cuda").manual_seed(W + n)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    y0, y1, x, bias = rnd(k0, n, W), rnd(max(k1, 1), n, W), rnd(n, W), rnd(W)
+    g0, g1, gp, gn = (rnd(W) for _ in range(4))
+    rms = lambda v: v * torch.rsqrt((v * v).mean(-1, keepdim=True) + 1e-5)  # noqa: E731
+    v = 0.7 * rms(y0.double().sum(0)) * g0
+    if k1:
+        v = v + 1.3 * rms(y1.double().sum(0)) * g1
+    want = x.double() + rms(v) * gp + bias
+    out, ptr = torch.empty(n, W, device="cuda"), lambda t: t.data_ptr()  # noqa: E731
+    _lib.check(lib.prl_sublayer_close(ptr(y0), W, k0, ptr(g0), 0.7, ptr(y1) if k1 else None, W, max(k1, 1), ptr(g1) if k1 else None, 1.3, ptr(gp),
+                                      ptr(bias), 1, ptr(gn), 1e-5, n, W, ptr(x), ptr(out), 1, _lib.stream_ptr()))
+    # every value passes at most four roundings of its own and norms whose sums are good to a few ulp: 1e-6 of the row's scale
+    assert (x.double() - want).abs().max() < 2e-5 * want.abs().max() and (x.double() - want).norm() < 1e-6 * want.norm()
+    assert (out.double() - rms(want) * gn).norm() < 2e-6 * (rms(want) * gn).norm()
+
+
+@pytest.mark.parametrize("n,H,G,dim,vdim,rot", [(1, 1, 0, 128, 32, 128), (33, 16, 4, 128, 128, 64), (297, 5, 1, 32, 96, 0), (300, 40, 8, 64, 64, 64),
+                                                (9, 3, 3, 96, 128, 64)])
+@pytest.mark.parametrize("norms", [False, True])
+def test_attention_front_end_rows(cuda_device, n, H, G, dim, vdim, rot, norms):
+    """prl_attn_front for heads of whole warps' widths, against 64 bits; idle rows leave the query buffer and the cache alone."""
+    from pipelinerl_b200 import _lib
+    lib, g = _lib.load(), torch.Generator(device="cuda").manual_seed(n + H)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    nq, nk, nv = H * dim, G * dim, G * vdim
+    P, qb, kb, vb, qg, kg = rnd(n, nq + nk + nv + 3), rnd(nq), rnd(max(nk, 1)), rnd(max(nv, 1)), rnd(dim), rnd(dim)
+    page, blocks = 16, 40
+    pos = torch.randint(0, page * blocks, (n,), generator=g, device="cuda", dtype=torch.int32)
+    slot = torch.arange(n, device="cuda", dtype=torch.int32)
+    slot[n // 2] = -1 if n > 1 else 0
+    table = torch.randperm(n * blocks, generator=g, device="cuda").to(torch.int32).view(n, blocks)
+    freq = 1e4 ** (-torch.arange(max(rot // 2, 1), device="cuda", dtype=torch.float64) / max(rot // 2, 1))
+    q = torch.full((n, H, dim), 9.0, device="cuda")
+    kp, vp = torch.full((n * blocks, max(G, 1), page, dim), 9.0, device="cuda"), torch.full((n * blocks, max(G, 1), page, vdim), 9.0, device="cuda")
+    first, lam, ptr = rnd(n, max(nv, 1)), torch.tensor([0.3], device="cuda"), lambda t: t.data_ptr()  # noqa: E731
+    blend = 2 if norms else 0
+    _lib.check(lib.prl_attn_front(ptr(P), P.shape[1], 0, nq, nq + nk, n, H, G, dim, vdim, ptr(qb), ptr(kb), ptr(vb), int(norms),
+                                  ptr(qg) if norms else None, ptr(kg) if norms else None, dim, 1e-5, rot, ptr(freq), 1.1, int(norms), blend,
+                                  ptr(lam), ptr(first), ptr(pos), ptr(slot), ptr(table), blocks, page, ptr(q), ptr(kp) if G else None,
+                                  ptr(vp) if G else None, 1, _lib.stream_ptr()))
+    rms = lambda v: v * torch.rsqrt((v * v).mean(-1, keepdim=True) + 1e-5) if norms else v  # noqa: E731
+    ang = pos.double()[:, None, None] * freq[:rot // 2]
+
+    def turned(v, gain):
+        v = rms(v.double()) * (gain.double() if norms else 1.0)
+        u, w = v[..., :rot // 2], v[..., rot // 2:rot]
+        c, s = 1.1 * torch.cos(ang), 1.1 * torch.sin(ang)
+        return torch.cat([u * c - w * s, w * c + u * s, v[..., rot:]], -1)
+    live = slot >= 0
+    near = lambda a, b: (a.double() - b).abs().max() <= 3e-6 * max(1.0, b.abs().max().item())  # noqa: E731
+    assert near(q[live], turned((P[:, :nq] + qb).view(n, H, dim), qg)[live]) and (q[~live] == 9).all()
+    written = torch.zeros(n * blocks, page, dtype=torch.bool, device="cuda")
+    if G:
+        at = table[torch.arange(n, device="cuda"), (pos // page).long()].long(), (pos % page).long()
+        written[at[0][live], at[1][live]] = True
+        v = rms((P[:, nq + nk:nq + nk + nv] + vb).view(n, G, vdim).double())
+        v = 0.7 * v + 0.3 * first.view(n, G, vdim).double() if norms else v
+        assert near(kp[at[0], :, at[1]][live], turned((P[:, nq:nq + nk] + kb).view(n, G, dim), kg)[live]) and near(vp[at[0], :, at[1]][live], v[live])
+    assert (kp.transpose(1, 2)[~written] == 9).all() and (vp.transpose(1, 2)[~written] == 9).all()
