@@ -246,19 +246,29 @@ int launch_mma(const void* q, const void* kp, const void* vp, const int32_t* bt,
 // The query heads that share a key / value head are the rows of one 16-row product (up to 16 per CTA), so a key is read once
 // for all of them.  CTA = 4 warps of one (segment, key / value head, group of 16 heads); the warps take the visible key tiles
 // (32 keys at absolute multiples of 32: the kept first tokens, then the window) in turn, each through a pipeline of its own
-// (two buffers filled by cp.async, no barrier between the warps), and their partial softmaxes are merged in warp order.
-constexpr int kDecWarps = 4, kDecKeys = 32, kDecHeads = 16;
+// (two to four buffers filled by cp.async, no barrier between the warps), and their partial softmaxes are merged in warp order.
+// Bound by latency: a warp's tiles are a chain, a tile's copies wait for its page.  So as many buffers as shared memory holds beside the
+// CTAs that the grid puts on an SM, and the pages of the next 32 tiles in the lanes of the warp.  Which keys a warp adds, and their
+// order, do not depend on the buffers.  24.6 -> 18.1 us for
+// 32 x 1024 keys, 16 / 4 heads of 128 (67 MB: 10.3 us at the copy rate), 72.8 -> 44.2 for 16 x 4000, 31.8 -> 26.6 for 32 x 2000, 8 / 8 of 64.
+constexpr int kDecWarps = 4, kDecKeys = 32, kDecHeads = 16, kDecMaxBufs = 4;
 
-template <int DV, bool OUT_BF16>
+// D: key size at compile time for square heads of 64 and 128 (score loop and copies without address arithmetic), or 0 = dim_rt.
+// TWO: more than eight heads share a key head; without, the upper eight rows of the products belong to none and take no softmax.
+template <int D, int DV, bool TWO, bool OUT_BF16>
 __global__ void __launch_bounds__(kDecWarps * 32) attn_mma_decode_kernel(
     const bf16* __restrict__ q, const bf16* __restrict__ k_pool, const bf16* __restrict__ v_pool, const int32_t* __restrict__ block_table,
     int max_blocks, int page_size, const int32_t* __restrict__ seg_start, const int32_t* __restrict__ seg_len,
-    const int32_t* __restrict__ seg_pos0, const int32_t* __restrict__ seg_slot, int H, int G, int dim, float scale, int window,
-    int keep_first, float softcap, const float* __restrict__ sink, const float* __restrict__ gate, int64_t ldg,
+    const int32_t* __restrict__ seg_pos0, const int32_t* __restrict__ seg_slot, int H, int G, int dim_rt, float scale, int window,
+    int keep_first, float softcap, const float* __restrict__ sink, const float* __restrict__ gate, int64_t ldg, int bufs,
     void* __restrict__ out_v) {
   pdl_wait();
+  pdl_launch_dependents();                               // the output projection's weights
   const int seg = blockIdx.y;
-  if (seg_len[seg] != 1) return;
+  const int len = seg_len[seg], slot = seg_slot[seg], pos = seg_pos0[seg];
+  const int64_t row = seg_start[seg];
+  if (len != 1) return;
+  const int dim = D ? D : dim_rt;
   const int LD = dim + kPadH, CH = dim / 8;
   constexpr int LDV = DV + kPadH, CHV = DV / 8;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -267,10 +277,8 @@ __global__ void __launch_bounds__(kDecWarps * 32) attn_mma_decode_kernel(
   const int g = blockIdx.x / groups, h0 = g * qpg + (blockIdx.x % groups) * kDecHeads;
   const int nh = min(kDecHeads, (g + 1) * qpg - h0);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int slot = seg_slot[seg], pos = seg_pos0[seg];
-  const int64_t row = seg_start[seg];
   const int tile_halves = kDecKeys * (LD + LDV);
-  bf16* mine = Qs + kDecHeads * LD + warp * 2 * tile_halves;      // this warp's two buffers: K [32][LD] | V [32][LDV]
+  bf16* mine = Qs + kDecHeads * LD + warp * bufs * tile_halves;   // this warp's buffers: K [32][LD] | V [32][LDV]
   const int lo = window > 0 ? max(0, pos - window + 1) : 0;
   const int sink_end = window > 0 ? min(keep_first, lo) : 0;
   const int tw = lo / kDecKeys, ts = min((sink_end + kDecKeys - 1) / kDecKeys, tw);
@@ -283,13 +291,32 @@ __global__ void __launch_bounds__(kDecWarps * 32) attn_mma_decode_kernel(
   auto first_key = [&](int t) { return (t < ts ? t : tw + t - ts) * kDecKeys; };
   const int dj = 32 / CH, dc = 32 % CH, j_first = lane / CH, c_first = lane % CH;
   const int djv = 32 / CHV, dcv = 32 % CHV, jv_first = lane / CHV, cv_first = lane % CHV;
-  auto stage = [&](int t, int buf) {                     // a tile lies inside one page: its rows are contiguous in the pools
+  int page = 0;                                          // lane i: the page of the warp's tile 32 * (i0 / 32) + i
+  auto stage = [&](int i, int buf) {                     // the warp's i-th tile, if it has one: a tile lies inside one page, its rows are contiguous in the pools
+    const int t = warp + kDecWarps * i;
+    if (t >= n_tiles) return;
+    if ((i & 31) == 0) {
+      const int tl = t + kDecWarps * lane;
+      page = tl < n_tiles ? bt[first_key(tl) / page_size] : 0;
+    }
     const int k0 = first_key(t), live = pos + 1 - k0;
-    const int64_t base = ((int64_t)bt[k0 / page_size] * G + g) * page_size + k0 % page_size;
+    const int64_t base = ((int64_t)__shfl_sync(0xffffffffu, page, i & 31) * G + g) * page_size + k0 % page_size;
     bf16* Ks = mine + buf * tile_halves;
     bf16* Vs = Ks + kDecKeys * LD;
     const bf16* kp = k_pool + base * dim;
     const bf16* vp = v_pool + base * DV;
+    if (D == DV && live >= kDecKeys) {                   // a lane keeps its 16-byte column of K and of V
+      constexpr int step = D ? 32 / (D / 8) : 1;
+      const bf16* ks = kp + j_first * D + c_first * 8;
+      const bf16* vs = vp + j_first * D + c_first * 8;
+      bf16* kd = Ks + j_first * LD + c_first * 8;
+      bf16* vd = Vs + j_first * LD + c_first * 8;
+#pragma unroll
+      for (int j = 0; j < kDecKeys; j += step) cp16(kd + j * LD, ks + j * D, 16);
+#pragma unroll
+      for (int j = 0; j < kDecKeys; j += step) cp16(vd + j * LD, vs + j * D, 16);
+      return;
+    }
     for (int j = j_first, c = c_first; j < kDecKeys;) {
       const bool ok = j < live;
       cp16(Ks + j * LD + c * 8, kp + (ok ? j * dim + c * 8 : 0), ok ? 16 : 0);
@@ -303,21 +330,30 @@ __global__ void __launch_bounds__(kDecWarps * 32) attn_mma_decode_kernel(
       if (c >= CHV) { c -= CHV; ++j; }
     }
   };
-  if (warp < n_tiles) stage(warp, 0);
-  asm volatile("cp.async.commit_group;" ::: "memory");   // the queries ride in this group
+  for (int i = 0; i < bufs - 1; ++i) {
+    stage(i, i);
+    asm volatile("cp.async.commit_group;" ::: "memory"); // the queries ride in the first group
+  }
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
   float o[DV / 8][4];
 #pragma unroll
   for (int j = 0; j < DV / 8; ++j)
 #pragma unroll
     for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  auto landed = [&](bool more) {                         // all but the last bufs - 2 (more: bufs - 1) groups
+    const int open = bufs - 2 + (more ? 1 : 0);
+    if (open == 0) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    else if (open == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else if (open == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else asm volatile("cp.async.wait_group 3;" ::: "memory");
+  };
+  landed(false);
   __syncthreads();                                       // the queries were staged by all warps
-  int buf = 0;
-  for (int t = warp; t < n_tiles; t += kDecWarps, buf ^= 1) {
-    if (t + kDecWarps < n_tiles) stage(t + kDecWarps, buf ^ 1);
+  int buf = 0, fill = bufs - 1;
+  for (int t = warp, i = 0; t < n_tiles; t += kDecWarps, ++i, buf = buf + 1 < bufs ? buf + 1 : 0, fill = fill + 1 < bufs ? fill + 1 : 0) {
+    stage(i + bufs - 1, fill);
     asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    landed(true);
     __syncwarp();
     const int k0 = first_key(t);
     const bf16* Ks = mine + buf * tile_halves;
@@ -327,7 +363,7 @@ __global__ void __launch_bounds__(kDecWarps * 32) attn_mma_decode_kernel(
     for (int j = 0; j < kDecKeys / 8; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) s[j][e] = 0.f;
-#pragma unroll 4
+#pragma unroll (D ? D / 16 : 4)
     for (int kk = 0; kk < dim; kk += 16) {
       uint32_t a[4];
       ldsm4(a, Qs + (lane & 15) * LD + kk + (lane >> 4) * 8);
@@ -339,21 +375,30 @@ __global__ void __launch_bounds__(kDecWarps * 32) attn_mma_decode_kernel(
         mma16816(s[2 * j + 1], a, b[2], b[3]);
       }
     }
+    constexpr int E = TWO ? 4 : 2;                       // accumulators of real rows in a fragment
+    if (softcap > 0.f) {                                 // one branch for the tile: sixteen small ones would serialise it
+#pragma unroll
+      for (int j = 0; j < kDecKeys / 8; ++j)
+#pragma unroll
+        for (int e = 0; e < E; ++e) s[j][e] = softcap * tanhf(s[j][e] * scale / softcap);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kDecKeys / 8; ++j)
+#pragma unroll
+        for (int e = 0; e < E; ++e) s[j][e] *= scale;
+    }
     float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
     for (int j = 0; j < kDecKeys / 8; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < E; ++e) {
         const int kt = k0 + 8 * j + (lane & 3) * 2 + (e & 1);
-        float v = s[j][e] * scale;
-        if (softcap > 0.f) v = softcap * tanhf(v / softcap);
-        v = kt <= pos && (kt >= lo || kt < keep_first) ? v : -INFINITY;
-        s[j][e] = v;
-        mx[e >> 1] = fmaxf(mx[e >> 1], v);
+        s[j][e] = kt <= pos && (kt >= lo || kt < keep_first) ? s[j][e] : -INFINITY;
+        mx[e >> 1] = fmaxf(mx[e >> 1], s[j][e]);
       }
     float corr[2], sum[2] = {0.f, 0.f};
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < E / 2; ++u) {
       mx[u] = fmaxf(mx[u], __shfl_xor_sync(0xffffffffu, mx[u], 1));
       mx[u] = fmaxf(mx[u], __shfl_xor_sync(0xffffffffu, mx[u], 2));
       const float m_new = fmaxf(m[u], mx[u]);            // finite: a listed tile has a visible key
@@ -363,20 +408,23 @@ __global__ void __launch_bounds__(kDecWarps * 32) attn_mma_decode_kernel(
 #pragma unroll
     for (int j = 0; j < kDecKeys / 8; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < E; ++e) {
         s[j][e] = expf(s[j][e] - m[e >> 1]);
         sum[e >> 1] += s[j][e];
       }
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < E / 2; ++u) {
       sum[u] += __shfl_xor_sync(0xffffffffu, sum[u], 1);
       sum[u] += __shfl_xor_sync(0xffffffffu, sum[u], 2);
       l[u] = l[u] * corr[u] + sum[u];
     }
 #pragma unroll
-    for (int j = 0; j < DV / 8; ++j) {
-      o[j][0] *= corr[0]; o[j][1] *= corr[0]; o[j][2] *= corr[1]; o[j][3] *= corr[1];
-    }
+    for (int j = 0; j < DV / 8; ++j)
+#pragma unroll
+      for (int e = 0; e < E; ++e) o[j][e] *= corr[e >> 1];
+    if (!TWO)
+#pragma unroll
+      for (int j = 0; j < kDecKeys / 8; ++j) s[j][2] = s[j][3] = 0.f;
 #pragma unroll
     for (int kt = 0; kt < kDecKeys / 16; ++kt) {
       const uint32_t a[4] = {pack_bf16(s[2 * kt][0], s[2 * kt][1]), pack_bf16(s[2 * kt][2], s[2 * kt][3]),
@@ -428,20 +476,26 @@ __global__ void __launch_bounds__(kDecWarps * 32) attn_mma_decode_kernel(
   }
 }
 
-template <int DV, bool OUT_BF16>
+template <int D, int DV, bool TWO, bool OUT_BF16>
 int launch_mma_decode(const void* q, const void* kp, const void* vp, const int32_t* bt, int max_blocks, int page_size,
                       const int32_t* ss, const int32_t* sl, const int32_t* sp, const int32_t* sslot, int n_seg, int H, int G, int dim,
                       float scale, int window, int keep_first, float softcap, const float* sink, const float* gate, int64_t ldg,
                       void* out, cudaStream_t st) {
-  const size_t tiles = ((size_t)kDecHeads * (dim + kPadH) + (size_t)kDecWarps * 2 * kDecKeys * (dim + DV + 2 * kPadH)) * sizeof(bf16);
+  const int groups = (H / G + kDecHeads - 1) / kDecHeads;
+  const size_t qs = (size_t)kDecHeads * (dim + kPadH) * sizeof(bf16);
+  const size_t set = (size_t)kDecWarps * kDecKeys * (dim + DV + 2 * kPadH) * sizeof(bf16);      // one buffer of every warp
+  // the CTAs that one SM gets share 224 KB (1 KB of each is the system's): more buffers than that would cost a wave
+  const int64_t per_sm = ((int64_t)G * groups * n_seg + 147) / 148;
+  int bufs = 2;
+  while (bufs < kDecMaxBufs && (int64_t)(qs + (bufs + 1) * set + 1024) * per_sm <= 224 * 1024) ++bufs;
+  const size_t tiles = qs + bufs * set;
   const size_t merge = (size_t)kDecWarps * kDecHeads * (DV + 2) * sizeof(float);
   const size_t smem = tiles > merge ? tiles : merge;
   static SmemAttr attr = {};
-  if (smem > 48 * 1024) PRL_CUDA(ensure_smem(attn_mma_decode_kernel<DV, OUT_BF16>, (int)smem, attr));
-  const int groups = (H / G + kDecHeads - 1) / kDecHeads;
-  PRL_CUDA(launch_pdl((attn_mma_decode_kernel<DV, OUT_BF16>), dim3(G * groups, n_seg), dim3(kDecWarps * 32), smem, st, (const bf16*)q,
+  if (smem > 48 * 1024) PRL_CUDA(ensure_smem(attn_mma_decode_kernel<D, DV, TWO, OUT_BF16>, (int)smem, attr));
+  PRL_CUDA(launch_pdl((attn_mma_decode_kernel<D, DV, TWO, OUT_BF16>), dim3(G * groups, n_seg), dim3(kDecWarps * 32), smem, st, (const bf16*)q,
                       (const bf16*)kp, (const bf16*)vp, bt, max_blocks, page_size, ss, sl, sp, sslot, H, G, dim, scale, window, keep_first,
-                      softcap, sink, gate, ldg, out));
+                      softcap, sink, gate, ldg, bufs, out));
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }
@@ -481,15 +535,18 @@ int attn_mma_decode_launch(const void* q, const void* kp, const void* vp, const 
                            const int32_t* ss, const int32_t* sl, const int32_t* sp, const int32_t* sslot, int n_seg, int H, int G,
                            int dim, int vdim, float scale, int window, int keep_first, float softcap, const float* sink,
                            const float* gate, int64_t ldg, int out_is_bf16, void* out, cudaStream_t st) {
-#define PRL_MMAD(DV) (out_is_bf16 ? launch_mma_decode<DV, true>(q, kp, vp, bt, max_blocks, page_size, ss, sl, sp, sslot, n_seg, H, G, dim, scale, window, keep_first, softcap, sink, gate, ldg, out, st) \
-                                  : launch_mma_decode<DV, false>(q, kp, vp, bt, max_blocks, page_size, ss, sl, sp, sslot, n_seg, H, G, dim, scale, window, keep_first, softcap, sink, gate, ldg, out, st))
+#define PRL_MMAD(D, DV, TWO) (out_is_bf16 ? launch_mma_decode<D, DV, TWO, true>(q, kp, vp, bt, max_blocks, page_size, ss, sl, sp, sslot, n_seg, H, G, dim, scale, window, keep_first, softcap, sink, gate, ldg, out, st) \
+                                  : launch_mma_decode<D, DV, TWO, false>(q, kp, vp, bt, max_blocks, page_size, ss, sl, sp, sslot, n_seg, H, G, dim, scale, window, keep_first, softcap, sink, gate, ldg, out, st))
+  const bool two = H / G > 8;
+  if (dim == 64 && vdim == 64) return two ? PRL_MMAD(64, 64, true) : PRL_MMAD(64, 64, false);
+  if (dim == 128 && vdim == 128) return two ? PRL_MMAD(128, 128, true) : PRL_MMAD(128, 128, false);
   switch (vdim) {
-    case 16: return PRL_MMAD(16);
-    case 32: return PRL_MMAD(32);
-    case 48: return PRL_MMAD(48);
-    case 64: return PRL_MMAD(64);
-    case 96: return PRL_MMAD(96);
-    default: return PRL_MMAD(128);
+    case 16: return two ? PRL_MMAD(0, 16, true) : PRL_MMAD(0, 16, false);
+    case 32: return two ? PRL_MMAD(0, 32, true) : PRL_MMAD(0, 32, false);
+    case 48: return two ? PRL_MMAD(0, 48, true) : PRL_MMAD(0, 48, false);
+    case 64: return two ? PRL_MMAD(0, 64, true) : PRL_MMAD(0, 64, false);
+    case 96: return two ? PRL_MMAD(0, 96, true) : PRL_MMAD(0, 96, false);
+    default: return two ? PRL_MMAD(0, 128, true) : PRL_MMAD(0, 128, false);
   }
 #undef PRL_MMAD
 }

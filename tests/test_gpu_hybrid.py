@@ -454,3 +454,32 @@ def test_attention_front_end_rows(cuda_device, n, H, G, dim, vdim, rot, norms):
         v = 0.7 * v + 0.3 * first.view(n, G, vdim).double() if norms else v
         assert near(kp[at[0], :, at[1]][live], turned((P[:, nq:nq + nk] + kb).view(n, G, dim), kg)[live]) and near(vp[at[0], :, at[1]][live], v[live])
     assert (kp.transpose(1, 2)[~written] == 9).all() and (vp.transpose(1, 2)[~written] == 9).all()
+
+
+@pytest.mark.parametrize("B,H,G,dim,vdim,window,keep_first", [(1, 4, 4, 128, 128, 0, 0), (3, 16, 1, 128, 128, 70, 5), (5, 9, 1, 64, 64, 0, 0), (40, 8, 8, 64, 64, 33, 0),
+                                                              (300, 4, 2, 32, 32, 0, 0), (2, 24, 2, 96, 64, 500, 40), (2, 40, 2, 256, 128, 0, 0)])
+def test_decode_attention_of_single_tokens(cuda_device, B, H, G, dim, vdim, window, keep_first):
+    """prl_attn_any_gated for one query per sequence: contexts around the key tiles (32), the warps' turns (128) and the pages a warp
+    holds at a time (32 tiles of four warps: 4096 keys), with sink and gate; two to four staging buffers, by the CTAs on an SM."""
+    from pipelinerl_b200 import _lib
+    lib, g = _lib.load(), torch.Generator(device="cuda").manual_seed(B + H)
+    lens = [1, 31, 32, 33, 129, 700, 4097, 4200]
+    n = torch.tensor([lens[(i + B) % (8 if B < 10 else 6)] for i in range(B)], dtype=torch.int32, device="cuda")
+    page, blocks = 64, 66
+    table = torch.randperm(B * blocks, generator=g, device="cuda").to(torch.int32).view(B, blocks)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()  # noqa: E731
+    q, kp, vp = rnd(B, H, dim), rnd(B * blocks, G, page, dim), rnd(B * blocks, G, page, vdim)
+    sink, gate, ids, ptr = rnd(H).float(), rnd(B, H).float(), torch.arange(B, dtype=torch.int32, device="cuda"), lambda t: t.data_ptr()  # noqa: E731
+    out, one, pos = torch.empty(B, H, vdim, device="cuda"), torch.ones(B, dtype=torch.int32, device="cuda"), n - 1
+    _lib.check(lib.prl_attn_any_gated(ptr(q), ptr(kp), ptr(vp), vdim, 0, ptr(table), blocks, page, ptr(ids), ptr(one), ptr(pos), ptr(ids), B, 1, H, G,
+                                      dim, vdim, dim ** -0.5, window, keep_first, 0.0, ptr(sink), ptr(gate), H, 0, ptr(out), _lib.stream_ptr()))
+    for b in range(0, B, max(1, B // 8)):
+        k, v = (t[table[b].long()].transpose(0, 1).reshape(G, -1, t.shape[-1])[:, :n[b]].double() for t in (kp, vp))
+        s = torch.einsum("ghd,gkd->ghk", q[b].double().view(G, H // G, dim), k) * dim ** -0.5
+        at = torch.arange(int(n[b]), device="cuda")
+        if window:
+            s = s.masked_fill((at < int(n[b]) - window) & (at >= keep_first), float("-inf"))
+        s = torch.cat([s, sink.double().view(G, -1, 1)], -1)
+        want = (torch.einsum("ghk,gkd->ghd", torch.softmax(s, -1)[..., :-1], v).view(H, vdim)) * torch.sigmoid(gate[b].double())[:, None]
+        # probabilities are rounded to bf16 before the second product: 2^-9 each, averaged over the keys
+        assert (out[b].double() - want).norm() < 4e-3 * want.norm() + 1e-6
