@@ -183,35 +183,51 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   const int kb_end = (int)(((int64_t)p.kblocks * (split + 1)) / p.split_k);
   const int n_kb = kb_end - kb_begin;
 
-  // Thread 0 arms the barriers and IMMEDIATELY fills the first ring pass with WEIGHT tiles: weights do not depend on
+  // Both issuing warps run CONVERGED and elect one lane around each batch of instructions: from inside `if (lane == 0)` every UMMA and
+  // TMA pays an operand waterfall of ~180 cycles (tc_ptx.cuh, elect_one).  A k-block of four UMMAs then took 0.36 us whatever the tile,
+  // twice what its 16 KB of weights take from HBM on one CTA per SM: 32 x 9232 x 2048 14.9 -> 12.9 us, 4 x 8192 x 1024 by two 5.2 -> 5.0,
+  // 64 x 152064 x 3584 193 -> 188.
+  auto load_weights = [&](int i, uint32_t a_dst, uint32_t bar) {
+    const int kcoord = (kb_begin + i) * kBlockK;
+    const int wc0 = p.tiled ? 0 : kcoord;
+    const int wc1 = p.tiled ? (n_tile * p.kblocks + kb_begin + i) * kBlockM : n0;
+    if (p.dual_kb && kb_begin + i >= p.dual_kb) {
+      ptx::tma_load_2d(a_dst, &tm_wlo, kcoord - p.dual_kb * kBlockK, n0, bar, ptx::kEvictFirst);
+    } else if (p.swiglu_I) {   // tm_w boxes are 64 rows here: gate half, then up half of the same 64 features
+      ptx::tma_load_2d(a_dst, &tm_w, wc0, n_tile * 64, bar, ptx::kEvictFirst);
+      ptx::tma_load_2d(a_dst + L::kABytes / 2, &tm_w, wc0, (int)p.swiglu_I + n_tile * 64, bar, ptx::kEvictFirst);
+    } else {
+      ptx::tma_load_2d(a_dst, &tm_w, wc0, wc1, bar, ptx::kEvictFirst);
+    }
+    if (lo) ptx::tma_load_2d(a_dst + L::kABytes, &tm_wlo, wc0, wc1, bar, ptx::kEvictFirst);
+  };
+  auto load_tokens = [&](int i, uint32_t a_dst, uint32_t bar) {
+    const bool second = p.dual_kb && kb_begin + i >= p.dual_kb;
+    ptx::tma_load_2d(a_dst + L::kABytes * (lo ? 2 : 1), second ? &tm_x2 : &tm_x, (kb_begin + i - (second ? p.dual_kb : 0)) * kBlockK, m0, bar,
+                     ptx::kEvictLast);
+  };
+  // Warp 0 arms the barriers and IMMEDIATELY fills the first ring pass with WEIGHT tiles: weights do not depend on
   // the preceding kernel (PDL lets this run under the predecessor's tail) nor on the rest of this CTA's prologue
   // (TMEM allocation, descriptor prefetch), so the first HBM round trip overlaps both.
   const int pre = n_kb < n_stages ? n_kb : n_stages;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < n_stages; ++s) {
-      ptx::mbar_init(full_bar(s), 1);
-      ptx::mbar_init(empty_bar(s), 1);
-    }
-    ptx::mbar_init(tmem_full_bar, 1);
-    ptx::fence_barrier_init();
-    ptx::fence_proxy_async();
-    for (int i = 0; i < pre; ++i) {
-      ptx::mbar_arrive_expect_tx(full_bar(i), (uint32_t)stage_bytes);
-      const uint32_t a_dst = smem_base + (uint32_t)(i * stage_bytes);
-      const int kcoord = (kb_begin + i) * kBlockK;
-      const int wc0 = p.tiled ? 0 : kcoord;
-      const int wc1 = p.tiled ? (n_tile * p.kblocks + kb_begin + i) * kBlockM : n0;
-      if (p.dual_kb && kb_begin + i >= p.dual_kb) {
-        ptx::tma_load_2d(a_dst, &tm_wlo, kcoord - p.dual_kb * kBlockK, n0, full_bar(i), ptx::kEvictFirst);
-      } else if (p.swiglu_I) {   // tm_w boxes are 64 rows here: gate half, then up half of the same 64 features
-        ptx::tma_load_2d(a_dst, &tm_w, wc0, n_tile * 64, full_bar(i), ptx::kEvictFirst);
-        ptx::tma_load_2d(a_dst + L::kABytes / 2, &tm_w, wc0, (int)p.swiglu_I + n_tile * 64, full_bar(i), ptx::kEvictFirst);
-      } else {
-        ptx::tma_load_2d(a_dst, &tm_w, wc0, wc1, full_bar(i), ptx::kEvictFirst);
+  if (warp == 0) {
+    if (ptx::elect_one()) {
+      for (int s = 0; s < n_stages; ++s) {
+        ptx::mbar_init(full_bar(s), 1);
+        ptx::mbar_init(empty_bar(s), 1);
       }
-      if (lo) ptx::tma_load_2d(a_dst + L::kABytes, &tm_wlo, wc0, wc1, full_bar(i), ptx::kEvictFirst);
+      ptx::mbar_init(tmem_full_bar, 1);
+      ptx::fence_barrier_init();
+      ptx::fence_proxy_async();
     }
-    ptx::prefetch_tensormap(&tm_x);
+    __syncwarp();
+    for (int i = 0; i < pre; ++i)
+      if (ptx::elect_one()) {
+        ptx::mbar_arrive_expect_tx(full_bar(i), (uint32_t)stage_bytes);
+        load_weights(i, smem_base + (uint32_t)(i * stage_bytes), full_bar(i));
+      }
+    if (ptx::elect_one()) ptx::prefetch_tensormap(&tm_x);
+    __syncwarp();
   }
   if (warp == 1) {
     ptx::tmem_alloc(tmem_slot, kNTile < 32 ? 32 : kNTile);
@@ -224,72 +240,51 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
 
   if (warp == 0) {
-    // ===== TMA producer =====  (first-pass weight tiles were issued by thread 0 before the CTA-wide sync)
-    if (lane == 0) {
-      const uint32_t tx = (uint32_t)stage_bytes;
-      pdl_wait();
-      for (int i = 0; i < pre; ++i) {
-        const uint32_t b_dst = smem_base + (uint32_t)(i * stage_bytes) + L::kABytes * (lo ? 2 : 1);
-        const bool second = p.dual_kb && kb_begin + i >= p.dual_kb;
-        ptx::tma_load_2d(b_dst, second ? &tm_x2 : &tm_x, (kb_begin + i - (second ? p.dual_kb : 0)) * kBlockK, m0, full_bar(i),
-                         ptx::kEvictLast);
+    // ===== TMA producer =====  (first-pass weight tiles were issued before the CTA-wide sync)
+    pdl_wait();
+    for (int i = 0; i < pre; ++i)
+      if (ptx::elect_one()) load_tokens(i, smem_base + (uint32_t)(i * stage_bytes), full_bar(i));
+    __syncwarp();
+    for (int i = pre; i < n_kb; ++i) {
+      const int s = i % n_stages;
+      const uint32_t ph = (uint32_t)((i / n_stages) & 1);
+      ptx::mbar_wait(empty_bar(s), ph ^ 1u);
+      if (ptx::elect_one()) {
+        ptx::mbar_arrive_expect_tx(full_bar(s), (uint32_t)stage_bytes);
+        load_weights(i, smem_base + (uint32_t)(s * stage_bytes), full_bar(s));
+        load_tokens(i, smem_base + (uint32_t)(s * stage_bytes), full_bar(s));
       }
-      for (int i = pre; i < n_kb; ++i) {
-        const int s = i % n_stages;
-        const uint32_t ph = (uint32_t)((i / n_stages) & 1);
-        ptx::mbar_wait(empty_bar(s), ph ^ 1u);
-        ptx::mbar_arrive_expect_tx(full_bar(s), tx);
-        const uint32_t a_dst = smem_base + (uint32_t)(s * stage_bytes);
-        const int kcoord = (kb_begin + i) * kBlockK;
-        const int wc0 = p.tiled ? 0 : kcoord;
-        const int wc1 = p.tiled ? (n_tile * p.kblocks + kb_begin + i) * kBlockM : n0;
-        const bool second = p.dual_kb && kb_begin + i >= p.dual_kb;
-        const int kcoord2 = second ? kcoord - p.dual_kb * kBlockK : kcoord;
-        if (second) {
-          ptx::tma_load_2d(a_dst, &tm_wlo, kcoord2, n0, full_bar(s), ptx::kEvictFirst);
-        } else if (p.swiglu_I) {
-          ptx::tma_load_2d(a_dst, &tm_w, wc0, n_tile * 64, full_bar(s), ptx::kEvictFirst);
-          ptx::tma_load_2d(a_dst + L::kABytes / 2, &tm_w, wc0, (int)p.swiglu_I + n_tile * 64, full_bar(s), ptx::kEvictFirst);
-        } else {
-          ptx::tma_load_2d(a_dst, &tm_w, wc0, wc1, full_bar(s), ptx::kEvictFirst);
-        }
-        uint32_t b_dst = a_dst + L::kABytes;
-        if (lo) {
-          ptx::tma_load_2d(a_dst + L::kABytes, &tm_wlo, wc0, wc1, full_bar(s), ptx::kEvictFirst);
-          b_dst += L::kABytes;
-        }
-        ptx::tma_load_2d(b_dst, second ? &tm_x2 : &tm_x, kcoord2, m0, full_bar(s), ptx::kEvictLast);
-      }
+      __syncwarp();
     }
   } else if (warp == 1) {
     // ===== MMA issuer =====
-    if (lane == 0) {
-      constexpr uint32_t idesc = ptx::make_idesc_bf16_f32(kBlockM, kNTile);
-      for (int i = 0; i < n_kb; ++i) {
-        const int s = i % n_stages;
-        const uint32_t ph = (uint32_t)((i / n_stages) & 1);
-        ptx::mbar_wait(full_bar(s), ph);
-        ptx::tc_fence_after_sync();
-        const uint32_t a_addr = smem_base + (uint32_t)(s * stage_bytes);
-        const uint32_t b_addr = a_addr + L::kABytes * (lo ? 2 : 1);
-        const uint64_t a_desc = ptx::make_kmajor_sw128_desc(a_addr);
-        const uint64_t b_desc = ptx::make_kmajor_sw128_desc(b_addr);
+    constexpr uint32_t idesc = ptx::make_idesc_bf16_f32(kBlockM, kNTile);
+    const uint32_t d_tmem = ptx::warp_uniform(tmem_base), sm0 = ptx::warp_uniform(smem_base);
+    for (int i = 0; i < n_kb; ++i) {
+      const int s = i % n_stages;
+      const uint32_t ph = (uint32_t)((i / n_stages) & 1);
+      ptx::mbar_wait(full_bar(s), ph);
+      ptx::tc_fence_after_sync();
+      const uint32_t a_addr = sm0 + (uint32_t)(s * stage_bytes);
+      const uint64_t a_desc = ptx::make_kmajor_sw128_desc(a_addr);
+      const uint64_t al_desc = ptx::make_kmajor_sw128_desc(a_addr + L::kABytes);
+      const uint64_t b_desc = ptx::make_kmajor_sw128_desc(a_addr + L::kABytes * (lo ? 2 : 1));
+      if (ptx::elect_one()) {
 #pragma unroll
         for (int k = 0; k < kBlockK / kUmmaK; ++k) {
           // advancing K by 16 bf16 = 32 B inside the 128-B swizzle atom: +2 in the (addr >> 4) field
-          ptx::mma_bf16_ss(tmem_base, a_desc + (uint64_t)(2 * k), b_desc + (uint64_t)(2 * k), idesc,
-                           (i > 0 || k > 0) ? 1u : 0u);
+          ptx::mma_bf16_ss(d_tmem, a_desc + (uint64_t)(2 * k), b_desc + (uint64_t)(2 * k), idesc, (i > 0 || k > 0) ? 1u : 0u);
         }
         if (lo) {
-          const uint64_t al_desc = ptx::make_kmajor_sw128_desc(a_addr + L::kABytes);
 #pragma unroll
           for (int k = 0; k < kBlockK / kUmmaK; ++k)
-            ptx::mma_bf16_ss(tmem_base, al_desc + (uint64_t)(2 * k), b_desc + (uint64_t)(2 * k), idesc, 1u);
+            ptx::mma_bf16_ss(d_tmem, al_desc + (uint64_t)(2 * k), b_desc + (uint64_t)(2 * k), idesc, 1u);
         }
         ptx::tc_commit(empty_bar(s));  // frees the smem slot when these MMAs have read it
       }
-      ptx::tc_commit(tmem_full_bar);   // accumulator complete
+      __syncwarp();
     }
+    if (ptx::elect_one()) ptx::tc_commit(tmem_full_bar);   // accumulator complete
     __syncwarp();
   } else {
     // ===== epilogue =====
