@@ -177,3 +177,20 @@ def test_token_step_swiglu_epilogue_is_bit_identical_to_gemm_plus_silu(cuda_devi
     ref = x.float() @ W.float().t()
     fp32 = torch.nn.functional.silu(ref[:, :I]) * ref[:, I:]
     assert (got.float() - fp32).abs().max().item() <= 2 ** -7 * fp32.abs().max().item() + 1e-6
+
+
+@pytest.mark.parametrize("M", [1, 17, 64])
+@pytest.mark.parametrize("N,K", [(8, 8), (1000, 2056), (4736, 72), (4737, 1024), (9232, 2048), (9472, 200), (9473, 64)])
+def test_short_weight_tiles_keep_the_bits(cuda_device, M, N, K):
+    """An unsplit product of few weight tiles takes tiles of 32 (up to 37 of 128 rows) or 64 rows (up to 74): the same bits as the
+    leading rows of a product wide enough for whole tiles, and the fp32 product within the rounding of its sums."""
+    from pipelinerl_b200 import _lib
+    lib, st, g = _lib.load(), _lib.stream_ptr(), torch.Generator(device="cuda").manual_seed(N + K + M)
+    x = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    w = torch.randn(9600, K, generator=g, device="cuda").bfloat16()
+    got, wide = torch.full((M, N), float("nan"), device="cuda"), torch.empty(M, 9600, device="cuda")
+    _lib.check(lib.prl_gemm_bf16_splitk(w.data_ptr(), None, x.data_ptr(), M, N, K, 1, got.data_ptr(), st))
+    _lib.check(lib.prl_gemm_bf16_splitk(w.data_ptr(), None, x.data_ptr(), M, 9600, K, 1, wide.data_ptr(), st))
+    assert torch.equal(got, wide[:, :N])
+    want = x.double() @ w[:N].double().T
+    assert (got - want).abs().max() <= 2.0 ** -20 * K ** 0.5 * 8 * max(1.0, want.abs().max().item() / K ** 0.5)
