@@ -1344,6 +1344,9 @@ class HybridEngine(EngineCore):
         self.split_scan = not self.f32
         self.split_min_rows = 256
         self.piece_tokens = 64             # tokens per piece (tests lower it); at most prl_lin_scan_piece_tokens()
+        # The two branches of an attention-beside-delta-rule layer on two streams; they share no buffer they write.  Off: one after the other.
+        self.side_branches = True
+        self._side = None                  # the second stream and its two events, made with the first such layer
         self._rows: _Rows | None = None
         super().__init__(cfg, arena, **kw)
 
@@ -2088,10 +2091,29 @@ class HybridEngine(EngineCore):
         a, g, W = L.attn, L.gdelta, self.cfg.width
         C = self.cfg.attn_delta_rows(L)
         self._mm(R.xa, W, w + "mix.in", C.total, R.P, n)
-        self._gated_window_attn(R, n, i, a, C, segs, max_q, row_pos, seg_pos0)
-        k0 = self._mm(R.ya, a.heads * a.vdim, w + "mix.left.o", W, R.y0, n, split=True)
-        self._gated_delta_cell(R, n, i, g, w + "mix.right.", segs, max_q, R.P.data_ptr(), C.total, C.right, C.b, C.a, C.right_g)
-        k1 = self._mm(R.yb, g.heads * g.vdim, w + "mix.right.o", W, R.y1, n, split=True)
+        # The attention branch (q, ya, y0, the caches) beside the delta rule's (aux, dprep, scratch, o, yb, y1, the states): neither fills the
+        # chip alone -- the walk over a prompt's pieces is a serial chain, a token step's state update and attention wait for memory.
+        main, st = torch.cuda.current_stream(), self._st
+        if self.side_branches:
+            if self._side is None:
+                self._side = (torch.cuda.Stream(self.dev), torch.cuda.Event(), torch.cuda.Event())
+            side, fork, join = self._side
+            fork.record(main)
+            side.wait_event(fork)
+            self._st = side.cuda_stream
+        try:
+            try:
+                self._gated_window_attn(R, n, i, a, C, segs, max_q, row_pos, seg_pos0)
+                k0 = self._mm(R.ya, a.heads * a.vdim, w + "mix.left.o", W, R.y0, n, split=True)
+            finally:
+                self._st = st
+                if self.side_branches:
+                    join.record(side)
+            self._gated_delta_cell(R, n, i, g, w + "mix.right.", segs, max_q, R.P.data_ptr(), C.total, C.right, C.b, C.a, C.right_g)
+            k1 = self._mm(R.yb, g.heads * g.vdim, w + "mix.right.o", W, R.y1, n, split=True)
+        finally:
+            if self.side_branches:
+                main.wait_event(join)
         return k0, k1
 
     def _gated_window_attn(self, R, n, i, a, C, segs, max_q, row_pos, seg_pos0) -> None:

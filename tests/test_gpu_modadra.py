@@ -365,6 +365,26 @@ def test_bf16_serving_mode(cuda_device, plain_gemm):
     assert mc.rel_err(whole[clear], ref[clear]) < 3 * least + 1e-3
 
 
+@pytest.mark.parametrize("graph", [False, True])
+def test_branches_on_two_streams_equal_one_after_the_other(cuda_device, graph):
+    """The attention and delta-rule branches of a layer run beside each other, in prompts and in the (captured) token step: the same
+    tokens and log-probabilities as one after the other, also from a stream of the caller's."""
+    from pipelinerl_b200.engine import SamplingParams
+    wt = mc.weights(BIG, 5)
+    prompts, got = [mc.tokens_for(BIG, n, seed=n) for n in (400, 300, 5)], []
+    for side, own in ((True, False), (False, False), (True, True)):
+        eng = mc.build_engine(BIG, wt, torch.bfloat16, cuda_device, max_batch=3, max_seq_len=700, use_cuda_graph=graph)
+        eng.side_branches = side
+        s = torch.cuda.Stream() if own else torch.cuda.current_stream()
+        s.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(s):
+            outs = eng.generate(prompts, SamplingParams(max_tokens=9, greedy=True, ignore_eos=True))
+        torch.cuda.synchronize()
+        assert (eng._side is not None) == side
+        got.append([(list(r.output_ids), list(r.output_logprobs)) for r in outs])
+    assert got[0] == got[1] == got[2]
+
+
 def test_grouped_tensor_core_experts_in_long_prompts(cuda_device):
     """More routed pairs per expert than the few-row grouped GEMM is for: the tcgen05 grouped GEMM with the gelu epilogue
     against the few-row kernel on the same weights."""
