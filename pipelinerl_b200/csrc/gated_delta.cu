@@ -123,7 +123,7 @@ struct StepArgs {
   void* out;                  // [row][heads * dv]
 };
 
-// blockDim = 256 * (value heads in flight, 1 or 2); R float4 of a column per lane, eight lanes per column; VEC: dk % 4 == 0
+// blockDim = 256 * (value heads in flight, 1 or 2: the same sums); R float4 of a column per lane, eight lanes per column; VEC: dk % 4 == 0
 template <typename T, int R, bool VEC>
 __global__ void __launch_bounds__(512) gated_delta_step_kernel(StepArgs a) {
   pdl_wait();
@@ -911,7 +911,10 @@ extern "C" int prl_gated_delta_step(const float* P, int64_t ldp, int32_t off, in
                 "prl_gated_delta_step: bad shape (heads=%d q/k heads=%d dk=%d dv=%d taps=%d)", heads, kh, dk, dv, taps);
   const StepArgs a{P, ldp, off, off_b, off_a, off_g, conv_w, taps, A_log, dt_bias, unit_eps, gain, eps, heads, kh, dk, dv,
                    seg_start, seg_len, seg_slot, conv_state, state, out};
-  const int rep = heads / kh, groups = rep > 1 ? 2 : 1, R = dk <= 32 ? 1 : dk <= 64 ? 2 : dk <= 128 ? 4 : 8;
+  // Two value heads at a time fill an SM's registers with one CTA: the shortest chain while every CTA has an SM of its own (8 / 16 heads of
+  // 128: 18 rows 9.3 us, one at a time 11.9).  Past that one head at a time, two CTAs on an SM, and room for another branch's kernel beside
+  // them (19 rows 16.1 -> 14.2, 32 rows 22.9 -> 19.5, 64 rows 42.4 -> 34.5).
+  const int rep = heads / kh, groups = rep > 1 && (int64_t)kh * n_seg <= 148 ? 2 : 1, R = dk <= 32 ? 1 : dk <= 64 ? 2 : dk <= 128 ? 4 : 8;
   const bool vec = dk % 4 == 0 && ((uintptr_t)state & 15) == 0;
   const size_t smem = ((size_t)2 * 32 * R + (size_t)(groups + rep) * dv) * sizeof(float);
   static SmemAttr attr[16] = {};

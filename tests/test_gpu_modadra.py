@@ -485,6 +485,29 @@ def test_token_step_of_the_gated_delta_rule(cuda_device, heads, kv, dk, dv, taps
     assert mc.rel_err(torch.cat(out).double().cpu(), ref[:at]) < F32_TOL
 
 
+@pytest.mark.parametrize("heads,kh,dk,dv", [(16, 8, 128, 128), (4, 2, 64, 48), (6, 2, 20, 36), (4, 4, 32, 64)])
+def test_token_step_of_many_rows_equals_few(cuda_device, heads, kh, dk, dv):
+    """One value head at a time in a CTA (more than 148 CTAs) or two: the same bits, for outputs, states and convolution inputs."""
+    from pipelinerl_b200 import _lib
+    lib, g = _lib.load(), torch.Generator(device="cuda").manual_seed(heads)
+    n = 148 // kh + 3
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    ch, ptr = 2 * kh * dk + heads * dv, lambda t: t.data_ptr()  # noqa: E731
+    P, conv_w, A, dt, gain = rnd(n, ch + heads * dv + 2 * heads), rnd(ch, 4), rnd(heads) * 0.1, rnd(heads), rnd(dv)
+    conv0, state0 = rnd(n, ch, 3), rnd(n, heads, dv, dk)
+    got = []
+    for part in (n, 3):
+        conv, state, out = conv0.clone(), state0.clone(), torch.full((n, heads * dv), float("nan"), device="cuda")
+        for a in range(0, n, part):
+            k = min(part, n - a)
+            rows, one = torch.arange(a, a + k, dtype=torch.int32, device="cuda"), torch.ones(k, dtype=torch.int32, device="cuda")
+            _lib.check(lib.prl_gated_delta_step(ptr(P), P.shape[1], 0, ch, ch + heads, ch + 2 * heads, ptr(conv_w), 4, ptr(A), ptr(dt), 1e-6, ptr(gain),
+                                                1e-5, heads, kh, dk, dv, ptr(rows), ptr(one), ptr(rows), k, ptr(conv), ptr(state), ptr(out), 1,
+                                                _lib.stream_ptr()))
+        got.append((out, state, conv))
+    assert all(torch.equal(a, b) for a, b in zip(*got)) and torch.isfinite(got[0][0]).all()
+
+
 @pytest.mark.parametrize("heads,kv_heads,window", [(2, 1, 37), (4, 1, 64), (8, 1, 129), (3, 3, 200), (16, 1, 90), (4, 2, 0), (4, 2, 1), (2, 2, 128)])
 def test_tcgen05_prompt_attention(cuda_device, heads, kv_heads, window):
     """Heads of 128 in bf16: the tcgen05 prompt kernel with its window, the constant sink and the head gates, against the
