@@ -806,6 +806,10 @@ int prl_moe_gemm_act(const void* A, int32_t a_is_f32, int64_t lda, int32_t a_mod
                      int64_t expert_stride, int64_t ldw, const int32_t* perm, const int32_t* meta, const int32_t* tiles,
                      int64_t max_tiles, int64_t N, int64_t K, int32_t act, const float* wsel, void* out, int64_t ld_out,
                      prl_stream_t stream);
+/* both products of ungated experts (prl_moe_gemm_act, then prl_moe_gemm in pair order) in one call */
+int prl_moe_mlp_act(const void* x, int32_t f32, int32_t n, const void* up, const void* down, int64_t W, int64_t F,
+                    const int32_t* perm, const int32_t* meta, const int32_t* tiles, int64_t max_tiles, int32_t act,
+                    const float* wsel, void* act_out, float* out, prl_stream_t stream);
 int prl_moe_glu(const float* gate_up, int64_t ld, int64_t pairs, int32_t F, const int32_t* perm, const float* wsel,
                 float limit, float beta, void* out, int32_t f32, prl_stream_t stream);
 

@@ -623,16 +623,25 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-template <int ACT>
+// Two products of a feed-forward launched together (prl_moe_mlp_act): the first (kPairFirst) lets the second start only after its own wait,
+// so the second (kPairSecond) knows its tile before it waits, and has its weights in flight when the first one's last CTA ends.  Both are
+// streams of weights with a ramp of four dependent loads: a hybrid token step of 32 rows, 4 layers 586 -> 579 us.  (The first's weights
+// asked for in L2 while the router runs: 512 or 1024 bytes of a row nothing, 2048 three us slower, whole rows ten.)
+enum { kPairNone = 0, kPairFirst = 1, kPairSecond = 2 };
+template <int ACT, int PAIR>
 __global__ void __launch_bounds__(256) moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, int a_mod,
                                                            const __nv_bfloat16* __restrict__ W, int64_t expert_stride,
                                                            int64_t ldw, const int32_t* __restrict__ perm,
                                                            const int32_t* __restrict__ meta, const int32_t* __restrict__ tiles,
                                                            int N, int K, void* __restrict__ C_v, int64_t ldc, int c_perm,
                                                            const float* __restrict__ wsel) {
-  pdl_wait();
   const int tile = blockIdx.y;
-  if (tile >= meta[0]) return;
+  if constexpr (PAIR != kPairSecond) pdl_wait();
+  if constexpr (PAIR == kPairFirst) pdl_launch_dependents();
+  if (tile >= meta[0]) {
+    if constexpr (PAIR == kPairSecond) pdl_wait();
+    return;
+  }
   extern __shared__ __align__(16) unsigned char mma_smem[];
   typedef __nv_bfloat16 (*ATile)[kTile][kLds];
   typedef __nv_bfloat16 (*BTile)[kBN][kLds];
@@ -663,30 +672,45 @@ __global__ void __launch_bounds__(256) moe_gemm_mma_kernel(const __nv_bfloat16* 
   // loaders: A 64 rows x 8 chunks of 8 halves (two per thread), B 128 rows x 8 chunks (four per thread)
   const int lr = tid >> 3, lc = (tid & 7) * 8;
   const int64_t a_off[2] = {(int64_t)a_row[lr] * lda, (int64_t)a_row[lr + 32] * lda};
-  auto stage = [&](int k0, int buf) {
+  auto stage_a = [&](int k0, int buf) {
     const int k = k0 + lc;
     const bool kin = k < K;
 #pragma unroll
     for (int h = 0; h < 2; ++h)
       if (32 * h < M)         // uniform: the upper half of a short tile is not staged, and the warps that own it do nothing
         cp_async16_zfill(&As[buf][lr + 32 * h][lc], A + a_off[h] + (kin ? k : 0), (kin && lr + 32 * h < M) ? 16 : 0);
+  };
+  auto stage_b = [&](int k0, int buf) {
+    const int k = k0 + lc;
+    const bool kin = k < K;
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
       const int r = lr + 32 * h, nn = n0 + r;
       const bool ok = kin && nn < N;
       cp_async16_zfill(&Bs[buf][r][lc], We + (int64_t)(ok ? nn : 0) * ldw + (kin ? k : 0), ok ? 16 : 0);
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
   };
   // kStages - 1 steps in flight; a commit per step keeps the group count regular (empty past the end, where `stage`
   // copies nothing but zero fill into a buffer nobody reads)
+  if constexpr (PAIR == kPairSecond) {      // the weights of the first steps ride in the first group
 #pragma unroll
-  for (int st = 0; st < kStages - 1; ++st) stage(st * kBK, st);
+    for (int st = 0; st < kStages - 1; ++st) stage_b(st * kBK, st);
+    pdl_wait();
+    pdl_launch_dependents();
+  }
+#pragma unroll
+  for (int st = 0; st < kStages - 1; ++st) {
+    stage_a(st * kBK, st);
+    if constexpr (PAIR != kPairSecond) stage_b(st * kBK, st);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
   int buf = 0;
   for (int k0 = 0; k0 < K; k0 += kBK, buf = (buf + 1) % kStages) {
     asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
     __syncthreads();            // step k0 has landed for every thread, and every warp is done with the buffer refilled next
-    stage(k0 + (kStages - 1) * kBK, (buf + kStages - 1) % kStages);
+    stage_a(k0 + (kStages - 1) * kBK, (buf + kStages - 1) % kStages);
+    stage_b(k0 + (kStages - 1) * kBK, (buf + kStages - 1) % kStages);
+    asm volatile("cp.async.commit_group;" ::: "memory");
     if (wm < M)                 // warp-uniform
 #pragma unroll
     for (int kk = 0; kk < kBK; kk += 16) {
@@ -901,7 +925,7 @@ extern "C" int prl_moe_gather(const void* x_bf16, const int32_t* perm, const int
   return PRL_OK;
 }
 
-template <int ACT>
+template <int ACT, int PAIR = kPairNone>
 static int moe_gemm_impl(const void* A, int32_t a_is_f32, int64_t lda, int32_t a_mod, const void* W, int32_t w_is_f32,
                          int64_t expert_stride, int64_t ldw, const int32_t* perm, const int32_t* meta, const int32_t* tiles,
                          int64_t max_tiles, int64_t N, int64_t K, void* C, int64_t ldc, int32_t c_perm, const float* wsel,
@@ -914,8 +938,8 @@ static int moe_gemm_impl(const void* A, int32_t a_is_f32, int64_t lda, int32_t a
       ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0) {
     dim3 grid_tc((unsigned)((N + kBN - 1) / kBN), (unsigned)max_tiles);
     static SmemAttr attr = {};
-    PRL_CUDA(ensure_smem(moe_gemm_mma_kernel<ACT>, (int)kMmaSmem, attr));
-    PRL_CUDA(launch_pdl(moe_gemm_mma_kernel<ACT>, grid_tc, dim3(256), kMmaSmem, s, (const bf16*)A, lda, a_mod, (const bf16*)W,
+    PRL_CUDA(ensure_smem((moe_gemm_mma_kernel<ACT, PAIR>), (int)kMmaSmem, attr));
+    PRL_CUDA(launch_pdl((moe_gemm_mma_kernel<ACT, PAIR>), grid_tc, dim3(256), kMmaSmem, s, (const bf16*)A, lda, a_mod, (const bf16*)W,
                         expert_stride, ldw, perm, meta, tiles, (int)N, (int)K, C, ldc, c_perm, wsel));
     PRL_LAUNCH_CHECK();
     return PRL_OK;
@@ -952,6 +976,25 @@ extern "C" int prl_moe_gemm_act(const void* A, int32_t a_is_f32, int64_t lda, in
                                                      N, K, out, ld_out, 0, wsel, st)
                           : moe_gemm_impl<kActGelu>(A, a_is_f32, lda, a_mod, W, w_is_f32, expert_stride, ldw, perm, meta, tiles, max_tiles,
                                                     N, K, out, ld_out, 0, wsel, st);
+}
+
+template <int ACT>
+static int moe_mlp_impl(const void* x, int32_t f32, int32_t n, const void* up, const void* down, int64_t W, int64_t F, const int32_t* perm,
+                        const int32_t* meta, const int32_t* tiles, int64_t max_tiles, const float* wsel, void* act_out, float* out,
+                        prl_stream_t st) {
+  const int rc = moe_gemm_impl<ACT, kPairFirst>(x, f32, W, n, up, f32, F * W, W, perm, meta, tiles, max_tiles, F, W, act_out, F, 0, wsel, st);
+  return rc ? rc : moe_gemm_impl<kActNone, kPairSecond>(act_out, f32, F, 0, down, f32, W * F, F, perm, meta, tiles, max_tiles, W, F, out, W, 1,
+                                                        nullptr, st);
+}
+
+// Both products of ungated experts, prl_moe_gemm_act and prl_moe_gemm in one call: x [n, W], up [experts * F, W], down [experts * W, F] of
+// one type (f32, else bf16); act_out (a row of F per pair, in that type) is scratch between them, out (a row of W per pair) fp32, pair order.
+extern "C" int prl_moe_mlp_act(const void* x, int32_t f32, int32_t n, const void* up, const void* down, int64_t W, int64_t F,
+                               const int32_t* perm, const int32_t* meta, const int32_t* tiles, int64_t max_tiles, int32_t act,
+                               const float* wsel, void* act_out, float* out, prl_stream_t st) {
+  PRL_CHECK_ARG(n >= 1 && act_out && (act == kActRelu2 || act == kActGelu), "prl_moe_mlp_act: bad argument (activation %d)", act);
+  return act == kActRelu2 ? moe_mlp_impl<kActRelu2>(x, f32, n, up, down, W, F, perm, meta, tiles, max_tiles, wsel, act_out, out, st)
+                          : moe_mlp_impl<kActGelu>(x, f32, n, up, down, W, F, perm, meta, tiles, max_tiles, wsel, act_out, out, st);
 }
 
 extern "C" int prl_moe_glu(const float* gate_up, int64_t ld, int64_t pairs, int32_t F, const int32_t* perm,

@@ -1971,10 +1971,8 @@ class HybridEngine(EngineCore):
             _lib.check(lib.prl_moe_gemm_tc(out, pairs, up, e.experts, e.ff, W, *table, R.wsel.data_ptr(), unit, act, e.ff, st))
             _lib.check(lib.prl_moe_gemm_tc(act, pairs, down, e.experts, W, e.ff, *table, None, 0, out, W, st))
             return R.moe_out
-        table += (int(lib.prl_moe_max_tiles(pairs, e.experts)),)
-        _lib.check(lib.prl_moe_gemm_act(R.xa.data_ptr(), f32, W, n, up, f32, e.ff * W, W, *table, e.ff, W, unit, R.wsel.data_ptr(), act,
-                                        e.ff, st))
-        _lib.check(lib.prl_moe_gemm(act, f32, e.ff, 0, down, f32, W * e.ff, e.ff, *table, W, e.ff, out, W, 1, st))
+        _lib.check(lib.prl_moe_mlp_act(R.xa.data_ptr(), f32, n, up, down, W, e.ff, *table,
+                                       int(lib.prl_moe_max_tiles(pairs, e.experts)), unit, R.wsel.data_ptr(), act, out, st))
         return R.moe_out
 
     def _attn_core(self, R, n, i, L, w, segs, max_q, row_pos, seg_pos0, ld, decode) -> torch.Tensor:

@@ -485,6 +485,35 @@ def test_token_step_of_the_gated_delta_rule(cuda_device, heads, kv, dk, dv, taps
     assert mc.rel_err(torch.cat(out).double().cpu(), ref[:at]) < F32_TOL
 
 
+@pytest.mark.parametrize("n,W,F,experts,top", [(1, 64, 72, 4, 2), (33, 200, 136, 5, 3), (300, 96, 128, 16, 4), (7, 20, 12, 3, 1)])
+@pytest.mark.parametrize("dtype,act", [(torch.bfloat16, 2), (torch.bfloat16, 1), (torch.float32, 2)])
+def test_both_expert_products_in_one_call(cuda_device, dtype, act, n, W, F, experts, top):
+    """prl_moe_mlp_act: the bits of prl_moe_gemm_act and prl_moe_gemm, back to back with the grouping that feeds them (several times, so
+    that a product that reads its tiles too early would see the former batch's)."""
+    from pipelinerl_b200 import _lib
+    lib, st, g = _lib.load(), _lib.stream_ptr(), torch.Generator(device="cuda").manual_seed(n + W)
+    f32, pairs, i32, ptr = int(dtype == torch.float32), n * top, dict(dtype=torch.int32, device="cuda"), lambda t: t.data_ptr()  # noqa: E731
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    up, down = (rnd(experts * F, W) * W ** -0.5).to(dtype), (rnd(experts * W, F) * F ** -0.5).to(dtype)
+    sel, wsel, perm, meta = torch.zeros(pairs, **i32), torch.zeros(pairs, device="cuda"), torch.zeros(pairs, **i32), torch.zeros(4, **i32)
+    most = int(lib.prl_moe_max_tiles(pairs, experts))
+    tiles, act_out = torch.zeros(3 * most, **i32), torch.zeros(pairs, F, dtype=dtype, device="cuda")
+    zs, xs, got = [rnd(n, experts) for _ in range(6)], [rnd(n, W).to(dtype) for _ in range(6)], []
+    for together in (False, True):
+        outs = [torch.full((pairs, W), float("nan"), device="cuda") for _ in zs]
+        for z, x, out in zip(zs, xs, outs):
+            _lib.check(lib.prl_moe_choose(ptr(z), experts, None, n, experts, experts, top, 1, 1, 1, 1, 1, 1.3, 64, ptr(sel), ptr(wsel), ptr(perm), ptr(meta),
+                                          ptr(tiles), st))
+            table = (ptr(perm), ptr(meta), ptr(tiles), most)
+            if together:
+                _lib.check(lib.prl_moe_mlp_act(ptr(x), f32, n, ptr(up), ptr(down), W, F, *table, act, ptr(wsel), ptr(act_out), ptr(out), st))
+            else:
+                _lib.check(lib.prl_moe_gemm_act(ptr(x), f32, W, n, ptr(up), f32, F * W, W, *table, F, W, act, ptr(wsel), ptr(act_out), F, st))
+                _lib.check(lib.prl_moe_gemm(ptr(act_out), f32, F, 0, ptr(down), f32, W * F, F, *table, W, F, ptr(out), W, 1, st))
+        got.append(outs)
+    assert all(torch.equal(a, b) and torch.isfinite(a).all() for a, b in zip(*got))
+
+
 @pytest.mark.parametrize("heads,kh,dk,dv", [(16, 8, 128, 128), (4, 2, 64, 48), (6, 2, 20, 36), (4, 4, 32, 64)])
 def test_token_step_of_many_rows_equals_few(cuda_device, heads, kh, dk, dv):
     """One value head at a time in a CTA (more than 148 CTAs) or two: the same bits, for outputs, states and convolution inputs."""
