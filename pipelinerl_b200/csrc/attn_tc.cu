@@ -56,6 +56,7 @@ struct TcPrefillParams {
   const float* gate;             // [rows][ld_gate] logits: a head's output times sigmoid(gate[row * ld_gate + head]), or NULL
   int64_t ld_gate;
   long long* timing;             // measurement only (prl_attn_debug_timing): per-phase cycle sums of one CTA, else NULL
+  int list_segs;                 // kContig, generation 2: > 0 = grid.x lists the tiles of this many sequences (tile_of_list)
 };
 
 __device__ __forceinline__ float ex2(float x) {
@@ -379,9 +380,13 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   pdl_launch_dependents();
   pdl_wait();                                            // the sequence tables below may be fresh
 
-  const int qtile = kContig ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
-  const int kvh = blockIdx.y, z = blockIdx.z;
-  const int q_len = ptx::warp_uniform(p.seq_q_len[z]);
+  int qtile = kContig ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x, z = blockIdx.z, q_len;
+  const int kvh = blockIdx.y;
+  if (kContig && p.list_segs > 0) {
+    if (!tile_of_list(p.seq_q_len, p.list_segs, p.nq, (int)blockIdx.x, z, qtile, q_len)) return;
+  } else {
+    q_len = ptx::warp_uniform(p.seq_q_len[z]);
+  }
   const int pos0 = (kContig && p.seq_pos0 == nullptr) ? 0 : ptx::warp_uniform(p.seq_pos0[z]);
   const int t0 = qtile * p.nq;
   if (t0 >= q_len) return;                               // before any barrier / TMEM use
@@ -415,11 +420,14 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   tmem_base = ptx::warp_uniform(tmem_base);
 
   if (warp == 0) {
-    // ===== TMA producer (as generation 1) =====
-    if (lane == 0) {
-      ptx::mbar_arrive_expect_tx(bar(0), (uint32_t)(2 * 128 * p.R * p.nq));
-      ptx::tma_load_3d(q_smem, &tm_q, 0, kvh * p.R, row0, bar(0), ptx::kEvictFirst);
-      ptx::tma_load_3d(q_smem + kTile16K, &tm_q, 64, kvh * p.R, row0, bar(0), ptx::kEvictFirst);
+    // ===== TMA producer, converged like the MMA issuer =====
+    {
+      if (ptx::elect_one()) {
+        ptx::mbar_arrive_expect_tx(bar(0), (uint32_t)(2 * 128 * p.R * p.nq));
+        ptx::tma_load_3d(q_smem, &tm_q, 0, kvh * p.R, row0, bar(0), ptx::kEvictFirst);
+        ptx::tma_load_3d(q_smem + kTile16K, &tm_q, 64, kvh * p.R, row0, bar(0), ptx::kEvictFirst);
+      }
+      __syncwarp();
       const int32_t* bt = kContig ? nullptr : p.block_table + (int64_t)p.seq_slot[z] * p.max_blocks;
       const int seq_row0 = (kContig && p.seq_kv_start != nullptr) ? p.seq_kv_start[z] : p.seq_q_start[z];
       auto load_page = [&](int it, int kv, uint32_t full_bar, uint32_t empty_bar) {
@@ -440,13 +448,16 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             row[half] = (int)(((((int64_t)p.layer * 2 + kv) * p.n_pages + row[half]) * p.n_kv + kvh) * kPageT);
         }
         ptx::mbar_wait(empty_bar + 8u * (uint32_t)s, ph ^ 1u);
-        ptx::mbar_arrive_expect_tx(full_bar + 8u * (uint32_t)s, (uint32_t)(2 * kTile16K));
+        if (ptx::elect_one()) {
+          ptx::mbar_arrive_expect_tx(full_bar + 8u * (uint32_t)s, (uint32_t)(2 * kTile16K));
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const uint32_t dst = kv_smem + (uint32_t)(s * kStageBytesT + kv * 2 * kTile16K + half * 8192);
-          ptx::tma_load_2d(dst, &tm_kv, c0, row[half], full_bar + 8u * (uint32_t)s, ptx::kEvictLast);
-          ptx::tma_load_2d(dst + kTile16K, &tm_kv, c0 + 64, row[half], full_bar + 8u * (uint32_t)s, ptx::kEvictLast);
+          for (int half = 0; half < 2; ++half) {
+            const uint32_t dst = kv_smem + (uint32_t)(s * kStageBytesT + kv * 2 * kTile16K + half * 8192);
+            ptx::tma_load_2d(dst, &tm_kv, c0, row[half], full_bar + 8u * (uint32_t)s, ptx::kEvictLast);
+            ptx::tma_load_2d(dst + kTile16K, &tm_kv, c0 + 64, row[half], full_bar + 8u * (uint32_t)s, ptx::kEvictLast);
+          }
         }
+        __syncwarp();
       };
       load_page(0, 0, bar(1), bar(4));
       for (int it = 0; it < n_it; ++it) {
@@ -716,6 +727,7 @@ static int prefill_tc_impl(const void* q, int32_t q_rows, const void* kv_cache, 
   const int64_t total_rows = (int64_t)n_layers * 2 * n_pages * n_kv * kPageT;
   PRL_CHECK_ARG(total_rows < (1ll << 31), "prl_paged_attn_prefill_tc: KV cache too large for 32-bit TMA row coordinates");
   TcPrefillParams p;
+  p.list_segs = 0;
   p.out = (__nv_bfloat16*)out_bf16;
   p.block_table = block_table; p.seq_q_start = seq_q_start; p.seq_q_len = seq_q_len; p.seq_pos0 = seq_pos0;
   p.seq_slot = seq_slot; p.seq_kv_start = nullptr; p.max_blocks = max_blocks; p.n_q = n_q; p.n_kv = n_kv; p.R = n_q / n_kv;
@@ -800,6 +812,7 @@ extern "C" int prl_attn_varlen_fwd(const void* qkv, int64_t qkv_stride, int32_t 
                 "prl_attn_varlen_fwd: bad shape");
   PRL_CHECK_ARG(qkv_stride >= (int64_t)(n_q + 2 * n_kv) * kDT && qkv_stride % 8 == 0, "prl_attn_varlen_fwd: bad row stride");
   TcPrefillParams p;
+  p.list_segs = 0;
   p.out = (__nv_bfloat16*)out_bf16;
   p.block_table = nullptr; p.seq_q_start = seg_start; p.seq_q_len = seg_len; p.seq_pos0 = nullptr; p.seq_slot = nullptr; p.seq_kv_start = nullptr;
   p.max_blocks = 0; p.n_q = n_q; p.n_kv = n_kv; p.R = n_q / n_kv; p.nq = 128 / p.R;
@@ -824,6 +837,7 @@ extern "C" int prl_attn_varlen_fwd(const void* qkv, int64_t qkv_stride, int32_t 
     PRL_CUDA(launch_pdl(attn_fwd_v2_kernel<true, true>, grid, dim3(kThreadsT), (size_t)smem, (cudaStream_t)stream_, tq, tkv, p));
   } else {
     static SmemAttr smem_attr2 = {};
+    if (n_seg > 1) { p.list_segs = n_seg; grid = dim3(list_tiles(T, n_seg, max_seg_len, p.nq), (unsigned)n_kv); }
     PRL_CUDA(ensure_smem(attn_fwd_v2_kernel<true>, smem, smem_attr2));
     PRL_CUDA(launch_pdl(attn_fwd_v2_kernel<true>, grid, dim3(kThreadsT), (size_t)smem, (cudaStream_t)stream_, tq, tkv, p));
   }
@@ -848,6 +862,7 @@ extern "C" int prl_attn_varlen_fwd_kv(const void* q, int64_t q_stride, int32_t T
   PRL_CHECK_ARG(q_stride >= (int64_t)n_q * kDT && q_stride % 8 == 0 && kv_stride >= (int64_t)2 * n_kv * kDT && kv_stride % 8 == 0,
                 "prl_attn_varlen_fwd_kv: bad row stride");
   TcPrefillParams p;
+  p.list_segs = 0;
   p.out = (__nv_bfloat16*)out_bf16;
   p.block_table = nullptr; p.seq_q_start = seg_q_start; p.seq_q_len = seg_q_len; p.seq_pos0 = seg_pos0; p.seq_slot = nullptr;
   p.seq_kv_start = seg_kv_start;

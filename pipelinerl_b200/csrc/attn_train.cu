@@ -61,6 +61,7 @@ struct BwdParams {
   int dkv_col_k, dkv_col_v;
   int n_lin;                     // generation-4 dK / dV kernel: kv heads x sequences, the fast index of its one-dimensional grid
   int split;                     // CTAs (one cluster) that share the queries of a key tile in the generation-4 dK / dV kernel
+  int list_segs;                 // dQ, generation 4: > 0 = grid.x lists the tiles of this many sequences (tile_of_list)
 };
 
 __device__ __forceinline__ float ex2f(float x) {
@@ -804,31 +805,37 @@ attn_bwd_dkdv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
   if (warp == 0) {
     // ===== TMA producer =====
-    if (lane == 0) {
-      ptx::mbar_arrive_expect_tx(bar(0), (uint32_t)kKvBytes);
-      const int krow = kv0 + key0;
+    {   // converged like the MMA issuer
+      if (ptx::elect_one()) {
+        ptx::mbar_arrive_expect_tx(bar(0), (uint32_t)kKvBytes);
+        const int krow = kv0 + key0;
 #pragma unroll
-      for (int kv = 0; kv < 2; ++kv) {
-        const int c0 = (kv ? p.col_v : p.col_k) + kvh * kD;
+        for (int kv = 0; kv < 2; ++kv) {
+          const int c0 = (kv ? p.col_v : p.col_k) + kvh * kD;
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const uint32_t dst = kv_smem + (uint32_t)((kv * 2 + half) * kT16);
-          ptx::tma_load_2d(dst, &tm_kv, c0 + 64 * half, krow, bar(0), ptx::kEvictFirst);
-          ptx::tma_load_2d(dst + kT8, &tm_kv, c0 + 64 * half, krow + 64, bar(0), ptx::kEvictFirst);
+          for (int half = 0; half < 2; ++half) {
+            const uint32_t dst = kv_smem + (uint32_t)((kv * 2 + half) * kT16);
+            ptx::tma_load_2d(dst, &tm_kv, c0 + 64 * half, krow, bar(0), ptx::kEvictFirst);
+            ptx::tma_load_2d(dst + kT8, &tm_kv, c0 + 64 * half, krow + 64, bar(0), ptx::kEvictFirst);
+          }
         }
       }
+      __syncwarp();
       const uint32_t q_bytes = (uint32_t)(4 * 128 * p.R * nqa);
       for (int it = 0; it < n_it; ++it) {
         const int st = it % kQStages4;
         const uint32_t ph = (uint32_t)((it / kQStages4) & 1);
         ptx::mbar_wait(bar(5 + st), ph ^ 1u);
-        ptx::mbar_arrive_expect_tx(bar(1 + st), q_bytes);
-        const int row = seg0 + (u_first + it) * nqa;
-        const uint32_t dst = q_ring + (uint32_t)(st * kQSlot);
-        ptx::tma_load_3d(dst, &tm_q, 0, kvh * p.R, row, bar(1 + st), ptx::kEvictLast);
-        ptx::tma_load_3d(dst + kT8, &tm_q, 64, kvh * p.R, row, bar(1 + st), ptx::kEvictLast);
-        ptx::tma_load_3d(dst + 2 * kT8, &tm_do, 0, kvh * p.R, row, bar(1 + st), ptx::kEvictLast);
-        ptx::tma_load_3d(dst + 3 * kT8, &tm_do, 64, kvh * p.R, row, bar(1 + st), ptx::kEvictLast);
+        if (ptx::elect_one()) {
+          ptx::mbar_arrive_expect_tx(bar(1 + st), q_bytes);
+          const int row = seg0 + (u_first + it) * nqa;
+          const uint32_t dst = q_ring + (uint32_t)(st * kQSlot);
+          ptx::tma_load_3d(dst, &tm_q, 0, kvh * p.R, row, bar(1 + st), ptx::kEvictLast);
+          ptx::tma_load_3d(dst + kT8, &tm_q, 64, kvh * p.R, row, bar(1 + st), ptx::kEvictLast);
+          ptx::tma_load_3d(dst + 2 * kT8, &tm_do, 0, kvh * p.R, row, bar(1 + st), ptx::kEvictLast);
+          ptx::tma_load_3d(dst + 3 * kT8, &tm_do, 64, kvh * p.R, row, bar(1 + st), ptx::kEvictLast);
+        }
+        __syncwarp();
       }
     }
   } else if (warp == 1) {
@@ -1093,9 +1100,13 @@ attn_bwd_dq4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const uint32_t tmem_slot = bar(18);
   constexpr uint32_t cDP = 256u, cDQ = 384u;            // TMEM columns: S[2] 0,128 | dP 256 | dQ 384
 
-  const int qtile = (int)(gridDim.x - 1 - blockIdx.x);
-  const int kvh = blockIdx.y, z = blockIdx.z;
-  const int q_len = ptx::warp_uniform(p.seg_len[z]);
+  int qtile = (int)(gridDim.x - 1 - blockIdx.x), z = blockIdx.z, q_len;
+  const int kvh = blockIdx.y;
+  if (p.list_segs > 0) {
+    if (!tile_of_list(p.seg_len, p.list_segs, p.nq, (int)blockIdx.x, z, qtile, q_len)) return;
+  } else {
+    q_len = ptx::warp_uniform(p.seg_len[z]);
+  }
   const int t0 = qtile * p.nq;
   if (t0 >= q_len) return;
   const int seg0 = ptx::warp_uniform(p.seg_start[z]);
@@ -1129,28 +1140,34 @@ attn_bwd_dq4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 
   if (warp == 0) {
     // ===== TMA producer =====
-    if (lane == 0) {
-      ptx::mbar_arrive_expect_tx(bar(0), (uint32_t)(4 * 128 * p.R * p.nq));
-      ptx::tma_load_3d(q_smem, &tm_q, 0, kvh * p.R, row0, bar(0), ptx::kEvictFirst);
-      ptx::tma_load_3d(q_smem + kT16, &tm_q, 64, kvh * p.R, row0, bar(0), ptx::kEvictFirst);
-      ptx::tma_load_3d(do_smem, &tm_do, 0, kvh * p.R, row0, bar(0), ptx::kEvictFirst);
-      ptx::tma_load_3d(do_smem + kT16, &tm_do, 64, kvh * p.R, row0, bar(0), ptx::kEvictFirst);
+    {   // converged like the MMA issuer
+      if (ptx::elect_one()) {
+        ptx::mbar_arrive_expect_tx(bar(0), (uint32_t)(4 * 128 * p.R * p.nq));
+        ptx::tma_load_3d(q_smem, &tm_q, 0, kvh * p.R, row0, bar(0), ptx::kEvictFirst);
+        ptx::tma_load_3d(q_smem + kT16, &tm_q, 64, kvh * p.R, row0, bar(0), ptx::kEvictFirst);
+        ptx::tma_load_3d(do_smem, &tm_do, 0, kvh * p.R, row0, bar(0), ptx::kEvictFirst);
+        ptx::tma_load_3d(do_smem + kT16, &tm_do, 64, kvh * p.R, row0, bar(0), ptx::kEvictFirst);
+      }
+      __syncwarp();
       auto load_page = [&](int it, int kv) {
         const int s = kv ? (it & 1) : (it % kKSlots4);
         const uint32_t ph = (uint32_t)((kv ? (it >> 1) : (it / kKSlots4)) & 1);
         const uint32_t full = bar((kv ? 13 : 1) + s), empty = bar((kv ? 15 : 4) + s);
         ptx::mbar_wait(empty, ph ^ 1u);
-        ptx::mbar_arrive_expect_tx(full, (uint32_t)(2 * kT16));
         const int c0 = (kv ? p.col_v : p.col_k) + kvh * kD;
+        if (ptx::elect_one()) {
+          ptx::mbar_arrive_expect_tx(full, (uint32_t)(2 * kT16));
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {          // the two 64-key pages of a step
-          int pg = 2 * it + half;
-          if (pg > last_page) pg = last_page;          // tail: re-read the last page, its keys are causally masked
-          const int row = kv0 + pg * 64;
-          const uint32_t dst = (kv ? v_smem : k_smem) + (uint32_t)(s * 2 * kT16) + (uint32_t)(half * kT8);
-          ptx::tma_load_2d(dst, &tm_kv, c0, row, full, ptx::kEvictLast);
-          ptx::tma_load_2d(dst + kT16, &tm_kv, c0 + 64, row, full, ptx::kEvictLast);
+          for (int half = 0; half < 2; ++half) {        // the two 64-key pages of a step
+            int pg = 2 * it + half;
+            if (pg > last_page) pg = last_page;        // tail: re-read the last page, its keys are causally masked
+            const int row = kv0 + pg * 64;
+            const uint32_t dst = (kv ? v_smem : k_smem) + (uint32_t)(s * 2 * kT16) + (uint32_t)(half * kT8);
+            ptx::tma_load_2d(dst, &tm_kv, c0, row, full, ptx::kEvictLast);
+            ptx::tma_load_2d(dst + kT16, &tm_kv, c0 + 64, row, full, ptx::kEvictLast);
+          }
         }
+        __syncwarp();
       };
       load_page(0, 0);
       for (int it = 0; it < n_it; ++it) {
@@ -1429,6 +1446,7 @@ extern "C" int prl_attn_varlen_bwd(const void* qkv, int64_t qkv_stride, int32_t 
     PRL_LAUNCH_CHECK();
   }
   BwdParams p;
+  p.list_segs = 0;
   p.lse = lse; p.delta = delta; p.dqkv = (__nv_bfloat16*)dqkv; p.dqkv_stride = dqkv_stride;
   p.seg_start = seg_start; p.seg_len = seg_len; p.n_q = n_q; p.n_kv = n_kv; p.R = n_q / n_kv;
   p.col_k = n_q * kD; p.col_v = (n_q + n_kv) * kD;
@@ -1488,6 +1506,7 @@ extern "C" int prl_attn_varlen_bwd(const void* qkv, int64_t qkv_stride, int32_t 
         PRL_CUDA(ensure_smem(attn_bwd_dq4_kernel<true>, kSmemDq4, attr4t));
         attn_bwd_dq4_kernel<true><<<grid, kThreadsB4, (size_t)kSmemDq4, stream>>>(tq, tdo, tkv, p);
       } else {
+        if (n_seg > 1) { p.list_segs = n_seg; grid = dim3(list_tiles(T, n_seg, max_seg_len, p.nq), (unsigned)n_kv); }
         PRL_CUDA(ensure_smem(attn_bwd_dq4_kernel<false>, kSmemDq4, attr4));
         attn_bwd_dq4_kernel<false><<<grid, kThreadsB4, (size_t)kSmemDq4, stream>>>(tq, tdo, tkv, p);
       }
@@ -1537,6 +1556,7 @@ extern "C" int prl_attn_varlen_bwd_kv(const void* q, int64_t q_stride, int32_t T
   }
   PRL_CUDA(cudaMemset2DAsync(dkv, (size_t)dkv_stride * 2, 0, (size_t)kvw * 2, (size_t)Tkv, stream));
   BwdParams p;
+  p.list_segs = 0;
   p.lse = lse; p.delta = delta; p.dqkv = (__nv_bfloat16*)dq; p.dqkv_stride = dq_stride;
   p.seg_start = seg_q_start; p.seg_len = seg_q_len; p.n_q = n_q; p.n_kv = n_kv; p.R = n_q / n_kv;
   p.col_k = 0; p.col_v = n_kv * kD;

@@ -312,4 +312,36 @@ int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner_elems, 
 int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1_bytes,
                       uint64_t stride2_bytes, uint32_t box0, uint32_t box1, uint32_t box2);
 
+// Query tiles of sequences of very different lengths: a grid of the longest one's tiles for each would be mostly CTAs that find nothing
+// to do, and each of them holds an SM alone for about a microsecond (samples of 1531, 977, 64, 2300, 1 and 411 tokens: 958 of 1536).  So
+// grid.x lists the tiles that are there, sequence by sequence, the last (longest) tile of each first.
+inline unsigned list_tiles(int T, int n_seg, int max_len, int nq) {       // the lengths add up to at most T
+  const int64_t most = ((int64_t)T + (int64_t)n_seg * (nq - 1)) / nq, all = (int64_t)n_seg * ((max_len + nq - 1) / nq);
+  return (unsigned)(most < all ? most : all);
+}
+// Place `at` of the list: its sequence, tile and the sequence's length (false: past the end).  Every warp looks for itself, 32 sequences
+// at a time.
+__device__ __forceinline__ bool tile_of_list(const int32_t* __restrict__ len, int n_seg, int nq, int at, int& z, int& tile, int& z_len) {
+  const int lane = threadIdx.x & 31;
+  for (int z0 = 0; z0 < n_seg; z0 += 32) {
+    const int mine = z0 + lane < n_seg ? len[z0 + lane] : 0, tiles = mine > 0 ? (mine + nq - 1) / nq : 0;
+    int end = tiles;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += v;
+    }
+    const uint32_t past = __ballot_sync(0xffffffffu, at < end);
+    if (past) {
+      const int src = __ffs(past) - 1;
+      z = z0 + src;
+      tile = __shfl_sync(0xffffffffu, end, src) - 1 - at;
+      z_len = __shfl_sync(0xffffffffu, mine, src);
+      return true;
+    }
+    at -= __shfl_sync(0xffffffffu, end, 31);
+  }
+  return false;
+}
+
 }  // namespace prl

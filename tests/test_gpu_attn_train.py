@@ -245,3 +245,31 @@ def test_varlen_backward_keeps_its_bits_with_cold_row_statistics(cuda_device, ge
     finally:
         _lib.check(o.lib.prl_attn_set_bwd_generation(4))
     assert all(torch.equal(runs[0], r) for r in runs[1:])
+
+
+@pytest.mark.parametrize("n_q,n_kv,lens", [(14, 2, [1, 700, 0, 18, 19, 300]), (4, 4, [0, 128, 129, 1, 0]), (5, 1, [3] * 31 + [40, 0, 26, 1, 77] + [2] * 40),
+                                           (8, 2, [64])])
+def test_listed_tiles_equal_each_sample_alone(cuda_device, n_q, n_kv, lens):
+    """Forward and dQ launch the tiles that are there, found in a list of the samples (more than one sample): the bits of each sample by
+    itself, for samples of no tokens, of one tile exactly and one more, and for more samples than a warp looks at together."""
+    from pipelinerl_b200 import _lib
+    lib, st, g = _lib.load(), _lib.stream_ptr(), torch.Generator(device="cuda").manual_seed(sum(lens))
+    T, width, ptr = sum(lens), (n_q + 2 * n_kv) * 128, lambda t: t.data_ptr()  # noqa: E731
+    qkv = torch.randn(T, width, generator=g, device="cuda").bfloat16()
+    d_out = torch.randn(T, n_q * 128, generator=g, device="cuda").bfloat16()
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+
+    def run(picked):
+        out = torch.zeros(T, n_q * 128, dtype=torch.bfloat16, device="cuda")
+        lse, dqkv, ws = torch.zeros(T, n_q, device="cuda"), torch.zeros_like(qkv), torch.empty(T * n_q, device="cuda")
+        start, length = (torch.tensor([v[i] for i in picked], dtype=torch.int32, device="cuda") for v in (starts, lens))
+        seg = (ptr(start), ptr(length), len(picked), max(max(lens[i] for i in picked), 1), n_q, n_kv, 128, 128 ** -0.5)
+        _lib.check(lib.prl_attn_varlen_fwd(ptr(qkv), width, T, *seg, ptr(out), ptr(lse), st))
+        _lib.check(lib.prl_attn_varlen_bwd(ptr(qkv), width, T, *seg, ptr(out), ptr(d_out), ptr(lse), ptr(dqkv), width, ptr(ws), ws.numel() * 4, st))
+        return out, lse, dqkv[:, :n_q * 128]
+    together = run(list(range(len(lens))))
+    for i, k in enumerate(lens):
+        if k and (len(lens) < 10 or i % 7 == 0 or k > 3):
+            rows = slice(starts[i], starts[i] + k)
+            assert all(torch.equal(a[rows], b[rows]) for a, b in zip(together, run([i])))
+    assert all(torch.isfinite(t.float()).all() for t in together)
