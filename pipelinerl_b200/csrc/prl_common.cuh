@@ -6,6 +6,7 @@
 #include <stdio.h>
 #include <stdarg.h>
 #include "../../include/prl.h"
+#include "smem_attr.cuh"
 
 #if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ < 1000)
 #error "libprl is written for sm_100a only"
@@ -67,22 +68,14 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// cudaFuncAttributeMaxDynamicSharedMemorySize is a per-DEVICE function attribute: remember the largest size granted
-// on each device (one static SmemAttr per launch site) instead of a per-process flag.
-constexpr int kMaxDevices = 16;
-struct SmemAttr { int bytes[kMaxDevices]; };
+// `smem` bytes of dynamic shared memory for a kernel on the current device
 template <typename K>
 inline cudaError_t ensure_smem(K kernel, int smem, SmemAttr& st) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= kMaxDevices) return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (st.bytes[dev] < smem) {
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    st.bytes[dev] = smem;
-  }
-  return cudaSuccess;
+  auto set = [&](int bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
+  return dev < 0 || dev >= kMaxDevices ? set(smem) : raise_smem(st, dev, smem, set);
 }
 
 constexpr int kWarp = 32;

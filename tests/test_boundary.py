@@ -117,6 +117,20 @@ def test_plain_c_client_links_and_calls(built_lib, tmp_path):
     assert r.returncode == 0 and r.stdout.startswith("ok version="), (r.returncode, r.stdout, r.stderr)
 
 
+def test_shared_memory_sizes_of_several_threads(tmp_path):
+    """Threads whose calls need different sizes of one kernel's shared memory: the largest stays granted (tests/c_abi/smem_attr.cpp)."""
+    import shutil
+    import subprocess
+    if shutil.which("g++") is None:
+        pytest.skip("g++ not available")
+    exe = tmp_path / "smem_attr"
+    r = subprocess.run(["g++", "-std=c++17", "-Wall", "-pthread", "-I", str(ROOT / "pipelinerl_b200" / "csrc"),
+                        str(ROOT / "tests" / "c_abi" / "smem_attr.cpp"), "-o", str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0 and r.stdout == "ok\n", (r.returncode, r.stdout, r.stderr)
+
+
 def test_no_load_is_delivered_to_several_ctas():
     """Ranks on several GPUs run every kernel here; a bulk or tensor load whose data goes to more than one CTA of a cluster is not to
     be among them (an arrival that tells several CTAs of finished products is)."""
