@@ -449,7 +449,8 @@ int prl_paged_attn_prefill_tc_gated(const void* q_bf16 /*[q_rows,n_q,128]*/, int
  * flash-attn varlen call the reference makes through HF with packed position_ids
  * (pipelinerl/finetune/rl/__init__.py:204 forward, finetune_loop.py:716-725 backward; conf/finetune/base.yaml:12-13,64).
  * qkv: [T, qkv_stride] bf16 rows = [n_q q heads | n_kv k heads | n_kv v heads] x 128, q / k already roped.
- * Segment z = rows [seg_start[z], seg_start[z] + seg_len[z]); head_dim must be 128, n_q / n_kv <= 64.
+ * Segment z = rows [seg_start[z], seg_start[z] + seg_len[z]); head_dim must be 128, n_q / n_kv <= 64.  Segments are disjoint
+ * rows of the T: the lengths (device data, which a launch cannot check) add up to at most T, none is above max_seg_len.
  * fwd: out [T, n_q*128] bf16, lse [T, n_q] fp32 (log2 domain of the scaled scores; NULL = not needed).
  * bwd: dqkv [T, dqkv_stride] bf16 in the layout of qkv (every segment row is written); dK / dV are reduced over
  * the GQA group inside the tensor core in a fixed order (deterministic, no atomics).
@@ -457,6 +458,9 @@ int prl_paged_attn_prefill_tc_gated(const void* q_bf16 /*[q_rows,n_q,128]*/, int
 int prl_attn_varlen_fwd(const void* qkv_bf16, int64_t qkv_stride, int32_t T, const int32_t* seg_start,
                         const int32_t* seg_len, int32_t n_seg, int32_t max_seg_len, int32_t n_q, int32_t n_kv,
                         int32_t head_dim, float sm_scale, void* out_bf16, float* lse, prl_stream_t stream);
+/* tiles per key head that the forward and dQ launch for such a row where they list the tiles that are there; 0 = they launch
+ * max_seg_len's tiles for every segment (host only) */
+int prl_attn_listed_tiles(int32_t T, int32_t max_seg_len, int32_t n_seg, int32_t n_q, int32_t n_kv);
 /* which forward kernel prl_attn_varlen_fwd launches: 2 (default) = two ping-pong softmax groups, O accumulated in TMEM
  * with conditional rescale; 1 = the first-generation kernel shared with chunked prefill.  For A/B runs and tests. */
 int prl_attn_set_fwd_generation(int32_t generation);

@@ -170,6 +170,7 @@ _SIGNATURES = {
                                       C.c_int32, C.c_int32, C.c_int32, C.c_float, C.c_void_p, C.c_void_p, C.c_void_p]),
     "prl_attn_set_fwd_generation": (C.c_int, [C.c_int32]),
     "prl_attn_set_bwd_generation": (C.c_int, [C.c_int32]),
+    "prl_attn_listed_tiles": (C.c_int, [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
     "prl_attn_bwd_split": (C.c_int, [C.c_int32] * 5),
     "prl_attn_set_prefill_generation": (C.c_int, [C.c_int32]),
     "prl_debug_tmem_read_bench": (C.c_int, [C.c_int32, C.c_int32, C.c_void_p, C.c_void_p]),

@@ -56,7 +56,7 @@ struct TcPrefillParams {
   const float* gate;             // [rows][ld_gate] logits: a head's output times sigmoid(gate[row * ld_gate + head]), or NULL
   int64_t ld_gate;
   long long* timing;             // measurement only (prl_attn_debug_timing): per-phase cycle sums of one CTA, else NULL
-  int list_segs;                 // kContig, generation 2: > 0 = grid.x lists the tiles of this many sequences (tile_of_list)
+  int list_segs, list_most;      // kContig, generation 2: > 0 = grid.x lists the tiles of this many sequences, list_most each (tile_of_list)
 };
 
 __device__ __forceinline__ float ex2(float x) {
@@ -383,7 +383,7 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   int qtile = kContig ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x, z = blockIdx.z, q_len;
   const int kvh = blockIdx.y;
   if (kContig && p.list_segs > 0) {
-    if (!tile_of_list(p.seq_q_len, p.list_segs, p.nq, (int)blockIdx.x, z, qtile, q_len)) return;
+    if (!tile_of_list(p.seq_q_len, p.list_segs, p.nq, p.list_most, (int)blockIdx.x, z, qtile, q_len)) return;
   } else {
     q_len = ptx::warp_uniform(p.seq_q_len[z]);
   }
@@ -727,7 +727,7 @@ static int prefill_tc_impl(const void* q, int32_t q_rows, const void* kv_cache, 
   const int64_t total_rows = (int64_t)n_layers * 2 * n_pages * n_kv * kPageT;
   PRL_CHECK_ARG(total_rows < (1ll << 31), "prl_paged_attn_prefill_tc: KV cache too large for 32-bit TMA row coordinates");
   TcPrefillParams p;
-  p.list_segs = 0;
+  p.list_segs = p.list_most = 0;
   p.out = (__nv_bfloat16*)out_bf16;
   p.block_table = block_table; p.seq_q_start = seq_q_start; p.seq_q_len = seq_q_len; p.seq_pos0 = seq_pos0;
   p.seq_slot = seq_slot; p.seq_kv_start = nullptr; p.max_blocks = max_blocks; p.n_q = n_q; p.n_kv = n_kv; p.R = n_q / n_kv;
@@ -797,6 +797,12 @@ extern "C" int prl_attn_set_fwd_generation(int32_t gen) {
   return PRL_OK;
 }
 
+extern "C" int prl_attn_listed_tiles(int32_t T, int32_t max_seg_len, int32_t n_seg, int32_t n_q, int32_t n_kv) {
+  PRL_CHECK_ARG(T >= 1 && n_seg >= 1 && max_seg_len >= 1 && n_kv >= 1 && n_q % n_kv == 0 && n_q / n_kv >= 1 && n_q / n_kv <= 64,
+                "prl_attn_listed_tiles: bad shape");
+  return (int)list_tiles(T, n_seg, max_seg_len, 128 / (n_q / n_kv), n_kv);
+}
+
 // Learner forward (hot path 2): block-diagonal causal attention over ONE packed row, the varlen flash-attention call
 // the reference makes through HF (pipelinerl/finetune/rl/__init__.py:204 with packed position_ids,
 // conf/finetune/base.yaml:12-13,64).  qkv: [T, qkv_stride] bf16 = [q heads | k heads | v heads], q / k already roped.
@@ -812,7 +818,7 @@ extern "C" int prl_attn_varlen_fwd(const void* qkv, int64_t qkv_stride, int32_t 
                 "prl_attn_varlen_fwd: bad shape");
   PRL_CHECK_ARG(qkv_stride >= (int64_t)(n_q + 2 * n_kv) * kDT && qkv_stride % 8 == 0, "prl_attn_varlen_fwd: bad row stride");
   TcPrefillParams p;
-  p.list_segs = 0;
+  p.list_segs = p.list_most = 0;
   p.out = (__nv_bfloat16*)out_bf16;
   p.block_table = nullptr; p.seq_q_start = seg_start; p.seq_q_len = seg_len; p.seq_pos0 = nullptr; p.seq_slot = nullptr; p.seq_kv_start = nullptr;
   p.max_blocks = 0; p.n_q = n_q; p.n_kv = n_kv; p.R = n_q / n_kv; p.nq = 128 / p.R;
@@ -837,7 +843,10 @@ extern "C" int prl_attn_varlen_fwd(const void* qkv, int64_t qkv_stride, int32_t 
     PRL_CUDA(launch_pdl(attn_fwd_v2_kernel<true, true>, grid, dim3(kThreadsT), (size_t)smem, (cudaStream_t)stream_, tq, tkv, p));
   } else {
     static SmemAttr smem_attr2 = {};
-    if (n_seg > 1) { p.list_segs = n_seg; grid = dim3(list_tiles(T, n_seg, max_seg_len, p.nq), (unsigned)n_kv); }
+    if (const unsigned tiles = list_tiles(T, n_seg, max_seg_len, p.nq, n_kv)) {
+      p.list_segs = n_seg; p.list_most = (int)grid.x;
+      grid = dim3(tiles, (unsigned)n_kv);
+    }
     PRL_CUDA(ensure_smem(attn_fwd_v2_kernel<true>, smem, smem_attr2));
     PRL_CUDA(launch_pdl(attn_fwd_v2_kernel<true>, grid, dim3(kThreadsT), (size_t)smem, (cudaStream_t)stream_, tq, tkv, p));
   }
@@ -862,7 +871,7 @@ extern "C" int prl_attn_varlen_fwd_kv(const void* q, int64_t q_stride, int32_t T
   PRL_CHECK_ARG(q_stride >= (int64_t)n_q * kDT && q_stride % 8 == 0 && kv_stride >= (int64_t)2 * n_kv * kDT && kv_stride % 8 == 0,
                 "prl_attn_varlen_fwd_kv: bad row stride");
   TcPrefillParams p;
-  p.list_segs = 0;
+  p.list_segs = p.list_most = 0;
   p.out = (__nv_bfloat16*)out_bf16;
   p.block_table = nullptr; p.seq_q_start = seg_q_start; p.seq_q_len = seg_q_len; p.seq_pos0 = seg_pos0; p.seq_slot = nullptr;
   p.seq_kv_start = seg_kv_start;

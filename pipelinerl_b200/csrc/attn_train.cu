@@ -61,7 +61,7 @@ struct BwdParams {
   int dkv_col_k, dkv_col_v;
   int n_lin;                     // generation-4 dK / dV kernel: kv heads x sequences, the fast index of its one-dimensional grid
   int split;                     // CTAs (one cluster) that share the queries of a key tile in the generation-4 dK / dV kernel
-  int list_segs;                 // dQ, generation 4: > 0 = grid.x lists the tiles of this many sequences (tile_of_list)
+  int list_segs, list_most;      // dQ, generation 4: > 0 = grid.x lists the tiles of this many sequences, list_most each (tile_of_list)
 };
 
 __device__ __forceinline__ float ex2f(float x) {
@@ -1103,7 +1103,7 @@ attn_bwd_dq4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   int qtile = (int)(gridDim.x - 1 - blockIdx.x), z = blockIdx.z, q_len;
   const int kvh = blockIdx.y;
   if (p.list_segs > 0) {
-    if (!tile_of_list(p.seg_len, p.list_segs, p.nq, (int)blockIdx.x, z, qtile, q_len)) return;
+    if (!tile_of_list(p.seg_len, p.list_segs, p.nq, p.list_most, (int)blockIdx.x, z, qtile, q_len)) return;
   } else {
     q_len = ptx::warp_uniform(p.seg_len[z]);
   }
@@ -1446,7 +1446,7 @@ extern "C" int prl_attn_varlen_bwd(const void* qkv, int64_t qkv_stride, int32_t 
     PRL_LAUNCH_CHECK();
   }
   BwdParams p;
-  p.list_segs = 0;
+  p.list_segs = p.list_most = 0;
   p.lse = lse; p.delta = delta; p.dqkv = (__nv_bfloat16*)dqkv; p.dqkv_stride = dqkv_stride;
   p.seg_start = seg_start; p.seg_len = seg_len; p.n_q = n_q; p.n_kv = n_kv; p.R = n_q / n_kv;
   p.col_k = n_q * kD; p.col_v = (n_q + n_kv) * kD;
@@ -1506,7 +1506,10 @@ extern "C" int prl_attn_varlen_bwd(const void* qkv, int64_t qkv_stride, int32_t 
         PRL_CUDA(ensure_smem(attn_bwd_dq4_kernel<true>, kSmemDq4, attr4t));
         attn_bwd_dq4_kernel<true><<<grid, kThreadsB4, (size_t)kSmemDq4, stream>>>(tq, tdo, tkv, p);
       } else {
-        if (n_seg > 1) { p.list_segs = n_seg; grid = dim3(list_tiles(T, n_seg, max_seg_len, p.nq), (unsigned)n_kv); }
+        if (const unsigned tiles = list_tiles(T, n_seg, max_seg_len, p.nq, n_kv)) {
+          p.list_segs = n_seg; p.list_most = (int)grid.x;
+          grid = dim3(tiles, (unsigned)n_kv);
+        }
         PRL_CUDA(ensure_smem(attn_bwd_dq4_kernel<false>, kSmemDq4, attr4));
         attn_bwd_dq4_kernel<false><<<grid, kThreadsB4, (size_t)kSmemDq4, stream>>>(tq, tdo, tkv, p);
       }
@@ -1556,7 +1559,7 @@ extern "C" int prl_attn_varlen_bwd_kv(const void* q, int64_t q_stride, int32_t T
   }
   PRL_CUDA(cudaMemset2DAsync(dkv, (size_t)dkv_stride * 2, 0, (size_t)kvw * 2, (size_t)Tkv, stream));
   BwdParams p;
-  p.list_segs = 0;
+  p.list_segs = p.list_most = 0;
   p.lse = lse; p.delta = delta; p.dqkv = (__nv_bfloat16*)dq; p.dqkv_stride = dq_stride;
   p.seg_start = seg_q_start; p.seg_len = seg_q_len; p.n_q = n_q; p.n_kv = n_kv; p.R = n_q / n_kv;
   p.col_k = 0; p.col_v = n_kv * kD;

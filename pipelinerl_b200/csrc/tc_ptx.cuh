@@ -312,19 +312,25 @@ int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner_elems, 
 int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1_bytes,
                       uint64_t stride2_bytes, uint32_t box0, uint32_t box1, uint32_t box2);
 
-// Query tiles of sequences of very different lengths: a grid of the longest one's tiles for each would be mostly CTAs that find nothing
-// to do, and each of them holds an SM alone for about a microsecond (samples of 1531, 977, 64, 2300, 1 and 411 tokens: 958 of 1536).  So
-// grid.x lists the tiles that are there, sequence by sequence, the last (longest) tile of each first.
-inline unsigned list_tiles(int T, int n_seg, int max_len, int nq) {       // the lengths add up to at most T
+// Query tiles of sequences of very different lengths: a grid of the longest one's tiles for each is mostly CTAs that find nothing to do,
+// and each of them holds an SM alone for 0.7 us.  So grid.x may list the tiles that are there, sequence by sequence, the last (longest)
+// tile of each first.  A tile that looks itself up pays 0.44 us for every 32 sequences in front of it, so the list is taken where the CTAs
+// it saves are worth more than that, and never for a grid that fits the SMs at once: the tiles per key head to launch, 0 = the plain grid.
+// Forward, 14 / 2 heads, plain -> list: samples of 1531, 977, 64, 2300, 1 and 411 tokens 59.1 -> 56.5 us, one of 3000 beside 300 short ones
+// 571 -> 85; but three of 1700 51.1 -> 52.2, 200 of 40 52.3 -> 65.7, 800 of 2 to 30 97 -> 206.
+// The sequences are disjoint rows of one packed row: their lengths add up to at most T.
+inline unsigned list_tiles(int T, int n_seg, int max_len, int nq, int n_kv) {
   const int64_t most = ((int64_t)T + (int64_t)n_seg * (nq - 1)) / nq, all = (int64_t)n_seg * ((max_len + nq - 1) / nq);
-  return (unsigned)(most < all ? most : all);
+  const int64_t looks = (n_seg + 31) / 32 + 1;           // twice the steps of a search, on average
+  return all * n_kv > num_sms() && 3 * (all - most) > looks * most ? (unsigned)most : 0u;
 }
-// Place `at` of the list: its sequence, tile and the sequence's length (false: past the end).  Every warp looks for itself, 32 sequences
-// at a time.
-__device__ __forceinline__ bool tile_of_list(const int32_t* __restrict__ len, int n_seg, int nq, int at, int& z, int& tile, int& z_len) {
+// Place `at` of the list: its sequence, tile and the sequence's length (false: past the end); a sequence has at most `most` tiles, as in
+// the plain grid.  Every warp looks for itself, 32 sequences at a time.
+__device__ __forceinline__ bool tile_of_list(const int32_t* __restrict__ len, int n_seg, int nq, int most, int at, int& z, int& tile,
+                                             int& z_len) {
   const int lane = threadIdx.x & 31;
   for (int z0 = 0; z0 < n_seg; z0 += 32) {
-    const int mine = z0 + lane < n_seg ? len[z0 + lane] : 0, tiles = mine > 0 ? (mine + nq - 1) / nq : 0;
+    const int mine = z0 + lane < n_seg ? len[z0 + lane] : 0, tiles = mine > 0 ? min((mine + nq - 1) / nq, most) : 0;
     int end = tiles;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {

@@ -134,7 +134,7 @@ class Ops:
                                             ws.numel(), _lib.stream_ptr()))
 
     def attn_fwd(self, qkv, seg_start, seg_len, max_len, n_q, n_kv, head_dim, need_lse=True):
-        """block-diagonal causal attention over the packed row qkv [T, (n_q + 2 n_kv) d] (q, k roped)"""
+        """block-diagonal causal attention over the packed row qkv [T, (n_q + 2 n_kv) d] (q, k roped); segments are disjoint rows of it"""
         T = qkv.shape[0]
         assert qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1
         out = torch.empty(T, n_q * head_dim, dtype=torch.bfloat16, device=qkv.device)
@@ -241,6 +241,7 @@ class NativeBody:
     def _segments(self, bounds, dev):
         key = tuple(bounds)
         if self._seg_cache is None or self._seg_cache[0] != key or self._seg_cache[1].device != dev:
+            assert all(e <= s for (_, e), (s, _) in zip(key, key[1:])), "segments of a packed row are disjoint, in order"
             st = torch.tensor([s for s, _ in bounds], dtype=torch.int32, device=dev)
             ln = torch.tensor([e - s for s, e in bounds], dtype=torch.int32, device=dev)
             self._seg_cache = (key, st, ln, max(e - s for s, e in bounds))

@@ -273,3 +273,32 @@ def test_listed_tiles_equal_each_sample_alone(cuda_device, n_q, n_kv, lens):
             rows = slice(starts[i], starts[i] + k)
             assert all(torch.equal(a[rows], b[rows]) for a, b in zip(together, run([i])))
     assert all(torch.isfinite(t.float()).all() for t in together)
+
+
+@pytest.mark.parametrize("n_q,n_kv,lens,listed", [(14, 2, [1, 700, 0, 18, 19, 300], True), (4, 4, [0, 128, 129, 1, 0, 1500, 3], True),
+                                                  (5, 1, [3] * 31 + [40, 0, 26, 1, 77] + [2] * 40, True), (14, 2, [40, 0, 17, 37, 18, 1] * 12, False)])
+def test_tiles_of_packed_samples_equal_each_sample_alone(cuda_device, n_q, n_kv, lens, listed):
+    """Outputs and all gradients of samples packed together against each sample alone, where the tiles are listed and where they are not.
+    dK and dV of a sample alone may be summed in another order (more CTAs share a key tile): fp32 partial sums rounded once to bf16 on
+    either side, 2 * 2^-9 of the norm."""
+    from pipelinerl_b200 import _lib
+    from pipelinerl_b200.learner_body import Ops
+    o, g = Ops(), torch.Generator(device="cuda").manual_seed(sum(lens))
+    assert (_lib.load().prl_attn_listed_tiles(sum(lens), max(lens), len(lens), n_q, n_kv) > 0) == listed
+    qkv = torch.randn(sum(lens), (n_q + 2 * n_kv) * 128, generator=g, device="cuda").bfloat16()
+    d_out = torch.randn(sum(lens), n_q * 128, generator=g, device="cuda").bfloat16()
+    tables = lambda st, ln: tuple(torch.tensor(v, dtype=torch.int32, device="cuda") for v in (st, ln))  # noqa: E731
+    starts, q = [sum(lens[:i]) for i in range(len(lens))], n_q * 128
+    shape = (*tables(starts, lens), max(lens), n_q, n_kv, 128)
+    out, lse = o.attn_fwd(qkv, *shape)
+    dqkv = o.attn_bwd(qkv, out, d_out, lse, *shape)
+    for i, n in enumerate(lens):
+        if n == 0 or (len(lens) > 10 and i % 7 and n <= 3):
+            continue
+        rows = slice(starts[i], starts[i] + n)
+        shape = (*tables([0], [n]), n, n_q, n_kv, 128)
+        out1, lse1 = o.attn_fwd(qkv[rows], *shape)
+        dqkv1 = o.attn_bwd(qkv[rows], out1, d_out[rows].contiguous(), lse1, *shape)
+        assert torch.equal(out[rows], out1) and torch.equal(lse[rows], lse1) and torch.equal(dqkv[rows, :q], dqkv1[:, :q])
+        both = [t[:, q:].float() for t in (dqkv[rows], dqkv1)]
+        assert (both[0] - both[1]).norm() <= 2.0 ** -8 * both[1].norm() + 1e-6
