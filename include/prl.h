@@ -943,6 +943,14 @@ int prl_gated_delta_step(const float* P, int64_t ldp, int32_t off, int32_t off_b
                          const float* gain, float eps, int32_t heads, int32_t kh, int32_t dk, int32_t dv,
                          const int32_t* seg_start, const int32_t* seg_len, const int32_t* seg_slot, int32_t n_seg,
                          float* conv_state, float* state, void* out, int32_t f32, prl_stream_t stream);
+/* The same where the caller knows how many of the n_seg segments have a token, at most: the split of the work goes by it, no result
+ * does (any value gives the same bits).  _heads: value heads that a CTA then takes at a time */
+int prl_gated_delta_step_live(const float* P, int64_t ldp, int32_t off, int32_t off_b, int32_t off_a, int32_t off_g,
+                              const float* conv_w, int32_t taps, const float* A_log, const float* dt_bias, float unit_eps,
+                              const float* gain, float eps, int32_t heads, int32_t kh, int32_t dk, int32_t dv,
+                              const int32_t* seg_start, const int32_t* seg_len, const int32_t* seg_slot, int32_t n_seg,
+                              int32_t live, float* conv_state, float* state, void* out, int32_t f32, prl_stream_t stream);
+int32_t prl_gated_delta_step_heads(int32_t heads, int32_t kh, int32_t live);
 int64_t prl_gated_delta_split_floats(int32_t heads, int32_t dk);
 int prl_gated_delta_split(const float* P, int64_t ldp, int32_t off, int32_t off_b, int32_t off_a, int32_t off_g,
                           const float* conv_w, int32_t taps, const float* A_log, const float* dt_bias, float unit_eps,

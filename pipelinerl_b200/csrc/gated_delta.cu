@@ -900,21 +900,36 @@ extern "C" int32_t prl_gated_delta_step_fits(int32_t heads, int32_t kh, int32_t 
   return geometry_ok(heads, kh, dk, dv, taps) && (2 * 256 + (int64_t)(heads / kh + 2) * dv) * 4 <= 200 * 1024;
 }
 
+// Value heads that a CTA takes at a time, for `live` rows with a token.  Two of them fill an SM's registers with one CTA: the shortest chain
+// while every CTA that has work has an SM of its own (8 / 16 heads of 128: 18 rows 12.1 us, one at a time 14.6; 8 rows 9.8, 12.8).  Past
+// that one head at a time, two CTAs on an SM, and room for another branch's kernel beside them (19 rows 19.0 -> 16.2, 32 rows 21.9 -> 18.4,
+// 64 rows 42.0 -> 33.8).  Idle slots leave at once: what counts is the rows, not the slots.  A pair of CTAs per row (a cluster, a head
+// each) took 13.0 us for 18 rows, but 23.3 for 32, and 29.3 where its second CTA left the first both heads.
+extern "C" int32_t prl_gated_delta_step_heads(int32_t heads, int32_t kh, int32_t live) {
+  return heads > kh && (int64_t)kh * live <= num_sms() ? 2 : 1;
+}
+
 extern "C" int prl_gated_delta_step(const float* P, int64_t ldp, int32_t off, int32_t off_b, int32_t off_a, int32_t off_g,
                                     const float* conv_w, int32_t taps, const float* A_log, const float* dt_bias, float unit_eps,
                                     const float* gain, float eps, int32_t heads, int32_t kh, int32_t dk, int32_t dv,
                                     const int32_t* seg_start, const int32_t* seg_len, const int32_t* seg_slot, int32_t n_seg,
                                     float* conv_state, float* state, void* out, int32_t f32, prl_stream_t st) {
+  return prl_gated_delta_step_live(P, ldp, off, off_b, off_a, off_g, conv_w, taps, A_log, dt_bias, unit_eps, gain, eps, heads, kh, dk, dv,
+                                   seg_start, seg_len, seg_slot, n_seg, n_seg, conv_state, state, out, f32, st);
+}
+
+extern "C" int prl_gated_delta_step_live(const float* P, int64_t ldp, int32_t off, int32_t off_b, int32_t off_a, int32_t off_g,
+                                         const float* conv_w, int32_t taps, const float* A_log, const float* dt_bias, float unit_eps,
+                                         const float* gain, float eps, int32_t heads, int32_t kh, int32_t dk, int32_t dv,
+                                         const int32_t* seg_start, const int32_t* seg_len, const int32_t* seg_slot, int32_t n_seg,
+                                         int32_t live, float* conv_state, float* state, void* out, int32_t f32, prl_stream_t st) {
   PRL_CHECK_ARG(P && conv_w && A_log && dt_bias && gain && seg_start && seg_len && seg_slot && conv_state && state && out,
                 "prl_gated_delta_step: NULL argument");
   PRL_CHECK_ARG(n_seg >= 1 && n_seg <= 65535 && prl_gated_delta_step_fits(heads, kh, dk, dv, taps),
                 "prl_gated_delta_step: bad shape (heads=%d q/k heads=%d dk=%d dv=%d taps=%d)", heads, kh, dk, dv, taps);
   const StepArgs a{P, ldp, off, off_b, off_a, off_g, conv_w, taps, A_log, dt_bias, unit_eps, gain, eps, heads, kh, dk, dv,
                    seg_start, seg_len, seg_slot, conv_state, state, out};
-  // Two value heads at a time fill an SM's registers with one CTA: the shortest chain while every CTA has an SM of its own (8 / 16 heads of
-  // 128: 18 rows 9.3 us, one at a time 11.9).  Past that one head at a time, two CTAs on an SM, and room for another branch's kernel beside
-  // them (19 rows 16.1 -> 14.2, 32 rows 22.9 -> 19.5, 64 rows 42.4 -> 34.5).
-  const int rep = heads / kh, groups = rep > 1 && (int64_t)kh * n_seg <= 148 ? 2 : 1, R = dk <= 32 ? 1 : dk <= 64 ? 2 : dk <= 128 ? 4 : 8;
+  const int rep = heads / kh, groups = prl_gated_delta_step_heads(heads, kh, live < n_seg ? live : n_seg), R = dk <= 32 ? 1 : dk <= 64 ? 2 : dk <= 128 ? 4 : 8;
   const bool vec = dk % 4 == 0 && ((uintptr_t)state & 15) == 0;
   const size_t smem = ((size_t)2 * 32 * R + (size_t)(groups + rep) * dv) * sizeof(float);
   static SmemAttr attr[16] = {};

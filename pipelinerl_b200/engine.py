@@ -116,7 +116,7 @@ class EngineCore:
         self.greedy_rows = torch.zeros(B, dtype=torch.uint8, device=d)
         self.ignore_eos_rows = torch.zeros(B, dtype=torch.uint8, device=d)
         self._temperature, self._greedy, self._ignore_eos = 1.0, False, False
-        self._graphs: dict[int, torch.cuda.CUDAGraph] = {}
+        self._graphs: dict[tuple, torch.cuda.CUDAGraph] = {}          # by parameter buffer and step plan
         # ---- chunked prefill + prefix sharing (GRPO attempts share their prompt) ----
         self.prefill_chunk = int(prefill_chunk)
         self.prefix_sharing = prefix_sharing and not self.recurrent
@@ -213,10 +213,10 @@ class EngineCore:
             else:
                 self.run_prefill()
         if self.use_graph:
-            key = self.arena.data.data_ptr()
+            key = (self.arena.data.data_ptr(), self._step_plan())
             g = self._graphs.get(key)
             if g is None:
-                # The first step on a parameter buffer runs eagerly (which also sets the kernels' attributes), then the
+                # The first step on a parameter buffer (and of a plan on it) runs eagerly (which also sets the kernels' attributes), then the
                 # same enqueue is captured for every later step.  Capture executes nothing, and the eager run is NOT
                 # followed by a replay: a model with recurrent state must see each token exactly once.
                 self._step_kernels()
@@ -231,6 +231,10 @@ class EngineCore:
             self._step_kernels()
         self._sample_and_advance()
         self.step_count += 1
+
+    def _step_plan(self):
+        """What the launches of a token step depend on beside the parameter buffer: a plan is captured as a graph of its own."""
+        return None
 
     def set_arena(self, arena: ParamArena) -> None:
         """Switch the parameter buffer between two token steps (weight update flip).  Graphs are cached per

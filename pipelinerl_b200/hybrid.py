@@ -1477,6 +1477,7 @@ class HybridEngine(EngineCore):
                 ws = max(ws, 16 * 160 * a.heads * a.vdim * 4)
         self.attn_ws = torch.zeros(max(ws, 16), dtype=torch.uint8, device=d)
         self._dec = _Rows(self, B)
+        self._delta_heads = sorted({(L.gdelta.heads, L.gdelta.kv_heads) for L in cfg.layers if L.gdelta is not None})
         i32 = dict(dtype=torch.int32, device=d)
         self._dec.seg[0].copy_(torch.arange(B, **i32))
         self._dec.seg[3].copy_(torch.arange(B, **i32))
@@ -2153,7 +2154,8 @@ class HybridEngine(EngineCore):
                 vec[p + "dt_bias"].data_ptr(), g.unit_eps, norm, self.cfg.eps, g.heads, g.kv_heads, g.dim, g.vdim)
         gate = (R.o.data_ptr(), 1, gv, P + 4 * off_g, ld, norm, g.vdim, g.vdim, n, gv, 0, 0, 1, self.cfg.eps, R.yb.data_ptr(), f32, st)
         if n == ns and not self.unfused_cell and lib.prl_gated_delta_step_fits(g.heads, g.kv_heads, g.dim, g.vdim, g.conv):
-            _lib.check(lib.prl_gated_delta_step(*head, seg_start, seg_len, seg_slot, ns, conv, state, R.yb.data_ptr(), f32, st))
+            _lib.check(lib.prl_gated_delta_step_live(*head, seg_start, seg_len, seg_slot, ns, self._live_rows() if R is self._dec else ns,
+                                                     conv, state, R.yb.data_ptr(), f32, st))
             return
         if R.n_sub:
             _lib.check(lib.prl_gated_delta_split(*head, n, R.row_slot.data_ptr(), R.row_back.data_ptr(), seg_start, seg_len, seg_slot, ns,
@@ -2365,6 +2367,16 @@ class HybridEngine(EngineCore):
             _lib.check(self.lib.prl_soft_cap(logits.data_ptr(), n * self.cfg.vocab_size, self.cfg.logit_softcap, self._st))
 
     # ---- one token for every slot (captured into the engine's CUDA graph) ---------------------------------------------
+    def _live_rows(self) -> int:
+        """At most so many slots have a token in the next step (slots that were filled without a request: all may have)."""
+        return len(self.slot_req) or self.B
+
+    def _step_plan(self):
+        """How the delta rule's token step splits its work over the CTAs depends on the rows with a token; a batch that drains passes
+        from one split to the other once, with the same bits, and its step is captured again."""
+        live = self._live_rows()
+        return tuple(self.lib.prl_gated_delta_step_heads(h, k, live) for h, k in self._delta_heads)
+
     def _step_kernels(self) -> None:
         cfg, lib, R, B = self.cfg, self.lib, self._dec, self.B
         self._st = st = _lib.stream_ptr()

@@ -485,6 +485,29 @@ def test_token_step_of_the_gated_delta_rule(cuda_device, heads, kv, dk, dv, taps
     assert mc.rel_err(torch.cat(out).double().cpu(), ref[:at]) < F32_TOL
 
 
+@pytest.mark.parametrize("graph", [False, True])
+def test_delta_step_of_a_draining_batch(cuda_device, graph):
+    """The split of the delta rule's token step goes by the rows that have a token, not by the slots: a batch that drains passes to two
+    value heads per CTA (148 SMs: at most 37 rows on 4 q / k heads), its captured step with it, and keeps its bits."""
+    from pipelinerl_b200.engine import SamplingParams
+    config = mc.model([P(heads=4, kv_heads=2, dim=32, vdim=32, rot_dims=32, window=50, r_heads=8, r_kv_heads=4, r_dim=32, r_vdim=32, conv=4)], width=64)
+    wt, got = mc.weights(config, 3), []
+    prompts = [mc.tokens_for(config, 3 + i % 5, seed=i) for i in range(44)]
+    for all_slots in (False, True):
+        eng = mc.build_engine(config, wt, torch.bfloat16, cuda_device, max_batch=44, max_seq_len=64, use_cuda_graph=graph)
+        seen, rule = set(), eng._step_plan
+        if all_slots:
+            eng._live_rows = lambda eng=eng: eng.B
+        eng._step_plan = lambda rule=rule, seen=seen: seen.add(rule()) or rule()
+        lone = [eng.add_request(p, SamplingParams(max_tokens=3 + 9 * (i % 4 == 0), greedy=True, ignore_eos=True)) for i, p in enumerate(prompts)]
+        for _ in range(12):
+            eng.step()
+            eng.harvest()
+        assert not eng.slot_req and (not graph or seen == ({(1,)} if all_slots else {(1,), (2,)}))
+        got.append([(list(r.output_ids), list(r.output_logprobs)) for r in lone])
+    assert got[0] == got[1] and all(len(ids) == 3 + 9 * (i % 4 == 0) for i, (ids, _) in enumerate(got[0]))
+
+
 @pytest.mark.parametrize("n,W,F,experts,top", [(1, 64, 72, 4, 2), (33, 200, 136, 5, 3), (300, 96, 128, 16, 4), (7, 20, 12, 3, 1)])
 @pytest.mark.parametrize("dtype,act", [(torch.bfloat16, 2), (torch.bfloat16, 1), (torch.float32, 2)])
 def test_both_expert_products_in_one_call(cuda_device, dtype, act, n, W, F, experts, top):
