@@ -520,15 +520,116 @@ __device__ __forceinline__ float2 block_sum2(float u, float v, float2* red) {
 }
 
 // sublayer_close_kernel for rows of a multiple of four channels: a thread keeps NC groups of four channels of the row (and of
-// the second branch) in registers from the sums to the normed store.
-// Bound by latency: a row is read once by one block, and a token step has fewer rows than SMs.  So all slices of both branches, the
-// residual and the branch gains are asked for before the first sum waits for any of them, the gains (which no kernel of a step writes)
-// come to L2 before the wait for the predecessor (asked for by the first block: all share them), and both branches' sums share their barriers: in L2 5.8 -> 5.5 us for 32 rows x 2048
-// of eight slices each (a token step of four such layers, with attn_front_lanes_kernel: 728 -> 704), 12.8 -> 11.7 for 1024 rows of one.
-// FEW: a token step's rows.  Many narrow rows (one group a thread, 256 threads) do better with one branch after the other and more blocks
-// on an SM: 1024 x 1024, one slice each 7.6 us, 8.6 with FEW's loads; 1024 threads of four groups have no registers for two branches.
-template <typename T, int NC, bool FEW>
-__global__ void __launch_bounds__(NC == 2 ? 512 : NC == 1 && !FEW ? 256 : 1024, NC == 2 ? 2 : NC == 1 && !FEW ? 8 : 1) sublayer_close_vec_kernel(
+// the second branch) in registers from the sums to the normed store.  Many rows share the SMs here, so what counts is the blocks on
+// an SM: one branch after the other, the gains where they are used, no launch bounds (eight blocks asked for by them spilled: 1024 x 1024, one
+// slice per branch 6.9 us, 5.2 without; one branch of 1024 x 2048 6.8 and 6.3 with the kernel below).  Also few rows of four groups, whose
+// registers do not hold two branches (32 x 8192, two slices per branch 7.7 us within 64 registers, 6.0 here).
+template <typename T, int NC>
+__global__ void sublayer_close_rows_kernel(const float* __restrict__ y0, int64_t ld0, int ns0, int64_t stride0,
+                                          const float* __restrict__ gain0, float s0, const float* __restrict__ y1, int64_t ld1,
+                                          int ns1, int64_t stride1, const float* __restrict__ gain1, float s1,
+                                          const float* __restrict__ post_gain, const float* __restrict__ bias, int add,
+                                          const float* __restrict__ next_gain, float eps, int W, float* __restrict__ x,
+                                          T* __restrict__ xa) {
+  pdl_wait();
+  __shared__ float red[32];
+  const int64_t r = blockIdx.x, at = r * W;
+  const int n4 = W / 4;
+  auto sumsq = [](const float4& a) { return a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w; };
+  auto scaled = [](const float4& a, float f, const float* g) {       // a * f * g (g NULL: a * f)
+    if (!g) return make_float4(a.x * f, a.y * f, a.z * f, a.w * f);
+    const float4 w = ld4(g);
+    return make_float4(a.x * f * w.x, a.y * f * w.y, a.z * f * w.z, a.w * f * w.w);
+  };
+  float4 v[NC], xr[NC];
+#pragma unroll
+  for (int u = 0; u < NC; ++u) {
+    v[u] = xr[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int c = threadIdx.x + u * blockDim.x;
+    if (c < n4 && add) xr[u] = ld4(x + at + 4 * c);
+  }
+#pragma unroll 4
+  for (int k = 0; k < ns0; ++k)
+#pragma unroll
+    for (int u = 0; u < NC; ++u) {
+      const int c = threadIdx.x + u * blockDim.x;
+      if (c < n4) add4(v[u], ld4(y0 + k * stride0 + r * ld0 + 4 * c));
+    }
+  float f0 = s0;
+  if (gain0) {
+    float ss = 0.f;
+#pragma unroll
+    for (int u = 0; u < NC; ++u) ss += sumsq(v[u]);
+    f0 = s0 / sqrtf(block_sum(ss, red) / (float)W + eps);
+  }
+#pragma unroll
+  for (int u = 0; u < NC; ++u) {
+    const int c = threadIdx.x + u * blockDim.x;
+    if (c < n4) v[u] = scaled(v[u], f0, gain0 ? gain0 + 4 * c : nullptr);
+  }
+  if (y1) {
+    float4 b[NC];
+#pragma unroll
+    for (int u = 0; u < NC; ++u) b[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int k = 0; k < ns1; ++k)
+#pragma unroll
+      for (int u = 0; u < NC; ++u) {
+        const int c = threadIdx.x + u * blockDim.x;
+        if (c < n4) add4(b[u], ld4(y1 + k * stride1 + r * ld1 + 4 * c));
+      }
+    float f1 = s1;
+    if (gain1) {
+      float ss = 0.f;
+#pragma unroll
+      for (int u = 0; u < NC; ++u) ss += sumsq(b[u]);
+      f1 = s1 / sqrtf(block_sum(ss, red) / (float)W + eps);
+    }
+#pragma unroll
+    for (int u = 0; u < NC; ++u) {
+      const int c = threadIdx.x + u * blockDim.x;
+      if (c < n4) add4(v[u], scaled(b[u], f1, gain1 ? gain1 + 4 * c : nullptr));
+    }
+  }
+  if (post_gain) {
+    float ss = 0.f;
+#pragma unroll
+    for (int u = 0; u < NC; ++u) ss += sumsq(v[u]);
+    const float fp = 1.f / sqrtf(block_sum(ss, red) / (float)W + eps);
+#pragma unroll
+    for (int u = 0; u < NC; ++u) {
+      const int c = threadIdx.x + u * blockDim.x;
+      if (c < n4) v[u] = scaled(v[u], fp, post_gain + 4 * c);
+    }
+  }
+  float sx = 0.f;
+#pragma unroll
+  for (int u = 0; u < NC; ++u) {
+    const int c = threadIdx.x + u * blockDim.x;
+    if (c < n4) {
+      if (bias) add4(v[u], ld4(bias + 4 * c));
+      add4(v[u], xr[u]);
+      st4(x + at + 4 * c, v[u]);
+      sx += sumsq(v[u]);
+    }
+  }
+  float fn = 1.f;
+  if (next_gain) fn = 1.f / sqrtf(block_sum(sx, red) / (float)W + eps);
+#pragma unroll
+  for (int u = 0; u < NC; ++u) {
+    const int c = threadIdx.x + u * blockDim.x;
+    if (c < n4) st4(xa + at + 4 * c, next_gain ? scaled(v[u], fn, next_gain + 4 * c) : v[u]);
+  }
+}
+
+// The same for few rows and for two branches: bound by latency, as a row is read once by one block and a token step has fewer rows than
+// SMs.  So all slices of both branches, the residual and the branch gains are asked for before the first sum waits for any of them, the
+// gains (which no kernel of a step writes) come to L2 before the wait for the predecessor (asked for by the first block: all share them),
+// the next kernel may start its weights, and both branches' sums share their barriers: 32 rows x 2048 of eight slices each 5.4 -> 5.2 us,
+// 256 x 1024 of two 3.8 -> 3.1, 1024 x 2048 of one 11.0 -> 10.5; one branch alone gains by the next kernel's early start (a token step of
+// 32 x 2048, 4 layers 604 -> 582).  Four groups: only blocks of more than 512 threads, which the kernel above has no registers for.
+template <typename T, int NC>
+__global__ void __launch_bounds__(NC == 2 ? 512 : 1024, NC == 2 ? 2 : 1) sublayer_close_vec_kernel(
     const float* __restrict__ y0, int64_t ld0, int ns0, int64_t stride0, const float* __restrict__ gain0, float s0,
     const float* __restrict__ y1, int64_t ld1, int ns1, int64_t stride1, const float* __restrict__ gain1, float s1,
     const float* __restrict__ post_gain, const float* __restrict__ bias, int add, const float* __restrict__ next_gain, float eps, int W,
@@ -542,7 +643,7 @@ __global__ void __launch_bounds__(NC == 2 ? 512 : NC == 1 && !FEW ? 256 : 1024, 
   pdl_launch_dependents();          // the next kernel's weights
   __shared__ float2 red2[32];
   __shared__ float red[32];
-  constexpr bool kAhead = NC == 2 || (NC == 1 && FEW);   // else one branch after the other, the gains where they are used
+  constexpr bool kAhead = NC <= 2;             // else one branch after the other, the gains where they are used
   const int64_t r = blockIdx.x, at = r * W;
   const int n4 = W / 4;
   auto sumsq = [](const float4& a) { return a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w; };
@@ -559,7 +660,7 @@ __global__ void __launch_bounds__(NC == 2 ? 512 : NC == 1 && !FEW ? 256 : 1024, 
     if (kAhead && gain1) g1[u] = ld4(gain1 + 4 * c);
   }
   auto slices = [&](float4 (&a)[NC], const float* y, int64_t ld, int ns, int64_t stride) {
-#pragma unroll (NC == 1 && FEW ? 8 : 4)
+#pragma unroll (NC == 1 ? 8 : 4)
     for (int k = 0; k < ns; ++k)
 #pragma unroll
       for (int u = 0; u < NC; ++u) {
@@ -1337,14 +1438,16 @@ extern "C" int prl_sublayer_close(const float* y0, int64_t ld0, int32_t n_split0
     const int n4 = W / 4, nc = n > 256 ? (n4 <= 256 ? 1 : n4 <= 1024 ? 2 : 4) : (n4 <= 1024 ? 1 : 4);
     const int th = ((n4 + nc - 1) / nc + 31) / 32 * 32;
     const int64_t st0 = (int64_t)n * ld0, st1 = (int64_t)n * ld1;
-#define PRL_SC(T, NC, FEW) PRL_CUDA(launch_pdl((sublayer_close_vec_kernel<T, NC, FEW>), dim3(n), dim3(th), (size_t)0, (cudaStream_t)st, y0, ld0, n_split0, st0, gain0, s0, \
-                                          y1, ld1, n_split1, st1, gain1, s1, post_gain, bias, add, next_gain, eps, W, x, (T*)xa))
-#define PRL_SCT(T)                                 \
-  do {                                             \
-    if (nc == 1 && n > 256) PRL_SC(T, 1, false);   \
-    else if (nc == 1) PRL_SC(T, 1, true);          \
-    else if (nc == 2) PRL_SC(T, 2, false);         \
-    else PRL_SC(T, 4, false);                      \
+#define PRL_SC(K, T, NC) PRL_CUDA(launch_pdl((K<T, NC>), dim3(n), dim3(th), (size_t)0, (cudaStream_t)st, y0, ld0, n_split0, st0, gain0, s0, \
+                                         y1, ld1, n_split1, st1, gain1, s1, post_gain, bias, add, next_gain, eps, W, x, (T*)xa))
+#define PRL_SCT(T)                                                   \
+  do {                                                               \
+    if (nc == 1 && n > 256) PRL_SC(sublayer_close_rows_kernel, T, 1);  \
+    else if (nc == 1) PRL_SC(sublayer_close_vec_kernel, T, 1);       \
+    else if (nc == 2 && !y1) PRL_SC(sublayer_close_rows_kernel, T, 2); \
+    else if (nc == 2) PRL_SC(sublayer_close_vec_kernel, T, 2);       \
+    else if (th <= 512) PRL_SC(sublayer_close_rows_kernel, T, 4);    \
+    else PRL_SC(sublayer_close_vec_kernel, T, 4);                    \
   } while (0)
     if (f32) PRL_SCT(float);
     else PRL_SCT(bf16);

@@ -411,6 +411,27 @@ def test_sublayer_close_rows(cuda_device, n, W, k0, k1):
     assert (out.double() - rms(want) * gn).norm() < 2e-6 * (rms(want) * gn).norm()
 
 
+@pytest.mark.parametrize("n,W,k0,k1", [(300, 1024, 1, 1), (257, 128, 2, 0), (300, 1024, 4, 4), (260, 2048, 2, 0), (5, 8192, 2, 1), (4, 8196, 1, 2), (256, 1024, 4, 0),
+                                       (3, 16384, 2, 0)])
+@pytest.mark.parametrize("f32", [1, 0])
+def test_sublayer_close_rows_of_every_schedule(cuda_device, n, W, k0, k1, f32):
+    """prl_sublayer_close without the post norm, against 64 bits: many and few rows of one, two and four groups of channels per thread, of
+    one branch and of two, stored in both types."""
+    from pipelinerl_b200 import _lib
+    lib, g = _lib.load(), torch.Generator(device="cuda").manual_seed(W + n)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    y0, y1, x, g0, g1, gn = rnd(k0, n, W), rnd(max(k1, 1), n, W), rnd(n, W), rnd(W), rnd(W), rnd(W)
+    rms = lambda v: v * torch.rsqrt((v * v).mean(-1, keepdim=True) + 1e-5)  # noqa: E731
+    want = x.double() + 0.7 * rms(y0.double().sum(0)) * g0 + (1.3 * rms(y1.double().sum(0)) * g1 if k1 else 0)
+    out, ptr = torch.empty(n, W, device="cuda", dtype=torch.float32 if f32 else torch.bfloat16), lambda t: t.data_ptr()  # noqa: E731
+    _lib.check(lib.prl_sublayer_close(ptr(y0), W, k0, ptr(g0), 0.7, ptr(y1) if k1 else None, W, max(k1, 1), ptr(g1) if k1 else None, 1.3, None,
+                                      None, 1, ptr(gn), 1e-5, n, W, ptr(x), ptr(out), f32, _lib.stream_ptr()))
+    # a few fp32 roundings and norms good to a few ulp: 1e-6 of the row's scale; the bf16 store rounds once more, 2^-9 a value at most
+    assert (x.double() - want).norm() < 1e-6 * want.norm()
+    final = rms(want) * gn
+    assert (out.double() - final).norm() < (2e-6 if f32 else 2.0 ** -9) * final.norm()
+
+
 @pytest.mark.parametrize("n,H,G,dim,vdim,rot", [(1, 1, 0, 128, 32, 128), (33, 16, 4, 128, 128, 64), (297, 5, 1, 32, 96, 0), (300, 40, 8, 64, 64, 64),
                                                 (9, 3, 3, 96, 128, 64)])
 @pytest.mark.parametrize("norms", [False, True])
