@@ -1145,9 +1145,10 @@ __global__ void attn_front_kernel(const float* __restrict__ P, int64_t ldp, int 
 // attn_front_kernel for heads of whole warps' widths (dim and vdim multiples of 32 up to 128, rot a multiple of 64): a lane holds channels
 // lane + 32 k of its head, so both channels of a turned pair are its own, and a head is read once.
 // Bound by the chain of its loads on a token step (row -> page -> store): the head's channels, the row's position and slot are asked for
-// together, the page while the angles are computed, and a warp has one head.  The values of attn_front_kernel, bit for bit.
-// 16 + 2 x 4 heads of 128, 64 turned channels: 32 rows 3.9 -> 3.4 us, 1024 rows 25.0 -> 12.4.
-template <typename T>
+// together, the page while the angles are computed, and a warp has one head (kOneHead), or takes heads in turn (kInTurn), the next one on its
+// way (kNextAhead).  The values of attn_front_kernel, bit for bit.
+enum FrontHeads { kOneHead, kInTurn, kNextAhead };
+template <typename T, FrontHeads HEADS>
 __global__ void __launch_bounds__(1024) attn_front_lanes_kernel(
     const float* __restrict__ P, int64_t ldp, int off_q, int off_k, int off_v, int H, int G, int dim, int vdim,
     const float* __restrict__ q_bias, const float* __restrict__ k_bias, const float* __restrict__ v_bias, int qk_norm,
@@ -1161,17 +1162,17 @@ __global__ void __launch_bounds__(1024) attn_front_lanes_kernel(
   pdl_wait();
   pdl_launch_dependents();
   const int r = blockIdx.x;
-  float raw[4];
-  auto fetch = [&](int hh) {         // past the head's width: not read
+  float raw[4], next[4];
+  auto fetch = [&](int hh, float (&to)[4]) {         // past the head's width: not read
     const bool is_v = hh >= H + G;
     const int head = hh < H ? hh : is_v ? hh - H - G : hh - H, width = is_v ? vdim : dim;
     const float* src = P + (int64_t)r * ldp + (hh < H ? off_q : is_v ? off_v : off_k) + head * width;
     const float* bias = hh < H ? q_bias : is_v ? v_bias : k_bias;
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      raw[k] = 32 * k < width ? src[lane + 32 * k] + (bias ? bias[head * width + lane + 32 * k] : 0.f) : 0.f;
+      to[k] = 32 * k < width ? src[lane + 32 * k] + (bias ? bias[head * width + lane + 32 * k] : 0.f) : 0.f;
   };
-  if (warp < H + 2 * G) fetch(warp);
+  if (warp < H + 2 * G) fetch(warp, raw);
   const int slot = row_slot[r], pos = row_pos[r];
   if (slot < 0) return;
   const int page = block_table[(int64_t)slot * max_blocks + pos / page_size], within = pos % page_size;
@@ -1185,8 +1186,14 @@ __global__ void __launch_bounds__(1024) attn_front_lanes_kernel(
     trig[half + tid] = sn * mag;
   }
   __syncthreads();
+  if (HEADS == kNextAhead && warp + nw < H + 2 * G) fetch(warp + nw, next);
   for (int hh = warp; hh < H + 2 * G; hh += nw) {
-    if (hh != warp) fetch(hh);
+    if (HEADS == kInTurn && hh != warp) fetch(hh, raw);
+    if (HEADS == kNextAhead && hh != warp) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) raw[k] = next[k];
+      if (hh + nw < H + 2 * G) fetch(hh + nw, next);
+    }
     const bool is_v = hh >= H + G;
     const int width = is_v ? vdim : dim;
     float inv = 1.f;
@@ -1618,15 +1625,28 @@ extern "C" int prl_attn_front(const float* P, int64_t ldp, int32_t off_q, int32_
                 "prl_attn_front: bad shape (H=%d G=%d dim=%d vdim=%d rot=%d)", H, G, dim, vdim, rot);
   PRL_CHECK_ARG(v_blend >= 0 && v_blend <= 2 && (v_blend == 0 || v_first) && (v_blend != 2 || v_lambda),
                 "prl_attn_front: blending the values needs the first layer's values and the weight");
-  if (dim % 32 == 0 && dim <= 128 && vdim % 32 == 0 && vdim <= 128 && rot % 64 == 0) {
-    // few rows: a warp per head, the shortest chain; rows that fill the SMs: eight warps, so that several blocks share one
-    const int heads = H + 2 * G, most = n > 2 * 148 ? 8 : 32, w = heads < most ? heads : most, th = 32 * (w < 2 ? 2 : w);   // rot / 2 <= th
-#define PRL_AF(T)                                                                                                                      \
-  PRL_CUDA(launch_pdl(attn_front_lanes_kernel<T>, dim3(n), dim3(th), (size_t)0, (cudaStream_t)st, P, ldp, off_q, off_k, off_v, H, G, dim, \
-                      vdim, q_bias, k_bias, v_bias, qk_norm, q_gain, k_gain, gain_period, eps, rot, freq, mag, v_norm, v_blend, v_lambda, \
-                      v_first, row_pos, row_slot, block_table, max_blocks, page_size, (T*)q_out, (T*)k_pool, (T*)v_pool))
-    if (f32) PRL_AF(float);
-    else PRL_AF(bf16);
+  const int heads = H + 2 * G, sms = num_sms();
+  // Warps for the lanes kernel, by rows and heads; 0 = attn_front_kernel, whose blocks of up to 16 warps leave room for a second one on an
+  // SM between one and two rows per SM, and whose rounds over many heads of few rows are shorter.  attn_front_kernel -> this one, us:
+  // 24 heads of 128: 32 rows 3.8 -> 3.1, 1024 rows 13.2 -> 9.0, 2500 rows 28.4 -> 17.0 (200 rows 4.1, 3.9; of 64: 3.3, 3.5); 48 heads of 128:
+  // 32 rows 4.3, 4.9; 450 rows 8.6, 9.9; 1024 rows 15.3 -> 14.7, 2500 rows 46.1 -> 40.6; 80 heads: 32 rows 5.5, 6.4; 2500 rows 71.9, 79.6.
+  int w = 0;
+  if (heads <= 32) w = n <= sms ? (heads < 2 ? 2 : heads) : n > 2 * sms ? (heads < 2 ? 2 : heads < 8 ? heads : 8) : 0;
+  else if (heads <= 64) w = n <= sms && rot < dim ? 32 : n > 8 * sms ? 8 : n > 4 * sms ? 12 : 0;
+  if (dim % 32 == 0 && dim <= 128 && vdim % 32 == 0 && vdim <= 128 && rot % 64 == 0 && w) {     // rot / 2 <= 32 * w
+#define PRL_AF(T, HEADS)                                                                                                               \
+  PRL_CUDA(launch_pdl((attn_front_lanes_kernel<T, HEADS>), dim3(n), dim3(32 * w), (size_t)0, (cudaStream_t)st, P, ldp, off_q, off_k, off_v, \
+                      H, G, dim, vdim, q_bias, k_bias, v_bias, qk_norm, q_gain, k_gain, gain_period, eps, rot, freq, mag, v_norm, v_blend, \
+                      v_lambda, v_first, row_pos, row_slot, block_table, max_blocks, page_size, (T*)q_out, (T*)k_pool, (T*)v_pool))
+#define PRL_AFT(T)                         \
+  do {                                     \
+    if (w >= heads) PRL_AF(T, kOneHead);     \
+    else if (w == 12) PRL_AF(T, kNextAhead); \
+    else PRL_AF(T, kInTurn);                \
+  } while (0)
+    if (f32) PRL_AFT(float);
+    else PRL_AFT(bf16);
+#undef PRL_AFT
 #undef PRL_AF
     PRL_LAUNCH_CHECK();
     return PRL_OK;
