@@ -343,6 +343,74 @@ def test_router_rows_equal_the_staged_router(cuda_device, dtype, n, W, experts, 
         assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
+def ranked_on_the_host(z, corr, top, groups, keep, group_top, sigmoid, renorm, scale):
+    """The choice for one row of logits, entry by entry: ties go to the lower index, NaN is never the largest, an entry or a group that
+    is minus infinity is never taken in a round, and a group that has not been taken is closed if it is anything but minus infinity."""
+    import numpy as np
+    with np.errstate(all="ignore"):
+        z = z.astype(np.float32)
+        e = np.exp(z - np.fmax.reduce(z))
+        score = (1 / (1 + np.exp(-z)) if sigmoid else e * (np.float32(1) / e.sum(dtype=np.float32))).astype(np.float32)
+        c, size = score + corr, len(z) // groups
+
+        def largest(v):
+            best, at = -np.inf, None
+            for i, x in enumerate(v):
+                if x > best:
+                    best, at = x, i
+            return at
+        if keep < groups:
+            gs = []
+            for g in range(groups):
+                m = m2 = np.float32(-np.inf)
+                for x in c[g * size:(g + 1) * size]:
+                    m2, m = np.fmax(m2, np.fmin(m, x)), np.fmax(m, x)
+                gs.append(m + m2 if group_top > 1 and size > 1 else m)
+            for _ in range(keep):
+                g = largest(gs)
+                if g is not None:
+                    gs[g] = -np.inf
+            c = np.array([-np.inf if gs[i // size] != -np.inf else x for i, x in enumerate(c)], dtype=np.float32)
+        sel, w = [], []
+        for _ in range(top):
+            i = largest(c)
+            sel.append(0 if i is None else i)
+            w.append(np.float32(0) if i is None else score[i])
+            if i is not None:
+                c[i] = -np.inf
+        w = np.array(w, dtype=np.float32)
+        return sel, w * np.float32(scale) / ((w.sum() + np.float32(1e-20)) if renorm else np.float32(1))
+
+
+@pytest.mark.parametrize("E,groups,keep,top", [(1, 1, 1, 1), (4, 1, 1, 4), (16, 8, 6, 4), (16, 8, 8, 5), (24, 3, 1, 8), (32, 32, 5, 3), (32, 4, 2, 16), (31, 1, 1, 31),
+                                               (32, 1, 1, 32), (33, 3, 1, 5), (64, 8, 3, 7)])
+def test_choice_of_outputs_against_the_host(cuda_device, E, groups, keep, top):
+    """Up to 32 outputs are ranked in registers, more in shared memory: both against a plain restatement, for equal logits, zeros of both
+    signs, infinities and NaN in logits and corrections.  The logits are those whose scores are exact on both sides (sigmoids 0, 1/2 and 1,
+    softmax shares 0 and 1 / k), so that every comparison falls the same way."""
+    import numpy as np
+    from pipelinerl_b200 import _lib
+    lib, st, rng, n = _lib.load(), _lib.stream_ptr(), np.random.default_rng(E + groups), 96
+    i32 = dict(dtype=torch.int32, device="cuda")
+    for trial in range(8):
+        z = rng.choice(np.array([-200.0, -0.0, 0.0, 0.0, 200.0, 200.0], dtype=np.float32), (n, E))
+        odd = rng.random((n, E)) < 0.2 * (rng.random((n, 1)) < 0.6)
+        z[odd] = rng.choice(np.array([np.inf, -np.inf, np.nan, -np.inf], dtype=np.float32), int(odd.sum()))
+        corr = (rng.integers(-24, 25, E) / (8 if trial < 4 else 64)).astype(np.float32)
+        corr[rng.random(E) < 0.15] = (0.0, -np.inf, -0.0, np.nan)[trial % 4]
+        sigmoid, renorm, group_top = trial & 1, trial >> 1 & 1, 1 + (trial >> 2 & 1)
+        sel, wsel, perm = torch.full((top, n), -7, **i32), torch.full((top, n), -7.0, device="cuda"), torch.zeros(top * n, **i32)
+        meta, tiles = torch.zeros(4, **i32), torch.zeros(3 * int(lib.prl_moe_max_tiles(top * n, E)), **i32)
+        zd, cd = torch.from_numpy(z).cuda(), torch.from_numpy(corr).cuda()
+        _lib.check(lib.prl_moe_choose(zd.data_ptr(), E, cd.data_ptr(), n, E, E, top, groups, keep, group_top, sigmoid, renorm, 1.25, 64, sel.data_ptr(),
+                                      wsel.data_ptr(), perm.data_ptr(), meta.data_ptr(), tiles.data_ptr(), st))
+        for t in range(n):
+            want, w = ranked_on_the_host(z[t], corr, top, groups, keep, group_top, sigmoid, renorm, 1.25)
+            assert sel[:, t].tolist() == want, (trial, t)
+            # the scores are exact or one rounding away (1 / k); the sum of up to 32 of them and the division add 2^-24 each at most
+            np.testing.assert_allclose(wsel[:, t].cpu().numpy(), w, rtol=5e-6, atol=1e-30, equal_nan=True)
+
+
 @pytest.mark.parametrize("plain_gemm", [False, True])
 def test_bf16_serving_mode(cuda_device, plain_gemm):
     """bf16 operands and cache with the tensor-core GEMMs (and with the CUDA-core GEMM) against the float64 oracle.  Only the
