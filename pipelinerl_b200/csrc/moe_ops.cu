@@ -105,7 +105,7 @@ __device__ __forceinline__ int warp_best(float v) {
   return top ? __ffs(at) - 1 : 0x7fffffff;
 }
 
-// choose_row for at most 32 outputs: a lane holds one, so that a round of the ranking is three instructions instead of a walk through
+// choose_row_walk for at most 32 outputs: a lane holds one, so that a round of the ranking is three instructions instead of a walk through
 // shared memory and a shuffle tree (16 outputs, 8 groups, 6 + 4 rounds: with the walk the choice was half of the router kernel's 13 us
 // on 32 rows).  The same values, sums and ties.
 __device__ __forceinline__ void choose_row_lanes(const float* z, int E, const ChoiceRule& r, int n, int t, int32_t* __restrict__ sel,
@@ -153,9 +153,8 @@ __device__ __forceinline__ void choose_row_lanes(const float* z, int E, const Ch
 
 // The choice for one row by one warp: c [E] and gs [groups] are the warp's scratch in shared memory, z [E] the logits.
 // Outputs are ranked by score + correction, closed groups count as minus infinity; ties go to the lower index.
-__device__ __forceinline__ void choose_row(const float* z, int E, const ChoiceRule& r, float* c, float* gs, int n, int t,
-                                           int32_t* __restrict__ sel, float* __restrict__ wsel) {
-  if (E <= 32) return choose_row_lanes(z, E, r, n, t, sel, wsel);
+__device__ __forceinline__ void choose_row_walk(const float* z, int E, const ChoiceRule& r, float* c, float* gs, int n, int t,
+                                                int32_t* __restrict__ sel, float* __restrict__ wsel) {
   const int lane = threadIdx.x & 31;
   float zmax = 0.f, inv = 1.f;
   if (!r.sigmoid) {
@@ -225,6 +224,12 @@ __device__ __forceinline__ void choose_row(const float* z, int E, const ChoiceRu
   }
 }
 
+__device__ __forceinline__ void choose_row(const float* z, int E, const ChoiceRule& r, float* c, float* gs, int n, int t,
+                                           int32_t* __restrict__ sel, float* __restrict__ wsel) {
+  if (E <= 32) choose_row_lanes(z, E, r, n, t, sel, wsel);
+  else choose_row_walk(z, E, r, c, gs, n, t, sel, wsel);
+}
+
 // Choice from ready logits, one warp per row.
 constexpr int kChooseWarps = 4;
 __global__ void __launch_bounds__(kChooseWarps * 32) moe_choose_kernel(const float* __restrict__ logits, int64_t ld, int n, int E,
@@ -285,7 +290,10 @@ __device__ __forceinline__ void top_of_row(const float* z, int E, int top, int s
 // Router and choice in one kernel: logits[e] = x . Wr[e] in fp32 (block per row, warps
 // take experts in turn, a lane sums every 32nd group of channels, then the warp's shuffle tree: a fixed order), then the top-k
 // pass of moe_route_kernel over the logits in shared memory (RULED: choose_row instead, with scratch behind the logits).
-template <typename TX, typename TW, bool RULED>
+// One element type and aligned rows: the row is read beside the weights, not staged.  Many rows share the SMs, so the two rankings are
+// instances of their own: both in one took registers that cost a block of six.
+enum { kTopOnly = 0, kRanked = 1, kRankedInLanes = 2 };
+template <typename TX, typename TW, int CHOICE>
 __global__ void __launch_bounds__(256) moe_router_kernel(const TX* __restrict__ x, const TW* __restrict__ Wr,
                                                          const float* __restrict__ bias, int n, int W, int E, int top,
                                                          int softmax_weights, ChoiceRule rule, int32_t* __restrict__ sel,
@@ -297,12 +305,25 @@ __global__ void __launch_bounds__(256) moe_router_kernel(const TX* __restrict__ 
   const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   constexpr int V = 16 / sizeof(TW);              // router weights per 16-byte load
   const bool vec = W % V == 0 && ((uintptr_t)Wr & 15) == 0;
-  for (int c = threadIdx.x; c < W; c += blockDim.x) xs[c] = to_f32(x[(int64_t)t * W + c]);
-  __syncthreads();
+  const bool direct = sizeof(TX) == sizeof(TW) && vec && ((uintptr_t)x & 15) == 0;
+  if (!direct) {
+    for (int c = threadIdx.x; c < W; c += blockDim.x) xs[c] = to_f32(x[(int64_t)t * W + c]);
+    __syncthreads();
+  }
   for (int e = warp; e < E; e += nw) {
     const TW* w = Wr + (int64_t)e * W;
     float a = 0.f;
-    if (vec) {
+    if (direct) {                                 // a lane sums its channels in ascending order
+      const TX* xr = x + (int64_t)t * W;
+#pragma unroll 4
+      for (int c = V * lane; c < W; c += 32 * V) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(w + c), xraw = *reinterpret_cast<const uint4*>(xr + c);
+        const TW* wv = reinterpret_cast<const TW*>(&raw);
+        const TX* xv = reinterpret_cast<const TX*>(&xraw);
+#pragma unroll
+        for (int j = 0; j < V; ++j) a = fmaf(to_f32(xv[j]), to_f32(wv[j]), a);
+      }
+    } else if (vec) {
 #pragma unroll 4
       for (int c = V * lane; c < W; c += 32 * V) {
         const uint4 raw = *reinterpret_cast<const uint4*>(w + c);
@@ -324,19 +345,17 @@ __global__ void __launch_bounds__(256) moe_router_kernel(const TX* __restrict__ 
   }
   __syncthreads();
   if (warp != 0) return;
-  if constexpr (RULED) {
-    choose_row(z, E, rule, z + E, z + 2 * E, n, t, sel, wsel);
-    return;
-  }
-  top_of_row(z, E, top, softmax_weights, n, t, sel, wsel);
+  if constexpr (CHOICE == kRankedInLanes) choose_row_lanes(z, E, rule, n, t, sel, wsel);
+  else if constexpr (CHOICE == kRanked) choose_row_walk(z, E, rule, z + E, z + 2 * E, n, t, sel, wsel);
+  else top_of_row(z, E, top, softmax_weights, n, t, sel, wsel);
 }
 
 // moe_router_kernel for rows and router weights of one element type, both on 16-byte boundaries: ROWS rows per block of 16 warps, which
 // take experts in turn.  A weight chunk is read once for the block's rows and the rows beside it, all chunks of a batch in flight
 // together; the first expert's weights, which no earlier kernel writes, are on their way before the wait for the row.  A lane sums its
 // channels in ascending order, then the shuffle tree: per (row, expert) the sums of moe_router_kernel.
-// Bound by the latency of its loads and of the choice.  2048 channels, 16 experts, with the grouping behind it: 1024 rows 24.8 -> 15.3 us,
-// 32 rows of a token step 17 -> 11 us (its weights come from HBM there), 128 experts on 32 rows 33.5 -> 20.0.
+// Bound by the latency of its loads and of the choice.  2048 channels, 16 experts, with the grouping behind it: 1024 rows 24.2 -> 14.5 us,
+// 32 rows of a token step 17 -> 11 us (its weights come from HBM there), 128 experts on 32 rows 32.4 -> 18.9.
 constexpr int kRouterWarps = 16;
 template <typename T, bool RULED, int ROWS>
 __global__ void __launch_bounds__(32 * kRouterWarps) moe_router_rows_kernel(const T* __restrict__ x, const T* __restrict__ Wr,
@@ -822,14 +841,22 @@ static int moe_router_impl(const void* x, int32_t x_is_f32, const void* Wr, int3
   PRL_CHECK_ARG(n >= 1 && W >= 1 && outputs >= 1 && outputs <= 32 * kMaxPerLane && top >= 1 && top <= outputs,
                 "prl_moe_router: bad shape (outputs=%d top=%d; at most %d outputs)", outputs, top, 32 * kMaxPerLane);
   const size_t smem = ((size_t)W + outputs + (rule ? outputs + rule->groups : 0)) * sizeof(float);
+  // one limit for every schedule, whether it stages the row or not: what is refused does not depend on alignment or on the rows
   PRL_CHECK_ARG(smem <= 160 * 1024, "prl_moe_router: a row of %d channels does not fit in shared memory", W);
   cudaStream_t s = (cudaStream_t)st;
-  const int per = x_is_f32 ? 4 : 8;
-  if (!x_is_f32 == !w_is_f32 && W % per == 0 && (((uintptr_t)x | (uintptr_t)Wr) & 15) == 0) {
-    // one block of 16 warps fits an SM: as many rows share a block as keep the blocks in one wave (with the grouping behind it, 2048
-    // channels, 16 experts: 452 rows 18.3 us by one, 10.9 by four; 1024 rows 17.9 by four, 15.3 by eight)
-    const size_t per_row = (outputs + (rule ? outputs + rule->groups : 0)) * sizeof(float);      // at most 12 KB
-    const int rows = n > 4 * 148 && 8 * per_row <= 48 * 1024 ? 8 : n > 148 ? 4 : 1;
+  const int per = x_is_f32 ? 4 : 8, sms = num_sms();
+  const size_t per_row = (outputs + (rule ? outputs + rule->groups : 0)) * sizeof(float);      // at most 12 KB
+  // A block of 16 warps for 1, 2, 4 or 8 rows (one fits an SM: as many rows share it as keep the blocks in one wave), or a block of eight for
+  // each row (six fit): rows that fill the SMs anyway, whose waves those fit better, and few experts, which leave warps of the former idle.
+  // Rows and type as on the lines; us, block per row / rows sharing one, with the grouping behind it, router of E outputs:
+  // 2048 channels bf16, E = 16: 149 rows 11.7 / 7.8, 296 12.7 / 8.7, 592 10.8 / 11.4, 850 12.7 / 15.1, 1024 16.8 / 14.5, 4096 40.9 / 49.0;
+  // E = 128: 149 rows 34 / 26, 592 43 / 40, 593 54 / 64, 1024 83 / 67, 4096 233 / 254; fp32: E = 16: 593 rows 16.6 / 14.0, 4096 72 / 46;
+  // E = 8: 593 rows 9.3 / 11.3, 850 10.2 / 11.5, 1024 15.3 / 11.6.
+  const bool alone = n <= 2 * sms ? false : n <= 4 * sms ? !x_is_f32 && outputs < 128 : n <= 6 * sms ? !x_is_f32 || outputs <= 8
+                   : n <= 8 * sms ? !x_is_f32 && outputs <= 8 : !x_is_f32;
+  int rows = alone ? 0 : n <= sms ? 1 : n <= 2 * sms ? 2 : n <= 4 * sms ? 4 : 8;
+  if (rows == 8 && 8 * per_row > 48 * 1024) rows = 4;
+  if (rows && !x_is_f32 == !w_is_f32 && W % per == 0 && (((uintptr_t)x | (uintptr_t)Wr) & 15) == 0) {
     const size_t sm = rows * per_row;
 #define PRL_RR(T, RULED, ROWS)                                                                                                    \
   PRL_CUDA(launch_pdl((moe_router_rows_kernel<T, RULED, ROWS>), dim3((n + ROWS - 1) / ROWS), dim3(32 * kRouterWarps), sm, s, (const T*)x, \
@@ -839,8 +866,8 @@ static int moe_router_impl(const void* x, int32_t x_is_f32, const void* Wr, int3
     if (rule) PRL_RR(T, true, ROWS);      \
     else PRL_RR(T, false, ROWS);          \
   } while (0)
-    if (x_is_f32) { if (rows == 8) PRL_RR2(float, 8); else if (rows == 4) PRL_RR2(float, 4); else PRL_RR2(float, 1); }
-    else { if (rows == 8) PRL_RR2(bf16, 8); else if (rows == 4) PRL_RR2(bf16, 4); else PRL_RR2(bf16, 1); }
+    if (x_is_f32) { if (rows == 8) PRL_RR2(float, 8); else if (rows == 4) PRL_RR2(float, 4); else if (rows == 2) PRL_RR2(float, 2); else PRL_RR2(float, 1); }
+    else { if (rows == 8) PRL_RR2(bf16, 8); else if (rows == 4) PRL_RR2(bf16, 4); else if (rows == 2) PRL_RR2(bf16, 2); else PRL_RR2(bf16, 1); }
 #undef PRL_RR2
 #undef PRL_RR
     PRL_LAUNCH_CHECK();
@@ -848,17 +875,18 @@ static int moe_router_impl(const void* x, int32_t x_is_f32, const void* Wr, int3
     PRL_LAUNCH_CHECK();
     return PRL_OK;
   }
-  static SmemAttr attr[8] = {};
-#define PRL_RT(TX, TW, RULED, I)                                                                                       \
+  static SmemAttr attr[12] = {};
+#define PRL_RT(TX, TW, CHOICE, I)                                                                                      \
   do {                                                                                                                 \
-    if (smem > 48 * 1024) PRL_CUDA(ensure_smem(moe_router_kernel<TX, TW, RULED>, (int)smem, attr[I]));                 \
-    PRL_CUDA(launch_pdl((moe_router_kernel<TX, TW, RULED>), dim3(n), dim3(256), smem, s, (const TX*)x, (const TW*)Wr, bias, n, W, \
+    if (smem > 48 * 1024) PRL_CUDA(ensure_smem(moe_router_kernel<TX, TW, CHOICE>, (int)smem, attr[I]));                \
+    PRL_CUDA(launch_pdl((moe_router_kernel<TX, TW, CHOICE>), dim3(n), dim3(256), smem, s, (const TX*)x, (const TW*)Wr, bias, n, W, \
                         outputs, top, softmax_weights, rule ? *rule : ChoiceRule{}, sel, wsel));                       \
   } while (0)
-#define PRL_RT2(TX, TW, I)                \
-  do {                                    \
-    if (rule) PRL_RT(TX, TW, true, I);    \
-    else PRL_RT(TX, TW, false, I + 4);    \
+#define PRL_RT2(TX, TW, I)                                       \
+  do {                                                           \
+    if (!rule) PRL_RT(TX, TW, kTopOnly, I);                      \
+    else if (outputs > 32) PRL_RT(TX, TW, kRanked, I + 4);       \
+    else PRL_RT(TX, TW, kRankedInLanes, I + 8);                  \
   } while (0)
   if (x_is_f32 && w_is_f32) PRL_RT2(float, float, 0);
   else if (x_is_f32) PRL_RT2(float, bf16, 1);

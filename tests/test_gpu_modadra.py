@@ -343,6 +343,14 @@ def test_router_rows_equal_the_staged_router(cuda_device, dtype, n, W, experts, 
         assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,W,experts,groups,keep,top", [(149, 264, 16, 4, 2, 3), (297, 136, 128, 8, 4, 8), (450, 1032, 8, 1, 1, 2), (600, 136, 8, 1, 1, 2), (889, 72, 16, 8, 6, 4),
+                                                         (1185, 264, 32, 4, 2, 6)])
+def test_router_of_every_schedule(cuda_device, dtype, n, W, experts, groups, keep, top):
+    """One, two, four and eight rows a block and a block per row: the lines lie at one, two, four, six and eight rows per SM (148)."""
+    test_router_rows_equal_the_staged_router(cuda_device, dtype, n, W, experts, groups, keep, top)
+
+
 def ranked_on_the_host(z, corr, top, groups, keep, group_top, sigmoid, renorm, scale):
     """The choice for one row of logits, entry by entry: ties go to the lower index, NaN is never the largest, an entry or a group that
     is minus infinity is never taken in a round, and a group that has not been taken is closed if it is anything but minus infinity."""
