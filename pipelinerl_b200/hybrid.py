@@ -1344,8 +1344,9 @@ class HybridEngine(EngineCore):
         self.split_scan = not self.f32
         self.split_min_rows = 256
         self.piece_tokens = 64             # tokens per piece (tests lower it); at most prl_lin_scan_piece_tokens()
-        # The two branches of an attention-beside-delta-rule layer on two streams; they share no buffer they write.  Off: one after the other.
-        self.side_branches = True
+        # The two branches of an attention-beside-delta-rule layer on two streams; they share no buffer they write.  None: where that pays
+        # (_branches_beside); True: always; False: one after the other.
+        self.side_branches: bool | None = None
         self._side = None                  # the second stream and its two events, made with the first such layer
         self._rows: _Rows | None = None
         super().__init__(cfg, arena, **kw)
@@ -2093,7 +2094,8 @@ class HybridEngine(EngineCore):
         # The attention branch (q, ya, y0, the caches) beside the delta rule's (aux, dprep, scratch, o, yb, y1, the states): neither fills the
         # chip alone -- the walk over a prompt's pieces is a serial chain, a token step's state update and attention wait for memory.
         main, st = torch.cuda.current_stream(), self._st
-        if self.side_branches:
+        beside = self._branches_beside(R)
+        if beside:
             if self._side is None:
                 self._side = (torch.cuda.Stream(self.dev), torch.cuda.Event(), torch.cuda.Event())
             side, fork, join = self._side
@@ -2106,14 +2108,24 @@ class HybridEngine(EngineCore):
                 k0 = self._mm(R.ya, a.heads * a.vdim, w + "mix.left.o", W, R.y0, n, split=True)
             finally:
                 self._st = st
-                if self.side_branches:
+                if beside:
                     join.record(side)
             self._gated_delta_cell(R, n, i, g, w + "mix.right.", segs, max_q, R.P.data_ptr(), C.total, C.right, C.b, C.a, C.right_g)
             k1 = self._mm(R.yb, g.heads * g.vdim, w + "mix.right.o", W, R.y1, n, split=True)
         finally:
-            if self.side_branches:
+            if beside:
                 main.wait_event(join)
         return k0, k1
+
+    def _branches_beside(self, R) -> bool:
+        """A captured token step takes the branches on two streams at no cost to the host (32 x 1100, 4 layers of 2048: 623 -> 583 us, of
+        1024: 413 -> 375; one sequence: 435 -> 405, 299 -> 260).  A prompt's launches come from the host one by one, and fork and join are
+        20 us more of them a layer: wide layers gain on the device (1024 tokens, 2 layers of 2048: 994 -> 975 us, of 1536: 887 -> 862; 150
+        tokens: 677 -> 662, 578 -> 539), narrow ones wait for the host (of 1024: 731 -> 760, 440 -> 476; of 512: 721 -> 755, 433 -> 473), and
+        so does a token step that is not captured."""
+        if self.side_branches is not None:
+            return self.side_branches
+        return self.use_graph if R is self._dec else self.cfg.width >= 1536
 
     def _gated_window_attn(self, R, n, i, a, C, segs, max_q, row_pos, seg_pos0) -> None:
         """Softmax attention from the projections in R.P (AttnDeltaRows) to the gated heads R.ya."""

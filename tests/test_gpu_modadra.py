@@ -461,6 +461,19 @@ def test_branches_on_two_streams_equal_one_after_the_other(cuda_device, graph):
     assert got[0] == got[1] == got[2]
 
 
+@pytest.mark.parametrize("graph", [False, True])
+def test_narrow_prompts_keep_one_stream(cuda_device, graph):
+    """Where nothing else is asked for, a narrow decoder's prompts and its uncaptured token steps run on one stream, captured steps on two."""
+    from pipelinerl_b200.engine import SamplingParams
+    eng = mc.build_engine(BIG, mc.weights(BIG, 5), torch.bfloat16, cuda_device, max_batch=2, max_seq_len=400, use_cuda_graph=graph)
+    s = eng.open_stream()
+    eng.feed([(s, mc.tokens_for(BIG, 300, seed=1), [299])])
+    eng.close_stream(s)
+    assert eng._side is None
+    eng.generate([mc.tokens_for(BIG, 9, seed=2)], SamplingParams(max_tokens=3, greedy=True, ignore_eos=True))
+    assert (eng._side is not None) == graph
+
+
 def test_grouped_tensor_core_experts_in_long_prompts(cuda_device):
     """More routed pairs per expert than the few-row grouped GEMM is for: the tcgen05 grouped GEMM with the gelu epilogue
     against the few-row kernel on the same weights."""
