@@ -778,7 +778,9 @@ int64_t prl_moe_max_tiles(int64_t pairs, int32_t experts);
 int prl_moe_route(const float* logits, int64_t ld, const float* bias /* [experts] added to the logits, or NULL */, int32_t n,
                   int32_t experts, int32_t top, int32_t softmax_weights,
                   int32_t* sel, float* wsel, int32_t* perm, int32_t* meta, int32_t* tiles, prl_stream_t stream);
-/* router product (fp32 sums in a fixed order), choice and grouping without the logits going through memory */
+/* router product (fp32 sums in a fixed order), choice and grouping without the logits going through memory.  Here and in
+ * prl_moe_router_choose the router matrix is read ahead of the wait for the stream's preceding kernel: no kernel that lets its
+ * successor start early (griddepcontrol.launch_dependents) may write it, as for the weights of the token-step products */
 int prl_moe_router(const void* x, int32_t x_is_f32, const void* Wr, int32_t w_is_f32, const float* bias, int32_t n, int32_t W, int32_t experts,
                    int32_t top, int32_t softmax_weights, int32_t* sel, float* wsel, int32_t* perm, int32_t* meta,
                    int32_t* tiles, prl_stream_t stream);
@@ -805,7 +807,8 @@ int prl_moe_gemm_tc(const void* A_bf16, int64_t rows_cap, const void* W_bf16, in
                     const int32_t* perm, const int32_t* meta, const int32_t* tiles, const float* wsel, int32_t act, void* out,
                     int64_t ldc, prl_stream_t stream);
 /* prl_moe_gemm with out[s] = act(product) * wsel[pair] written in sorted order in A's type (the second product's operand);
- * act 1: relu(.)^2, 2: gelu (error function) */
+ * act 1: relu(.)^2, 2: gelu (error function).  The engine runs prl_moe_mlp_act; this and prl_moe_gemm are its products
+ * one at a time */
 int prl_moe_gemm_act(const void* A, int32_t a_is_f32, int64_t lda, int32_t a_mod, const void* W, int32_t w_is_f32,
                      int64_t expert_stride, int64_t ldw, const int32_t* perm, const int32_t* meta, const int32_t* tiles,
                      int64_t max_tiles, int64_t N, int64_t K, int32_t act, const float* wsel, void* out, int64_t ld_out,

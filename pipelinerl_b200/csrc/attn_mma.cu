@@ -485,7 +485,7 @@ int launch_mma_decode(const void* q, const void* kp, const void* vp, const int32
   const size_t qs = (size_t)kDecHeads * (dim + kPadH) * sizeof(bf16);
   const size_t set = (size_t)kDecWarps * kDecKeys * (dim + DV + 2 * kPadH) * sizeof(bf16);      // one buffer of every warp
   // the CTAs that one SM gets share 224 KB (1 KB of each is the system's): more buffers than that would cost a wave
-  const int64_t per_sm = ((int64_t)G * groups * n_seg + 147) / 148;
+  const int64_t per_sm = ((int64_t)G * groups * n_seg + num_sms() - 1) / num_sms();
   int bufs = 2;
   while (bufs < kDecMaxBufs && (int64_t)(qs + (bufs + 1) * set + 1024) * per_sm <= 224 * 1024) ++bufs;
   const size_t tiles = qs + bufs * set;

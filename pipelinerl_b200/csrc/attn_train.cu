@@ -20,7 +20,7 @@
 //   * attn_bwd_dq_kernel    (Q stationary): the forward's structure (a query tile per CTA, 128 keys per step) with
 //     dP = dO V^T  as a third MMA and  dQ += dS K  in place of P V (K read as stored, MN-major).  TMEM: S double-buffered + dP + dQ.
 // Both: warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner (the WHOLE warp runs converged and elects one lane per batch of
-// UMMAs: issued from `if (lane == 0)` every UMMA costs ~180 cycles of R2UR + ELECT waterfall, tc_ptx.cuh: elect_one), the other
+// UMMAs: issued from `if (lane == 0)` every UMMA takes ~180 cycles to issue, tc_ptx.cuh: elect_one), the other
 // warps = softmax: 8 in lock-step in generations 1-3, 16 that never meet in generation 4 (the default; further down).
 // All four generations produce the same bits (generation 4 where its dK / dV kernel takes one CTA per key tile, see dkdv_split).
 //

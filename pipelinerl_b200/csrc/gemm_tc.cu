@@ -107,9 +107,8 @@ constexpr int kBlockM = 128;  // output features per CTA (UMMA M)
 constexpr int kBlockK = 64;   // bf16 elements per stage row = 128 B = one swizzle atom
 constexpr int kUmmaK = 16;
 constexpr int kThreads = 192;
-constexpr int kSMs = 148;
-static int g_smem_budget = 100 * 1024;
-static int g_tiled_weights = 0;  // weights stored as contiguous [N/128][K/64][128][64] tiles  // per-CTA tile ring; <= 100 KB lets two CTAs share an SM
+static int g_smem_budget = 100 * 1024;   // per-CTA tile ring; <= 100 KB lets two CTAs share an SM
+static int g_tiled_weights = 0;          // weights stored as contiguous [N/128][K/64][128][64] tiles
 
 struct HeadPart { float m, s, u, key, z; int idx; };  // per (vocab tile, token): online-softmax state + best sample
 
@@ -141,7 +140,7 @@ struct GemmParams {
   // two products in one accumulation (split_k, no lo part): k-blocks >= dual_kb are k-blocks (kb - dual_kb) of a second
   // weight (the map in the lo weight's place) and a second activation.  0 = off
   int dual_kb;
-  // output features per CTA: kBlockM, or fewer (a multiple of 32) for a plain product of too few tiles; see launch_gemm
+  // output features per CTA: kBlockM, or fewer (a multiple of 32) for a plain product of too few tiles; see gemm_splitk_impl
   int tile_rows;
 };
 
@@ -184,7 +183,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   const int n_kb = kb_end - kb_begin;
 
   // Both issuing warps run CONVERGED and elect one lane around each batch of instructions: from inside `if (lane == 0)` every UMMA and
-  // TMA pays an operand waterfall of ~180 cycles (tc_ptx.cuh, elect_one).  A k-block of four UMMAs then took 0.36 us whatever the tile,
+  // TMA takes ~180 cycles to issue (tc_ptx.cuh, elect_one).  A k-block of four UMMAs then took 0.36 us whatever the tile,
   // twice what its 16 KB of weights take from HBM on one CTA per SM: 32 x 9232 x 2048 14.9 -> 12.9 us, 4 x 8192 x 1024 by two 5.2 -> 5.0,
   // 64 x 152064 x 3584 193 -> 188.
   // For the same reason their loops divide nothing and look nothing up: a k-block's stage, parity and coordinates follow from the last one's
@@ -773,7 +772,7 @@ static int gemm_splitk_impl(const void* W, const void* W_lo, const void* X, int6
   // that every SM reads weights: 32 x 9232 x 2048 11.1 -> 10.0 us (5.8 at the copy rate), 64 x 9232 x 2048 13.8 -> 11.8, 4 x 4640 x 1024
   // 5.3 -> 4.5.  Each result is the same sum in the same order.
   const int64_t tiles = (N + kBlockM - 1) / kBlockM;
-  if (split_k == 1 && nt <= 64 && !W_lo && !peer_partials && !p.tiled && tiles <= kSMs / 2) p.tile_rows = tiles <= kSMs / 4 ? 32 : 64;
+  if (split_k == 1 && nt <= 64 && !W_lo && !peer_partials && !p.tiled && tiles <= num_sms() / 2) p.tile_rows = tiles <= num_sms() / 4 ? 32 : 64;
   int rc = p.tile_rows < kBlockM ? make_tmap_2d_bf16(&tw, W, (uint64_t)K, (uint64_t)N, (uint64_t)K * 2, kBlockK, (uint32_t)p.tile_rows)
                                  : make_weight_tmap(&tw, W, N, K, p.tiled);
   if (rc) return rc;

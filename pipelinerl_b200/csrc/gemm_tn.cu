@@ -249,7 +249,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
   if (warp == 0) {
     // ===== TMA producer (both CTAs) =====
     // Both issuing warps run CONVERGED and elect one lane around each batch of instructions: from inside `if (lane == 0)`
-    // every UMMA / TMA pays an operand waterfall of ~180 cycles (tc_ptx.cuh, elect_one), more than the 128 cycles of a
+    // every UMMA / TMA takes ~180 cycles to issue (tc_ptx.cuh, elect_one), more than the 128 cycles of a
     // 256 x 256 x 16 UMMA -- the main loop then took ~700 cycles per k-block whatever the tile's width.
     int it = 0;
     for (int t = cluster; t < total_tiles; t += n_clusters) {

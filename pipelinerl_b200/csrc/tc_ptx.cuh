@@ -110,10 +110,9 @@ __device__ __forceinline__ void tc_fence_after_sync() {
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-// One lane of a CONVERGED warp.  tcgen05.mma / commit take their operands from uniform registers: issued from inside an
-// `if (lane == 0)` region the compiler cannot prove the operands warp-uniform and wraps every UMMA in a
-// R2UR + ELECT "waterfall" loop (~180 cycles per instruction, measured with prl_debug_mma_bench) -- more than the 64 cycles
-// a 128 x 128 x 16 UMMA occupies the tensor core.  The MMA warp therefore runs its whole loop converged, computes the
+// One lane of a CONVERGED warp.  From inside an `if (lane == 0)` region every UMMA, commit and TMA takes about 180 cycles to issue
+// (measured with prl_debug_mma_bench), more than the 64 cycles a 128 x 128 x 16 UMMA occupies the tensor core; a warp that runs
+// converged, with operands that are the same in all its lanes, does not pay that.  The MMA warp therefore runs its whole loop converged, computes the
 // descriptors on all lanes (uniform values), and elects one lane around each instruction only.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;

@@ -250,7 +250,7 @@ def test_varlen_backward_keeps_its_bits_with_cold_row_statistics(cuda_device, ge
 @pytest.mark.parametrize("n_q,n_kv,lens", [(14, 2, [1, 700, 0, 18, 19, 300]), (4, 4, [0, 128, 129, 1, 0]), (5, 1, [3] * 31 + [40, 0, 26, 1, 77] + [2] * 40),
                                            (8, 2, [64])])
 def test_listed_tiles_equal_each_sample_alone(cuda_device, n_q, n_kv, lens):
-    """Forward and dQ launch the tiles that are there, found in a list of the samples (more than one sample): the bits of each sample by
+    """Forward and dQ launch the tiles that are there, found in a list of the samples (where that pays): the bits of each sample by
     itself, for samples of no tokens, of one tile exactly and one more, and for more samples than a warp looks at together."""
     from pipelinerl_b200 import _lib
     lib, st, g = _lib.load(), _lib.stream_ptr(), torch.Generator(device="cuda").manual_seed(sum(lens))
