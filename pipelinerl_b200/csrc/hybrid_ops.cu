@@ -1630,9 +1630,10 @@ extern "C" int prl_attn_front(const float* P, int64_t ldp, int32_t off_q, int32_
   // SM between one and two rows per SM, and whose rounds over many heads of few rows are shorter.  attn_front_kernel -> this one, us:
   // 24 heads of 128: 32 rows 3.8 -> 3.1, 1024 rows 13.2 -> 9.0, 2500 rows 28.4 -> 17.0 (200 rows 4.1, 3.9; of 64: 3.3, 3.5); 48 heads of 128:
   // 32 rows 4.3, 4.9; 450 rows 8.6, 9.9; 1024 rows 15.3 -> 14.7, 2500 rows 46.1 -> 40.6; 80 heads: 32 rows 5.5, 6.4; 2500 rows 71.9, 79.6.
+  // Channels that do not turn are a second loop there: 36 heads of 128, 64 turned: 32 rows 4.8 -> 4.5, 450 rows 9.2 -> 8.3, 593 rows 12.3 -> 8.4.
   int w = 0;
   if (heads <= 32) w = n <= sms ? (heads < 2 ? 2 : heads) : n > 2 * sms ? (heads < 2 ? 2 : heads < 8 ? heads : 8) : 0;
-  else if (heads <= 64) w = n <= sms && rot < dim ? 32 : n > 8 * sms ? 8 : n > 4 * sms ? 12 : 0;
+  else if (heads <= 64) w = n <= sms && rot < dim ? 32 : n > 8 * sms ? 8 : n > 4 * sms ? 12 : n > 2 * sms && rot < dim && heads <= 40 ? 8 : 0;
   if (dim % 32 == 0 && dim <= 128 && vdim % 32 == 0 && vdim <= 128 && rot % 64 == 0 && w) {     // rot / 2 <= 32 * w
 #define PRL_AF(T, HEADS)                                                                                                               \
   PRL_CUDA(launch_pdl((attn_front_lanes_kernel<T, HEADS>), dim3(n), dim3(32 * w), (size_t)0, (cudaStream_t)st, P, ldp, off_q, off_k, off_v, \

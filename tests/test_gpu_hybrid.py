@@ -478,7 +478,7 @@ def test_attention_front_end_rows(cuda_device, n, H, G, dim, vdim, rot, norms):
 
 
 @pytest.mark.parametrize("n,H,G,dim,vdim,rot", [(148, 30, 1, 64, 64, 64), (149, 16, 4, 128, 128, 64), (297, 11, 2, 32, 64, 0), (40, 40, 8, 96, 96, 64), (148, 31, 1, 128, 128, 64),
-                                                (593, 28, 4, 128, 128, 128), (600, 60, 2, 64, 96, 64), (600, 64, 1, 32, 32, 0)])
+                                                (301, 28, 4, 64, 64, 0), (593, 28, 4, 128, 128, 128), (600, 60, 2, 64, 96, 64), (600, 64, 1, 32, 32, 0)])
 def test_attention_front_end_of_every_schedule(cuda_device, n, H, G, dim, vdim, rot):
     """A warp per head, heads in turn, the next head on its way, and the kernel for any width between them: the lines lie at one, two and
     four rows per SM (148), 32 and 64 heads."""
