@@ -850,9 +850,9 @@ static int moe_router_impl(const void* x, int32_t x_is_f32, const void* Wr, int3
   // each row (six fit): rows that fill the SMs anyway, whose waves those fit better, and few experts, which leave warps of the former idle.
   // Rows and type as on the lines; us, block per row / rows sharing one, with the grouping behind it, router of E outputs:
   // 2048 channels bf16, E = 16: 149 rows 11.7 / 7.8, 296 12.7 / 8.7, 592 10.8 / 11.4, 850 12.7 / 15.1, 1024 16.8 / 14.5, 4096 40.9 / 49.0;
-  // E = 128: 149 rows 34 / 26, 592 43 / 40, 593 54 / 64, 1024 83 / 67, 4096 233 / 254; fp32: E = 16: 593 rows 16.6 / 14.0, 4096 72 / 46;
+  // E = 128: 149 rows 34 / 26, 400 37 / 39, 592 43 / 40, 593 54 / 64, 1024 83 / 67, 4096 233 / 254; fp32: E = 16: 593 rows 16.6 / 14.0, 4096 72 / 46;
   // E = 8: 593 rows 9.3 / 11.3, 850 10.2 / 11.5, 1024 15.3 / 11.6.
-  const bool alone = n <= 2 * sms ? false : n <= 4 * sms ? !x_is_f32 && outputs < 128 : n <= 6 * sms ? !x_is_f32 || outputs <= 8
+  const bool alone = n <= 2 * sms ? false : n <= 4 * sms ? !x_is_f32 && (outputs < 128 || n <= 3 * sms) : n <= 6 * sms ? !x_is_f32 || outputs <= 8
                    : n <= 8 * sms ? !x_is_f32 && outputs <= 8 : !x_is_f32;
   int rows = alone ? 0 : n <= sms ? 1 : n <= 2 * sms ? 2 : n <= 4 * sms ? 4 : 8;
   if (rows == 8 && 8 * per_row > 48 * 1024) rows = 4;

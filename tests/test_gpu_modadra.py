@@ -344,10 +344,10 @@ def test_router_rows_equal_the_staged_router(cuda_device, dtype, n, W, experts, 
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("n,W,experts,groups,keep,top", [(149, 264, 16, 4, 2, 3), (297, 136, 128, 8, 4, 8), (450, 1032, 8, 1, 1, 2), (600, 136, 8, 1, 1, 2), (889, 72, 16, 8, 6, 4),
+@pytest.mark.parametrize("n,W,experts,groups,keep,top", [(149, 264, 16, 4, 2, 3), (297, 136, 128, 8, 4, 8), (450, 136, 128, 8, 4, 8), (450, 1032, 8, 1, 1, 2), (600, 136, 8, 1, 1, 2), (889, 72, 16, 8, 6, 4),
                                                          (1185, 264, 32, 4, 2, 6)])
 def test_router_of_every_schedule(cuda_device, dtype, n, W, experts, groups, keep, top):
-    """One, two, four and eight rows a block and a block per row: the lines lie at one, two, four, six and eight rows per SM (148)."""
+    """One, two, four and eight rows a block and a block per row: the lines lie at one, two, three, four, six and eight rows per SM (148)."""
     test_router_rows_equal_the_staged_router(cuda_device, dtype, n, W, experts, groups, keep, top)
 
 
