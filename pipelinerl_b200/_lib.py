@@ -241,6 +241,18 @@ _SIGNATURES = {
                                        C.c_void_p]),
     "prl_head_dlogits": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_float, C.c_void_p,
                                    C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]),
+    "prl_live_rows": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p]),
+    "prl_gather_live_rows": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64,
+                                       C.c_int64, C.c_int64, C.c_void_p]),
+    "prl_spread_rows": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]),
+    "prl_head_dlogits_rows": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_float] +
+                              [C.c_void_p] * 8 + [C.c_int64, C.c_void_p]),
+    "prl_head_dlogits_kept": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_float] + [C.c_void_p] * 8),
+    "prl_head_logprob_keep": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_float] +
+                              [C.c_void_p] * 5 + [C.c_int64, C.c_int64, C.c_void_p, C.c_size_t, C.c_void_p]),
+    "prl_gemm_ex_counted": (C.c_int, [C.c_void_p, C.c_int64, C.c_int32, C.c_void_p, C.c_int64, C.c_int32, C.c_int64, C.c_int64,
+                                      C.c_int64, C.c_void_p, C.c_int32, C.c_void_p, C.c_int64, C.c_int32, C.c_int32, C.c_float,
+                                      C.c_void_p]),
     "prl_adamw_sharded_reduce": (C.c_int, [C.POINTER(AdamwShardArgs), C.c_void_p, C.c_size_t, C.c_void_p]),
     "prl_adamw_sharded_update": (C.c_int, [C.POINTER(AdamwShardArgs), C.c_void_p, C.c_void_p]),
     "prl_adamw_workspace_bytes": (C.c_size_t, []),

@@ -27,8 +27,8 @@
 namespace prl {
 
 int head_logprob_tn(const void* W, const void* W_lo, const void* X, int64_t M, int64_t V, int64_t K, float temperature,
-                    const int64_t* targets, float* logprob_target, float* entropy, float* lse, void* workspace,
-                    cudaStream_t stream);  // gemm_tn.cu
+                    const int64_t* targets, float* logprob_target, float* entropy, float* lse, float* keep_logits, int64_t ld_keep,
+                    int64_t keep_rows, void* workspace, cudaStream_t stream);  // gemm_tn.cu
 
 // ------------------------------------------------------------------------------------
 // host: tensor maps
@@ -852,7 +852,7 @@ extern "C" int prl_head_logprob(const void* W, const void* W_lo, const void* X, 
   if (M > kBlockM && !sampled_ids && !sampled_logprobs && g_use_2cta && !g_tiled_weights) {
     // many tokens, statistics only (learner forward, reference-logprob scoring): CTA-pair kernel, token-per-thread
     // epilogue (csrc/gemm_tn.cu)
-    return head_logprob_tn(W, W_lo, X, M, V, K, temperature, targets, logprob_target, entropy, lse, workspace,
+    return head_logprob_tn(W, W_lo, X, M, V, K, temperature, targets, logprob_target, entropy, lse, nullptr, 0, 0, workspace,
                            (cudaStream_t)stream_);
   }
   const int nt = pick_ntile(M);
@@ -885,4 +885,19 @@ extern "C" int prl_head_logprob(const void* W, const void* W_lo, const void* X, 
                       sampled_logprobs));
   PRL_LAUNCH_CHECK();
   return PRL_OK;
+}
+
+// prl_head_logprob of a learner's forward that also keeps the products of the first keep_rows tokens, logits[keep_rows, ld_logits] in
+// fp32 and before the temperature, for prl_head_dlogits_kept.
+extern "C" int prl_head_logprob_keep(const void* W, const void* W_lo, const void* X, int64_t M, int64_t V, int64_t K, float temperature,
+                                     const int64_t* targets, float* logprob_target, float* entropy, float* lse, float* logits,
+                                     int64_t ld_logits, int64_t keep_rows, void* workspace, size_t workspace_bytes, prl_stream_t stream_) {
+  PRL_CHECK_ARG(W && X && targets && logits && workspace, "prl_head_logprob_keep: NULL argument");
+  PRL_CHECK_ARG(M >= 1 && V >= 1 && K >= 8 && K % 8 == 0, "prl_head_logprob_keep: need M,V >= 1 and K %% 8 == 0");
+  PRL_CHECK_ARG(temperature > 0.f, "prl_head_logprob_keep: temperature must be > 0");
+  PRL_CHECK_ARG(ld_logits >= V && keep_rows >= 1 && keep_rows <= M, "prl_head_logprob_keep: bad logits buffer (ld=%lld rows=%lld)",
+                (long long)ld_logits, (long long)keep_rows);
+  PRL_CHECK_ARG(workspace_bytes >= prl_head_workspace_bytes(M, V), "prl_head_logprob_keep: workspace too small");
+  return head_logprob_tn(W, W_lo, X, M, V, K, temperature, targets, logprob_target, entropy, lse, logits, ld_logits, keep_rows, workspace,
+                         (cudaStream_t)stream_);
 }

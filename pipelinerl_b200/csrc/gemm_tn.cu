@@ -81,6 +81,9 @@ struct TnParams {
   // head epilogue (kHead): logits never leave TMEM/registers
   const int64_t* targets;  // [M] or NULL
   float4* head_part;       // [n_tiles, M]: (max, sum exp, sum exp*z, target logit or -inf) of one 256-column vocabulary tile
+  float* keep_logits;      // [keep_rows, ld_keep] or NULL: the products of the first rows, kept for the backward
+  int64_t ld_keep;
+  int64_t keep_rows;
   // head BACKWARD epilogue (kHead, dz != NULL): the logits tile is turned into d loss / d logits in registers and only its
   // bf16 value reaches HBM -- dz[row, col] = inv_T * (g_lp * ([col == target] - p) - g_ent * p * (log p + H))
   __nv_bfloat16* dz;       // [M, ld_dz]
@@ -94,6 +97,10 @@ struct TnParams {
   const __nv_bfloat16* bwd_gu;   // [M, ld_gu] gate | up of the forward
   __nv_bfloat16* dgu;            // [M, ld_gu] d gate | d up
   int64_t ld_gu;
+  // rows counted on the device (d_count != NULL, plain and d-logits epilogues): the first *d_count rows of A and C, or of the contraction
+  // (count_is_k), are there; row r of the d-logits epilogue takes its target and statistics from row g_perm[r]
+  const int32_t* d_count;
+  int count_is_k;
 };
 
 // 0.5 z (1 + tanh(u)) = z sigmoid(2 u), u = sqrt(2 / pi) (z + 0.044715 z^3)
@@ -102,13 +109,13 @@ __device__ __forceinline__ float gelu_tanh(float z) {
 }
 
 // k-blocks of work item t: all of them, or the item's share of a split tile (items of a tile are neighbours)
-__device__ __forceinline__ void k_range(int t, const TnParams& p, int& kb0, int& kb1) {
+__device__ __forceinline__ void k_range(int t, const TnParams& p, int kblocks, int& kb0, int& kb1) {
   const int split = p.split > 1 ? p.split : 1, s = t % split;
-  kb0 = (int)((int64_t)p.kblocks * s / split);
-  kb1 = (int)((int64_t)p.kblocks * (s + 1) / split);
+  kb0 = (int)((int64_t)kblocks * s / split);
+  kb1 = (int)((int64_t)kblocks * (s + 1) / split);
 }
 
-__device__ __forceinline__ void tile_coords(int t, const TnParams& p, int& tm, int& tn) {
+__device__ __forceinline__ void tile_coords(int t, const TnParams& p, int m_tiles, int& tm, int& tn) {
   if (p.g_tiles) {
     tm = t / p.n_tiles;
     tn = t - tm * p.n_tiles;
@@ -118,7 +125,7 @@ __device__ __forceinline__ void tile_coords(int t, const TnParams& p, int& tm, i
   const int per_group = kGroupM * p.n_tiles;
   const int g = t / per_group;
   const int first_m = g * kGroupM;
-  const int rows = (p.m_tiles - first_m) < kGroupM ? (p.m_tiles - first_m) : kGroupM;
+  const int rows = (m_tiles - first_m) < kGroupM ? (m_tiles - first_m) : kGroupM;
   const int r = t - g * per_group;
   tm = first_m + r % rows;
   tn = r / rows;
@@ -166,6 +173,26 @@ __device__ __forceinline__ void store_bf16_chunk(uint32_t st, int lane, int my_r
 #pragma unroll
         for (int e = 0; e < 8; ++e)
           if (c * 8 + e < n_ok) d[e] = h[e];
+      }
+    }
+  }
+}
+// ... and its 32 x 32 fp32 chunk, written once and read after the launch: 8 lanes per row, 16 bytes each
+__device__ __forceinline__ void store_f32_chunk(uint32_t st, int lane, int my_row, float* dst, int64_t ld, int n_ok, bool vec) {
+  const int c4 = (lane & 7) * 4, sub = lane >> 3;
+#pragma unroll
+  for (int it = 0; it < 8; ++it) {
+    const int row = __shfl_sync(0xffffffffu, my_row, it * 4 + sub);
+    const uint4 u = lds16(at128(st, it * 4 + sub, lane & 7));
+    if (row >= 0) {
+      float* d = dst + (int64_t)row * ld + c4;
+      if (vec && c4 + 4 <= n_ok) {
+        __stcs(reinterpret_cast<uint4*>(d), u);
+      } else {
+        const uint32_t e4[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (c4 + e < n_ok) d[e] = __uint_as_float(e4[e]);
       }
     }
   }
@@ -244,7 +271,15 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
   pdl_wait();
-  const int total_tiles = p.g_tiles ? p.g_meta[0] * p.n_tiles : p.m_tiles * p.n_tiles * (p.split > 1 ? p.split : 1);
+  int m_tiles = p.m_tiles, kblocks = p.kblocks;
+  int64_t n_rows = p.M;
+  if (p.d_count) {
+    const int n = *p.d_count;
+    if (p.count_is_k) kblocks = (n + kBK - 1) / kBK;
+    else n_rows = n;
+    if (!p.count_is_k || n == 0) m_tiles = (n + kTile - 1) / kTile;
+  }
+  const int total_tiles = p.g_tiles ? p.g_meta[0] * p.n_tiles : m_tiles * p.n_tiles * (p.split > 1 ? p.split : 1);
 
   if (warp == 0) {
     // ===== TMA producer (both CTAs) =====
@@ -254,9 +289,9 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     int it = 0;
     for (int t = cluster; t < total_tiles; t += n_clusters) {
       int tm, tn;
-      tile_coords(t, p, tm, tn);
+      tile_coords(t, p, m_tiles, tm, tn);
       int kb0, kb1;
-      k_range(t, p, kb0, kb1);
+      k_range(t, p, kblocks, kb0, kb1);
       const int half_n = p.tile_n >> 1;
       const int a_row = ptx::warp_uniform((p.g_tiles ? p.g_tiles[3 * tm + 1] : tm * kTile) + (int)rank * kHalf);
       const int b_row = ptx::warp_uniform(p.g_tiles ? p.g_tiles[3 * tm] * (int)p.N + tn * kTile + (int)rank * kHalf
@@ -306,7 +341,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
         ptx::tc_fence_after_sync();
         const uint32_t d_tmem = tm0 + (uint32_t)(acc * kTile);
         int kb0, kb1;
-        k_range(t, p, kb0, kb1);
+        k_range(t, p, kblocks, kb0, kb1);
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (uint32_t)((it / kStages) & 1);
@@ -338,13 +373,13 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     int local = 0;
     for (int t = cluster; t < total_tiles; t += n_clusters, ++local) {
       int tm, tn;
-      tile_coords(t, p, tm, tn);
+      tile_coords(t, p, m_tiles, tm, tn);
       const int acc = local & 1;
       const uint32_t acc_ph = (uint32_t)((local >> 1) & 1);
       const uint32_t acc_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kTile);
       int64_t row = (int64_t)tm * kTile + (int64_t)rank * kHalf + q * 32 + lane;
       const int64_t col0 = (int64_t)tn * p.tile_n;
-      bool row_ok = row < p.M;
+      bool row_ok = row < n_rows;
       float row_w = 0.f;
       if (!kHead && !kAcc && p.g_tiles) {
         const int local_row = (int)rank * kHalf + q * 32 + lane;
@@ -362,13 +397,14 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
       if constexpr (kHead) {
         // thread = one token; online softmax statistics over this tile's 256 vocabulary columns, all thread-local
         constexpr float kLog2e = 1.4426950408889634f;
-        const int64_t tgt = (p.targets && row_ok) ? p.targets[row] : -1;
+        const int64_t src = p.g_perm && row_ok ? p.g_perm[row] : row;
+        const int64_t tgt = (p.targets && row_ok) ? p.targets[src] : -1;
         if (p.dz != nullptr) {
           // ---- backward: logits -> d logits (same formula as tail_bwd_kernel, logprob_tail.cu), written as bf16 ----
-          const float lse = row_ok ? p.bwd_lse[row] : 0.f;
-          const float gl = (p.bwd_g_lp && row_ok) ? p.bwd_g_lp[row] : 0.f;
-          const float ge = (p.bwd_g_ent && row_ok) ? p.bwd_g_ent[row] : 0.f;
-          const float H = (p.bwd_g_ent && p.bwd_ent && row_ok) ? p.bwd_ent[row] : 0.f;
+          const float lse = row_ok ? p.bwd_lse[src] : 0.f;
+          const float gl = (p.bwd_g_lp && row_ok) ? p.bwd_g_lp[src] : 0.f;
+          const float ge = (p.bwd_g_ent && row_ok) ? p.bwd_g_ent[src] : 0.f;
+          const float H = (p.bwd_g_ent && p.bwd_ent && row_ok) ? p.bwd_ent[src] : 0.f;
 #pragma unroll 1
           for (int c0 = 0; c0 < kTile; c0 += 32) {
             if (col0 + c0 >= p.N) break;
@@ -399,6 +435,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
           }
         } else {
         float m = -INFINITY, ssum = 0.f, usum = 0.f, zt = -INFINITY;
+        const bool keep = p.keep_logits != nullptr && (int64_t)tm * kTile < p.keep_rows;
+        const int keep_row = row_ok && row < p.keep_rows ? (int)row : -1;
 #pragma unroll 1
         for (int c0 = 0; c0 < kTile; c0 += 32) {
           if (col0 + c0 >= p.N) break;
@@ -407,6 +445,13 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
           ptx::tmem_ld_wait();
           const int64_t col = col0 + c0;
           const int n_ok = (int)((p.N - col) < 32 ? (p.N - col) : 32);
+          if (keep) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) sts16(at128(st, lane, c), r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
+            __syncwarp();
+            store_f32_chunk(st, lane, keep_row, p.keep_logits + col, p.ld_keep, n_ok, aligned16(p.keep_logits, p.ld_keep * 4));
+            __syncwarp();
+          }
           float z[32];
           float cm = -INFINITY;
 #pragma unroll
@@ -742,10 +787,9 @@ extern "C" int prl_gemm_tn(const void* A, int64_t lda, const void* B, int64_t ld
   return prl_gemm_ex(A, lda, 0, B, ldb, 0, M, N, K, C, ldc, c_is_f32, accumulate, bias, residual, ldr, alpha, stream_);
 }
 
-extern "C" int prl_gemm_ex(const void* A, int64_t lda, int32_t a_mn_major, const void* B, int64_t ldb,
-                           int32_t b_mn_major, int64_t M, int64_t N, int64_t K, void* C, int64_t ldc, int32_t c_is_f32,
-                           int32_t accumulate, const void* bias, const void* residual, int64_t ldr, float alpha,
-                           prl_stream_t stream_) {
+static int gemm_ex_impl(const void* A, int64_t lda, int32_t a_mn_major, const void* B, int64_t ldb, int32_t b_mn_major, int64_t M,
+                        int64_t N, int64_t K, void* C, int64_t ldc, int32_t c_is_f32, int32_t accumulate, const void* bias,
+                        const void* residual, int64_t ldr, float alpha, const int32_t* d_count, int count_is_k, prl_stream_t stream_) {
   PRL_CHECK_ARG(A && B && C, "prl_gemm_tn: NULL argument");
   PRL_CHECK_ARG(M >= 1 && N >= 1 && K >= 8, "prl_gemm_tn: need M, N >= 1 and K >= 8 (M=%lld N=%lld K=%lld)", (long long)M,
                 (long long)N, (long long)K);
@@ -770,6 +814,7 @@ extern "C" int prl_gemm_ex(const void* A, int64_t lda, int32_t a_mn_major, const
   p.alpha = alpha;
   p.a_mn = a_mn_major ? 1 : 0;
   p.b_mn = b_mn_major ? 1 : 0;
+  p.d_count = d_count; p.count_is_k = count_is_k;
   CUtensorMap ta, tb;
   int rc = a_mn_major ? make_tmap_2d_bf16(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, 64, kBK)
                       : make_tmap_2d_bf16(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2, kBK, kHalf);
@@ -787,6 +832,25 @@ extern "C" int prl_gemm_ex(const void* A, int64_t lda, int32_t a_mn_major, const
   PRL_CUDA(launch_pdl(kernel, dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<false>), (size_t)smem, (cudaStream_t)stream_, ta, tb, ta, tb, p));
   PRL_LAUNCH_CHECK();
   return PRL_OK;
+}
+
+extern "C" int prl_gemm_ex(const void* A, int64_t lda, int32_t a_mn_major, const void* B, int64_t ldb,
+                           int32_t b_mn_major, int64_t M, int64_t N, int64_t K, void* C, int64_t ldc, int32_t c_is_f32,
+                           int32_t accumulate, const void* bias, const void* residual, int64_t ldr, float alpha,
+                           prl_stream_t stream_) {
+  return gemm_ex_impl(A, lda, a_mn_major, B, ldb, b_mn_major, M, N, K, C, ldc, c_is_f32, accumulate, bias, residual, ldr, alpha, nullptr, 0,
+                      stream_);
+}
+
+// prl_gemm_ex over as many rows as *count says (device memory, at most M, or K with count_is_k): tiles and k-blocks beyond it are not
+// walked.  A counted contraction reads whole k-blocks of 64: the rows up to the next multiple of 64 (or K) hold zeros in both operands.
+extern "C" int prl_gemm_ex_counted(const void* A, int64_t lda, int32_t a_mn_major, const void* B, int64_t ldb, int32_t b_mn_major,
+                                   int64_t M, int64_t N, int64_t K, const int32_t* count, int32_t count_is_k, void* C, int64_t ldc,
+                                   int32_t c_is_f32, int32_t accumulate, float alpha, prl_stream_t stream_) {
+  PRL_CHECK_ARG(count != nullptr, "prl_gemm_ex_counted: NULL count");
+  PRL_CHECK_ARG(!count_is_k || accumulate, "prl_gemm_ex_counted: a counted contraction adds to C (no rows: nothing is written)");
+  return gemm_ex_impl(A, lda, a_mn_major, B, ldb, b_mn_major, M, N, K, C, ldc, c_is_f32, accumulate, nullptr, nullptr, 0, alpha, count,
+                      count_is_k ? 1 : 0, stream_);
 }
 
 // Two products in one accumulation, C[M, N] (fp32) = A1[M, K1] * B1[N, K1]^T + A2[M, K2] * B2[N, K2]^T: the output projections of two
@@ -980,8 +1044,8 @@ namespace prl {
 // fused output head for many tokens (M > 128): logprob of the target, entropy and logsumexp of softmax(X W^T / T)
 // without storing logits.  Called by prl_head_logprob (gemm_tc.cu).  workspace: ceil(V/256) * M float4.
 int head_logprob_tn(const void* W, const void* W_lo, const void* X, int64_t M, int64_t V, int64_t K, float temperature,
-                    const int64_t* targets, float* logprob_target, float* entropy, float* lse, void* workspace,
-                    cudaStream_t stream) {
+                    const int64_t* targets, float* logprob_target, float* entropy, float* lse, float* keep_logits, int64_t ld_keep,
+                    int64_t keep_rows, void* workspace, cudaStream_t stream) {
   TnParams p = {};
   p.tile_n = kTile;
   p.M = M; p.N = V; p.K = K;
@@ -993,6 +1057,7 @@ int head_logprob_tn(const void* W, const void* W_lo, const void* X, int64_t M, i
   p.alpha = 1.f / temperature;
   p.targets = targets;
   p.head_part = (float4*)workspace;
+  p.keep_logits = keep_logits; p.ld_keep = ld_keep; p.keep_rows = keep_rows;
   CUtensorMap ta, tb, tb2;
   int rc = make_tmap_2d_bf16(&ta, X, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, kBK, kHalf);
   if (rc) return rc;
@@ -1020,11 +1085,13 @@ int head_logprob_tn(const void* W, const void* W_lo, const void* X, int64_t M, i
 //   dz = inv_T * (g_lp * (onehot(target) - p) - g_ent * p * (log p + H)),   p = exp(z * inv_T - lse)
 // in registers (reference: autograd through logits/T -> log_softmax / entropy, rl/__init__.py:207-233).  dz is the operand of
 // the dX and dW GEMMs that follow; fp32 logits, fp32 d logits and the cast pass never exist.
-extern "C" int prl_head_dlogits(const void* W, const void* W_lo, const void* X, int64_t M, int64_t V, int64_t K,
-                                float temperature, const int64_t* targets, const float* lse, const float* entropy,
-                                const float* g_logprobs, const float* g_entropy, void* dz_bf16, int64_t ld_dz,
-                                prl_stream_t stream_) {
+// Row c of X and dz is then token rows[c] of targets, statistics and gradients (c < *count), or, without rows, token c.
+extern "C" int prl_head_dlogits_rows(const void* W, const void* W_lo, const void* X, int64_t M, int64_t V, int64_t K,
+                                     float temperature, const int64_t* targets, const float* lse, const float* entropy,
+                                     const float* g_logprobs, const float* g_entropy, const int32_t* rows, const int32_t* count,
+                                     void* dz_bf16, int64_t ld_dz, prl_stream_t stream_) {
   using namespace prl;
+  PRL_CHECK_ARG(!rows == !count, "prl_head_dlogits: rows and their count come together");
   PRL_CHECK_ARG(W && X && targets && lse && dz_bf16, "prl_head_dlogits: NULL argument");
   PRL_CHECK_ARG(M >= 1 && V >= 1 && K >= 8 && K % 8 == 0 && ld_dz >= V && ld_dz % 8 == 0 && temperature > 0.f,
                 "prl_head_dlogits: bad shape (M=%lld V=%lld K=%lld ld_dz=%lld)", (long long)M, (long long)V, (long long)K,
@@ -1042,6 +1109,7 @@ extern "C" int prl_head_dlogits(const void* W, const void* W_lo, const void* X, 
   p.targets = targets;
   p.dz = (__nv_bfloat16*)dz_bf16; p.ld_dz = ld_dz;
   p.bwd_lse = lse; p.bwd_ent = entropy; p.bwd_g_lp = g_logprobs; p.bwd_g_ent = g_entropy;
+  p.g_perm = rows; p.d_count = count;
   CUtensorMap ta, tb, tb2;
   int rc = make_tmap_2d_bf16(&ta, X, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, kBK, kHalf);
   if (rc) return rc;
@@ -1058,6 +1126,13 @@ extern "C" int prl_head_dlogits(const void* W, const void* W_lo, const void* X, 
   PRL_CUDA(launch_pdl(gemm_tn_kernel<true>, dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<true>), (size_t)smem, (cudaStream_t)stream_, ta, tb, ta, tb2, p));
   PRL_LAUNCH_CHECK();
   return PRL_OK;
+}
+
+extern "C" int prl_head_dlogits(const void* W, const void* W_lo, const void* X, int64_t M, int64_t V, int64_t K, float temperature,
+                                const int64_t* targets, const float* lse, const float* entropy, const float* g_logprobs,
+                                const float* g_entropy, void* dz_bf16, int64_t ld_dz, prl_stream_t stream_) {
+  return prl_head_dlogits_rows(W, W_lo, X, M, V, K, temperature, targets, lse, entropy, g_logprobs, g_entropy, nullptr, nullptr, dz_bf16,
+                               ld_dz, stream_);
 }
 
 extern "C" int prl_transpose_bf16(const void* in, int64_t rows, int64_t cols, int64_t ld_in, void* out, int64_t ld_out,

@@ -149,6 +149,155 @@ __global__ void __launch_bounds__(kThreads) tail_bwd_kernel(const float* __restr
   for (int64_t i = v4 * 4 + threadIdx.x; i < V; i += kThreads) d[i] = one(z[i], i);
 }
 
+// ---- head backward over the rows that have a gradient (the tokens of prompts have none: their labels are masked) -------------------
+// Order of the `count` rows with a gradient: slot c holds row rows[c], row r's slot is place[r], or -1.  A row below `count` keeps its own
+// slot and the others fill the slots of rows without one, in turn: d logits of a row can then take the place of the logits it is made
+// from.  One block: 2048 rows of two columns are 16 KB.
+__global__ void __launch_bounds__(1024) live_rows_kernel(const float* __restrict__ g_lp, const float* __restrict__ g_ent, int n,
+                                                         int32_t* rows, int32_t* place, int32_t* open, int32_t* __restrict__ count) {
+  __shared__ int s_warp[2][32];
+  __shared__ int s_total;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) s_total = 0;
+  __syncthreads();
+  int mine = 0;
+  for (int r = threadIdx.x; r < n; r += 1024) {
+    // a gradient that is not a number is one, too
+    const bool live = (g_lp && !(g_lp[r] == 0.f)) || (g_ent && !(g_ent[r] == 0.f));
+    place[r] = live ? r : -1;
+    mine += live;
+  }
+  atomicAdd(&s_total, mine);
+  __syncthreads();
+  const int total = s_total;
+  int n_open = 0, n_moved = 0;             // slots without a row, rows without a slot: as many of either
+  for (int r0 = 0; r0 < n; r0 += 1024) {
+    const int r = r0 + (int)threadIdx.x;
+    const bool live = r < n && place[r] >= 0, is_open = r < total && !live, moved = live && r >= total;
+    const unsigned mo = __ballot_sync(0xffffffffu, is_open), mm = __ballot_sync(0xffffffffu, moved);
+    if (lane == 0) { s_warp[0][warp] = __popc(mo); s_warp[1][warp] = __popc(mm); }
+    __syncthreads();
+    int at_open = n_open + __popc(mo & ((1u << lane) - 1u)), at_moved = n_moved + __popc(mm & ((1u << lane) - 1u));
+    for (int w = 0; w < 32; ++w) {
+      if (w < warp) { at_open += s_warp[0][w]; at_moved += s_warp[1][w]; }
+      n_open += s_warp[0][w];
+      n_moved += s_warp[1][w];
+    }
+    if (is_open) open[at_open] = r;
+    if (moved) place[r] = n + at_moved;    // until every open slot is known
+    if (live && r < total) rows[r] = r;
+    __syncthreads();
+  }
+  for (int r = threadIdx.x; r < n; r += 1024) {
+    const int p = place[r];
+    if (p >= n) {
+      const int slot = open[p - n];
+      rows[slot] = r;
+      place[r] = slot;
+    }
+  }
+  if (threadIdx.x == 0) *count = total;
+}
+
+// xc[c] = x[rows[c]], and zeros in both operands of dW up to the k-block's end (rows count .. the next multiple of 64).
+// Rows are K channels (a multiple of 8) wide.
+__global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* __restrict__ x, const int32_t* __restrict__ rows,
+                                                          const int32_t* __restrict__ count, int64_t k8, uint4* __restrict__ xc,
+                                                          __nv_bfloat16* __restrict__ dz, int64_t dz_rows, int64_t V, int64_t ld_dz) {
+  const int c = blockIdx.x, n = *count;
+  if (c >= (n + 63) / 64 * 64) return;
+  if (c < n) {
+    const uint4* src = x + (int64_t)rows[c] * k8;
+    for (int64_t i = threadIdx.x; i < k8; i += 256) xc[c * k8 + i] = src[i];
+    return;
+  }
+  for (int64_t i = threadIdx.x; i < k8; i += 256) xc[c * k8 + i] = make_uint4(0u, 0u, 0u, 0u);
+  if (c >= dz_rows) return;
+  __nv_bfloat16* d = dz + c * ld_dz;
+  if ((reinterpret_cast<uintptr_t>(d) & 15) == 0 && (V & 7) == 0)
+    for (int64_t i = threadIdx.x; i < V / 8; i += 256) reinterpret_cast<uint4*>(d)[i] = make_uint4(0u, 0u, 0u, 0u);
+  else
+    for (int64_t i = threadIdx.x; i < V; i += 256) d[i] = __float2bfloat16_rn(0.f);
+}
+
+// out[r] = src[place[r]], or zeros
+__global__ void __launch_bounds__(256) spread_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ place, int64_t k8,
+                                                          uint4* __restrict__ out) {
+  const int64_t r = blockIdx.x;
+  const int c = place[r];
+  for (int64_t i = threadIdx.x; i < k8; i += 256) out[r * k8 + i] = c >= 0 ? src[c * k8 + i] : make_uint4(0u, 0u, 0u, 0u);
+}
+
+// d logits (bf16) of the rows with a gradient from logits that the forward kept: the formula of the head's GEMM epilogue, whose
+// products these are, so the bits of a recomputation.  They take the place of the logits, slot c = the first half of row c, so that no second buffer is
+// needed: a piece is written once all threads have read theirs, and lies in a part of the row that was read by then.
+// Reads 4 bytes and writes 2 per logit: HBM-bound.
+constexpr int kKept = 16;                  // logits per thread and piece
+__device__ __forceinline__ float4 ld_rw_f4(const float4* p) {      // not the read-only path: this launch writes there
+  float4 r;
+  asm volatile("ld.global.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p) : "memory");
+  return r;
+}
+__global__ void __launch_bounds__(kThreads) dlogits_kept_kernel(float* logits, int64_t ld, int64_t V, const int32_t* __restrict__ rows,
+                                                                const int32_t* __restrict__ count, const int64_t* __restrict__ targets,
+                                                                float inv_temp, const float* __restrict__ lse_in,
+                                                                const float* __restrict__ entropy, const float* __restrict__ g_lp,
+                                                                const float* __restrict__ g_ent) {
+  const int64_t c = blockIdx.x;
+  if (c >= *count) return;
+  const int64_t row = rows[c];
+  const float4* z = reinterpret_cast<const float4*>(logits + row * ld);
+  uint4* d = reinterpret_cast<uint4*>(logits + c * ld);
+  const float lse = lse_in[row], gl = g_lp ? g_lp[row] : 0.f, ge = g_ent ? g_ent[row] : 0.f;
+  const float H = (g_ent && entropy) ? entropy[row] : 0.f;
+  const int64_t tgt = targets[row];
+  const int64_t v8 = V / 8;
+  constexpr int kP = kKept / 8;
+  auto load = [&](int64_t i0, float4 (&x)[2 * kP]) {
+#pragma unroll
+    for (int k = 0; k < kP; ++k) {
+      const int64_t i = i0 + k * kThreads + threadIdx.x;
+      if (i < v8) { x[2 * k] = ld_rw_f4(z + 2 * i); x[2 * k + 1] = ld_rw_f4(z + 2 * i + 1); }
+    }
+  };
+  float4 next[2 * kP];
+  load(0, next);
+  for (int64_t i0 = 0; i0 < v8; i0 += kP * kThreads) {
+    float4 x[2 * kP];
+#pragma unroll
+    for (int k = 0; k < 2 * kP; ++k) x[k] = next[k];
+    load(i0 + kP * kThreads, next);
+    uint4 h[kP];
+#pragma unroll
+    for (int k = 0; k < kP; ++k) {
+      const int64_t rel = tgt - 8 * (i0 + k * kThreads + threadIdx.x);
+      const float v[8] = {x[2 * k].x, x[2 * k].y, x[2 * k].z, x[2 * k].w, x[2 * k + 1].x, x[2 * k + 1].y, x[2 * k + 1].z, x[2 * k + 1].w};
+      uint32_t u[4];
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) {
+        float o[2];
+#pragma unroll
+        for (int f = 0; f < 2; ++f) {
+          const float lp = v[e + f] * inv_temp - lse;
+          const float pr = __expf(lp);
+          float w = -gl * pr - ge * pr * (lp + H);
+          if (rel == e + f) w += gl;
+          o[f] = w * inv_temp;
+        }
+        const __nv_bfloat162 p = __floats2bfloat162_rn(o[0], o[1]);
+        u[e / 2] = *reinterpret_cast<const uint32_t*>(&p);
+      }
+      h[k] = make_uint4(u[0], u[1], u[2], u[3]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kP; ++k) {
+      const int64_t i = i0 + k * kThreads + threadIdx.x;
+      if (i < v8) d[i] = h[k];
+    }
+  }
+}
+
 }  // namespace
 }  // namespace prl
 
@@ -197,6 +346,54 @@ extern "C" int prl_logprob_rows_bwd(const float* logits, int64_t n_rows, int64_t
   tail_bwd_kernel<<<(unsigned)n_rows, kThreads, 0, (cudaStream_t)stream_>>>(
       logits, V, row_stride, n_rows, targets - 1, 1.f / temperature, lse, entropy, g_logprobs, g_entropy, dlogits,
       dlogits_stride);
+  PRL_LAUNCH_CHECK();
+  return PRL_OK;
+}
+
+// Rows of [n] gradient columns that are not zero: slot c < *count holds row rows[c], row r has slot place[r] or -1; a row below *count
+// has its own.  index: room for 3 n + 1 (rows, places, scratch, count).
+extern "C" int prl_live_rows(const float* g_logprobs, const float* g_entropy, int64_t n, int32_t* index, prl_stream_t stream_) {
+  PRL_CHECK_ARG(index && (g_logprobs || g_entropy), "prl_live_rows: NULL argument");
+  PRL_CHECK_ARG(n >= 1 && n < (1ll << 30), "prl_live_rows: bad row count %lld", (long long)n);
+  live_rows_kernel<<<1, 1024, 0, (cudaStream_t)stream_>>>(g_logprobs, g_entropy, (int)n, index, index + n, index + 2 * n, index + 3 * n);
+  PRL_LAUNCH_CHECK();
+  return PRL_OK;
+}
+
+// xc[c] = x[rows[c]] (c < *count, bf16 rows of K); xc and dz are zeroed from there up to the next multiple of 64 rows, dz to its last row
+// (dz_rows) at most.  xc has room for n rounded up to 64 rows.
+extern "C" int prl_gather_live_rows(const void* x, int64_t n, int64_t K, const int32_t* rows, const int32_t* count, void* xc, void* dz,
+                                    int64_t dz_rows, int64_t V, int64_t ld_dz, prl_stream_t stream_) {
+  PRL_CHECK_ARG(x && rows && count && xc && dz, "prl_gather_live_rows: NULL argument");
+  PRL_CHECK_ARG(n >= 1 && K >= 8 && K % 8 == 0 && V >= 1 && ld_dz >= V, "prl_gather_live_rows: bad shape");
+  PRL_CHECK_ARG((((uintptr_t)x | (uintptr_t)xc) & 15) == 0, "prl_gather_live_rows: rows must be 16-byte aligned");
+  gather_rows_kernel<<<(unsigned)((n + 63) / 64 * 64), 256, 0, (cudaStream_t)stream_>>>((const uint4*)x, rows, count, K / 8, (uint4*)xc,
+                                                                                         (__nv_bfloat16*)dz, dz_rows, V, ld_dz);
+  PRL_LAUNCH_CHECK();
+  return PRL_OK;
+}
+
+// out[r] = src[place[r]] for n bf16 rows of K, zeros where place[r] is -1
+extern "C" int prl_spread_rows(const void* src, const int32_t* place, int64_t n, int64_t K, void* out, prl_stream_t stream_) {
+  PRL_CHECK_ARG(src && place && out, "prl_spread_rows: NULL argument");
+  PRL_CHECK_ARG(n >= 1 && K >= 8 && K % 8 == 0, "prl_spread_rows: bad shape");
+  PRL_CHECK_ARG((((uintptr_t)src | (uintptr_t)out) & 15) == 0, "prl_spread_rows: rows must be 16-byte aligned");
+  spread_rows_kernel<<<(unsigned)n, 256, 0, (cudaStream_t)stream_>>>((const uint4*)src, place, K / 8, (uint4*)out);
+  PRL_LAUNCH_CHECK();
+  return PRL_OK;
+}
+
+// d loss / d logits (bf16) of row rows[c] into the first half of row c of the logits that prl_head_logprob_keep left: a [n, V] matrix of
+// row stride 2 ld_logits
+extern "C" int prl_head_dlogits_kept(float* logits, int64_t ld_logits, int64_t n, int64_t V, float temperature, const int32_t* rows,
+                                     const int32_t* count, const int64_t* targets, const float* lse, const float* entropy,
+                                     const float* g_logprobs, const float* g_entropy, prl_stream_t stream_) {
+  PRL_CHECK_ARG(logits && rows && count && targets && lse, "prl_head_dlogits_kept: NULL argument");
+  PRL_CHECK_ARG(n >= 1 && V >= 8 && V % 8 == 0 && ld_logits >= V && ld_logits % 4 == 0 && ((uintptr_t)logits & 15) == 0 && temperature > 0.f,
+                "prl_head_dlogits_kept: bad shape (rows of a multiple of 8 logits that start on 16 bytes)");
+  PRL_CHECK_ARG(!g_entropy || entropy, "prl_head_dlogits_kept: g_entropy needs the forward entropy");
+  dlogits_kept_kernel<<<(unsigned)n, kThreads, 0, (cudaStream_t)stream_>>>(logits, ld_logits, V, rows, count, targets, 1.f / temperature,
+                                                                           lse, entropy, g_logprobs, g_entropy);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }

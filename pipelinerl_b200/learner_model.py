@@ -122,9 +122,26 @@ class TorchQwen2(torch.nn.Module):
 
 class _NativeHead(torch.autograd.Function):
     """Final projection + log-softmax statistics of the native learner.  Forward: one tcgen05 GEMM whose epilogue
-    reduces logits in TMEM (prl_head_logprob).  Backward: per chunk of rows, the same GEMM again with an epilogue that turns
-    the logits tile into d logits in registers and stores it as bf16 (prl_head_dlogits), then dX = dZ W and dW += dZ^T X
-    (prl_gemm_ex, operands read as stored), the latter accumulated in fp32 in the optimizer's gradient arena."""
+    reduces logits in TMEM (prl_head_logprob) and, where memory allows, stores them for the backward.  Backward, per chunk of
+    rows: d logits in bf16, from the stored logits (prl_head_dlogits_kept) or from the same GEMM again with an epilogue that
+    turns the logits tile into d logits in registers (prl_head_dlogits_rows), then dX = dZ W and dW += dZ^T X (operands read as
+    stored), the latter accumulated in fp32 in the optimizer's gradient arena.  All of it over the rows that have a gradient:
+    the tokens of prompts have none, and their rows of d logits are zeros.
+
+    3071 tokens of 152064 outputs, 3584 channels, hi + lo weights, a third of them prompts: the second GEMM took 4.1 ms of a
+    two-layer step's 23.2; reading the stored logits takes 0.28, dX and dW of the other two thirds 4.0 instead of 6.2, and the step
+    17.8."""
+
+    @staticmethod
+    def _rows_to_keep(M: int, V: int, dev) -> int:
+        """Rows whose fp32 logits (4 V bytes each) the forward stores: at most a quarter of the memory that is free now, so that
+        what the backward allocates beside them finds its place; few rows are not worth a buffer, since the products' time is the
+        weights' way through the memory then (up to 256 rows: one row tile)."""
+        if M <= 256 or V % 8:
+            return 0
+        free = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
+        rows = min(M, free // 4 // (4 * V))
+        return rows if rows == M else rows // 256 * 256
 
     @staticmethod
     def forward(ctx, hidden, model, targets, temperature: float, chunk_rows: int):
@@ -138,11 +155,25 @@ class _NativeHead(torch.autograd.Function):
         ent, lse = torch.empty_like(lp), torch.empty_like(lp)
         ws = torch.empty(int(lib.prl_head_workspace_bytes(M, V)), dtype=torch.uint8, device=x.device)
         W_lo = model.head_lo
-        _lib.check(lib.prl_head_logprob(W.data_ptr(), W_lo.data_ptr() if W_lo is not None else None, x.data_ptr(), M, V, K,
-                                        float(temperature), tg.data_ptr(), 1, 0,
-                                        0, lp.data_ptr(), ent.data_ptr(), lse.data_ptr(), None, None, ws.data_ptr(),
-                                        ws.numel(), _lib.stream_ptr()))
+        logits = None
+        if ctx.needs_input_grad[0]:
+            kept = _NativeHead._rows_to_keep(M, V, x.device)
+            if kept:
+                try:
+                    logits = torch.empty(kept, V, dtype=torch.float32, device=x.device)
+                except torch.cuda.OutOfMemoryError:      # free memory in pieces: the backward recomputes
+                    pass
+        if logits is not None:
+            _lib.check(lib.prl_head_logprob_keep(W.data_ptr(), W_lo.data_ptr() if W_lo is not None else None, x.data_ptr(), M, V, K,
+                                                 float(temperature), tg.data_ptr(), lp.data_ptr(), ent.data_ptr(), lse.data_ptr(),
+                                                 logits.data_ptr(), V, logits.shape[0], ws.data_ptr(), ws.numel(), _lib.stream_ptr()))
+        else:
+            _lib.check(lib.prl_head_logprob(W.data_ptr(), W_lo.data_ptr() if W_lo is not None else None, x.data_ptr(), M, V, K,
+                                            float(temperature), tg.data_ptr(), 1, 0,
+                                            0, lp.data_ptr(), ent.data_ptr(), lse.data_ptr(), None, None, ws.data_ptr(),
+                                            ws.numel(), _lib.stream_ptr()))
         ctx.save_for_backward(x, tg, lse, ent)
+        ctx.logits = logits                  # for one backward: the next one over a retained graph recomputes
         ctx.model, ctx.temperature, ctx.chunk_rows = model, float(temperature), int(chunk_rows)
         return lp, ent
 
@@ -161,8 +192,8 @@ class _NativeHead(torch.autograd.Function):
         g_ent = g_ent.contiguous() if use_ent else None
         dx = torch.empty(M, K, dtype=torch.bfloat16, device=dev)
         Cn = min(ctx.chunk_rows, M)
-        # d logits of a chunk of rows, bf16, straight out of the GEMM that recomputes the logits (prl_head_dlogits): fp32
-        # logits / d logits never reach HBM (the reference's autograd keeps 608 KB of fp32 logits per token alive)
+        # recomputed rows: bf16 d logits of a chunk straight out of the GEMM (prl_head_dlogits), whose fp32 logits never reach HBM
+        # (the reference's autograd keeps 608 KB of them per token alive)
         st = _lib.stream_ptr()
         W_lo = model.head_lo
         if os.environ.get("PRL_HEAD_BWD_FUSED", "1") == "0":
@@ -184,16 +215,43 @@ class _NativeHead(torch.autograd.Function):
                 ops.gemm(dz, W, out=dx[r0:r0 + n], b_mn=True)
                 ops.wgrad(gW, dz, xs)
             return dx, None, None, None, None
-        dz_buf = torch.empty(Cn, V, dtype=torch.bfloat16, device=dev)
-        for r0 in range(0, M, Cn):
-            n = min(Cn, M - r0)
-            xs, dz = x[r0:r0 + n], dz_buf[:n]
-            _lib.check(lib.prl_head_dlogits(W.data_ptr(), W_lo.data_ptr() if W_lo is not None else None, xs.data_ptr(), n, V, K,
-                                            ctx.temperature, tg[r0:r0 + n].data_ptr(), lse[r0:r0 + n].data_ptr(),
-                                            ent[r0:r0 + n].data_ptr(), g_lp[r0:r0 + n].data_ptr(),
-                                            g_ent[r0:r0 + n].data_ptr() if use_ent else None, dz.data_ptr(), V, st))
-            ops.gemm(dz, W, out=dx[r0:r0 + n], b_mn=True)
-            ops.wgrad(gW, dz, xs)
+        logits, ctx.logits = ctx.logits, None
+        kept = 0 if logits is None else logits.shape[0]
+        wp, wlp = W.data_ptr(), W_lo.data_ptr() if W_lo is not None else None
+        # the kept rows are one chunk (d logits take their place), the others come through a buffer of their own
+        chunks = ([(0, kept)] if kept else []) + [(r0, min(r0 + Cn, M)) for r0 in range(kept, M, Cn)]
+        dz_buf = torch.empty((Cn + 63) // 64 * 64, V, dtype=torch.bfloat16, device=dev) if kept < M else None
+        most = max(r1 - r0 for r0, r1 in chunks)
+        if M > 256:
+            xc = torch.empty((most + 63) // 64 * 64, K, dtype=torch.bfloat16, device=dev)
+            dxc = torch.empty(most, K, dtype=torch.bfloat16, device=dev)
+            index = torch.empty(3 * most + 1, dtype=torch.int32, device=dev)
+        for r0, r1 in chunks:
+            n = r1 - r0
+            xs = x[r0:r1]
+            at = (tg[r0:r1].data_ptr(), lse[r0:r1].data_ptr(), ent[r0:r1].data_ptr(), g_lp[r0:r1].data_ptr(),
+                  g_ent[r0:r1].data_ptr() if use_ent else None)
+            if M <= 256:
+                dz = dz_buf[:n]
+                _lib.check(lib.prl_head_dlogits(wp, wlp, xs.data_ptr(), n, V, K, ctx.temperature, *at, dz.data_ptr(), V, st))
+                ops.gemm(dz, W, out=dx[r0:r1], b_mn=True)
+                ops.wgrad(gW, dz, xs)
+                continue
+            rows = index.data_ptr()
+            place, count = rows + 4 * n, rows + 12 * n
+            _lib.check(lib.prl_live_rows(at[3], at[4], n, rows, st))
+            if r1 <= kept:
+                dz, ld, k_rows = logits.data_ptr(), 2 * V, n
+                _lib.check(lib.prl_head_dlogits_kept(dz, V, n, V, ctx.temperature, rows, count, *at, st))
+            else:
+                dz, ld, k_rows = dz_buf.data_ptr(), V, (n + 63) // 64 * 64
+            _lib.check(lib.prl_gather_live_rows(xs.data_ptr(), n, K, rows, count, xc.data_ptr(), dz, k_rows, V, ld, st))
+            if r1 > kept:
+                _lib.check(lib.prl_head_dlogits_rows(wp, wlp, xc.data_ptr(), n, V, K, ctx.temperature, *at, rows, count, dz, V, st))
+            _lib.check(lib.prl_gemm_ex_counted(dz, ld, 0, wp, W.stride(0), 1, n, K, V, count, 0, dxc.data_ptr(), K, 0, 0, 1.0, st))
+            _lib.check(lib.prl_spread_rows(dxc.data_ptr(), place, n, K, dx[r0:r1].data_ptr(), st))
+            _lib.check(lib.prl_gemm_ex_counted(dz, ld, 1, xc.data_ptr(), K, 1, V, K, k_rows, count, 1, gW.data_ptr(), gW.stride(0), 1, 1,
+                                               1.0, st))
         return dx, None, None, None, None
 
 

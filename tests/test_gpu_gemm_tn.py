@@ -526,3 +526,56 @@ def test_grouped_products_into_unaligned_rows(cuda_device, N, ldc):
             assert (out[:, N:] == 7.0).all() and (flat[:off] == 7.0).all() and (flat[off + top * n * ld:] == 7.0).all()
             got.append(out[:, :N].clone())
         assert torch.equal(got[0], got[1]) and got[0].float().abs().max() < 100 and (got[0] != 7.0).any()
+
+
+@pytest.mark.parametrize("M,V,K,chunk,with_lo,live", [(257, 520, 64, 2048, True, "some"), (700, 1032, 256, 200, True, "some"),
+                                                       (640, 264, 72, 256, False, "all"), (300, 776, 128, 2048, True, "none"),
+                                                       (513, 2056, 128, 128, True, "one"), (130, 520, 64, 2048, False, "some")])
+def test_head_backward_of_kept_logits_and_live_rows(cuda_device, monkeypatch, M, V, K, chunk, with_lo, live):
+    """The learner's head with all, some and none of its logits kept, and gradients on all, some, one and no rows: d hidden of
+    the three ways agrees in its bits (one product, one formula; dW differs in the order of its terms), and both gradients with autograd in fp64 up to the bf16
+    rounding of d logits (2^-9 of each term) and of d hidden."""
+    import types
+    from pipelinerl_b200.learner_body import Ops
+    from pipelinerl_b200.learner_model import _NativeHead
+    dev, T = cuda_device, 0.7
+    g = torch.Generator(device=dev).manual_seed(M + V + K)
+    x = (torch.randn(M, K, generator=g, device=dev) * 0.7).to(torch.bfloat16)
+    Wf = torch.randn(V, K, generator=g, device=dev) * K ** -0.5
+    W = Wf.to(torch.bfloat16)
+    lo = (Wf - W.float()).to(torch.bfloat16) if with_lo else None
+    tg = torch.randint(0, V, (M,), generator=g, device=dev)
+    g_lp, g_ent = torch.randn(M, generator=g, device=dev), torch.randn(M, generator=g, device=dev) * 0.3
+    on = {"all": torch.ones(M, device=dev), "none": torch.zeros(M, device=dev),
+          "some": (torch.rand(M, generator=g, device=dev) < 0.6).float(), "one": (torch.arange(M, device=dev) == M // 2).float()}[live]
+    g_lp, g_ent = g_lp * on, g_ent * on
+
+    def run(kept):
+        monkeypatch.setattr(_NativeHead, "_rows_to_keep", staticmethod(lambda *a: kept if M > 256 else 0))
+        gW = torch.full((V, K), 0.25, device=dev)
+        model = types.SimpleNamespace(p=lambda n: W, head_lo=lo, body=types.SimpleNamespace(ops=Ops(), g={"lm_head.weight": gW}))
+        h = x.clone().requires_grad_()
+        lp, ent = _NativeHead.apply(h, model, tg, T, chunk)
+        obj = (lp * g_lp).sum() + (ent * g_ent).sum()
+        obj.backward(retain_graph=True)
+        first, dW = h.grad.clone(), gW.clone()
+        h.grad = None
+        obj.backward()                                     # a retained graph: nothing is kept any more
+        assert torch.equal(h.grad, first)
+        return first, dW, (gW - dW, lp, ent)
+
+    whole, part, none = run(M), run(256 if M > 256 else 0), run(0)
+    assert torch.equal(whole[0], none[0]) and torch.equal(part[0], none[0])
+    assert torch.equal(whole[2][1], none[2][1]) and torch.equal(whole[2][2], none[2][2])
+    z = x.double() @ (W.double() + (lo.double() if with_lo else 0.0)).T / T
+    ls = torch.log_softmax(z, -1)
+    p, H = ls.exp(), -(ls.exp() * ls).sum(-1, keepdim=True)
+    gl, ge = g_lp.double()[:, None], g_ent.double()[:, None]
+    dz = (gl * (torch.nn.functional.one_hot(tg, V) - p) - ge * p * (ls + H)) / T
+    Ws = W.double()
+    size = dz.abs() + (gl.abs() + ge.abs()) * p * 2.0 ** -13 / T          # fp32 exponent of a logit of up to 2^7
+    for got in (whole, part, none):
+        want = dz @ Ws
+        assert ((got[0].double() - want).abs() <= 2.0 ** -8 * (size @ Ws.abs()) + 2.0 ** -8 * want.abs() + 1e-9).all()
+        for d in (got[1].double() - 0.25, got[2][0].double()):
+            assert ((d - dz.T @ x.double()).abs() <= 2.0 ** -8 * (size.T @ x.double().abs()) + 2.0 ** -21).all()
