@@ -354,3 +354,50 @@ def test_rl_step_over_several_rows_of_logits(cuda_device):
     scale = both.logits.grad.abs().max()
     assert (model.logits.grad.float() - both.logits.grad).abs().max() <= 0.05 * scale   # 2^-8 logits: their log-probs are ~1e-2 off
     assert both.logits.grad.shape[0] > 1 and all(g.abs().max() > 0 for g in both.logits.grad)
+
+
+@pytest.mark.parametrize("T,V,policy,bonus,dtype", [(2, 3, "ppo", 0.0, "float32"), (7, 4096, "reinforce", 0.01, "float32"), (61, 1031, "gspo", 0.0, "float32"),
+                                                    (300, 1204, "ppo", 0.01, "bfloat16"), (1500, 20001, "ppo", 0.0, "float32")])
+def test_gradient_of_logits_made_ahead_of_the_backward(cuda_device, policy, T, V, bonus, dtype):
+    """d logits of rl_step against the kernels called in turn with the loss kernel's gradients: the same bits for a loss gradient of 1, also
+    again over a retained graph, and for another gradient those of the scaled columns; rows without a gradient are zeros."""
+    from pipelinerl_b200 import _lib
+    from pipelinerl_b200.finetune import rl
+    from pipelinerl_b200.finetune.types import PipelineBatchEncoding
+    dev, g = cuda_device, torch.Generator().manual_seed(T + V)
+    logits = (2 * torch.randn(1, T, V, generator=g)).to(getattr(torch, dtype)).to(dev)
+    ids = torch.randint(0, V, (1, T), generator=g)
+    labels = torch.where(torch.rand(1, T, generator=g) < 0.3, -100, ids)
+    labels[0, -1] = ids[0, -1]
+    col = lambda f: f(torch.rand(1, T, generator=g))  # noqa: E731
+    lp0 = torch.log_softmax(logits[0, :-1].float(), -1).gather(1, ids[0, 1:, None].to(dev))[:, 0].cpu()
+    old = torch.cat([torch.zeros(1), lp0])[None] + col(lambda u: 0.3 * (u - 0.5))
+    batch = PipelineBatchEncoding(
+        input_ids=ids, attention_mask=torch.ones(1, T, dtype=torch.long), labels=labels, position_ids=torch.arange(T)[None],
+        segment_ids=torch.zeros(1, T, dtype=torch.long), rewards=col(lambda u: u), advantages=col(lambda u: 2 * u - 1), ref_logprobs=old + 0.1,
+        old_logprobs=old, group_tokens=torch.full((1, T), float(T)), num_labels=torch.full((1, T), float(T)), overflow=torch.zeros(1, T),
+        seq_boundaries=torch.tensor([0, T], dtype=torch.int32), model_version=0, is_packed=True).to_device(dev)
+    cfg = rl.RLConfig(policy_loss=policy, batch_size=2, entropy_bonus=bonus, final_entropy_bonus=bonus, temperature=0.7)
+    model = LogitsModel(logits)
+
+    def grad(loss, keep=False):
+        model.logits.grad = None
+        loss.backward(retain_graph=keep)
+        return model.logits.grad.clone()
+
+    loss, stats = rl.rl_step(model, batch, 0, 10, cfg)
+    first = grad(loss, keep=True)
+    assert first.abs().max() > 0 and torch.equal(grad(loss), first)
+    held, _ = rl.rl_step(model, batch, 0, 10, cfg)
+    saved = dict(zip(("logits", "ids", "stats", "grads"), held.grad_fn.saved_tensors))
+    lib, z, d = _lib.load(), saved["logits"], torch.full((T, V), 7.0, device=dev)
+    lp, ent, lse = saved["stats"]
+    for scale in (1.0, 0.375):
+        g = saved["grads"] * scale
+        _lib.check(lib.prl_logprob_tail_bwd(z.data_ptr(), T, V, z.stride(0), saved["ids"].data_ptr(), 0.7, lse.data_ptr(), ent.data_ptr(),
+                                            g[0].data_ptr(), g[1].data_ptr(), d.data_ptr(), V, _lib.stream_ptr()))
+        assert torch.equal(grad(scale * rl.rl_step(model, batch, 0, 10, cfg)[0]), d[None].to(logits.dtype))
+    assert torch.count_nonzero(first[0, :-1][(labels[0, 1:] == -100).to(dev)]) == 0 and torch.count_nonzero(first[0, -1]) == 0
+    with torch.no_grad():
+        quiet, stats2 = rl.rl_step(model, batch, 0, 10, cfg)
+    assert not quiet.requires_grad and stats2 == stats
