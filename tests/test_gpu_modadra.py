@@ -626,6 +626,35 @@ def test_both_expert_products_in_one_call(cuda_device, dtype, act, n, W, F, expe
     assert all(torch.equal(a, b) and torch.isfinite(a).all() for a, b in zip(*got))
 
 
+@pytest.mark.parametrize("counts,N,K", [((1,), 8, 8), ((16, 0, 17), 72, 64), ((64, 33, 1, 48), 136, 328), ((5, 64) * 12, 64, 72),
+                                        ((2, 3, 9, 16) * 4, 2048, 1000)])
+def test_few_rows_per_expert_equal_many(cuda_device, counts, N, K):
+    """The grouped product of few rows per expert (tokens given) has the bits of the one of many (gathered rows): tiles of one to 64 rows, remainders
+    of its 64 features and 64 channels, more steps than its ring holds."""
+    from pipelinerl_b200 import _lib
+    lib, st, g = _lib.load(), _lib.stream_ptr(), torch.Generator(device="cuda").manual_seed(N + K)
+    i32, ptr, bf16 = dict(dtype=torch.int32, device="cuda"), lambda t: t.data_ptr(), torch.bfloat16  # noqa: E731
+    pairs, experts = sum(counts), len(counts)
+    n = min(pairs, 3 * experts)
+    x, W = torch.randn(n, K, generator=g, device="cuda").to(bf16), torch.randn(experts * N, K, generator=g, device="cuda").to(bf16)
+    perm = torch.randperm(pairs, generator=g, device="cuda").to(torch.int32)
+    starts = [sum(counts[:e]) for e in range(experts)]
+    tiles = torch.tensor([(e, starts[e], c) for e, c in enumerate(counts) if c], **i32)
+    meta, wsel = torch.tensor([tiles.shape[0], 0, 0, 0], **i32), torch.rand(pairs, generator=g, device="cuda")
+    few, many = (torch.full((pairs, N), float("nan"), device="cuda") for _ in range(2))
+    few_act, many_act = (torch.zeros(pairs, N, dtype=bf16, device="cuda") for _ in range(2))
+    rows = x[perm.long() % n].contiguous()
+    for a, mod, out, act in ((x, n, few, few_act), (rows, 0, many, many_act)):
+        table = (ptr(perm), ptr(meta), ptr(tiles), experts)
+        _lib.check(lib.prl_moe_gemm(ptr(a), 0, K, mod, ptr(W), 0, N * K, K, *table, N, K, ptr(out), N, 1, st))
+        _lib.check(lib.prl_moe_gemm_act(ptr(a), 0, K, mod, ptr(W), 0, N * K, K, *table, N, K, 2, ptr(wsel), ptr(act), N, st))
+    assert torch.equal(few, many) and torch.equal(few_act, many_act)
+    expert = torch.repeat_interleave(torch.arange(experts, device="cuda"), torch.tensor(counts, device="cuda"))
+    want = torch.einsum("sk,snk->sn", rows.double(), W.double().view(experts, N, K)[expert])
+    got = few[perm.long()].double()
+    assert ((got - want).abs() <= K * 2.0 ** -24 * torch.einsum("sk,snk->sn", rows.double().abs(), W.double().abs().view(experts, N, K)[expert])).all()
+
+
 @pytest.mark.parametrize("heads,kh,dk,dv", [(16, 8, 128, 128), (4, 2, 64, 48), (6, 2, 20, 36), (4, 4, 32, 64)])
 def test_token_step_of_many_rows_equals_few(cuda_device, heads, kh, dk, dv):
     """One value head at a time in a CTA (more than 148 CTAs) or two: the same bits, for outputs, states and convolution inputs."""
