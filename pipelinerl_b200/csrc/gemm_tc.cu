@@ -129,8 +129,8 @@ struct GemmParams {
   unsigned long long seed;
   unsigned int step;
   HeadPart* head_part;      // [n_tiles, M]
-  // SwiGLU epilogue of the token step's gate_up GEMM (split_k == 1): the CTA's 128 weight rows are 64 GATE rows
-  // [64 t, 64 t + 64) and the 64 UP rows of the same features (I rows further down), and the epilogue writes
+  // SwiGLU epilogue of the token step's gate_up GEMM (split_k == 1): the first half of the CTA's tile_rows weight rows are h = 64 or 32 GATE rows
+  // [h t, h t + h), the second half the UP rows of the same features (I rows further down), and the epilogue writes
   // act[token, feature] = bf16(SiLU(gate) * up) -- the bits of the partial tile + silu_mul_kernel pair, without the pair
   int64_t swiglu_I;         // 0 = off
   __nv_bfloat16* act;       // [M, swiglu_I]
@@ -191,14 +191,14 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   // 170 now, the tokens' copies by a warp of their own: 4 x 1536 x 1024 by four 2.7 -> 2.3 us, 32 x 9232 x 2048 12.4 -> 10.0).
   const uint32_t b_off = (uint32_t)(a_bytes * (lo ? 2 : 1));
   const int w0 = p.tiled ? 0 : kBlockK, w1 = p.tiled ? kBlockM : 0;      // steps of the weight tile's coordinates per k-block
-  const int wrow = p.tiled ? n_tile * p.kblocks * kBlockM : p.swiglu_I ? n_tile * 64 : n0;
+  const int wrow = p.tiled ? n_tile * p.kblocks * kBlockM : p.swiglu_I ? n_tile * (p.tile_rows / 2) : n0;
   auto load_weights = [&](int kb, uint32_t a_dst, uint32_t bar) {
     if (p.dual_kb && kb >= p.dual_kb) {
       ptx::tma_load_2d(a_dst, &tm_wlo, (kb - p.dual_kb) * kBlockK, n0, bar, ptx::kEvictFirst);
       return;
     }
     ptx::tma_load_2d(a_dst, &tm_w, kb * w0, wrow + kb * w1, bar, ptx::kEvictFirst);
-    // swiglu: tm_w boxes are 64 rows: gate half, then up half of the same 64 features
+    // swiglu: tm_w boxes are half a tile: gate half, then up half of the same features
     if (p.swiglu_I) ptx::tma_load_2d(a_dst + (uint32_t)(a_bytes / 2), &tm_w, kb * kBlockK, (int)p.swiglu_I + wrow, bar, ptx::kEvictFirst);
     if (lo) ptx::tma_load_2d(a_dst + (uint32_t)a_bytes, &tm_wlo, kb * w0, wrow + kb * w1, bar, ptx::kEvictFirst);
   };
@@ -308,41 +308,48 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     constexpr int kChunk = kNTile < 32 ? 16 : 32;
     if constexpr (!kHead) {
       if (p.swiglu_I) {
-        // ---- SwiGLU: accumulator rows 0..63 = gate, 64..127 = up of features [64 t, 64 t + 64); columns = tokens.  The up
-        //      half crosses to the gate half's threads through shared memory (the tile ring is drained), token-major so
-        //      that both the stores and the loads are conflict-free ----
-        float* xch = reinterpret_cast<float*>(smem_raw + (smem_base - ptx::smem_u32(smem_raw)));   // [kNTile][64]
-        const int r = (q & 1) * 32 + lane;             // feature inside the 64
+        // ---- SwiGLU: accumulator rows 0..h-1 = gate, h..2h-1 = up of features [h t, h t + h); columns = tokens.  All of it goes through
+        //      shared memory (the tile ring is drained), token-major and conflict-free, and the four warps share the activations, two
+        //      neighbouring features a thread: 64 rows have 4096 or 2048 of them, each an exponential and a division, which the one or two
+        //      warps that hold the gates took longer for than for the product (64 rows, 4096 features of 1024 channels 15.1 -> 8.7 us, 128 rows 23.5 -> 13.2, 64 x 18944 x 3584 49.6 -> 45.8) ----
+        float* xch = reinterpret_cast<float*>(smem_raw + (smem_base - ptx::smem_u32(smem_raw)));   // [kNTile][2 h]
+        const int h = p.tile_rows / 2;
+        if (q * 32 < 2 * h) {
 #pragma unroll 1
-        for (int c0 = 0; c0 < kNTile; c0 += kChunk) {
-          uint32_t v[kChunk];
-          const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
-          if constexpr (kChunk == 32) ptx::tmem_ld_32x32b_x32(taddr, v);
-          else ptx::tmem_ld_32x32b_x16(taddr, v);
-          ptx::tmem_ld_wait();
-          if (q >= 2) {
+          for (int c0 = 0; c0 < kNTile; c0 += kChunk) {
+            if (c0 >= m_valid) break;
+            uint32_t v[kChunk];
+            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
+            if constexpr (kChunk == 32) ptx::tmem_ld_32x32b_x32(taddr, v);
+            else ptx::tmem_ld_32x32b_x16(taddr, v);
+            ptx::tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < kChunk; ++j) xch[(c0 + j) * 64 + r] = __uint_as_float(v[j]);
+            for (int j = 0; j < kChunk; ++j) xch[(c0 + j) * 2 * h + q * 32 + lane] = __uint_as_float(v[j]);
           }
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-          if (q < 2) {
-            const int64_t f = (int64_t)n_tile * 64 + r;
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        const int per = h / 2, step = 128 / per;         // pairs of features per token, tokens per pass of the four warps
+        const int et = threadIdx.x - 64, f = 2 * (et & (per - 1));
+        __nv_bfloat16* dst = p.act + (int64_t)n_tile * h + f;
+        const bool whole = (reinterpret_cast<uintptr_t>(p.act) & 3) == 0;       // swiglu_I is even
+#pragma unroll 4
+        for (int tkn = et / per; tkn < m_valid; tkn += step) {
+          const float2 g2 = *reinterpret_cast<const float2*>(xch + tkn * 2 * h + f);
+          const float2 u2 = *reinterpret_cast<const float2*>(xch + tkn * 2 * h + h + f);
+          const float gs[2] = {g2.x, g2.y}, us[2] = {u2.x, u2.y};
+          float av[2];
 #pragma unroll
-            for (int j = 0; j < kChunk; ++j) {
-              if (c0 + j < m_valid) {
-                const float gg = __uint_as_float(v[j]), uu = xch[(c0 + j) * 64 + r];
-                float av;
-                if (p.glu_limit > 0.f) {
-                  const float gc = fminf(gg, p.glu_limit), uc = fminf(fmaxf(uu, -p.glu_limit), p.glu_limit);
-                  av = gc / (1.f + __expf(-p.glu_beta * gc)) * (uc + 1.f);
-                } else {
-                  av = (gg / (1.f + __expf(-gg))) * uu;
-                }
-                p.act[(int64_t)(m0 + c0 + j) * p.swiglu_I + f] = __float2bfloat16_rn(av);
-              }
+          for (int e = 0; e < 2; ++e) {
+            if (p.glu_limit > 0.f) {
+              const float gc = fminf(gs[e], p.glu_limit), uc = fminf(fmaxf(us[e], -p.glu_limit), p.glu_limit);
+              av[e] = gc / (1.f + __expf(-p.glu_beta * gc)) * (uc + 1.f);
+            } else {
+              av[e] = (gs[e] / (1.f + __expf(-gs[e]))) * us[e];
             }
           }
-          asm volatile("bar.sync 1, 128;" ::: "memory");   // xch is rewritten by the next chunk
+          __nv_bfloat16* to = dst + (int64_t)(m0 + tkn) * p.swiglu_I;
+          if (whole) *reinterpret_cast<__nv_bfloat162*>(to) = __floats2bfloat162_rn(av[0], av[1]);
+          else { to[0] = __float2bfloat16_rn(av[0]); to[1] = __float2bfloat16_rn(av[1]); }
         }
       } else {
       // ---- TMEM -> registers -> fp32 partial tile ----
@@ -474,7 +481,7 @@ int launch_gemm(const CUtensorMap& tw, const CUtensorMap& twl, const CUtensorMap
                 cudaStream_t stream, const CUtensorMap* tx2 = nullptr) {
   using L = SmemLayout<kNTile>;
   const bool lo = p.has_lo != 0;
-  const int64_t feat_tiles = p.swiglu_I ? p.swiglu_I / 64 : (p.N + p.tile_rows - 1) / p.tile_rows;
+  const int64_t feat_tiles = p.swiglu_I ? p.swiglu_I / (p.tile_rows / 2) : (p.N + p.tile_rows - 1) / p.tile_rows;
   dim3 grid((unsigned)(feat_tiles * ((p.M + kNTile - 1) / kNTile)), (unsigned)p.split_k, 1);
   // The ring: 100 KB let two CTAs share an SM (compute-bound tiles of 128 tokens and more: 200 KB), and never more stages than the CTA
   // has k-blocks, so that a short chain leaves room for its successor's weights.  (Twice the ring where CTAs are alone on their SMs:
@@ -712,11 +719,12 @@ static int gemm_glu_decode_impl(const void* W, const void* X, int64_t M, int64_t
   PRL_CHECK_ARG(!g_tiled_weights, "prl_gemm_swiglu_decode: not available with pre-tiled weights");
   const int nt = pick_ntile(M);
   GemmParams p = {};
-  p.tile_rows = kBlockM;
+  // 64 features a tile, or 32 where that still leaves every tile an SM of its own (as the plain product's short tiles): 4 x 8192 x 1024 7.3 -> 6.7 us, 4 x 9472 x 2048 11.3 -> 10.2
+  p.tile_rows = nt <= 64 && I / 64 <= num_sms() / 2 ? 64 : kBlockM;
   p.M = M; p.N = 2 * I; p.K = K; p.kblocks = (int)((K + kBlockK - 1) / kBlockK); p.split_k = 1;
   p.swiglu_I = I; p.act = (__nv_bfloat16*)act_bf16; p.glu_limit = glu_limit; p.glu_beta = glu_beta;
   CUtensorMap tw, tx;
-  int rc = make_tmap_2d_bf16(&tw, W, (uint64_t)K, (uint64_t)(2 * I), (uint64_t)K * 2, kBlockK, 64);   // 64-row boxes
+  int rc = make_tmap_2d_bf16(&tw, W, (uint64_t)K, (uint64_t)(2 * I), (uint64_t)K * 2, kBlockK, (uint32_t)(p.tile_rows / 2));
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tx, X, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, kBlockK, (uint32_t)nt);
   if (rc) return rc;

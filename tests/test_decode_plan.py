@@ -1,7 +1,7 @@
 """Rules that a decode engine plans its token step by, on the CPU."""
 import pytest
 
-from pipelinerl_b200.engine import swiglu_epilogue_pays
+from pipelinerl_b200.engine import short_swiglu_tiles_pay, swiglu_epilogue_pays
 
 
 @pytest.mark.parametrize("I,H,split,pays", [(18944, 3584, 1, True), (8192, 2048, 8, True), (4096, 1024, 2, False), (8000, 2048, 8, True),
@@ -10,3 +10,10 @@ from pipelinerl_b200.engine import swiglu_epilogue_pays
 def test_swiglu_epilogue_rule(I, H, split, pays):
     """Unsplit always; else while the idle SMs of I / 64 tiles on 148 cost at most 5 k-blocks of 64."""
     assert swiglu_epilogue_pays(I, H, split, 148) is pays
+
+
+@pytest.mark.parametrize("I,H,rows,pays", [(4096, 1024, 4, True), (4096, 1024, 64, True), (4096, 1024, 65, False), (4736, 2048, 8, True),
+                                           (4800, 2048, 8, False), (3264, 1088, 8, False), (3392, 1024, 8, True), (3264, 1024, 8, True), (3200, 1024, 8, False), (64, 320, 2, True)])
+def test_short_swiglu_tiles_rule(I, H, rows, pays):
+    """Up to 64 rows, tiles of 32 features on at most 148 SMs, and the idle ones cost at most 5 k-blocks of 64."""
+    assert short_swiglu_tiles_pay(I, H, rows, 148) is pays

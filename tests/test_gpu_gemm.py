@@ -179,6 +179,28 @@ def test_token_step_swiglu_epilogue_is_bit_identical_to_gemm_plus_silu(cuda_devi
     assert (got.float() - fp32).abs().max().item() <= 2 ** -7 * fp32.abs().max().item() + 1e-6
 
 
+@pytest.mark.parametrize("B", [1, 17, 64, 65])
+@pytest.mark.parametrize("I,K,limit", [(64, 8, 0.0), (4096, 1024, 0.0), (4736, 200, 7.0), (4800, 72, 0.0)])
+def test_short_gated_tiles_keep_the_bits(cuda_device, B, I, K, limit):
+    """The gated epilogue's tiles of 32 features (up to 4736 of them and 64 rows) against the product and the activation by themselves,
+    at both sides of the lines, bit for bit; one k-block and ragged ones."""
+    from pipelinerl_b200 import _lib
+    lib, st, g = _lib.load(), _lib.stream_ptr(), torch.Generator(device="cuda").manual_seed(B + I + K)
+    x = torch.randn(B, K, generator=g, device="cuda").bfloat16()
+    W = (torch.randn(2 * I, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    part, want = torch.empty(B, 2 * I, device="cuda"), torch.empty(B, I, dtype=torch.bfloat16, device="cuda")
+    got = torch.full((B, I), float("nan"), dtype=torch.bfloat16, device="cuda")
+    _lib.check(lib.prl_gemm_bf16_splitk(W.data_ptr(), None, x.data_ptr(), B, 2 * I, K, 1, part.data_ptr(), st))
+    if limit:
+        _lib.check(lib.prl_glu_clamped(part.data_ptr(), 2 * I, B, I, limit, 1.7, want.data_ptr(), 0, st))
+        _lib.check(lib.prl_gemm_glu_clamped_decode(W.data_ptr(), x.data_ptr(), B, I, K, limit, 1.7, got.data_ptr(), st))
+        assert (got.float() - want.float()).abs().max() <= 2.0 ** -8 * want.float().abs().max()        # another division of the same quotient
+    else:
+        _lib.check(lib.prl_silu_mul(part.data_ptr(), 1, B, I, want.data_ptr(), None, 0, st))
+        _lib.check(lib.prl_gemm_swiglu_decode(W.data_ptr(), x.data_ptr(), B, I, K, got.data_ptr(), st))
+        assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("M", [1, 17, 64])
 @pytest.mark.parametrize("N,K", [(8, 8), (1000, 2056), (4736, 72), (4737, 1024), (9232, 2048), (9472, 200), (9473, 64)])
 def test_short_weight_tiles_keep_the_bits(cuda_device, M, N, K):
