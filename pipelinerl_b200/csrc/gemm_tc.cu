@@ -483,13 +483,17 @@ int launch_gemm(const CUtensorMap& tw, const CUtensorMap& twl, const CUtensorMap
   const bool lo = p.has_lo != 0;
   const int64_t feat_tiles = p.swiglu_I ? p.swiglu_I / (p.tile_rows / 2) : (p.N + p.tile_rows - 1) / p.tile_rows;
   dim3 grid((unsigned)(feat_tiles * ((p.M + kNTile - 1) / kNTile)), (unsigned)p.split_k, 1);
-  // The ring: 100 KB let two CTAs share an SM (compute-bound tiles of 128 tokens and more: 200 KB), and never more stages than the CTA
-  // has k-blocks, so that a short chain leaves room for its successor's weights.  (Twice the ring where CTAs are alone on their SMs:
-  // 32 x 9232 x 2048 12.9 -> 12.2 us, but 4 x 8192 x 1024 by two 5.0 -> 5.8: an SM has no more than some 64 KB under way anyway.)
+  // The ring: 100 KB let two CTAs share an SM (200 KB for compute-bound tiles of 128 tokens and more), and never more stages than the CTA
+  // has k-blocks, so that a short chain leaves room for its successor's weights.  Whole tiles that are alone on their SMs take 200 KB:
+  // with 100 such a CTA has 64 KB of weights under way beside 64 tokens (64 x 3584 x 18944 by five 26.3 -> 22.6 us, 64 x 2048 x 8192 by nine
+  // 10.4 -> 9.3, 16 x 3584 x 18944 22.0 -> 20.4; a token step of 64 rows, four layers of 2048 349 -> 333).  Short tiles share their SMs with
+  // another branch's kernel (a hybrid step of 32 rows 557 -> 560 with the larger ring), and where two tiles share an SM the larger ring
+  // drives one out (64 x 152064 x 3584 187 -> 209).
   const int stage = p.tile_rows * kBlockK * 2 * (lo ? 2 : 1) + L::kBBytes;
   const int kb = (p.kblocks + p.split_k - 1) / p.split_k;
   const int most = 8 * (kBlockM / p.tile_rows);
-  int n_stages = (kNTile >= 128 ? 200 * 1024 : g_smem_budget) / stage;
+  const bool alone = (int64_t)grid.x * grid.y <= num_sms() && p.tile_rows == kBlockM;
+  int n_stages = (kNTile >= 128 || alone ? 200 * 1024 : g_smem_budget) / stage;
   n_stages = n_stages > most ? most : n_stages;
   n_stages = n_stages > kb ? kb : n_stages;
   if (n_stages < 2) n_stages = 2;
