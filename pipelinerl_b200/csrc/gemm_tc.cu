@@ -107,7 +107,7 @@ constexpr int kBlockM = 128;  // output features per CTA (UMMA M)
 constexpr int kBlockK = 64;   // bf16 elements per stage row = 128 B = one swizzle atom
 constexpr int kUmmaK = 16;
 constexpr int kThreads = 192;
-static int g_smem_budget = 100 * 1024;   // per-CTA tile ring; <= 100 KB lets two CTAs share an SM
+static int g_smem_budget = 0;            // per-CTA tile ring in bytes; 0: by the rule in launch_gemm
 static int g_tiled_weights = 0;          // weights stored as contiguous [N/128][K/64][128][64] tiles
 
 struct HeadPart { float m, s, u, key, z; int idx; };  // per (vocab tile, token): online-softmax state + best sample
@@ -483,17 +483,27 @@ int launch_gemm(const CUtensorMap& tw, const CUtensorMap& twl, const CUtensorMap
   const bool lo = p.has_lo != 0;
   const int64_t feat_tiles = p.swiglu_I ? p.swiglu_I / (p.tile_rows / 2) : (p.N + p.tile_rows - 1) / p.tile_rows;
   dim3 grid((unsigned)(feat_tiles * ((p.M + kNTile - 1) / kNTile)), (unsigned)p.split_k, 1);
-  // The ring: 100 KB let two CTAs share an SM (200 KB for compute-bound tiles of 128 tokens and more), and never more stages than the CTA
-  // has k-blocks, so that a short chain leaves room for its successor's weights.  Whole tiles that are alone on their SMs take 200 KB:
-  // with 100 such a CTA has 64 KB of weights under way beside 64 tokens (64 x 3584 x 18944 by five 26.3 -> 22.6 us, 64 x 2048 x 8192 by nine
-  // 10.4 -> 9.3, 16 x 3584 x 18944 22.0 -> 20.4; a token step of 64 rows, four layers of 2048 349 -> 333).  Short tiles share their SMs with
-  // another branch's kernel (a hybrid step of 32 rows 557 -> 560 with the larger ring), and where two tiles share an SM the larger ring
-  // drives one out (64 x 152064 x 3584 187 -> 209).
+  // The ring, never more stages than the CTA has k-blocks, so that a short chain leaves room for its successor's weights:
+  //  * compute-bound tiles of 128 tokens and more: 200 KB;
+  //  * whole tiles that are alone on their SMs, in chains of at least twice the stages of 111 KB: 200 KB.  With 100 such a CTA has 64 KB
+  //    of weights under way beside 64 tokens (64 x 3584 x 18944 by five 26.3 -> 22.6 us, 64 x 2048 x 8192 by nine 10.4 -> 9.3, 16 x 3584 x
+  //    18944 22.0 -> 20.4; a token step of 64 rows, four layers of 2048 349 -> 333); shorter chains only lose their successor's early
+  //    weights (32 x 3072 x 2048 by six 4.9 -> 5.4);
+  //  * two to an SM: 111 KB, which is what fits (hi + lo weights, up to 32 tokens: three stages for two, x 32768 x 1024 30 -> 23 us, x 32768 x
+  //    2048 46 -> 38; plain ones of up to 16 tokens: six for five, 16 x 152064 x 3584 159 -> 157);
+  //  * hi + lo weights in many waves: with up to 32 tokens 100 KB, three CTAs an SM of two stages each (x 152064 x 3584 298 us, 303 with
+  //    111 KB); with 64 tokens, where two stages are 80 KB, one CTA of five (348 -> 334);
+  //  * short tiles share their SMs with another branch's kernel: 100 KB (a hybrid step of 32 rows 557 us, 560 with more).
   const int stage = p.tile_rows * kBlockK * 2 * (lo ? 2 : 1) + L::kBBytes;
   const int kb = (p.kblocks + p.split_k - 1) / p.split_k;
   const int most = 8 * (kBlockM / p.tile_rows);
-  const bool alone = (int64_t)grid.x * grid.y <= num_sms() && p.tile_rows == kBlockM;
-  int n_stages = (kNTile >= 128 || alone ? 200 * 1024 : g_smem_budget) / stage;
+  const int64_t ctas = (int64_t)grid.x * grid.y, sms = num_sms();
+  const bool whole = p.tile_rows == kBlockM;
+  int ring = (whole ? 111 : 100) * 1024;
+  if (kNTile >= 128 || (whole && ctas <= sms && kb >= 2 * (ring / stage)) || (lo && kNTile == 64 && ctas >= 4 * sms)) ring = 200 * 1024;
+  else if (lo && kNTile < 64 && ctas > 2 * sms) ring = 100 * 1024;
+  if (g_smem_budget && kNTile < 128) ring = g_smem_budget;
+  int n_stages = ring / stage;
   n_stages = n_stages > most ? most : n_stages;
   n_stages = n_stages > kb ? kb : n_stages;
   if (n_stages < 2) n_stages = 2;
