@@ -408,7 +408,35 @@ constexpr int kSampleParts = 16;   // CTAs per row: 64 rows x 16 = 1024 CTAs kee
 constexpr int kSampleThreads = 256;
 struct SamplePartial { float m, s, v, z; int i; int pad[3]; };  // z = logit/T of the best key (logprob without re-reading logits)
 
-// phase 1: each CTA scans a contiguous 1/16 of the vocabulary of one row
+// phase 1: each CTA scans a contiguous 1/16 of the vocabulary of one row.  Issue-bound: a value's noise alone is some 35 instructions.  Values
+// come in groups of eight per thread, with their loads together, one comparison with the maximum and no branch per value:
+// 64 x 152064 33.7 -> 26.5 us, without noise 21.4 -> 13.3; the same ids.
+template <int n>
+__device__ __forceinline__ void sample_group(const float (&x)[n], int i, float inv_temp, int greedy, uint64_t seed, uint32_t step, int b,
+                                             int vocab_offset, float& m, float& s, ArgMax& best, float& best_z) {
+  float z[n], top = -INFINITY;
+#pragma unroll
+  for (int k = 0; k < n; ++k) {
+    z[k] = x[k] * inv_temp;
+    top = fmaxf(top, z[k]);
+  }
+  if (top > m) {
+    s *= __expf(m - top);          // exp(-inf) = 0 for the first group
+    m = top;
+  }
+  const float base = m == -INFINITY ? 0.f : m;
+#pragma unroll
+  for (int k = 0; k < n; ++k) s += __expf(z[k] - base);
+#pragma unroll
+  for (int k = 0; k < n; ++k) {
+    const int gid = vocab_offset + i + k * kSampleThreads;   // global vocabulary id (vocab-parallel head: this rank owns a slice)
+    const float key = greedy ? z[k] : z[k] + gumbel(seed, step, (uint32_t)b, (uint32_t)gid);
+    if (key > best.v) {            // a thread's ids ascend: the lowest of equal keys stays
+      best = ArgMax{key, gid};
+      best_z = z[k];
+    }
+  }
+}
 __global__ void __launch_bounds__(kSampleThreads) sample_partial_kernel(const float* __restrict__ logits, int V,
                                                                        float inv_temp, int greedy, uint64_t seed,
                                                                        uint32_t step, int vocab_offset,
@@ -427,15 +455,16 @@ __global__ void __launch_bounds__(kSampleThreads) sample_partial_kernel(const fl
   float m = -INFINITY, s = 0.f;
   ArgMax best{-INFINITY, 0x7fffffff};
   float best_z = 0.f;
-  for (int i = lo + threadIdx.x; i < hi; i += kSampleThreads) {
-    const float zi = z[i] * inv_temp;
-    if (zi > m) { s = s * __expf(m - zi) + 1.f; m = zi; } else { s += __expf(zi - m); }
-    const int gid = vocab_offset + i;   // global vocabulary id (vocab-parallel head: this rank owns a slice)
-    const float key = greedy ? zi : zi + gumbel(seed, step, (uint32_t)b, (uint32_t)gid);
-    const ArgMax cand{key, gid};
-    const ArgMax nb = better(best, cand);
-    if (nb.i != best.i) best_z = zi;
-    best = nb;
+  int i = lo + threadIdx.x;
+  for (; i + 7 * kSampleThreads < hi; i += 8 * kSampleThreads) {
+    float x[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = z[i + k * kSampleThreads];
+    sample_group(x, i, inv_temp, greedy, seed, step, b, vocab_offset, m, s, best, best_z);
+  }
+  for (; i < hi; i += kSampleThreads) {
+    const float x[1] = {z[i]};
+    sample_group(x, i, inv_temp, greedy, seed, step, b, vocab_offset, m, s, best, best_z);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
