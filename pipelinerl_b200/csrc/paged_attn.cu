@@ -74,14 +74,14 @@ __device__ __forceinline__ float fast_exp2(float x) {
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p) {
+paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p, int n_st) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - ptx::smem_u32(smem_raw));
-  const uint32_t bar_base = base + kStages * kStageBytes;
+  const uint32_t bar_base = base + (uint32_t)(n_st * kStageBytes);
   auto full_bar = [&](int s) { return bar_base + 8u * (uint32_t)s; };
-  auto empty_bar = [&](int s) { return bar_base + 8u * (uint32_t)(kStages + s); };
-  int32_t* s_pages = reinterpret_cast<int32_t*>(base_ptr + kStages * kStageBytes + 8 * 2 * kStages);
+  auto empty_bar = [&](int s) { return bar_base + 8u * (uint32_t)(n_st + s); };
+  int32_t* s_pages = reinterpret_cast<int32_t*>(base_ptr + n_st * kStageBytes + 8 * 2 * n_st);
 
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -142,7 +142,7 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p
   }
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < n_st; ++s) {
       ptx::mbar_init(full_bar(s), 1);
       ptx::mbar_init(empty_bar(s), kConsumers);
     }
@@ -162,10 +162,10 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p
   if (warp == kConsumers) {
     // ===== producer: TMA whole pages into the ring =====
     if (lane == 0) {
+      int s = 0;
+      uint32_t ph = 1u;
       for (int it = 0; it < n_it; ++it) {
-        const int s = it % kStages;
-        const uint32_t ph = (uint32_t)((it / kStages) & 1);
-        ptx::mbar_wait(empty_bar(s), ph ^ 1u);
+        ptx::mbar_wait(empty_bar(s), ph);
         ptx::mbar_arrive_expect_tx(full_bar(s), kStageBytes);
         const int page = s_pages[it];
         const int row_k = (int)(((((int64_t)p.layer * 2 + 0) * p.n_pages + page) * p.n_kv + kvh) * kPage);
@@ -175,6 +175,7 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p
         ptx::tma_load_2d(dst + 8192, &tm_kv, 64, row_k, full_bar(s), ptx::kEvictFirst);
         ptx::tma_load_2d(dst + 16384, &tm_kv, 0, row_v, full_bar(s), ptx::kEvictFirst);
         ptx::tma_load_2d(dst + 24576, &tm_kv, 64, row_v, full_bar(s), ptx::kEvictFirst);
+        if (++s == n_st) { s = 0; ph ^= 1u; }
       }
     }
   } else {
@@ -193,9 +194,9 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p
       }
     }
     const int mi = lane >> 3, lr = lane & 7;
+    int s = 0;
+    uint32_t ph = 0u;
     for (int it = 0; it < n_it; ++it) {
-      const int s = it % kStages;
-      const uint32_t ph = (uint32_t)((it / kStages) & 1);
       ptx::mbar_wait(full_bar(s), ph);
       const uint32_t kbase = base + (uint32_t)(s * kStageBytes);
       const uint32_t vbase = kbase + 16384;
@@ -258,6 +259,7 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p
       }
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(empty_bar(s));
+      if (++s == n_st) { s = 0; ph ^= 1u; }
     }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
@@ -533,12 +535,16 @@ extern "C" int prl_attn_set_fused_combine(int32_t on) {
   return PRL_OK;
 }
 
+// Shares that a context is cut into.  A share costs a start, a merge and its part of the combine kernel, so contexts are cut
+// while the CTAs stay one per SM (pages of 64 keys, us by 1 / 2 / 4 / 8 / 16): 4 CTAs of 47 pages 18.9 / 13.2 / 10.3 / 8.3 / 8.4, 24 of 11 10.6 / 10.6 /
+// 9.4, 48 of 8 9.0 / 10.2, 64 of 47 22.8 / 20.1 / 19.5 / 23.3, 128 of 63 39.0 / 40.8.  One more cut where long contexts leave SMs idle or unevenly filled: 96
+// of 125 60.5 / 56.2, 256 of 129 145 / 137, 256 of 86 100 / 94, but 256 of 47 55.9 / 58.7, of 10 16.3 / 21.4, 160 of 128 96 / 106, 512 of 125 255 / 268.
 extern "C" int prl_paged_attn_splits(int32_t B, int32_t n_kv, int32_t max_seq_len) {
   const int pages = (max_seq_len + kPage - 1) / kPage;
-  const int sms = num_sms();
+  const int sms = num_sms(), ctas = B * n_kv;
   int splits = 1;
-  // enough CTAs for >= 2 waves, at least 4 pages per CTA, never more pages than the smem page list holds
-  while (B * n_kv * splits < 2 * sms && pages / (splits * 2) >= 4) splits *= 2;
+  while (splits < 16 && ctas * splits * 2 <= sms && pages > 8 && pages >= 5 * splits) splits *= 2;
+  if (splits == 1 && ((ctas <= sms && pages >= 96) || (4 * ctas > 5 * sms && ctas <= 2 * sms && pages >= 64))) splits = 2;
   while ((pages + splits - 1) / splits > kMaxPagesPerSplit) splits *= 2;
   return splits;
 }
@@ -579,12 +585,15 @@ extern "C" int prl_paged_attn_decode(const void* q, const void* kv_cache, int64_
   p.out = (__nv_bfloat16*)out_bf16;
   p.direct = n_splits == 1;    // 4 x 333 keys, eight layers: one launch of nine a layer less, 285 -> 274 us a step
   if (p.direct) p.tickets = nullptr;
-  const int smem = kStages * kStageBytes + 1024 + 8 * 2 * kStages + 4 * kMaxPagesPerSplit + 16;
+  // Six stages for a CTA that has its SM alone, three where there are more CTAs than SMs: as many bytes under way, and one's start and
+  // merge under the other's pages (us: 64 x 600 keys of 4 heads by two 25.8 -> 21.6, 64 x 200 12.6 -> 10.1, 64 x 7000 by two 133 -> 128)
+  const int n_st = (int64_t)n_splits * n_kv * B > num_sms() ? kStages / 2 : kStages;
+  const int smem = n_st * kStageBytes + 1024 + 8 * 2 * n_st + 4 * kMaxPagesPerSplit + 16;
   static SmemAttr smem_attr = {};
   PRL_CUDA(ensure_smem(paged_attn_decode_kernel, smem, smem_attr));
   cudaStream_t stream = (cudaStream_t)stream_;
   dim3 grid((unsigned)n_splits, (unsigned)n_kv, (unsigned)B);
-  PRL_CUDA(launch_pdl(paged_attn_decode_kernel, grid, dim3(kThreads), (size_t)smem, stream, tm, p));
+  PRL_CUDA(launch_pdl(paged_attn_decode_kernel, grid, dim3(kThreads), (size_t)smem, stream, tm, p, n_st));
   PRL_LAUNCH_CHECK();
   if (!g_fused_combine && !p.direct) {
     PRL_CUDA(launch_pdl(attn_combine_kernel, dim3((unsigned)(B * n_q)), dim3(kD), 0, stream, (const float*)p.o_part,
