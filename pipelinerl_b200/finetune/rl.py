@@ -168,7 +168,7 @@ class _LogitsLoss(torch.autograd.Function):
         ctx.save_for_backward(logits, ids, stats, grads)
         ctx.temperature = float(temperature)
         ctx.dlogits = None
-        if ctx.needs_input_grad[0]:
+        if ctx.needs_input_grad[0] and T > 1:        # one row has no next token: its loss is made, a gradient is refused by the kernel's entry
             ctx.dlogits = d = torch.empty((T, V), dtype=torch.float32, device=logits.device)
             later.append(lambda: _LogitsLoss._d_logits(logits, ids, stats, grads, float(temperature), None, d))
         return loss
@@ -230,8 +230,8 @@ def rl_step(model, batch: PipelineBatchEncoding, current_step: int, max_step: in
 
     `model` is either any module whose output has `.logits` (the reference contract,
     rl/__init__.py:190-207) or a pipelinerl_b200 model exposing
-    `forward_logprobs(batch, temperature) -> (new_logprobs[B, L-1], entropy[B, L-1])`, in which case
-    full-vocabulary logits never reach HBM.
+    `forward_logprobs(batch, temperature) -> (new_logprobs[B, L-1], entropy[B, L-1])`: what is held of
+    the full-vocabulary logits is then its own affair (NativeQwen2: for its backward, in a quarter of the free memory at most).
     """
     if seq_parallel_group is not None:
         # The batch is this rank's slice of a packed row (PipelineBatchEncoding.make_slices); like the reference, logits

@@ -401,3 +401,16 @@ def test_gradient_of_logits_made_ahead_of_the_backward(cuda_device, policy, T, V
     with torch.no_grad():
         quiet, stats2 = rl.rl_step(model, batch, 0, 10, cfg)
     assert not quiet.requires_grad and stats2 == stats
+
+
+def test_row_of_one_token_has_a_loss(cuda_device):
+    """No next token: rl_step gives its loss (none) and reports the input's size; nothing of d logits is made ahead."""
+    from pipelinerl_b200.finetune import rl
+    from pipelinerl_b200.finetune.types import PipelineBatchEncoding
+    z = torch.zeros(1, 1)
+    batch = PipelineBatchEncoding(
+        input_ids=z.long(), attention_mask=z.long() + 1, labels=z.long(), position_ids=z.long(), segment_ids=z.long(), rewards=z, advantages=z,
+        ref_logprobs=z, old_logprobs=z, group_tokens=z + 1, num_labels=z + 1, overflow=z, seq_boundaries=torch.tensor([0, 1], dtype=torch.int32),
+        model_version=0, is_packed=True).to_device(cuda_device)
+    loss, stats = rl.rl_step(LogitsModel(torch.randn(1, 1, 64, device=cuda_device)), batch, 0, 10, rl.RLConfig(policy_loss="ppo", batch_size=1))
+    assert loss.item() == 0.0 and stats == {"input_size": 1.0}
