@@ -804,3 +804,45 @@ def test_trace_runner_command_line(cuda_device, tmp_path):
         for i, ref in expect.items():
             got = torch.from_numpy(np.fromfile(out / f"{i}.f32", dtype="<f4")).view(-1, config["vocab"])
             assert got.shape == ref.shape and mc.rel_err(got, ref) < tol
+
+
+@pytest.mark.parametrize("segs,heads,kh,dk,dv,taps", [((1,), 2, 1, 4, 4, 2), ((5, 1, 2, 9), 4, 2, 128, 128, 4), ((3, 70), 2, 2, 124, 132, 3), ((66,), 2, 1, 256, 260, 4),
+                                                       ((7, 2, 30), 3, 3, 20, 300, 2), ((2, 3, 4), 6, 2, 36, 8, 4), ((130,), 16, 8, 128, 128, 3)])
+def test_front_rows_of_the_gated_delta_rule(cuda_device, segs, heads, kh, dk, dv, taps):
+    """Convolution with carried inputs, SiLU and unit length against 64 bits.  Bound: `taps` products and sums of 2^-24 each relative to
+    the sum of magnitudes, a SiLU of a few units of 2^-24 of a slope of at most 1.1, and the same again for the length."""
+    from pipelinerl_b200 import _lib
+    lib, dev, g = _lib.load(), cuda_device, torch.Generator().manual_seed(sum(segs) + dv)
+    n, ns, ch = sum(segs), len(segs), 2 * kh * dk + heads * dv
+    ld = (ch + heads * dv + 2 * heads + 3) // 4 * 4
+    rnd = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    P, w, conv0 = rnd(n, ld), rnd(ch, taps), rnd(ns, ch, taps - 1)
+    starts = [sum(segs[:i]) for i in range(ns)]
+    subs = [(i, s + a, min(64, l - a)) for i, (s, l) in enumerate(zip(starts, segs)) for a in range(0, l, 64)]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)  # noqa: E731
+    tabs = [i32([i for i, l in enumerate(segs) for _ in range(l)]), i32([t for l in segs for t in range(l)]), i32(starts), i32(list(segs)), i32(list(range(ns))),
+            i32([sum(1 for j, _, _ in subs if j < i) for i in range(ns)]), i32([sum(1 for j, _, _ in subs if j == i) for i in range(ns)]),
+            i32([s for _, s, _ in subs]), i32([l for _, _, l in subs])]
+    f = lambda *s: torch.zeros(*s, device=dev)  # noqa: E731
+    on = lambda t: t.to(dev)  # noqa: E731
+    Pd, wd, conv, A, dt, gain = on(P), on(w), on(conv0.clone()), on(0.1 * rnd(heads)), on(rnd(heads)), on(rnd(dv))
+    C, scr = f(n, ch), f(n * int(lib.prl_gated_delta_split_floats(heads, dk)))
+    S0, D, state, out = f(len(subs), heads, dk, dv), f(n, heads * dv), f(ns, heads, dv, dk), f(n, heads * dv)
+    p = lambda t: t.data_ptr()  # noqa: E731
+    _lib.check(lib.prl_gated_delta_split(p(Pd), ld, 0, ch, ch + heads, ch + 2 * heads, p(wd), taps, p(A), p(dt), 1e-6, p(gain), 1e-5, heads, kh, dk, dv, n,
+                                         p(tabs[0]), p(tabs[1]), p(tabs[2]), p(tabs[3]), p(tabs[4]), ns, p(tabs[5]), p(tabs[6]), p(tabs[7]), p(tabs[8]),
+                                         len(subs), p(C), p(scr), p(S0), p(D), p(conv), p(state), p(out), 1, _lib.stream_ptr()))
+    want, size = torch.empty(n, ch, dtype=torch.float64), torch.empty(n, ch, dtype=torch.float64)
+    for i, (s, l) in enumerate(zip(starts, segs)):
+        x = torch.cat([conv0[i].double(), P[s:s + l, :ch].double().T], 1)          # [ch, taps - 1 + l]
+        t = x.unfold(1, taps, 1) * w.double()[:, None]
+        want[s:s + l], size[s:s + l] = torch.nn.functional.silu(t.sum(-1)).T, t.abs().sum(-1).T
+    bound = 2.0 ** -24 * ((taps + 2) * size + 8 * want.abs())
+    for h in range(2 * kh):
+        c = slice(h * dk, (h + 1) * dk)
+        length = (want[:, c].square().sum(-1, keepdim=True) + 1e-6).sqrt()
+        by = (dk ** -0.5 if h < kh else 1.0) / length
+        worst = bound[:, c].norm(dim=-1, keepdim=True) / length                    # of the length, relative
+        bound[:, c] = by * (bound[:, c] + want[:, c].abs() * (worst + 2.0 ** -24 * (dk / 16 + 8)))
+        want[:, c] *= by
+    assert bool(((C.cpu().double() - want).abs() <= bound).all())
