@@ -355,6 +355,8 @@ int prl_rope_inplace(void* x, int64_t ld, int64_t T, int32_t n_heads, int32_t he
 /* gate_up [T, 2I] = [gate | up] -> act [T, I] = silu(gate) * up, and its backward */
 int prl_silu_mul_fwd(const void* gate_up, int64_t T, int64_t I, void* act, prl_stream_t stream);
 int prl_silu_mul_bwd(const void* gate_up, const void* dact, int64_t T, int64_t I, void* dgate_up, prl_stream_t stream);
+/* the same, and `act` of the forward takes the place of dact (the bits of prl_silu_mul_fwd) */
+int prl_silu_mul_bwd_act(const void* gate_up, void* dact, int64_t T, int64_t I, void* dgate_up, prl_stream_t stream);
 int prl_embed_gather(const void* table, const int64_t* ids, int64_t T, int64_t H, void* out, prl_stream_t stream);
 /* dtable[ids[t]] += dh[t] (fp32 atomics: the one reduction here whose order is not fixed, as in torch); dh starts on 16 bytes,
  * dtable anywhere (four sums per access where it starts on 16 bytes too) */

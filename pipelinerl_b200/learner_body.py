@@ -126,6 +126,13 @@ class Ops:
                                              _lib.stream_ptr()))
         return dgu
 
+    def silu_mul_bwd_act(self, gu, dact):
+        """d gate_up, and act = silu_mul(gu) in the place of dact"""
+        T, two_i = gu.shape
+        dgu = torch.empty_like(gu)
+        _lib.check(self.lib.prl_silu_mul_bwd_act(gu.data_ptr(), dact.data_ptr(), T, two_i // 2, dgu.data_ptr(), _lib.stream_ptr()))
+        return dgu, dact
+
     def colsum_acc(self, x, out_f32):
         """out[C] (fp32) += sum over rows of x [T, C] (bf16), fixed reduction order"""
         T, Cc = x.shape
@@ -315,15 +322,20 @@ class NativeBody:
             x2, rstd2, gu, act, _ = self._mlp_half(l, h2, need_out=False)
         else:               # gate_up output kept too: norm and SiLU*up are one pass each, no GEMM
             x2, rstd2 = o.rmsnorm(h2, w[p + "post_attention_layernorm.weight"], c.rms_eps)
-            act = o.silu_mul(gu)
+            act = None      # made beside d gate_up, or below
         T = h.shape[0]
-        o.wgrad(g[p + "down_proj.weight"], dh3, act)
-        del act
         if c.intermediate_size % 32 == 0 and self.fuse_silu_bwd:     # SiLU * up backward in the dgrad GEMM's epilogue: d act never reaches HBM
+            o.wgrad(g[p + "down_proj.weight"], dh3, act if act is not None else o.silu_mul(gu))
             d_gu = o.dgrad_swiglu(dh3, w[p + "down_proj.weight"], gu)
+        elif act is None:
+            d_gu, act = o.silu_mul_bwd_act(gu, o.dgrad(dh3, w[p + "down_proj.weight"]))
+            del gu
+            o.wgrad(g[p + "down_proj.weight"], dh3, act)
         else:
+            o.wgrad(g[p + "down_proj.weight"], dh3, act)
+            act = None
             d_gu = o.silu_mul_bwd(gu, o.dgrad(dh3, w[p + "down_proj.weight"]))
-        del gu
+        gu = act = None
         dx2 = o.dgrad(d_gu, w[p + "gate_up_proj.weight"])
         o.wgrad(g[p + "gate_up_proj.weight"], d_gu, x2)
         del d_gu, x2

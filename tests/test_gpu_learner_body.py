@@ -428,3 +428,17 @@ def test_silu_rows_cut_over_blocks(cuda_device, T, I):
     dgu = o.silu_mul_bwd(gu, da).double()
     want = torch.cat([d * u * (s + a * s * (1 - s)), d * a * s], 1)
     assert ((dgu - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
+
+
+@pytest.mark.parametrize("T,I", [(1, 8), (2, 18944), (37, 2056), (700, 24), (1500, 4096), (1003, 256), (9, 264)])
+def test_activation_beside_its_backward(cuda_device, T, I):
+    """act in the place of d act, and d gate_up: the bits of the two launches"""
+    from pipelinerl_b200.learner_body import Ops
+    o, g = Ops(), torch.Generator().manual_seed(T + I)
+    gu = (3 * torch.randn(T, 2 * I, generator=g)).to(torch.bfloat16).to(cuda_device)
+    gu[0, 0], gu[0, 1], gu[-1, -1] = 200.0, -200.0, float("inf")
+    da = torch.randn(T, I, generator=g).to(torch.bfloat16).to(cuda_device)
+    want_act, want = o.silu_mul(gu), o.silu_mul_bwd(gu, da)
+    dgu, act = o.silu_mul_bwd_act(gu, da)
+    assert act.data_ptr() == da.data_ptr()
+    assert torch.equal(act.view(torch.int16), want_act.view(torch.int16)) and torch.equal(dgu.view(torch.int16), want.view(torch.int16))
