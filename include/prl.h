@@ -448,6 +448,13 @@ int prl_paged_attn_decode(const void* q_bf16, const void* kv_cache_bf16, int64_t
                           int32_t B, int32_t n_q, int32_t n_kv, int32_t head_dim, int32_t page_size,
                           int32_t n_splits, float sm_scale, void* out_bf16 /*[B, n_q*128]*/,
                           void* workspace, size_t workspace_bytes, prl_stream_t stream);
+/* The same straight from the projection's split-K partials [n_split][B][(n_q + 2 n_kv) * 128]: each sequence's token is at position
+ * seq_lens - 1 (0: no token), its q, k and v are those of prl_qkv_rope_cache, and k and v are written to its page. */
+int prl_paged_attn_decode_qkv(const float* partials, int32_t n_split, const void* bias /*[(n_q + 2 n_kv) * 128] bf16 or NULL*/,
+                              const float* inv_freq /*[64]*/, void* kv_cache_bf16, int64_t n_pages, int32_t n_layers, int32_t layer,
+                              const int32_t* block_table, int32_t max_blocks, const int32_t* seq_lens, int32_t B, int32_t n_q,
+                              int32_t n_kv, int32_t head_dim, int32_t page_size, int32_t n_splits, float sm_scale, void* out_bf16,
+                              void* workspace, size_t workspace_bytes, prl_stream_t stream);
 /* Chunked prefill: causal attention of seq_q_len[z] query rows (starting at row seq_q_start[z], first
  * position seq_pos0[z]) against the paged KV of block-table row seq_slot[z]; the chunk's own K/V must
  * already be in the cache (prl_qkv_rope_cache).  Replaces vLLM's chunked-prefill attention

@@ -222,10 +222,6 @@ __global__ void __launch_bounds__(256) residual_rmsnorm_rows_kernel(const float*
   }
 }
 
-// the rotated pair, contracted one way in every kernel
-__device__ __forceinline__ float rot_first(float a, float c, float cs, float sn) { return fmaf(a, cs, -__fmul_rn(c, sn)); }
-__device__ __forceinline__ float rot_second(float a, float c, float cs, float sn) { return fmaf(c, cs, __fmul_rn(a, sn)); }
-
 // ---- split-K reduce + bias + RoPE + KV-page write ---------------------------------------
 // part [n_split, B, (n_q + 2 n_kv) * 128]; one block per (token, head), 64 threads = 64 rotation pairs.
 // q -> q_out [B, n_q, 128] bf16 ; k, v -> cache rows ((layer*2 + kv) * n_pages + page) * n_kv * PAGE + kvh*PAGE + slot

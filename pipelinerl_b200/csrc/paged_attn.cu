@@ -49,6 +49,16 @@ struct AttnParams {
   int direct;                  // one split: the output is written here, no partials
 };
 
+// The token's own q, k and v straight from the projection's split-K partials (kNew): q, k, v of qkv_rope_cache_kernel, bit for bit
+struct NewToken {
+  const float* part;           // [n_split, B, (n_q + 2 n_kv) * 128]
+  int n_split, B;
+  const __nv_bfloat16* bias;   // [(n_q + 2 n_kv) * 128] or NULL
+  const float* inv_freq;       // [64]
+  __nv_bfloat16* kv_cache;     // the token's place in it is written
+};
+constexpr int kQRow = kD + 8;  // a row of q in shared memory: fragment reads of eight rows touch every bank once
+
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
@@ -73,8 +83,14 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
-paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p, int n_st) {
+// kRows > 0: a sequence's token is at position seq_lens - 1, and every CTA makes the q of its heads while the first pages are on their way, so
+// the launch between the projection and the attention and the round trip of q fall away.  The CTA of the last page makes k and v too: into
+// their places in the cache for later steps and, once that page has arrived, over the same places in the ring.  Two launches and one, in
+// a graph, us: 4 x 333 keys of 2 key heads 6.87 -> 5.68, 64 x 60 of 4 8.8 -> 7.0, 64 x 8192 154.1 -> 152.4, 256 x 300 42.3 -> 37.9; with the partials asked for
+// only after the pages 6.59 where it is 5.68 (and 198 registers, one CTA on an SM: 64 x 60 11.0).
+template <int kRows>   // 0: q and the cache are ready; else rows of a thread, 5 for up to eight heads and 9 for 16
+__global__ void __launch_bounds__(kThreads + 32, 2)   // 168 registers: three warps of two CTAs share a quarter of an SM
+paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p, int n_st, NewToken nt_) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - ptx::smem_u32(smem_raw));
@@ -86,14 +102,48 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_launch_dependents();
+  const int R = p.R;
+  // kNew: a consumer thread has the pair (i, i + 64), i = its number mod 64, of every second row; rows 0 .. R - 1: q heads, then k and v.  What
+  // needs no wait is read before it, and the sums of the partials do not wait for the sequence's length and pages.
+  constexpr bool kNew = kRows > 0;
+  float x1[kRows + !kNew], x2[kRows + !kNew], inv_freq = 0.f;
+  __nv_bfloat16 b1[kRows + !kNew], b2[kRows + !kNew];
+  const auto column = [&](int j) {
+    const int r = ((int)threadIdx.x >> 6) + 2 * j;
+    return (r < R ? kvh * R + r : p.n_q + (r - R) * p.n_kv + kvh) * kD + (int)(threadIdx.x & 63);
+  };
+  const auto mine = [&](int j) { return ((int)threadIdx.x >> 6) + 2 * j < R + 2; };
+  if (kNew && warp < kConsumers) {
+    inv_freq = nt_.inv_freq[threadIdx.x & 63];
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+      x1[j] = x2[j] = 0.f;
+      b1[j] = b2[j] = __nv_bfloat16();
+      if (nt_.bias && mine(j)) {
+        b1[j] = nt_.bias[column(j)];
+        b2[j] = nt_.bias[column(j) + 64];
+      }
+    }
+  }
   pdl_wait();  // q, the current token's K/V and the scheduler state come from the preceding kernels
   const int seq_len = p.seq_lens[b];
+  if (kNew && warp < kConsumers) {
+    const int64_t ncol = (int64_t)(p.n_q + 2 * p.n_kv) * kD;
+    const float* src = nt_.part + (int64_t)b * ncol;
+#pragma unroll 2
+    for (int s = 0; s < nt_.n_split; ++s, src += nt_.B * ncol)
+#pragma unroll
+      for (int j = 0; j < kRows; ++j)
+        if (mine(j)) {
+          x1[j] += src[column(j)];
+          x2[j] += src[column(j) + 64];
+        }
+  }
   const int n_pages_b = (seq_len + kPage - 1) / kPage;
   const int per_split = (n_pages_b + p.n_splits - 1) / p.n_splits;
   const int p_begin = split * per_split;
   const int p_end = (p_begin + per_split < n_pages_b) ? p_begin + per_split : n_pages_b;
   const int n_it = p_end > p_begin ? p_end - p_begin : 0;
-  const int R = p.R;
 
   auto store = [&](int r, int d, float O, float M, float L) {
     const int64_t head = (int64_t)b * p.n_q + kvh * R + r;
@@ -159,6 +209,10 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p
   for (int i = 0; i < 16; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
   const int g = lane >> 2, t = lane & 3;
 
+  __shared__ __align__(16) __nv_bfloat16 s_q[kNew ? 16 * kQRow : 8];
+  __shared__ __align__(16) __nv_bfloat16 s_kv[kNew ? 2 * kD : 8];
+  const bool last_here = kNew && p_end == n_pages_b;     // the page that the token is written to
+
   if (warp == kConsumers) {
     // ===== producer: TMA whole pages into the ring =====
     if (lane == 0) {
@@ -182,15 +236,43 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p
     // ===== consumers =====
     // Q fragments (A operand, rows = the R heads sharing this kv head, zero-padded to 16)
     uint32_t qa[8][4];
+    if constexpr (kNew) {
+      const int i = threadIdx.x & 63, pos = seq_len - 1;
+      const int rows = last_here ? R + 2 : R, r0 = threadIdx.x >> 6;
+      float sn, cs;
+      sincosf((float)pos * inv_freq, &sn, &cs);
+#pragma unroll
+      for (int j = 0; j < kRows; ++j) {
+        const int r = r0 + 2 * j;
+        if (r >= rows) break;
+        if (nt_.bias) {
+          x1[j] += __bfloat162float(b1[j]);
+          x2[j] += __bfloat162float(b2[j]);
+        }
+        const bool turn = r <= R;                                    // not v
+        const __nv_bfloat16 o1 = __float2bfloat16_rn(turn ? rot_first(x1[j], x2[j], cs, sn) : x1[j]);
+        const __nv_bfloat16 o2 = __float2bfloat16_rn(turn ? rot_second(x1[j], x2[j], cs, sn) : x2[j]);
+        __nv_bfloat16* dst = r < R ? s_q + r * kQRow : s_kv + (r - R) * kD;
+        dst[i] = o1;
+        dst[i + 64] = o2;
+        if (r >= R) {
+          const int64_t row = (((int64_t)(p.layer * 2 + (r - R)) * p.n_pages + s_pages[n_it - 1]) * p.n_kv + kvh) * kPage + pos % kPage;
+          nt_.kv_cache[row * kD + i] = o1;
+          nt_.kv_cache[row * kD + i + 64] = o2;
+        }
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(kConsumers * 32) : "memory");
+    }
     {
-      const __nv_bfloat16* qb = p.q + ((int64_t)b * p.n_q + kvh * R) * kD;
+      const __nv_bfloat16* qb = kNew ? s_q : p.q + ((int64_t)b * p.n_q + kvh * R) * kD;
+      constexpr int ld = kNew ? kQRow : kD;
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks) {
         const int c = ks * 16 + 2 * t;
-        qa[ks][0] = (g < R) ? *reinterpret_cast<const uint32_t*>(qb + g * kD + c) : 0u;
-        qa[ks][1] = (g + 8 < R) ? *reinterpret_cast<const uint32_t*>(qb + (g + 8) * kD + c) : 0u;
-        qa[ks][2] = (g < R) ? *reinterpret_cast<const uint32_t*>(qb + g * kD + c + 8) : 0u;
-        qa[ks][3] = (g + 8 < R) ? *reinterpret_cast<const uint32_t*>(qb + (g + 8) * kD + c + 8) : 0u;
+        qa[ks][0] = (g < R) ? *reinterpret_cast<const uint32_t*>(qb + g * ld + c) : 0u;
+        qa[ks][1] = (g + 8 < R) ? *reinterpret_cast<const uint32_t*>(qb + (g + 8) * ld + c) : 0u;
+        qa[ks][2] = (g < R) ? *reinterpret_cast<const uint32_t*>(qb + g * ld + c + 8) : 0u;
+        qa[ks][3] = (g + 8 < R) ? *reinterpret_cast<const uint32_t*>(qb + (g + 8) * ld + c + 8) : 0u;
       }
     }
     const int mi = lane >> 3, lr = lane & 7;
@@ -200,6 +282,15 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap tm_kv, AttnParams p
       ptx::mbar_wait(full_bar(s), ph);
       const uint32_t kbase = base + (uint32_t)(s * kStageBytes);
       const uint32_t vbase = kbase + 16384;
+      if (kNew && last_here && it == n_it - 1) {          // the token's k and v, by the warp that reads their row
+        const int row = (seq_len - 1) % kPage, chunk = lane & 15;
+        if (row / 16 == warp) {
+          const uint4 v = *reinterpret_cast<const uint4*>(s_kv + (lane >> 4) * kD + chunk * 8);
+          const uint32_t at = (lane < 16 ? kbase : vbase) + (uint32_t)((chunk >> 3) * 8192 + row * 128 + (((chunk & 7) ^ (row & 7)) << 4));
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+          __syncwarp();
+        }
+      }
 
       // ---- S = Q K^T over this warp's 16 tokens ----
       float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
@@ -554,12 +645,11 @@ extern "C" size_t prl_paged_attn_workspace_bytes(int32_t B, int32_t n_q, int32_t
   return (size_t)B * n_q * n_splits * (kD + 2) * sizeof(float) + (size_t)B * n_q * sizeof(unsigned int);
 }
 
-extern "C" int prl_paged_attn_decode(const void* q, const void* kv_cache, int64_t n_pages, int32_t n_layers,
-                                     int32_t layer, const int32_t* block_table, int32_t max_blocks,
-                                     const int32_t* seq_lens, int32_t B, int32_t n_q, int32_t n_kv, int32_t head_dim,
-                                     int32_t page_size, int32_t n_splits, float sm_scale, void* out_bf16,
-                                     void* workspace, size_t workspace_bytes, prl_stream_t stream_) {
-  PRL_CHECK_ARG(q && kv_cache && block_table && seq_lens && out_bf16 && workspace, "prl_paged_attn_decode: NULL argument");
+static int paged_attn_decode_impl(const void* q, const NewToken& fresh, const void* kv_cache, int64_t n_pages, int32_t n_layers, int32_t layer,
+                                  const int32_t* block_table, int32_t max_blocks, const int32_t* seq_lens, int32_t B, int32_t n_q, int32_t n_kv,
+                                  int32_t head_dim, int32_t page_size, int32_t n_splits, float sm_scale, void* out_bf16, void* workspace,
+                                  size_t workspace_bytes, prl_stream_t stream_) {
+  PRL_CHECK_ARG((q || fresh.part) && kv_cache && block_table && seq_lens && out_bf16 && workspace, "prl_paged_attn_decode: NULL argument");
   PRL_CHECK_ARG(head_dim == kD && page_size == kPage, "prl_paged_attn_decode: head_dim must be 128 and page_size 64");
   PRL_CHECK_ARG(B >= 1 && n_kv >= 1 && n_q % n_kv == 0 && n_q / n_kv <= 16, "prl_paged_attn_decode: need n_q/n_kv <= 16");
   PRL_CHECK_ARG(n_splits >= 1 && layer >= 0 && layer < n_layers, "prl_paged_attn_decode: bad layer/splits");
@@ -589,11 +679,13 @@ extern "C" int prl_paged_attn_decode(const void* q, const void* kv_cache, int64_
   // merge under the other's pages (us: 64 x 600 keys of 4 heads by two 25.8 -> 21.6, 64 x 200 12.6 -> 10.1, 64 x 7000 by two 133 -> 128)
   const int n_st = (int64_t)n_splits * n_kv * B > num_sms() ? kStages / 2 : kStages;
   const int smem = n_st * kStageBytes + 1024 + 8 * 2 * n_st + 4 * kMaxPagesPerSplit + 16;
-  static SmemAttr smem_attr = {};
-  PRL_CUDA(ensure_smem(paged_attn_decode_kernel, smem, smem_attr));
+  static SmemAttr smem_attr[3] = {};
+  const int form = fresh.part ? (p.R <= 8 ? 1 : 2) : 0;
+  const auto kernel = form == 1 ? paged_attn_decode_kernel<5> : form == 2 ? paged_attn_decode_kernel<9> : paged_attn_decode_kernel<0>;
+  PRL_CUDA(ensure_smem(kernel, smem, smem_attr[form]));
   cudaStream_t stream = (cudaStream_t)stream_;
   dim3 grid((unsigned)n_splits, (unsigned)n_kv, (unsigned)B);
-  PRL_CUDA(launch_pdl(paged_attn_decode_kernel, grid, dim3(kThreads), (size_t)smem, stream, tm, p, n_st));
+  PRL_CUDA(launch_pdl(kernel, grid, dim3(kThreads), (size_t)smem, stream, tm, p, n_st, fresh));
   PRL_LAUNCH_CHECK();
   if (!g_fused_combine && !p.direct) {
     PRL_CUDA(launch_pdl(attn_combine_kernel, dim3((unsigned)(B * n_q)), dim3(kD), 0, stream, (const float*)p.o_part,
@@ -601,6 +693,27 @@ extern "C" int prl_paged_attn_decode(const void* q, const void* kv_cache, int64_
     PRL_LAUNCH_CHECK();
   }
   return PRL_OK;
+}
+
+extern "C" int prl_paged_attn_decode(const void* q, const void* kv_cache, int64_t n_pages, int32_t n_layers,
+                                     int32_t layer, const int32_t* block_table, int32_t max_blocks,
+                                     const int32_t* seq_lens, int32_t B, int32_t n_q, int32_t n_kv, int32_t head_dim,
+                                     int32_t page_size, int32_t n_splits, float sm_scale, void* out_bf16,
+                                     void* workspace, size_t workspace_bytes, prl_stream_t stream_) {
+  PRL_CHECK_ARG(q != nullptr, "prl_paged_attn_decode: NULL argument");
+  return paged_attn_decode_impl(q, NewToken{}, kv_cache, n_pages, n_layers, layer, block_table, max_blocks, seq_lens, B, n_q, n_kv, head_dim,
+                                page_size, n_splits, sm_scale, out_bf16, workspace, workspace_bytes, stream_);
+}
+
+extern "C" int prl_paged_attn_decode_qkv(const float* partials, int32_t n_split, const void* bias, const float* inv_freq, void* kv_cache,
+                                         int64_t n_pages, int32_t n_layers, int32_t layer, const int32_t* block_table, int32_t max_blocks,
+                                         const int32_t* seq_lens, int32_t B, int32_t n_q, int32_t n_kv, int32_t head_dim, int32_t page_size,
+                                         int32_t n_splits, float sm_scale, void* out_bf16, void* workspace, size_t workspace_bytes,
+                                         prl_stream_t stream_) {
+  PRL_CHECK_ARG(partials && n_split >= 1 && inv_freq, "prl_paged_attn_decode_qkv: bad argument");
+  const NewToken fresh{partials, n_split, B, (const __nv_bfloat16*)bias, inv_freq, (__nv_bfloat16*)kv_cache};
+  return paged_attn_decode_impl(nullptr, fresh, kv_cache, n_pages, n_layers, layer, block_table, max_blocks, seq_lens, B, n_q, n_kv, head_dim,
+                                page_size, n_splits, sm_scale, out_bf16, workspace, workspace_bytes, stream_);
 }
 
 extern "C" int prl_paged_attn_prefill(const void* q, const void* kv_cache, int64_t n_pages, int32_t n_layers,

@@ -153,6 +153,10 @@ __device__ __forceinline__ float div_ge1(float a, float b) {
   return fabsf(rem) > 0.f ? fmaf(rem, r, q) : q;
 }
 
+// the rotated pair, contracted one way in every kernel
+__device__ __forceinline__ float rot_first(float a, float c, float cs, float sn) { return fmaf(a, cs, -__fmul_rn(c, sn)); }
+__device__ __forceinline__ float rot_second(float a, float c, float cs, float sn) { return fmaf(c, cs, __fmul_rn(a, sn)); }
+
 __device__ __forceinline__ float bf16_bits_to_float(uint32_t hi16) {
   return __uint_as_float(hi16 << 16);
 }

@@ -666,7 +666,13 @@ class DecodeEngine(EngineCore):
             p = f"layers.{l}."
             if "gemm" not in skip:
                 self._gemm(p + "qkv_proj.weight", self.x, cfg.qkv_size, H, self.split_k["qkv"], part)
-            if "small" not in skip:
+            if not skip and not pf:
+                _lib.check(lib.prl_paged_attn_decode_qkv(part.data_ptr(), self.split_k["qkv"], a.ptr(p + "qkv_proj.bias") if cfg.qkv_bias else None,
+                                                         self.inv_freq.data_ptr(), self.kv_cache.data_ptr(), self.n_pages, cfg.num_layers, l,
+                                                         self.block_table.data_ptr(), self.max_blocks, self.seq_lens.data_ptr(), B,
+                                                         cfg.num_q_heads, cfg.num_kv_heads, cfg.head_dim, PAGE_SIZE, self.attn_splits, sm_scale,
+                                                         self.attn_out.data_ptr(), self.attn_ws.data_ptr(), self.attn_ws.numel(), st))
+            elif "small" not in skip:
                 # while attention streams the KV cache, L2 fetches o_proj's weights
                 _lib.check(lib.prl_qkv_rope_cache(part.data_ptr(), self.split_k["qkv"], B,
                                                   a.ptr(p + "qkv_proj.bias") if cfg.qkv_bias else None, cfg.num_q_heads,
@@ -675,7 +681,7 @@ class DecodeEngine(EngineCore):
                                                   self.inv_freq.data_ptr(), self.q.data_ptr(), self.kv_cache.data_ptr(),
                                                   self.n_pages, l, PAGE_SIZE,
                                                   a.ptr(p + "o_proj.weight") if pf else None, wbytes(p + "o_proj.weight"), st))
-            if "attn" not in skip:
+            if (skip or pf) and "attn" not in skip:
                 _lib.check(lib.prl_paged_attn_decode(self.q.data_ptr(), self.kv_cache.data_ptr(), self.n_pages,
                                                      cfg.num_layers, l, self.block_table.data_ptr(), self.max_blocks,
                                                      self.seq_lens.data_ptr(), B, cfg.num_q_heads, cfg.num_kv_heads,

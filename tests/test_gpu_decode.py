@@ -563,3 +563,38 @@ def test_attention_of_one_split_writes_the_output(cuda_device, R, n_kv):
         w = torch.softmax(torch.einsum("grd,gsd->grs", q[b].view(n_kv, R, D).double(), K) * D ** -0.5, -1)
         want, bound = torch.einsum("grs,gsd->grd", w, V), torch.einsum("grs,gsd->grd", w, V.abs())
         assert ((out[b].double() - want).abs() <= 2.0 ** -7 * bound + 1e-30).all(), l
+
+
+@pytest.mark.parametrize("lens,R,n_kv,n_split,key_splits,bias", [((1,), 1, 1, 1, 1, True), ((64, 0, 65), 7, 4, 2, 1, True), ((63, 128, 1, 200), 8, 2, 3, 1, False),
+                                                                  ((700, 65, 0, 129), 9, 2, 8, 4, True), ((40, 641), 16, 1, 5, 2, True), ((96,) * 90, 4, 4, 1, 1, True)])
+def test_attention_from_the_projection_equals_two_launches(cuda_device, lens, R, n_kv, n_split, key_splits, bias):
+    """q, k and v made in the attention kernel: the output and the cache of prl_qkv_rope_cache and prl_paged_attn_decode, bit for bit; a row
+    without a token writes nothing."""
+    from pipelinerl_b200 import _lib
+    lib, dev, g = _lib.load(), cuda_device, torch.Generator().manual_seed(sum(lens) + R)
+    B, n_q, mb, L, layer = len(lens), R * n_kv, (max(lens) + 63) // 64 + 1, 2, 1
+    pages = 1 + B * mb
+    bt = (1 + torch.randperm(B * mb, generator=g)).to(torch.int32).view(B, mb).to(dev)
+    sl = torch.tensor(lens, dtype=torch.int32, device=dev)
+    pos = (sl - 1).clamp_min(0)
+    kv0 = torch.randn(L * 2 * pages * n_kv * 64 * 128, generator=g).to(torch.bfloat16).to(dev)
+    part = torch.randn(n_split, B, (n_q + 2 * n_kv) * 128, generator=g).to(dev)
+    bi = torch.randn((n_q + 2 * n_kv) * 128, generator=g).to(torch.bfloat16).to(dev) if bias else None
+    inv = (1.0 / (1e6 ** (torch.arange(0, 128, 2).float() / 128))).to(dev)
+    ws = torch.zeros(int(lib.prl_paged_attn_workspace_bytes(B, n_q, key_splits)), dtype=torch.uint8, device=dev)
+    p = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+    two, one = kv0.clone(), kv0.clone()
+    q, want, got = (torch.full((B, n_q * 128), 7.0, dtype=torch.bfloat16, device=dev) for _ in range(3))
+    tail = (B, n_q, n_kv, 128, 64, key_splits, 128 ** -0.5)
+    _lib.check(lib.prl_qkv_rope_cache(p(part), n_split, B, p(bi), n_q, n_kv, 128, p(pos), p(bt), mb, None, p(inv), p(q), p(two), pages, layer, 64, None, 0,
+                                      _lib.stream_ptr()))
+    _lib.check(lib.prl_paged_attn_decode(p(q), p(two), pages, L, layer, p(bt), mb, p(sl), *tail, p(want), p(ws), ws.numel(), _lib.stream_ptr()))
+    _lib.check(lib.prl_paged_attn_decode_qkv(p(part), n_split, p(bi), p(inv), p(one), pages, L, layer, p(bt), mb, p(sl), *tail, p(got), p(ws), ws.numel(),
+                                             _lib.stream_ptr()))
+    assert torch.equal(got, want)
+    for b, n in enumerate(lens):
+        if n == 0:                                   # the two launches write a row without a token to its first page
+            for t in (two, kv0):
+                t.view(L, 2, pages, n_kv, 64, 128)[layer, :, bt[b, 0].item(), :, 0] = 0
+            one.view(L, 2, pages, n_kv, 64, 128)[layer, :, bt[b, 0].item(), :, 0] = 0
+    assert torch.equal(one, two) and not torch.equal(one, kv0)
