@@ -18,7 +18,7 @@
 //     prl_attn_set_fused_combine), A/B measured in profiles/r1_ablation*.jsonl.  Splits as one cluster that merges through its
 //     shared memory were slower where it counts (64 x 8192: 1498 -> 1515 us a step of four layers).
 // KV cache layout (bf16): row = (((layer*2 + kv) * n_pages + page) * n_kv + kvh) * 64 + slot,
-// 128 contiguous d per row — written by qkv_rope_cache_kernel (decode_ops.cu).
+// 128 contiguous d per row — written by qkv_rope_cache_kernel (decode_ops.cu), or here from the projection's partials.
 #include "prl_common.cuh"
 #include "tc_ptx.cuh"
 #include <math.h>

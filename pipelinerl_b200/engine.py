@@ -3,7 +3,7 @@
 This is what replaces the vLLM server of the reference for hot path 1 (launch:
 pipelinerl/launch.py:191-247; per-request client: pipelinerl/async_llm.py:86-212).  One engine
 owns one GPU: a parameter arena (model.ParamArena), a paged KV pool, device-resident per-slot
-scheduler state, and a CUDA graph of the whole token step (all ~290 kernel launches of a 28-layer
+scheduler state, and a CUDA graph of the whole token step (all ~230 kernel launches of a 28-layer
 model replayed with one call).  The host only admits requests into free slots and harvests
 finished ones; token feeding, sampling, logprob capture and retirement happen on the device
 (prl_advance_state), so there is no per-token host round trip.
