@@ -5,6 +5,7 @@
 // Reductions over the token dimension (RMSNorm gain, qkv bias) are two-stage with a FIXED order: per-block partial
 // rows in a workspace, then one pass that adds them into the fp32 gradient arena -> bitwise reproducible.
 #include "prl_common.cuh"
+#include "tc_ptx.cuh"
 
 namespace prl {
 namespace {
@@ -70,6 +71,53 @@ __device__ __forceinline__ void load_row(const __nv_bfloat16* __restrict__ p, in
   }
 }
 
+// The backward's rows of up to three matrices on their way into shared memory, `slots` rows of the block's walk ahead: a thread asks for whole rows
+// (bulk copies), so what is under way does not hang on the registers (one row ahead: 48 KB an SM).  A row's slot is asked for again
+// once the block's sum has brought all threads past their reads.
+struct RowRing {
+  uint32_t data, bars;
+  uint32_t row_bytes, slot_bytes;
+  int slots, mats;
+  const __nv_bfloat16* src[3];
+  __device__ __forceinline__ void ask(int64_t row, int H, int s) const {        // one thread
+    const uint32_t bar = bars + 8u * (uint32_t)s;
+    ptx::mbar_arrive_expect_tx(bar, row_bytes * (uint32_t)mats);
+    for (int m = 0; m < mats; ++m)
+      ptx::bulk_load_1d(data + (uint32_t)s * slot_bytes + (uint32_t)m * row_bytes, src[m] + row * H, row_bytes, bar, ptx::kEvictFirst);
+  }
+  __device__ __forceinline__ void start(int64_t T, int H) const {
+    if (threadIdx.x == 0) {
+      for (int s = 0; s < slots; ++s) ptx::mbar_init(bars + 8u * (uint32_t)s, 1);
+      ptx::fence_barrier_init();
+      ptx::fence_proxy_async();
+      int64_t row = blockIdx.x;
+      for (int s = 0; s < slots && row < T; ++s, row += gridDim.x) ask(row, H, s);
+    }
+    __syncthreads();
+  }
+  template <int kVec>
+  __device__ __forceinline__ void get(int s, int m, int nvec, uint4 (&r)[kVec]) const {
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) {
+      const int v = threadIdx.x + i * blockDim.x;
+      if (v < nvec)
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[i].x), "=r"(r[i].y), "=r"(r[i].z), "=r"(r[i].w)
+                     : "r"(data + (uint32_t)s * slot_bytes + (uint32_t)m * row_bytes + (uint32_t)v * 16u) : "memory");
+    }
+  }
+};
+__device__ __forceinline__ RowRing row_ring(uint8_t* raw, int H, int slots, int mats) {
+  RowRing r;
+  const uint32_t base = (ptx::smem_u32(raw) + 127u) & ~127u;
+  r.bars = base;
+  r.data = base + 128u;
+  r.row_bytes = 2u * (uint32_t)H;
+  r.slot_bytes = r.row_bytes * (uint32_t)mats;
+  r.slots = slots;
+  r.mats = mats;
+  return r;
+}
+
 // y = bf16(x * rstd) * gamma  (the rounding order of HF's Qwen2RMSNorm); rstd kept for the backward
 template <int kVec>
 __global__ void __launch_bounds__(kRowThreads) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
@@ -113,11 +161,12 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_fwd_kernel(const __nv_bfl
 }
 
 // dx = dres + rstd * (dy*gamma - xhat * mean(dy*gamma*xhat));  partial[block][c] = sum over this block's rows of dy*xhat
-template <int kVec>
+template <int kVec, bool kRing>
 __global__ void __launch_bounds__(kRowThreads, kVec == 1 ? 4 : (kVec == 2 ? 2 : 1))
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ rstd,
                    const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ dres, int64_t T, int H,
-                   __nv_bfloat16* __restrict__ dx, float* __restrict__ partial) {
+                   __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int slots) {
+  extern __shared__ uint8_t row_raw[];
   __shared__ float s_red[2][kRowThreads / 32];
   const int nvec = H >> 3;
   uint4 g[kVec], xn[kVec], dn[kVec], sn[kVec];
@@ -128,23 +177,41 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[i].v[e] = 0.f;
   }
+  RowRing ring = row_ring(row_raw, H, slots, dres ? 3 : 2);
+  ring.src[0] = x;
+  ring.src[1] = dy;
+  ring.src[2] = dres;
+  if (kRing) ring.start(T, H);
   load_row<kVec>(gamma, 0, H, g);
-  load_row<kVec>(x, blockIdx.x, H, xn);
-  load_row<kVec>(dy, blockIdx.x, H, dn);
-  if (dres) load_row<kVec>(dres, blockIdx.x, H, sn);
+  if (!kRing) {
+    load_row<kVec>(x, blockIdx.x, H, xn);
+    load_row<kVec>(dy, blockIdx.x, H, dn);
+    if (dres) load_row<kVec>(dres, blockIdx.x, H, sn);
+  }
   float rn = rstd[blockIdx.x];
-  int buf = 0;
+  int buf = 0, slot = 0;
+  uint32_t ph = 0;
   for (int64_t row = blockIdx.x; row < T; row += gridDim.x, buf ^= 1) {
     uint4 xr[kVec], dr[kVec], sr[kVec];
     const float r = rn;
-#pragma unroll
-    for (int i = 0; i < kVec; ++i) { xr[i] = xn[i]; dr[i] = dn[i]; sr[i] = sn[i]; }
     const int64_t nx = row + gridDim.x;
-    if (nx < T) {
-      load_row<kVec>(x, nx, H, xn);
-      load_row<kVec>(dy, nx, H, dn);
-      if (dres) load_row<kVec>(dres, nx, H, sn);
-      rn = rstd[nx];
+    if constexpr (kRing) {
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) sr[i] = sn[i];
+      if (nx < T) rn = rstd[nx];
+      ptx::mbar_wait(ring.bars + 8u * (uint32_t)slot, ph);
+      ring.get<kVec>(slot, 0, nvec, xr);
+      ring.get<kVec>(slot, 1, nvec, dr);
+      if (dres) ring.get<kVec>(slot, 2, nvec, sr);
+    } else {
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) { xr[i] = xn[i]; dr[i] = dn[i]; sr[i] = sn[i]; }
+      if (nx < T) {
+        load_row<kVec>(x, nx, H, xn);
+        load_row<kVec>(dy, nx, H, dn);
+        if (dres) load_row<kVec>(dres, nx, H, sn);
+        rn = rstd[nx];
+      }
     }
     float dot = 0.f;
 #pragma unroll
@@ -160,6 +227,11 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
       }
     }
     const float m = block_sum(dot, s_red[buf]) / (float)H;
+    if constexpr (kRing) {
+      const int64_t ahead = row + (int64_t)ring.slots * gridDim.x;
+      if (threadIdx.x == 0 && ahead < T) ring.ask(ahead, H, slot);
+      if (++slot == ring.slots) { slot = 0; ph ^= 1u; }
+    }
 #pragma unroll
     for (int i = 0; i < kVec; ++i) {
       const int v = threadIdx.x + i * blockDim.x;
@@ -389,6 +461,18 @@ int row_bwd_grid(int64_t T, int64_t H) {
   const int64_t most = n < kPartialBlocks ? n : kPartialBlocks;
   return (int)(T < most ? T : most);
 }
+// Slots of the backward's ring: what an SM's shared memory holds beside its other blocks, 16 at most; 0: rows through registers.  The ring pays
+// where a block has many rows to be ahead of (it costs a start, and the SM another split of its L1) and rows are whole lines.  Rows, registers /
+// ring, us: 3584 channels (two blocks an SM) 4096 25.0 / 27.9, 8192 43.5 / 43.9, 12000 63.9 / 62.0, 16384 84.0 / 81.0, 32768 158 / 150; 5120 (one) 4096 35.1 / 37.2,
+// 6000 51.6 / 49.5, 16384 132 / 118; 2048 (four) 4096 20.8 / 20.9, 6000 26.9 / 26.0, 16384 55.8 / 51.9; 128 12000 18.7 / 16.7; 2056 16384 65.6 / 67.8; 4096,
+// where two blocks have four slots each, 32768 173 / 177.  The forward lost throughout (16384 x 3584 43.4 / 46.1): one row in flight a block was enough.
+int ring_slots(int64_t T, int64_t H, int64_t grid, int mats) {
+  const int vecs = row_vecs(H);
+  if (H % 64 != 0 || T < (vecs == 1 ? 10 : 40) * grid) return 0;
+  const int64_t per_sm = (grid + num_sms() - 1) / num_sms(), n = (216 * 1024 / per_sm - 1536) / (2 * H * mats);
+  return (int)(n < (vecs == 2 ? 5 : 4) ? 0 : n > 16 ? 16 : n);
+}
+int ring_bytes(int64_t H, int slots, int mats) { return slots ? (int)(256 + 2 * H * mats * slots) : 0; }
 cudaError_t launch_partial_reduce(const float* ws, int blocks, int64_t cols, float* out, cudaStream_t stream) {
   return launch_pdl(partial_reduce_kernel, dim3((unsigned)((cols + 31) / 32)), dim3(32 * kReduceWarps), 0, stream, ws, blocks, (int)cols, out);
 }
@@ -426,11 +510,20 @@ extern "C" int prl_rmsnorm_bwd(const void* x, const void* gamma, const float* rs
   PRL_ROW_ARGS("prl_rmsnorm_bwd", H);
   PRL_CHECK_ARG(workspace_bytes >= prl_rowops_workspace_bytes(H), "prl_rmsnorm_bwd: workspace too small");
   const int g = row_bwd_grid(T, H), threads = row_threads(H);
-#define PRL_BWD(V) rmsnorm_bwd_kernel<V><<<g, threads, 0, (cudaStream_t)stream>>>( \
-      (const __nv_bfloat16*)x, (const __nv_bfloat16*)gamma, rstd, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)dres, T, \
-      (int)H, (__nv_bfloat16*)dx, (float*)workspace)
+  const int mats = dres ? 3 : 2;
+  const int slots = ring_slots(T, H, g, mats), smem = ring_bytes(H, slots, mats);
+#define PRL_BWD_(V, RING)                                                                                                         \
+  do {                                                                                                                            \
+    static SmemAttr attr = {};                                                                                                    \
+    if (RING) PRL_CUDA(ensure_smem((rmsnorm_bwd_kernel<V, RING>), smem, attr));                                                   \
+    rmsnorm_bwd_kernel<V, RING><<<g, threads, smem, (cudaStream_t)stream>>>(                                                      \
+        (const __nv_bfloat16*)x, (const __nv_bfloat16*)gamma, rstd, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)dres, T,      \
+        (int)H, (__nv_bfloat16*)dx, (float*)workspace, slots);                                                                    \
+  } while (0)
+#define PRL_BWD(V) do { if (slots) PRL_BWD_(V, true); else PRL_BWD_(V, false); } while (0)
   switch (row_vecs(H)) { case 1: PRL_BWD(1); break; case 2: PRL_BWD(2); break; case 3: PRL_BWD(3); break; default: PRL_BWD(4); }
 #undef PRL_BWD
+#undef PRL_BWD_
   PRL_LAUNCH_CHECK();
   PRL_CUDA(launch_partial_reduce((const float*)workspace, g, H, dgamma, (cudaStream_t)stream));
   PRL_LAUNCH_CHECK();

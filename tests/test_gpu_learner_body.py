@@ -442,3 +442,23 @@ def test_activation_beside_its_backward(cuda_device, T, I):
     dgu, act = o.silu_mul_bwd_act(gu, da)
     assert act.data_ptr() == da.data_ptr()
     assert torch.equal(act.view(torch.int16), want_act.view(torch.int16)) and torch.equal(dgu.view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("T,H", [(12003, 3584), (6007, 2048), (11841, 896), (12001, 128), (6001, 5120), (6000, 8192), (5920, 1088)])
+@pytest.mark.parametrize("res", [True, False])
+def test_norm_backward_of_rows_ahead(cuda_device, T, H, res):
+    """Many rows per block come through a ring: each row's gradient has the bits of the same row among few; the gain's gradient against 64 bits,
+    a sum of T products in fp32 by at most T / blocks + blocks additions."""
+    from pipelinerl_b200.learner_body import Ops
+    o, g = Ops(), torch.Generator(device=cuda_device).manual_seed(T + H)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=cuda_device).to(torch.bfloat16)  # noqa: E731
+    x, dy, gamma = rnd(T, H), rnd(T, H), rnd(H)
+    dr = rnd(T, H) if res else None
+    _, rstd = o.rmsnorm(x, gamma, 1e-6)
+    dg = torch.zeros(H, device=cuda_device)
+    dx = o.rmsnorm_bwd(x, gamma, rstd, dy, dr, dg)
+    few = torch.cat([o.rmsnorm_bwd(x[i:i + 900], gamma, rstd[i:i + 900].contiguous(), dy[i:i + 900], dr[i:i + 900] if res else None, torch.zeros(H, device=cuda_device))
+                     for i in range(0, T, 900)])
+    assert torch.equal(dx, few)
+    terms = dy.double() * x.double() * rstd.double()[:, None]
+    assert ((dg.double() - terms.sum(0)).abs() <= 2.0 ** -24 * (T / 148 + 1200) * terms.abs().sum(0)).all()
