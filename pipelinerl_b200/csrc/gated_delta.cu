@@ -391,6 +391,7 @@ __global__ void __launch_bounds__(kThreads, U == 1 ? 3 : 2) gated_delta_front_ti
   };
   if (h < 2 * a.kh + H) taps_of(0);
   pdl_wait();
+  pdl_launch_dependents();
   int slot[RT], back[RT];
 #pragma unroll
   for (int r = 0; r < RT; ++r) {
@@ -502,6 +503,8 @@ __device__ __forceinline__ int blk_at(int b, int q) { return (b * (b + 1) / 2 + 
 
 __global__ void __launch_bounds__(kPieceThreads, 2) gated_delta_piece_kernel(SplitArgs a) {
   pdl_wait();
+  pdl_launch_dependents();   // here, in the front rows, the closing rows and the experts' gather: a prompt of 2500 tokens 2436 -> 2393 us (in the walk, the
+                             // read-out and the token step too: 2402, and 564 -> 572 a token step of 32 rows: the next kernel's blocks take their SMs' room)
   extern __shared__ __align__(16) float sm[];
   const int piece = blockIdx.x, head = blockIdx.y, len = a.sub_len[piece];
   const int64_t row0 = a.sub_start[piece];

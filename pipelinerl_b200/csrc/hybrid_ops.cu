@@ -39,8 +39,9 @@ __device__ __forceinline__ float silu_f(float x) { return x / (1.f + expf(-x)); 
 template <typename T>
 __global__ void embed_scale_kernel(const int32_t* __restrict__ tokens, const T* __restrict__ embed, float scale, int W,
                                    int vocab, float* __restrict__ x, T* __restrict__ xa) {
-  pdl_wait();   // launched with the programmatic-serialization attribute like the engine's other step kernels; no early
-                // trigger: letting the next grid become resident early measured +3 ms on a 4096-token prefill and +-0 on decode
+  pdl_wait();
+  pdl_launch_dependents();   // behind the wait, so that what the next kernel reads ahead of its own is complete; the hybrids' small row kernels
+                             // and the experts' grouping together: 32 x 1100, 4 layers 573 -> 561 us, a prompt of 2500 tokens 2463 -> 2436
   const int r = blockIdx.x;
   int tok = tokens[r];
   tok = tok < 0 ? 0 : (tok >= vocab ? vocab - 1 : tok);
@@ -96,8 +97,8 @@ __global__ void postnorm_residual_kernel(const float* __restrict__ y0, int64_t l
 template <typename T>
 __global__ void rmsnorm_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows,
                                     const float* __restrict__ gain, float eps, int W, T* __restrict__ out) {
-  pdl_wait();   // launched with the programmatic-serialization attribute like the engine's other step kernels; no early
-                // trigger: letting the next grid become resident early measured +3 ms on a 4096-token prefill and +-0 on decode
+  pdl_wait();
+  pdl_launch_dependents();   // behind the wait, so that what the next kernel reads ahead of its own is complete
   __shared__ float red[32];
   const int i = blockIdx.x;
   const int64_t r = rows ? rows[i] : i;
@@ -532,6 +533,7 @@ __global__ void sublayer_close_rows_kernel(const float* __restrict__ y0, int64_t
                                           const float* __restrict__ next_gain, float eps, int W, float* __restrict__ x,
                                           T* __restrict__ xa) {
   pdl_wait();
+  pdl_launch_dependents();
   __shared__ float red[32];
   const int64_t r = blockIdx.x, at = r * W;
   const int n4 = W / 4;
@@ -1249,6 +1251,7 @@ __global__ void __launch_bounds__(1024) attn_front_lanes_kernel(
 // z <- cap * tanh(z / cap): the model's capped logits, in place
 __global__ void soft_cap_kernel(float* __restrict__ z, int64_t count, float cap) {
   pdl_wait();
+  pdl_launch_dependents();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x)
     z[i] = cap * tanhf(z[i] / cap);
 }

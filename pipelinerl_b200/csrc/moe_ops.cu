@@ -465,6 +465,7 @@ __global__ void __launch_bounds__(32 * kGroupWarps) moe_group_runs_kernel(const 
                                                                          int32_t* __restrict__ perm, int32_t* __restrict__ meta,
                                                                          int32_t* __restrict__ tiles) {
   pdl_wait();
+  pdl_launch_dependents();
   extern __shared__ int32_t cnt[];      // [warps][E] counts, then first places; [E] totals; [E] first place and first tile
   int32_t* total = cnt + kGroupWarps * E;
   int32_t* off = total + E;
@@ -531,6 +532,7 @@ __global__ void __launch_bounds__(32 * kGroupWarps) moe_group_runs_kernel(const 
 __global__ void __launch_bounds__(128) moe_gather_kernel(const uint4* __restrict__ x, const int32_t* __restrict__ perm,
                                                          const int32_t* __restrict__ meta, int n, int units, uint4* __restrict__ out) {
   pdl_wait();
+  pdl_launch_dependents();
   const int s = blockIdx.x;
   if (s >= meta[1]) return;
   const uint4* src = x + (int64_t)(perm[s] % n) * units;
