@@ -396,6 +396,10 @@ int prl_gemm_bf16_splitk(const void* W, const void* W_lo /*or NULL*/, const void
  * gate_up_proj GEMM).  W = gate_up_proj.weight [2 I, K] as stored, gate rows first. */
 int prl_gemm_swiglu_decode(const void* W_bf16, const void* X_bf16, int64_t M, int64_t I, int64_t K, void* act_bf16,
                            prl_stream_t stream);
+/* ... = the bits of prl_gemm_bf16_splitk(split_k = slices) followed by prl_silu_mul; slices is 1, or 2 with M <= 8, K > 64: each half of
+ * the k-blocks is summed by itself and the epilogue adds the two (weights are finite: the other half's sums meet them with zeros). */
+int prl_gemm_swiglu_decode_sliced(const void* W_bf16, const void* X_bf16, int64_t M, int64_t I, int64_t K, int32_t slices, void* act_bf16,
+                                  prl_stream_t stream);
 
 /* Fused output head with IN-KERNEL logprob capture: logits = X W^T (+ W_lo) are produced tile by tile in
  * TMEM and reduced on the spot — per token logsumexp, exact entropy, the log-probability of a given target

@@ -137,6 +137,11 @@ struct GemmParams {
   // gated activation of the epilogue: glu_limit == 0: SiLU(gate) * up; glu_limit > 0: the clamped form of the hybrid decoders,
   // g = min(gate, limit), u = clamp(up, +-limit), act = g * sigmoid(glu_beta * g) * (u + 1)
   float glu_limit, glu_beta;
+  // the sums of a pair that is split in two, in one accumulator (gated epilogue, M <= late_rows = 8): the tokens of k-blocks >= late_kb go to
+  // columns 8 .. 15, behind as many zeros, and those of the others have zeros behind them (rows out of the map's range), so each half of the
+  // columns sums its own k-blocks and the epilogue adds the two: a step of eight layers (4 rows, 1024 wide, I 4096) 236.8 us, in one sum 235.5, as
+  // the pair 252.6; with an accumulator per half and a loop over them in the issuing warp 244 (0.25 us for each product of the step).  0 = off
+  int late_kb, late_rows;
   // two products in one accumulation (split_k, no lo part): k-blocks >= dual_kb are k-blocks (kb - dual_kb) of a second
   // weight (the map in the lo weight's place) and a second activation.  0 = off
   int dual_kb;
@@ -204,7 +209,8 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   };
   auto load_tokens = [&](int kb, uint32_t a_dst, uint32_t bar) {
     const bool second = p.dual_kb && kb >= p.dual_kb;
-    ptx::tma_load_2d(a_dst + b_off, second ? &tm_x2 : &tm_x, (second ? kb - p.dual_kb : kb) * kBlockK, m0, bar, ptx::kEvictLast);
+    ptx::tma_load_2d(a_dst + b_off, second ? &tm_x2 : &tm_x, (second ? kb - p.dual_kb : kb) * kBlockK,
+                     kb >= p.late_kb ? m0 - p.late_rows : m0, bar, ptx::kEvictLast);
   };
   // Warp 0 arms the barriers and IMMEDIATELY fills the first ring pass with WEIGHT tiles: weights do not depend on
   // the preceding kernel (PDL lets this run under the predecessor's tail) nor on the rest of this CTA's prologue
@@ -334,8 +340,13 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         const bool whole = (reinterpret_cast<uintptr_t>(p.act) & 3) == 0;       // swiglu_I is even
 #pragma unroll 4
         for (int tkn = et / per; tkn < m_valid; tkn += step) {
-          const float2 g2 = *reinterpret_cast<const float2*>(xch + tkn * 2 * h + f);
-          const float2 u2 = *reinterpret_cast<const float2*>(xch + tkn * 2 * h + h + f);
+          float2 g2 = *reinterpret_cast<const float2*>(xch + tkn * 2 * h + f);
+          float2 u2 = *reinterpret_cast<const float2*>(xch + tkn * 2 * h + h + f);
+          if (p.late_rows) {
+            const float2 g1 = *reinterpret_cast<const float2*>(xch + (tkn + p.late_rows) * 2 * h + f);
+            const float2 u1 = *reinterpret_cast<const float2*>(xch + (tkn + p.late_rows) * 2 * h + h + f);
+            g2.x += g1.x; g2.y += g1.y; u2.x += u1.x; u2.y += u1.y;
+          }
           const float gs[2] = {g2.x, g2.y}, us[2] = {u2.x, u2.y};
           float av[2];
 #pragma unroll
@@ -722,21 +733,24 @@ static int gemm_splitk_impl(const void* W, const void* W_lo, const void* X, int6
                             int32_t split_k, float* partials, float* peer_partials, prl_stream_t stream_);
 
 // Token-step gate_up GEMM with SiLU(gate) * up in its epilogue (sampler side, M <= 128 tokens, no split-K: 2 I / 128 tiles
-// already fill the SMs): act[M, I] bf16 = the bits prl_gemm_bf16_splitk(split_k = 1) + prl_silu_mul produce, one launch and
+// already fill the SMs): act[M, I] bf16 = the bits prl_gemm_bf16_splitk(split_k = slices) + prl_silu_mul produce, one launch and
 // no [M, 2 I] fp32 tile in between.  W = gate_up_proj [2 I, K] as stored (gate rows first).
-static int gemm_glu_decode_impl(const void* W, const void* X, int64_t M, int64_t I, int64_t K, float glu_limit, float glu_beta,
-                                void* act_bf16, prl_stream_t stream_) {
+static int gemm_glu_decode_impl(const void* W, const void* X, int64_t M, int64_t I, int64_t K, int32_t slices, float glu_limit,
+                                float glu_beta, void* act_bf16, prl_stream_t stream_) {
   PRL_CHECK_ARG(W && X && act_bf16, "prl_gemm_swiglu_decode: NULL argument");
   PRL_CHECK_ARG(M >= 1 && M <= 128 && I >= 64 && I % 64 == 0 && K >= 8 && K % 8 == 0,
                 "prl_gemm_swiglu_decode: need 1 <= M <= 128, I %% 64 == 0, K %% 8 == 0 (M=%lld I=%lld K=%lld)", (long long)M,
                 (long long)I, (long long)K);
   PRL_CHECK_ARG(!g_tiled_weights, "prl_gemm_swiglu_decode: not available with pre-tiled weights");
+  PRL_CHECK_ARG(slices == 1 || (slices == 2 && M <= 8 && K > kBlockK), "prl_gemm_swiglu_decode: slices are 1, or 2 of at most 8 tokens (slices=%d)",
+                (int)slices);
   const int nt = pick_ntile(M);
   GemmParams p = {};
   // 64 features a tile, or 32 where that still leaves every tile an SM of its own (as the plain product's short tiles): 4 x 8192 x 1024 7.3 -> 6.7 us, 4 x 9472 x 2048 11.3 -> 10.2
   p.tile_rows = nt <= 64 && I / 64 <= num_sms() / 2 ? 64 : kBlockM;
   p.M = M; p.N = 2 * I; p.K = K; p.kblocks = (int)((K + kBlockK - 1) / kBlockK); p.split_k = 1;
   p.swiglu_I = I; p.act = (__nv_bfloat16*)act_bf16; p.glu_limit = glu_limit; p.glu_beta = glu_beta;
+  if (slices == 2) { p.late_kb = p.kblocks / 2; p.late_rows = 8; }
   CUtensorMap tw, tx;
   int rc = make_tmap_2d_bf16(&tw, W, (uint64_t)K, (uint64_t)(2 * I), (uint64_t)K * 2, kBlockK, (uint32_t)(p.tile_rows / 2));
   if (rc) return rc;
@@ -753,7 +767,13 @@ static int gemm_glu_decode_impl(const void* W, const void* X, int64_t M, int64_t
 
 extern "C" int prl_gemm_swiglu_decode(const void* W, const void* X, int64_t M, int64_t I, int64_t K, void* act_bf16,
                                       prl_stream_t stream_) {
-  return gemm_glu_decode_impl(W, X, M, I, K, 0.f, 0.f, act_bf16, stream_);
+  return gemm_glu_decode_impl(W, X, M, I, K, 1, 0.f, 0.f, act_bf16, stream_);
+}
+
+// ... with the sums of a pair that is split into `slices`, 1 or 2
+extern "C" int prl_gemm_swiglu_decode_sliced(const void* W, const void* X, int64_t M, int64_t I, int64_t K, int32_t slices, void* act_bf16,
+                                             prl_stream_t stream_) {
+  return gemm_glu_decode_impl(W, X, M, I, K, slices, 0.f, 0.f, act_bf16, stream_);
 }
 
 // the same kernel with the clamped gate of the hybrid decoders in its epilogue (csrc/hybrid_ops.cu glu_clamped_kernel's formula
@@ -761,7 +781,7 @@ extern "C" int prl_gemm_swiglu_decode(const void* W, const void* X, int64_t M, i
 extern "C" int prl_gemm_glu_clamped_decode(const void* W, const void* X, int64_t M, int64_t I, int64_t K, float limit, float beta,
                                            void* act_bf16, prl_stream_t stream_) {
   PRL_CHECK_ARG(limit > 0.f, "prl_gemm_glu_clamped_decode: limit must be positive");
-  return gemm_glu_decode_impl(W, X, M, I, K, limit, beta, act_bf16, stream_);
+  return gemm_glu_decode_impl(W, X, M, I, K, 1, limit, beta, act_bf16, stream_);
 }
 
 extern "C" int prl_gemm_bf16_splitk(const void* W, const void* W_lo, const void* X, int64_t M, int64_t N, int64_t K,

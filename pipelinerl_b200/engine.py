@@ -538,11 +538,13 @@ def swiglu_epilogue_pays(I: int, H: int, split_k: int, sms: int) -> bool:
     return split_k == 1 or (I // 64 < sms and -(-H // 64) * (sms - I // 64) <= 5 * sms)
 
 
-def short_swiglu_tiles_pay(I: int, H: int, rows: int, sms: int) -> bool:
+def short_swiglu_tiles_pay(I: int, H: int, rows: int, sms: int, slices: int = 1) -> bool:
     """The same for the gated epilogue's tiles of 32 features, which up to 64 rows take where the I / 64 tiles of 64 are at most half as
     many as the SMs (prl_gemm_swiglu_decode).  1024 wide, I 4096 (128 tiles of 148): a step of eight layers
-    at 4 sequences 252 -> 241 us."""
-    return rows <= 64 and 2 * (I // 64) <= sms and -(-H // 64) * (sms - I // 32) <= 5 * sms
+    at 4 sequences 252 -> 241 us.  The sums stay those of the split pair, of which the epilogue
+    can add two `slices` of up to 8 rows: they share the 16 columns of the tile that the step's other products of so few rows have (in one of
+    32 columns, another kernel among the step's, 256 us)."""
+    return rows <= 64 and 2 * (I // 64) <= sms and -(-H // 64) * (sms - I // 32) <= 5 * sms and (slices == 1 or (slices == 2 and rows <= 8))
 
 
 class DecodeEngine(EngineCore):
@@ -632,8 +634,10 @@ class DecodeEngine(EngineCore):
         self.split_k = {k: int(self.lib.prl_gemm_auto_split_k(B, n, kk)) for k, (n, kk) in shapes.items()}
         self.split_k["head"] = 1  # the sampler reads plain logits
         I, H, sms = cfg.intermediate_size, cfg.hidden_size, torch.cuda.get_device_properties(self.dev).multi_processor_count
-        self.swiglu_epilogue = I % 64 == 0 and B <= 128 and (swiglu_epilogue_pays(I, H, self.split_k["gate_up"], sms)
-                                                             or short_swiglu_tiles_pay(I, H, B, sms))
+        split = self.split_k["gate_up"]
+        whole = swiglu_epilogue_pays(I, H, split, sms)
+        self.swiglu_slices = 1 if whole else split
+        self.swiglu_epilogue = I % 64 == 0 and B <= 128 and (whole or short_swiglu_tiles_pay(I, H, B, sms, split))
         need = max(self.split_k[k] * B * shapes[k][0] for k in ("qkv", "o", "gate_up", "down"))
         self.partials = torch.zeros(need, dtype=torch.float32, device=self.dev)
 
@@ -700,9 +704,9 @@ class DecodeEngine(EngineCore):
             nxt_qkv = f"layers.{l + 1}.qkv_proj.weight" if l + 1 < cfg.num_layers else None
             if fuse_swiglu:
                 # SiLU(gate) * up in the gate_up GEMM's epilogue: one launch less per layer and no [B, 2 I] fp32 tiles between
-                # the two; same bits as the pair below without a split
-                _lib.check(lib.prl_gemm_swiglu_decode(a.ptr(p + "gate_up_proj.weight"), self.x.data_ptr(), B, I, H,
-                                                      self.act.data_ptr(), st))
+                # the two; same bits as the pair below with a split of `swiglu_slices`
+                _lib.check(lib.prl_gemm_swiglu_decode_sliced(a.ptr(p + "gate_up_proj.weight"), self.x.data_ptr(), B, I, H,
+                                                             self.swiglu_slices, self.act.data_ptr(), st))
             else:
                 if "gemm" not in skip:
                     self._gemm(p + "gate_up_proj.weight", self.x, 2 * I, H, self.split_k["gate_up"], part)

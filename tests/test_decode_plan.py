@@ -17,3 +17,9 @@ def test_swiglu_epilogue_rule(I, H, split, pays):
 def test_short_swiglu_tiles_rule(I, H, rows, pays):
     """Up to 64 rows, tiles of 32 features on at most 148 SMs, and the idle ones cost at most 5 k-blocks of 64."""
     assert short_swiglu_tiles_pay(I, H, rows, 148) is pays
+
+
+@pytest.mark.parametrize("rows,slices,pays", [(8, 1, True), (8, 2, True), (9, 2, False), (9, 1, True), (64, 1, True), (8, 3, False), (1, 7, False)])
+def test_short_swiglu_tiles_keep_the_sums_of_the_split_pair(rows, slices, pays):
+    """Two slices of up to 8 rows are added in the epilogue; more of either take the split pair."""
+    assert short_swiglu_tiles_pay(4096, 1024, rows, 148, slices) is pays

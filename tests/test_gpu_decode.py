@@ -423,6 +423,30 @@ def test_token_step_with_and_without_the_swiglu_epilogue_is_bit_identical(cuda_d
     assert torch.equal(logits[True], logits[False])
 
 
+def test_token_step_of_short_gated_tiles_has_the_bits_of_the_split_pair(cuda_device):
+    """1024 wide, I 4096: gate_up is planned in two slices and takes the gated epilogue's tiles of 32 features; logits of every step are those of
+    the split pair, bit for bit."""
+    from pipelinerl_b200.engine import SamplingParams
+    from pipelinerl_b200.model import ModelConfig
+    cfg = ModelConfig(vocab_size=2048, hidden_size=1024, intermediate_size=4096, num_layers=2, num_q_heads=8, num_kv_heads=2)
+    w = tiny_weights(cfg, std=0.03, bias_std=0.1)
+    tokens = torch.randint(0, cfg.vocab_size, (12,), generator=torch.Generator().manual_seed(8)).tolist()
+    logits = {}
+    for fuse in (True, False):
+        eng = make_engine(cfg, w, cuda_device, max_batch=4, max_seq_len=128, max_new_tokens=4, use_cuda_graph=False,
+                          prefill_chunk=0, fused_head=False)
+        eng.fuse_swiglu = fuse
+        assert eng.split_k["gate_up"] == 2 and eng.swiglu_epilogue     # otherwise neither side is what its name says
+        eng.add_request(tokens, SamplingParams(max_tokens=2, temperature=1.0, greedy=True))
+        rows = []
+        for _ in range(len(tokens) - 1):
+            eng.step()
+            rows.append(eng.logits[0].clone())
+        logits[fuse] = torch.stack(rows)
+        del eng
+    assert torch.equal(logits[True], logits[False])
+
+
 def test_token_step_takes_the_swiglu_epilogue_where_gate_up_could_split_k(cuda_device):
     """2048 wide, I 8192: 128 tiles, which the planner would cut in K.  The engine takes the gated epilogue all the same; its
     log-probs and those of the split pair meet the oracle within the bar that the 7B width has (bf16 activations, one layer), and

@@ -201,6 +201,24 @@ def test_short_gated_tiles_keep_the_bits(cuda_device, B, I, K, limit):
         assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("B", [1, 4, 7, 8])
+@pytest.mark.parametrize("I,K", [(64, 72), (4096, 1024), (4736, 200), (4800, 1088)])
+def test_gated_epilogue_adds_the_slices_of_a_split_pair(cuda_device, B, I, K):
+    """The epilogue's sums over two slices of the k-blocks, even and odd numbers of them, tiles of 32 and 64 features: the bits of the split
+    product and the activation by themselves."""
+    slices = 2
+    from pipelinerl_b200 import _lib
+    lib, st, g = _lib.load(), _lib.stream_ptr(), torch.Generator(device="cuda").manual_seed(B + I + K)
+    x = torch.randn(B, K, generator=g, device="cuda").bfloat16()
+    W = (torch.randn(2 * I, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    part, want = torch.empty(slices, B, 2 * I, device="cuda"), torch.empty(B, I, dtype=torch.bfloat16, device="cuda")
+    got = torch.full((B, I), float("nan"), dtype=torch.bfloat16, device="cuda")
+    _lib.check(lib.prl_gemm_bf16_splitk(W.data_ptr(), None, x.data_ptr(), B, 2 * I, K, slices, part.data_ptr(), st))
+    _lib.check(lib.prl_silu_mul(part.data_ptr(), slices, B, I, want.data_ptr(), None, 0, st))
+    _lib.check(lib.prl_gemm_swiglu_decode_sliced(W.data_ptr(), x.data_ptr(), B, I, K, slices, got.data_ptr(), st))
+    assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("M", [1, 17, 64])
 @pytest.mark.parametrize("N,K", [(8, 8), (1000, 2056), (4736, 72), (4737, 1024), (9232, 2048), (9472, 200), (9473, 64)])
 def test_short_weight_tiles_keep_the_bits(cuda_device, M, N, K):
