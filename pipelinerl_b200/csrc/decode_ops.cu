@@ -462,6 +462,13 @@ __global__ void __launch_bounds__(kSampleThreads) sample_partial_kernel(const fl
     const float x[1] = {z[i]};
     sample_group(x, i, inv_temp, greedy, seed, step, b, vocab_offset, m, s, best, best_z);
   }
+  if (best.i == 0x7fffffff)          // no key above -inf: the lowest id of those that are -inf, as in a comparison of equal keys
+    for (i = lo + threadIdx.x; i < hi; i += kSampleThreads)
+      if (z[i] * inv_temp == -INFINITY) {
+        best = ArgMax{-INFINITY, vocab_offset + i};
+        best_z = -INFINITY;
+        break;
+      }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float m2 = __shfl_xor_sync(0xffffffffu, m, o), s2 = __shfl_xor_sync(0xffffffffu, s, o);

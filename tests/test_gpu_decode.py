@@ -9,6 +9,8 @@ recorded on a B200: tests/golden/vllm_tiny_*.json) differs from this engine by 1
 -- the same size as this engine's difference to the fp32 oracle (1.29e-2 / 1.79e-2 max).  Every end-to-end bound below is
 1.5 x the value measured on a B200 (the tests print what they measure); greedy token ids must equal the oracle's wherever its
 top-2 logit margin exceeds 5e-2."""
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -116,6 +118,27 @@ def test_sampling_distribution_and_logprob_capture(cuda_device):
     # greedy == argmax, ties to the lowest index
     _lib.check(lib.prl_sample_logprob(logits.data_ptr(), B, V, 1.0, 1, 0, 0, ids.data_ptr(), lps.data_ptr(), ws.data_ptr(), ws.numel(), None))
     assert (ids.cpu() == int(torch.argmax(logits[0].cpu()))).all()
+
+
+@pytest.mark.parametrize("greedy", [0, 1])
+@pytest.mark.parametrize("V", [3, 257, 40000])
+def test_sampled_id_of_a_row_of_minus_infinity(cuda_device, V, greedy):
+    """No logit above -inf, given or by its temperature: the lowest id of equal keys, as torch.argmax gives, and no number for a log-probability;
+    one that is above is the choice."""
+    from pipelinerl_b200 import _lib
+    lib = _lib.load()
+    logits = torch.full((4, V), -math.inf, device=cuda_device)
+    logits[1] = -3e38
+    logits[2, V - 1] = -5.0
+    logits[3, V // 2:] = -3e38
+    inv_t = torch.tensor([1.0, 10.0, 0.5, 2.0], device=cuda_device)
+    ids, lps = torch.full((4,), -1, dtype=torch.int32, device=cuda_device), torch.zeros(4, device=cuda_device)
+    ws = torch.zeros(int(lib.prl_sample_workspace_bytes(4)), dtype=torch.uint8, device=cuda_device)
+    choose = torch.full((4,), greedy, dtype=torch.uint8, device=cuda_device)
+    _lib.check(lib.prl_sample_logprob_rows(logits.data_ptr(), 4, V, inv_t.data_ptr(), choose.data_ptr(), 11, 3, ids.data_ptr(), lps.data_ptr(),
+                                           ws.data_ptr(), ws.numel(), _lib.stream_ptr()))
+    assert ids.tolist() == [0, 0, V - 1, 0]
+    assert lps[[0, 1, 3]].isnan().all() and lps[2].item() == 0.0
 
 
 def test_paged_attention_long_context_vs_fp32(cuda_device):
