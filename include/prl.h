@@ -159,10 +159,10 @@ int prl_logprob_tail_bwd(const float* logits, int64_t T, int64_t V, int64_t row_
                          const float* g_logprobs, const float* g_entropy,
                          float* dlogits, int64_t dlogits_stride, prl_stream_t stream);
 
-/* The same, the gradients scaled by *g_loss (device); skip_one: nothing is written where that is 1. */
+/* The same, the gradients scaled by *g_loss (device); where that is 1 the last rows_done rows are not written (they are there already). */
 int prl_logprob_tail_bwd_scaled(const float* logits, int64_t T, int64_t V, int64_t row_stride, const int64_t* input_ids, float temperature,
                                 const float* lse, const float* entropy, const float* g_logprobs, const float* g_entropy,
-                                const float* g_loss, int32_t skip_one, float* dlogits, int64_t dlogits_stride, prl_stream_t stream);
+                                const float* g_loss, int32_t rows_done, float* dlogits, int64_t dlogits_stride, prl_stream_t stream);
 
 /* Same backward for an explicit list of rows with their targets (logits [n_rows, V] of a recomputed chunk). */
 int prl_logprob_rows_bwd(const float* logits, int64_t n_rows, int64_t V, int64_t row_stride,

@@ -112,8 +112,8 @@ __global__ void __launch_bounds__(kThreads) tail_fwd_kernel(const float* __restr
 }
 
 // d logits: reads 4 bytes and writes 4 per logit, or writes alone where a row has no gradient (prompts): 2001 x 151936, HBM-bound, 390 us,
-// 332 with a third of the rows masked.  Rows go from the last to the first, whose logits the forward has left in L2.  g_loss (device memory, or NULL: 1) scales the
-// gradients; with skip_one nothing is done where it is 1 (d logits of that scale are there already).
+// 332 with a third of the rows masked.  Rows go from the last to the first, whose logits the forward has left in L2.  g_loss (device memory,
+// or NULL: 1) scales the gradients; where it is 1 the last rows_done rows are left alone: they hold d logits of that scale already.
 __global__ void __launch_bounds__(kThreads) tail_bwd_kernel(const float* __restrict__ logits, int64_t V,
                                                            int64_t row_stride, int64_t n_rows,
                                                            const int64_t* __restrict__ ids, float inv_temp,
@@ -121,10 +121,10 @@ __global__ void __launch_bounds__(kThreads) tail_bwd_kernel(const float* __restr
                                                            const float* __restrict__ entropy,
                                                            const float* __restrict__ g_lp,
                                                            const float* __restrict__ g_ent,
-                                                           const float* __restrict__ g_loss, int skip_one,
+                                                           const float* __restrict__ g_loss, int rows_done,
                                                            float* __restrict__ dlogits, int64_t d_stride) {
   const float gs = g_loss ? *g_loss : 1.f;
-  if (skip_one && gs == 1.f) return;
+  if ((int)blockIdx.x < rows_done && gs == 1.f) return;
   const int64_t row = (int64_t)gridDim.x - 1 - blockIdx.x;
   float* d = dlogits + row * d_stride;
   const bool has_target = row < n_rows;  // the last position has none (logits[:, :-1])
@@ -340,17 +340,18 @@ extern "C" int prl_logprob_tail_bwd(const float* logits, int64_t T, int64_t V, i
   return PRL_OK;
 }
 
-// prl_logprob_tail_bwd with the gradients scaled by *g_loss (device memory); skip_one: nothing is written where that is 1
+// prl_logprob_tail_bwd with the gradients scaled by *g_loss (device memory); where that is 1 the last rows_done rows are not written
 extern "C" int prl_logprob_tail_bwd_scaled(const float* logits, int64_t T, int64_t V, int64_t row_stride, const int64_t* input_ids,
                                            float temperature, const float* lse, const float* entropy, const float* g_logprobs,
-                                           const float* g_entropy, const float* g_loss, int32_t skip_one, float* dlogits,
+                                           const float* g_entropy, const float* g_loss, int32_t rows_done, float* dlogits,
                                            int64_t dlogits_stride, prl_stream_t stream_) {
   PRL_CHECK_ARG(T >= 1 && V >= 1 && row_stride >= V && dlogits_stride >= V, "prl_logprob_tail_bwd_scaled: bad shape");
   PRL_CHECK_ARG(temperature > 0.f, "prl_logprob_tail_bwd_scaled: temperature must be > 0");
   PRL_CHECK_ARG(logits && input_ids && lse && g_loss && dlogits, "prl_logprob_tail_bwd_scaled: NULL argument");
   PRL_CHECK_ARG(!g_entropy || entropy, "prl_logprob_tail_bwd_scaled: g_entropy needs the forward entropy");
+  PRL_CHECK_ARG(rows_done >= 0 && rows_done <= T, "prl_logprob_tail_bwd_scaled: bad rows_done");
   tail_bwd_kernel<<<(unsigned)T, kThreads, 0, (cudaStream_t)stream_>>>(logits, V, row_stride, T - 1, input_ids, 1.f / temperature, lse, entropy,
-                                                                       g_logprobs, g_entropy, g_loss, skip_one, dlogits, dlogits_stride);
+                                                                       g_logprobs, g_entropy, g_loss, rows_done, dlogits, dlogits_stride);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }

@@ -145,11 +145,22 @@ class _PgLoss(torch.autograd.Function):
         return g[0], g[1] if ctx.has_entropy else None, None, None, None, None
 
 
+AHEAD_LOGITS = 130_000_000
+
+
+def _rows_ahead(T: int, V: int, rows: int) -> int:
+    """Rows (the last ones, which the forward left in L2) whose d logits are made before the loss's gradient is known: what the GPU does in the time that
+    the host takes from the statistics to the backward's first launch, some 200 us.  2001 x 151936, us a step with the loss's gradient 1 / another /
+    without a backward, for 0, 70, 130, 200 and all 304 million logits: 718 / 721 / 319, 603 / 719 / 334, 579 / 725 / 378, 575 / 795 / 444, 566 / 910 / 559
+    (5000 rows: 1421 / 1447 / 568, 1315 / 1466 / 648 with 130, 1305 / 2119 / 1297 with all)."""
+    return min(T, max(2, AHEAD_LOGITS // rows // V))
+
+
 class _LogitsLoss(torch.autograd.Function):
-    """logits [T, V] -> loss.  The gradient of the loss kernel gives d logits of a loss gradient of one, and they are made without
-    waiting for the backward: their launch is appended to `later`, for rl_step to make once the statistics are on their way
-    to the host, so that the GPU has them to do while the host reads the statistics and autograd starts.  Another loss gradient makes them again.
-    2001 x 151936, steps in a row: 807 -> 556 us."""
+    """logits [T, V] -> loss.  The gradient of the loss kernel gives d logits of a loss gradient of one, and some of them (_rows_ahead) are
+    made without waiting for the backward: their launch is appended to `later`, for rl_step to make once the statistics are on their
+    way to the host, so that the GPU has them to do while the host reads the statistics and autograd starts.  The backward makes the others, and
+    all of them for another loss gradient (a scaled loss), so that what was made ahead cost the GPU only time that it had."""
 
     @staticmethod
     def forward(ctx, logits, input_ids, temperature: float, row: dict, cfg_struct, meta: dict, report, later: list):
@@ -170,30 +181,37 @@ class _LogitsLoss(torch.autograd.Function):
         ctx.dlogits = None
         if ctx.needs_input_grad[0] and T > 1:        # one row has no next token: its loss is made, a gradient is refused by the kernel's entry
             ctx.dlogits = d = torch.empty((T, V), dtype=torch.float32, device=logits.device)
-            later.append(lambda: _LogitsLoss._d_logits(logits, ids, stats, grads, float(temperature), None, d))
+            ctx.ahead = ahead = _rows_ahead(T, V, meta["num_sequences"])
+            later.append(lambda: _LogitsLoss._d_logits_ahead(logits, ids, stats, grads, float(temperature), d, T - ahead))
         return loss
 
     @staticmethod
-    def _d_logits(logits, ids, stats, grads, temperature, g_loss, d):
-        """d logits into `d`; with g_loss (on the device) they are there already for a gradient of one"""
-        lib = _lib.load()
+    def _tail(logits, ids, stats, grads, temperature, r):
+        """Arguments of the tail's backward from row r on (addresses: slices of six tensors cost the host 20 us a step)"""
         T, V = logits.shape
-        lp, ent, lse = stats
-        tail = (logits.data_ptr(), T, V, logits.stride(0), ids.data_ptr(), temperature, lse.data_ptr(), ent.data_ptr(), grads[0].data_ptr(),
-                grads[1].data_ptr())
-        if g_loss is None:
-            _lib.check(lib.prl_logprob_tail_bwd(*tail, d.data_ptr(), V, _lib.stream_ptr()))
-        else:
-            _lib.check(lib.prl_logprob_tail_bwd_scaled(*tail, g_loss.data_ptr(), 1, d.data_ptr(), V, _lib.stream_ptr()))
+        n, ld = T - 1, logits.stride(0)
+        ent, g = stats.data_ptr() + 4 * (n + r), grads.data_ptr() + 4 * r
+        return logits.data_ptr() + 4 * r * ld, T - r, V, ld, ids.data_ptr() + 8 * r, temperature, ent + 4 * n, ent, g, g + 4 * n
+
+    @staticmethod
+    def _d_logits_ahead(logits, ids, stats, grads, temperature, d, r):
+        """Rows r .. T - 1, at least two (the last one has no column of gradients), for a loss gradient of one"""
+        V = logits.shape[1]
+        _lib.check(_lib.load().prl_logprob_tail_bwd(*_LogitsLoss._tail(logits, ids, stats, grads, temperature, r), d.data_ptr() + 4 * r * V, V,
+                                                    _lib.stream_ptr()))
 
     @staticmethod
     def backward(ctx, g_loss):
         logits, ids, stats, grads = ctx.saved_tensors
+        T, V = logits.shape
+        if T == 1:
+            raise RuntimeError("a row of one token has no log-probability and no gradient")
         d, ctx.dlogits = ctx.dlogits, None           # given away: a second backward over a retained graph makes its own
+        done = 0 if d is None else ctx.ahead
         if d is None:
-            d = torch.empty(logits.shape, dtype=torch.float32, device=logits.device)
-            _LogitsLoss._d_logits(logits, ids, stats, grads, ctx.temperature, None, d)
-        _LogitsLoss._d_logits(logits, ids, stats, grads, ctx.temperature, g_loss.contiguous(), d)
+            d = torch.empty((T, V), dtype=torch.float32, device=logits.device)
+        _lib.check(_lib.load().prl_logprob_tail_bwd_scaled(*_LogitsLoss._tail(logits, ids, stats, grads, ctx.temperature, 0), g_loss.contiguous().data_ptr(),
+                                                           done, d.data_ptr(), V, _lib.stream_ptr()))
         return d, None, None, None, None, None, None, None
 
 

@@ -403,6 +403,47 @@ def test_gradient_of_logits_made_ahead_of_the_backward(cuda_device, policy, T, V
     assert not quiet.requires_grad and stats2 == stats
 
 
+@pytest.mark.parametrize("ahead", [2, 90, 1000])
+def test_part_of_the_gradient_is_made_ahead(cuda_device, monkeypatch, ahead):
+    """Few rows of d logits are made before the loss's gradient is known, the others by the backward, in one launch, whatever that gradient is and however
+    often: the same bits as made in one."""
+    from pipelinerl_b200 import _lib
+    from pipelinerl_b200.finetune import rl
+    from pipelinerl_b200.finetune.types import PipelineBatchEncoding
+    T, V, g = 300, 1203, torch.Generator().manual_seed(5)
+    z, ids, one = 2 * torch.randn(2, T, V, generator=g), torch.randint(0, V, (2, T), generator=g), torch.ones(2, T)
+    batch = PipelineBatchEncoding(
+        input_ids=ids, attention_mask=one.long(), labels=torch.where(torch.rand(2, T, generator=g) < 0.3, -100, ids), rewards=one, advantages=one - 2 * torch.rand(2, T, generator=g),
+        ref_logprobs=-7 * one, old_logprobs=-7 * one, group_tokens=one * T, num_labels=one * T, overflow=0 * one, model_version=0, is_packed=False).to_device(cuda_device)
+    cfg, lib = rl.RLConfig(policy_loss="reinforce", batch_size=2, entropy_bonus=0.01, final_entropy_bonus=0.01), _lib.load()
+    calls = []
+    for name, rows in (("prl_logprob_tail_bwd", 1), ("prl_logprob_tail_bwd_scaled", 1)):
+        def spy(*a, f=getattr(lib, name), name=name, rows=rows):
+            calls.append((name, a[rows]))
+            return f(*a)
+        monkeypatch.setattr(lib, name, spy)
+
+    def grads(rows):
+        monkeypatch.setattr(rl, "AHEAD_LOGITS", rows * 2 * V)
+        model, got = LogitsModel(z.to(cuda_device)), []
+        for scale in (1.0, 0.5):
+            calls.clear()
+            loss, _ = rl.rl_step(model, batch, 0, 10, cfg)
+            early = [c for c in calls if c[0] == "prl_logprob_tail_bwd"]
+            assert early == [("prl_logprob_tail_bwd", min(rows, T))] * 2
+            for keep in (True, False):
+                calls.clear()
+                model.logits.grad = None
+                (scale * loss).backward(retain_graph=keep)
+                assert calls == [("prl_logprob_tail_bwd_scaled", T)] * 2
+                got.append(model.logits.grad.clone())
+        return got
+
+    want, got = grads(T), grads(ahead)
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) and torch.equal(got[0], got[1]) and torch.equal(got[2], got[3]) and got[0].abs().max() > 0
+    assert not torch.equal(got[0], got[2])
+
+
 def test_row_of_one_token_has_a_loss(cuda_device):
     """No next token: rl_step gives its loss (none) and reports the input's size; nothing of d logits is made ahead."""
     from pipelinerl_b200.finetune import rl
