@@ -176,14 +176,16 @@ int prl_logprob_rows_bwd(const float* logits, int64_t n_rows, int64_t V, int64_t
 int prl_head_dlogits(const void* W_bf16, const void* W_lo_bf16, const void* X_bf16, int64_t M, int64_t V, int64_t K,
                      float temperature, const int64_t* targets, const float* lse, const float* entropy,
                      const float* g_logprobs, const float* g_entropy, void* dz_bf16, int64_t ld_dz, prl_stream_t stream);
-/* Head backward over the rows that have a gradient (tokens of prompts have none).  prl_live_rows gives them slots: slot c < *count holds
+/* Head backward over the rows that have a gradient (tokens of prompts have none, unless a logit of theirs is not a number: then nor is
+ * their gradient).  prl_live_rows gives them slots: slot c < *count holds
  * row rows[c], row r has slot place[r] or -1, a row below *count its own; index = rows[n] | places[n] | scratch[n] | count.
  * prl_gather_live_rows: xc[c] = x[rows[c]] (bf16, K wide), and zeros in xc and dz from row *count up to the next multiple of 64 (xc has
  * room for n rounded up to 64 rows, dz for dz_rows).  prl_head_dlogits_rows: prl_head_dlogits with X and dz in that order (token rows[c]
  * of targets, statistics, gradients).  prl_head_dlogits_kept: the same from the fp32 logits that prl_head_logprob_keep stored in the
  * forward for its first keep_rows tokens, in their place: bf16 [n, V] of row stride 2 ld_logits.  prl_gemm_ex_counted: prl_gemm_ex over
  * *count rows of A and C, or of the contraction (count_is_k, accumulating).  prl_spread_rows: out[r] = src[place[r]], or zeros. */
-int prl_live_rows(const float* g_logprobs, const float* g_entropy, int64_t n, int32_t* index, prl_stream_t stream);
+int prl_live_rows(const float* g_logprobs, const float* g_entropy, const float* lse, const float* entropy, int64_t n, int32_t* index,
+                  prl_stream_t stream);
 int prl_gather_live_rows(const void* x, int64_t n, int64_t K, const int32_t* rows, const int32_t* count, void* xc, void* dz,
                          int64_t dz_rows, int64_t V, int64_t ld_dz, prl_stream_t stream);
 int prl_spread_rows(const void* src, const int32_t* place, int64_t n, int64_t K, void* out, prl_stream_t stream);

@@ -129,7 +129,9 @@ __global__ void __launch_bounds__(kThreads) tail_bwd_kernel(const float* __restr
   float* d = dlogits + row * d_stride;
   const bool has_target = row < n_rows;  // the last position has none (logits[:, :-1])
   const float gl = has_target && g_lp ? g_lp[row] * gs : 0.f, ge = has_target && g_ent ? g_ent[row] * gs : 0.f;
-  if (gl == 0.f && ge == 0.f) {
+  // no gradient: zeros, without a look at the logits where the statistics say that they are numbers; a logit that is not one (entropy or
+  // log-sum-exp are none either) makes the row's gradient none, masked or not, as the formula has it
+  if (gl == 0.f && ge == 0.f && (!has_target || (entropy && isfinite(lse_in[row]) && isfinite(entropy[row])))) {
     const int64_t v4 = (reinterpret_cast<uintptr_t>(d) & 15) == 0 ? V / 4 : 0;
     for (int64_t i = threadIdx.x; i < v4; i += kThreads) st_stream_f4(reinterpret_cast<float4*>(d) + i, make_float4(0.f, 0.f, 0.f, 0.f));
     for (int64_t i = v4 * 4 + threadIdx.x; i < V; i += kThreads) d[i] = 0.f;
@@ -161,7 +163,8 @@ __global__ void __launch_bounds__(kThreads) tail_bwd_kernel(const float* __restr
 // Order of the `count` rows with a gradient: slot c holds row rows[c], row r's slot is place[r], or -1.  A row below `count` keeps its own
 // slot and the others fill the slots of rows without one, in turn: d logits of a row can then take the place of the logits it is made
 // from.  One block: 2048 rows of two columns are 16 KB.
-__global__ void __launch_bounds__(1024) live_rows_kernel(const float* __restrict__ g_lp, const float* __restrict__ g_ent, int n,
+__global__ void __launch_bounds__(1024) live_rows_kernel(const float* __restrict__ g_lp, const float* __restrict__ g_ent,
+                                                         const float* __restrict__ lse, const float* __restrict__ entropy, int n,
                                                          int32_t* rows, int32_t* place, int32_t* open, int32_t* __restrict__ count) {
   __shared__ int s_warp[2][32];
   __shared__ int s_total;
@@ -170,8 +173,8 @@ __global__ void __launch_bounds__(1024) live_rows_kernel(const float* __restrict
   __syncthreads();
   int mine = 0;
   for (int r = threadIdx.x; r < n; r += 1024) {
-    // a gradient that is not a number is one, too
-    const bool live = (g_lp && !(g_lp[r] == 0.f)) || (g_ent && !(g_ent[r] == 0.f));
+    // a gradient that is not a number is one, too, and so is none on a row of which a logit is not a number
+    const bool live = (g_lp && !(g_lp[r] == 0.f)) || (g_ent && !(g_ent[r] == 0.f)) || !isfinite(lse[r]) || !isfinite(entropy[r]);
     place[r] = live ? r : -1;
     mine += live;
   }
@@ -374,12 +377,13 @@ extern "C" int prl_logprob_rows_bwd(const float* logits, int64_t n_rows, int64_t
   return PRL_OK;
 }
 
-// Rows of [n] gradient columns that are not zero: slot c < *count holds row rows[c], row r has slot place[r] or -1; a row below *count
+// Rows of [n] gradient columns that are not zero, or of statistics that are no numbers: slot c < *count holds row rows[c], row r has slot place[r] or -1; a row below *count
 // has its own.  index: room for 3 n + 1 (rows, places, scratch, count).
-extern "C" int prl_live_rows(const float* g_logprobs, const float* g_entropy, int64_t n, int32_t* index, prl_stream_t stream_) {
-  PRL_CHECK_ARG(index && (g_logprobs || g_entropy), "prl_live_rows: NULL argument");
+extern "C" int prl_live_rows(const float* g_logprobs, const float* g_entropy, const float* lse, const float* entropy, int64_t n,
+                             int32_t* index, prl_stream_t stream_) {
+  PRL_CHECK_ARG(index && (g_logprobs || g_entropy) && lse && entropy, "prl_live_rows: NULL argument");
   PRL_CHECK_ARG(n >= 1 && n < (1ll << 30), "prl_live_rows: bad row count %lld", (long long)n);
-  live_rows_kernel<<<1, 1024, 0, (cudaStream_t)stream_>>>(g_logprobs, g_entropy, (int)n, index, index + n, index + 2 * n, index + 3 * n);
+  live_rows_kernel<<<1, 1024, 0, (cudaStream_t)stream_>>>(g_logprobs, g_entropy, lse, entropy, (int)n, index, index + n, index + 2 * n, index + 3 * n);
   PRL_LAUNCH_CHECK();
   return PRL_OK;
 }

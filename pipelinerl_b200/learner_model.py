@@ -239,7 +239,7 @@ class _NativeHead(torch.autograd.Function):
                 continue
             rows = index.data_ptr()
             place, count = rows + 4 * n, rows + 12 * n
-            _lib.check(lib.prl_live_rows(at[3], at[4], n, rows, st))
+            _lib.check(lib.prl_live_rows(at[3], at[4], at[1], at[2], n, rows, st))
             if r1 <= kept:
                 dz, ld, k_rows = logits.data_ptr(), 2 * V, n
                 _lib.check(lib.prl_head_dlogits_kept(dz, V, n, V, ctx.temperature, rows, count, *at, st))

@@ -1,6 +1,8 @@
 """CTA-pair persistent tcgen05 GEMM of the learner body (csrc/gemm_tn.cu) against fp32 torch matmuls of the
 same bf16 operands.  Tolerance: fp32 accumulation of bf16 products (1e-4 of the output scale) plus one bf16
 rounding (2^-8 relative) where the output is bf16."""
+import math
+
 import pytest
 import torch
 
@@ -579,3 +581,30 @@ def test_head_backward_of_kept_logits_and_live_rows(cuda_device, monkeypatch, M,
         assert ((got[0].double() - want).abs() <= 2.0 ** -8 * (size @ Ws.abs()) + 2.0 ** -8 * want.abs() + 1e-9).all()
         for d in (got[1].double() - 0.25, got[2][0].double()):
             assert ((d - dz.T @ x.double()).abs() <= 2.0 ** -8 * (size.T @ x.double().abs()) + 2.0 ** -21).all()
+
+
+@pytest.mark.parametrize("M,kept", [(300, 0), (300, 300), (200, 0)])
+def test_head_backward_of_a_masked_row_that_is_no_number(cuda_device, monkeypatch, M, kept):
+    """A token without a gradient whose hidden state is not a number: its d hidden and dW are none either (0 x NaN), the other rows' stay what they are."""
+    import types
+    from pipelinerl_b200.learner_body import Ops
+    from pipelinerl_b200.learner_model import _NativeHead
+    dev, V, K = cuda_device, 520, 64
+    g = torch.Generator(device=dev).manual_seed(M)
+    x, W = (torch.randn(n, K, generator=g, device=dev).to(torch.bfloat16) for n in (M, V))
+    tg, on = torch.randint(0, V, (M,), generator=g, device=dev), (torch.arange(M, device=dev) % 3 > 0).float()
+    monkeypatch.setattr(_NativeHead, "_rows_to_keep", staticmethod(lambda *a: kept))
+    got = []
+    for bad in (False, True):
+        if bad:
+            x[6, 5], x[9, 0] = math.nan, math.inf
+        gW = torch.zeros(V, K, device=dev)
+        model = types.SimpleNamespace(p=lambda n: W, head_lo=None, body=types.SimpleNamespace(ops=Ops(), g={"lm_head.weight": gW}))
+        h = x.clone().requires_grad_()
+        lp, ent = _NativeHead.apply(h, model, tg, 1.0, 2048)
+        torch.autograd.backward([lp, ent], [on, 0.1 * on])
+        got.append((h.grad, gW))
+    rows = torch.arange(M, device=dev)
+    rest = (rows != 6) & (rows != 9)
+    assert torch.equal(got[0][0][rest], got[1][0][rest]) and torch.count_nonzero(got[0][0][[6, 9]]) == 0
+    assert got[1][0][[6, 9]].isnan().all() and got[1][1].isnan().all() and not got[0][1].isnan().any()

@@ -1,6 +1,8 @@
 """Parity of the CUDA PG-loss path (through the C ABI / rl_step facade) with the oracle and with the
 reference's own outputs (golden fixtures).  Tolerances: loss / logprobs / stats 1e-4 relative;
 gradients 1e-4 relative + 1e-7 absolute."""
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -442,6 +444,27 @@ def test_part_of_the_gradient_is_made_ahead(cuda_device, monkeypatch, ahead):
     want, got = grads(T), grads(ahead)
     assert all(torch.equal(a, b) for a, b in zip(got, want)) and torch.equal(got[0], got[1]) and torch.equal(got[2], got[3]) and got[0].abs().max() > 0
     assert not torch.equal(got[0], got[2])
+
+
+@pytest.mark.parametrize("bad", [math.nan, math.inf, -math.inf])
+@pytest.mark.parametrize("with_entropy", [True, False])
+def test_masked_row_with_a_logit_that_is_no_number(cuda_device, bad, with_entropy):
+    """A row without a gradient: zeros where its logits are numbers, and what 0 x NaN gives where the formula meets one that is not."""
+    from pipelinerl_b200 import _lib
+    lib, T, V, dev = _lib.load(), 6, 2001, cuda_device
+    z = torch.randn(T, V, generator=torch.Generator().manual_seed(2)).to(dev)
+    z[1, 77], z[3, 2000] = bad, bad
+    ids = torch.arange(T, device=dev) + 5
+    lp, ent, lse = torch.empty(3, T - 1, device=dev)
+    p = lambda t: t.data_ptr()  # noqa: E731
+    _lib.check(lib.prl_logprob_tail_fwd(p(z), T, V, V, p(ids), 1.0, p(lp), p(ent), p(lse), _lib.stream_ptr()))
+    g_lp, g_ent, d = torch.tensor([0.5, 0.0, 0.0, 0.0, 1.0], device=dev), torch.zeros(T - 1, device=dev), torch.full((T, V), 7.0, device=dev)
+    _lib.check(lib.prl_logprob_tail_bwd(p(z), T, V, V, p(ids), 1.0, p(lse), p(ent) if with_entropy else None, p(g_lp), p(g_ent) if with_entropy else None,
+                                        p(d), V, _lib.stream_ptr()))
+    at = torch.zeros(T, V, dtype=torch.bool, device=dev)
+    at[1] = at[3] = bad != -math.inf or with_entropy       # a log-sum-exp or entropy (0 x -inf) that is no number is in every column, -inf in its own
+    at[1, 77] = at[3, 2000] = True
+    assert torch.equal(d.isnan(), at) and torch.count_nonzero(d[[2, 5]]) == 0 and d[[0, 4]].abs().min() > 0
 
 
 def test_row_of_one_token_has_a_loss(cuda_device):
