@@ -133,15 +133,23 @@ class _NativeHead(torch.autograd.Function):
     17.8."""
 
     @staticmethod
-    def _rows_to_keep(M: int, V: int, dev) -> int:
+    def _chunk_rows(M: int) -> int:
+        """Rows whose dW is one sum: all up to 4096, more in equal chunks.  A chunk reads and writes the fp32 gradients of all weights (2.2 GB: 3071 rows in
+        two chunks 19.3 ms a step, in one 18.1) and, where its logits are not kept, holds its d logits (0.6 GB for 2048 rows)."""
+        n = max(1, -(-M // 4096))
+        return (-(-M // n) + 63) // 64 * 64
+
+    @staticmethod
+    def _rows_to_keep(M: int, V: int, dev, chunk: int = 256) -> int:
         """Rows whose fp32 logits (4 V bytes each) the forward stores: at most a quarter of the memory that is free now, so that
         what the backward allocates beside them finds its place; few rows are not worth a buffer, since the products' time is the
-        weights' way through the memory then (up to 256 rows: one row tile)."""
+        weights' way through the memory then (up to 256 rows: one row tile).  All rows or whole chunks: memory decides where a chunk's d logits come
+        from, and nothing of how dW is summed."""
         if M <= 256 or V % 8:
             return 0
         free = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
         rows = min(M, free // 4 // (4 * V))
-        return rows if rows == M else rows // 256 * 256
+        return rows if rows == M else rows // chunk * chunk
 
     @staticmethod
     def forward(ctx, hidden, model, targets, temperature: float, chunk_rows: int):
@@ -155,25 +163,25 @@ class _NativeHead(torch.autograd.Function):
         ent, lse = torch.empty_like(lp), torch.empty_like(lp)
         ws = torch.empty(int(lib.prl_head_workspace_bytes(M, V)), dtype=torch.uint8, device=x.device)
         W_lo = model.head_lo
-        logits = None
+        logits, kept = None, 0
         if ctx.needs_input_grad[0]:
-            kept = _NativeHead._rows_to_keep(M, V, x.device)
+            kept = _NativeHead._rows_to_keep(M, V, x.device, chunk_rows)
             if kept:
-                try:
-                    logits = torch.empty(kept, V, dtype=torch.float32, device=x.device)
+                try:                                     # the last chunk's d logits end on a whole k-block
+                    logits = torch.empty((kept + 63) // 64 * 64 if kept == M else kept, V, dtype=torch.float32, device=x.device)
                 except torch.cuda.OutOfMemoryError:      # free memory in pieces: the backward recomputes
-                    pass
+                    kept = 0
         if logits is not None:
             _lib.check(lib.prl_head_logprob_keep(W.data_ptr(), W_lo.data_ptr() if W_lo is not None else None, x.data_ptr(), M, V, K,
                                                  float(temperature), tg.data_ptr(), lp.data_ptr(), ent.data_ptr(), lse.data_ptr(),
-                                                 logits.data_ptr(), V, logits.shape[0], ws.data_ptr(), ws.numel(), _lib.stream_ptr()))
+                                                 logits.data_ptr(), V, kept, ws.data_ptr(), ws.numel(), _lib.stream_ptr()))
         else:
             _lib.check(lib.prl_head_logprob(W.data_ptr(), W_lo.data_ptr() if W_lo is not None else None, x.data_ptr(), M, V, K,
                                             float(temperature), tg.data_ptr(), 1, 0,
                                             0, lp.data_ptr(), ent.data_ptr(), lse.data_ptr(), None, None, ws.data_ptr(),
                                             ws.numel(), _lib.stream_ptr()))
         ctx.save_for_backward(x, tg, lse, ent)
-        ctx.logits = logits                  # for one backward: the next one over a retained graph recomputes
+        ctx.logits, ctx.kept = logits, kept  # for one backward: the next one over a retained graph recomputes
         ctx.model, ctx.temperature, ctx.chunk_rows = model, float(temperature), int(chunk_rows)
         return lp, ent
 
@@ -216,19 +224,20 @@ class _NativeHead(torch.autograd.Function):
                 ops.wgrad(gW, dz, xs)
             return dx, None, None, None, None
         logits, ctx.logits = ctx.logits, None
-        kept = 0 if logits is None else logits.shape[0]
+        kept = 0 if logits is None else M if ctx.kept == M else ctx.kept // Cn * Cn
         wp, wlp = W.data_ptr(), W_lo.data_ptr() if W_lo is not None else None
-        # the kept rows are one chunk (d logits take their place), the others come through a buffer of their own
-        chunks = ([(0, kept)] if kept else []) + [(r0, min(r0 + Cn, M)) for r0 in range(kept, M, Cn)]
-        dz_buf = torch.empty((Cn + 63) // 64 * 64, V, dtype=torch.bfloat16, device=dev) if kept < M else None
-        most = max(r1 - r0 for r0, r1 in chunks)
+        dz_buf = None
         if M > 256:
-            xc = torch.empty((most + 63) // 64 * 64, K, dtype=torch.bfloat16, device=dev)
-            dxc = torch.empty(most, K, dtype=torch.bfloat16, device=dev)
-            index = torch.empty(3 * most + 1, dtype=torch.int32, device=dev)
-        for r0, r1 in chunks:
+            xc = torch.empty((Cn + 63) // 64 * 64, K, dtype=torch.bfloat16, device=dev)
+            dxc = torch.empty(Cn, K, dtype=torch.bfloat16, device=dev)
+            index = torch.empty(3 * Cn + 1, dtype=torch.int32, device=dev)
+        for r0 in range(0, M, Cn):
+            r1 = min(r0 + Cn, M)
             n = r1 - r0
             xs = x[r0:r1]
+            if r0 >= kept and dz_buf is None:        # d logits of kept rows take the logits' place, the others have a buffer of their own
+                logits = None
+                dz_buf = torch.empty((Cn + 63) // 64 * 64, V, dtype=torch.bfloat16, device=dev)
             at = (tg[r0:r1].data_ptr(), lse[r0:r1].data_ptr(), ent[r0:r1].data_ptr(), g_lp[r0:r1].data_ptr(),
                   g_ent[r0:r1].data_ptr() if use_ent else None)
             if M <= 256:
@@ -241,7 +250,7 @@ class _NativeHead(torch.autograd.Function):
             place, count = rows + 4 * n, rows + 12 * n
             _lib.check(lib.prl_live_rows(at[3], at[4], at[1], at[2], n, rows, st))
             if r1 <= kept:
-                dz, ld, k_rows = logits.data_ptr(), 2 * V, n
+                dz, ld, k_rows = logits.data_ptr() + 4 * r0 * V, 2 * V, (n + 63) // 64 * 64 if r1 == M else n
                 _lib.check(lib.prl_head_dlogits_kept(dz, V, n, V, ctx.temperature, rows, count, *at, st))
             else:
                 dz, ld, k_rows = dz_buf.data_ptr(), V, (n + 63) // 64 * 64
@@ -333,7 +342,8 @@ class NativeQwen2(torch.nn.Module):
         hidden = self.hidden_states(batch.input_ids, batch.position_ids if batch.is_packed else None)
         lps, ents = [], []
         for b in range(hidden.shape[0]):
-            lp, ent = _NativeHead.apply(hidden[b, :-1], self, batch.input_ids[b, 1:], temperature, 2048)
+            lp, ent = _NativeHead.apply(hidden[b, :-1], self, batch.input_ids[b, 1:], temperature,
+                                       _NativeHead._chunk_rows(hidden.shape[1] - 1))
             lps.append(lp)
             ents.append(ent)
         return torch.stack(lps), torch.stack(ents)

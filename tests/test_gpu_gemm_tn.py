@@ -583,6 +583,29 @@ def test_head_backward_of_kept_logits_and_live_rows(cuda_device, monkeypatch, M,
             assert ((d - dz.T @ x.double()).abs() <= 2.0 ** -8 * (size.T @ x.double().abs()) + 2.0 ** -21).all()
 
 
+@pytest.mark.parametrize("M,V,K,chunk", [(700, 1032, 256, 200), (640, 264, 72, 256), (513, 2056, 128, 128), (257, 520, 64, 2048)])
+def test_head_gradients_do_not_depend_on_what_is_kept(cuda_device, monkeypatch, M, V, K, chunk):
+    """d hidden and dW have the same bits whether the memory held the logits of all rows, of the first chunks, of none, or the buffer was refused: dW is summed chunk
+    by chunk in any case."""
+    import types
+    from pipelinerl_b200.learner_body import Ops
+    from pipelinerl_b200.learner_model import _NativeHead
+    dev, g = cuda_device, torch.Generator(device=cuda_device).manual_seed(M + V)
+    x, W, lo = (torch.randn(n, K, generator=g, device=dev).to(torch.bfloat16) * s for n, s in ((M, 1.0), (V, 0.1), (V, 0.0005)))
+    tg, on = torch.randint(0, V, (M,), generator=g, device=dev), (torch.rand(M, generator=g, device=dev) < 0.7).float()
+    got = []
+    for kept in (0, chunk, 2 * chunk, M, 1 << 36):           # the last is more than any memory: the forward goes on without a buffer
+        if kept <= M or kept == 1 << 36:
+            monkeypatch.setattr(_NativeHead, "_rows_to_keep", staticmethod(lambda *a: kept))
+            gW = torch.full((V, K), 0.25, device=dev)
+            model = types.SimpleNamespace(p=lambda n: W, head_lo=lo, body=types.SimpleNamespace(ops=Ops(), g={"lm_head.weight": gW}))
+            h = x.clone().requires_grad_()
+            lp, ent = _NativeHead.apply(h, model, tg, 0.8, chunk)
+            torch.autograd.backward([lp, ent], [on * 0.5, on * 0.1])
+            got.append((h.grad, gW, lp.detach(), ent.detach()))
+    assert len(got) >= 3 and all(torch.equal(a, b) for other in got[1:] for a, b in zip(got[0], other)) and got[0][1].std() > 0
+
+
 @pytest.mark.parametrize("M,kept", [(300, 0), (300, 300), (200, 0)])
 def test_head_backward_of_a_masked_row_that_is_no_number(cuda_device, monkeypatch, M, kept):
     """A token without a gradient whose hidden state is not a number: its d hidden and dW are none either (0 x NaN), the other rows' stay what they are."""
