@@ -136,7 +136,8 @@ class _NativeHead(torch.autograd.Function):
     def _chunk_rows(M: int) -> int:
         """Rows whose dW is one sum: all up to 4096, more in equal chunks.  A chunk reads and writes the fp32 gradients of all weights (2.2 GB: 3071 rows in
         two chunks 19.3 ms a step, in one 18.1) and, where its logits are not kept, holds its d logits (0.6 GB for 2048 rows)."""
-        n = max(1, -(-M // 4096))
+        M = max(M, 1)
+        n = -(-M // 4096)
         return (-(-M // n) + 63) // 64 * 64
 
     @staticmethod
