@@ -16,9 +16,11 @@ arena layout and can be pushed as raw bytes.
 """
 from __future__ import annotations
 
+import itertools
 import math
 import os
 import types
+import weakref
 
 import torch
 import torch.nn.functional as F
@@ -120,6 +122,11 @@ class TorchQwen2(torch.nn.Module):
         return (hf * torch.rsqrt((hf * hf).mean(-1, keepdim=True) + self.cfg.rms_eps)).to(h.dtype) * g
 
 
+# logits that wait for their backward
+_KEPT: "weakref.WeakValueDictionary[int, torch.Tensor]" = weakref.WeakValueDictionary()
+_KEPT_KEYS = itertools.count()
+
+
 class _NativeHead(torch.autograd.Function):
     """Final projection + log-softmax statistics of the native learner.  Forward: one tcgen05 GEMM whose epilogue
     reduces logits in TMEM (prl_head_logprob) and, where memory allows, stores them for the backward.  Backward, per chunk of
@@ -141,15 +148,16 @@ class _NativeHead(torch.autograd.Function):
         return (-(-M // n) + 63) // 64 * 64
 
     @staticmethod
-    def _rows_to_keep(M: int, V: int, dev, chunk: int = 256) -> int:
-        """Rows whose fp32 logits (4 V bytes each) the forward stores: at most a quarter of the memory that is free now, so that
-        what the backward allocates beside them finds its place; few rows are not worth a buffer, since the products' time is the
-        weights' way through the memory then (up to 256 rows: one row tile).  All rows or whole chunks: memory decides where a chunk's d logits come
-        from, and nothing of how dW is summed."""
+    def _rows_to_keep(M: int, V: int, dev, chunk: int = 256, held: int = 0) -> int:
+        """Rows whose fp32 logits (4 V bytes each) the forward stores: at most a quarter of the memory that is free now for all
+        rows of a batch together (`held`: bytes that the others keep already), so that what the backward allocates beside them
+        finds its place; few rows are not worth a buffer, since the products' time is the weights' way through the memory then
+        (up to 256 rows: one row tile).  All rows or whole chunks: memory decides where a chunk's d logits come from, and nothing
+        of how dW is summed."""
         if M <= 256 or V % 8:
             return 0
         free = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
-        rows = min(M, free // 4 // (4 * V))
+        rows = min(M, max(0, (free + held) // 4 - held) // (4 * V))
         return rows if rows == M else rows // chunk * chunk
 
     @staticmethod
@@ -166,10 +174,12 @@ class _NativeHead(torch.autograd.Function):
         W_lo = model.head_lo
         logits, kept = None, 0
         if ctx.needs_input_grad[0]:
-            kept = _NativeHead._rows_to_keep(M, V, x.device, chunk_rows)
+            held = sum(4 * t.numel() for t in list(_KEPT.values()) if t.device == x.device)
+            kept = _NativeHead._rows_to_keep(M, V, x.device, chunk_rows, held)
             if kept:
                 try:                                     # the last chunk's d logits end on a whole k-block
                     logits = torch.empty((kept + 63) // 64 * 64 if kept == M else kept, V, dtype=torch.float32, device=x.device)
+                    _KEPT[next(_KEPT_KEYS)] = logits
                 except torch.cuda.OutOfMemoryError:      # free memory in pieces: the backward recomputes
                     kept = 0
         if logits is not None:
@@ -232,13 +242,21 @@ class _NativeHead(torch.autograd.Function):
             xc = torch.empty((Cn + 63) // 64 * 64, K, dtype=torch.bfloat16, device=dev)
             dxc = torch.empty(Cn, K, dtype=torch.bfloat16, device=dev)
             index = torch.empty(3 * Cn + 1, dtype=torch.int32, device=dev)
-        for r0 in range(0, M, Cn):
+        r1 = 0
+        while r1 < M:
+            r0 = r1
+            if r0 >= kept and dz_buf is None:        # d logits of kept rows take the logits' place, the others have a buffer of their own
+                logits = None
+                while dz_buf is None:
+                    try:
+                        dz_buf = torch.empty((Cn + 63) // 64 * 64, V, dtype=torch.bfloat16, device=dev)
+                    except torch.cuda.OutOfMemoryError:      # no room for a chunk: half of it at a time, dW in as many sums more
+                        if Cn <= 256:
+                            raise
+                        Cn = max(256, Cn // 2 // 64 * 64)
             r1 = min(r0 + Cn, M)
             n = r1 - r0
             xs = x[r0:r1]
-            if r0 >= kept and dz_buf is None:        # d logits of kept rows take the logits' place, the others have a buffer of their own
-                logits = None
-                dz_buf = torch.empty((Cn + 63) // 64 * 64, V, dtype=torch.bfloat16, device=dev)
             at = (tg[r0:r1].data_ptr(), lse[r0:r1].data_ptr(), ent[r0:r1].data_ptr(), g_lp[r0:r1].data_ptr(),
                   g_ent[r0:r1].data_ptr() if use_ent else None)
             if M <= 256:

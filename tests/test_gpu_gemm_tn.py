@@ -606,6 +606,44 @@ def test_head_gradients_do_not_depend_on_what_is_kept(cuda_device, monkeypatch, 
     assert len(got) >= 3 and all(torch.equal(a, b) for other in got[1:] for a, b in zip(got[0], other)) and got[0][1].std() > 0
 
 
+def test_head_backward_with_little_memory(cuda_device, monkeypatch):
+    """Logits that wait for a backward count as held until it took them; where a chunk's d logits find no room the chunk is halved."""
+    import types
+    from pipelinerl_b200 import learner_model
+    from pipelinerl_b200.learner_body import Ops
+    dev, M, V, K = cuda_device, 1100, 520, 64
+    g = torch.Generator(device=dev).manual_seed(3)
+    x, W = (torch.randn(n, K, generator=g, device=dev).to(torch.bfloat16) for n in (M, V))
+    tg = torch.randint(0, V, (M,), generator=g, device=dev)
+    empty, seen, asked = torch.empty, [], []
+
+    def keep(M_, V_, d, chunk, held):
+        seen.append(held)
+        return M if len(seen) < 3 else 0
+
+    def small(*a, **k):
+        if k.get("dtype") == torch.bfloat16 and a[1:] == (V,):
+            asked.append(a[0])
+            if a[0] > 320:
+                raise torch.cuda.OutOfMemoryError("no room")
+        return empty(*a, **k)
+
+    monkeypatch.setattr(learner_model._NativeHead, "_rows_to_keep", staticmethod(keep))
+    gW = [torch.zeros(V, K, device=dev) for _ in range(3)]
+    hs = [x.clone().requires_grad_() for _ in range(3)]
+    outs = [learner_model._NativeHead.apply(h, types.SimpleNamespace(p=lambda n: W, head_lo=None, body=types.SimpleNamespace(ops=Ops(), g={"lm_head.weight": w})),
+                                            tg, 1.0, 1152) for h, w in zip(hs, gW)]
+    one = 4 * 1152 * V
+    assert seen == [0, one, 2 * one]
+    for lp, ent in outs[:2]:
+        torch.autograd.backward([lp, ent], [torch.ones_like(lp), torch.ones_like(ent)])
+    assert not list(learner_model._KEPT.values())
+    monkeypatch.setattr(torch, "empty", small)
+    torch.autograd.backward(outs[2], [torch.ones_like(outs[2][0]), torch.ones_like(outs[2][1])])
+    assert asked == [1152, 512, 256] and torch.equal(hs[2].grad, hs[0].grad) and torch.equal(gW[0], gW[1])
+    assert (gW[2] - gW[0]).norm() <= M * 2.0 ** -24 * gW[0].norm()          # the same M fp32 terms in more sums
+
+
 @pytest.mark.parametrize("M,kept", [(300, 0), (300, 300), (200, 0)])
 def test_head_backward_of_a_masked_row_that_is_no_number(cuda_device, monkeypatch, M, kept):
     """A token without a gradient whose hidden state is not a number: its d hidden and dW are none either (0 x NaN), the other rows' stay what they are."""

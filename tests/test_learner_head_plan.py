@@ -19,3 +19,15 @@ def test_rows_whose_logits_are_kept(monkeypatch, M, V, chunk, free_gb, rows):
     monkeypatch.setattr(torch.cuda, "memory_reserved", lambda dev: 13 * 10 ** 9)
     monkeypatch.setattr(torch.cuda, "memory_allocated", lambda dev: 10 ** 10)
     assert _NativeHead._rows_to_keep(M, V, None, chunk) == rows
+
+
+@pytest.mark.parametrize("rows", [1, 3, 8])
+def test_kept_logits_of_a_batch_share_a_quarter(monkeypatch, rows):
+    """Row after row of a batch, each with less memory left: together they take no more than a quarter of what was free before the first."""
+    free, held, M, V = 40 * 10 ** 9, 0, 4096, 152064
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda dev: (free - held, 0))
+    monkeypatch.setattr(torch.cuda, "memory_reserved", lambda dev: held)
+    monkeypatch.setattr(torch.cuda, "memory_allocated", lambda dev: held)
+    for _ in range(rows):
+        held += 4 * V * _NativeHead._rows_to_keep(M, V, None, M, held)
+    assert held == 4 * V * M * min(rows, 4) <= free // 4
