@@ -122,6 +122,10 @@ class TorchQwen2(torch.nn.Module):
         return (hf * torch.rsqrt((hf * hf).mean(-1, keepdim=True) + self.cfg.rms_eps)).to(h.dtype) * g
 
 
+def _fused_head_bwd() -> bool:
+    return os.environ.get("PRL_HEAD_BWD_FUSED", "1") != "0"
+
+
 # logits that wait for their backward
 _KEPT: "weakref.WeakValueDictionary[int, torch.Tensor]" = weakref.WeakValueDictionary()
 _KEPT_KEYS = itertools.count()
@@ -173,7 +177,7 @@ class _NativeHead(torch.autograd.Function):
         ws = torch.empty(int(lib.prl_head_workspace_bytes(M, V)), dtype=torch.uint8, device=x.device)
         W_lo = model.head_lo
         logits, kept = None, 0
-        if ctx.needs_input_grad[0]:
+        if ctx.needs_input_grad[0] and _fused_head_bwd():        # the other formulation recomputes
             held = sum(4 * t.numel() for t in list(_KEPT.values()) if t.device == x.device)
             kept = _NativeHead._rows_to_keep(M, V, x.device, chunk_rows, held)
             if kept:
@@ -215,7 +219,8 @@ class _NativeHead(torch.autograd.Function):
         # (the reference's autograd keeps 608 KB of them per token alive)
         st = _lib.stream_ptr()
         W_lo = model.head_lo
-        if os.environ.get("PRL_HEAD_BWD_FUSED", "1") == "0":
+        if not _fused_head_bwd():
+            ctx.logits = None
             # A/B only: the previous formulation -- logits recomputed (hi GEMM, lo GEMM accumulating), one row kernel, a cast
             logits_buf = torch.empty(Cn, V, dtype=torch.float32, device=dev)
             dlogits_buf = torch.empty(Cn, V, dtype=torch.float32, device=dev)

@@ -606,6 +606,28 @@ def test_head_gradients_do_not_depend_on_what_is_kept(cuda_device, monkeypatch, 
     assert len(got) >= 3 and all(torch.equal(a, b) for other in got[1:] for a, b in zip(got[0], other)) and got[0][1].std() > 0
 
 
+def test_former_head_backward_keeps_no_logits(cuda_device, monkeypatch):
+    """PRL_HEAD_BWD_FUSED=0 recomputes: nothing is stored for it, and what a forward before the switch stored is let go."""
+    import types
+    from pipelinerl_b200 import learner_model
+    from pipelinerl_b200.learner_body import Ops
+    dev, M, V, K = cuda_device, 300, 520, 64
+    g = torch.Generator(device=dev).manual_seed(3)
+    x, W = (torch.randn(n, K, generator=g, device=dev).to(torch.bfloat16) for n in (M, V))
+    tg, got = torch.randint(0, V, (M,), generator=g, device=dev), []
+    for before, after in (("1", "1"), ("0", "0"), ("1", "0")):
+        monkeypatch.setenv("PRL_HEAD_BWD_FUSED", before)
+        model = types.SimpleNamespace(p=lambda n: W, head_lo=None, body=types.SimpleNamespace(ops=Ops(), g={"lm_head.weight": torch.zeros(V, K, device=dev)}))
+        h = x.clone().requires_grad_()
+        lp, ent = learner_model._NativeHead.apply(h, model, tg, 1.0, 320)
+        assert len(learner_model._KEPT) == int(before)
+        monkeypatch.setenv("PRL_HEAD_BWD_FUSED", after)
+        torch.autograd.backward([lp, ent], [torch.ones_like(lp), torch.ones_like(ent)], retain_graph=True)
+        assert not len(learner_model._KEPT)
+        got.append(h.grad)
+    assert torch.equal(got[1], got[2]) and (got[0] - got[1]).abs().max() <= 2.0 ** -6 * got[1].abs().max()
+
+
 def test_head_backward_with_little_memory(cuda_device, monkeypatch):
     """Logits that wait for a backward count as held until it took them; where a chunk's d logits find no room the chunk is halved."""
     import types
