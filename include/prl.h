@@ -461,6 +461,19 @@ int prl_paged_attn_decode_qkv(const float* partials, int32_t n_split, const void
                               const int32_t* block_table, int32_t max_blocks, const int32_t* seq_lens, int32_t B, int32_t n_q,
                               int32_t n_kv, int32_t head_dim, int32_t page_size, int32_t n_splits, float sm_scale, void* out_bf16,
                               void* workspace, size_t workspace_bytes, prl_stream_t stream);
+/* Shares and ring stages for a batch of `slots` of which `live` (1 .. slots) have a token, in contexts of up to `longest` keys (fewer, if they are
+ * of unequal lengths: as many as the longest would make of all pages); live = slots and longest = max_seq_len give prl_paged_attn_splits.  The
+ * workspace is for the most shares asked for.  The two entries take what it gave: stages 3 or 6 pages in flight per CTA (the same bits), 0 as above. */
+int prl_paged_attn_plan(int32_t slots, int32_t live, int32_t n_kv, int32_t longest, int32_t max_seq_len, int32_t* stages);
+int prl_paged_attn_decode_planned(const void* q_bf16, const void* kv_cache_bf16, int64_t n_pages, int32_t n_layers, int32_t layer,
+                                  const int32_t* block_table, int32_t max_blocks, const int32_t* seq_lens, int32_t B, int32_t n_q, int32_t n_kv,
+                                  int32_t head_dim, int32_t page_size, int32_t n_splits, int32_t stages, float sm_scale, void* out_bf16,
+                                  void* workspace, size_t workspace_bytes, prl_stream_t stream);
+int prl_paged_attn_decode_qkv_planned(const float* partials, int32_t n_split, const void* bias, const float* inv_freq, void* kv_cache_bf16,
+                                      int64_t n_pages, int32_t n_layers, int32_t layer, const int32_t* block_table, int32_t max_blocks,
+                                      const int32_t* seq_lens, int32_t B, int32_t n_q, int32_t n_kv, int32_t head_dim, int32_t page_size,
+                                      int32_t n_splits, int32_t stages, float sm_scale, void* out_bf16, void* workspace, size_t workspace_bytes,
+                                      prl_stream_t stream);
 /* Chunked prefill: causal attention of seq_q_len[z] query rows (starting at row seq_q_start[z], first
  * position seq_pos0[z]) against the paged KV of block-table row seq_slot[z]; the chunk's own K/V must
  * already be in the cache (prl_qkv_rope_cache).  Replaces vLLM's chunked-prefill attention

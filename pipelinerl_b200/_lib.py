@@ -208,6 +208,12 @@ _SIGNATURES = {
     "prl_paged_attn_decode_qkv": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32,
                                             C.c_void_p, C.c_int32, C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int32,
                                             C.c_int32, C.c_int32, C.c_float, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),
+    "prl_paged_attn_plan": (C.c_int, [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.POINTER(C.c_int32)]),
+    "prl_paged_attn_decode_planned": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32, C.c_void_p, C.c_int32, C.c_void_p] +
+                                      [C.c_int32] * 7 + [C.c_float, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),
+    "prl_paged_attn_decode_qkv_planned": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32,
+                                                    C.c_void_p, C.c_int32, C.c_void_p] + [C.c_int32] * 7 +
+                                          [C.c_float, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),
     "prl_sample_workspace_bytes": (C.c_size_t, [C.c_int32]),
     "prl_sample_logprob": (C.c_int, [C.c_void_p, C.c_int32, C.c_int32, C.c_float, C.c_int32, C.c_uint64,
                                      C.c_uint32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),

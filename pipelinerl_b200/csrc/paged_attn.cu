@@ -627,16 +627,37 @@ extern "C" int prl_attn_set_fused_combine(int32_t on) {
 }
 
 // Shares that a context is cut into.  A share costs a start, a merge and its part of the combine kernel, so contexts are cut
-// while the CTAs stay one per SM (pages of 64 keys, us by 1 / 2 / 4 / 8 / 16): 4 CTAs of 47 pages 18.9 / 13.2 / 10.3 / 8.3 / 8.4, 24 of 11 10.6 / 10.6 /
-// 9.4, 48 of 8 9.0 / 10.2, 64 of 47 22.8 / 20.1 / 19.5 / 23.3, 128 of 63 39.0 / 40.8.  One more cut where long contexts leave SMs idle or unevenly filled: 96
-// of 125 60.5 / 56.2, 256 of 129 145 / 137, 256 of 86 100 / 94, but 256 of 47 55.9 / 58.7, of 10 16.3 / 21.4, 160 of 128 96 / 106, 512 of 125 255 / 268.
+// while the CTAs stay one per SM (pages of 64 keys, us by 1 / 2 / 4 / 8 / 16): 4 CTAs of 47 pages 18.9 / 13.2 / 10.3 / 8.3 / 8.4, 24 of
+// 11 10.6 / 10.6 / 9.4, 48 of 8 9.0 / 10.2, 64 of 47 22.8 / 20.1 / 19.5 / 23.3, 128 of 63 39.0 / 40.8.  From 16 on the combine kernel's walk over the shares
+// counts, which grows with their number and is paid by each head (us by 16 / 32 / 64): one CTA of 64 pages 7.2 / 7.7 / 9.8, of 128 8.9 / 8.5 /
+// 10.2, of 256 12.1 / 10.2 / 11.3, of 1024 31.1 / 20.3 / 17.8; two of 128 9.6 / 9.6 / 12.2, of 256 12.9 / 11.8 / 14.2, of 2048 56.2 / 33.4 /
+// 31.3; four of 256 13.2 / 13.5 / 19.9, of 1024 32.0 / 28.0 / 34.8.  One more cut where long contexts leave SMs idle or unevenly filled: 96 of 125 60.5 / 56.2,
+// 256 of 129 145 / 137, 256 of 86 100 / 94, but 256 of 47 55.9 / 58.7, of 10 16.3 / 21.4, 160 of 128 96 / 106, 512 of 125 255 / 268.
+static int cuts_of(int ctas, int pages) {
+  const int sms = num_sms();
+  int s = 1;
+  while (s < 64 && ctas * s * 2 <= sms && pages > 8 && pages >= 5 * s && (s < 16 || (int64_t)4 * pages > (int64_t)s * s * ctas)) s *= 2;
+  if (s == 1 && ((ctas <= sms && pages >= 96) || (4 * ctas > 5 * sms && ctas <= 2 * sms && pages >= 64))) s = 2;
+  return s;
+}
+
 extern "C" int prl_paged_attn_splits(int32_t B, int32_t n_kv, int32_t max_seq_len) {
   const int pages = (max_seq_len + kPage - 1) / kPage;
-  const int sms = num_sms(), ctas = B * n_kv;
-  int splits = 1;
-  while (splits < 16 && ctas * splits * 2 <= sms && pages > 8 && pages >= 5 * splits) splits *= 2;
-  if (splits == 1 && ((ctas <= sms && pages >= 96) || (4 * ctas > 5 * sms && ctas <= 2 * sms && pages >= 64))) splits = 2;
+  int splits = cuts_of(B * n_kv, pages);
   while ((pages + splits - 1) / splits > kMaxPagesPerSplit) splits *= 2;
+  return splits;
+}
+
+// The same for `slots` of which `live` have a token, in contexts of up to `longest` (fewer, if they are of unequal lengths: as many as the longest
+// would make of all pages), and the ring's stages for it.  Slots without a token cost a CTA's start per share, so shares beyond those of full slots stay
+// below four CTAs per SM.  us a layer, 4 key heads, by the capacity / by what is there: one of 16 x 16384 56 / 18.6, four of 32 x
+// 4096 28.8 / 12.8, and with six stages for three, where the live CTAs have an SM each: eight of 64 x 8192 42.6 / 32.4.
+extern "C" int prl_paged_attn_plan(int32_t slots, int32_t live, int32_t n_kv, int32_t longest, int32_t max_seq_len, int32_t* stages) {
+  const int sms = num_sms(), full = prl_paged_attn_splits(slots, n_kv, max_seq_len);
+  int splits = cuts_of(live * n_kv, (longest + kPage - 1) / kPage);
+  while (splits > full && slots * n_kv * splits >= 4 * sms) splits /= 2;
+  while (((max_seq_len + kPage - 1) / kPage + splits - 1) / splits > kMaxPagesPerSplit) splits *= 2;
+  if (stages) *stages = live * n_kv * splits > sms ? kStages / 2 : kStages;
   return splits;
 }
 
@@ -647,12 +668,13 @@ extern "C" size_t prl_paged_attn_workspace_bytes(int32_t B, int32_t n_q, int32_t
 
 static int paged_attn_decode_impl(const void* q, const NewToken& fresh, const void* kv_cache, int64_t n_pages, int32_t n_layers, int32_t layer,
                                   const int32_t* block_table, int32_t max_blocks, const int32_t* seq_lens, int32_t B, int32_t n_q, int32_t n_kv,
-                                  int32_t head_dim, int32_t page_size, int32_t n_splits, float sm_scale, void* out_bf16, void* workspace,
+                                  int32_t head_dim, int32_t page_size, int32_t n_splits, int32_t stages, float sm_scale, void* out_bf16, void* workspace,
                                   size_t workspace_bytes, prl_stream_t stream_) {
   PRL_CHECK_ARG((q || fresh.part) && kv_cache && block_table && seq_lens && out_bf16 && workspace, "prl_paged_attn_decode: NULL argument");
   PRL_CHECK_ARG(head_dim == kD && page_size == kPage, "prl_paged_attn_decode: head_dim must be 128 and page_size 64");
   PRL_CHECK_ARG(B >= 1 && n_kv >= 1 && n_q % n_kv == 0 && n_q / n_kv <= 16, "prl_paged_attn_decode: need n_q/n_kv <= 16");
   PRL_CHECK_ARG(n_splits >= 1 && layer >= 0 && layer < n_layers, "prl_paged_attn_decode: bad layer/splits");
+  PRL_CHECK_ARG(stages == 0 || stages == kStages / 2 || stages == kStages, "prl_paged_attn_decode: stages are 3 or 6");
   PRL_CHECK_ARG((max_blocks + n_splits - 1) / n_splits <= kMaxPagesPerSplit,
                 "prl_paged_attn_decode: %d blocks / %d splits exceeds %d pages per CTA", max_blocks, n_splits,
                 kMaxPagesPerSplit);
@@ -671,13 +693,14 @@ static int paged_attn_decode_impl(const void* q, const NewToken& fresh, const vo
   p.scale_log2 = sm_scale * 1.4426950408889634f;
   p.o_part = (float*)workspace;
   p.ml_part = p.o_part + (size_t)B * n_q * n_splits * kD;
-  p.tickets = g_fused_combine ? reinterpret_cast<unsigned int*>(p.ml_part + (size_t)B * n_q * n_splits * 2) : nullptr;
+  // the workspace's last words, whatever n_splits: one that is made for more shares is no other place for them
+  p.tickets = g_fused_combine ? reinterpret_cast<unsigned int*>((uint8_t*)workspace + (workspace_bytes & ~(size_t)3)) - (size_t)B * n_q : nullptr;
   p.out = (__nv_bfloat16*)out_bf16;
   p.direct = n_splits == 1;    // 4 x 333 keys, eight layers: one launch of nine a layer less, 285 -> 274 us a step
   if (p.direct) p.tickets = nullptr;
   // Six stages for a CTA that has its SM alone, three where there are more CTAs than SMs: as many bytes under way, and one's start and
   // merge under the other's pages (us: 64 x 600 keys of 4 heads by two 25.8 -> 21.6, 64 x 200 12.6 -> 10.1, 64 x 7000 by two 133 -> 128)
-  const int n_st = (int64_t)n_splits * n_kv * B > num_sms() ? kStages / 2 : kStages;
+  const int n_st = stages ? stages : (int64_t)n_splits * n_kv * B > num_sms() ? kStages / 2 : kStages;
   const int smem = n_st * kStageBytes + 1024 + 8 * 2 * n_st + 4 * kMaxPagesPerSplit + 16;
   static SmemAttr smem_attr[3] = {};
   const int form = fresh.part ? (p.R <= 8 ? 1 : 2) : 0;
@@ -695,14 +718,33 @@ static int paged_attn_decode_impl(const void* q, const NewToken& fresh, const vo
   return PRL_OK;
 }
 
+extern "C" int prl_paged_attn_decode_planned(const void* q, const void* kv_cache, int64_t n_pages, int32_t n_layers, int32_t layer,
+                                             const int32_t* block_table, int32_t max_blocks, const int32_t* seq_lens, int32_t B, int32_t n_q,
+                                             int32_t n_kv, int32_t head_dim, int32_t page_size, int32_t n_splits, int32_t stages, float sm_scale,
+                                             void* out_bf16, void* workspace, size_t workspace_bytes, prl_stream_t stream_) {
+  PRL_CHECK_ARG(q != nullptr, "prl_paged_attn_decode: NULL argument");
+  return paged_attn_decode_impl(q, NewToken{}, kv_cache, n_pages, n_layers, layer, block_table, max_blocks, seq_lens, B, n_q, n_kv, head_dim,
+                                page_size, n_splits, stages, sm_scale, out_bf16, workspace, workspace_bytes, stream_);
+}
+
 extern "C" int prl_paged_attn_decode(const void* q, const void* kv_cache, int64_t n_pages, int32_t n_layers,
                                      int32_t layer, const int32_t* block_table, int32_t max_blocks,
                                      const int32_t* seq_lens, int32_t B, int32_t n_q, int32_t n_kv, int32_t head_dim,
                                      int32_t page_size, int32_t n_splits, float sm_scale, void* out_bf16,
                                      void* workspace, size_t workspace_bytes, prl_stream_t stream_) {
-  PRL_CHECK_ARG(q != nullptr, "prl_paged_attn_decode: NULL argument");
-  return paged_attn_decode_impl(q, NewToken{}, kv_cache, n_pages, n_layers, layer, block_table, max_blocks, seq_lens, B, n_q, n_kv, head_dim,
-                                page_size, n_splits, sm_scale, out_bf16, workspace, workspace_bytes, stream_);
+  return prl_paged_attn_decode_planned(q, kv_cache, n_pages, n_layers, layer, block_table, max_blocks, seq_lens, B, n_q, n_kv, head_dim, page_size,
+                                       n_splits, 0, sm_scale, out_bf16, workspace, workspace_bytes, stream_);
+}
+
+extern "C" int prl_paged_attn_decode_qkv_planned(const float* partials, int32_t n_split, const void* bias, const float* inv_freq, void* kv_cache,
+                                                 int64_t n_pages, int32_t n_layers, int32_t layer, const int32_t* block_table, int32_t max_blocks,
+                                                 const int32_t* seq_lens, int32_t B, int32_t n_q, int32_t n_kv, int32_t head_dim,
+                                                 int32_t page_size, int32_t n_splits, int32_t stages, float sm_scale, void* out_bf16,
+                                                 void* workspace, size_t workspace_bytes, prl_stream_t stream_) {
+  PRL_CHECK_ARG(partials && n_split >= 1 && inv_freq, "prl_paged_attn_decode_qkv: bad argument");
+  const NewToken fresh{partials, n_split, B, (const __nv_bfloat16*)bias, inv_freq, (__nv_bfloat16*)kv_cache};
+  return paged_attn_decode_impl(nullptr, fresh, kv_cache, n_pages, n_layers, layer, block_table, max_blocks, seq_lens, B, n_q, n_kv, head_dim,
+                                page_size, n_splits, stages, sm_scale, out_bf16, workspace, workspace_bytes, stream_);
 }
 
 extern "C" int prl_paged_attn_decode_qkv(const float* partials, int32_t n_split, const void* bias, const float* inv_freq, void* kv_cache,
@@ -710,10 +752,8 @@ extern "C" int prl_paged_attn_decode_qkv(const float* partials, int32_t n_split,
                                          const int32_t* seq_lens, int32_t B, int32_t n_q, int32_t n_kv, int32_t head_dim, int32_t page_size,
                                          int32_t n_splits, float sm_scale, void* out_bf16, void* workspace, size_t workspace_bytes,
                                          prl_stream_t stream_) {
-  PRL_CHECK_ARG(partials && n_split >= 1 && inv_freq, "prl_paged_attn_decode_qkv: bad argument");
-  const NewToken fresh{partials, n_split, B, (const __nv_bfloat16*)bias, inv_freq, (__nv_bfloat16*)kv_cache};
-  return paged_attn_decode_impl(nullptr, fresh, kv_cache, n_pages, n_layers, layer, block_table, max_blocks, seq_lens, B, n_q, n_kv, head_dim,
-                                page_size, n_splits, sm_scale, out_bf16, workspace, workspace_bytes, stream_);
+  return prl_paged_attn_decode_qkv_planned(partials, n_split, bias, inv_freq, kv_cache, n_pages, n_layers, layer, block_table, max_blocks, seq_lens,
+                                           B, n_q, n_kv, head_dim, page_size, n_splits, 0, sm_scale, out_bf16, workspace, workspace_bytes, stream_);
 }
 
 extern "C" int prl_paged_attn_prefill(const void* q, const void* kv_cache, int64_t n_pages, int32_t n_layers,

@@ -48,6 +48,13 @@ class Request:
     waits_for: list = field(default_factory=list)        # [(request filling a shared page, tokens it must reach)]
 
 
+def batch_contexts(lengths: list[int]) -> tuple[int, int]:
+    """(how many contexts as long as the longest make the pages of all of them, the longest): what a batch of unequal contexts is for the
+    rules that ask for a number of equal ones."""
+    pages = [-(-n // PAGE_SIZE) for n in lengths]
+    return -(-sum(pages) // max(pages)), max(lengths)
+
+
 class EngineCore:
     """Everything of a sampler engine that does not depend on the model: slots and KV pages (cache.PagePool /
     cache.SlotStates), admission with page-granular prefix sharing, the chunked-prefill scheduler, the device-resident
@@ -126,6 +133,7 @@ class EngineCore:
         self._hash_of_page: dict[int, int] = {}
         self._tokens_of_page: dict[int, tuple] = {}                   # page -> its 64 tokens (verified on every hit)
         self._page_pending: dict[int, tuple[Request, int]] = {}       # page -> (request that fills it, tokens needed)
+        self._contexts: tuple = (None, None)           # what _batch_contexts made of the requests that are there
         self.stats = {"prefill_tokens": 0, "prefix_hits": 0, "prefix_hit_tokens": 0}
         self.profile_timing = False                    # benches: wall time spent inside run_prefill (costs two syncs per call)
         self._next_id = 0
@@ -235,6 +243,27 @@ class EngineCore:
     def _step_plan(self):
         """What the launches of a token step depend on beside the parameter buffer: a plan is captured as a graph of its own."""
         return None
+
+    def _batch_contexts(self) -> tuple[int, int]:
+        """batch_contexts of the requests that have a slot, each as long as it may become (slots that were filled without a request: all)."""
+        at = (self._next_id, len(self.slot_req))       # a request that comes counts up, one that goes alone leaves fewer
+        if self._contexts[0] != at:
+            reqs = self.slot_req.values()
+            self._contexts = at, batch_contexts([min(self.max_seq_len, len(r.prompt_ids) + r.params.max_tokens) for r in reqs]
+                                                or [self.max_seq_len] * self.B)
+        return self._contexts[1]
+
+    def _attn_plan(self, n_kv: int) -> tuple[int, int]:
+        """Decode attention's shares of a context and ring stages, by the requests that are there: a batch that drains, or one long sequence beside
+        short ones, has its contexts cut further than full slots have (prl_paged_attn_plan), and its step is captured again.  The
+        shares' partial sums are merged in fp32: outputs move in their last bits with the plan."""
+        stages = C.c_int32()
+        live, longest = self._batch_contexts()
+        return int(self.lib.prl_paged_attn_plan(self.B, live, n_kv, longest, self.max_seq_len, C.byref(stages))), stages.value
+
+    def _attn_most_splits(self, n_kv: int) -> int:
+        """The most shares of any plan: of the longest contexts, for some number of them."""
+        return max(int(self.lib.prl_paged_attn_plan(self.B, live, n_kv, self.max_seq_len, self.max_seq_len, None)) for live in range(1, self.B + 1))
 
     def set_arena(self, arena: ParamArena) -> None:
         """Switch the parameter buffer between two token steps (weight update flip).  Graphs are cached per
@@ -589,7 +618,7 @@ class DecodeEngine(EngineCore):
                                                    / cfg.head_dim))).to(d)
         self._plan_gemms()
         self.attn_splits = int(self.lib.prl_paged_attn_splits(B, cfg.num_kv_heads, self.max_seq_len))
-        self.attn_ws = torch.zeros(int(self.lib.prl_paged_attn_workspace_bytes(B, cfg.num_q_heads, self.attn_splits)),
+        self.attn_ws = torch.zeros(int(self.lib.prl_paged_attn_workspace_bytes(B, cfg.num_q_heads, self._attn_most_splits(cfg.num_kv_heads))),
                                    dtype=torch.uint8, device=d)
         self.head_ws = torch.zeros(int(self.lib.prl_head_workspace_bytes(B, cfg.vocab_size)), dtype=torch.uint8, device=d)
 
@@ -648,6 +677,9 @@ class DecodeEngine(EngineCore):
                                                  x.data_ptr(), self.B if m is None else m, n, k, split,
                                                  out.data_ptr(), self._st))
 
+    def _step_plan(self):
+        return self._attn_plan(self.cfg.num_kv_heads)
+
     def _step_kernels(self) -> None:
         """Enqueue one token step for all B slots on the current stream (graph-capturable)."""
         cfg, lib, B, a = self.cfg, self.lib, self.B, self.arena
@@ -666,16 +698,19 @@ class DecodeEngine(EngineCore):
                                          a.ptr("layers.0.input_layernorm.weight"), cfg.rms_eps, B, H, cfg.vocab_size,
                                          self.h.data_ptr(), self.x.data_ptr(), st))
         sm_scale = 1.0 / math.sqrt(cfg.head_dim)
+        splits, stages = self._attn_plan(cfg.num_kv_heads)
         for l in range(cfg.num_layers):
             p = f"layers.{l}."
             if "gemm" not in skip:
                 self._gemm(p + "qkv_proj.weight", self.x, cfg.qkv_size, H, self.split_k["qkv"], part)
             if not skip and not pf:
-                _lib.check(lib.prl_paged_attn_decode_qkv(part.data_ptr(), self.split_k["qkv"], a.ptr(p + "qkv_proj.bias") if cfg.qkv_bias else None,
-                                                         self.inv_freq.data_ptr(), self.kv_cache.data_ptr(), self.n_pages, cfg.num_layers, l,
-                                                         self.block_table.data_ptr(), self.max_blocks, self.seq_lens.data_ptr(), B,
-                                                         cfg.num_q_heads, cfg.num_kv_heads, cfg.head_dim, PAGE_SIZE, self.attn_splits, sm_scale,
-                                                         self.attn_out.data_ptr(), self.attn_ws.data_ptr(), self.attn_ws.numel(), st))
+                _lib.check(lib.prl_paged_attn_decode_qkv_planned(part.data_ptr(), self.split_k["qkv"],
+                                                                 a.ptr(p + "qkv_proj.bias") if cfg.qkv_bias else None, self.inv_freq.data_ptr(),
+                                                                 self.kv_cache.data_ptr(), self.n_pages, cfg.num_layers, l,
+                                                                 self.block_table.data_ptr(), self.max_blocks, self.seq_lens.data_ptr(), B,
+                                                                 cfg.num_q_heads, cfg.num_kv_heads, cfg.head_dim, PAGE_SIZE, splits, stages,
+                                                                 sm_scale, self.attn_out.data_ptr(), self.attn_ws.data_ptr(),
+                                                                 self.attn_ws.numel(), st))
             elif "small" not in skip:
                 # while attention streams the KV cache, L2 fetches o_proj's weights
                 _lib.check(lib.prl_qkv_rope_cache(part.data_ptr(), self.split_k["qkv"], B,
@@ -686,12 +721,12 @@ class DecodeEngine(EngineCore):
                                                   self.n_pages, l, PAGE_SIZE,
                                                   a.ptr(p + "o_proj.weight") if pf else None, wbytes(p + "o_proj.weight"), st))
             if (skip or pf) and "attn" not in skip:
-                _lib.check(lib.prl_paged_attn_decode(self.q.data_ptr(), self.kv_cache.data_ptr(), self.n_pages,
-                                                     cfg.num_layers, l, self.block_table.data_ptr(), self.max_blocks,
-                                                     self.seq_lens.data_ptr(), B, cfg.num_q_heads, cfg.num_kv_heads,
-                                                     cfg.head_dim, PAGE_SIZE, self.attn_splits, sm_scale,
-                                                     self.attn_out.data_ptr(), self.attn_ws.data_ptr(),
-                                                     self.attn_ws.numel(), st))
+                _lib.check(lib.prl_paged_attn_decode_planned(self.q.data_ptr(), self.kv_cache.data_ptr(), self.n_pages,
+                                                             cfg.num_layers, l, self.block_table.data_ptr(), self.max_blocks,
+                                                             self.seq_lens.data_ptr(), B, cfg.num_q_heads, cfg.num_kv_heads,
+                                                             cfg.head_dim, PAGE_SIZE, splits, stages, sm_scale,
+                                                             self.attn_out.data_ptr(), self.attn_ws.data_ptr(),
+                                                             self.attn_ws.numel(), st))
             if "gemm" not in skip:
                 self._gemm(p + "o_proj.weight", self.attn_out, H, cfg.q_size, self.split_k["o"], part)
             if "small" not in skip:

@@ -1464,7 +1464,7 @@ class HybridEngine(EngineCore):
             if on:
                 a = cfg.layers[i].attn
                 self.attn_splits[i] = int(lib.prl_paged_attn_splits(B, a.kv_heads, self.max_seq_len))
-                ws = max(ws, int(lib.prl_paged_attn_workspace_bytes(B, a.heads, self.attn_splits[i])))
+                ws = max(ws, int(lib.prl_paged_attn_workspace_bytes(B, a.heads, self._attn_most_splits(a.kv_heads))))
         for L in cfg.layers:                              # latent attention: the key splits' shares of a batch of single tokens
             if L.latent is not None:
                 for n_seg in range(1, max(B, 4) + 1):     # the split count falls as the batch grows; the product need not
@@ -1611,10 +1611,10 @@ class HybridEngine(EngineCore):
                 if self.tc_attn[i] and not self.force_plain_attn:
                     kv = self.k_pool[i].data_ptr()       # K pool, V pool right behind it (one "layer" of the Qwen2 pool layout)
                     if decode:
-                        _lib.check(lib.prl_paged_attn_decode(R.q.data_ptr(), kv, self.n_pages, 1, 0, self.block_table.data_ptr(),
-                                                             self.max_blocks, self.seq_lens.data_ptr(), n, a.heads, a.kv_heads,
-                                                             a.dim, PAGE_SIZE, self.attn_splits[i], a.scale, R.ob.data_ptr(),
-                                                             self.attn_ws.data_ptr(), self.attn_ws.numel(), st))
+                        _lib.check(lib.prl_paged_attn_decode_planned(R.q.data_ptr(), kv, self.n_pages, 1, 0, self.block_table.data_ptr(),
+                                                                     self.max_blocks, self.seq_lens.data_ptr(), n, a.heads, a.kv_heads,
+                                                                     a.dim, PAGE_SIZE, *self._attn_plan(a.kv_heads), a.scale,
+                                                                     R.ob.data_ptr(), self.attn_ws.data_ptr(), self.attn_ws.numel(), st))
                     else:
                         _lib.check(lib.prl_paged_attn_prefill_tc(R.q.data_ptr(), n, kv, self.n_pages, 1, 0,
                                                                  self.block_table.data_ptr(), self.max_blocks, seg_start,
@@ -1993,9 +1993,9 @@ class HybridEngine(EngineCore):
                                       R.row_slot.data_ptr(), *bt, R.q.data_ptr(), *(kv if own else (None, None)), f32, st))
         if self.tc_attn[i] and not self.force_plain_attn:
             if decode:
-                _lib.check(lib.prl_paged_attn_decode(R.q.data_ptr(), kv[0], self.n_pages, 1, 0, *bt[:2], self.seq_lens.data_ptr(),
-                                                     n, a.heads, a.kv_heads, a.dim, PAGE_SIZE, self.attn_splits[i], a.scale,
-                                                     R.ob.data_ptr(), self.attn_ws.data_ptr(), self.attn_ws.numel(), st))
+                _lib.check(lib.prl_paged_attn_decode_planned(R.q.data_ptr(), kv[0], self.n_pages, 1, 0, *bt[:2], self.seq_lens.data_ptr(),
+                                                             n, a.heads, a.kv_heads, a.dim, PAGE_SIZE, *self._attn_plan(a.kv_heads), a.scale,
+                                                             R.ob.data_ptr(), self.attn_ws.data_ptr(), self.attn_ws.numel(), st))
             else:
                 _lib.check(lib.prl_paged_attn_prefill_tc(R.q.data_ptr(), n, kv[0], self.n_pages, 1, 0, *bt[:2], seg_start, seg_len,
                                                          seg_pos0.data_ptr(), seg_slot, ns, max_q, a.heads, a.kv_heads, a.dim,
@@ -2385,9 +2385,11 @@ class HybridEngine(EngineCore):
 
     def _step_plan(self):
         """How the delta rule's token step splits its work over the CTAs depends on the rows with a token; a batch that drains passes
-        from one split to the other once, with the same bits, and its step is captured again."""
+        from one split to the other once, with the same bits, and its step is captured again.  So do the shares of layers that
+        keep pages of 128-wide heads (_attn_plan)."""
         live = self._live_rows()
-        return tuple(self.lib.prl_gated_delta_step_heads(h, k, live) for h, k in self._delta_heads)
+        heads = sorted({self.cfg.layers[i].attn.kv_heads for i in self.attn_splits})
+        return tuple(self.lib.prl_gated_delta_step_heads(h, k, live) for h, k in self._delta_heads) + tuple(self._attn_plan(k) for k in heads)
 
     def _step_kernels(self) -> None:
         cfg, lib, R, B = self.cfg, self.lib, self._dec, self.B

@@ -96,6 +96,7 @@ class TPDecodeEngine(DecodeEngine):
                                          self.h.data_ptr(), self.x.data_ptr(), st))
         sm_scale = 1.0 / math.sqrt(cfg.head_dim)
         s_dense = self._slot_elems // (B * H)
+        splits, stages = self._attn_plan(cfg.num_kv_heads)
         for l in range(cfg.num_layers):
             p = f"layers.{l}."
             self._gemm(p + "qkv_proj.weight", self.x, cfg.qkv_size, H, self.split_k["qkv"], part)
@@ -105,11 +106,11 @@ class TPDecodeEngine(DecodeEngine):
                                               self.block_table.data_ptr(), self.max_blocks, None, self.inv_freq.data_ptr(),
                                               self.q.data_ptr(), self.kv_cache.data_ptr(), self.n_pages, l, PAGE_SIZE,
                                               None, 0, st))
-            _lib.check(lib.prl_paged_attn_decode(self.q.data_ptr(), self.kv_cache.data_ptr(), self.n_pages, cfg.num_layers,
-                                                 l, self.block_table.data_ptr(), self.max_blocks, self.seq_lens.data_ptr(),
-                                                 B, cfg.num_q_heads, cfg.num_kv_heads, cfg.head_dim, PAGE_SIZE,
-                                                 self.attn_splits, sm_scale, self.attn_out.data_ptr(),
-                                                 self.attn_ws.data_ptr(), self.attn_ws.numel(), st))
+            _lib.check(lib.prl_paged_attn_decode_planned(self.q.data_ptr(), self.kv_cache.data_ptr(), self.n_pages, cfg.num_layers,
+                                                         l, self.block_table.data_ptr(), self.max_blocks, self.seq_lens.data_ptr(),
+                                                         B, cfg.num_q_heads, cfg.num_kv_heads, cfg.head_dim, PAGE_SIZE,
+                                                         splits, stages, sm_scale, self.attn_out.data_ptr(),
+                                                         self.attn_ws.data_ptr(), self.attn_ws.numel(), st))
             self._row_parallel(p + "o_proj.weight", self.attn_out, H, cfg.q_size, 0, s_dense, 2 * l + 1,
                                a.ptr(p + "post_attention_layernorm.weight"))
             self._gemm(p + "gate_up_proj.weight", self.x, 2 * I, H, self.split_k["gate_up"], part)
@@ -120,10 +121,10 @@ class TPDecodeEngine(DecodeEngine):
 
     def step(self) -> None:
         """Like DecodeEngine.step, but the base class's eager warm-up before graph capture would deliver every
-        peer signal twice in that step; here the first step of a parameter buffer runs eagerly AS the step (it also
+        peer signal twice in that step; here the first step of a parameter buffer (and of a plan on it) runs eagerly AS the step (it also
         sets the kernel attributes) and the graph is captured, without a dry run, on the next one."""
         if self.use_graph:
-            key = self.arena.data.data_ptr()
+            key = (self.arena.data.data_ptr(), self._step_plan())      # equal on all ranks: they hold the same requests
             g = self._graphs.get(key)
             if g is None:
                 if key not in self._eager_done:

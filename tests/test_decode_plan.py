@@ -1,7 +1,10 @@
 """Rules that a decode engine plans its token step by, on the CPU."""
+import ctypes
+
 import pytest
 
-from pipelinerl_b200.engine import short_swiglu_tiles_pay, swiglu_epilogue_pays
+from pipelinerl_b200 import _lib
+from pipelinerl_b200.engine import batch_contexts, short_swiglu_tiles_pay, swiglu_epilogue_pays
 
 
 @pytest.mark.parametrize("I,H,split,pays", [(18944, 3584, 1, True), (8192, 2048, 8, True), (4096, 1024, 2, False), (8000, 2048, 8, True),
@@ -23,3 +26,37 @@ def test_short_swiglu_tiles_rule(I, H, rows, pays):
 def test_short_swiglu_tiles_keep_the_sums_of_the_split_pair(rows, slices, pays):
     """Two slices of up to 8 rows are added in the epilogue; more of either take the split pair."""
     assert short_swiglu_tiles_pay(4096, 1024, rows, 148, slices) is pays
+
+
+@pytest.mark.parametrize("lengths,want", [([5], (1, 5)), ([64, 64, 64], (3, 64)), ([64, 65], (2, 65)), ([16384] + [100] * 15, (2, 16384)), ([8192] * 32 + [1] * 32, (33, 8192))])
+def test_unequal_contexts_as_a_number_of_equal_ones(lengths, want):
+    assert batch_contexts(lengths) == want
+
+
+def attn_plan(slots, live, n_kv, longest, max_seq_len):
+    stages = ctypes.c_int32()
+    return _lib.load().prl_paged_attn_plan(slots, live, n_kv, longest, max_seq_len, ctypes.byref(stages)), stages.value
+
+
+@pytest.mark.parametrize("slots,live,n_kv,longest,plan", [
+    (16, 16, 4, 16384, (2, 6)), (16, 8, 4, 16384, (4, 6)), (16, 1, 4, 16384, (8, 6)), (32, 32, 4, 4096, (1, 6)), (32, 4, 4, 4096, (4, 6)),      # a batch that drains
+    (64, 64, 4, 8192, (2, 3)), (64, 19, 4, 8192, (2, 3)), (64, 18, 4, 8192, (2, 6)), (128, 128, 4, 4096, (1, 3)), (128, 37, 4, 4096, (1, 6)),
+    (74, 74, 2, 6080, (1, 6)), (74, 74, 2, 6081, (2, 3)), (185, 185, 1, 8192, (1, 3)), (186, 186, 1, 4032, (1, 3)), (186, 186, 1, 4033, (2, 3)), (297, 297, 1, 8192, (1, 3)),
+    (1, 1, 1, 512, (1, 6)), (1, 1, 1, 513, (2, 6)), (1, 1, 1, 5056, (16, 6)), (1, 1, 1, 5057, (32, 6)), (1, 1, 2, 8192, (16, 6)), (1, 1, 2, 8193, (32, 6)),
+    (1, 1, 1, 16384, (32, 6)), (1, 1, 1, 16385, (64, 6)), (1, 1, 4, 131072, (32, 6)), (1, 1, 1, 1 << 23, (128, 6))])
+def test_shares_of_decode_attention(slots, live, n_kv, longest, plan):
+    """Both sides of the rule's lines on 148 SMs; full slots have what prl_paged_attn_splits says."""
+    assert attn_plan(slots, live, n_kv, longest, longest) == plan
+    if live == slots:
+        assert _lib.load().prl_paged_attn_splits(slots, n_kv, longest) == plan[0]
+
+
+@pytest.mark.parametrize("slots", [1, 3, 16, 40, 64, 130])
+@pytest.mark.parametrize("n_kv,max_seq_len", [(1, 640), (2, 2048), (4, 16384), (8, 131072)])
+def test_workspace_of_the_longest_contexts_is_enough(slots, n_kv, max_seq_len):
+    """What an engine allocates for (the longest contexts, any number of them) covers every plan of shorter ones."""
+    most = max(attn_plan(slots, live, n_kv, max_seq_len, max_seq_len)[0] for live in range(1, slots + 1))
+    for live in range(1, slots + 1):
+        for longest in (1, 64, 513, 700, 4033, 6081, 10000, max_seq_len):
+            splits, _ = attn_plan(slots, live, n_kv, min(longest, max_seq_len), max_seq_len)
+            assert splits <= most and -(-max_seq_len // 64) <= 1024 * splits

@@ -612,6 +612,75 @@ def test_attention_of_one_split_writes_the_output(cuda_device, R, n_kv):
         assert ((out[b].double() - want).abs() <= 2.0 ** -7 * bound + 1e-30).all(), l
 
 
+LONG = tuple(257 + (443 * i) // 49 for i in range(50))
+
+
+@pytest.mark.parametrize("lens,R,n_kv,key_splits", [((1000, 449, 4097), 7, 2, 1), ((1000, 449, 4097), 9, 1, 1), ((1024, 0, 447, 4096), 8, 1, 2), (LONG, 4, 4, 1), (LONG, 16, 4, 1),
+                                                    (tuple(n // 64 * 64 + 64 for n in LONG), 7, 4, 1), (tuple(n // 64 * 64 + 63 for n in LONG), 2, 4, 2),
+                                                    (tuple(n // 64 * 64 + 1 for n in LONG), 12, 4, 1), ((2000,) + (0,) * 15, 7, 4, 8), ((5000, 70, 3), 7, 4, 32)])
+def test_attention_of_contexts_longer_than_its_ring(cuda_device, lens, R, n_kv, key_splits):
+    """More pages than stages, so that a stage is used again and the token's own row is laid over a page in one of them; last pages of 1, 63 and 64
+    keys; three and six stages, shares without a page: the output and the cache of the two launches, bit for bit, and the output against 64 bits."""
+    from pipelinerl_b200 import _lib
+    lib, dev, g = _lib.load(), cuda_device, torch.Generator(device=cuda_device).manual_seed(sum(lens) + R)
+    B, n_q, mb = len(lens), R * n_kv, (max(lens) + 63) // 64
+    pages = 1 + B * mb
+    bt = (1 + torch.randperm(B * mb, generator=g, device=dev)).to(torch.int32).view(B, mb)
+    sl = torch.tensor(lens, dtype=torch.int32, device=dev)
+    pos = (sl - 1).clamp_min(0)
+    kv0 = torch.randn(2 * pages * n_kv * 64 * 128, generator=g, device=dev).to(torch.bfloat16)
+    part = torch.randn(2, B, (n_q + 2 * n_kv) * 128, generator=g, device=dev)
+    inv = (1.0 / (1e6 ** (torch.arange(0, 128, 2).float() / 128))).to(dev)
+    ws = torch.zeros(int(lib.prl_paged_attn_workspace_bytes(B, n_q, key_splits)), dtype=torch.uint8, device=dev)
+    p = lambda t: t.data_ptr()  # noqa: E731
+    want = None
+    for stages in (0, 3, 6):
+        two, one = kv0.clone(), kv0.clone()
+        q, a, b = (torch.full((B, n_q * 128), 7.0, dtype=torch.bfloat16, device=dev) for _ in range(3))
+        tail = (B, n_q, n_kv, 128, 64, key_splits, stages, 128 ** -0.5)
+        _lib.check(lib.prl_qkv_rope_cache(p(part), 2, B, None, n_q, n_kv, 128, p(pos), p(bt), mb, None, p(inv), p(q), p(two), pages, 0, 64, None, 0,
+                                          _lib.stream_ptr()))
+        _lib.check(lib.prl_paged_attn_decode_planned(p(q), p(two), pages, 1, 0, p(bt), mb, p(sl), *tail, p(a), p(ws), ws.numel(), _lib.stream_ptr()))
+        _lib.check(lib.prl_paged_attn_decode_qkv_planned(p(part), 2, None, p(inv), p(one), pages, 1, 0, p(bt), mb, p(sl), *tail, p(b), p(ws), ws.numel(),
+                                                         _lib.stream_ptr()))
+        want = a if want is None else want
+        assert torch.equal(a, want) and torch.equal(b, want)
+        for i in (i for i, n in enumerate(lens) if n == 0):      # the two launches write a row without a token to its first page
+            for t in (two, one):
+                t.view(2, pages, n_kv, 64, 128)[:, bt[i, 0].item(), :, 0] = 0
+        assert torch.equal(one, two)
+    for i, n in enumerate(lens):
+        K, V = (two.view(2, pages, n_kv, 64, 128)[j, bt[i].long()].transpose(0, 1).reshape(n_kv, mb * 64, 128)[:, :n].double() for j in (0, 1))
+        w = torch.softmax(torch.einsum("grd,gsd->grs", q[i].view(n_kv, R, 128).double(), K) * 128 ** -0.5, -1)
+        ref, bound = torch.einsum("grs,gsd->grd", w, V), torch.einsum("grs,gsd->grd", w, V.abs())
+        assert ((want[i].view(n_kv, R, 128).double() - ref).abs() <= 2.0 ** -7 * bound + 1e-30).all(), n
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_attention_of_a_draining_batch(cuda_device, graph):
+    """40 sequences of 1500 tokens, of which one goes on when the others are done: its contexts are then cut further (one key head, 24 pages: 2
+    shares, 8), its captured step with it, and its log-probs stay the oracle's (bars of the end-to-end tests)."""
+    from pipelinerl_b200.engine import SamplingParams
+    cfg = tiny_cfg("gqa7")
+    w = tiny_weights(cfg)
+    prompt = torch.randint(0, cfg.vocab_size, (1500,), generator=torch.Generator().manual_seed(4)).tolist()
+    eng = make_engine(cfg, w, cuda_device, max_batch=40, max_seq_len=1536, max_new_tokens=16, use_cuda_graph=graph, prefill_chunk=512, fused_head=False)
+    seen = []
+    rule = eng._attn_plan
+    eng._attn_plan = lambda n_kv: seen.append(rule(n_kv)) or seen[-1]
+    one = eng.add_request(prompt, SamplingParams(max_tokens=12, greedy=True, ignore_eos=True))
+    others = [eng.add_request(prompt, SamplingParams(max_tokens=3, greedy=True, ignore_eos=True)) for _ in range(39)]
+    for _ in range(12):
+        eng.step()
+        eng.harvest()
+    plans = list(dict.fromkeys(seen))
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert not eng.slot_req and len(plans) >= 2 and plans[1][0] == 8 and plans[0][0] * 40 * cfg.num_kv_heads <= 2 * sms
+    lp = OracleQwen2(cfg, w).score(prompt + one.output_ids, 1.0).numpy()[len(prompt) - 1:]
+    diff = np.abs(lp - np.array(one.output_logprobs))
+    assert all(r.output_ids == one.output_ids[:3] for r in others) and diff.max() <= E2E_BOUNDS["gqa7"][0] and diff.mean() <= E2E_BOUNDS["gqa7"][1], (diff.max(), diff.mean())
+
+
 @pytest.mark.parametrize("lens,R,n_kv,n_split,key_splits,bias", [((1,), 1, 1, 1, 1, True), ((64, 0, 65), 7, 4, 2, 1, True), ((63, 128, 1, 200), 8, 2, 3, 1, False),
                                                                   ((700, 65, 0, 129), 9, 2, 8, 4, True), ((40, 641), 16, 1, 5, 2, True), ((96,) * 90, 4, 4, 1, 1, True)])
 def test_attention_from_the_projection_equals_two_launches(cuda_device, lens, R, n_kv, n_split, key_splits, bias):
