@@ -696,7 +696,7 @@ int pick_ntile(int64_t M) {
 using namespace prl;
 
 extern "C" int prl_gemm_set_smem_budget_kb(int32_t kb) {
-  PRL_CHECK_ARG(kb >= 48 && kb <= 220, "prl_gemm_set_smem_budget_kb: 48..220 KB");
+  PRL_CHECK_ARG(kb == 0 || (kb >= 48 && kb <= 220), "prl_gemm_set_smem_budget_kb: 48..220 KB, or 0 for the rule");
   g_smem_budget = kb * 1024;
   return PRL_OK;
 }

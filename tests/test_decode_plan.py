@@ -60,3 +60,10 @@ def test_workspace_of_the_longest_contexts_is_enough(slots, n_kv, max_seq_len):
         for longest in (1, 64, 513, 700, 4033, 6081, 10000, max_seq_len):
             splits, _ = attn_plan(slots, live, n_kv, min(longest, max_seq_len), max_seq_len)
             assert splits <= most and -(-max_seq_len // 64) <= 1024 * splits
+
+
+def test_ring_budget_goes_back_to_the_rule():
+    """A set budget is taken back by 0, the default; what no ring fits in stays refused."""
+    lib = _lib.load()
+    assert [lib.prl_gemm_set_smem_budget_kb(kb) for kb in (100, 220, 48, 0)] == [0] * 4
+    assert all(lib.prl_gemm_set_smem_budget_kb(kb) != 0 for kb in (-1, 1, 47, 221))
