@@ -1130,10 +1130,22 @@ extern "C" int prl_moe_gather(const void* x_bf16, const int32_t* perm, const int
   return PRL_OK;
 }
 
+// Few rows per expert, where the ring kernel is the faster one: few tokens for the experts (max_tiles is the experts and a 64th of the pairs, rounded
+// up), which with four choices a token are 15 rows per expert at most, but with eight 38; so where the pairs are told, at most 22 of them per
+// expert.  Former kernel / ring, both products, us: 64 experts of 2048 x 1024, 12.5 rows 119 / 93, 18.8 125 / 115, 22.5 127 / 122, 25 135 / 129,
+// 28.8 140 / 142, 38.6 155 / 168; 64 of 1024 x 512, 25 42.9 / 43.6, 38.6 48.8 / 54.0; 128 of them 18.8 73 / 64; 32 of 2048 x 1024, 25 69.4 / 71.5, 30 77.6 / 81.2;
+// 16 of 2048 x 2048, 15 59.4 / 59.0, 18 59.7 / 61.1.
+static bool moe_few_rows(int64_t tokens, int64_t pairs, int64_t max_tiles) {
+  return tokens > 0 && tokens <= 3 * max_tiles && (pairs <= 0 || pairs <= 22 * (max_tiles - (pairs + kTile - 1) / kTile));
+}
+extern "C" int prl_moe_few_rows(int64_t tokens, int64_t pairs, int32_t experts) {
+  return moe_few_rows(tokens, pairs, prl_moe_max_tiles(pairs, experts));
+}
+
 template <int ACT, int PAIR = kPairNone>
 static int moe_gemm_impl(const void* A, int32_t a_is_f32, int64_t lda, int32_t a_mod, const void* W, int32_t w_is_f32,
                          int64_t expert_stride, int64_t ldw, const int32_t* perm, const int32_t* meta, const int32_t* tiles,
-                         int64_t max_tiles, int64_t N, int64_t K, void* C, int64_t ldc, int32_t c_perm, const float* wsel, int64_t tokens,
+                         int64_t max_tiles, int64_t N, int64_t K, void* C, int64_t ldc, int32_t c_perm, const float* wsel, bool few,
                          prl_stream_t st) {
   PRL_CHECK_ARG(A && W && perm && meta && tiles && C && (ACT == kActNone || wsel), "prl_moe_gemm: NULL argument");
   PRL_CHECK_ARG(max_tiles >= 1 && max_tiles <= 65535 && N >= 1 && K >= 1 && lda >= K && ldw >= K && ldc >= N && a_mod >= 0,
@@ -1141,9 +1153,7 @@ static int moe_gemm_impl(const void* A, int32_t a_is_f32, int64_t lda, int32_t a
   cudaStream_t s = (cudaStream_t)st;
   if (!a_is_f32 && !w_is_f32 && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && expert_stride % 8 == 0 &&
       ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0) {
-    // Few rows per expert: at most about 20 of `tokens`.  Neither the experts nor the choices per token are known here, but max_tiles holds
-    // the experts and a 64th of the pairs: 16 experts, top 4 up to 57 tokens, 64 experts, top 8 up to 200.
-    if (tokens > 0 && tokens <= 3 * max_tiles && expert_stride > 0) {
+    if (few && expert_stride > 0) {
       CUtensorMap tw;
       const int rc = make_tmap_3d_bf16(&tw, W, (uint64_t)K, (uint64_t)N, 1u << 16, (uint64_t)ldw * 2, (uint64_t)expert_stride * 2, kBK, kFeatures, 1);
       if (rc) return rc;
@@ -1180,7 +1190,16 @@ extern "C" int prl_moe_gemm(const void* A, int32_t a_is_f32, int64_t lda, int32_
                             const int32_t* tiles, int64_t max_tiles, int64_t N, int64_t K, float* C, int64_t ldc,
                             int32_t c_perm, prl_stream_t st) {
   return moe_gemm_impl<kActNone>(A, a_is_f32, lda, a_mod, W, w_is_f32, expert_stride, ldw, perm, meta, tiles, max_tiles, N, K, C, ldc,
-                              c_perm, nullptr, a_mod, st);
+                                 c_perm, nullptr, moe_few_rows(a_mod, 0, max_tiles), st);
+}
+
+// ... told how many pairs there are
+extern "C" int prl_moe_gemm_pairs(const void* A, int32_t a_is_f32, int64_t lda, int32_t a_mod, const void* W, int32_t w_is_f32,
+                                  int64_t expert_stride, int64_t ldw, const int32_t* perm, const int32_t* meta, const int32_t* tiles,
+                                  int64_t max_tiles, int64_t pairs, int64_t N, int64_t K, float* C, int64_t ldc, int32_t c_perm, prl_stream_t st) {
+  PRL_CHECK_ARG(pairs >= 1, "prl_moe_gemm_pairs: no pairs");
+  return moe_gemm_impl<kActNone>(A, a_is_f32, lda, a_mod, W, w_is_f32, expert_stride, ldw, perm, meta, tiles, max_tiles, N, K, C, ldc,
+                                 c_perm, nullptr, moe_few_rows(a_mod, pairs, max_tiles), st);
 }
 
 // First product of ungated experts: out[s] = act(A[row of s] W_e^T) * wsel[pair of s], in the operand type of A and in sorted
@@ -1192,28 +1211,42 @@ extern "C" int prl_moe_gemm_act(const void* A, int32_t a_is_f32, int64_t lda, in
                                 void* out, int64_t ld_out, prl_stream_t st) {
   PRL_CHECK_ARG(act == kActRelu2 || act == kActGelu, "prl_moe_gemm_act: unknown activation %d", act);
   return act == kActRelu2 ? moe_gemm_impl<kActRelu2>(A, a_is_f32, lda, a_mod, W, w_is_f32, expert_stride, ldw, perm, meta, tiles, max_tiles,
-                                                     N, K, out, ld_out, 0, wsel, a_mod, st)
+                                                     N, K, out, ld_out, 0, wsel, moe_few_rows(a_mod, 0, max_tiles), st)
                           : moe_gemm_impl<kActGelu>(A, a_is_f32, lda, a_mod, W, w_is_f32, expert_stride, ldw, perm, meta, tiles, max_tiles,
-                                                    N, K, out, ld_out, 0, wsel, a_mod, st);
+                                                    N, K, out, ld_out, 0, wsel, moe_few_rows(a_mod, 0, max_tiles), st);
 }
 
 template <int ACT>
 static int moe_mlp_impl(const void* x, int32_t f32, int32_t n, const void* up, const void* down, int64_t W, int64_t F, const int32_t* perm,
-                        const int32_t* meta, const int32_t* tiles, int64_t max_tiles, const float* wsel, void* act_out, float* out,
-                        prl_stream_t st) {
-  const int rc = moe_gemm_impl<ACT, kPairFirst>(x, f32, W, n, up, f32, F * W, W, perm, meta, tiles, max_tiles, F, W, act_out, F, 0, wsel, n, st);
+                        const int32_t* meta, const int32_t* tiles, int64_t max_tiles, int64_t pairs, const float* wsel, void* act_out,
+                        float* out, prl_stream_t st) {
+  const bool few = moe_few_rows(n, pairs, max_tiles);
+  const int rc = moe_gemm_impl<ACT, kPairFirst>(x, f32, W, n, up, f32, F * W, W, perm, meta, tiles, max_tiles, F, W, act_out, F, 0, wsel, few, st);
   return rc ? rc : moe_gemm_impl<kActNone, kPairSecond>(act_out, f32, F, 0, down, f32, W * F, F, perm, meta, tiles, max_tiles, W, F, out, W, 1,
-                                                        nullptr, n, st);
+                                                        nullptr, few, st);
 }
 
 // Both products of ungated experts, prl_moe_gemm_act and prl_moe_gemm in one call: x [n, W], up [experts * F, W], down [experts * W, F] of
 // one type (f32, else bf16); act_out (a row of F per pair, in that type) is scratch between them, out (a row of W per pair) fp32, pair order.
+static int moe_mlp_any(const void* x, int32_t f32, int32_t n, const void* up, const void* down, int64_t W, int64_t F, const int32_t* perm,
+                       const int32_t* meta, const int32_t* tiles, int64_t max_tiles, int64_t pairs, int32_t act, const float* wsel,
+                       void* act_out, float* out, prl_stream_t st) {
+  PRL_CHECK_ARG(n >= 1 && act_out && (act == kActRelu2 || act == kActGelu), "prl_moe_mlp_act: bad argument (activation %d)", act);
+  return act == kActRelu2 ? moe_mlp_impl<kActRelu2>(x, f32, n, up, down, W, F, perm, meta, tiles, max_tiles, pairs, wsel, act_out, out, st)
+                          : moe_mlp_impl<kActGelu>(x, f32, n, up, down, W, F, perm, meta, tiles, max_tiles, pairs, wsel, act_out, out, st);
+}
 extern "C" int prl_moe_mlp_act(const void* x, int32_t f32, int32_t n, const void* up, const void* down, int64_t W, int64_t F,
                                const int32_t* perm, const int32_t* meta, const int32_t* tiles, int64_t max_tiles, int32_t act,
                                const float* wsel, void* act_out, float* out, prl_stream_t st) {
-  PRL_CHECK_ARG(n >= 1 && act_out && (act == kActRelu2 || act == kActGelu), "prl_moe_mlp_act: bad argument (activation %d)", act);
-  return act == kActRelu2 ? moe_mlp_impl<kActRelu2>(x, f32, n, up, down, W, F, perm, meta, tiles, max_tiles, wsel, act_out, out, st)
-                          : moe_mlp_impl<kActGelu>(x, f32, n, up, down, W, F, perm, meta, tiles, max_tiles, wsel, act_out, out, st);
+  return moe_mlp_any(x, f32, n, up, down, W, F, perm, meta, tiles, max_tiles, 0, act, wsel, act_out, out, st);
+}
+
+// ... told how many pairs there are
+extern "C" int prl_moe_mlp_act_pairs(const void* x, int32_t f32, int32_t n, const void* up, const void* down, int64_t W, int64_t F,
+                                     const int32_t* perm, const int32_t* meta, const int32_t* tiles, int64_t max_tiles, int64_t pairs,
+                                     int32_t act, const float* wsel, void* act_out, float* out, prl_stream_t st) {
+  PRL_CHECK_ARG(pairs >= 1, "prl_moe_mlp_act_pairs: no pairs");
+  return moe_mlp_any(x, f32, n, up, down, W, F, perm, meta, tiles, max_tiles, pairs, act, wsel, act_out, out, st);
 }
 
 extern "C" int prl_moe_glu(const float* gate_up, int64_t ld, int64_t pairs, int32_t F, const int32_t* perm,
