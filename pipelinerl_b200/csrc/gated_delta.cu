@@ -294,6 +294,7 @@ struct SplitArgs {
   const float* gain;
   float eps;
   int heads, kh, dk, dv, vec;
+  int early_piece, early_walk;   // the kernel behind this one may start before its end
   const int32_t* row_slot;
   const int32_t* row_back;
   const int32_t* seg_start;
@@ -391,7 +392,7 @@ __global__ void __launch_bounds__(kThreads, U == 1 ? 3 : 2) gated_delta_front_ti
   };
   if (h < 2 * a.kh + H) taps_of(0);
   pdl_wait();
-  pdl_launch_dependents();
+  if (a.early_piece) pdl_launch_dependents();
   int slot[RT], back[RT];
 #pragma unroll
   for (int r = 0; r < RT; ++r) {
@@ -503,8 +504,7 @@ __device__ __forceinline__ int blk_at(int b, int q) { return (b * (b + 1) / 2 + 
 
 __global__ void __launch_bounds__(kPieceThreads, 2) gated_delta_piece_kernel(SplitArgs a) {
   pdl_wait();
-  pdl_launch_dependents();   // here, in the front rows, the closing rows and the experts' gather: a prompt of 2500 tokens 2436 -> 2393 us (in the walk, the
-                             // read-out and the token step too: 2402, and 564 -> 572 a token step of 32 rows: the next kernel's blocks take their SMs' room)
+  if (a.early_walk) pdl_launch_dependents();
   extern __shared__ __align__(16) float sm[];
   const int piece = blockIdx.x, head = blockIdx.y, len = a.sub_len[piece];
   const int64_t row0 = a.sub_start[piece];
@@ -1013,7 +1013,7 @@ extern "C" int prl_gated_delta_split(const float* P, int64_t ldp, int32_t off, i
                 "prl_gated_delta_split: NULL argument");
   PRL_CHECK_ARG(n_rows >= 1 && n_seg >= 1 && n_seg <= 65535 && n_sub >= 1 && geometry_ok(heads, kh, dk, dv, taps),
                 "prl_gated_delta_split: bad shape (heads=%d q/k heads=%d dk=%d dv=%d taps=%d)", heads, kh, dk, dv, taps);
-  SplitArgs a{P, ldp, off, off_b, off_a, off_g, conv_w, taps, A_log, dt_bias, unit_eps, gain, eps, heads, kh, dk, dv, 0,
+  SplitArgs a{P, ldp, off, off_b, off_a, off_g, conv_w, taps, A_log, dt_bias, unit_eps, gain, eps, heads, kh, dk, dv, 0, 0, 0,
               row_slot, row_back, seg_start, seg_len, seg_slot, seg_sub0, seg_nsub, sub_start, sub_len, C, nullptr, nullptr, nullptr, D,
               S0, conv_state, state, out};
   a.E = scratch;                                  // the widest first: 16-byte aligned rows whatever dk is
@@ -1021,6 +1021,20 @@ extern "C" int prl_gated_delta_split(const float* P, int64_t ldp, int32_t off, i
   a.gates = a.W + (int64_t)n_rows * heads * dk;
   PRL_CHECK_ARG(((uintptr_t)scratch & 15) == 0, "prl_gated_delta_split: the scratch must be 16-byte aligned");
   a.vec = dk % 4 == 0 && dv % 4 == 0 && (((uintptr_t)C | (uintptr_t)S0 | (uintptr_t)D) & 15) == 0;
+  const int dk4 = (dk + 3) & ~3, ldk = dk4 + 4;
+  const dim3 gw((dv + kWalkCols - 1) / kWalkCols, heads, n_seg);
+  // partial sums: four quarters of the key channels for 64 rows, later one half of the update
+  const size_t red = (size_t)kWalkCols * (4 * kPieceMax > dk4 ? 4 * kPieceMax : dk4);
+  const int stages = dk4 <= 128 && (int64_t)gw.x * gw.y * gw.z <= num_sms() ? 2 : 1;
+  const size_t sm_walk = ((size_t)stages * 2 * kPieceMax * ldk + (size_t)(dk4 + kPieceMax) * (kWalkCols + 4) + red) * sizeof(float);
+  const size_t x_rows = (size_t)(kPieceMax - kBlk) * 2 * kPieceThreads, q_rows = (size_t)kPieceMax * ldk;
+  const size_t sm_piece = (10 * (size_t)kBlkFloats + q_rows + (q_rows > x_rows ? q_rows : x_rows)) * sizeof(float);
+  // The next kernel's blocks may come early where this one's fill the chip, and the walk's where they find no room beside a piece's: elsewhere they settle
+  // two to an SM while others idle (four kernels, us, with / without: front rows first, 128 rows of 16 heads of 128 74 / 66, 452 of 16 of 64 and 128
+  // 95 / 80; the walk early, 1024 of them 150 / 128).  A prompt of 2500 tokens, 16 heads of 128, 2437 -> 2391 us, of 700 796 -> 806.  Behind the walk, the
+  // read-out and the token step it was slower (2402; 564 -> 572 a token step of 32 rows).
+  a.early_piece = (int64_t)n_sub * heads >= num_sms();
+  a.early_walk = a.early_piece && sm_walk + sm_piece > 227 * 1024;
   cudaStream_t s = (cudaStream_t)st_;
   const bool tiled = a.vec && taps >= 2 && taps <= 4 && off % 4 == 0 && ldp % 4 == 0 && ((uintptr_t)P & 15) == 0;
   const dim3 gf((n_rows + kFrontRows - 1) / kFrontRows, (2 * kh + heads + kThreads / 32 - 1) / (kThreads / 32));
@@ -1035,18 +1049,10 @@ extern "C" int prl_gated_delta_split(const float* P, int64_t ldp, int32_t off, i
   else PRL_CUDA(launch_pdl(gated_delta_front_kernel, dim3(n_rows), dim3(kThreads), (size_t)0, s, a));
 #undef PRL_GF
   PRL_LAUNCH_CHECK();
-  const int dk4 = (dk + 3) & ~3, ldk = dk4 + 4;
-  const size_t x_rows = (size_t)(kPieceMax - kBlk) * 2 * kPieceThreads, q_rows = (size_t)kPieceMax * ldk;
-  const size_t sm_piece = (10 * (size_t)kBlkFloats + q_rows + (q_rows > x_rows ? q_rows : x_rows)) * sizeof(float);
   static SmemAttr at_piece = {};
   PRL_CUDA(ensure_smem(gated_delta_piece_kernel, (int)sm_piece, at_piece));
   PRL_CUDA(launch_pdl(gated_delta_piece_kernel, dim3(n_sub, heads), dim3(kPieceThreads), sm_piece, s, a));
   PRL_LAUNCH_CHECK();
-  const dim3 gw((dv + kWalkCols - 1) / kWalkCols, heads, n_seg);
-  // partial sums: four quarters of the key channels for 64 rows, later one half of the update
-  const size_t red = (size_t)kWalkCols * (4 * kPieceMax > dk4 ? 4 * kPieceMax : dk4);
-  const int stages = dk4 <= 128 && (int64_t)gw.x * gw.y * gw.z <= num_sms() ? 2 : 1;
-  const size_t sm_walk = ((size_t)stages * 2 * kPieceMax * ldk + (size_t)(dk4 + kPieceMax) * (kWalkCols + 4) + red) * sizeof(float);
   static SmemAttr at_walk[2] = {};
   if (stages == 2) {
     PRL_CUDA(ensure_smem(gated_delta_walk_kernel<2>, (int)sm_walk, at_walk[0]));

@@ -871,3 +871,40 @@ def test_front_rows_of_the_gated_delta_rule(cuda_device, segs, heads, kh, dk, dv
         bound[:, c] = by * (bound[:, c] + want[:, c].abs() * (worst + 2.0 ** -24 * (dk / 16 + 8)))
         want[:, c] *= by
     assert bool(((C.cpu().double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("segs,dk", [((640,), 128), ((300, 340), 128), ((640,), 64), ((610, 5), 64)])
+def test_gated_delta_rule_of_heads_that_fill_the_chip(cuda_device, segs, dk):
+    """16 value heads of ten pieces (more blocks than SMs, so that the next kernels start early) against the first 8 of them by themselves: a head's outputs and
+    state depend on its own inputs only, bit for bit, several times over."""
+    from pipelinerl_b200 import _lib
+    lib, dev, dv, taps, g = _lib.load(), cuda_device, 128, 4, torch.Generator().manual_seed(sum(segs) + dk)
+    n, ns = sum(segs), len(segs)
+    on = lambda *s: torch.randn(*s, generator=g).to(dev)  # noqa: E731
+    q, k, v, gate, b, a = on(n, 8, dk), on(n, 8, dk), on(n, 16, dv), on(n, 16, dv), on(n, 16), on(n, 16)
+    wq, wk, wv, A, dt, gain = on(8, dk, taps), on(8, dk, taps), on(16, dv, taps), 0.1 * on(16), on(16), on(dv)
+    starts = [sum(segs[:i]) for i in range(ns)]
+    subs = [(i, s + c, min(64, l - c)) for i, (s, l) in enumerate(zip(starts, segs)) for c in range(0, l, 64)]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)  # noqa: E731
+    tabs = [i32([i for i, l in enumerate(segs) for _ in range(l)]), i32([t for l in segs for t in range(l)]), i32(starts), i32(list(segs)), i32(list(range(ns))),
+            i32([sum(1 for j, _, _ in subs if j < i) for i in range(ns)]), i32([sum(1 for j, _, _ in subs if j == i) for i in range(ns)]),
+            i32([s for _, s, _ in subs]), i32([l for _, _, l in subs])]
+    p = lambda t: t.data_ptr()  # noqa: E731
+
+    def run(H):
+        kh, ch = H // 2, H * dk + H * dv
+        P = torch.cat([q[:, :kh].reshape(n, -1), k[:, :kh].reshape(n, -1), v[:, :H].reshape(n, -1), b[:, :H], a[:, :H], gate[:, :H].reshape(n, -1)], 1).contiguous()
+        w = torch.cat([wq[:kh].reshape(-1, taps), wk[:kh].reshape(-1, taps), wv[:H].reshape(-1, taps)]).contiguous()
+        f = lambda *s: torch.zeros(*s, device=dev)  # noqa: E731
+        C, scr = f(n, ch), f(n * int(lib.prl_gated_delta_split_floats(H, dk)))
+        S0, D, conv, state, out = f(len(subs), H, dk, dv), f(n, H * dv), f(ns, ch, taps - 1), f(ns, H, dv, dk), f(n, H * dv)
+        _lib.check(lib.prl_gated_delta_split(p(P), P.shape[1], 0, ch, ch + H, ch + 2 * H, p(w), taps, p(A), p(dt), 1e-6, p(gain), 1e-5, H, kh, dk, dv, n,
+                                             *(p(t) for t in tabs[:5]), ns, *(p(t) for t in tabs[5:]), len(subs), p(C), p(scr), p(S0), p(D), p(conv), p(state),
+                                             p(out), 1, _lib.stream_ptr()))
+        return out.view(n, H, dv), state
+
+    want, want_state = run(8)
+    assert want.isfinite().all() and want.abs().max() > 0
+    for _ in range(4):
+        out, state = run(16)
+        assert torch.equal(out[:, :8], want) and torch.equal(state[:, :8], want_state)
