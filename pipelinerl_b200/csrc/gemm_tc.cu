@@ -503,7 +503,9 @@ int launch_gemm(const CUtensorMap& tw, const CUtensorMap& twl, const CUtensorMap
   //  * two to an SM: 111 KB, which is what fits (hi + lo weights, up to 32 tokens: three stages for two, x 32768 x 1024 30 -> 23 us, x 32768 x
   //    2048 46 -> 38; plain ones of up to 16 tokens: six for five, 16 x 152064 x 3584 159 -> 157);
   //  * hi + lo weights in many waves: with up to 32 tokens 100 KB, three CTAs an SM of two stages each (x 152064 x 3584 298 us, 303 with
-  //    111 KB); with 64 tokens, where two stages are 80 KB, one CTA of five (348 -> 334);
+  //    111 KB); with 64 tokens, where two stages are 80 KB, one CTA of five if chains are long and two to an SM would leave a last wave nearly empty
+  //    (111 / 200 KB: 1188 tiles x 3584 361 / 346, 594 200 / 184, 1187 x 2048 207 / 200, x 1792 185 / 181, but x 1152 122.5 / 124, x 896 98 / 103, and 2000
+  //    tiles x 2304 389 / 407, 1002 x 2048 173 / 176);
   //  * short tiles share their SMs with another branch's kernel: 100 KB (a hybrid step of 32 rows 557 us, 560 with more).
   const int stage = p.tile_rows * kBlockK * 2 * (lo ? 2 : 1) + L::kBBytes;
   const int kb = (p.kblocks + p.split_k - 1) / p.split_k;
@@ -511,7 +513,8 @@ int launch_gemm(const CUtensorMap& tw, const CUtensorMap& twl, const CUtensorMap
   const int64_t ctas = (int64_t)grid.x * grid.y, sms = num_sms();
   const bool whole = p.tile_rows == kBlockM;
   int ring = (whole ? 111 : 100) * 1024;
-  if (kNTile >= 128 || (whole && ctas <= sms && kb >= 2 * (ring / stage)) || (lo && kNTile == 64 && ctas >= 4 * sms)) ring = 200 * 1024;
+  if (kNTile >= 128 || (whole && ctas <= sms && kb >= 2 * (ring / stage)) ||
+      (lo && kNTile == 64 && ctas >= 4 * sms && kb >= 28 && ctas % (2 * sms) > 0 && 2 * (ctas % (2 * sms)) <= sms)) ring = 200 * 1024;
   else if (lo && kNTile < 64 && ctas > 2 * sms) ring = 100 * 1024;
   if (g_smem_budget && kNTile < 128) ring = g_smem_budget;
   int n_stages = ring / stage;
