@@ -78,7 +78,7 @@ struct TnParams {
   const int32_t* g_perm;
   const float* g_w;
   int g_act;               // 1: relu(.)^2, 2: gelu in its error-function form
-  // head epilogue (kHead): logits never leave TMEM/registers
+  // head epilogue (kHead): the statistics of the logits, which leave TMEM / registers only where they are kept
   const int64_t* targets;  // [M] or NULL
   float4* head_part;       // [n_tiles, M]: (max, sum exp, sum exp*z, target logit or -inf) of one 256-column vocabulary tile
   float* keep_logits;      // [keep_rows, ld_keep] or NULL: the products of the first rows, kept for the backward
@@ -224,7 +224,9 @@ __device__ __forceinline__ bool aligned16(const void* p, int64_t ld_bytes) {
 
 // kAcc: the launch adds into an fp32 C (plain epilogue only).  An instance of its own, since the other epilogues feel every register:
 // 3584 x 18944, K = 1000, without accumulation 142 us beside this branch, 114 without it
-template <bool kHead, bool kAcc = false>
+// kKeep: the head's forward that keeps its logits; an instance of its own, for where few channels make the epilogue what the statistics wait for its
+// code alone costs 12 % (2000 x 50257 x 768 287 -> 320 us)
+template <bool kHead, bool kAcc = false, bool kKeep = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsTN<kHead>, 1)
 gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                const __grid_constant__ CUtensorMap tm_a2, const __grid_constant__ CUtensorMap tm_b2, TnParams p) {
@@ -435,8 +437,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
           }
         } else {
         float m = -INFINITY, ssum = 0.f, usum = 0.f, zt = -INFINITY;
-        const bool keep = p.keep_logits != nullptr && (int64_t)tm * kTile < p.keep_rows;
-        const int keep_row = row_ok && row < p.keep_rows ? (int)row : -1;
+        const bool keep = kKeep && (int64_t)tm * kTile < p.keep_rows;
+        const int keep_row = kKeep && row_ok && row < p.keep_rows ? (int)row : -1;
 #pragma unroll 1
         for (int c0 = 0; c0 < kTile; c0 += 32) {
           if (col0 + c0 >= p.N) break;
@@ -1066,12 +1068,13 @@ int head_logprob_tn(const void* W, const void* W_lo, const void* X, int64_t M, i
   rc = make_tmap_2d_bf16(&tb2, W_lo ? W_lo : W, (uint64_t)K, (uint64_t)V, (uint64_t)K * 2, kBK, kHalf);
   if (rc) return rc;
   const int smem = kSmemTN;
-  static SmemAttr smem_attr = {};
-  PRL_CUDA(ensure_smem(gemm_tn_kernel<true>, smem, smem_attr));
+  const auto kernel = keep_logits ? gemm_tn_kernel<true, false, true> : gemm_tn_kernel<true>;
+  static SmemAttr smem_attr[2] = {};
+  PRL_CUDA(ensure_smem(kernel, smem, smem_attr[keep_logits ? 1 : 0]));
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   int clusters = num_sms() / 2;
   if (tiles < clusters) clusters = (int)tiles;
-  PRL_CUDA(launch_pdl(gemm_tn_kernel<true>, dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<true>), (size_t)smem, stream, ta, tb, ta, tb2, p));
+  PRL_CUDA(launch_pdl(kernel, dim3((unsigned)(2 * clusters)), dim3(kThreadsTN<true>), (size_t)smem, stream, ta, tb, ta, tb2, p));
   PRL_LAUNCH_CHECK();
   head_tn_combine_kernel<<<(unsigned)((M + 3) / 4), 128, 0, stream>>>((const float4*)workspace, p.n_tiles, M,
                                                                       targets ? 1 : 0, logprob_target, entropy, lse);
