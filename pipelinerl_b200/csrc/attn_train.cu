@@ -1089,8 +1089,8 @@ __global__ void __launch_bounds__(kThreadsB4, 1)
 attn_bwd_dq4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                     const __grid_constant__ CUtensorMap tm_kv, BwdParams p) {
   // Runs beside the end of the dK / dV kernel (other columns of the gradient, other inputs); the one block that waits for it makes this
-  // kernel's end the end of both.  Forward and backward, us: six samples of 1 to 2300 tokens, 14 / 2 heads 232.2 -> 221.4, one of 16384, 28 / 4 heads
-  // 7984 -> 7885.
+  // kernel's end the end of both (launched plainly, as by the sequence-parallel entry, it starts behind it and waits for nothing).  Forward
+  // and backward, us: six samples of 1 to 2300 tokens, 14 / 2 heads 232.2 -> 221.4; of one long sample no more than runs differ.
   if (blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1 && blockIdx.z == gridDim.z - 1) pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;

@@ -567,13 +567,18 @@ def swiglu_epilogue_pays(I: int, H: int, split_k: int, sms: int) -> bool:
     return split_k == 1 or (I // 64 < sms and -(-H // 64) * (sms - I // 64) <= 5 * sms)
 
 
-def short_swiglu_tiles_pay(I: int, H: int, rows: int, sms: int, slices: int = 1) -> bool:
+def short_swiglu_tiles_pay(I: int, H: int, rows: int, sms: int) -> bool:
     """The same for the gated epilogue's tiles of 32 features, which up to 64 rows take where the I / 64 tiles of 64 are at most half as
     many as the SMs (prl_gemm_swiglu_decode).  1024 wide, I 4096 (128 tiles of 148): a step of eight layers
-    at 4 sequences 252 -> 241 us.  The sums stay those of the split pair, of which the epilogue
-    can add two `slices` of up to 8 rows: they share the 16 columns of the tile that the step's other products of so few rows have (in one of
-    32 columns, another kernel among the step's, 256 us)."""
-    return rows <= 64 and 2 * (I // 64) <= sms and -(-H // 64) * (sms - I // 32) <= 5 * sms and (slices == 1 or (slices == 2 and rows <= 8))
+    at 4 sequences 252 -> 241 us."""
+    return rows <= 64 and 2 * (I // 64) <= sms and -(-H // 64) * (sms - I // 32) <= 5 * sms
+
+
+def short_swiglu_slices(split_k: int, rows: int) -> int:
+    """Slices whose sums those tiles add in order, as the split pair in whose place they run would: its two for up to 8 rows, which share the 16
+    columns of the tile that the step's other products of so few rows have.  Else all k-blocks are one sum: with a tile of 32 columns, another kernel
+    among the step's, the step took 256 us, and as the pair one of 16 rows takes 267 instead of 251, of 64 rows 354 instead of 340."""
+    return 2 if split_k == 2 and rows <= 8 else 1
 
 
 class DecodeEngine(EngineCore):
@@ -665,8 +670,8 @@ class DecodeEngine(EngineCore):
         I, H, sms = cfg.intermediate_size, cfg.hidden_size, torch.cuda.get_device_properties(self.dev).multi_processor_count
         split = self.split_k["gate_up"]
         whole = swiglu_epilogue_pays(I, H, split, sms)
-        self.swiglu_slices = 1 if whole else split
-        self.swiglu_epilogue = I % 64 == 0 and B <= 128 and (whole or short_swiglu_tiles_pay(I, H, B, sms, split))
+        self.swiglu_slices = 1 if whole else short_swiglu_slices(split, B)
+        self.swiglu_epilogue = I % 64 == 0 and B <= 128 and (whole or short_swiglu_tiles_pay(I, H, B, sms))
         need = max(self.split_k[k] * B * shapes[k][0] for k in ("qkv", "o", "gate_up", "down"))
         self.partials = torch.zeros(need, dtype=torch.float32, device=self.dev)
 

@@ -4,7 +4,7 @@ import ctypes
 import pytest
 
 from pipelinerl_b200 import _lib
-from pipelinerl_b200.engine import batch_contexts, short_swiglu_tiles_pay, swiglu_epilogue_pays
+from pipelinerl_b200.engine import batch_contexts, short_swiglu_slices, short_swiglu_tiles_pay, swiglu_epilogue_pays
 
 
 @pytest.mark.parametrize("I,H,split,pays", [(18944, 3584, 1, True), (8192, 2048, 8, True), (4096, 1024, 2, False), (8000, 2048, 8, True),
@@ -22,10 +22,10 @@ def test_short_swiglu_tiles_rule(I, H, rows, pays):
     assert short_swiglu_tiles_pay(I, H, rows, 148) is pays
 
 
-@pytest.mark.parametrize("rows,slices,pays", [(8, 1, True), (8, 2, True), (9, 2, False), (9, 1, True), (64, 1, True), (8, 3, False), (1, 7, False)])
-def test_short_swiglu_tiles_keep_the_sums_of_the_split_pair(rows, slices, pays):
-    """Two slices of up to 8 rows are added in the epilogue; more of either take the split pair."""
-    assert short_swiglu_tiles_pay(4096, 1024, rows, 148, slices) is pays
+@pytest.mark.parametrize("split,rows,slices", [(2, 1, 2), (2, 8, 2), (2, 9, 1), (2, 64, 1), (1, 4, 1), (3, 4, 1), (7, 8, 1)])
+def test_short_swiglu_tiles_keep_the_sums_of_the_split_pair(split, rows, slices):
+    """Two slices of up to 8 rows are added in order; more of either are one sum."""
+    assert short_swiglu_slices(split, rows) == slices
 
 
 @pytest.mark.parametrize("lengths,want", [([5], (1, 5)), ([64, 64, 64], (3, 64)), ([64, 65], (2, 65)), ([16384] + [100] * 15, (2, 16384)), ([8192] * 32 + [1] * 32, (33, 8192))])
