@@ -317,7 +317,8 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         // ---- SwiGLU: accumulator rows 0..h-1 = gate, h..2h-1 = up of features [h t, h t + h); columns = tokens.  All of it goes through
         //      shared memory (the tile ring is drained), token-major and conflict-free, and the four warps share the activations, two
         //      neighbouring features a thread: 64 rows have 4096 or 2048 of them, each an exponential and a division, which the one or two
-        //      warps that hold the gates took longer for than for the product (64 rows, 4096 features of 1024 channels 15.1 -> 8.7 us, 128 rows 23.5 -> 13.2, 64 x 18944 x 3584 49.6 -> 45.8) ----
+        //      warps that hold the gates took longer for than for the product (64 rows, 4096 features of 1024 channels 15.1 -> 8.7 us,
+        //      128 rows 23.5 -> 13.2, 64 x 18944 x 3584 49.6 -> 45.8) ----
         float* xch = reinterpret_cast<float*>(smem_raw + (smem_base - ptx::smem_u32(smem_raw)));   // [kNTile][2 h]
         const int h = p.tile_rows / 2;
         if (q * 32 < 2 * h) {

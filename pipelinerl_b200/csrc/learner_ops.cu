@@ -466,7 +466,8 @@ int row_bwd_grid(int64_t T, int64_t H) {
 // ring, us: 3584 channels (two blocks an SM) 4096 25.0 / 27.9, 8192 43.5 / 43.9, 12000 63.9 / 62.0, 16384 84.0 / 81.0, 32768 158 / 150; 5120 (one) 4096 35.1 / 37.2,
 // 6000 51.6 / 49.5, 16384 132 / 118; 2048 (four) 4096 20.8 / 20.9, 6000 26.9 / 26.0, 16384 55.8 / 51.9; 128 12000 18.7 / 16.7; 2056 16384 65.6 / 67.8; 4096,
 // where two blocks have four slots each, 32768 173 / 177; 384 and 512 (two warps a block) 14000 19.5 / 20.7 and 20.1 / 21.2, 24000 27.1 / 28.5 and
-// 28.2 / 28.8, 60000 55.9 / 56.2 and 62.7 / 57.0; 640 (three) 14000 24.4 / 24.6, 24000 35.3 / 34.4; 1024 (four) 14000 29.4 / 28.3.  The forward lost throughout (16384 x 3584 43.4 / 46.1): one row in flight a block was enough.
+// 28.2 / 28.8, 60000 55.9 / 56.2 and 62.7 / 57.0; 640 (three) 14000 24.4 / 24.6, 24000 35.3 / 34.4; 1024 (four) 14000 29.4 / 28.3.
+// The forward lost throughout (16384 x 3584 43.4 / 46.1): one row in flight a block was enough.
 int ring_slots(int64_t T, int64_t H, int64_t grid, int mats) {
   const int vecs = row_vecs(H), warps = row_threads(H) / 32;
   if (H % 64 != 0 || T < (vecs > 1 ? 40 : warps == 2 ? 50 : warps == 3 ? 20 : 10) * grid) return 0;

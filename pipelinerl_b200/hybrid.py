@@ -30,7 +30,8 @@ their share of the chosen scores; tanh-capped logits.
 Numerics: the residual stream, every norm, softmax, router-like gate, decay, step size and recurrent state are fp32.
 GEMM operands and the KV cache are bf16, or fp32 when the arena is fp32 (the true-fp32 mode: CUDA-core GEMMs with fp32
 accumulation in a fixed order, no TF32).  One code path serves prompt chunks, single decoded tokens and mixtures of
-both ("ragged rows"); a token's result depends only on its own sequence.
+both ("ragged rows"); a token's result depends only on its own sequence (and, in the last bits of decode attention, on the
+shares that contexts are cut into, EngineCore._attn_plan).
 """
 from __future__ import annotations
 
