@@ -633,10 +633,18 @@ extern "C" int prl_attn_set_fused_combine(int32_t on) {
 // 10.2, of 256 12.1 / 10.2 / 11.3, of 1024 31.1 / 20.3 / 17.8; two of 128 9.6 / 9.6 / 12.2, of 256 12.9 / 11.8 / 14.2, of 2048 56.2 / 33.4 /
 // 31.3; four of 256 13.2 / 13.5 / 19.9, of 1024 32.0 / 28.0 / 34.8.  One more cut where long contexts leave SMs idle or unevenly filled: 96 of 125 60.5 / 56.2,
 // 256 of 129 145 / 137, 256 of 86 100 / 94, but 256 of 47 55.9 / 58.7, of 10 16.3 / 21.4, 160 of 128 96 / 106, 512 of 125 255 / 268.
-static int cuts_of(int ctas, int pages) {
+//
+// Beside `empty` CTAs per share, of slots without a token, a cut has to save more, for theirs come on top of it (32 slots, us by 1 / 2 / 4 shares: 16 of 21
+// pages 12.9 / 13.3 / 16.2, of 32 17.1 / 16.4 / 19.8; 8 of 10 8.0 / 8.3 / 9.1, of 15 10.0 / 9.4 / 9.8, of 32 16.7 / 12.8 / 12.1; 4 of 10 7.9 / 7.9 / 7.1; 64 slots, 8 of
+// 10 8.0 / 8.9, of 15 10.1 / 10.1, of 21 12.3 / 11.2; 16 slots by 4 / 8, 4 of 21 8.2 / 8.9, of 47 10.9 / 11.1).
+static int cuts_of(int ctas, int pages, int empty = 0) {
   const int sms = num_sms();
+  const int first = !empty ? 9 : 4 * ctas > sms ? 32 : ctas + empty > sms ? 14 : 9;       // pages of a context that is cut at all
   int s = 1;
-  while (s < 64 && ctas * s * 2 <= sms && pages > 8 && pages >= 5 * s && (s < 16 || (int64_t)4 * pages > (int64_t)s * s * ctas)) s *= 2;
+  while (s < 64 && ctas * s * 2 <= sms && pages >= first && pages >= 5 * s && (s < 16 || (int64_t)4 * pages > (int64_t)s * s * ctas)) {
+    if (empty && s > 1 && ctas * s * 4 > sms && pages < 12 * s) break;
+    s *= 2;
+  }
   if (s == 1 && ((ctas <= sms && pages >= 96) || (4 * ctas > 5 * sms && ctas <= 2 * sms && pages >= 64))) s = 2;
   return s;
 }
@@ -654,7 +662,7 @@ extern "C" int prl_paged_attn_splits(int32_t B, int32_t n_kv, int32_t max_seq_le
 // 4096 28.8 / 12.8, and with six stages for three, where the live CTAs have an SM each: eight of 64 x 8192 42.6 / 32.4.
 extern "C" int prl_paged_attn_plan(int32_t slots, int32_t live, int32_t n_kv, int32_t longest, int32_t max_seq_len, int32_t* stages) {
   const int sms = num_sms(), full = prl_paged_attn_splits(slots, n_kv, max_seq_len);
-  int splits = cuts_of(live * n_kv, (longest + kPage - 1) / kPage);
+  int splits = cuts_of(live * n_kv, (longest + kPage - 1) / kPage, (slots - live) * n_kv);
   while (splits > full && slots * n_kv * splits >= 4 * sms) splits /= 2;
   while (((max_seq_len + kPage - 1) / kPage + splits - 1) / splits > kMaxPagesPerSplit) splits *= 2;
   if (stages) *stages = live * n_kv * splits > sms ? kStages / 2 : kStages;

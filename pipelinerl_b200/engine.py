@@ -46,6 +46,7 @@ class Request:
     model_version: int = 0
     prefilled: int = 0                                   # prompt tokens whose KV is in the cache
     waits_for: list = field(default_factory=list)        # [(request filling a shared page, tokens it must reach)]
+    first_step: int = 0                                  # the engine's step count when it was admitted
 
 
 def batch_contexts(lengths: list[int]) -> tuple[int, int]:
@@ -245,12 +246,14 @@ class EngineCore:
         return None
 
     def _batch_contexts(self) -> tuple[int, int]:
-        """batch_contexts of the requests that have a slot, each as long as it may become (slots that were filled without a request: all)."""
-        at = (self._next_id, len(self.slot_req))       # a request that comes counts up, one that goes alone leaves fewer
+        """batch_contexts of the requests that have a slot, looked at anew for each page of steps (slots that were filled without a request: all
+        as long as may be)."""
+        # a request that comes counts up, one that goes alone leaves fewer
+        at = (self._next_id, len(self.slot_req), self.step_count // PAGE_SIZE)
         if self._contexts[0] != at:
-            reqs = self.slot_req.values()
-            self._contexts = at, batch_contexts([min(self.max_seq_len, len(r.prompt_ids) + r.params.max_tokens) for r in reqs]
-                                                or [self.max_seq_len] * self.B)
+            end = (at[2] + 1) * PAGE_SIZE
+            self._contexts = at, batch_contexts([min(len(r.prompt_ids) + min(r.params.max_tokens, end - r.first_step), self.max_seq_len)
+                                                 for r in self.slot_req.values()] or [self.max_seq_len] * self.B)
         return self._contexts[1]
 
     def _attn_plan(self, n_kv: int) -> tuple[int, int]:
@@ -377,7 +380,7 @@ class EngineCore:
         self._check_params(params)
         if not self.can_admit(n, params.max_tokens):
             raise RuntimeError("engine full")
-        req = Request(self._next_id, list(prompt_ids), params, model_version=model_version)
+        req = Request(self._next_id, list(prompt_ids), params, model_version=model_version, first_step=self.step_count)
         self._next_id += 1
         slot = self.free_slots.pop()
         n_pages = (n + params.max_tokens + PAGE_SIZE - 1) // PAGE_SIZE

@@ -51,6 +51,13 @@ def test_shares_of_decode_attention(slots, live, n_kv, longest, plan):
         assert _lib.load().prl_paged_attn_splits(slots, n_kv, longest) == plan[0]
 
 
+@pytest.mark.parametrize("slots,live,longest,splits", [(32, 8, 512, 1), (32, 8, 513, 2), (32, 8, 1472, 2), (32, 8, 1473, 4), (32, 16, 1984, 1), (32, 16, 1985, 2), (64, 4, 832, 1),
+                                                        (64, 4, 833, 2), (16, 4, 640, 4), (16, 4, 3008, 4), (16, 4, 3009, 8), (16, 1, 1216, 4), (16, 1, 1217, 8)])
+def test_shares_beside_empty_slots(slots, live, longest, splits):
+    """Both sides of the lines for batches with slots that have no token (four key heads)."""
+    assert attn_plan(slots, live, 4, longest, 16384)[0] == splits
+
+
 @pytest.mark.parametrize("slots", [1, 3, 16, 40, 64, 130])
 @pytest.mark.parametrize("n_kv,max_seq_len", [(1, 640), (2, 2048), (4, 16384), (8, 131072)])
 def test_workspace_of_the_longest_contexts_is_enough(slots, n_kv, max_seq_len):
