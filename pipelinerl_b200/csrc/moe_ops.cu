@@ -649,12 +649,11 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// Two products of a feed-forward launched together (prl_moe_mlp_act): the first (kPairFirst) lets the second start only after its own wait,
-// so the second (kPairSecond) knows its tile before it waits, and has its weights in flight when the first one's last CTA ends.  Both are
-// streams of weights with a ramp of four dependent loads: a hybrid token step of 32 rows, 4 layers 586 -> 579 us.  (The first's weights
-// asked for in L2 while the router runs: 512 or 1024 bytes of a row nothing, 2048 three us slower, whole rows ten.)
-enum { kPairNone = 0, kPairFirst = 1, kPairSecond = 2 };
-template <int ACT, int PAIR>
+// EARLY: the two products of a feed-forward launched together (prl_moe_mlp_act) let the next kernel start behind their own wait, so that its
+// blocks are there when this one's last ends.  Nothing of the row table is read ahead of the wait, which alone makes another kernel's writes
+// visible, also of one two kernels back.  (The second product's weights asked for there, by a table read ahead of the wait: 559 us
+// for 562 of a hybrid token step of 32 rows, 4 layers.)
+template <int ACT, bool EARLY>
 __global__ void __launch_bounds__(256) moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, int a_mod,
                                                            const __nv_bfloat16* __restrict__ W, int64_t expert_stride,
                                                            int64_t ldw, const int32_t* __restrict__ perm,
@@ -662,12 +661,9 @@ __global__ void __launch_bounds__(256) moe_gemm_mma_kernel(const __nv_bfloat16* 
                                                            int N, int K, void* __restrict__ C_v, int64_t ldc, int c_perm,
                                                            const float* __restrict__ wsel) {
   const int tile = blockIdx.y;
-  if constexpr (PAIR != kPairSecond) pdl_wait();
-  if constexpr (PAIR == kPairFirst) pdl_launch_dependents();
-  if (tile >= meta[0]) {
-    if constexpr (PAIR == kPairSecond) pdl_wait();
-    return;
-  }
+  pdl_wait();
+  if constexpr (EARLY) pdl_launch_dependents();
+  if (tile >= meta[0]) return;
   extern __shared__ __align__(16) unsigned char mma_smem[];
   typedef __nv_bfloat16 (*ATile)[kTile][kLds];
   typedef __nv_bfloat16 (*BTile)[kBN][kLds];
@@ -718,16 +714,10 @@ __global__ void __launch_bounds__(256) moe_gemm_mma_kernel(const __nv_bfloat16* 
   };
   // kStages - 1 steps in flight; a commit per step keeps the group count regular (empty past the end, where `stage`
   // copies nothing but zero fill into a buffer nobody reads)
-  if constexpr (PAIR == kPairSecond) {      // the weights of the first steps ride in the first group
-#pragma unroll
-    for (int st = 0; st < kStages - 1; ++st) stage_b(st * kBK, st);
-    pdl_wait();
-    pdl_launch_dependents();
-  }
 #pragma unroll
   for (int st = 0; st < kStages - 1; ++st) {
     stage_a(st * kBK, st);
-    if constexpr (PAIR != kPairSecond) stage_b(st * kBK, st);
+    stage_b(st * kBK, st);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   int buf = 0;
@@ -802,19 +792,16 @@ __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t a) {
 // 128 features a block: 54.4 at 32 tokens; 32 features: 53.1.  A hybrid token step of 32 rows, 4 layers: 581 -> 570 us.
 constexpr int kFeatures = 64;
 constexpr int kRingBytes = 53 * 1024;             // four blocks share an SM
-template <int ACT, int PAIR>
+template <int ACT, bool EARLY>
 __global__ void __launch_bounds__(64 + 2 * kFeatures) moe_gemm_ring_kernel(const __grid_constant__ CUtensorMap tm_w, const __nv_bfloat16* __restrict__ A,
                                                                   int64_t lda, int a_mod, const int32_t* __restrict__ perm,
                                                                   const int32_t* __restrict__ meta, const int32_t* __restrict__ tiles, int N, int K,
                                                                   void* __restrict__ C_v, int64_t ldc, int c_perm,
                                                                   const float* __restrict__ wsel) {
   const int tile = blockIdx.y;
-  if constexpr (PAIR != kPairSecond) pdl_wait();
-  if constexpr (PAIR == kPairFirst) pdl_launch_dependents();
-  if (tile >= meta[0]) {
-    if constexpr (PAIR == kPairSecond) pdl_wait();
-    return;
-  }
+  pdl_wait();
+  if constexpr (EARLY) pdl_launch_dependents();
+  if (tile >= meta[0]) return;
   extern __shared__ uint8_t ring_raw[];
   constexpr int kWarps = kFeatures / 16, kMost = 5, kWBytes = kFeatures * kBK * 2;
   __shared__ int32_t a_row[kTile], c_row[kTile];
@@ -868,10 +855,6 @@ __global__ void __launch_bounds__(64 + 2 * kFeatures) moe_gemm_ring_kernel(const
   }
   if (warp == 1) {
     // ===== rows: lane = 16-byte piece of one row in four =====
-    if constexpr (PAIR == kPairSecond) {
-      pdl_wait();
-      pdl_launch_dependents();
-    }
     const int c = lane & 7, r0 = lane >> 3;
     int s = 0;
     uint32_t ph = 1;
@@ -925,7 +908,6 @@ __global__ void __launch_bounds__(64 + 2 * kFeatures) moe_gemm_ring_kernel(const
     if (lane == 0) ptx::mbar_arrive(empty + 8u * (uint32_t)st);
     if (++st == n_st) { st = 0; ph ^= 1u; }
   }
-  if constexpr (PAIR == kPairSecond) pdl_wait();      // the output may still be read by what ran before the first product
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -1142,7 +1124,7 @@ extern "C" int prl_moe_few_rows(int64_t tokens, int64_t pairs, int32_t experts) 
   return moe_few_rows(tokens, pairs, prl_moe_max_tiles(pairs, experts));
 }
 
-template <int ACT, int PAIR = kPairNone>
+template <int ACT, bool EARLY = false>
 static int moe_gemm_impl(const void* A, int32_t a_is_f32, int64_t lda, int32_t a_mod, const void* W, int32_t w_is_f32,
                          int64_t expert_stride, int64_t ldw, const int32_t* perm, const int32_t* meta, const int32_t* tiles,
                          int64_t max_tiles, int64_t N, int64_t K, void* C, int64_t ldc, int32_t c_perm, const float* wsel, bool few,
@@ -1158,8 +1140,8 @@ static int moe_gemm_impl(const void* A, int32_t a_is_f32, int64_t lda, int32_t a
       const int rc = make_tmap_3d_bf16(&tw, W, (uint64_t)K, (uint64_t)N, 1u << 16, (uint64_t)ldw * 2, (uint64_t)expert_stride * 2, kBK, kFeatures, 1);
       if (rc) return rc;
       static SmemAttr ring_attr = {};
-      PRL_CUDA(ensure_smem((moe_gemm_ring_kernel<ACT, PAIR>), kRingBytes + 1024, ring_attr));
-      PRL_CUDA(launch_pdl((moe_gemm_ring_kernel<ACT, PAIR>), dim3((unsigned)((N + kFeatures - 1) / kFeatures), (unsigned)max_tiles),
+      PRL_CUDA(ensure_smem((moe_gemm_ring_kernel<ACT, EARLY>), kRingBytes + 1024, ring_attr));
+      PRL_CUDA(launch_pdl((moe_gemm_ring_kernel<ACT, EARLY>), dim3((unsigned)((N + kFeatures - 1) / kFeatures), (unsigned)max_tiles),
                           dim3(64 + 2 * kFeatures), (size_t)(kRingBytes + 1024), s, tw, (const bf16*)A, lda, a_mod, perm, meta, tiles, (int)N, (int)K,
                           C, ldc, c_perm, wsel));
       PRL_LAUNCH_CHECK();
@@ -1167,8 +1149,8 @@ static int moe_gemm_impl(const void* A, int32_t a_is_f32, int64_t lda, int32_t a
     }
     dim3 grid_tc((unsigned)((N + kBN - 1) / kBN), (unsigned)max_tiles);
     static SmemAttr attr = {};
-    PRL_CUDA(ensure_smem((moe_gemm_mma_kernel<ACT, PAIR>), (int)kMmaSmem, attr));
-    PRL_CUDA(launch_pdl((moe_gemm_mma_kernel<ACT, PAIR>), grid_tc, dim3(256), kMmaSmem, s, (const bf16*)A, lda, a_mod, (const bf16*)W,
+    PRL_CUDA(ensure_smem((moe_gemm_mma_kernel<ACT, EARLY>), (int)kMmaSmem, attr));
+    PRL_CUDA(launch_pdl((moe_gemm_mma_kernel<ACT, EARLY>), grid_tc, dim3(256), kMmaSmem, s, (const bf16*)A, lda, a_mod, (const bf16*)W,
                         expert_stride, ldw, perm, meta, tiles, (int)N, (int)K, C, ldc, c_perm, wsel));
     PRL_LAUNCH_CHECK();
     return PRL_OK;
@@ -1221,8 +1203,8 @@ static int moe_mlp_impl(const void* x, int32_t f32, int32_t n, const void* up, c
                         const int32_t* meta, const int32_t* tiles, int64_t max_tiles, int64_t pairs, const float* wsel, void* act_out,
                         float* out, prl_stream_t st) {
   const bool few = moe_few_rows(n, pairs, max_tiles);
-  const int rc = moe_gemm_impl<ACT, kPairFirst>(x, f32, W, n, up, f32, F * W, W, perm, meta, tiles, max_tiles, F, W, act_out, F, 0, wsel, few, st);
-  return rc ? rc : moe_gemm_impl<kActNone, kPairSecond>(act_out, f32, F, 0, down, f32, W * F, F, perm, meta, tiles, max_tiles, W, F, out, W, 1,
+  const int rc = moe_gemm_impl<ACT, true>(x, f32, W, n, up, f32, F * W, W, perm, meta, tiles, max_tiles, F, W, act_out, F, 0, wsel, few, st);
+  return rc ? rc : moe_gemm_impl<kActNone, true>(act_out, f32, F, 0, down, f32, W * F, F, perm, meta, tiles, max_tiles, W, F, out, W, 1,
                                                         nullptr, few, st);
 }
 
