@@ -874,15 +874,6 @@ int prl_moe_gemm_act(const void* A, int32_t a_is_f32, int64_t lda, int32_t a_mod
 int prl_moe_mlp_act(const void* x, int32_t f32, int32_t n, const void* up, const void* down, int64_t W, int64_t F,
                     const int32_t* perm, const int32_t* meta, const int32_t* tiles, int64_t max_tiles, int32_t act,
                     const float* wsel, void* act_out, float* out, prl_stream_t stream);
-/* prl_moe_gemm and prl_moe_mlp_act told how many pairs the experts share: a kernel for few rows runs, with the same bits, for few tokens and
- * up to 22 pairs per expert (prl_moe_few_rows); the entries above know the tokens only */
-int prl_moe_few_rows(int64_t tokens, int64_t pairs, int32_t experts);
-int prl_moe_gemm_pairs(const void* A, int32_t a_is_f32, int64_t lda, int32_t a_mod, const void* W, int32_t w_is_f32,
-                       int64_t expert_stride, int64_t ldw, const int32_t* perm, const int32_t* meta, const int32_t* tiles,
-                       int64_t max_tiles, int64_t pairs, int64_t N, int64_t K, float* C, int64_t ldc, int32_t c_perm, prl_stream_t stream);
-int prl_moe_mlp_act_pairs(const void* x, int32_t f32, int32_t n, const void* up, const void* down, int64_t W, int64_t F,
-                          const int32_t* perm, const int32_t* meta, const int32_t* tiles, int64_t max_tiles, int64_t pairs, int32_t act,
-                          const float* wsel, void* act_out, float* out, prl_stream_t stream);
 int prl_moe_glu(const float* gate_up, int64_t ld, int64_t pairs, int32_t F, const int32_t* perm, const float* wsel,
                 float limit, float beta, void* out, int32_t f32, prl_stream_t stream);
 

@@ -24,12 +24,8 @@
 // warps, operands staged by cp.async (zero-filled past the edges) into a double buffer and read with ldmatrix.  A
 // row's result depends only on the row and the expert's weights, never on which rows share its tile.
 #include "prl_common.cuh"
-#include "tc_ptx.cuh"
 
 namespace prl {
-
-int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1_bytes,
-                      uint64_t stride2_bytes, uint32_t box0, uint32_t box1, uint32_t box2);  // gemm_tc.cu
 
 namespace {
 
@@ -651,8 +647,7 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
 
 // EARLY: the two products of a feed-forward launched together (prl_moe_mlp_act) let the next kernel start behind their own wait, so that its
 // blocks are there when this one's last ends.  Nothing of the row table is read ahead of the wait, which alone makes another kernel's writes
-// visible, also of one two kernels back.  (The second product's weights asked for there, by a table read ahead of the wait: 559 us
-// for 562 of a hybrid token step of 32 rows, 4 layers.)
+// visible, also of one two kernels back.
 template <int ACT, bool EARLY>
 __global__ void __launch_bounds__(256) moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, int a_mod,
                                                            const __nv_bfloat16* __restrict__ W, int64_t expert_stride,
@@ -766,168 +761,6 @@ __global__ void __launch_bounds__(256) moe_gemm_mma_kernel(const __nv_bfloat16* 
         const int nn = n0 + wn + 8 * j + (lane & 3) * 2;
         if (nn < N) crow[nn] = acc[i][j][2 * half];
         if (nn + 1 < N) crow[nn + 1] = acc[i][j][2 * half + 1];
-      }
-    }
-}
-
-// ---- ... for few rows per expert ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, int bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-// the barrier's count goes down by one when this thread's copies so far have landed
-__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t a) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
-}
-// A token step's experts are a stream of weights: 134 MB per product of 16 experts of 2048 x 2048, 20.5 us at the copy rate, whatever the
-// rows.  One warp asks for weight tiles (TMA, 128-byte swizzle) and one for the tokens' rows (cp.async through the row table, in the same
-// swizzle), as far ahead as the ring goes; four read what has come, 16 output features each, and multiply.  Nothing holds the block
-// together but the ring's barriers.  (In the kernel above all threads copy, meet at a barrier and are three steps ahead: a step of 64 channels takes
-// 0.65 us whatever the experts.)  The products and their order are those of the kernel above, so the same bits.  Both products with the
-// router, us, that kernel / this one: 16 experts of 2048 x 2048, top 4: 1 token 50.7 / 33.0, 4 tokens 61.8 / 39.2, 32 tokens 63.7 / 52.1, 48 64.8 /
-// 59.0, 80 66.2 / 66.3, 128 83.6 / 86.8, 1024 327 / 410; 64 of 2048 x 1024, top 8: 32 tokens 129 / 103, 100 136 / 116, 380 193 / 223.
-// 128 features a block: 54.4 at 32 tokens; 32 features: 53.1.  A hybrid token step of 32 rows, 4 layers: 581 -> 570 us.
-constexpr int kFeatures = 64;
-constexpr int kRingBytes = 53 * 1024;             // four blocks share an SM
-template <int ACT, bool EARLY>
-__global__ void __launch_bounds__(64 + 2 * kFeatures) moe_gemm_ring_kernel(const __grid_constant__ CUtensorMap tm_w, const __nv_bfloat16* __restrict__ A,
-                                                                  int64_t lda, int a_mod, const int32_t* __restrict__ perm,
-                                                                  const int32_t* __restrict__ meta, const int32_t* __restrict__ tiles, int N, int K,
-                                                                  void* __restrict__ C_v, int64_t ldc, int c_perm,
-                                                                  const float* __restrict__ wsel) {
-  const int tile = blockIdx.y;
-  pdl_wait();
-  if constexpr (EARLY) pdl_launch_dependents();
-  if (tile >= meta[0]) return;
-  extern __shared__ uint8_t ring_raw[];
-  constexpr int kWarps = kFeatures / 16, kMost = 5, kWBytes = kFeatures * kBK * 2;
-  __shared__ int32_t a_row[kTile], c_row[kTile];
-  __shared__ float c_w[kTile];
-  __shared__ uint64_t bars[2 * kMost];
-  const uint32_t ring = (ptx::smem_u32(ring_raw) + 1023u) & ~1023u, full = ptx::smem_u32(bars), empty = full + 8u * kMost;
-  const int e = tiles[3 * tile], s0 = tiles[3 * tile + 1], M = tiles[3 * tile + 2];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n0 = blockIdx.x * kFeatures, steps = (K + kBK - 1) / kBK, blocks = (M + 15) / 16;
-  const int stage_bytes = kWBytes + blocks * 16 * kBK * 2;                       // weights, then the rows of this tile, 16 at a time
-  const int fit = kRingBytes / stage_bytes, n_st = fit < kMost ? fit : kMost;
-  auto ask_weights = [&](int i, int s) {
-    if (ptx::elect_one()) {
-      ptx::mbar_arrive_expect_tx(full + 8u * (uint32_t)s, (uint32_t)kWBytes);
-      ptx::tma_load_3d(ring + (uint32_t)(s * stage_bytes), &tm_w, i * kBK, n0, e, full + 8u * (uint32_t)s, ptx::kEvictFirst);
-    }
-    __syncwarp();
-  };
-  const int pre = steps < n_st ? steps : n_st;
-  if (warp == 0) {
-    if (ptx::elect_one()) {
-      for (int s = 0; s < n_st; ++s) {
-        ptx::mbar_init(full + 8u * (uint32_t)s, 33);       // the weights, and each lane of the rows' warp
-        ptx::mbar_init(empty + 8u * (uint32_t)s, kWarps);
-      }
-      ptx::fence_barrier_init();
-      ptx::fence_proxy_async();
-    }
-    __syncwarp();
-    for (int i = 0; i < pre; ++i) ask_weights(i, i);
-  } else {
-    for (int r = tid - 32; r < kTile; r += 32 + 2 * kFeatures) {
-      const int s = s0 + min(r, M - 1);
-      const int p = perm[s];
-      if constexpr (ACT != kActNone) c_w[r] = wsel[p];
-      a_row[r] = a_mod > 0 ? p % a_mod : s;
-      c_row[r] = c_perm ? p : s;
-    }
-  }
-  __syncthreads();
-  if (warp == 0) {
-    // ===== weights =====
-    int s = pre == n_st ? 0 : pre;
-    uint32_t ph = 0;
-    for (int i = pre; i < steps; ++i) {
-      ptx::mbar_wait(empty + 8u * (uint32_t)s, ph);
-      ask_weights(i, s);
-      if (++s == n_st) { s = 0; ph ^= 1u; }
-    }
-    return;
-  }
-  if (warp == 1) {
-    // ===== rows: lane = 16-byte piece of one row in four =====
-    const int c = lane & 7, r0 = lane >> 3;
-    int s = 0;
-    uint32_t ph = 1;
-    for (int i = 0; i < steps; ++i) {
-      ptx::mbar_wait(empty + 8u * (uint32_t)s, ph);
-      const int k = i * kBK + c * 8;
-      const uint32_t dst = ring + (uint32_t)(s * stage_bytes + kWBytes);
-      for (int r = r0; r < blocks * 16; r += 4) {
-        const bool in = r < M && k < K;
-        cp_async16_zfill(dst + (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)), A + (in ? a_row[r] * lda + k : 0), in ? 16 : 0);
-      }
-      cp_async_arrive(full + 8u * (uint32_t)s);
-      if (++s == n_st) { s = 0; ph ^= 1u; }
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    return;
-  }
-  // ===== products: a warp's 16 features for all rows =====
-  const int f0 = (warp - 2) * 16;
-  float acc[4][2][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.f;
-  const int b_r = f0 + (lane & 7) + ((lane >> 4) << 3), b_c = (lane >> 3) & 1;
-  const int a_r = lane & 15, a_c = lane >> 4;
-  const uint32_t b_off = (uint32_t)(b_r * 128), a_off = (uint32_t)(kWBytes + a_r * 128);
-  int st = 0;
-  uint32_t ph = 0;
-  for (int i = 0; i < steps; ++i) {
-    ptx::mbar_wait(full + 8u * (uint32_t)st, ph);
-    const uint32_t base = ring + (uint32_t)(st * stage_bytes);
-    uint32_t bf[4][4];
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) ldsm_x4(bf[kk], base + b_off + (uint32_t)(((2 * kk + b_c) ^ (b_r & 7)) << 4));
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      if (m < blocks) {
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          uint32_t af[4];
-          ldsm_x4(af, base + a_off + (uint32_t)(m * 2048 + (((2 * kk + a_c) ^ (a_r & 7)) << 4)));
-          mma_bf16(acc[m][0], af, bf[kk][0], bf[kk][1]);
-          mma_bf16(acc[m][1], af, bf[kk][2], bf[kk][3]);
-        }
-      }
-    }
-    __syncwarp();
-    if (lane == 0) ptx::mbar_arrive(empty + 8u * (uint32_t)st);
-    if (++st == n_st) { st = 0; ph ^= 1u; }
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int m = 16 * i + (lane >> 2) + 8 * half;
-      if (m >= M) continue;
-      const int64_t at = (int64_t)c_row[m] * ldc;
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int nn = n0 + f0 + 8 * j + (lane & 3) * 2;
-        if constexpr (ACT != kActNone) {
-          __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(C_v) + at;
-          const float w = c_w[m];
-          if (nn < N) crow[nn] = __float2bfloat16_rn(expert_act<ACT>(acc[i][j][2 * half]) * w);
-          if (nn + 1 < N) crow[nn + 1] = __float2bfloat16_rn(expert_act<ACT>(acc[i][j][2 * half + 1]) * w);
-        } else {
-          float* crow = reinterpret_cast<float*>(C_v) + at;
-          if (nn < N) crow[nn] = acc[i][j][2 * half];
-          if (nn + 1 < N) crow[nn + 1] = acc[i][j][2 * half + 1];
-        }
       }
     }
 }
@@ -1112,22 +945,10 @@ extern "C" int prl_moe_gather(const void* x_bf16, const int32_t* perm, const int
   return PRL_OK;
 }
 
-// Few rows per expert, where the ring kernel is the faster one: few tokens for the experts (max_tiles is the experts and a 64th of the pairs, rounded
-// up), which with four choices a token are 15 rows per expert at most, but with eight 38; so where the pairs are told, at most 22 of them per
-// expert.  Former kernel / ring, both products, us: 64 experts of 2048 x 1024, 12.5 rows 119 / 93, 18.8 125 / 115, 22.5 127 / 122, 25 135 / 129,
-// 28.8 140 / 142, 38.6 155 / 168; 64 of 1024 x 512, 25 42.9 / 43.6, 38.6 48.8 / 54.0; 128 of them 18.8 73 / 64; 32 of 2048 x 1024, 25 69.4 / 71.5, 30 77.6 / 81.2;
-// 16 of 2048 x 2048, 15 59.4 / 59.0, 18 59.7 / 61.1.
-static bool moe_few_rows(int64_t tokens, int64_t pairs, int64_t max_tiles) {
-  return tokens > 0 && tokens <= 3 * max_tiles && (pairs <= 0 || pairs <= 22 * (max_tiles - (pairs + kTile - 1) / kTile));
-}
-extern "C" int prl_moe_few_rows(int64_t tokens, int64_t pairs, int32_t experts) {
-  return moe_few_rows(tokens, pairs, prl_moe_max_tiles(pairs, experts));
-}
-
 template <int ACT, bool EARLY = false>
 static int moe_gemm_impl(const void* A, int32_t a_is_f32, int64_t lda, int32_t a_mod, const void* W, int32_t w_is_f32,
                          int64_t expert_stride, int64_t ldw, const int32_t* perm, const int32_t* meta, const int32_t* tiles,
-                         int64_t max_tiles, int64_t N, int64_t K, void* C, int64_t ldc, int32_t c_perm, const float* wsel, bool few,
+                         int64_t max_tiles, int64_t N, int64_t K, void* C, int64_t ldc, int32_t c_perm, const float* wsel,
                          prl_stream_t st) {
   PRL_CHECK_ARG(A && W && perm && meta && tiles && C && (ACT == kActNone || wsel), "prl_moe_gemm: NULL argument");
   PRL_CHECK_ARG(max_tiles >= 1 && max_tiles <= 65535 && N >= 1 && K >= 1 && lda >= K && ldw >= K && ldc >= N && a_mod >= 0,
@@ -1135,18 +956,6 @@ static int moe_gemm_impl(const void* A, int32_t a_is_f32, int64_t lda, int32_t a
   cudaStream_t s = (cudaStream_t)st;
   if (!a_is_f32 && !w_is_f32 && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && expert_stride % 8 == 0 &&
       ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0) {
-    if (few && expert_stride > 0) {
-      CUtensorMap tw;
-      const int rc = make_tmap_3d_bf16(&tw, W, (uint64_t)K, (uint64_t)N, 1u << 16, (uint64_t)ldw * 2, (uint64_t)expert_stride * 2, kBK, kFeatures, 1);
-      if (rc) return rc;
-      static SmemAttr ring_attr = {};
-      PRL_CUDA(ensure_smem((moe_gemm_ring_kernel<ACT, EARLY>), kRingBytes + 1024, ring_attr));
-      PRL_CUDA(launch_pdl((moe_gemm_ring_kernel<ACT, EARLY>), dim3((unsigned)((N + kFeatures - 1) / kFeatures), (unsigned)max_tiles),
-                          dim3(64 + 2 * kFeatures), (size_t)(kRingBytes + 1024), s, tw, (const bf16*)A, lda, a_mod, perm, meta, tiles, (int)N, (int)K,
-                          C, ldc, c_perm, wsel));
-      PRL_LAUNCH_CHECK();
-      return PRL_OK;
-    }
     dim3 grid_tc((unsigned)((N + kBN - 1) / kBN), (unsigned)max_tiles);
     static SmemAttr attr = {};
     PRL_CUDA(ensure_smem((moe_gemm_mma_kernel<ACT, EARLY>), (int)kMmaSmem, attr));
@@ -1172,16 +981,7 @@ extern "C" int prl_moe_gemm(const void* A, int32_t a_is_f32, int64_t lda, int32_
                             const int32_t* tiles, int64_t max_tiles, int64_t N, int64_t K, float* C, int64_t ldc,
                             int32_t c_perm, prl_stream_t st) {
   return moe_gemm_impl<kActNone>(A, a_is_f32, lda, a_mod, W, w_is_f32, expert_stride, ldw, perm, meta, tiles, max_tiles, N, K, C, ldc,
-                                 c_perm, nullptr, moe_few_rows(a_mod, 0, max_tiles), st);
-}
-
-// ... told how many pairs there are
-extern "C" int prl_moe_gemm_pairs(const void* A, int32_t a_is_f32, int64_t lda, int32_t a_mod, const void* W, int32_t w_is_f32,
-                                  int64_t expert_stride, int64_t ldw, const int32_t* perm, const int32_t* meta, const int32_t* tiles,
-                                  int64_t max_tiles, int64_t pairs, int64_t N, int64_t K, float* C, int64_t ldc, int32_t c_perm, prl_stream_t st) {
-  PRL_CHECK_ARG(pairs >= 1, "prl_moe_gemm_pairs: no pairs");
-  return moe_gemm_impl<kActNone>(A, a_is_f32, lda, a_mod, W, w_is_f32, expert_stride, ldw, perm, meta, tiles, max_tiles, N, K, C, ldc,
-                                 c_perm, nullptr, moe_few_rows(a_mod, pairs, max_tiles), st);
+                              c_perm, nullptr, st);
 }
 
 // First product of ungated experts: out[s] = act(A[row of s] W_e^T) * wsel[pair of s], in the operand type of A and in sorted
@@ -1193,42 +993,28 @@ extern "C" int prl_moe_gemm_act(const void* A, int32_t a_is_f32, int64_t lda, in
                                 void* out, int64_t ld_out, prl_stream_t st) {
   PRL_CHECK_ARG(act == kActRelu2 || act == kActGelu, "prl_moe_gemm_act: unknown activation %d", act);
   return act == kActRelu2 ? moe_gemm_impl<kActRelu2>(A, a_is_f32, lda, a_mod, W, w_is_f32, expert_stride, ldw, perm, meta, tiles, max_tiles,
-                                                     N, K, out, ld_out, 0, wsel, moe_few_rows(a_mod, 0, max_tiles), st)
+                                                     N, K, out, ld_out, 0, wsel, st)
                           : moe_gemm_impl<kActGelu>(A, a_is_f32, lda, a_mod, W, w_is_f32, expert_stride, ldw, perm, meta, tiles, max_tiles,
-                                                    N, K, out, ld_out, 0, wsel, moe_few_rows(a_mod, 0, max_tiles), st);
+                                                    N, K, out, ld_out, 0, wsel, st);
 }
 
 template <int ACT>
 static int moe_mlp_impl(const void* x, int32_t f32, int32_t n, const void* up, const void* down, int64_t W, int64_t F, const int32_t* perm,
-                        const int32_t* meta, const int32_t* tiles, int64_t max_tiles, int64_t pairs, const float* wsel, void* act_out,
-                        float* out, prl_stream_t st) {
-  const bool few = moe_few_rows(n, pairs, max_tiles);
-  const int rc = moe_gemm_impl<ACT, true>(x, f32, W, n, up, f32, F * W, W, perm, meta, tiles, max_tiles, F, W, act_out, F, 0, wsel, few, st);
+                        const int32_t* meta, const int32_t* tiles, int64_t max_tiles, const float* wsel, void* act_out, float* out,
+                        prl_stream_t st) {
+  const int rc = moe_gemm_impl<ACT, true>(x, f32, W, n, up, f32, F * W, W, perm, meta, tiles, max_tiles, F, W, act_out, F, 0, wsel, st);
   return rc ? rc : moe_gemm_impl<kActNone, true>(act_out, f32, F, 0, down, f32, W * F, F, perm, meta, tiles, max_tiles, W, F, out, W, 1,
-                                                        nullptr, few, st);
+                                                 nullptr, st);
 }
 
 // Both products of ungated experts, prl_moe_gemm_act and prl_moe_gemm in one call: x [n, W], up [experts * F, W], down [experts * W, F] of
 // one type (f32, else bf16); act_out (a row of F per pair, in that type) is scratch between them, out (a row of W per pair) fp32, pair order.
-static int moe_mlp_any(const void* x, int32_t f32, int32_t n, const void* up, const void* down, int64_t W, int64_t F, const int32_t* perm,
-                       const int32_t* meta, const int32_t* tiles, int64_t max_tiles, int64_t pairs, int32_t act, const float* wsel,
-                       void* act_out, float* out, prl_stream_t st) {
-  PRL_CHECK_ARG(n >= 1 && act_out && (act == kActRelu2 || act == kActGelu), "prl_moe_mlp_act: bad argument (activation %d)", act);
-  return act == kActRelu2 ? moe_mlp_impl<kActRelu2>(x, f32, n, up, down, W, F, perm, meta, tiles, max_tiles, pairs, wsel, act_out, out, st)
-                          : moe_mlp_impl<kActGelu>(x, f32, n, up, down, W, F, perm, meta, tiles, max_tiles, pairs, wsel, act_out, out, st);
-}
 extern "C" int prl_moe_mlp_act(const void* x, int32_t f32, int32_t n, const void* up, const void* down, int64_t W, int64_t F,
                                const int32_t* perm, const int32_t* meta, const int32_t* tiles, int64_t max_tiles, int32_t act,
                                const float* wsel, void* act_out, float* out, prl_stream_t st) {
-  return moe_mlp_any(x, f32, n, up, down, W, F, perm, meta, tiles, max_tiles, 0, act, wsel, act_out, out, st);
-}
-
-// ... told how many pairs there are
-extern "C" int prl_moe_mlp_act_pairs(const void* x, int32_t f32, int32_t n, const void* up, const void* down, int64_t W, int64_t F,
-                                     const int32_t* perm, const int32_t* meta, const int32_t* tiles, int64_t max_tiles, int64_t pairs,
-                                     int32_t act, const float* wsel, void* act_out, float* out, prl_stream_t st) {
-  PRL_CHECK_ARG(pairs >= 1, "prl_moe_mlp_act_pairs: no pairs");
-  return moe_mlp_any(x, f32, n, up, down, W, F, perm, meta, tiles, max_tiles, pairs, act, wsel, act_out, out, st);
+  PRL_CHECK_ARG(n >= 1 && act_out && (act == kActRelu2 || act == kActGelu), "prl_moe_mlp_act: bad argument (activation %d)", act);
+  return act == kActRelu2 ? moe_mlp_impl<kActRelu2>(x, f32, n, up, down, W, F, perm, meta, tiles, max_tiles, wsel, act_out, out, st)
+                          : moe_mlp_impl<kActGelu>(x, f32, n, up, down, W, F, perm, meta, tiles, max_tiles, wsel, act_out, out, st);
 }
 
 extern "C" int prl_moe_glu(const float* gate_up, int64_t ld, int64_t pairs, int32_t F, const int32_t* perm,

@@ -1733,8 +1733,8 @@ class HybridEngine(EngineCore):
             _lib.check(lib.prl_moe_route(R.router.data_ptr(), e.experts, bias, n, e.experts, e.top, mode, *route))
         tiles = int(lib.prl_moe_max_tiles(pairs, e.experts))
         table = (R.perm.data_ptr(), R.moe_meta.data_ptr(), R.moe_tiles.data_ptr(), tiles)
-        _lib.check(lib.prl_moe_gemm_pairs(R.xa.data_ptr(), f32, W, n, self.arena.ptr(w + "mlp.experts.gate_up"), f32,
-                                          2 * e.ff * W, W, *table, pairs, 2 * e.ff, W, R.P.data_ptr(), 2 * e.ff, 0, st))
+        _lib.check(lib.prl_moe_gemm(R.xa.data_ptr(), f32, W, n, self.arena.ptr(w + "mlp.experts.gate_up"), f32,
+                                    2 * e.ff * W, W, *table, 2 * e.ff, W, R.P.data_ptr(), 2 * e.ff, 0, st))
         if e.weight_on == "output":      # plain SiLU unit, the score (times a constant) on the expert's output
             _lib.check(lib.prl_moe_glu_out(R.P.data_ptr(), 2 * e.ff, pairs, e.ff, R.perm.data_ptr(), R.wsel.data_ptr(),
                                            e.weight_scale, R.moe_act.data_ptr(), f32, st))
@@ -1974,8 +1974,8 @@ class HybridEngine(EngineCore):
             _lib.check(lib.prl_moe_gemm_tc(out, pairs, up, e.experts, e.ff, W, *table, R.wsel.data_ptr(), unit, act, e.ff, st))
             _lib.check(lib.prl_moe_gemm_tc(act, pairs, down, e.experts, W, e.ff, *table, None, 0, out, W, st))
             return R.moe_out
-        _lib.check(lib.prl_moe_mlp_act_pairs(R.xa.data_ptr(), f32, n, up, down, W, e.ff, *table, int(lib.prl_moe_max_tiles(pairs, e.experts)),
-                                             pairs, unit, R.wsel.data_ptr(), act, out, st))
+        _lib.check(lib.prl_moe_mlp_act(R.xa.data_ptr(), f32, n, up, down, W, e.ff, *table,
+                                       int(lib.prl_moe_max_tiles(pairs, e.experts)), unit, R.wsel.data_ptr(), act, out, st))
         return R.moe_out
 
     def _attn_core(self, R, n, i, L, w, segs, max_q, row_pos, seg_pos0, ld, decode) -> torch.Tensor:

@@ -69,13 +69,6 @@ def test_workspace_of_the_longest_contexts_is_enough(slots, n_kv, max_seq_len):
             assert splits <= most and -(-max_seq_len // 64) <= 1024 * splits
 
 
-@pytest.mark.parametrize("experts,top,tokens,few", [(16, 4, 1, 1), (16, 4, 60, 1), (16, 4, 61, 0), (16, 8, 44, 1), (16, 8, 45, 0), (64, 8, 176, 1), (64, 8, 177, 0),
-                                                    (64, 8, 309, 0), (3, 1, 9, 1), (3, 1, 13, 0), (1, 1, 3, 1), (4, 4, 22, 0)])
-def test_few_rows_per_expert(experts, top, tokens, few):
-    """Few tokens for the experts, and at most 22 rows each."""
-    assert _lib.load().prl_moe_few_rows(tokens, tokens * top, experts) == few
-
-
 def test_ring_budget_goes_back_to_the_rule():
     """A set budget is taken back by 0, the default; what no ring fits in stays refused."""
     lib = _lib.load()

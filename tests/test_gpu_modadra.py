@@ -655,31 +655,6 @@ def test_few_rows_per_expert_equal_many(cuda_device, counts, N, K):
     assert ((got - want).abs() <= K * 2.0 ** -24 * torch.einsum("sk,snk->sn", rows.double().abs(), W.double().abs().view(experts, N, K)[expert])).all()
 
 
-@pytest.mark.parametrize("experts,top,n", [(16, 8, 44), (16, 8, 45), (5, 2, 18), (5, 2, 19), (4, 4, 1), (24, 1, 70), (24, 1, 300)])
-def test_products_told_their_pairs(cuda_device, experts, top, n):
-    """prl_moe_mlp_act_pairs and prl_moe_gemm_pairs at both sides of the rule for few rows per expert: the bits of the products one at a time over gathered rows."""
-    from pipelinerl_b200 import _lib
-    lib, st, g = _lib.load(), _lib.stream_ptr(), torch.Generator(device="cuda").manual_seed(experts + n)
-    W, F, bf16, i32, ptr = 136, 72, torch.bfloat16, dict(dtype=torch.int32, device="cuda"), lambda t: t.data_ptr()  # noqa: E731
-    x, up, down = (torch.randn(r, c, generator=g, device="cuda").to(bf16) for r, c in ((n, W), (experts * F, W), (experts * W, F)))
-    choice = torch.rand(n, experts, generator=g, device="cuda").argsort(1)[:, :top].T.reshape(-1)       # pair j * n + token
-    perm, counts = choice.argsort(stable=True).to(torch.int32), torch.bincount(choice, minlength=experts).tolist()
-    rows = [(e, sum(counts[:e]) + r, min(64, c - r)) for e, c in enumerate(counts) for r in range(0, c, 64)]
-    pairs, most = n * top, int(lib.prl_moe_max_tiles(n * top, experts))
-    tiles, meta = torch.zeros(3 * most, **i32), torch.tensor([len(rows), 0, 0, 0], **i32)
-    tiles[:3 * len(rows)] = torch.tensor(rows, **i32).reshape(-1)
-    wsel, table = torch.rand(pairs, generator=g, device="cuda"), (ptr(perm), ptr(meta), ptr(tiles), most)
-    act, out, first = torch.zeros(pairs, F, dtype=bf16, device="cuda"), torch.zeros(pairs, W, device="cuda"), torch.zeros(pairs, F, device="cuda")
-    _lib.check(lib.prl_moe_mlp_act_pairs(ptr(x), 0, n, ptr(up), ptr(down), W, F, *table, pairs, 1, ptr(wsel), ptr(act), ptr(out), st))
-    _lib.check(lib.prl_moe_gemm_pairs(ptr(x), 0, W, n, ptr(up), 0, F * W, W, *table, pairs, F, W, ptr(first), F, 0, st))
-    xs = x[perm.long() % n].contiguous()
-    want_act, want, want_first = torch.zeros_like(act), torch.zeros_like(out), torch.zeros_like(first)
-    _lib.check(lib.prl_moe_gemm_act(ptr(xs), 0, W, 0, ptr(up), 0, F * W, W, *table, F, W, 1, ptr(wsel), ptr(want_act), F, st))
-    _lib.check(lib.prl_moe_gemm(ptr(want_act), 0, F, 0, ptr(down), 0, W * F, F, *table, W, F, ptr(want), W, 1, st))
-    _lib.check(lib.prl_moe_gemm(ptr(xs), 0, W, 0, ptr(up), 0, F * W, W, *table, F, W, ptr(want_first), F, 0, st))
-    assert torch.equal(act, want_act) and torch.equal(out, want) and torch.equal(first, want_first) and out.abs().max() > 0
-
-
 @pytest.mark.parametrize("heads,kh,dk,dv", [(16, 8, 128, 128), (4, 2, 64, 48), (6, 2, 20, 36), (4, 4, 32, 64)])
 def test_token_step_of_many_rows_equals_few(cuda_device, heads, kh, dk, dv):
     """One value head at a time in a CTA (more than 148 CTAs) or two: the same bits, for outputs, states and convolution inputs."""
